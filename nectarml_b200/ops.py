@@ -1,5 +1,6 @@
 """Tensor-level entry to the contraction path: torch tensors in (they only supply device memory
-and the stream), the C ABI underneath.
+and the stream), the C ABI underneath.  The per-call work (shape checks, allocation of the result, descriptor,
+workspace, stream) is done in ``csrc/nml_torch.cpp``.
 
 Each function corresponds to one host op of the reference:
 
@@ -28,11 +29,28 @@ import torch
 
 from . import _lib
 from ._lib import (NML_F16, NML_F32, NML_MATH_3XTF32, NML_MATH_F16, NML_MATH_TF32, NML_NCHW,
-                   NML_NHWC, NML_PASS_BACKWARD_DATA, NML_PASS_BACKWARD_WEIGHT, NML_PASS_FORWARD,
-                   ConvDesc, LinearDesc, check)
+                   NML_NHWC, ConvDesc, LinearDesc, check)
 
 _MATH = {"f16": NML_MATH_F16, "3xtf32": NML_MATH_3XTF32, "tf32": NML_MATH_TF32}
 _LAYOUT = {"nchw": NML_NCHW, "nhwc": NML_NHWC}
+
+
+class _LazyNative:
+    """Stands in for the native module until its first use, so that this file can be imported before the build."""
+
+    def __getattr__(self, name):
+        global _native
+        _lib.load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise _lib.NectarB200Error(f"nectarml_b200/_native.so: {e}; build it with `python -m nectarml_b200.build`") from e
+        _native = module
+        return getattr(module, name)
+
+
+_native = _LazyNative()
+_DTYPE = {torch.float32: NML_F32, torch.float16: NML_F16, None: -1}
 
 
 def _dt(t: torch.dtype) -> int:
@@ -57,6 +75,12 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+def _out_dtype(t: Optional[torch.dtype]) -> int:
+    """Code of a result dtype; -1: that of the call's first tensor."""
+    code = _DTYPE.get(t)
+    return _dt(t) if code is None else code
+
+
 @dataclass(frozen=True)
 class ConvGeometry:
     """Shape of one Conv2d (``transposed=False``) or ConvTranspose2d layer, input side first."""
@@ -72,6 +96,18 @@ class ConvGeometry:
     dilation: Tuple[int, int] = (1, 1)
     output_padding: Tuple[int, int] = (0, 0)
     transposed: bool = False
+
+    def native(self):
+        """The geometry as the native host path takes it; parsed once per object."""
+        h = self.__dict__.get("_native")
+        if h is None:
+            h = _native.geometry(self.batch, self.c_in, self.h, self.w, self.c_out, self.kh, self.kw, *self.stride, *self.padding,
+                                 *self.dilation, *self.output_padding, int(self.transposed))
+            self.__dict__["_native"] = h  # (a frozen dataclass: fields, equality and hash are not touched)
+        return h
+
+    def __getstate__(self):  # copies and pickles carry the fields alone
+        return {k: v for k, v in self.__dict__.items() if k != "_native"}
 
     def out_hw(self) -> Tuple[int, int]:
         d = self.desc(NML_F32, "nchw", NML_F32, "nchw", NML_F32, "f16", False)
@@ -127,44 +163,22 @@ class Workspace:
 _default_ws = Workspace()
 
 
-def _conv_ws(d: ConvDesc, which: int, ws: Optional[Workspace], device):
-    need = C.c_size_t()
-    check(_lib.load().nml_conv_workspace_size(C.byref(d), which, C.byref(need)))
-    return (ws or _default_ws).get(need.value, device)
-
-
 def conv_forward(g: ConvGeometry, x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, *,
                  layout: str = "nchw", out_layout: Optional[str] = None, math: str = "f16",
                  out_dtype: Optional[torch.dtype] = None, round_out_f16: bool = False,
                  out: Optional[torch.Tensor] = None, ws: Optional[Workspace] = None) -> torch.Tensor:
-    out_layout = out_layout or layout
-    out_dtype = out_dtype or x.dtype
-    assert tuple(x.shape) == g.act_shape("in", layout), (tuple(x.shape), g.act_shape("in", layout))
-    assert tuple(w.shape) == g.weight_shape()
-    if bias is not None:
-        assert bias.dtype == w.dtype and bias.numel() == g.c_out
-    if out is None:
-        out = torch.empty(g.act_shape("out", out_layout), dtype=out_dtype, device=x.device)
-    d = g.desc(_dt(x.dtype), layout, _dt(out.dtype), out_layout, _dt(w.dtype), math, round_out_f16)
-    wp, wb = _conv_ws(d, NML_PASS_FORWARD, ws, x.device)
-    check(_lib.load().nml_conv_forward(C.byref(d), _ptr(x), _ptr(w), _ptr(bias), _ptr(out), wp, wb, _stream()))
-    return out
+    lay = _LAYOUT[layout]
+    return _native.conv_forward(g.native(), x, w, bias, out, lay, _LAYOUT[out_layout] if out_layout else lay, _MATH[math],
+                                _out_dtype(out_dtype), 1 if round_out_f16 else 0, ws or _default_ws)
 
 
 def conv_backward_data(g: ConvGeometry, dy: torch.Tensor, w: torch.Tensor, *, layout: str = "nchw",
                        out_layout: Optional[str] = None, math: str = "f16",
                        out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None,
                        ws: Optional[Workspace] = None) -> torch.Tensor:
-    out_layout = out_layout or layout
-    out_dtype = out_dtype or dy.dtype
-    assert tuple(dy.shape) == g.act_shape("out", layout)
-    assert tuple(w.shape) == g.weight_shape()
-    if out is None:
-        out = torch.empty(g.act_shape("in", out_layout), dtype=out_dtype, device=dy.device)
-    d = g.desc(_dt(dy.dtype), layout, _dt(out.dtype), out_layout, _dt(w.dtype), math, False)
-    wp, wb = _conv_ws(d, NML_PASS_BACKWARD_DATA, ws, dy.device)
-    check(_lib.load().nml_conv_backward_data(C.byref(d), _ptr(dy), _ptr(w), _ptr(out), wp, wb, _stream()))
-    return out
+    lay = _LAYOUT[layout]
+    return _native.conv_backward_data(g.native(), dy, w, out, lay, _LAYOUT[out_layout] if out_layout else lay, _MATH[math],
+                                      _out_dtype(out_dtype), ws or _default_ws)
 
 
 def conv_backward_weight(g: ConvGeometry, x: torch.Tensor, dy: torch.Tensor, *, layout: str = "nchw",
@@ -173,19 +187,8 @@ def conv_backward_weight(g: ConvGeometry, x: torch.Tensor, dy: torch.Tensor, *, 
                          ws: Optional[Workspace] = None) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """dw (fp32, weight-shaped) and db (fp32, c_out); pass ``dw`` / ``db`` to have them written in place, e.g.
     into the views of a flat gradient bucket."""
-    assert tuple(x.shape) == g.act_shape("in", layout)
-    assert tuple(dy.shape) == g.act_shape("out", layout)
-    assert x.dtype == dy.dtype
-    if dw is None:
-        dw = torch.empty(g.weight_shape(), dtype=torch.float32, device=x.device)
-    if db is None and want_bias_grad:
-        db = torch.empty(g.c_out, dtype=torch.float32, device=x.device)
-    assert dw.dtype == torch.float32 and dw.numel() == g.c_in * g.c_out * g.kh * g.kw
-    d = g.desc(_dt(x.dtype), layout, NML_F32, layout, NML_F32, math, False)
-    wp, wb = _conv_ws(d, NML_PASS_BACKWARD_WEIGHT, ws, x.device)
-    check(_lib.load().nml_conv_backward_weight(C.byref(d), _ptr(x), _ptr(dy), _ptr(dw), _ptr(db), wp, wb,
-                                               _stream()))
-    return dw, db
+    return _native.conv_backward_weight(g.native(), x, dy, dw, db, _LAYOUT[layout], _MATH[math], 1 if want_bias_grad else 0,
+                                        ws or _default_ws)
 
 
 def _linear_desc(rows, fin, fout, in_dtype, out_dtype, w_dtype, math, round_out_f16) -> LinearDesc:
@@ -197,58 +200,25 @@ def _linear_desc(rows, fin, fout, in_dtype, out_dtype, w_dtype, math, round_out_
     return d
 
 
-def _linear_ws(d: LinearDesc, which: int, ws: Optional[Workspace], device):
-    need = C.c_size_t()
-    check(_lib.load().nml_linear_workspace_size(C.byref(d), which, C.byref(need)))
-    return (ws or _default_ws).get(need.value, device)
-
-
 def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, *, math: str = "f16",
                    out_dtype: Optional[torch.dtype] = None, round_out_f16: bool = False,
                    out: Optional[torch.Tensor] = None, ws: Optional[Workspace] = None) -> torch.Tensor:
     """y[rows, out] = x[rows, in] @ w[out, in].T + bias."""
-    rows, fin = x.shape
-    fout = w.shape[0]
-    assert w.shape[1] == fin
-    if out is None:
-        out = torch.empty((rows, fout), dtype=out_dtype or x.dtype, device=x.device)
-    d = _linear_desc(rows, fin, fout, _dt(x.dtype), _dt(out.dtype), _dt(w.dtype), math, round_out_f16)
-    wp, wb = _linear_ws(d, NML_PASS_FORWARD, ws, x.device)
-    check(_lib.load().nml_linear_forward(C.byref(d), _ptr(x), _ptr(w), _ptr(bias), _ptr(out), wp, wb, _stream()))
-    return out
+    return _native.linear_forward(x, w, bias, out, _MATH[math], _out_dtype(out_dtype), 1 if round_out_f16 else 0, ws or _default_ws)
 
 
 def linear_backward_data(dy: torch.Tensor, w: torch.Tensor, *, math: str = "f16",
                          out_dtype: Optional[torch.dtype] = None, out: Optional[torch.Tensor] = None,
                          ws: Optional[Workspace] = None) -> torch.Tensor:
     """dx[rows, in] = dy[rows, out] @ w[out, in]."""
-    rows, fout = dy.shape
-    fin = w.shape[1]
-    assert w.shape[0] == fout
-    if out is None:
-        out = torch.empty((rows, fin), dtype=out_dtype or dy.dtype, device=dy.device)
-    d = _linear_desc(rows, fin, fout, _dt(dy.dtype), _dt(out.dtype), _dt(w.dtype), math, False)
-    wp, wb = _linear_ws(d, NML_PASS_BACKWARD_DATA, ws, dy.device)
-    check(_lib.load().nml_linear_backward_data(C.byref(d), _ptr(dy), _ptr(w), _ptr(out), wp, wb, _stream()))
-    return out
+    return _native.linear_backward_data(dy, w, out, _MATH[math], _out_dtype(out_dtype), ws or _default_ws)
 
 
 def linear_backward_weight(x: torch.Tensor, dy: torch.Tensor, *, math: str = "f16", want_bias_grad: bool = True,
                            dw: Optional[torch.Tensor] = None, db: Optional[torch.Tensor] = None,
                            ws: Optional[Workspace] = None) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """dw[out, in] = dy.T @ x (fp32), db[out] = dy.sum(0) (fp32)."""
-    rows, fin = x.shape
-    fout = dy.shape[1]
-    assert dy.shape[0] == rows and x.dtype == dy.dtype
-    if dw is None:
-        dw = torch.empty((fout, fin), dtype=torch.float32, device=x.device)
-    if db is None and want_bias_grad:
-        db = torch.empty(fout, dtype=torch.float32, device=x.device)
-    d = _linear_desc(rows, fin, fout, _dt(x.dtype), NML_F32, NML_F32, math, False)
-    wp, wb = _linear_ws(d, NML_PASS_BACKWARD_WEIGHT, ws, x.device)
-    check(_lib.load().nml_linear_backward_weight(C.byref(d), _ptr(x), _ptr(dy), _ptr(dw), _ptr(db), wp, wb,
-                                                 _stream()))
-    return dw, db
+    return _native.linear_backward_weight(x, dy, dw, db, _MATH[math], 1 if want_bias_grad else 0, ws or _default_ws)
 
 
 def device_status() -> int:

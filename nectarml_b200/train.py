@@ -19,7 +19,6 @@ layer, so the exchange starts as early as it can).
 from __future__ import annotations
 
 import contextlib
-import ctypes as C
 import gc
 from typing import List, Optional, Sequence, Tuple
 
@@ -110,12 +109,22 @@ class ParamStore:
         # per SM; see nml_set_sm_limit)
         self.sm_reserve = 16
         self.sms = torch.cuda.get_device_properties(self.device).multi_processor_count if self.device.type == "cuda" else 0
+        self._views = {}
+        self._bucket_index = {a: self._bucket_of(a) for a, _ in self.layer_ranges}
 
     def _view(self, buf, i):
+        """Parameter i's part of one of the flat buffers, made once per buffer (a view costs more host time than the
+        rest of a small layer's call)."""
+        key = (id(buf), i)
+        hit = self._views.get(key)
+        if hit is not None and hit[0] is buf:
+            return hit[1]
         cnt = 1
         for d in self.shapes[i]:
             cnt *= d
-        return buf[self.offsets[i]:self.offsets[i] + cnt].view(self.shapes[i])
+        v = buf[self.offsets[i]:self.offsets[i] + cnt].view(self.shapes[i])
+        self._views[key] = (buf, v)
+        return v
 
     def w32(self, i): return self._view(self.p32, i)
     def w16(self, i): return self._view(self.p16, i)
@@ -128,8 +137,8 @@ class ParamStore:
     def begin_backward(self, last_micro_batch: bool) -> None:
         nb = len(self.bucket_bounds) - 1
         self._bucket_left = [0] * nb
-        for (a, e) in self.layer_ranges:
-            self._bucket_left[self._bucket_of(a)] += 1
+        for b in self._bucket_index.values():
+            self._bucket_left[b] += 1
         self._exchange = last_micro_batch and self.world > 1 and self.communicate
 
     def _bucket_of(self, elem: int) -> int:
@@ -140,7 +149,7 @@ class ParamStore:
 
     def layer_done(self, first_elem: int) -> None:
         """Called when a layer has written its gradients; all-reduces the layer's bucket once it is complete."""
-        b = self._bucket_of(first_elem)
+        b = self._bucket_index[first_elem]
         self._bucket_left[b] -= 1
         if self._bucket_left[b] == 0 and self._exchange:
             lo, hi = self.bucket_bounds[b], self.bucket_bounds[b + 1]
@@ -166,12 +175,6 @@ class ParamStore:
 
 
 _bn_ws = ops.Workspace()
-
-
-def _bn_workspace(rows: int, c: int, device):
-    need = C.c_size_t()
-    _lib.check(_lib.load().nml_bn_workspace_size(rows, c, C.byref(need)))
-    return _bn_ws.get(need.value, device)
 
 
 # ------------------------------------------------------------------ autograd nodes --
@@ -223,15 +226,7 @@ class _BnActFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, residual, token, layer, act):
-        rows, c = x.numel() // x.shape[-1], x.shape[-1]
-        y = torch.empty_like(x)
-        mean = torch.empty(c, dtype=torch.float32, device=x.device)
-        rstd = torch.empty(c, dtype=torch.float32, device=x.device)
-        wp, wb = _bn_workspace(rows, c, x.device)
-        _lib.check(_lib.load().nml_bn_forward(x.data_ptr(), rows, c, layer.gamma.data_ptr(), layer.beta.data_ptr(),
-                                              residual.data_ptr() if residual is not None else None, act, 0.2, layer.eps,
-                                              y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), wp, wb,
-                                              torch.cuda.current_stream().cuda_stream))
+        y, mean, rstd = ops._native.bn_forward(x, residual, layer.gamma, layer.beta, act, 0.2, layer.eps, _bn_ws)
         ctx.layer, ctx.act, ctx.has_res = layer, act, residual is not None
         ctx.save_for_backward(x, y, mean, rstd)
         return y
@@ -241,18 +236,13 @@ class _BnActFn(torch.autograd.Function):
         layer = ctx.layer
         x, y, mean, rstd = ctx.saved_tensors
         dy = dy.contiguous()
-        rows, c = x.numel() // x.shape[-1], x.shape[-1]
-        dx = torch.empty_like(x)
-        dres = torch.empty_like(x) if ctx.has_res else None
-        wp, wb = _bn_workspace(rows, c, x.device)
+        grads = None
 
         def run(dgamma, dbeta):
-            _lib.check(_lib.load().nml_bn_backward(dy.data_ptr(), y.data_ptr(), x.data_ptr(), rows, c, layer.gamma.data_ptr(),
-                                                   mean.data_ptr(), rstd.data_ptr(), ctx.act, 0.2, dx.data_ptr(),
-                                                   dres.data_ptr() if dres is not None else None, dgamma.data_ptr(),
-                                                   dbeta.data_ptr(), wp, wb, torch.cuda.current_stream().cuda_stream))
+            nonlocal grads
+            grads = ops._native.bn_backward(dy, y, x, layer.gamma, mean, rstd, ctx.act, 0.2, int(ctx.has_res), dgamma, dbeta, _bn_ws)
         layer.weight_gradient(run)
-        return dx, dres, None, None, None
+        return grads[0], grads[1], None, None, None
 
 
 class _MaxPoolFn(torch.autograd.Function):
@@ -321,6 +311,7 @@ class Conv(_Layer):
         super().__init__(store, wshape, (c_out,) if bias else None)
         self.c_in, self.c_out, self.k, self.stride, self.pad, self.transposed = c_in, c_out, k, stride, pad, transposed
         self.needs_dx = needs_dx
+        self._geometries = {}    # by input shape
 
     @property
     def w16(self): return self.store.w16(self.ia)
@@ -328,10 +319,17 @@ class Conv(_Layer):
     def b16(self): return self.store.w16(self.ib) if self.ib is not None else None
 
     def geometry(self, x) -> ConvGeometry:
-        n, h, w, c = x.shape
-        assert c == self.c_in, (c, self.c_in)
-        return ConvGeometry(n, c, h, w, self.c_out, self.k, self.k, (self.stride, self.stride), (self.pad, self.pad),
-                            transposed=self.transposed)
+        shape = tuple(x.shape)
+        g = self._geometries.get(shape)
+        if g is None:
+            n, h, w, c = shape
+            assert c == self.c_in, (c, self.c_in)
+            g = ConvGeometry(n, c, h, w, self.c_out, self.k, self.k, (self.stride, self.stride), (self.pad, self.pad),
+                             transposed=self.transposed)
+            if len(self._geometries) >= 16:  # (a program with ever new image sizes)
+                self._geometries.clear()
+            self._geometries[shape] = g
+        return g
 
     def __call__(self, x, token):
         return _ConvFn.apply(x, token, self)

@@ -89,6 +89,8 @@ struct KParams {
     int ka;              // K atoms (128-byte-wide operand slices) per stage; narrow tiles take 2 to amortise the
                          // per-stage barrier round trip over 8 MMAs
     int a_mn_major, b_mn_major;
+    int b_batched;       // 1: every image (batch entry) has a B of its own, the outermost dimension of tmB (batched matmul;
+                         // tiles of one image each, no pairs, no patch walk)
     int a_grouped, b_grouped;  // MN-major operand fetched as ONE box whose outermost dimension walks
                                // the 128-byte column groups (needs the channel count to be a multiple of kb)
     // Patch walk (forward walk, unit stride, several taps): instead of one 128-row box per tap, the A
@@ -217,56 +219,20 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Stores 32 (or fewer) consecutive output columns of one accumulator row.
-__device__ __noinline__ void store_row_chunk(const KParams& P, const float (&v)[32], size_t row_off,
-                                                size_t col_stride, int cg, int ncols) {
-    if (P.out_mode == OUT_NHWC) {
-        if (P.out_f16) {
-            __half* o = reinterpret_cast<__half*>(P.out) + row_off + cg;
-            if (ncols == 32 && (P.ld_out & 7) == 0) {
+// Stores 32 (or fewer) consecutive output channels of one accumulator row to a channel-major output: lanes are
+// consecutive pixels, so each column store coalesces.
+__device__ __noinline__ void store_row_chunk(const KParams& P, const float (&v)[32], size_t row_off, size_t col_stride,
+                                             int cg, int ncols) {
+    if (P.out_f16) {
+        __half* o = reinterpret_cast<__half*>(P.out) + row_off + static_cast<size_t>(cg) * col_stride;
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    uint4 pk;
-                    __half2 h0 = __floats2half2_rn(v[8 * q + 0], v[8 * q + 1]);
-                    __half2 h1 = __floats2half2_rn(v[8 * q + 2], v[8 * q + 3]);
-                    __half2 h2 = __floats2half2_rn(v[8 * q + 4], v[8 * q + 5]);
-                    __half2 h3 = __floats2half2_rn(v[8 * q + 6], v[8 * q + 7]);
-                    pk.x = *reinterpret_cast<uint32_t*>(&h0);
-                    pk.y = *reinterpret_cast<uint32_t*>(&h1);
-                    pk.z = *reinterpret_cast<uint32_t*>(&h2);
-                    pk.w = *reinterpret_cast<uint32_t*>(&h3);
-                    reinterpret_cast<uint4*>(o)[q] = pk;
-                }
-            } else {
+        for (int j = 0; j < 32; ++j)
+            if (j < ncols) o[j * col_stride] = __float2half_rn(v[j]);
+    } else {
+        float* o = reinterpret_cast<float*>(P.out) + row_off + static_cast<size_t>(cg) * col_stride;
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (j < ncols) o[j] = __float2half_rn(v[j]);
-            }
-        } else {
-            float* o = reinterpret_cast<float*>(P.out) + row_off + cg;
-            if (ncols == 32 && (P.ld_out & 3) == 0) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    reinterpret_cast<float4*>(o)[q] =
-                        make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (j < ncols) o[j] = v[j];
-            }
-        }
-    } else {  // OUT_NCHW: lanes are consecutive pixels, so each column store coalesces
-        if (P.out_f16) {
-            __half* o = reinterpret_cast<__half*>(P.out) + row_off + static_cast<size_t>(cg) * col_stride;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (j < ncols) o[j * col_stride] = __float2half_rn(v[j]);
-        } else {
-            float* o = reinterpret_cast<float*>(P.out) + row_off + static_cast<size_t>(cg) * col_stride;
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (j < ncols) o[j * col_stride] = v[j];
-        }
+        for (int j = 0; j < 32; ++j)
+            if (j < ncols) o[j * col_stride] = v[j];
     }
 }
 
@@ -450,9 +416,19 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             int issued = 0;
             const uint32_t a_bytes = kStageABytes;
             const uint32_t tx_bytes = do_a ? a_bytes : stage_b_bytes;  // this producer's share of one atom
-            // B slice of (tap, channel block, column tile) -> shared memory at sb
-            auto load_b = [&](uint32_t sb, const CUtensorMap* tb, uint32_t fb, const Tap& tap, int cb, int ntile) {
-                if (!P.b_mn_major) {
+            // B slice of (tap, channel block, column tile[, image]) -> shared memory at sb
+            auto load_b = [&](uint32_t sb, const CUtensorMap* tb, uint32_t fb, const Tap& tap, int cb, int ntile, int image) {
+                if (P.b_batched) {
+                    if (!P.b_mn_major) {
+                        tma_load_3d(sb, tb, fb, tap.wk + cb * P.kb, ntile * P.bn, image);
+                    } else if (P.b_grouped) {
+                        tma_load_4d(sb, tb, fb, 0, tap.wk + cb * P.kb, (ntile * P.bn) / P.kb, image);
+                    } else {
+                        const int nb = P.bn / P.kb;
+                        for (int j = 0; j < nb; ++j)
+                            tma_load_3d(sb + j * box_bytes, tb, fb, ntile * P.bn + j * P.kb, tap.wk + cb * P.kb, image);
+                    }
+                } else if (!P.b_mn_major) {
                     tma_load_2d(sb, tb, fb, tap.wk + cb * P.kb, ntile * P.bn);
                 } else if (P.b_grouped) {
                     tma_load_3d(sb, tb, fb, 0, tap.wk + cb * P.kb, (ntile * P.bn) / P.kb);
@@ -544,7 +520,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                                     mbar_arrive_expect_tx(fb, n * stage_b_bytes);
                                     for (int j = 0; j < n; ++j)
                                         load_b(smem_u32(smem) + (stage * P.ka + j) * stage_b_bytes, tb, fb,
-                                               P.taps[pt.tap_begin + t + j], cb, ntile);
+                                               P.taps[pt.tap_begin + t + j], cb, ntile, 0);
                                     ++issued;
                                     if (++stage == P.stages) {
                                         stage = 0;
@@ -627,7 +603,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             } else if (do_a) {
                                 tma_load_4d(sa, ta, fb, cb * P.kb, w0 + tap.dw, h0 + tap.dh, n0);
                             } else {
-                                load_b(sb, tb, fb, tap, cb, ntile);
+                                load_b(sb, tb, fb, tap, cb, ntile, n0);
                             }
                         }
                         advance(P.ka);
@@ -1603,7 +1579,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 for (int c0 = 0; c0 < P.bn; c0 += cpi) {
                     const int cg = col_base + c0;
                     if (cg >= P.c_out) break;  // uniform across the warp
-                    const int ncols = min(min(cpi, P.bn - c0), P.c_out - cg);
+                    const int ncols = min(min(cpi, P.bn - c0), P.c_out - cg);  // (a tail of the tile or of the row)
                     const int cn = c0 + cpi;   // next piece
                     const bool more = live && cn < P.bn && col_base + cn < P.c_out;
                     if (ncols == cpi && aligned) {
@@ -1672,28 +1648,64 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         __syncwarp();
                         if (more) tmem_ld_wait();
                     } else {
-                        // ragged tail or unaligned rows: per-thread stores, 32 columns at a time
-#pragma unroll 1
-                        for (int half = 0; half < 2; ++half) {
-                            const int cgh = cg + half * 32;
-                            const int nh = min(32, ncols - half * 32);
-                            if (nh <= 0) break;
-                            float v[32];
+                        // Ragged tail, or rows that do not start on 16 bytes: the piece goes through the staging tile as
+                        // above and leaves row by row, the lanes along the row.  (A thread storing its own row touches
+                        // 32 sectors per instruction: 333 x 64 x 333 matmuls spent 22 us each in it.)
+                        const float bias_lo = (has_bias && lane < ncols) ? __ldg(P.bias + cg + lane) : 0.f;
+                        const float bias_hi = (kOutF16 && has_bias && lane + 32 < ncols) ? __ldg(P.bias + cg + 32 + lane) : 0.f;
+                        if (kOutF16) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) {  // one bank per lane: word (lane, j) of a 33-word pitch
+                                const float b0 = __shfl_sync(0xffffffffu, j < 16 ? bias_lo : bias_hi, (2 * j) & 31);
+                                const float b1 = __shfl_sync(0xffffffffu, j < 16 ? bias_lo : bias_hi, (2 * j + 1) & 31);
+                                const uint32_t* src = j < 16 ? &r0[2 * j] : &r1[2 * j - 32];
+                                const uint32_t pk = pack_half2(__uint_as_float(src[0]) + b0, __uint_as_float(src[1]) + b1);
+                                asm volatile("st.shared.b32 [%0], %1;" ::"r"(stg + lane * 128 + ((j ^ lane) << 2)), "r"(pk) : "memory");
+                            }
+                        } else {
 #pragma unroll
                             for (int j = 0; j < 32; ++j) {
-                                float xv = __uint_as_float(half == 0 ? r0[j] : r1[j]);
-                                if (has_bias && j < nh) xv += P.bias[cgh + j];
+                                float xv = __uint_as_float(r0[j]) + __shfl_sync(0xffffffffu, bias_lo, j);
                                 if (P.round_f16) xv = round_through_f16(xv);
-                                v[j] = xv;
+                                asm volatile("st.shared.b32 [%0], %1;" ::"r"(stg + lane * 128 + ((j ^ lane) << 2)), "r"(__float_as_uint(xv)) : "memory");
                             }
-                            if (row_valid) store_row_chunk(P, v, row_off, col_stride, cgh, nh);
                         }
-                        __syncwarp();
                         if (more) {
                             tmem_ld_32x32(t_row + cn, r0);
                             if (cpi == 64 && cn + 32 < P.bn) tmem_ld_32x32(t_row + cn + 32, r1);
-                            tmem_ld_wait();
                         }
+                        __syncwarp();
+#pragma unroll 1
+                        for (int rb = 0; rb < 32; rb += 8) {  // eight rows at a time: their loads and stores overlap
+                            uint32_t v[8];
+                            unsigned long long off[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const int rr = rb + i;
+                                off[i] = __shfl_sync(0xffffffffu, row_valid ? static_cast<unsigned long long>(row_off) + cg : ~0ull, rr);
+                                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v[i]) : "r"(stg + rr * 128 + ((lane ^ rr) << 2)));
+                            }
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                const bool valid = off[i] != ~0ull;
+                                if (!kOutF16) {
+                                    if (valid && lane < ncols) reinterpret_cast<float*>(P.out)[off[i] + lane] = __uint_as_float(v[i]);
+                                } else {
+                                    // columns 2 * lane, 2 * lane + 1; a row on an odd element is stored as pairs one column later
+                                    __half* o = reinterpret_cast<__half*>(P.out) + off[i];
+                                    const int odd = static_cast<int>((reinterpret_cast<uintptr_t>(o) >> 1) & 1);
+                                    const uint32_t next = __shfl_down_sync(0xffffffffu, v[i], 1);
+                                    const uint32_t w = odd ? __funnelshift_r(v[i], next, 16) : v[i];
+                                    const int c = 2 * lane + odd;
+                                    const bool both = c + 1 < ncols;
+                                    if (valid && both) *reinterpret_cast<uint32_t*>(o + c) = w;
+                                    if (valid && !both && c < ncols) reinterpret_cast<uint16_t*>(o)[c] = static_cast<uint16_t>(w);
+                                    if (valid && odd && lane == 0) reinterpret_cast<uint16_t*>(o)[0] = static_cast<uint16_t>(v[i]);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                        if (more) tmem_ld_wait();
                     }
                 }
             } else

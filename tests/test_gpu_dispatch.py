@@ -1,0 +1,29 @@
+"""Sizes at the edges of the dispatch rules: batched products in one launch, rows that do not start on 16 bytes, K
+split over CTAs for few-tile layers.  fp16 results are compared with the oracle on fp16-rounded inputs (1e-2 rel / 1e-3
+abs), fp32 ones with 1e-5 of max|ref|, as everywhere in this suite."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import F16, F32, assert_f16, assert_f32, dev, fetch, host
+from nectarml_b200 import _nectarml, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fout", [1, 2, 9, 31, 33, 63, 65, 127, 257, 333])
+@pytest.mark.parametrize("rows", [1, 130])
+def test_rows_that_do_not_start_on_16_bytes(rows, fout, oracle):
+    rng = np.random.default_rng(rows * 1000 + fout)
+    x = rng.standard_normal((rows, 72), dtype=np.float32)
+    w = (rng.standard_normal((fout, 72), dtype=np.float32) * 0.2).astype(np.float32)
+    b = rng.standard_normal(fout, dtype=np.float32)
+    assert_f32(host(ops.linear_forward(dev(x), dev(w), dev(b), math="3xtf32")), oracle.linear_forward(x, w, b), "fp32")
+    r, h = oracle.round_f16, torch.float16
+    want = oracle.linear_forward(r(x), r(w), r(b))
+    assert_f16(host(ops.linear_forward(dev(x, h), dev(w, h), dev(b, h))), want, "fp16")
+    assert_f16(host(ops.linear_forward(dev(x, h), dev(w, h))), oracle.linear_forward(r(x), r(w), None), "fp16, no bias")
+    got = host(ops.linear_forward(dev(x), dev(w), dev(b), math="f16", round_out_f16=True))
+    assert_f16(got, want, "fp32 tensors, fp16 arithmetic")
+    assert np.array_equal(got, r(got)), "rounded through fp16"
+    ops.device_status()

@@ -329,6 +329,13 @@ static int colsum_finish(const ColsumScratch& cs, int C, float* out, cudaStream_
     return NML_OK;
 }
 
+static void convert_rows(const void* src, int dtype, void* p0, void* p1, int enc, size_t rows, int c, int cp, cudaStream_t st) {
+    const int blocks = static_cast<int>(std::min<size_t>((rows * (cp / 4) + 255) / 256, 148 * 16));
+    if (dtype == NML_F32) convert_rows_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(src), p0, p1, enc, rows, c, cp);
+    else convert_rows_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(src), p0, p1, enc, rows, c, cp);
+    ++g_launches;
+}
+
 // Converts an activation tensor into the NHWC operand encoding of `mi` unless it already is one.
 // planes[0..1] receive the operand pointers, *cp the padded channel count.  With `colsum` the
 // per-channel sums of the tensor (the bias gradient) are produced in the same pass where there is one.
@@ -390,14 +397,7 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
             if (rc) return rc;
         }
     } else {
-        size_t total = pixels * Cp;
-        int blocks = static_cast<int>(std::min<size_t>((total + 255) / 256, 148 * 16));
-        if (dtype == NML_F32)
-            { convert_rows_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(src), p0, p1, mi.enc, pixels,
-                                                              c, Cp); ++g_launches; }
-        else
-            { convert_rows_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(src), p0, p1, mi.enc,
-                                                               pixels, c, Cp); ++g_launches; }
+        convert_rows(src, dtype, p0, p1, mi.enc, pixels, c, Cp, st);
         if (colsum) {
             int rc = rows_colsum(cs);
             if (rc) return rc;
@@ -618,6 +618,10 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     return NML_OK;
 }
 
+// Microseconds one 128-byte-deep K slice of a 128-row tile keeps an SM busy, by tile width: 512 clocks of MMA at 256
+// columns; narrower tiles cost more per column (measured: 1.28x at 128, 2.24x at 64).
+static double slice_us(int bn) { return 0.27 * (bn / 256.0) * (bn > 128 ? 1.0 : bn > 64 ? 1.28 : 2.24); }
+
 // ------------------------------------------------------- fprop-like problems --
 struct FpropLike {
     const void* a;
@@ -633,6 +637,7 @@ struct FpropLike {
     int math, round_f16;
     // phase-packed gather walk (set by run_fprop_like itself): the real output behind the packed columns
     int shuf_sh, shuf_sw, shuf_c, shuf_oh, shuf_ow;
+    int w_batched;  // every image has its own [d0][d1] weights, one after the other (batched matmul; kh = kw = 1)
 };
 
 static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
@@ -747,7 +752,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     } else if (direct_w) {
         b_mn_major = f.k_is_dim0 ? 1 : 0;
     } else {
-        size_t bytes = static_cast<size_t>(N) * T * kp * mi.es;
+        size_t bytes = static_cast<size_t>(N) * T * kp * mi.es * (f.w_batched ? f.batch : 1);
         void* p0 = ws.take(bytes);
         void* p1 = (mi.planes == 2) ? ws.take(bytes) : nullptr;
         w_planes[0] = p0;
@@ -755,8 +760,12 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         if (!ws.dry) {
             if (!ws.fits()) return NML_ERR_WORKSPACE;
             // out[n][t][k] = w[...]: a swap of the two inner dimensions of [B][R][Cc] (see repack_weight_*_kernel)
-            const int rB = f.k_is_dim0 ? 1 : f.d0, rR = f.k_is_dim0 ? f.d0 : f.d1, rC = f.k_is_dim0 ? f.d1 * T : T;
+            // (batched: one such array per image)
+            const int rB = f.w_batched ? f.batch : (f.k_is_dim0 || T == 1) ? 1 : f.d0, rR = f.k_is_dim0 ? f.d0 : f.d1, rC = f.k_is_dim0 ? f.d1 * T : T;
             if (rB > 65535) return NML_ERR_UNSUPPORTED;
+            // One tap and K innermost already: nothing to transpose, rows are only converted and padded (the repack
+            // would have run one 64-element block per row: 24 us for 1000 x 2048).
+            const bool rows_only = T == 1 && !f.k_is_dim0;
 #define NML_REPACK(T)                                                                                                           \
     do {                                                                                                                        \
         if (rC <= 64)                                                                                                           \
@@ -766,9 +775,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             repack_weight_tile_kernel<T><<<dim3(ceil_div(rC, 64), ceil_div(kp, 64), rB), 256, 0, st>>>(                          \
                 static_cast<const T*>(f.w), p0, p1, mi.enc, rR, rC, kp);                                                         \
     } while (0)
-            if (f.w_dtype == NML_F32) NML_REPACK(float); else NML_REPACK(__half);
+            if (rows_only) convert_rows(f.w, f.w_dtype, p0, p1, mi.enc, static_cast<size_t>(rB) * f.d0, f.d1, kp, st);
+            else if (f.w_dtype == NML_F32) NML_REPACK(float); else NML_REPACK(__half);
 #undef NML_REPACK
-            ++g_launches;
+            if (!rows_only) ++g_launches;
             NML_CUDA(cudaGetLastError());
         }
     }
@@ -779,19 +789,21 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     const bool bias_is_f16 = f.bias && f.bias_dtype == NML_F16;
     float* bias_widened = bias_is_f16 ? static_cast<float*>(ws.take(sizeof(float) * N)) : nullptr;
     if (bias_is_f16) bias32 = bias_widened;
-    // Few output pixels under a long K loop (the 2x2 ... 8x8 layers of a U-Net): room for the fp32 partial
-    // sums of a K-split walk.
+    // Few output pixels under a long K loop (the 2x2 ... 8x8 layers of a U-Net, Linear layers on a few hundred rows):
+    // room for the fp32 partial sums of a K-split walk.
     const size_t out_pixels = static_cast<size_t>(f.batch) * f.out_h * f.out_w;
-    const bool may_split = !window && !f.shuf_sh && T >= 4 && out_pixels <= 8192 && 1ll * T * c_blocks >= 32 && tune().fsplit;
+    const int k_slices = (mi.planes == 2 ? 3 : 1) * T * c_blocks;
+    const bool may_split = !window && !f.shuf_sh && !f.w_batched && out_pixels <= 8192 && k_slices >= 32 && tune().fsplit;
     // one fp32 plane per K slice; the bound on the slice count below holds for every plan made further down
     // (tiles >= tiles_lb, at least 4 K iterations per slice)
     int z_cap = 1;
     if (may_split) {
         const long long tiles_lb = 1ll * ((out_pixels + 127) / 128) * ceil_div(N, 256);
         const int sms = ds ? limited(ds->sms) : planning_sms();
-        z_cap = static_cast<int>(std::max<long long>(1, std::min<long long>(sms / tiles_lb, 1ll * (mi.planes == 2 ? 3 : 1) * T * c_blocks / 4)));
+        z_cap = static_cast<int>(std::max<long long>(1, std::min<long long>(sms / tiles_lb, k_slices / 4)));
     }
-    float* split_acc = may_split ? static_cast<float*>(ws.take(static_cast<size_t>(z_cap) * out_pixels * N * sizeof(float))) : nullptr;
+    const bool can_split = may_split && z_cap >= 2;
+    float* split_acc = can_split ? static_cast<float*>(ws.take(static_cast<size_t>(z_cap) * out_pixels * N * sizeof(float))) : nullptr;
     if (ws.dry) return NML_OK;
     if (!ws.fits()) return NML_ERR_WORKSPACE;
 
@@ -890,8 +902,13 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     P.n_phases = n_phases;
     // M-tile box from the largest phase grid
     const int esw = (f.gather || window) ? 1 : f.s_w, esh = f.gather ? 1 : f.s_h;
-    choose_box(7, P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, &P.wb_log2, &P.hb_log2, &P.nb_log2,
-               (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0);
+    if (f.w_batched) {  // a tile never straddles two images
+        P.b_batched = 1;
+        P.wb_log2 = 7;
+    } else {
+        choose_box(7, P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, &P.wb_log2, &P.hb_log2, &P.nb_log2,
+                   (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0);
+    }
     bool patch_resident = false;
     // Patch walk: unit-stride walks with several taps load one haloed patch per channel block instead of
     // one box per tap (8 x 16 pixel tiles of a single image).  Taken when the fixed tile shape does not
@@ -952,6 +969,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             P.nb_log2 = 0;
         }
     }
+    int z_plan = 1;  // K slices per tile
     // Tile width: 256 columns run the tensor pipe best, but when that leaves SMs idle (few row tiles,
     // narrow N) a narrower tile wins.  Cost per column relative to a 256-wide tile, measured on B200:
     // 128 -> 1.28, 64 -> 2.24; the makespan is rounds x width x cost.
@@ -976,6 +994,36 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                 best = t;
                 P.n_tiles = nt;
                 P.bn = bn;
+            }
+        }
+        // Tiles that leave half the SMs idle under a long K loop: tile width and number of K slices together, against
+        // the plan above without a split.
+        if (can_split && !P.patch) {
+            int k_min = 1 << 30;  // every slice of every phase gets at least 4 K iterations
+            for (int p = 0; p < n_phases; ++p)
+                if (P.phases[p].tap_count > 0) k_min = std::min(k_min, P.passes * P.c_blocks * P.phases[p].tap_count);
+            const double plane_us = static_cast<double>(out_pixels) * N * 4.0 / 6e6;
+            auto cost_us = [&](int nt, int bn, int z) {
+                const long long tiles = m_tiles_all * nt;
+                const double rounds = static_cast<double>((tiles * z + limited(ds->sms) - 1) / limited(ds->sms));
+                return rounds * (ceil_div(k_min, z) * slice_us(bn) + 2.5) + (z > 1 ? 3.0 + (2 * z + 1) * plane_us : 0.0);
+            };
+            double best_us = cost_us(P.n_tiles, P.bn, 1);
+            for (int i = 0; i < 4; ++i) {
+                if (tune().bn ? i != 3 : i == 3) continue;
+                const int nt = ceil_div(N, i == 3 ? tune().bn : cand[i]);
+                const int bn = static_cast<int>(round_up(ceil_div(N, nt), b_mn_major ? 64 : 32));
+                if (m_tiles_all * nt * 2 > limited(ds->sms)) continue;
+                const int z_max = std::min(z_cap, std::min(static_cast<int>(limited(ds->sms) / (m_tiles_all * nt)), k_min / 4));
+                for (int z = 2; z <= z_max; ++z) {
+                    const double us = cost_us(nt, bn, z);
+                    if (us < best_us) {
+                        best_us = us;
+                        z_plan = z;
+                        P.n_tiles = nt;
+                        P.bn = bn;
+                    }
+                }
             }
         }
     }
@@ -1025,12 +1073,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     // tile id then names two consecutive row tiles of one phase.
     // (short K loops are epilogue-bound, where pairing only halves the number of independent tiles)
     const int k_iters_min = P.passes * P.c_blocks * std::max<int>(1, P.phases[0].tap_count);
-    // (a problem with so few tiles that half the SMs would idle is K-split instead, see below)
     long long tiles_single = 0;
     for (int p = 0; p < n_phases; ++p)
         tiles_single += 1ll * ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) *
                         ceil_div(f.batch, 1 << P.nb_log2) * P.n_tiles;
-    const bool will_split = may_split && !P.patch && tiles_single * 2 <= limited(ds->sms) && k_iters_min >= 8;
     // 128-column tiles pair up too (two K slices per stage, see launch_kernel) where every phase has a K loop
     // of at least four slices and the tiles fill most of the GPU: measured 5-15 % on such layers, a loss on
     // the short phases of strided gathers and on few-tile problems.
@@ -1038,7 +1084,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     for (int p = 0; p < n_phases; ++p)
         if (P.phases[p].tap_count > 0) k_iters_all = std::min(k_iters_all, P.passes * P.c_blocks * P.phases[p].tap_count);
     const bool pair_width = P.bn == 256 || (tune().pair128 && P.bn == 128 && k_iters_all >= 4 && tiles_single * 4 >= 3ll * limited(ds->sms));
-    P.pair = (tune().pair && !P.patch && !will_split && pair_width && (!b_mn_major || N % mi.kb == 0) && k_iters_min >= 4 &&
+    P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && k_iters_min >= 4 &&
               (P.out_mode == OUT_NHWC_TMA || P.out_mode == OUT_NCHW_TMA || P.out_mode == OUT_NCHW) && limited(ds->sms) >= 2) ? 1 : 0;
     int tiles = 0;
     for (int p = 0; p < n_phases; ++p) {
@@ -1065,24 +1111,18 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         P.fastdiv = (2ll * tiles < (1ll << 23) && 2ll * tiles * dmax < (1ll << 40)) ? 1 : 0;
     }
     P.fsplit = 1;
-    if (may_split && !P.pair && !P.patch && tiles * 2 <= limited(ds->sms)) {
-        int k_min = k_iters_min;
-        for (int p = 0; p < n_phases; ++p)
-            if (P.phases[p].tap_count > 0) k_min = std::min(k_min, P.passes * P.c_blocks * P.phases[p].tap_count);
-        const int z = std::min(z_cap, std::min(limited(ds->sms) / tiles, k_min / 4));  // at least 4 K iterations per slice
-        if (z >= 2) {
-            P.fsplit = z;
-            P.num_tiles = tiles * z;
-            // slice z stores into plane z of the scratch; the finishing pass adds the planes in order and
-            // applies bias, rounding, cast and layout
-            P.plane_elems = out_pixels * N;
-            P.out = split_acc;
-            P.out_mode = OUT_NHWC;
-            P.out_f16 = 0;
-            P.round_f16 = 0;
-            P.bias = nullptr;
-            P.ld_out = N;
-        }
+    if (z_plan >= 2) {
+        P.fsplit = z_plan;
+        P.num_tiles = tiles * z_plan;
+        // slice z stores into plane z of the scratch; the finishing pass adds the planes in order and
+        // applies bias, rounding, cast and layout
+        P.plane_elems = out_pixels * N;
+        P.out = split_acc;
+        P.out_mode = OUT_NHWC;
+        P.out_f16 = 0;
+        P.round_f16 = 0;
+        P.bias = nullptr;
+        P.ld_out = N;
     }
 
     // tensor maps
@@ -1110,7 +1150,26 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         }
         if (rc) return rc;
         uint32_t one[2] = {1, 1};
-        if (!b_mn_major) {
+        if (f.w_batched) {  // as below, with the image as the outermost dimension
+            const uint64_t images = static_cast<uint64_t>(f.batch), es = static_cast<uint64_t>(mi.es);
+            const uint32_t kb = static_cast<uint32_t>(mi.kb), bn = static_cast<uint32_t>(P.bn);
+            uint32_t one4[4] = {1, 1, 1, 1};
+            if (!b_mn_major) {
+                uint64_t d[3] = {static_cast<uint64_t>(direct_w ? K : kp), static_cast<uint64_t>(N), images};
+                uint32_t box[3] = {kb, bn, 1};
+                rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 3, d, box, one4, SWZ_128B);
+            } else if (N % mi.kb == 0) {
+                P.b_grouped = 1;
+                uint64_t d[4] = {kb, static_cast<uint64_t>(K), static_cast<uint64_t>(N / mi.kb), images};
+                uint64_t str[3] = {N * es, kb * es, static_cast<uint64_t>(K) * N * es};
+                uint32_t box[4] = {kb, kb, bn / kb, 1};
+                rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 4, d, box, one4, SWZ_128B, str);
+            } else {
+                uint64_t d[3] = {static_cast<uint64_t>(N), static_cast<uint64_t>(K), images};
+                uint32_t box[3] = {kb, kb, 1};
+                rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 3, d, box, one4, SWZ_128B);
+            }
+        } else if (!b_mn_major) {
             uint64_t bdims[2] = {static_cast<uint64_t>(direct_w ? K : (window ? f.kh * 64 : T * kp)), static_cast<uint64_t>(N)};
             uint32_t bbox[2] = {static_cast<uint32_t>(mi.kb), static_cast<uint32_t>(P.pair ? P.bn / 2 : P.bn)};
             rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 2, bdims, bbox, one, SWZ_128B);
@@ -1155,14 +1214,15 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     if (P.fsplit <= 1) return profile_stop(slot, st);
     {
         const size_t total = out_pixels * N;
-        const int blocks = static_cast<int>(std::min<size_t>((total + 255) / 256, 148 * 8));
+        const int blocks = static_cast<int>(std::min<size_t>((total + 1023) / 1024, 148 * 8));
         const int nchw = (f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1)) ? 1 : 0;
+        const int vec = (!nchw && N % 4 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0) ? 1 : 0;
         if (f.out_dtype == NML_F16)
             { finish_rows_kernel<__half><<<blocks, 256, 0, st>>>(split_acc, P.fsplit, bias32, static_cast<__half*>(f.out), out_pixels, N,
-                                                              f.out_h * f.out_w, nchw, 0); ++g_launches; }
+                                                              f.out_h * f.out_w, nchw, 0, vec); ++g_launches; }
         else
             { finish_rows_kernel<float><<<blocks, 256, 0, st>>>(split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
-                                                             f.out_h * f.out_w, nchw, f.round_f16); ++g_launches; }
+                                                             f.out_h * f.out_w, nchw, f.round_f16, vec); ++g_launches; }
         NML_CUDA(cudaGetLastError());
     }
     return profile_stop(slot, st);
@@ -1294,38 +1354,46 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     P.ktiles_w = ceil_div(g.plain_w, 1 << P.wb_log2);
     P.ktiles_h = ceil_div(g.plain_h, 1 << P.hb_log2);
     P.kblocks_total = P.ktiles_w * P.ktiles_h * ceil_div(g.batch, 1 << P.nb_log2);
-    // CTA pairs when both operands come as grouped boxes and the tile is 256 columns wide
+    // Tile width and K split so that the CTAs finish together: the makespan is (rounds of tiles per CTA) x (K
+    // blocks per slice, plus a few blocks' worth of prologue / epilogue per tile), plus, for more than one slice,
+    // the second-stage reduction: it writes and re-reads one plane of dW per slice and then writes dW (~5 TB/s), plus its
+    // launch.  256-wide tiles whose operands both come as grouped boxes run as CTA pairs.  Narrower tiles are for gradients
+    // with few tiles over a short K (256 rows of a 2048 -> 1000 Linear layer: 64 tiles of 256 columns for 148 SMs).
     const int G_ = kTileM / mi.kb;
     const bool a_grp = !window && (cpa % mi.kb == 0) && (P.c_blocks % G_ == 0);
     const bool b_grp = (cpb % mi.kb == 0);
-    P.pair = (tune().pair && !P.wpatch && P.bn == 256 && a_grp && b_grp && sms >= 2) ? 1 : 0;
-    const int m_tiles = P.wpatch ? 1 : P.pair ? ceil_div(ceil_div(P.groups_total * mi.kb, kTileM), 2) : ceil_div(P.groups_total * mi.kb, kTileM);
-    const int mn_tiles = m_tiles * P.n_tiles;
-    // Split K so that the CTAs finish together: the makespan is (rounds of tiles per CTA) x (K
-    // blocks per slice, plus a few blocks' worth of prologue / epilogue per tile).  Pick the split
-    // that minimises it; ties go to the smaller split (fewer atomics).
-    int split = 1;
-    {
-        // Costs in microseconds: a K block of a 256-wide tile keeps the tensor pipe busy for ~0.27 us (four
-        // 128-clock MMAs); more than one slice adds the second-stage reduction, which writes and re-reads one
-        // plane of dW per slice and then writes dW (~5 TB/s), plus its launch.
-        const double block_us = 0.27 * P.bn / 256.0 * P.passes;
+    const int row_tiles = ceil_div(P.groups_total * mi.kb, kTileM);
+    int split = 1, m_tiles = 1;
+    if (!P.wpatch) {
         const double dw_bytes = 4.0 * g.plain_c * g.patch_c * T;
-        double best = -1;
         const int max_split = std::min(P.kblocks_total, 64);
-        for (int sp = 1; sp <= max_split; ++sp) {
-            int per_sp = ceil_div(P.kblocks_total, sp);
-            int real = ceil_div(P.kblocks_total, per_sp);  // every slice gets at least one K block
-            if (real != sp) continue;
-            long long rounds = ceil_div(mn_tiles * sp, P.pair ? sms / 2 : sms);
-            double cost = rounds * (per_sp + 4) * block_us;
-            if (sp > 1) cost += 3.0 + (2.0 * sp + 1.0) * dw_bytes / 5e6;
-            if (best < 0 || cost < best) {
-                best = cost;
-                split = sp;
+        double best = -1;
+        for (int width = 256; width >= 64; width /= 2) {
+            const int nt = ceil_div(g.plain_c, width);
+            const int bn = static_cast<int>(round_up(ceil_div(g.plain_c, nt), 64));
+            if (width < 256 && bn > width) continue;
+            const bool pair = tune().pair && bn == 256 && a_grp && b_grp && sms >= 2;
+            const int mt = pair ? ceil_div(row_tiles, 2) : row_tiles;
+            const double block_us = slice_us(bn) * P.passes;
+            for (int sp = 1; sp <= max_split; ++sp) {
+                int per_sp = ceil_div(P.kblocks_total, sp);
+                int real = ceil_div(P.kblocks_total, per_sp);  // every slice gets at least one K block
+                if (real != sp) continue;
+                long long rounds = ceil_div(mt * nt * sp, pair ? sms / 2 : sms);
+                double cost = rounds * (per_sp + 4) * block_us;
+                if (sp > 1) cost += 3.0 + (2.0 * sp + 1.0) * dw_bytes / 5e6;
+                if (best < 0 || cost < best * (width == 256 ? 1.0 : 0.95)) {  // the wider tile unless the gain is clear
+                    best = cost;
+                    split = sp;
+                    m_tiles = mt;
+                    P.n_tiles = nt;
+                    P.bn = bn;
+                    P.pair = pair ? 1 : 0;
+                }
             }
         }
     }
+    const int mn_tiles = m_tiles * P.n_tiles;
     if (P.wpatch) {  // one tile per CTA, no empty slice
         split = std::max(1, std::min(P.kblocks_total, sms / std::max(1, P.n_tiles)));
         split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, split));
@@ -2075,27 +2143,56 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
     // A 2-D right operand is shared by every batch entry; a batched one must match.
     if (b_batch != 1 && b_batch != batch) return NML_ERR_INVALID;
     const int es = (dtype == NML_F16) ? 2 : 4;
-    // C = A * B with B [K][N]: the backward-data form of a Linear layer whose weight is B.
-    nml_linear_desc d;
-    memset(&d, 0, sizeof(d));
-    d.rows = M; d.out_features = K; d.in_features = N;
-    d.in_dtype = d.out_dtype = d.w_dtype = dtype;
-    d.math = (dtype == NML_F16) ? NML_MATH_F16 : NML_MATH_3XTF32;
-    size_t need = 0;
-    int rc = nml_linear_workspace_size(&d, NML_PASS_BACKWARD_DATA, &need);
+    if (batch == 0 || M <= 0 || K <= 0 || N <= 0) return NML_ERR_INVALID;
+    // C = A * B with B [K][N]: the input-gradient form of a Linear layer whose weight is B.  A shared B makes all
+    // rows of A one problem.  Otherwise the entries run as the images of ONE launch, each with its own B (tiles of one
+    // entry each), because an entry of an attention-sized product fills a handful of SMs for a few microseconds:
+    // 64 x [333 x 64] x [64 x 333] in fp16 took 1740 us as 64 launches.  Entries that fill the GPU by themselves
+    // keep their own launches, where the planner may pair CTAs and split K.
+    const int math = (dtype == NML_F16) ? NML_MATH_F16 : NML_MATH_3XTF32;
+    const bool shared_b = b_batch == 1 && batch * static_cast<size_t>(M) < (1u << 30);
+    const long long tiles = 1ll * ceil_div(M, 128) * ceil_div(N, 256);
+    const size_t c_entry = static_cast<size_t>(M) * N * es, a_entry = static_cast<size_t>(M) * K * es, b_entry = static_cast<size_t>(K) * N * es;
+    size_t per_call = 1;  // entries per launch
+    if (!shared_b && b_batch != 1 && tiles < 2ll * planning_sms()) {
+        // bounded by the scratch of the converted operands (1 GB) and by the grid of the weight repack
+        const size_t scratch = (a_entry + b_entry) * 2 + 4096;
+        per_call = std::max<size_t>(1, std::min<size_t>({batch, 32768, (1ull << 30) / scratch}));
+    }
+    auto entries = [&](const uint8_t* A, const uint8_t* B, uint8_t* C, size_t n, Bump& bump) -> int {
+        if (per_call == 1 || shared_b) {
+            nml_linear_desc d;
+            memset(&d, 0, sizeof(d));
+            d.rows = static_cast<int>(n * M); d.out_features = K; d.in_features = N;
+            d.in_dtype = d.out_dtype = d.w_dtype = dtype;
+            d.math = math;
+            return linear_pass(&d, NML_PASS_BACKWARD_DATA, A, B, nullptr, C, nullptr, bump, nullptr);
+        }
+        FpropLike f;
+        memset(&f, 0, sizeof(f));
+        f.a = A; f.a_dtype = dtype; f.a_layout = NML_NHWC; f.batch = static_cast<int>(n); f.a_h = 1; f.a_w = M; f.a_c = K;
+        f.w = B; f.w_dtype = dtype; f.d0 = K; f.d1 = N; f.kh = f.kw = 1; f.k_is_dim0 = 1; f.w_direct = 1; f.w_batched = 1;
+        f.s_h = f.s_w = f.d_h = f.d_w = 1;
+        f.out = C; f.out_dtype = dtype; f.out_layout = NML_NHWC; f.out_c = N; f.out_h = 1; f.out_w = M;
+        f.math = math;
+        return run_fprop_like(f, bump, nullptr);
+    };
+    if (shared_b) per_call = batch;
+    Bump dry{nullptr, 0, 0, true};
+    int rc = entries(nullptr, nullptr, nullptr, per_call, dry);
     if (rc) return rc;
+    const size_t need = round_up(dry.off, 256);
     void* ws = nullptr;
     rc = ref_workspace(need, &ws);
     if (rc) return rc;
     void* out = nullptr;
-    rc = ref_alloc(&out, batch * M * N * es);
+    rc = ref_alloc(&out, batch * c_entry);
     if (rc) return rc;
-    for (size_t b = 0; b < batch; ++b) {
-        const uint8_t* A = reinterpret_cast<const uint8_t*>(a_ptr) + b * M * K * es;
-        const uint8_t* Bm = reinterpret_cast<const uint8_t*>(b_ptr) + (b_batch == 1 ? 0 : b) * K * N * es;
-        uint8_t* C = static_cast<uint8_t*>(out) + b * M * N * es;
+    for (size_t b = 0; b < batch; b += per_call) {
         Bump bump{static_cast<uint8_t*>(ws), 0, need, false};
-        rc = linear_pass(&d, NML_PASS_BACKWARD_DATA, A, Bm, nullptr, C, nullptr, bump, nullptr);
+        rc = entries(reinterpret_cast<const uint8_t*>(a_ptr) + b * a_entry,
+                     reinterpret_cast<const uint8_t*>(b_ptr) + (b_batch == 1 ? 0 : b) * b_entry, static_cast<uint8_t*>(out) + b * c_entry,
+                     std::min(per_call, batch - b), bump);
         if (rc) {
             ref_release(out);
             return rc;

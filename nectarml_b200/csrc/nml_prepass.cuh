@@ -114,17 +114,53 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict
     }
 }
 
-// Row-major [R][C] -> [R][Cp] with encoding change (fp32/fp16 -> fp16 / tf32 pair), zero pad.
+// Row-major [R][C] -> [R][Cp] with encoding change (fp32/fp16 -> fp16 / tf32 pair), zero pad; Cp is a multiple of 4.
+// Four outputs per thread: a 16-byte load where the rows allow it, one 8-byte (fp16) or one or two 16-byte stores.
+// An element per thread with a 64-bit division each ran at 1.8 TB/s on 2 MB; this is bound by the launch there.
+__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load4(const __half* p) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
 template <typename TIn>
 __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict__ in, void* out0,
                                                            void* out1, int enc, size_t R, int C, int Cp) {
-    size_t total = R * static_cast<size_t>(Cp);
+    const size_t per_row = Cp / 4, total = R * per_row;
+    const bool dense = C == Cp;  // rows follow one another on both sides
+    const bool vec = (dense || C % 4 == 0) && (reinterpret_cast<uintptr_t>(in) & (4 * sizeof(TIn) - 1)) == 0;
+    const bool small = total < 0xffffffffull;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        size_t r = i / Cp;
-        int c = static_cast<int>(i - r * Cp);
-        float v = (c < C) ? load_as_float(in, r * C + c) : 0.f;
-        store_enc(enc, out0, out1, i, v);
+        size_t src = 4 * i;
+        int left = 4;  // source elements under this thread's four outputs
+        if (!dense) {
+            const size_t r = small ? static_cast<uint32_t>(i) / static_cast<uint32_t>(per_row) : i / per_row;
+            const int c = static_cast<int>(i - r * per_row) * 4;
+            src = r * C + c;
+            left = C - c;
+        }
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vec && left >= 4) {
+            v = load4(in + src);
+        } else {
+            if (left > 0) v.x = load_as_float(in, src);
+            if (left > 1) v.y = load_as_float(in, src + 1);
+            if (left > 2) v.z = load_as_float(in, src + 2);
+            if (left > 3) v.w = load_as_float(in, src + 3);
+        }
+        if (enc == ENC_F16) {
+            uint2 h;
+            *reinterpret_cast<__half2*>(&h.x) = __floats2half2_rn(v.x, v.y);
+            *reinterpret_cast<__half2*>(&h.y) = __floats2half2_rn(v.z, v.w);
+            reinterpret_cast<uint2*>(out0)[i] = h;
+        } else {
+            const float4 hi = make_float4(to_tf32_rna(v.x), to_tf32_rna(v.y), to_tf32_rna(v.z), to_tf32_rna(v.w));
+            reinterpret_cast<float4*>(out0)[i] = hi;
+            if (enc == ENC_TF32_PAIR)
+                reinterpret_cast<float4*>(out1)[i] = make_float4(to_tf32_rna(v.x - hi.x), to_tf32_rna(v.y - hi.y),
+                                                                 to_tf32_rna(v.z - hi.z), to_tf32_rna(v.w - hi.w));
+        }
     }
 }
 
@@ -314,11 +350,45 @@ __global__ void __launch_bounds__(256) repack_weight_c8_kernel(const TIn* __rest
 // Partial sums of a K-split forward walk, `planes` fp32 planes of [pixels][C] (one per K slice) -> the
 // output tensor: the planes are added in slice order (so the result is bitwise repeatable), then bias,
 // optional rounding through fp16, cast, and the caller's layout (nchw: out[n][c][pixel of the image]).
+// Row-major outputs whose channel count is a multiple of 4 take four values per thread (`vec`).
+__device__ __forceinline__ float4 finish4(float4 v, const float* bias, int c, int round_f16) {
+    if (bias != nullptr) {
+        v.x += bias[c]; v.y += bias[c + 1]; v.z += bias[c + 2]; v.w += bias[c + 3];
+    }
+    if (round_f16) {
+        v.x = __half2float(__float2half_rn(v.x)); v.y = __half2float(__float2half_rn(v.y));
+        v.z = __half2float(__float2half_rn(v.z)); v.w = __half2float(__float2half_rn(v.w));
+    }
+    return v;
+}
 template <typename TOut>
 __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restrict__ acc, int planes, const float* __restrict__ bias,
                                                           TOut* __restrict__ out, size_t pixels, int C, int hw, int nchw,
-                                                          int round_f16) {
+                                                          int round_f16, int vec) {
     const size_t total = pixels * C;
+    if (vec) {
+        const uint32_t c4n = static_cast<uint32_t>(C / 4);
+        const size_t total4 = total / 4;
+        const float4* src = reinterpret_cast<const float4*>(acc);
+        for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total4; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+            float4 v = __ldg(src + i);
+#pragma unroll 8
+            for (int z = 1; z < planes; ++z) {
+                const float4 b = __ldg(src + static_cast<size_t>(z) * total4 + i);
+                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+            }
+            v = finish4(v, bias, static_cast<int>(static_cast<uint32_t>(i) % c4n) * 4, round_f16);
+            if (sizeof(TOut) == 2) {
+                uint2 h;
+                *reinterpret_cast<__half2*>(&h.x) = __floats2half2_rn(v.x, v.y);
+                *reinterpret_cast<__half2*>(&h.y) = __floats2half2_rn(v.z, v.w);
+                reinterpret_cast<uint2*>(out)[i] = h;
+            } else {
+                reinterpret_cast<float4*>(out)[i] = v;
+            }
+        }
+        return;
+    }
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const size_t p = i / C;

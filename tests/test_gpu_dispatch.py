@@ -11,6 +11,25 @@ from nectarml_b200 import _nectarml, ops
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("batch,m,k,n", [
+    (3, 1, 8, 1), (5, 127, 64, 63), (2, 128, 64, 64), (4, 129, 96, 65), (3, 333, 64, 333), (2, 40, 130, 257), (7, 130, 72, 264),
+    (2, 300, 200, 512)])
+def test_batched_matmul_entries_share_a_launch(batch, m, k, n, oracle):
+    rng = np.random.default_rng(m * n + k)
+    a = rng.standard_normal((batch, m, k), dtype=np.float32)
+    b = rng.standard_normal((batch, k, n), dtype=np.float32)
+    a32, b32 = dev(a), dev(b)
+    launches = ops.launch_count()
+    ptr = _nectarml.tensor.matmul(a32.data_ptr(), b32.data_ptr(), a.shape, b.shape, F32)
+    assert ops.launch_count() - launches <= 4  # conversion of A and of B, the product, at most one more
+    assert_f32(fetch(ptr, (batch, m, n)), oracle.matmul(a, b), "fp32")
+    a16, b16 = dev(a, torch.float16), dev(b, torch.float16)
+    ptr = _nectarml.tensor.matmul(a16.data_ptr(), b16.data_ptr(), a.shape, b.shape, F16)
+    r = oracle.round_f16
+    assert_f16(fetch(ptr, (batch, m, n), np.float16), oracle.matmul(r(a), r(b)), "fp16")
+    ops.device_status()
+
+
 @pytest.mark.parametrize("fout", [1, 2, 9, 31, 33, 63, 65, 127, 257, 333])
 @pytest.mark.parametrize("rows", [1, 130])
 def test_rows_that_do_not_start_on_16_bytes(rows, fout, oracle):

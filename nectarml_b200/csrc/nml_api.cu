@@ -318,7 +318,7 @@ static int colsum_finish(const ColsumScratch& cs, int C, float* out, cudaStream_
     for (;;) {
         const int S = ceil_div(P, 256);
         float* dst = (S == 1) ? out : (src == cs.partial ? cs.second : cs.partial);
-        colsum_finish_kernel<<<dim3(ceil_div(C, 32), S), dim3(32, 8), 0, st>>>(src, P, stride, C, dst, cs.stride, 256);
+        launch_short(colsum_finish_kernel, dim3(ceil_div(C, 32), S), dim3(32, 8), 0, st, src, P, stride, C, dst, cs.stride, 256);
         ++g_launches;
         if (S == 1) break;
         src = dst;
@@ -331,8 +331,8 @@ static int colsum_finish(const ColsumScratch& cs, int C, float* out, cudaStream_
 
 static void convert_rows(const void* src, int dtype, void* p0, void* p1, int enc, size_t rows, int c, int cp, cudaStream_t st) {
     const int blocks = static_cast<int>(std::min<size_t>((rows * (cp / 4) + 255) / 256, 148 * 16));
-    if (dtype == NML_F32) convert_rows_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(src), p0, p1, enc, rows, c, cp);
-    else convert_rows_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(src), p0, p1, enc, rows, c, cp);
+    if (dtype == NML_F32) launch_short(convert_rows_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(src), p0, p1, enc, rows, c, cp);
+    else launch_short(convert_rows_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(src), p0, p1, enc, rows, c, cp);
     ++g_launches;
 }
 
@@ -353,11 +353,11 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
     auto rows_colsum = [&](const ColsumScratch& cs) -> int {
         dim3 grid(col_blocks, static_cast<unsigned>(row_blocks));
         if (dtype == NML_F16 && c % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0)
-            colsum_rows_f16x8_kernel<<<grid, 256, 0, st>>>(static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
+            launch(colsum_rows_f16x8_kernel, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
         else if (dtype == NML_F16)
-            colsum_rows_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
+            launch(colsum_rows_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
         else
-            colsum_rows_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(src), cs.partial, pixels, c, rows_per_block);
+            launch(colsum_rows_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), cs.partial, pixels, c, rows_per_block);
         ++g_launches;
         return colsum_finish(cs, c, colsum, st);
     };
@@ -387,10 +387,10 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
     if (transposing) {
         dim3 grid(ceil_div(h * w, 64), ceil_div(Cp, 64), batch);
         if (dtype == NML_F32)
-            { nchw_to_nhwc_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(src), p0, p1, mi.enc, c, Cp,
+            { launch(nchw_to_nhwc_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), p0, p1, mi.enc, c, Cp,
                                                             h * w, cs.partial); ++g_launches; }
         else
-            { nchw_to_nhwc_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(src), p0, p1, mi.enc, c,
+            { launch(nchw_to_nhwc_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), p0, p1, mi.enc, c,
                                                              Cp, h * w, cs.partial); ++g_launches; }
         if (colsum) {
             int rc = colsum_finish(cs, c, colsum, st);
@@ -428,9 +428,9 @@ static int prepare_window(const void* src, int dtype, int layout, int batch, int
     if (!ws.fits()) return NML_ERR_WORKSPACE;
     const int nchw = (layout == NML_NCHW) ? 1 : 0;
     if (dtype == NML_F32)
-        { pad_pack_c8_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(src), nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial); ++g_launches; }
+        { launch(pad_pack_c8_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(src), nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial); ++g_launches; }
     else
-        { pad_pack_c8_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(src), nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial); ++g_launches; }
+        { launch(pad_pack_c8_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(src), nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial); ++g_launches; }
     NML_CUDA(cudaGetLastError());
     if (colsum) return colsum_finish(cs, c, colsum, st);
     return NML_OK;
@@ -594,23 +594,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     }
     const bool rec = rec_slot >= 0;
     if (rec && !pre_opened) NML_CUDA(cudaEventRecord(g_prof.start[rec_slot], st));
-    if (P.pair) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC));
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        NML_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(P), P));
-    } else {
-        kernel_for(P)<<<grid, threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st>>>(P);
-    }
+    launch_with(true, P.pair ? 2 : 1, kernel_for(P), grid, threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st, P);
     NML_CUDA(cudaGetLastError());
     if (open_slot) *open_slot = rec_slot;
     else if (rec) NML_CUDA(cudaEventRecord(g_prof.stop[rec_slot], st));
@@ -678,7 +662,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                 const int total = np * Kc * khp * kwp;
                 const int blocks = std::min(ceil_div(total, 256), 148 * 8);
 #define NML_PACK(TW, TB)                                                                                            \
-    pack_phase_weights_kernel<TW, TB><<<blocks, 256, 0, st>>>(static_cast<const TW*>(f.w), wp,                      \
+    launch_short(pack_phase_weights_kernel<TW, TB>, blocks, 256, 0, st, static_cast<const TW*>(f.w), wp,                      \
                                                               static_cast<const TB*>(f.bias), bp, Kc, C, f.kh, f.kw, \
                                                               f.s_h, f.s_w, f.p_h, f.p_w, khp, kwp, dh_min, dw_min)
                 if (f.w_dtype == NML_F32) {
@@ -744,9 +728,9 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             if (!ws.fits()) return NML_ERR_WORKSPACE;
             int blocks = std::min(ceil_div(N * f.kh * 64, 256), 148 * 8);
             if (f.w_dtype == NML_F32)
-                { repack_weight_c8_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw); ++g_launches; }
+                { launch_short(repack_weight_c8_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw); ++g_launches; }
             else
-                { repack_weight_c8_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw); ++g_launches; }
+                { launch_short(repack_weight_c8_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw); ++g_launches; }
             NML_CUDA(cudaGetLastError());
         }
     } else if (direct_w) {
@@ -769,10 +753,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
 #define NML_REPACK(T)                                                                                                           \
     do {                                                                                                                        \
         if (rC <= 64)                                                                                                           \
-            repack_weight_rows_kernel<T><<<dim3(ceil_div(kp, 64), rB), 256, 0, st>>>(static_cast<const T*>(f.w), p0, p1, mi.enc, \
+            launch_short(repack_weight_rows_kernel<T>, dim3(ceil_div(kp, 64), rB), 256, 0, st, static_cast<const T*>(f.w), p0, p1, mi.enc, \
                                                                                      rR, rC, kp);                               \
         else                                                                                                                    \
-            repack_weight_tile_kernel<T><<<dim3(ceil_div(rC, 64), ceil_div(kp, 64), rB), 256, 0, st>>>(                          \
+            launch_short(repack_weight_tile_kernel<T>, dim3(ceil_div(rC, 64), ceil_div(kp, 64), rB), 256, 0, st,                           \
                 static_cast<const T*>(f.w), p0, p1, mi.enc, rR, rC, kp);                                                         \
     } while (0)
             if (rows_only) convert_rows(f.w, f.w_dtype, p0, p1, mi.enc, static_cast<size_t>(rB) * f.d0, f.d1, kp, st);
@@ -1204,7 +1188,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             P.bias = static_cast<const float*>(f.bias);  // read as __half by the kernel
             P.bias_f16 = 1;
         } else {
-            to_float_kernel<__half><<<ceil_div(N, 256), 256, 0, st>>>(static_cast<const __half*>(f.bias), bias_widened, N);
+            launch_short(to_float_kernel<__half>, ceil_div(N, 256), 256, 0, st, static_cast<const __half*>(f.bias), bias_widened, N);
             ++g_launches;
         }
     }
@@ -1218,10 +1202,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const int nchw = (f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1)) ? 1 : 0;
         const int vec = (!nchw && N % 4 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0) ? 1 : 0;
         if (f.out_dtype == NML_F16)
-            { finish_rows_kernel<__half><<<blocks, 256, 0, st>>>(split_acc, P.fsplit, bias32, static_cast<__half*>(f.out), out_pixels, N,
+            { launch_short(finish_rows_kernel<__half>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<__half*>(f.out), out_pixels, N,
                                                               f.out_h * f.out_w, nchw, 0, vec); ++g_launches; }
         else
-            { finish_rows_kernel<float><<<blocks, 256, 0, st>>>(split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
+            { launch_short(finish_rows_kernel<float>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
                                                              f.out_h * f.out_w, nchw, f.round_f16, vec); ++g_launches; }
         NML_CUDA(cudaGetLastError());
     }
@@ -1487,18 +1471,18 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         const bool vec_ok = (reinterpret_cast<uintptr_t>(g.dw) & 15) == 0;
         if (P.wpatch && vec_ok && dw_elems % 4 == 0 && split > 8) {
             const size_t total4 = dw_elems / 4;
-            wgrad_reduce_deep4_kernel<<<static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st>>>(planes, g.dw, split, plane_elems, total4);
+            launch_short(wgrad_reduce_deep4_kernel, static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st, planes, g.dw, split, plane_elems, total4);
         } else if (P.wpatch && vec_ok && dw_elems % 4 == 0) {
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems / 4 + 255) / 256, 148 * 8));
-            wgrad_reduce_rows4_kernel<<<blocks, 256, 0, st>>>(planes, g.dw, split, plane_elems, 1, static_cast<int>(dw_elems / 4), 0);
+            launch_short(wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, 1, static_cast<int>(dw_elems / 4), 0);
         } else if (!P.wpatch && !P.kw_pack && T == 1 && vec_ok && g.patch_c % 4 == 0) {
             const size_t total4 = dw_elems / 4;
             const int blocks = static_cast<int>(std::min<size_t>((total4 + 255) / 256, 148 * 16));
-            wgrad_reduce_rows4_kernel<<<blocks, 256, 0, st>>>(planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
+            launch_short(wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
         } else {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + 255) / 256, 148 * 16));
-            wgrad_reduce_kernel<<<blocks, 256, 0, st>>>(planes, g.dw, split, plane_elems, dw_elems, layout, g.patch_c, P.n_taps,
+            launch_short(wgrad_reduce_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, dw_elems, layout, g.patch_c, P.n_taps,
                                                         P.kw_count, P.c_blocks, mi.kb, plane_rows);
         }
         ++g_launches;
@@ -1613,7 +1597,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
             int rc = profile_open(st);
             if (rc) return rc;
             const dim3 grid(ceil_div(d->in_features, 64), ceil_div(d->out_features, 64), 1);
-            repack_weight_tile_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(in1), wt, nullptr, ENC_F16,
+            launch_short(repack_weight_tile_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in1), wt, nullptr, ENC_F16,
                                                                    d->out_features, d->in_features, d->out_features);
             ++g_launches;
             NML_CUDA(cudaGetLastError());

@@ -16,6 +16,7 @@
 #include <atomic>
 
 #include "../../include/nectarml_b200.h"
+#include "nml_launch.cuh"
 
 namespace nml_layers {
 
@@ -24,6 +25,9 @@ namespace nml_layers {
         cudaError_t e_ = (expr);                     \
         if (e_ != cudaSuccess) return NML_ERR_CUDA;  \
     } while (0)
+
+using nml::launch;
+using nml::pdl_enter;
 
 static inline size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
 static std::atomic<long long> g_layer_launches{0};
@@ -63,6 +67,7 @@ template <bool kBackward>
 __global__ void __launch_bounds__(256) bn_reduce_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy,
                                                         const uint4* __restrict__ y, int act, float slope,
                                                         float* __restrict__ partial, size_t M, int C) {
+    pdl_enter();
     __shared__ float sm[256][17];
     const int cpr = C >> 3;
     const int rpb = blockDim.x / cpr;
@@ -144,6 +149,7 @@ __global__ void __launch_bounds__(256) bn_reduce_kernel(const uint4* __restrict_
 __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict__ partial, int P, int C, int mode, double inv_M,
                                                         float eps, const float* __restrict__ mean, const float* __restrict__ rstd,
                                                         float* __restrict__ out0, float* __restrict__ out1) {
+    pdl_enter();
     __shared__ double pa[32][33], pb[32][33];
     const int c = blockIdx.x * 32 + threadIdx.x;
     double sa = 0.0, sb = 0.0;
@@ -182,6 +188,7 @@ __global__ void __launch_bounds__(256) bn_apply_kernel(const uint4* __restrict__
                                                        uint4* __restrict__ y, const float* __restrict__ gamma,
                                                        const float* __restrict__ beta, const float* __restrict__ mean,
                                                        const float* __restrict__ rstd, int act, float slope, size_t M, int C) {
+    pdl_enter();
     const int cpr = C >> 3;
     const int rpb = blockDim.x / cpr;
     const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
@@ -230,6 +237,7 @@ __global__ void __launch_bounds__(256) bn_dx_kernel(const uint4* __restrict__ x,
                                                     const float* __restrict__ rstd, const float* __restrict__ dbeta,
                                                     const float* __restrict__ dgamma, int act, float slope, float inv_M,
                                                     size_t M, int C) {
+    pdl_enter();
     const int cpr = C >> 3;
     const int rpb = blockDim.x / cpr;
     const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
@@ -282,6 +290,7 @@ __global__ void __launch_bounds__(256) bn_dx_kernel(const uint4* __restrict__ x,
 
 // any(!isfinite(g * inv_scale)) over a flat fp32 buffer -> *found (set, never cleared, here)
 __global__ void __launch_bounds__(256) grads_check_kernel(const float4* __restrict__ g, size_t n4, float inv_scale, int* found) {
+    pdl_enter();
     bool bad = false;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const float4 v = __ldg(g + i);
@@ -296,6 +305,7 @@ __global__ void __launch_bounds__(256) grads_check_kernel(const float4* __restri
 __global__ void __launch_bounds__(256) sgd_momentum_kernel(float4* __restrict__ p, const float4* __restrict__ g, float4* __restrict__ vel,
                                                            uint2* __restrict__ p16, size_t n4, float lr, float momentum, float dampening,
                                                            float wd, float inv_scale, const int* __restrict__ found_inf) {
+    pdl_enter();
     if (found_inf && *found_inf) return;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n4; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         float4 pv = p[i], vv = vel[i];
@@ -326,6 +336,7 @@ __global__ void __launch_bounds__(256) sgd_momentum_kernel(float4* __restrict__ 
 // (no zero-fill pass).  Out-of-image taps are skipped (i.e. padded with -inf).
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, uint2* __restrict__ idx,
                                                           int N, int H, int W, int C, int k, int s, int p, int Ho, int Wo) {
+    pdl_enter();
     const int cpr = C >> 3;
     const size_t total = static_cast<size_t>(N) * Ho * Wo * cpr;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -368,6 +379,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const uint4* __restric
 
 __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const uint4* __restrict__ dy, const uint2* __restrict__ idx, uint4* __restrict__ dx,
                                                           int N, int H, int W, int C, int k, int s, int p, int Ho, int Wo) {
+    pdl_enter();
     const int cpr = C >> 3;
     const size_t total = static_cast<size_t>(N) * H * W * cpr;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -442,11 +454,11 @@ int nml_bn_forward(const void* x, long long rows, int channels, const float* gam
     int threads;
     const int P = bn_grid(rows, channels, &threads);
     float* partial = static_cast<float*>(workspace);
-    bn_reduce_kernel<false><<<P, threads, 0, st>>>(static_cast<const uint4*>(x), nullptr, nullptr, 0, 0.f, partial,
+    launch(bn_reduce_kernel<false>, P, threads, 0, st, static_cast<const uint4*>(x), nullptr, nullptr, 0, 0.f, partial,
                                                    static_cast<size_t>(rows), channels);
-    bn_finish_kernel<<<(channels + 31) / 32, dim3(32, 32), 0, st>>>(partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
+    launch(bn_finish_kernel, (channels + 31) / 32, dim3(32, 32), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
                                                                    nullptr, nullptr, mean, rstd);
-    bn_apply_kernel<<<bn_grid_elementwise(rows, channels), threads, 0, st>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(residual),
+    launch(bn_apply_kernel, bn_grid_elementwise(rows, channels), threads, 0, st, static_cast<const uint4*>(x), static_cast<const uint4*>(residual),
                                            static_cast<uint4*>(y), gamma, beta, mean, rstd, act, slope,
                                            static_cast<size_t>(rows), channels);
     NMLL_CUDA(cudaGetLastError());
@@ -467,11 +479,11 @@ int nml_bn_backward(const void* dy, const void* y, const void* x, long long rows
     int threads;
     const int P = bn_grid(rows, channels, &threads);
     float* partial = static_cast<float*>(workspace);
-    bn_reduce_kernel<true><<<P, threads, 0, st>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(dy),
+    launch(bn_reduce_kernel<true>, P, threads, 0, st, static_cast<const uint4*>(x), static_cast<const uint4*>(dy),
                                                   static_cast<const uint4*>(y), act, slope, partial,
                                                   static_cast<size_t>(rows), channels);
-    bn_finish_kernel<<<(channels + 31) / 32, dim3(32, 32), 0, st>>>(partial, P, channels, 1, 0.0, 0.f, mean, rstd, dbeta, dgamma);
-    bn_dx_kernel<<<bn_grid_elementwise(rows, channels), threads, 0, st>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<const uint4*>(y),
+    launch(bn_finish_kernel, (channels + 31) / 32, dim3(32, 32), 0, st, partial, P, channels, 1, 0.0, 0.f, mean, rstd, dbeta, dgamma);
+    launch(bn_dx_kernel, bn_grid_elementwise(rows, channels), threads, 0, st, static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<const uint4*>(y),
                                         static_cast<uint4*>(dx), static_cast<uint4*>(dres), gamma, mean, rstd, dbeta, dgamma, act,
                                         slope, static_cast<float>(1.0 / static_cast<double>(rows)), static_cast<size_t>(rows),
                                         channels);
@@ -492,7 +504,7 @@ int nml_maxpool_forward(const void* x, int batch, int h, int w, int channels, in
     if (ho <= 0 || wo <= 0) return NML_ERR_INVALID;
     const size_t total = static_cast<size_t>(batch) * ho * wo * (channels / 8);
     const int blocks = static_cast<int>((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-    maxpool_fwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(x), static_cast<uint4*>(y),
+    launch(maxpool_fwd_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<uint4*>(y),
                                                                              static_cast<uint2*>(index), batch, h, w, channels, k,
                                                                              stride, pad, ho, wo);
     NMLL_CUDA(cudaGetLastError());
@@ -510,7 +522,7 @@ int nml_maxpool_backward(const void* dy, const void* index, int batch, int h, in
     if (ho <= 0 || wo <= 0) return NML_ERR_INVALID;
     const size_t total = static_cast<size_t>(batch) * h * w * (channels / 8);
     const int blocks = static_cast<int>((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
-    maxpool_bwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(dy), static_cast<const uint2*>(index),
+    launch(maxpool_bwd_kernel, blocks, 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(dy), static_cast<const uint2*>(index),
                                                                              static_cast<uint4*>(dx), batch, h, w, channels, k, stride,
                                                                              pad, ho, wo);
     NMLL_CUDA(cudaGetLastError());
@@ -524,7 +536,7 @@ int nml_grads_check(const float* grads, size_t n, float inv_scale, int* found_in
     NMLL_CUDA(cudaMemsetAsync(found_inf, 0, sizeof(int), st));
     const size_t n4 = n / 4;
     const int blocks = static_cast<int>(n4 / 256 + 1 < 148 * 8 ? n4 / 256 + 1 : 148 * 8);
-    grads_check_kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<const float4*>(grads), n4, inv_scale, found_inf);
+    launch(grads_check_kernel, blocks, 256, 0, st, reinterpret_cast<const float4*>(grads), n4, inv_scale, found_inf);
     NMLL_CUDA(cudaGetLastError());
     ++g_layer_launches;
     return NML_OK;
@@ -539,7 +551,7 @@ int nml_sgd_momentum_step(float* params, const float* grads, float* velocity, vo
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t n4 = n / 4;
     const int blocks = static_cast<int>(n4 / 256 + 1 < 148 * 8 ? n4 / 256 + 1 : 148 * 8);
-    sgd_momentum_kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<float4*>(params), reinterpret_cast<const float4*>(grads),
+    launch(sgd_momentum_kernel, blocks, 256, 0, st, reinterpret_cast<float4*>(params), reinterpret_cast<const float4*>(grads),
                                                 reinterpret_cast<float4*>(velocity), static_cast<uint2*>(params_f16), n4, lr,
                                                 momentum, dampening, weight_decay, inv_scale, found_inf);
     NMLL_CUDA(cudaGetLastError());

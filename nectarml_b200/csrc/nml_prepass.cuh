@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "nml_launch.cuh"
+
 namespace nml {
 
 __device__ __forceinline__ float to_tf32_rna(float x) {
@@ -43,6 +45,7 @@ template <typename TIn>
 __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict__ in, void* out0,
                                                            void* out1, int enc, int C, int Cp, int HW,
                                                            float* colsum) {
+    pdl_enter();
     __shared__ float tile[64][65];
     const int n = blockIdx.z;
     const int c0 = blockIdx.y * 64;
@@ -126,6 +129,7 @@ __device__ __forceinline__ float4 load4(const __half* p) {
 template <typename TIn>
 __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict__ in, void* out0,
                                                            void* out1, int enc, size_t R, int C, int Cp) {
+    pdl_enter();
     const size_t per_row = Cp / 4, total = R * per_row;
     const bool dense = C == Cp;  // rows follow one another on both sides
     const bool vec = (dense || C % 4 == 0) && (reinterpret_cast<uintptr_t>(in) & (4 * sizeof(TIn) - 1)) == 0;
@@ -169,6 +173,7 @@ __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict
 template <typename TIn>
 __global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* __restrict__ in, float* colsum,
                                                           size_t R, int C, int rows_per_block) {
+    pdl_enter();
     size_t r0 = static_cast<size_t>(blockIdx.y) * rows_per_block;
     size_t r1 = r0 + rows_per_block < R ? r0 + rows_per_block : R;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
@@ -183,6 +188,7 @@ __global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* __restrict_
 // interleaved rows, and each block writes its partial sums to its row of the partial-sum matrix.
 __global__ void __launch_bounds__(256) colsum_rows_f16x8_kernel(const __half* __restrict__ in, float* colsum,
                                                                 size_t R, int C, int rows_per_block) {
+    pdl_enter();
     __shared__ float part[8][256];
     const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
     const int c0 = (blockIdx.x * 32 + lane) * 8;
@@ -239,6 +245,7 @@ __device__ __forceinline__ void store_enc2(int enc, void* out0, void* out1, size
 template <typename TIn>
 __global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* __restrict__ w, void* out0, void* out1, int enc,
                                                                  int R, int Cc, int Rp) {
+    pdl_enter();
     __shared__ float tile[64][65];  // [r][c]
     const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
     const size_t b = blockIdx.z;
@@ -259,6 +266,7 @@ __global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* __re
 template <typename TIn>
 __global__ void __launch_bounds__(256) repack_weight_rows_kernel(const TIn* __restrict__ w, void* out0, void* out1, int enc,
                                                                  int R, int Cc, int Rp) {
+    pdl_enter();
     __shared__ float tile[64][65];  // [c][r]
     const int r0 = blockIdx.x * 64;
     const size_t b = blockIdx.y;
@@ -284,6 +292,7 @@ template <typename TIn>
 __global__ void __launch_bounds__(256) pad_pack_c8_kernel(const TIn* __restrict__ in, int nchw, __half* __restrict__ out,
                                                           int N, int C, int H, int W, int pad_h, int pad_w, int Hp,
                                                           int Wp, float* colsum) {
+    pdl_enter();
     const size_t total = static_cast<size_t>(N) * Hp * Wp;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // per-channel sums of the values read (bias gradient)
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -335,6 +344,7 @@ __global__ void __launch_bounds__(256) pad_pack_c8_kernel(const TIn* __restrict_
 template <typename TIn>
 __global__ void __launch_bounds__(256) repack_weight_c8_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
                                                                int Cout, int C, int KH, int KW) {
+    pdl_enter();
     const int total = Cout * KH * 64;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int k = i & 63;
@@ -365,6 +375,7 @@ template <typename TOut>
 __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restrict__ acc, int planes, const float* __restrict__ bias,
                                                           TOut* __restrict__ out, size_t pixels, int C, int hw, int nchw,
                                                           int round_f16, int vec) {
+    pdl_enter();
     const size_t total = pixels * C;
     if (vec) {
         const uint32_t c4n = static_cast<uint32_t>(C / 4);
@@ -418,6 +429,7 @@ __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __re
                                                                  const TBias* __restrict__ bias, float* __restrict__ bias_out,
                                                                  int K, int C, int KH, int KW, int s_h, int s_w, int p_h,
                                                                  int p_w, int khp, int kwp, int dh_min, int dw_min) {
+    pdl_enter();
     const int np = s_h * s_w * C;
     const int total = np * K * khp * kwp;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -447,6 +459,7 @@ __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __re
 // than one segment is left.  blockDim = (32, 8).
 __global__ void __launch_bounds__(256) colsum_finish_kernel(const float* __restrict__ partial, int P, int stride, int C,
                                                             float* __restrict__ out, int out_stride, int rows_per_block) {
+    pdl_enter();
     __shared__ float part[8][33];
     const int c = blockIdx.x * 32 + threadIdx.x;
     const int p0 = blockIdx.y * rows_per_block;
@@ -472,6 +485,7 @@ __global__ void __launch_bounds__(256) colsum_finish_kernel(const float* __restr
 __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __restrict__ planes, float* __restrict__ dw,
                                                                  int split, size_t plane_elems, size_t rows, int row_len4,
                                                                  size_t src_pitch) {
+    pdl_enter();
     const size_t total = rows * row_len4;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -495,6 +509,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __
 // fixed association, so still bitwise repeatable.  Planes are laid out like dW.
 __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __restrict__ planes, float* __restrict__ dw,
                                                                  int split, size_t plane_elems, size_t total4) {
+    pdl_enter();
     __shared__ float4 part[8][32];
     const size_t i = blockIdx.x * 32ull + threadIdx.x;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -527,6 +542,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ planes, float* __restrict__ dw, int split,
                                                            size_t plane_elems, size_t total, int layout, int c_patch,
                                                            int n_taps, int kw_count, int c_blocks, int kb, int R) {
+    pdl_enter();
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         size_t src = i;
@@ -553,6 +569,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
 
 template <typename TIn>
 __global__ void __launch_bounds__(256) to_float_kernel(const TIn* __restrict__ in, float* out, int n) {
+    pdl_enter();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = load_as_float(in, i);
 }

@@ -26,6 +26,7 @@
 //               Covers Conv2d / ConvTranspose2d weight-gradient and Linear weight-gradient.
 // 256-wide tiles of long-K problems run as CTA pairs (cta_group::2, see the kernel's comment).
 #pragma once
+#include "nml_launch.cuh"
 #include "nml_ptx.cuh"
 
 namespace nml {
@@ -313,6 +314,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     if (kPair) cluster_sync_all();  // the partner's barriers must be initialised before anything arrives on them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_enter();  // everything above overlaps the tail of the kernel in front
 
     const int box_bytes = P.kb * 128;  // one MN-major box: kb k-rows of 128 bytes
     const int wb = 1 << P.wb_log2, hb = 1 << P.hb_log2;

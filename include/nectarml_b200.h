@@ -209,6 +209,18 @@ int nml_bn_backward(const void* dy, const void* y, const void* x, long long rows
                     void* dres, float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes,
                     void* stream);
 
+/* The same without the forward's output y in the backward.  Where nothing was added before the activation its
+ * derivative follows from x (pass mask = NULL on both sides, and the forward's beta to the backward); where a residual
+ * was added, `mask` holds one bit per element, set where y > 0 (rows * channels / 8 bytes, byte v the channels 8v ... 8v+7
+ * of the row-major matrix; written by the forward). */
+int nml_bn_forward_masked(const void* x, long long rows, int channels, const float* gamma, const float* beta,
+                          const void* residual, int act, float slope, float eps, void* y, void* mask, float* mean,
+                          float* rstd, void* workspace, size_t workspace_bytes, void* stream);
+int nml_bn_backward_masked(const void* dy, const void* mask, const void* x, long long rows, int channels,
+                           const float* gamma, const float* beta, const float* mean, const float* rstd, int act,
+                           float slope, void* dx, void* dres, float* dgamma, float* dbeta, void* workspace,
+                           size_t workspace_bytes, void* stream);
+
 /* Max pooling of an NHWC fp16 tensor (channels a multiple of 8), output size (h + 2 pad - k)/stride + 1.
  * The forward also writes one byte per output value naming the window tap that won (`index`,
  * batch * ho * wo * channels bytes); the backward gathers dy through it, writes every element of

@@ -48,79 +48,65 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     for (int j = 0; j < 4; ++j) h[j] = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
     return v;
 }
-// derivative of the activation, read off the activation's OUTPUT: 0 none, 1 ReLU, 2 LeakyReLU(slope)
-__device__ __forceinline__ float act_grad(int act, float slope, float y) {
-    return act == 0 ? 1.f : (y > 0.f ? 1.f : (act == 1 ? 0.f : slope));
-}
-
 // Thread layout shared by the kernels below: the matrix is [M][C] fp16 with C a multiple of 8, a
 // vector is 8 adjacent channels (16 bytes), cpr = C / 8 vectors per row.  A block has
 // (256 / cpr) * cpr threads; thread t owns vector column t % cpr for good (its per-channel
 // constants sit in registers) and walks rows t / cpr, + rows-per-pass, ...: consecutive threads read
 // consecutive 16-byte vectors, so every access is fully coalesced whatever C is.
 
-// First stage of a per-channel reduction over rows.  kBackward == false: a = sum x, b = sum x^2.
-// kBackward == true: with dz = dy * act'(y): a = sum dz, b = sum dz * x (the second stage turns b into
-// d gamma = rstd * (b - mean * a), so this pass needs no per-channel constants).  Two rows are in flight
-// per thread.  Block p writes its sums to partial[p][0..C) and partial[p][C..2C).
-template <bool kBackward>
-__global__ void __launch_bounds__(256) bn_reduce_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy,
-                                                        const uint4* __restrict__ y, int act, float slope,
-                                                        float* __restrict__ partial, size_t M, int C) {
-    pdl_enter();
-    __shared__ float sm[256][17];
-    const int cpr = C >> 3;
-    const int rpb = blockDim.x / cpr;
-    const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
-    float a[8], b[8];
+// How a backward pass finds the derivative of the activation.
+enum {
+    D_NONE = 0,  // no activation
+    D_Y = 1,     // from the activation's output, which is read again (the C entry point that is given y alone)
+    D_X = 2,     // from the normalisation's input, which the pass reads anyway: the sign of gamma * xhat + beta
+    D_MASK = 3   // from one bit per element that the forward wrote (a residual was added, so x alone does not tell)
+};
+// D_X and D_MASK keep y out of the backward: a 256-channel 56 x 56 layer at batch 256 (411 MB per tensor) reads 1.23 -> 0.85
+// GB in the reduction and moves 2.05 -> 1.67 GB in the second pass.
+
+// y = half(t) is positive exactly when t is above half of the smallest fp16 subnormal (ties go to zero).
+__device__ __forceinline__ bool positive_as_half(float t) { return t > 2.98023223876953125e-8f; }
+
+// Per-channel constants of the forward's y = act(sc * x + sh), as the forward computes them.
+__device__ __forceinline__ void bn_affine(int col, const float* __restrict__ gamma, const float* __restrict__ beta,
+                                          const float* __restrict__ mean, const float* __restrict__ rstd, float (&sc)[8], float (&sh)[8]) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
-    auto add = [&](const uint4& xv, const uint4& dv, const uint4& yv) {
-        float xf[8];
-        unpack8(xv, xf);
-        if (!kBackward) {
+    for (int j = 0; j < 8; ++j) {
+        const int c = col * 8 + j;
+        sc[j] = (gamma ? gamma[c] : 1.f) * rstd[c];
+        sh[j] = (beta ? beta[c] : 0.f) - mean[c] * sc[j];
+    }
+}
+
+// dz = dy * act'(.) of one vector.
+template <int kDeriv>
+__device__ __forceinline__ void act_backward(float (&df)[8], const float (&xf)[8], const uint4& yv, unsigned bits, const float (&sc)[8],
+                                             const float (&sh)[8], float below) {
+    if (kDeriv == D_Y) {
+        float yf[8];
+        unpack8(yv, yf);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                a[j] += xf[j];
-                b[j] += xf[j] * xf[j];
-            }
-        } else {
-            float df[8], yf[8];
-            unpack8(dv, df);
-            if (act != 0) unpack8(yv, yf);
+        for (int j = 0; j < 8; ++j) df[j] *= yf[j] > 0.f ? 1.f : below;
+    } else if (kDeriv == D_X) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float dz = df[j] * (act != 0 ? act_grad(act, slope, yf[j]) : 1.f);
-                a[j] += dz;
-                b[j] += dz * xf[j];
-            }
-        }
-    };
-    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
-    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    if (!kBackward) {  // one input stream only: four rows in flight keep as many bytes outstanding as the backward pass has
-        for (; row + 3 * stride < M; row += 4 * stride) {
-            const uint4 x0 = __ldg(x + row * cpr + col), x1 = __ldg(x + (row + stride) * cpr + col);
-            const uint4 x2 = __ldg(x + (row + 2 * stride) * cpr + col), x3 = __ldg(x + (row + 3 * stride) * cpr + col);
-            add(x0, zero, zero);
-            add(x1, zero, zero);
-            add(x2, zero, zero);
-            add(x3, zero, zero);
-        }
+        for (int j = 0; j < 8; ++j) df[j] *= positive_as_half(xf[j] * sc[j] + sh[j]) ? 1.f : below;
+    } else if (kDeriv == D_MASK) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) df[j] *= ((bits >> j) & 1u) ? 1.f : below;
     }
-    for (; row + stride < M; row += 2 * stride) {
-        const size_t v0 = row * cpr + col, v1 = (row + stride) * cpr + col;
-        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
-        const uint4 d0 = kBackward ? __ldg(dy + v0) : zero, d1 = kBackward ? __ldg(dy + v1) : zero;
-        const uint4 y0 = (kBackward && act != 0) ? __ldg(y + v0) : zero, y1 = (kBackward && act != 0) ? __ldg(y + v1) : zero;
-        add(x0, d0, y0);
-        add(x1, d1, y1);
-    }
-    if (row < M) {
-        const size_t v0 = row * cpr + col;
-        add(__ldg(x + v0), kBackward ? __ldg(dy + v0) : zero, (kBackward && act != 0) ? __ldg(y + v0) : zero);
-    }
+}
+
+// What a backward pass reads of the forward besides x: see the D_* above.  `below` is the derivative where y <= 0.
+struct BnForward {
+    const uint4* y;
+    const uint8_t* mask;
+    const float *gamma, *beta, *mean, *rstd;
+    float below;
+};
+
+// First stage of a per-channel reduction over rows.  Block p writes its sums to partial[p][0..C) and partial[p][C..2C).
+__device__ __forceinline__ void bn_store_partial(float (*sm)[17], const float (&a)[8], const float (&b)[8], int cpr, int rpb, int C,
+                                                 float* __restrict__ partial) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         sm[threadIdx.x][j] = a[j];
@@ -142,34 +128,111 @@ __global__ void __launch_bounds__(256) bn_reduce_kernel(const uint4* __restrict_
     }
 }
 
-// Second stage: adds the P rows of partial sums in a fixed order (32 interleaved running sums in double,
-// then those 32 in order).  mode 0: out0 = mean, out1 = 1 / sqrt(biased variance + eps).
-// mode 1: out0 = sum a (d beta), out1 = rstd * (sum b - mean * sum a) (d gamma).  blockDim = (32, 32): the
-// pass is a chain of load latencies, so it is spread over as many threads as a block has.
+// Forward statistics: a = sum x, b = sum x^2; four rows in flight per thread.
+__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* __restrict__ x, float* __restrict__ partial, size_t M, int C) {
+    pdl_enter();
+    __shared__ float sm[256][17];
+    const int cpr = C >> 3;
+    const int rpb = blockDim.x / cpr;
+    const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
+    float a[8], b[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
+    auto add = [&](const uint4& xv) {
+        float xf[8];
+        unpack8(xv, xf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            a[j] += xf[j];
+            b[j] += xf[j] * xf[j];
+        }
+    };
+    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
+    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
+    for (; row + 3 * stride < M; row += 4 * stride) {
+        const uint4 x0 = __ldg(x + row * cpr + col), x1 = __ldg(x + (row + stride) * cpr + col);
+        const uint4 x2 = __ldg(x + (row + 2 * stride) * cpr + col), x3 = __ldg(x + (row + 3 * stride) * cpr + col);
+        add(x0);
+        add(x1);
+        add(x2);
+        add(x3);
+    }
+    for (; row < M; row += stride) add(__ldg(x + row * cpr + col));
+    bn_store_partial(sm, a, b, cpr, rpb, C, partial);
+}
+
+// Backward sums: with dz = dy * act'(.): a = sum dz, b = sum dz * x (the second stage turns b into
+// d gamma = rstd * (b - mean * a), so this pass needs no per-channel constants but those of D_X).  Two rows in flight per
+// thread.
+template <int kDeriv>
+__global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, const BnForward f,
+                                                           float* __restrict__ partial, size_t M, int C) {
+    pdl_enter();
+    __shared__ float sm[256][17];
+    const int cpr = C >> 3;
+    const int rpb = blockDim.x / cpr;
+    const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
+    float a[8], b[8], sc[8], sh[8];
+    if (kDeriv == D_X) bn_affine(col, f.gamma, f.beta, f.mean, f.rstd, sc, sh);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
+    auto add = [&](const uint4& xv, const uint4& dv, const uint4& yv, unsigned bits) {
+        float xf[8], df[8];
+        unpack8(xv, xf);
+        unpack8(dv, df);
+        act_backward<kDeriv>(df, xf, yv, bits, sc, sh, f.below);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            a[j] += df[j];
+            b[j] += df[j] * xf[j];
+        }
+    };
+    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
+    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (; row + stride < M; row += 2 * stride) {
+        const size_t v0 = row * cpr + col, v1 = (row + stride) * cpr + col;
+        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1), d0 = __ldg(dy + v0), d1 = __ldg(dy + v1);
+        const uint4 y0 = kDeriv == D_Y ? __ldg(f.y + v0) : zero, y1 = kDeriv == D_Y ? __ldg(f.y + v1) : zero;
+        const unsigned m0 = kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? __ldg(f.mask + v1) : 0u;
+        add(x0, d0, y0, m0);
+        add(x1, d1, y1, m1);
+    }
+    if (row < M) {
+        const size_t v0 = row * cpr + col;
+        add(__ldg(x + v0), __ldg(dy + v0), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
+    }
+    bn_store_partial(sm, a, b, cpr, rpb, C, partial);
+}
+
+// Second stage: adds the P rows of partial sums in a fixed order (128 interleaved running sums in double,
+// then those 128 in a tree).  mode 0: out0 = mean, out1 = 1 / sqrt(biased variance + eps).
+// mode 1: out0 = sum a (d beta), out1 = rstd * (sum b - mean * sum a) (d gamma).  blockDim = (8, 128): the pass is a chain of
+// load latencies, so it is spread over many blocks and a thread's few loads are all in flight (32 channels a block and
+// 19 rows a thread took 6 us; a U-Net step runs it 26 times).
 __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict__ partial, int P, int C, int mode, double inv_M,
                                                         float eps, const float* __restrict__ mean, const float* __restrict__ rstd,
                                                         float* __restrict__ out0, float* __restrict__ out1) {
     pdl_enter();
-    __shared__ double pa[32][33], pb[32][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
+    __shared__ double pa[128][9], pb[128][9];
+    const int c = blockIdx.x * 8 + threadIdx.x;
     double sa = 0.0, sb = 0.0;
-    if (c < C) {
-#pragma unroll 4
-        for (int p = threadIdx.y; p < P; p += 32) {
-            sa += static_cast<double>(__ldg(partial + static_cast<size_t>(p) * 2 * C + c));
-            sb += static_cast<double>(__ldg(partial + static_cast<size_t>(p) * 2 * C + C + c));
-        }
+#pragma unroll 5
+    for (int p = threadIdx.y; p < P; p += 128) {
+        sa += static_cast<double>(__ldg(partial + static_cast<size_t>(p) * 2 * C + c));
+        sb += static_cast<double>(__ldg(partial + static_cast<size_t>(p) * 2 * C + C + c));
     }
     pa[threadIdx.y][threadIdx.x] = sa;
     pb[threadIdx.y][threadIdx.x] = sb;
-    __syncthreads();
-    if (threadIdx.y == 0 && c < C) {
-        double ta = 0.0, tb = 0.0;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            ta += pa[k][threadIdx.x];
-            tb += pb[k][threadIdx.x];
+    for (int half = 64; half > 0; half /= 2) {
+        __syncthreads();
+        if (threadIdx.y < half) {
+            pa[threadIdx.y][threadIdx.x] += pa[threadIdx.y + half][threadIdx.x];
+            pb[threadIdx.y][threadIdx.x] += pb[threadIdx.y + half][threadIdx.x];
         }
+    }
+    if (threadIdx.y == 0) {
+        const double ta = pa[0][threadIdx.x], tb = pb[0][threadIdx.x];
         if (mode == 0) {
             const double m = ta * inv_M;
             double var = tb * inv_M - m * m;
@@ -183,9 +246,11 @@ __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict
     }
 }
 
-// y = act(gamma * (x - mean) * rstd + beta [+ residual]), fp16 in and out; two rows in flight per thread.
-__global__ void __launch_bounds__(256) bn_apply_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res,
-                                                       uint4* __restrict__ y, const float* __restrict__ gamma,
+// y = act(gamma * (x - mean) * rstd + beta [+ residual]), fp16 in and out; two rows in flight per thread.  With `mask`
+// one bit per element, set where y > 0, for D_MASK.  The rows are walked from the last to the first: the statistics pass
+// has just read x in the other direction, so what of it is still in L2 (126 MB) is read first.
+__global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res,
+                                                       uint4* __restrict__ y, uint8_t* __restrict__ mask, const float* __restrict__ gamma,
                                                        const float* __restrict__ beta, const float* __restrict__ mean,
                                                        const float* __restrict__ rstd, int act, float slope, size_t M, int C) {
     pdl_enter();
@@ -193,98 +258,85 @@ __global__ void __launch_bounds__(256) bn_apply_kernel(const uint4* __restrict__
     const int rpb = blockDim.x / cpr;
     const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
     float sc[8], sh[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int c = col * 8 + j;
-        sc[j] = (gamma ? gamma[c] : 1.f) * rstd[c];
-        sh[j] = (beta ? beta[c] : 0.f) - mean[c] * sc[j];
-    }
-    auto one = [&](const uint4& xv, const uint4& rv) -> uint4 {
+    bn_affine(col, gamma, beta, mean, rstd, sc, sh);
+    auto one = [&](size_t v, const uint4& xv, const uint4& rv) {
         float xf[8], rf[8];
         unpack8(xv, xf);
         if (res) unpack8(rv, rf);
+        unsigned bits = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             float t = xf[j] * sc[j] + sh[j];
             if (res) t += rf[j];
+            bits |= (positive_as_half(t) ? 1u : 0u) << j;
             if (act != 0 && t < 0.f) t = (act == 1) ? 0.f : t * slope;
             xf[j] = t;
         }
-        return pack8(xf);
+        y[v] = pack8(xf);
+        if (mask) mask[v] = static_cast<uint8_t>(bits);
     };
     const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
-    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
+    size_t k = static_cast<size_t>(blockIdx.x) * rpb + rsub;  // rows counted from the end
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    for (; row + stride < M; row += 2 * stride) {
-        const size_t v0 = row * cpr + col, v1 = (row + stride) * cpr + col;
+    for (; k + stride < M; k += 2 * stride) {
+        const size_t v0 = (M - 1 - k) * cpr + col, v1 = (M - 1 - k - stride) * cpr + col;
         const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
         const uint4 r0 = res ? __ldg(res + v0) : zero, r1 = res ? __ldg(res + v1) : zero;
-        y[v0] = one(x0, r0);
-        y[v1] = one(x1, r1);
+        one(v0, x0, r0);
+        one(v1, x1, r1);
     }
-    if (row < M) {
-        const size_t v0 = row * cpr + col;
-        y[v0] = one(__ldg(x + v0), res ? __ldg(res + v0) : zero);
+    if (k < M) {
+        const size_t v0 = (M - 1 - k) * cpr + col;
+        one(v0, __ldg(x + v0), res ? __ldg(res + v0) : zero);
     }
 }
 
-// dx = gamma * rstd * (dz - dbeta / M - xhat * dgamma / M) with dz = dy * act'(y), folded into
+// dx = gamma * rstd * (dz - dbeta / M - xhat * dgamma / M) with dz = dy * act'(.), folded into
 // dx = A * dz + B * x + C per channel; optionally dres = dz (the gradient of the residual input that was
-// added before the activation).  Two rows in flight per thread.
-__global__ void __launch_bounds__(256) bn_dx_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy,
-                                                    const uint4* __restrict__ y, uint4* __restrict__ dx, uint4* __restrict__ dres,
-                                                    const float* __restrict__ gamma, const float* __restrict__ mean,
-                                                    const float* __restrict__ rstd, const float* __restrict__ dbeta,
-                                                    const float* __restrict__ dgamma, int act, float slope, float inv_M,
-                                                    size_t M, int C) {
+// added before the activation).  Two rows in flight per thread, from the last row to the first as in bn_apply_kernel.
+template <int kDeriv>
+__global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, const BnForward f,
+                                                    uint4* __restrict__ dx, uint4* __restrict__ dres, const float* __restrict__ dbeta,
+                                                    const float* __restrict__ dgamma, float inv_M, size_t M, int C) {
     pdl_enter();
     const int cpr = C >> 3;
     const int rpb = blockDim.x / cpr;
     const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
-    float ka[8], kb[8], kc[8];
+    float ka[8], kb[8], kc[8], sc[8], sh[8];
+    if (kDeriv == D_X) bn_affine(col, f.gamma, f.beta, f.mean, f.rstd, sc, sh);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int c = col * 8 + j;
-        const float rs = rstd[c], mu = mean[c];
-        const float k0 = (gamma ? gamma[c] : 1.f) * rs, k1 = dbeta[c] * inv_M, k2 = dgamma[c] * inv_M;
+        const float rs = f.rstd[c], mu = f.mean[c];
+        const float k0 = (f.gamma ? f.gamma[c] : 1.f) * rs, k1 = dbeta[c] * inv_M, k2 = dgamma[c] * inv_M;
         ka[j] = k0;
         kb[j] = -k0 * rs * k2;
         kc[j] = k0 * (mu * rs * k2 - k1);
     }
-    auto one = [&](const uint4& xv, const uint4& dv, const uint4& yv, uint4& dz_out) -> uint4 {
-        float xf[8], df[8], yf[8];
+    auto one = [&](size_t v, const uint4& xv, const uint4& dv, const uint4& yv, unsigned bits) {
+        float xf[8], df[8];
         unpack8(xv, xf);
         unpack8(dv, df);
-        if (act != 0) unpack8(yv, yf);
+        act_backward<kDeriv>(df, xf, yv, bits, sc, sh, f.below);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float dz = df[j] * (act != 0 ? act_grad(act, slope, yf[j]) : 1.f);
-            df[j] = dz;
-            xf[j] = ka[j] * dz + kb[j] * xf[j] + kc[j];
-        }
-        dz_out = pack8(df);
-        return pack8(xf);
+        for (int j = 0; j < 8; ++j) xf[j] = ka[j] * df[j] + kb[j] * xf[j] + kc[j];
+        dx[v] = pack8(xf);
+        if (dres) dres[v] = pack8(df);
     };
     const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
-    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
+    size_t k = static_cast<size_t>(blockIdx.x) * rpb + rsub;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    for (; row + stride < M; row += 2 * stride) {
-        const size_t v0 = row * cpr + col, v1 = (row + stride) * cpr + col;
+    for (; k + stride < M; k += 2 * stride) {
+        const size_t v0 = (M - 1 - k) * cpr + col, v1 = (M - 1 - k - stride) * cpr + col;
         const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1), d0 = __ldg(dy + v0), d1 = __ldg(dy + v1);
-        const uint4 y0 = act != 0 ? __ldg(y + v0) : zero, y1 = act != 0 ? __ldg(y + v1) : zero;
-        uint4 z0, z1;
-        dx[v0] = one(x0, d0, y0, z0);
-        dx[v1] = one(x1, d1, y1, z1);
-        if (dres) {
-            dres[v0] = z0;
-            dres[v1] = z1;
-        }
+        const uint4 y0 = kDeriv == D_Y ? __ldg(f.y + v0) : zero, y1 = kDeriv == D_Y ? __ldg(f.y + v1) : zero;
+        const unsigned m0 = kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? __ldg(f.mask + v1) : 0u;
+        one(v0, x0, d0, y0, m0);
+        one(v1, x1, d1, y1, m1);
     }
-    if (row < M) {
-        const size_t v0 = row * cpr + col;
-        uint4 z0;
-        dx[v0] = one(__ldg(x + v0), __ldg(dy + v0), act != 0 ? __ldg(y + v0) : zero, z0);
-        if (dres) dres[v0] = z0;
+    if (k < M) {
+        const size_t v0 = (M - 1 - k) * cpr + col;
+        one(v0, __ldg(x + v0), __ldg(dy + v0), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
     }
 }
 
@@ -444,6 +496,13 @@ int nml_bn_workspace_size(long long rows, int channels, size_t* bytes) {
 int nml_bn_forward(const void* x, long long rows, int channels, const float* gamma, const float* beta, const void* residual,
                    int act, float slope, float eps, void* y, float* mean, float* rstd, void* workspace,
                    size_t workspace_bytes, void* stream) {
+    return nml_bn_forward_masked(x, rows, channels, gamma, beta, residual, act, slope, eps, y, nullptr, mean, rstd, workspace,
+                                 workspace_bytes, stream);
+}
+
+int nml_bn_forward_masked(const void* x, long long rows, int channels, const float* gamma, const float* beta, const void* residual,
+                          int act, float slope, float eps, void* y, void* mask, float* mean, float* rstd, void* workspace,
+                          size_t workspace_bytes, void* stream) {
     if (!x || !y || !mean || !rstd || act < 0 || act > 2) return NML_ERR_INVALID;
     if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
     if (!aligned16(x) || !aligned16(y) || (residual && !aligned16(residual))) return NML_ERR_INVALID;
@@ -454,13 +513,38 @@ int nml_bn_forward(const void* x, long long rows, int channels, const float* gam
     int threads;
     const int P = bn_grid(rows, channels, &threads);
     float* partial = static_cast<float*>(workspace);
-    launch(bn_reduce_kernel<false>, P, threads, 0, st, static_cast<const uint4*>(x), nullptr, nullptr, 0, 0.f, partial,
-                                                   static_cast<size_t>(rows), channels);
-    launch(bn_finish_kernel, (channels + 31) / 32, dim3(32, 32), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
-                                                                   nullptr, nullptr, mean, rstd);
-    launch(bn_apply_kernel, bn_grid_elementwise(rows, channels), threads, 0, st, static_cast<const uint4*>(x), static_cast<const uint4*>(residual),
-                                           static_cast<uint4*>(y), gamma, beta, mean, rstd, act, slope,
-                                           static_cast<size_t>(rows), channels);
+    const size_t M = static_cast<size_t>(rows);
+    const uint4* xv = static_cast<const uint4*>(x);
+    launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels);
+    launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
+           nullptr, nullptr, mean, rstd);
+    launch(bn_apply_kernel, bn_grid_elementwise(rows, channels), threads, 0, st, xv, static_cast<const uint4*>(residual),
+           static_cast<uint4*>(y), static_cast<uint8_t*>(mask), gamma, beta, mean, rstd, act, slope, M, channels);
+    NMLL_CUDA(cudaGetLastError());
+    g_layer_launches += 3;
+    return NML_OK;
+}
+
+static int bn_backward(const void* dy, const void* x, long long rows, int channels, int deriv, const BnForward& f, void* dx, void* dres,
+                       float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+    if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
+    if (!aligned16(dy) || !aligned16(x) || !aligned16(dx) || (f.y && !aligned16(f.y)) || (dres && !aligned16(dres))) return NML_ERR_INVALID;
+    size_t need = 0;
+    nml_bn_workspace_size(rows, channels, &need);
+    if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
+    int threads;
+    const int P = bn_grid(rows, channels, &threads);
+    float* partial = static_cast<float*>(workspace);
+    const size_t M = static_cast<size_t>(rows);
+    const uint4 *xv = static_cast<const uint4*>(x), *dyv = static_cast<const uint4*>(dy);
+    auto sums = deriv == D_NONE ? bn_grad_sums_kernel<D_NONE> : deriv == D_Y ? bn_grad_sums_kernel<D_Y>
+              : deriv == D_X ? bn_grad_sums_kernel<D_X> : bn_grad_sums_kernel<D_MASK>;
+    auto apply = deriv == D_NONE ? bn_dx_kernel<D_NONE> : deriv == D_Y ? bn_dx_kernel<D_Y>
+               : deriv == D_X ? bn_dx_kernel<D_X> : bn_dx_kernel<D_MASK>;
+    launch(sums, P, threads, 0, st, xv, dyv, f, partial, M, channels);
+    launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 1, 0.0, 0.f, f.mean, f.rstd, dbeta, dgamma);
+    launch(apply, bn_grid_elementwise(rows, channels), threads, 0, st, xv, dyv, f, static_cast<uint4*>(dx), static_cast<uint4*>(dres),
+           dbeta, dgamma, static_cast<float>(1.0 / static_cast<double>(rows)), M, channels);
     NMLL_CUDA(cudaGetLastError());
     g_layer_launches += 3;
     return NML_OK;
@@ -470,26 +554,18 @@ int nml_bn_backward(const void* dy, const void* y, const void* x, long long rows
                     const float* mean, const float* rstd, int act, float slope, void* dx, void* dres, float* dgamma,
                     float* dbeta, void* workspace, size_t workspace_bytes, void* stream) {
     if (!dy || !x || !mean || !rstd || !dx || !dgamma || !dbeta || act < 0 || act > 2 || (act != 0 && !y)) return NML_ERR_INVALID;
-    if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
-    if (!aligned16(dy) || !aligned16(x) || !aligned16(dx) || (y && !aligned16(y)) || (dres && !aligned16(dres))) return NML_ERR_INVALID;
-    size_t need = 0;
-    nml_bn_workspace_size(rows, channels, &need);
-    if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int threads;
-    const int P = bn_grid(rows, channels, &threads);
-    float* partial = static_cast<float*>(workspace);
-    launch(bn_reduce_kernel<true>, P, threads, 0, st, static_cast<const uint4*>(x), static_cast<const uint4*>(dy),
-                                                  static_cast<const uint4*>(y), act, slope, partial,
-                                                  static_cast<size_t>(rows), channels);
-    launch(bn_finish_kernel, (channels + 31) / 32, dim3(32, 32), 0, st, partial, P, channels, 1, 0.0, 0.f, mean, rstd, dbeta, dgamma);
-    launch(bn_dx_kernel, bn_grid_elementwise(rows, channels), threads, 0, st, static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<const uint4*>(y),
-                                        static_cast<uint4*>(dx), static_cast<uint4*>(dres), gamma, mean, rstd, dbeta, dgamma, act,
-                                        slope, static_cast<float>(1.0 / static_cast<double>(rows)), static_cast<size_t>(rows),
-                                        channels);
-    NMLL_CUDA(cudaGetLastError());
-    g_layer_launches += 3;
-    return NML_OK;
+    const BnForward f = {act != 0 ? static_cast<const uint4*>(y) : nullptr, nullptr, gamma, nullptr, mean, rstd, act == 1 ? 0.f : slope};
+    return bn_backward(dy, x, rows, channels, act != 0 ? D_Y : D_NONE, f, dx, dres, dgamma, dbeta, workspace, workspace_bytes,
+                       static_cast<cudaStream_t>(stream));
+}
+
+int nml_bn_backward_masked(const void* dy, const void* mask, const void* x, long long rows, int channels, const float* gamma,
+                           const float* beta, const float* mean, const float* rstd, int act, float slope, void* dx, void* dres,
+                           float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!dy || !x || !mean || !rstd || !dx || !dgamma || !dbeta || act < 0 || act > 2) return NML_ERR_INVALID;
+    const BnForward f = {nullptr, static_cast<const uint8_t*>(mask), gamma, beta, mean, rstd, act == 1 ? 0.f : slope};
+    return bn_backward(dy, x, rows, channels, act == 0 ? D_NONE : mask ? D_MASK : D_X, f, dx, dres, dgamma, dbeta, workspace,
+                       workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
 long long nml_layers_launch_count(void) { return g_layer_launches.load(); }

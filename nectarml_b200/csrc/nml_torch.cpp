@@ -372,49 +372,57 @@ PyObject* py_linear_backward_weight(PyObject*, PyObject* const* a, Py_ssize_t n)
 }
 
 // ------------------------------------------------------------------ batch norm --
-// bn_forward(x, residual, gamma, beta, act, slope, eps, workspace) -> (y, mean, rstd)
+// bn_forward(x, residual, gamma, beta, act, slope, eps, workspace) -> (y, mean, rstd, mask): the mask of y > 0 where the
+// backward cannot tell it from x, else None
 PyObject* py_bn_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!arity(n, 8)) return nullptr;
     return guarded([&]() -> PyObject* {
         const at::Tensor &x = tensor(a[0], "x"), &gamma = tensor(a[2], "gamma"), &beta = tensor(a[3], "beta");
         const at::Tensor* res = tensor_or_none(a[1], "residual");
         const int64_t c = x.size(-1), rows = x.numel() / c;
+        const int act = static_cast<int>(as_int(a[4]));
         const at::Tensor y = at::empty(x.sizes(), x.options());
         const auto fopt = at::TensorOptions().dtype(at::kFloat).device(x.device());
         const at::Tensor mean = at::empty({c}, fopt), rstd = at::empty({c}, fopt);
+        at::Tensor mask;
+        const bool has_mask = res != nullptr && act != 0;
+        if (has_mask) mask = at::empty({x.numel() / 8}, fopt.dtype(at::kByte));
         size_t need = 0;
         check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
         const Scratch ws = scratch(a[7], need, x);
-        check(nml_bn_forward(ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)), static_cast<const float*>(ptr(beta)),
-                             ptr_or_null(res), static_cast<int>(as_int(a[4])), static_cast<float>(as_double(a[5])),
-                             static_cast<float>(as_double(a[6])), ptr(y), static_cast<float*>(ptr(mean)),
-                             static_cast<float*>(ptr(rstd)), ws.p, ws.bytes, stream()));
-        PyObject* t = PyTuple_New(3);
+        check(nml_bn_forward_masked(ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)),
+                                    static_cast<const float*>(ptr(beta)), ptr_or_null(res), act, static_cast<float>(as_double(a[5])),
+                                    static_cast<float>(as_double(a[6])), ptr(y), has_mask ? ptr(mask) : nullptr,
+                                    static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), ws.p, ws.bytes, stream()));
+        PyObject* t = PyTuple_New(4);
         PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(y));
         PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(mean));
         PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(rstd));
+        PyTuple_SET_ITEM(t, 3, has_mask ? THPVariable_Wrap(mask) : Py_NewRef(Py_None));
         return t;
     });
 }
 
-// bn_backward(dy, y, x, gamma, mean, rstd, act, slope, want_residual_grad, dgamma, dbeta, workspace) -> (dx, dres)
+// bn_backward(dy, mask, x, gamma, beta, mean, rstd, act, slope, want_residual_grad, dgamma, dbeta, workspace) -> (dx, dres)
 PyObject* py_bn_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (!arity(n, 12)) return nullptr;
+    if (!arity(n, 13)) return nullptr;
     return guarded([&]() -> PyObject* {
-        const at::Tensor &dy = tensor(a[0], "dy"), &y = tensor(a[1], "y"), &x = tensor(a[2], "x"), &gamma = tensor(a[3], "gamma"),
-                         &mean = tensor(a[4], "mean"), &rstd = tensor(a[5], "rstd"), &dgamma = tensor(a[9], "dgamma"), &dbeta = tensor(a[10], "dbeta");
+        const at::Tensor &dy = tensor(a[0], "dy"), &x = tensor(a[2], "x"), &gamma = tensor(a[3], "gamma"), &beta = tensor(a[4], "beta"),
+                         &mean = tensor(a[5], "mean"), &rstd = tensor(a[6], "rstd"), &dgamma = tensor(a[10], "dgamma"), &dbeta = tensor(a[11], "dbeta");
+        const at::Tensor* mask = tensor_or_none(a[1], "mask");
         const int64_t c = x.size(-1), rows = x.numel() / c;
         const at::Tensor dx = at::empty(x.sizes(), x.options());
         at::Tensor dres;
-        const bool has_res = as_int(a[8]) != 0;
+        const bool has_res = as_int(a[9]) != 0;
         if (has_res) dres = at::empty(x.sizes(), x.options());
         size_t need = 0;
         check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
-        const Scratch ws = scratch(a[11], need, x);
-        check(nml_bn_backward(ptr(dy), ptr(y), ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)),
-                              static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), static_cast<int>(as_int(a[6])),
-                              static_cast<float>(as_double(a[7])), ptr(dx), has_res ? ptr(dres) : nullptr,
-                              static_cast<float*>(ptr(dgamma)), static_cast<float*>(ptr(dbeta)), ws.p, ws.bytes, stream()));
+        const Scratch ws = scratch(a[12], need, x);
+        check(nml_bn_backward_masked(ptr(dy), ptr_or_null(mask), ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)),
+                                     static_cast<const float*>(ptr(beta)), static_cast<const float*>(ptr(mean)),
+                                     static_cast<const float*>(ptr(rstd)), static_cast<int>(as_int(a[7])),
+                                     static_cast<float>(as_double(a[8])), ptr(dx), has_res ? ptr(dres) : nullptr,
+                                     static_cast<float*>(ptr(dgamma)), static_cast<float*>(ptr(dbeta)), ws.p, ws.bytes, stream()));
         return pair(dx, has_res ? &dres : nullptr);
     });
 }

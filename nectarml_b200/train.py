@@ -226,21 +226,22 @@ class _BnActFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, residual, token, layer, act):
-        y, mean, rstd = ops._native.bn_forward(x, residual, layer.gamma, layer.beta, act, 0.2, layer.eps, _bn_ws)
+        y, mean, rstd, mask = ops._native.bn_forward(x, residual, layer.gamma, layer.beta, act, 0.2, layer.eps, _bn_ws)
         ctx.layer, ctx.act, ctx.has_res = layer, act, residual is not None
-        ctx.save_for_backward(x, y, mean, rstd)
+        ctx.save_for_backward(x, mean, rstd, mask)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         layer = ctx.layer
-        x, y, mean, rstd = ctx.saved_tensors
+        x, mean, rstd, mask = ctx.saved_tensors
         dy = dy.contiguous()
         grads = None
 
         def run(dgamma, dbeta):
             nonlocal grads
-            grads = ops._native.bn_backward(dy, y, x, layer.gamma, mean, rstd, ctx.act, 0.2, int(ctx.has_res), dgamma, dbeta, _bn_ws)
+            grads = ops._native.bn_backward(dy, mask, x, layer.gamma, layer.beta, mean, rstd, ctx.act, 0.2, int(ctx.has_res),
+                                            dgamma, dbeta, _bn_ws)
         layer.weight_gradient(run)
         return grads[0], grads[1], None, None, None
 

@@ -46,3 +46,44 @@ def test_rows_that_do_not_start_on_16_bytes(rows, fout, oracle):
     assert_f16(got, want, "fp32 tensors, fp16 arithmetic")
     assert np.array_equal(got, r(got)), "rounded through fp16"
     ops.device_status()
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (3, 64), (1000, 24), (37, 2048)])
+@pytest.mark.parametrize("act", [0, 1, 2])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_batch_norm_backward_with_and_without_y(rows, c, act, with_res):
+    """The activation's derivative from y, from x, and from the forward's mask: the same bits, zeros and values that
+    round to zero included."""
+    import ctypes as C
+    from nectarml_b200 import _lib
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    gen = torch.Generator(device="cuda").manual_seed(rows + c + act)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
+    x, dy, res = rnd(rows, c).half(), rnd(rows, c).half(), (rnd(rows, c).half() if with_res else None)
+    gamma, beta = rnd(c), rnd(c) * 0.3
+    gamma[::3] = 0.0     # y is beta there ...
+    beta[::6] = 2.0e-8   # ... and rounds to zero, or is zero
+    beta[3::6] = 0.0
+    need = C.c_size_t()
+    _lib.check(lib.nml_bn_workspace_size(rows, c, C.byref(need)))
+    ws = torch.empty(need.value, dtype=torch.uint8, device="cuda")
+    p = lambda t: t.data_ptr() if t is not None else None  # noqa: E731
+    got = []
+    for masked in (False, True):
+        y, dx, dres = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+        mask = torch.zeros(rows * c // 8, dtype=torch.uint8, device="cuda") if with_res else None
+        mean, rstd, dg, db = (torch.empty(c, device="cuda") for _ in range(4))
+        if masked:
+            _lib.check(lib.nml_bn_forward_masked(p(x), rows, c, p(gamma), p(beta), p(res), act, 0.2, 1e-5, p(y), p(mask), p(mean), p(rstd),
+                                                 p(ws), need.value, st))
+            _lib.check(lib.nml_bn_backward_masked(p(dy), p(mask), p(x), rows, c, p(gamma), p(beta), p(mean), p(rstd), act, 0.2, p(dx),
+                                                  p(dres), p(dg), p(db), p(ws), need.value, st))
+        else:
+            _lib.check(lib.nml_bn_forward(p(x), rows, c, p(gamma), p(beta), p(res), act, 0.2, 1e-5, p(y), p(mean), p(rstd), p(ws),
+                                          need.value, st))
+            _lib.check(lib.nml_bn_backward(p(dy), p(y), p(x), rows, c, p(gamma), p(mean), p(rstd), act, 0.2, p(dx), p(dres), p(dg), p(db),
+                                           p(ws), need.value, st))
+        got.append((y, dx, dres, mean, rstd, dg, db))
+    ops.device_status()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

@@ -229,6 +229,7 @@ static int load_helper_kernels() {
         (const void*)pack_phase_weights_kernel<float, float>, (const void*)pack_phase_weights_kernel<float, __half>,
         (const void*)pack_phase_weights_kernel<__half, float>, (const void*)pack_phase_weights_kernel<__half, __half>,
         (const void*)to_float_kernel<__half>, (const void*)colsum_finish_kernel,
+        (const void*)repack_half_tile_kernel, (const void*)repack_half_rows_kernel, (const void*)wgrad_reduce_taps_kernel,
         (const void*)wgrad_reduce_rows4_kernel, (const void*)wgrad_reduce_kernel, (const void*)wgrad_reduce_deep4_kernel,
     };
     for (const void* f : fns) {
@@ -334,6 +335,22 @@ static void convert_rows(const void* src, int dtype, void* p0, void* p1, int enc
     if (dtype == NML_F32) launch_short(convert_rows_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(src), p0, p1, enc, rows, c, cp);
     else launch_short(convert_rows_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(src), p0, p1, enc, rows, c, cp);
     ++g_launches;
+}
+
+// [B][R][Cc] fp16 -> [B][Cc][Rp] fp16 through the 16-byte kernels; false where the shape does not allow them.
+static bool repack_half(const void* src, void* dst, int B, int R, int Cc, int Rp, cudaStream_t st) {
+    const __half* w = static_cast<const __half*>(src);
+    __half* o = static_cast<__half*>(dst);
+    if ((reinterpret_cast<uintptr_t>(src) & 15) || Rp % 8) return false;
+    if (Cc > 64) {
+        if (Cc % 8) return false;
+        launch_short(repack_half_tile_kernel, dim3(ceil_div(Cc, 64), ceil_div(Rp, 64), B), 256, 0, st, w, o, R, Cc, Rp);
+    } else {
+        if ((static_cast<size_t>(R) * Cc) % 8) return false;
+        launch_short(repack_half_rows_kernel, dim3(ceil_div(Rp, 256), B), 256, 256 * (Cc | 1) * sizeof(__half), st, w, o, R, Cc, Rp);
+    }
+    ++g_launches;
+    return true;
 }
 
 // Converts an activation tensor into the NHWC operand encoding of `mi` unless it already is one.
@@ -760,9 +777,12 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                 static_cast<const T*>(f.w), p0, p1, mi.enc, rR, rC, kp);                                                         \
     } while (0)
             if (rows_only) convert_rows(f.w, f.w_dtype, p0, p1, mi.enc, static_cast<size_t>(rB) * f.d0, f.d1, kp, st);
-            else if (f.w_dtype == NML_F32) NML_REPACK(float); else NML_REPACK(__half);
+            else if (f.w_dtype == NML_F16 && mi.enc == ENC_F16 && repack_half(f.w, p0, rB, rR, rC, kp, st)) {}
+            else {
+                if (f.w_dtype == NML_F32) NML_REPACK(float); else NML_REPACK(__half);
+                ++g_launches;
+            }
 #undef NML_REPACK
-            if (!rows_only) ++g_launches;
             NML_CUDA(cudaGetLastError());
         }
     }
@@ -1479,6 +1499,9 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             const size_t total4 = dw_elems / 4;
             const int blocks = static_cast<int>(std::min<size_t>((total4 + 255) / 256, 148 * 16));
             launch_short(wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
+        } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535) {
+            launch_short(wgrad_reduce_taps_kernel, dim3(ceil_div(g.patch_c, 64), g.plain_c), 256, 64 * (P.n_taps | 1) * sizeof(float), st,
+                         planes, g.dw, split, plane_elems, g.patch_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
         } else {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + 255) / 256, 148 * 16));
@@ -1596,10 +1619,12 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
             if (!ws.fits()) return NML_ERR_WORKSPACE;
             int rc = profile_open(st);
             if (rc) return rc;
-            const dim3 grid(ceil_div(d->in_features, 64), ceil_div(d->out_features, 64), 1);
-            launch_short(repack_weight_tile_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in1), wt, nullptr, ENC_F16,
-                                                                   d->out_features, d->in_features, d->out_features);
-            ++g_launches;
+            if (!repack_half(in1, wt, 1, d->out_features, d->in_features, d->out_features, st)) {
+                const dim3 grid(ceil_div(d->in_features, 64), ceil_div(d->out_features, 64), 1);
+                launch_short(repack_weight_tile_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in1), wt, nullptr, ENC_F16,
+                             d->out_features, d->in_features, d->out_features);
+                ++g_launches;
+            }
             NML_CUDA(cudaGetLastError());
         }
         f.w = wt; f.d0 = d->in_features; f.d1 = d->out_features; f.k_is_dim0 = 0;

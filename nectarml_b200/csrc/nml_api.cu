@@ -1385,7 +1385,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                 if (real != sp) continue;
                 long long rounds = ceil_div(mt * nt * sp, pair ? sms / 2 : sms);
                 double cost = rounds * (per_sp + 4) * block_us;
-                if (sp > 1) cost += 3.0 + (2.0 * sp + 1.0) * dw_bytes / 5e6;
+                if (sp > 1 || T > 1) cost += 3.0 + (2.0 * sp + 1.0) * dw_bytes / 5e6;
                 if (best < 0 || cost < best * (width == 256 ? 1.0 : 0.95)) {  // the wider tile unless the gain is clear
                     best = cost;
                     split = sp;
@@ -1404,18 +1404,21 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     }
     P.split_k = split;
     P.num_tiles = mn_tiles * split;
-    // One K slice writes dW itself.  Several slices store their partial sums into one fp32 plane each
+    // One K slice of a one-tap layer writes dW itself.  With several taps the rows of a tile are 4 * taps bytes apart in dW
+    // (a store instruction would touch 32 sectors: 4x4 512->512 on 4x4 images took 29 us for its 17 MB of gradient), so
+    // they go through a plane even when there is one slice.  Several slices store their partial sums into one fp32 plane each
     // (like dW for the patch walk, else [plain channel][rows of the tile walk]); wgrad_reduce_* then adds
     // the planes in slice order and writes dW once -- no zero-fill, no atomics, bitwise repeatable.
     const size_t dw_elems = static_cast<size_t>(g.plain_c) * g.patch_c * T;
     const int plane_rows = P.wpatch ? 0 : m_tiles * (P.pair ? 2 : 1) * kTileM;
-    const size_t plane_elems = (split <= 1) ? 0 : P.wpatch ? round_up(dw_elems, 4) : static_cast<size_t>(g.plain_c) * plane_rows;
-    float* planes = (split > 1) ? static_cast<float*>(ws.take(static_cast<size_t>(split) * plane_elems * sizeof(float))) : nullptr;
+    const bool staged = split > 1 || (!P.wpatch && !P.kw_pack && T > 1);
+    const size_t plane_elems = !staged ? 0 : P.wpatch ? round_up(dw_elems, 4) : static_cast<size_t>(g.plain_c) * plane_rows;
+    float* planes = staged ? static_cast<float*>(ws.take(static_cast<size_t>(split) * plane_elems * sizeof(float))) : nullptr;
     if (ws.dry) return NML_OK;
     if (!ws.fits()) return NML_ERR_WORKSPACE;
-    P.out = (split > 1) ? planes : g.dw;
+    P.out = staged ? planes : g.dw;
     P.plane_elems = plane_elems;
-    P.ld_plane = plane_rows;
+    P.ld_plane = staged ? plane_rows : 0;
     // A wave of CTAs re-reads one operand in full; make that the smaller tensor.
     {
         const double patch_bytes = static_cast<double>(g.batch) * g.patch_h * g.patch_w * cpa * mi.es;
@@ -1487,7 +1490,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     int slot = -1;
     rc = launch_kernel(P, ds, st, &slot);
     if (rc) return rc;
-    if (split > 1) {
+    if (staged) {
         const bool vec_ok = (reinterpret_cast<uintptr_t>(g.dw) & 15) == 0;
         if (P.wpatch && vec_ok && dw_elems % 4 == 0 && split > 8) {
             const size_t total4 = dw_elems / 4;

@@ -162,7 +162,7 @@ struct KParams {
     // apart) and a second kernel adds the planes in slice order, so results are bitwise repeatable.
     // wgrad planes are laid out [plain channel][ld_plane rows of the tile walk] (patch walk: like dW).
     unsigned long long plane_elems;
-    int ld_plane;
+    int ld_plane;        // wgrad: rows of a plane; 0: the tile is stored into dW itself (or, patch walk, a copy of its layout)
     Phase phases[kMaxPhases];
     Tap taps[kMaxTaps];
 };
@@ -220,20 +220,27 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Stores 32 (or fewer) consecutive output channels of one accumulator row to a channel-major output: lanes are
-// consecutive pixels, so each column store coalesces.
-__device__ __noinline__ void store_row_chunk(const KParams& P, const float (&v)[32], size_t row_off, size_t col_stride,
-                                             int cg, int ncols) {
-    if (P.out_f16) {
-        __half* o = reinterpret_cast<__half*>(P.out) + row_off + static_cast<size_t>(cg) * col_stride;
+// Stores columns 0 .. ncols-1 (at most 32) of one accumulator row `stride` elements apart; lanes are consecutive rows, so
+// each column store coalesces.  The address is advanced, not computed per column: 64-bit products and a bound check per
+// element made 20 instructions of a store, and a 128 x 256 tile of a weight gradient took 25000 clocks to leave.
+template <typename T>
+__device__ __forceinline__ void store_columns(T* o, size_t stride, const uint32_t (&r)[32], int ncols) {
+    auto value = [](uint32_t bits) {
+        if constexpr (sizeof(T) == 2) return __float2half_rn(__uint_as_float(bits));
+        else return __uint_as_float(bits);
+    };
+    if (ncols == 32) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (j < ncols) o[j * col_stride] = __float2half_rn(v[j]);
+        for (int j = 0; j < 32; ++j) {
+            *o = value(r[j]);
+            o += stride;
+        }
     } else {
-        float* o = reinterpret_cast<float*>(P.out) + row_off + static_cast<size_t>(cg) * col_stride;
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (j < ncols) o[j * col_stride] = v[j];
+        for (int j = 0; j < 32; ++j) {
+            if (j < ncols) *o = value(r[j]);
+            o += stride;
+        }
     }
 }
 
@@ -1172,11 +1179,11 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             uint32_t r[32];
                             tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + i * P.bn + c0, r);
                             tmem_ld_wait();
-                            if (w_valid) {
+                            if (!w_live) {
 #pragma unroll
-                                for (int j = 0; j < 32; ++j)
-                                    if (j < ncols) S[j * run + w_off] = w_live ? __uint_as_float(r[j]) : 0.f;
+                                for (int j = 0; j < 32; ++j) r[j] = 0u;
                             }
+                            if (w_valid) store_columns(S + w_off, run, r, ncols);
                             __syncwarp();
                         }
                         if (!meet()) {
@@ -1217,12 +1224,11 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         tmem_ld_wait();
                         const int cg = w_col_base + c0;
                         const int ncols = min(32, P.c_out - cg);
-                        if (w_valid) {
-                            float* o = w_plane + w_off + static_cast<size_t>(cg) * w_stride;
+                        if (!w_live) {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (j < ncols) o[j * w_stride] = w_live ? __uint_as_float(r[j]) : 0.f;
+                            for (int j = 0; j < 32; ++j) r[j] = 0u;
                         }
+                        if (w_valid) store_columns(w_plane + w_off + static_cast<size_t>(cg) * w_stride, w_stride, r, ncols);
                         __syncwarp();  // tcgen05.ld is warp-collective: reconverge before the next chunk
                     }
                 }
@@ -1295,7 +1301,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     row_off = static_cast<size_t>(pc) * P.n_taps + t;
                     col_stride = static_cast<size_t>(P.c_patch) * P.n_taps;
                 }
-                if (P.split_k > 1) {
+                if (P.ld_plane > 0) {
                     // partial sums go to this slice's plane, [column][row of the tile walk]: lanes are consecutive
                     // rows, so every column store coalesces; rows beyond the gradient are written too (the planes
                     // are padded to whole tiles) and never read
@@ -1735,21 +1741,26 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                                 reinterpret_cast<float4*>(o)[q] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
                                                                               __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
                         } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (j < ncols) o[j * col_stride] = __uint_as_float(r[j]);
+                            store_columns(o, col_stride, r, ncols);
                         }
                     }
                 } else {
-                    float v[32];
+                    // channel-major output
+                    if (P.bias != nullptr) {
+                        const float bl = lane < ncols ? __ldg(P.bias + cg + lane) : 0.f;  // one load, handed round
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        float x = __uint_as_float(r[j]);
-                        if (P.bias != nullptr && j < ncols) x += P.bias[cg + j];
-                        if (P.round_f16) x = round_through_f16(x);
-                        v[j] = x;
+                        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __shfl_sync(0xffffffffu, bl, j));
                     }
-                    if (row_valid) store_row_chunk(P, v, row_off, col_stride, cg, ncols);
+                    const size_t o = row_off + static_cast<size_t>(cg) * col_stride;
+                    if (kOutF16) {
+                        if (row_valid) store_columns(reinterpret_cast<__half*>(P.out) + o, col_stride, r, ncols);
+                    } else {
+                        if (P.round_f16) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(round_through_f16(__uint_as_float(r[j])));
+                        }
+                        if (row_valid) store_columns(reinterpret_cast<float*>(P.out) + o, col_stride, r, ncols);
+                    }
                 }
                 __syncwarp();  // tcgen05.ld is warp-collective: reconverge before the next chunk
             }

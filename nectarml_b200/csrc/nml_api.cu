@@ -220,7 +220,7 @@ static int load_helper_kernels() {
         (const void*)nchw_to_nhwc_kernel<float>, (const void*)nchw_to_nhwc_kernel<__half>,
         (const void*)convert_rows_kernel<float>, (const void*)convert_rows_kernel<__half>,
         (const void*)colsum_rows_kernel<float>, (const void*)colsum_rows_kernel<__half>,
-        (const void*)colsum_rows_f16x8_kernel,
+        (const void*)colsum_vectors_kernel<float>, (const void*)colsum_vectors_kernel<__half>,
         (const void*)repack_weight_tile_kernel<float>, (const void*)repack_weight_tile_kernel<__half>,
         (const void*)repack_weight_rows_kernel<float>, (const void*)repack_weight_rows_kernel<__half>,
         (const void*)pad_pack_c8_kernel<float>, (const void*)pad_pack_c8_kernel<__half>,
@@ -300,6 +300,7 @@ static bool math_info(int math, MathInfo* m) {
 // Bias gradient = column sums of dY, in two stages so that the result is bitwise repeatable: the pass
 // that reads dY writes rows of partial sums ([P][stride], one row per block), colsum_finish_kernel adds
 // the rows in a fixed order.  Both scratch matrices come from the workspace.
+constexpr int kColsumSegment = 4096;  // rows one block of the second stage adds up
 struct ColsumScratch {
     float* partial = nullptr;
     float* second = nullptr;
@@ -310,16 +311,16 @@ static ColsumScratch colsum_scratch(Bump& ws, size_t P, int stride) {
     c.P = static_cast<int>(P);
     c.stride = stride;
     c.partial = static_cast<float*>(ws.take(P * stride * sizeof(float)));
-    if (P > 256) c.second = static_cast<float*>(ws.take(((P + 255) / 256) * stride * sizeof(float)));
+    if (P > kColsumSegment) c.second = static_cast<float*>(ws.take(((P + kColsumSegment - 1) / kColsumSegment) * stride * sizeof(float)));
     return c;
 }
 static int colsum_finish(const ColsumScratch& cs, int C, float* out, cudaStream_t st) {
     const float* src = cs.partial;
     int P = cs.P, stride = cs.stride;
     for (;;) {
-        const int S = ceil_div(P, 256);
+        const int S = ceil_div(P, kColsumSegment);
         float* dst = (S == 1) ? out : (src == cs.partial ? cs.second : cs.partial);
-        launch_short(colsum_finish_kernel, dim3(ceil_div(C, 32), S), dim3(32, 8), 0, st, src, P, stride, C, dst, cs.stride, 256);
+        launch_short(colsum_finish_kernel, dim3(ceil_div(C, 8), S), dim3(8, 128), 0, st, src, P, stride, C, dst, cs.stride, kColsumSegment);
         ++g_launches;
         if (S == 1) break;
         src = dst;
@@ -364,13 +365,18 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
                         (layout == NML_NHWC || (h == 1 && w == 1) || c == 1);
     const size_t pixels = static_cast<size_t>(batch) * h * w;
     // row-major column sums: enough row blocks to fill the GPU, few enough that the second stage stays negligible
-    const int col_blocks = ceil_div(c, 256);
+    // (the width of a column block has to follow from the shape alone: workspace queries pass no pointer)
+    const int vector = dtype == NML_F16 ? 8 : 4;
+    const int col_blocks = ceil_div(c, c % vector == 0 ? 32 * vector : 256);
+    const bool vectors = c % vector == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
     const int rows_per_block = static_cast<int>(std::max<size_t>(64, round_up(ceil_div(static_cast<int>(std::min<size_t>(pixels, 1u << 30)), std::max(1, 1184 / col_blocks)), 8)));
     const size_t row_blocks = (pixels + rows_per_block - 1) / rows_per_block;
     auto rows_colsum = [&](const ColsumScratch& cs) -> int {
         dim3 grid(col_blocks, static_cast<unsigned>(row_blocks));
-        if (dtype == NML_F16 && c % 8 == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0)
-            launch(colsum_rows_f16x8_kernel, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
+        if (dtype == NML_F16 && vectors)
+            launch(colsum_vectors_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
+        else if (vectors)
+            launch(colsum_vectors_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), cs.partial, pixels, c, rows_per_block);
         else if (dtype == NML_F16)
             launch(colsum_rows_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
         else
@@ -515,7 +521,9 @@ static int profile_open(cudaStream_t st) {
 static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open_slot = nullptr) {
     // Narrow tiles finish a 64-deep K slice in well under the barrier round trip of a stage, so they
     // take two slices per stage (8 MMAs per round trip); 256-wide tiles already fill 512 clocks.
-    P.ka = (P.pair && P.bn == 256) ? 1 : std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
+    // The 3xTF32 split takes one slice: its two planes are 12 MMAs.
+    P.ka = P.planes == 2 ? 2 : (P.pair && P.bn == 256) ? 1 : std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
+    P.tbufs = 2 * P.bn * P.planes <= 512 ? 2 : 1;
     const int stage_bytes = P.ka * (kStageABytes + (P.pair ? P.bn / 2 : P.bn) * 128);
     // Shared memory: the operand ring, then the epilogue's staging buffers (two per warp if that does not
     // cost a ring stage, else one), the per-warp bias tiles, and the barriers.
@@ -526,9 +534,9 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     {
         const int cpi = P.out_f16 ? 64 : 32;
         int k_slices = 0;  // 64-deep (fp16) K slices per tile, longest phase
-        for (int p = 0; p < P.n_phases; ++p) k_slices = std::max(k_slices, P.passes * P.c_blocks * P.phases[p].tap_count);
+        for (int p = 0; p < P.n_phases; ++p) k_slices = std::max(k_slices, P.c_blocks * P.phases[p].tap_count);
         const bool short_k = k_slices <= tune().epi8_k;
-        P.epi_warps = (tma_out && short_k && P.bn / cpi >= 2 && tune().epi8) ? 8 : 4;
+        P.epi_warps = (tma_out && short_k && P.planes == 1 && P.bn / cpi >= 2 && tune().epi8) ? 8 : 4;
     }
     size_t smem;
     if (P.wpatch) {
@@ -552,7 +560,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         const int res_bytes = P.c_blocks * P.n_taps * b_slice;  // the taps of every phase
         P.stg_bufs = 2;
         int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
-        const bool res_wanted = P.n_tiles == 1 && P.passes == 1 && tune().bres;
+        const bool res_wanted = P.n_tiles == 1 && P.planes == 1 && tune().bres;
         if (res_wanted && res_bytes + 2 * P.patch_bytes > avail) {  // trade staging for residency
             P.stg_bufs = 1;
             avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
@@ -570,9 +578,9 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         } else {
             P.b_resident = 0;
             // B streams tap by tap; narrow tiles take two taps per stage (8 MMAs per barrier round trip)
-            P.ka = std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
+            P.ka = P.planes == 2 ? 2 : std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
             const int b_stage = P.ka * b_slice;
-            P.a_stages = std::min(3, std::max(2, P.passes * P.c_blocks));
+            P.a_stages = P.planes == 2 ? 4 : std::min(3, std::max(2, P.c_blocks));  // (the split takes its patches in pairs)
             P.stages = std::min(8, (avail - P.a_stages * P.patch_bytes) / b_stage);
             if (P.stages < 3) {  // wide tiles: give the B ring room
                 P.a_stages = 2;
@@ -816,7 +824,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     P.mode = MODE_FPROP;
     P.out_mode = (f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1)) ? OUT_NCHW : OUT_NHWC;
     P.kind = mi.kind;
-    P.passes = (mi.planes == 2) ? 3 : 1;
+    P.planes = mi.planes;
+    const int products = mi.planes == 2 ? 3 : 1;  // tensor-core products per K slice
     P.kb = mi.kb;
     P.c_blocks = c_blocks;
     P.a_mn_major = 0;
@@ -953,9 +962,9 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         // streaming B tap by tap pays only for the 3xTF32 split (a barrier round trip per 4 short MMAs otherwise)
         const int bn_res = (N <= 16 && !b_mn_major) ? 16 : static_cast<int>(round_up(N, 32));
         const long long res_need = 1ll * c_blocks * n_taps * bn_res * 128 + 2 * round_up(pw_ * ph_ * 128, 1024);
-        const bool res_ok = P.passes == 1 && N <= 256 &&
+        const bool res_ok = P.planes == 1 && N <= 256 &&
                             res_need <= 232448 - (1024 + 256 + kBiasTileBytes) - 4 * kStagingBufBytes;
-        const bool streamed_ok = N <= 128 && (P.passes == 3 || mode >= 3);
+        const bool streamed_ok = N <= 128 && (P.planes == 2 || mode >= 3);
         if (can && mode && (mode == 2 || (eff_patch >= 0.8 * eff_box && (res_ok || streamed_ok)))) {
             patch_resident = res_ok;
             P.patch = 1;
@@ -983,7 +992,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             m_tiles_all += 1ll * ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) *
                            ceil_div(f.batch, 1 << P.nb_log2);
         const int forced = (P.patch && patch_resident) ? ((N <= 16 && !b_mn_major) ? 16 : static_cast<int>(round_up(N, 32)))
-                                                       : tune().bn;
+                                                       : P.planes == 2 ? std::min(tune().bn, 128) : tune().bn;
         const int cand[4] = {256, 128, 64, forced};
         const double cost[3] = {1.0, 1.28, 2.24};
         double best = -1;
@@ -991,7 +1000,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             if (forced ? i != 3 : i == 3) continue;
             int nt = ceil_div(N, cand[i]);
             int bn = static_cast<int>(round_up(ceil_div(N, nt), b_mn_major ? 64 : (forced == 16 ? 16 : 32)));
-            if (bn > 256) continue;
+            // (the split keeps two accumulators per tile; 256 columns would leave one buffer: 16384 x 1024 -> 1024 125 -> 150 us)
+            if (bn > 256 || (bn > 128 && P.planes == 2)) continue;
             double rounds = static_cast<double>(ceil_div(static_cast<int>(std::min<long long>(m_tiles_all * nt, 1 << 30)), limited(ds->sms)));
             double t = rounds * bn * (bn > 128 ? cost[0] : bn > 64 ? cost[1] : cost[2]);
             if (best < 0 || t < best * 0.97) {  // prefer the wider tile unless the gain is clear
@@ -1003,22 +1013,22 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         // Tiles that leave half the SMs idle under a long K loop: tile width and number of K slices together, against
         // the plan above without a split.
         if (can_split && !P.patch) {
-            int k_min = 1 << 30;  // every slice of every phase gets at least 4 K iterations
+            int k_min = 1 << 30;  // every slice of every phase gets at least 4 K iterations (2 of three products each)
             for (int p = 0; p < n_phases; ++p)
-                if (P.phases[p].tap_count > 0) k_min = std::min(k_min, P.passes * P.c_blocks * P.phases[p].tap_count);
+                if (P.phases[p].tap_count > 0) k_min = std::min(k_min, P.c_blocks * P.phases[p].tap_count);
             const double plane_us = static_cast<double>(out_pixels) * N * 4.0 / 6e6;
             auto cost_us = [&](int nt, int bn, int z) {
                 const long long tiles = m_tiles_all * nt;
                 const double rounds = static_cast<double>((tiles * z + limited(ds->sms) - 1) / limited(ds->sms));
-                return rounds * (ceil_div(k_min, z) * slice_us(bn) + 2.5) + (z > 1 ? 3.0 + (2 * z + 1) * plane_us : 0.0);
+                return rounds * (ceil_div(k_min, z) * slice_us(bn) * products + 2.5) + (z > 1 ? 3.0 + (2 * z + 1) * plane_us : 0.0);
             };
             double best_us = cost_us(P.n_tiles, P.bn, 1);
             for (int i = 0; i < 4; ++i) {
-                if (tune().bn ? i != 3 : i == 3) continue;
-                const int nt = ceil_div(N, i == 3 ? tune().bn : cand[i]);
+                if (forced ? i != 3 : i == 3) continue;
+                const int nt = ceil_div(N, cand[i]);
                 const int bn = static_cast<int>(round_up(ceil_div(N, nt), b_mn_major ? 64 : 32));
-                if (m_tiles_all * nt * 2 > limited(ds->sms)) continue;
-                const int z_max = std::min(z_cap, std::min(static_cast<int>(limited(ds->sms) / (m_tiles_all * nt)), k_min / 4));
+                if (m_tiles_all * nt * 2 > limited(ds->sms) || (bn > 128 && P.planes == 2)) continue;
+                const int z_max = std::min(z_cap, std::min(static_cast<int>(limited(ds->sms) / (m_tiles_all * nt)), k_min / (P.planes == 2 ? 2 : 4)));
                 for (int z = 2; z <= z_max; ++z) {
                     const double us = cost_us(nt, bn, z);
                     if (us < best_us) {
@@ -1076,7 +1086,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     // Pairs of CTAs (cta_group::2) for 256-wide tiles of problems large enough to fill the pairs: a
     // tile id then names two consecutive row tiles of one phase.
     // (short K loops are epilogue-bound, where pairing only halves the number of independent tiles)
-    const int k_iters_min = P.passes * P.c_blocks * std::max<int>(1, P.phases[0].tap_count);
+    const int k_iters_min = products * P.c_blocks * std::max<int>(1, P.phases[0].tap_count);
     long long tiles_single = 0;
     for (int p = 0; p < n_phases; ++p)
         tiles_single += 1ll * ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) *
@@ -1086,7 +1096,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     // the short phases of strided gathers and on few-tile problems.
     int k_iters_all = k_iters_min;
     for (int p = 0; p < n_phases; ++p)
-        if (P.phases[p].tap_count > 0) k_iters_all = std::min(k_iters_all, P.passes * P.c_blocks * P.phases[p].tap_count);
+        if (P.phases[p].tap_count > 0) k_iters_all = std::min(k_iters_all, products * P.c_blocks * P.phases[p].tap_count);
     const bool pair_width = P.bn == 256 || (tune().pair128 && P.bn == 128 && k_iters_all >= 4 && tiles_single * 4 >= 3ll * limited(ds->sms));
     P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && k_iters_min >= 4 &&
               (P.out_mode == OUT_NHWC_TMA || P.out_mode == OUT_NCHW_TMA || P.out_mode == OUT_NCHW) && limited(ds->sms) >= 2) ? 1 : 0;
@@ -1286,7 +1296,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     memset(&P, 0, sizeof(P));
     P.mode = MODE_WGRAD;
     P.kind = mi.kind;
-    P.passes = (mi.planes == 2) ? 3 : 1;
+    P.planes = mi.planes;
     P.kb = mi.kb;
     P.a_mn_major = 1;
     P.b_mn_major = 1;
@@ -1375,12 +1385,14 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         for (int width = 256; width >= 64; width /= 2) {
             const int nt = ceil_div(g.plain_c, width);
             const int bn = static_cast<int>(round_up(ceil_div(g.plain_c, nt), 64));
-            if (width < 256 && bn > width) continue;
             const bool pair = tune().pair && bn == 256 && a_grp && b_grp && sms >= 2;
+            if ((width < 256 && bn > width) || (bn > 128 && P.planes == 2 && !pair)) continue;
             const int mt = pair ? ceil_div(row_tiles, 2) : row_tiles;
-            const double block_us = slice_us(bn) * P.passes;
+            const double block_us = slice_us(bn) * (P.planes == 2 ? 3 : 1);
             for (int sp = 1; sp <= max_split; ++sp) {
                 int per_sp = ceil_div(P.kblocks_total, sp);
+                // the tensor core truncates as it accumulates: at most 4096 terms per sum of the 3xTF32 split
+                if (P.planes == 2 && per_sp * mi.kb > 4096 && sp < max_split) continue;
                 int real = ceil_div(P.kblocks_total, per_sp);  // every slice gets at least one K block
                 if (real != sp) continue;
                 long long rounds = ceil_div(mt * nt * sp, pair ? sms / 2 : sms);

@@ -74,10 +74,14 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict
         }
     }
     __syncthreads();
-    if (colsum != nullptr && threadIdx.x < 64 && c0 + threadIdx.x < C) {
+    if (colsum != nullptr) {  // four threads per channel, 16 pixels each (all lanes of a warp on different banks)
+        const int c = threadIdx.x >> 2, q = threadIdx.x & 3;
         float s = 0.f;
-        for (int p = 0; p < 64; ++p) s += tile[threadIdx.x][(p + threadIdx.x) & 63];
-        colsum[(static_cast<size_t>(n) * gridDim.x + blockIdx.x) * C + c0 + threadIdx.x] = s;
+#pragma unroll
+        for (int p = 0; p < 16; ++p) s += tile[c][4 * p + q];
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (q == 0 && c0 + c < C) colsum[(static_cast<size_t>(n) * gridDim.x + blockIdx.x) * C + c0 + c] = s;
     }
     // store: 8 threads per pixel, 8 channels each
     const int j = threadIdx.x & 7, pp = threadIdx.x >> 3;  // 8 x 32
@@ -183,36 +187,52 @@ __global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* __restrict_
     }
 }
 
-// Vectorised column sums for fp16 rows whose length is a multiple of 8: every thread owns 8
-// adjacent columns (one 16-byte load per row), a warp covers 256 columns, blockDim.y warps take
-// interleaved rows, and each block writes its partial sums to its row of the partial-sum matrix.
-__global__ void __launch_bounds__(256) colsum_rows_f16x8_kernel(const __half* __restrict__ in, float* colsum,
-                                                                size_t R, int C, int rows_per_block) {
+// Vectorised column sums for rows that are whole 16-byte vectors (8 fp16 or 4 fp32 columns each): every thread owns one
+// vector column, a warp covers 32 of them, the block's 8 warps take interleaved rows, eight loads in flight each (the pass
+// is HBM-bound; four left 16384 x 8192 at 4.9 TB/s), and each block writes its partial sums to its row of the
+// partial-sum matrix.
+__device__ __forceinline__ void add_vector(float (&acc)[8], const uint4& v, const __half*) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f = __half22float2(h[j]);
+        acc[2 * j] += f.x;
+        acc[2 * j + 1] += f.y;
+    }
+}
+__device__ __forceinline__ void add_vector(float (&acc)[4], const uint4& v, const float*) {
+    acc[0] += __uint_as_float(v.x); acc[1] += __uint_as_float(v.y); acc[2] += __uint_as_float(v.z); acc[3] += __uint_as_float(v.w);
+}
+template <typename TIn>
+__global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* __restrict__ in, float* colsum,
+                                                             size_t R, int C, int rows_per_block) {
     pdl_enter();
-    __shared__ float part[8][256];
+    constexpr int V = 16 / sizeof(TIn);
+    __shared__ float part[8][32 * V];
     const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-    const int c0 = (blockIdx.x * 32 + lane) * 8;
+    const int c0 = (blockIdx.x * 32 + lane) * V;
     size_t r0 = static_cast<size_t>(blockIdx.y) * rows_per_block;
     size_t r1 = r0 + rows_per_block < R ? r0 + rows_per_block : R;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (c0 < C) {
-#pragma unroll 4  // several 16-byte loads in flight per thread: the pass is HBM-bound
-        for (size_t r = r0 + wy; r < r1; r += 8) {
-            uint4 v = __ldg(reinterpret_cast<const uint4*>(in + r * C + c0));
-            const __half2* h = reinterpret_cast<const __half2*>(&v);
+    float acc[V];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float2 f = __half22float2(h[j]);
-                acc[2 * j] += f.x;
-                acc[2 * j + 1] += f.y;
-            }
+    for (int j = 0; j < V; ++j) acc[j] = 0.f;
+    if (c0 < C) {
+        const TIn* p = in + c0;
+        size_t r = r0 + wy;
+        for (; r + 56 < r1; r += 64) {
+            uint4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p + (r + 8 * i) * C));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) add_vector(acc, v[i], p);
         }
+        for (; r < r1; r += 8) add_vector(acc, __ldg(reinterpret_cast<const uint4*>(p + r * C)), p);
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) part[wy][lane * 8 + j] = acc[j];
+    for (int j = 0; j < V; ++j) part[wy][lane * V + j] = acc[j];
     __syncthreads();
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    if (c < C) {
+    const int c = blockIdx.x * 32 * V + threadIdx.x;
+    if (threadIdx.x < 32 * V && c < C) {
         float sum = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) sum += part[w][threadIdx.x];
@@ -522,29 +542,27 @@ __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __re
 }
 
 // Second stage of the column sums: adds rows [blockIdx.y * rows_per_block, ...) of the [P][stride]
-// partial-sum matrix in a fixed order (eight interleaved running sums, then those eight in order) and
-// writes row blockIdx.y of `out` ([segments][out_stride]).  Launched again on its own output while more
-// than one segment is left.  blockDim = (32, 8).
-__global__ void __launch_bounds__(256) colsum_finish_kernel(const float* __restrict__ partial, int P, int stride, int C,
-                                                            float* __restrict__ out, int out_stride, int rows_per_block) {
+// partial-sum matrix in a fixed order (128 interleaved running sums, then those in a tree) and writes row blockIdx.y of
+// `out` ([segments][out_stride]).  Launched again on its own output while more than one segment is left.
+// blockDim = (8, 128): few channels and a chain of load latencies, so many threads take few rows each.
+__global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __restrict__ partial, int P, int stride, int C,
+                                                             float* __restrict__ out, int out_stride, int rows_per_block) {
     pdl_enter();
-    __shared__ float part[8][33];
-    const int c = blockIdx.x * 32 + threadIdx.x;
+    __shared__ float part[128][9];
+    const int c = blockIdx.x * 8 + threadIdx.x;
     const int p0 = blockIdx.y * rows_per_block;
     const int p1 = min(P, p0 + rows_per_block);
     float s = 0.f;
     if (c < C) {
-#pragma unroll 4
-        for (int p = p0 + threadIdx.y; p < p1; p += 8) s += __ldg(partial + static_cast<size_t>(p) * stride + c);
+#pragma unroll 8
+        for (int p = p0 + threadIdx.y; p < p1; p += 128) s += __ldg(partial + static_cast<size_t>(p) * stride + c);
     }
     part[threadIdx.y][threadIdx.x] = s;
-    __syncthreads();
-    if (threadIdx.y == 0 && c < C) {
-        float t = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t += part[k][threadIdx.x];
-        out[static_cast<size_t>(blockIdx.y) * out_stride + c] = t;
+    for (int half = 64; half > 0; half /= 2) {
+        __syncthreads();
+        if (threadIdx.y < half) part[threadIdx.y][threadIdx.x] += part[threadIdx.y + half][threadIdx.x];
     }
+    if (threadIdx.y == 0 && c < C) out[static_cast<size_t>(blockIdx.y) * out_stride + c] = part[0][threadIdx.x];
 }
 
 // Second stage of a split-K weight gradient: adds the K slices' planes in slice order (bitwise

@@ -82,13 +82,16 @@ struct KParams {
     unsigned long long mul_nt;  // 2^40 / n_tiles + 1
     int fastdiv;         // 1: tile ids and divisors are small enough for the multiply-and-shift division to be exact
     int bn;              // UMMA N of one tile
+    int tbufs;           // accumulator buffers in TMEM: 2, or 1 where planes * bn takes more than half of it (256-column
+                         // pair tiles of the 3xTF32 split: their K loops are long, and what they save in operand feed is
+                         // more than the epilogue they do not overlap)
     int stages;
     int cm_bw_log2, cm_bh_log2;  // OUT_NCHW_TMA: pixel sub-box (w, h) of one epilogue warp's 32 rows
     int epi_warps;       // 4, or 8 on the TMA-store instances when the epilogue is the critical path
     int pair;            // 1: launched as clusters of two CTAs sharing 256x256 tiles (cta_group::2)
     int stg_bufs;        // staging buffers per epilogue warp (4 KB each): 2 when shared memory allows, else 1
-    int ka;              // K atoms (128-byte-wide operand slices) per stage; narrow tiles take 2 to amortise the
-                         // per-stage barrier round trip over 8 MMAs
+    int ka;              // K atoms (128-byte-wide operand slices, times planes) per stage; narrow tiles take 2 to amortise
+                         // the per-stage barrier round trip over 8 MMAs
     int a_mn_major, b_mn_major;
     int b_batched;       // 1: every image (batch entry) has a B of its own, the outermost dimension of tmB (batched matmul;
                          // tiles of one image each, no pairs, no patch walk)
@@ -132,7 +135,11 @@ struct KParams {
     int ring_bytes;      // bytes of the operand ring(s) in front of the staging buffers
     int a_ring_off;      // patch walk: offset of the patch buffers within the ring region
     int kind;            // KIND_F16 / KIND_TF32
-    int passes;          // 1, or 3 for the 3xTF32 split (hi*lo, lo*hi, hi*hi in that order)
+    int planes;          // 1, or 2 for the 3xTF32 split: a stage then holds the hi and the lo atom of both operands (ka counts
+                         // atoms), and its three products are issued together: hi*lo and lo*hi into an accumulator of
+                         // their own, hi*hi into the main one.  The epilogue adds the two in fp32.  Each plane is loaded
+                         // once (three passes over K loaded the hi planes twice), a barrier round trip covers 12 MMAs, and
+                         // the small cross terms are never truncated against the large accumulator.
     int kb;              // elements per 128-byte row (64 fp16, 32 tf32)
     int c_blocks;        // channel blocks of kb per tap (fprop) / per patch tensor (wgrad)
     int wb_log2, hb_log2, nb_log2;  // fprop: M-tile box; wgrad: K-block pixel box
@@ -280,7 +287,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     // two accumulators; the epilogue reads 32 columns at a time, so a 16-column tile still needs 16 + 32
-    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : 2 * P.bn;
+    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : P.tbufs * P.bn * P.planes;
     const uint32_t tmem_cols = (tmem_need <= 32) ? 32 : (tmem_need <= 64) ? 64 : (tmem_need <= 128) ? 128
                                : (tmem_need <= 256) ? 256 : 512;
 
@@ -302,7 +309,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         fence_mbar_init();
         tma_prefetch_desc(&P.tmA[0]);
         tma_prefetch_desc(&P.tmB[0]);
-        if (P.passes > 1) {
+        if (P.planes > 1) {
             tma_prefetch_desc(&P.tmA[1]);
             tma_prefetch_desc(&P.tmB[1]);
         }
@@ -323,6 +330,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     const uint32_t tmem_base = *tmem_slot;
     pdl_enter();  // everything above overlaps the tail of the kernel in front
 
+    const int ks = P.ka / P.planes;    // K slices per stage
     const int box_bytes = P.kb * 128;  // one MN-major box: kb k-rows of 128 bytes
     const int wb = 1 << P.wb_log2, hb = 1 << P.hb_log2;
 
@@ -350,8 +358,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             const Tap* tp = &P.taps[P.phases[p].tap_begin];
             const int nt = P.phases[p].tap_count;
             const int tb0 = P.phases[p].tap_begin;
-            const int buf = titer & 1;
-            const uint32_t tpar = (titer >> 1) & 1;
+            const int buf = P.tbufs == 2 ? (titer & 1) : 0;
+            const uint32_t tpar = P.tbufs == 2 ? (titer >> 1) & 1 : titer & 1;
             if (!mbar_wait(smem_u32(&tempty_bar[buf]), tpar ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) return;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + buf * P.bn;
@@ -397,12 +405,13 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     if (warp == 0 || warp == 6) {
         const bool do_a = (warp == 0), do_b = (warp == 6);
         // Issuing one TMA keeps its thread busy for ~300 clocks, more than the MMAs of a narrow K atom last.
-        // The atoms of a stage are therefore issued by one lane each, in the same instruction (the patch
-        // walk, with one box per tile, is driven by lane 0 alone).
+        // The atoms of a stage are therefore issued by one lane each, in the same instruction (patches, one box per
+        // tile and plane, by lane 0 alone).
         // Weight-gradient operands that cannot be fetched as one box per K block get a lane per box.
         const int boxes_per_atom = (kMode != MODE_WGRAD || kPair) ? 1
                                    : do_a ? (P.a_grouped ? 1 : kTileM / P.kb) : (P.b_grouped ? 1 : P.bn / P.kb);
-        const int issue_lanes = (P.patch || P.wpatch) ? 1 : P.ka * boxes_per_atom;
+        const int issue_lanes = P.wpatch || (kMode == MODE_WGRAD && kPair) ? 1
+                                : P.patch ? ((do_a || P.b_resident) ? 1 : P.ka) : P.ka * boxes_per_atom;
         const uint32_t issue_mask = (1u << issue_lanes) - 1u;
         if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident && do_b) {
             // Resident weights: every slice once, for the whole launch (one column tile, one pass plane, K-major
@@ -447,7 +456,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         tma_load_2d(sb + j * box_bytes, tb, fb, ntile * P.bn + j * P.kb, tap.wk + cb * P.kb);
                 }
             };
-            if (kMode == MODE_FPROP && !kPair && P.patch) {  // (issue_lanes == 1 here)
+            if (kMode == MODE_FPROP && !kPair && P.patch) {
                 if (do_a) {
                     const uint32_t a_base = smem_u32(smem + P.a_ring_off);
                     const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * 128u;
@@ -461,16 +470,15 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         decode_fprop_tile<false>(P, pt, tile - pt.tile_begin, 0u, nt_unused, tw, th, tn);
                         const int w0 = (tw << P.wb_log2) * P.a_stride_w + pt.org_w;
                         const int h0 = (th << P.hb_log2) * P.a_stride_h + pt.org_h;
-                        for (int pass = 0; ok && pass < P.passes; ++pass) {
-                            const CUtensorMap* ta = &P.tmA[(P.passes == 3 && pass == 1) ? 1 : 0];
-                            for (int cb = 0; cb < P.c_blocks; ++cb) {
+                        for (int cb = 0; ok && cb < P.c_blocks; ++cb) {
+                            for (int pl = 0; pl < P.planes; ++pl) {
                                 if (!mbar_wait(smem_u32(&aempty_bar[abuf]), apar ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
                                     ok = false;
                                     break;
                                 }
                                 const uint32_t fb = smem_u32(&afull_bar[abuf]);
                                 mbar_arrive_expect_tx(fb, patch_tx);
-                                tma_load_4d(a_base + abuf * P.patch_bytes, ta, fb, cb * P.kb, w0, h0, tn);
+                                tma_load_4d(a_base + abuf * P.patch_bytes, &P.tmA[pl], fb, cb * P.kb, w0, h0, tn);
                                 ++issued;
                                 if (++abuf == P.a_stages) {
                                     abuf = 0;
@@ -510,33 +518,33 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         }
                     }
                 } else {
-                    // B streams through the ring, P.ka tap slices per stage
+                    // B streams through the ring, ks tap slices (of every plane) per stage
                     int p = 0;
                     for (int tile = tile_first; ok && tile < P.num_tiles; tile += tile_step) {
                         while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
                         const Phase& pt = P.phases[p];
                         const int ntile = (tile - pt.tile_begin) % P.n_tiles;
-                        for (int pass = 0; ok && pass < P.passes; ++pass) {
-                            const CUtensorMap* tb = &P.tmB[(P.passes == 3 && pass == 0) ? 1 : 0];
-                            for (int cb = 0; ok && cb < P.c_blocks; ++cb)
-                                for (int t = 0; t < pt.tap_count; t += P.ka) {
-                                    if (!mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
-                                        ok = false;
-                                        break;
-                                    }
-                                    const int n = min(P.ka, pt.tap_count - t);
-                                    const uint32_t fb = smem_u32(&full_bar[stage]);
-                                    mbar_arrive_expect_tx(fb, n * stage_b_bytes);
-                                    for (int j = 0; j < n; ++j)
-                                        load_b(smem_u32(smem) + (stage * P.ka + j) * stage_b_bytes, tb, fb,
-                                               P.taps[pt.tap_begin + t + j], cb, ntile, 0);
-                                    ++issued;
-                                    if (++stage == P.stages) {
-                                        stage = 0;
-                                        parity ^= 1;
-                                    }
+                        for (int cb = 0; ok && cb < P.c_blocks; ++cb)
+                            for (int t = 0; t < pt.tap_count; t += ks) {
+                                // (one lane per atom: a second load from one thread costs what the stage's MMAs last)
+                                if (!__all_sync(issue_mask, mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
+                                                                      ERR_WAIT_EMPTY))) {
+                                    ok = false;
+                                    break;
                                 }
-                        }
+                                const int n = min(ks, pt.tap_count - t) * P.planes;
+                                const uint32_t fb = smem_u32(&full_bar[stage]);
+                                if (lane == 0) mbar_arrive_expect_tx(fb, n * stage_b_bytes);
+                                __syncwarp(issue_mask);
+                                if (lane < n)
+                                    load_b(smem_u32(smem) + (stage * P.ka + lane) * stage_b_bytes, &P.tmB[P.planes == 2 ? (lane & 1) : 0], fb,
+                                           P.taps[pt.tap_begin + t + (P.planes == 2 ? lane >> 1 : lane)], cb, ntile, 0);
+                                ++issued;
+                                if (++stage == P.stages) {
+                                    stage = 0;
+                                    parity ^= 1;
+                                }
+                            }
                     }
                 }
             } else
@@ -556,28 +564,27 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     int w0 = (tw << P.wb_log2) * P.a_stride_w;
                     int h0 = (th << P.hb_log2) * P.a_stride_h;
                     int n0 = tn << P.nb_log2;
-                    int k_iters = P.passes * ph.tap_count * P.c_blocks;
+                    int k_iters = ph.tap_count * P.c_blocks;
                     int k_first = 0;
                     if (P.fsplit > 1) {  // this slice's share of the K iterations
                         const int per = (k_iters + P.fsplit - 1) / P.fsplit;
                         k_first = min(kz * per, k_iters);
                         k_iters = min(k_first + per, k_iters) - k_first;
                     }
-                    // this lane's position in the K loop, (pass, tap, channel block) of iteration it + lane, kept
-                    // by counting: a division per stage is time the 256-wide tiles' producer does not have
-                    int pass = 0, t = 0, cb = 0;
+                    // this lane's atom of a stage: plane, and its position in the K loop, (tap, channel block) of iteration
+                    // it + lane / planes, kept by counting: a division per stage is time the 256-wide tiles' producer does
+                    // not have
+                    const int plane = P.planes == 2 ? (lane & 1) : 0;
+                    int t = 0, cb = 0;
                     auto advance = [&](int steps) {
                         cb += steps;
                         while (cb >= P.c_blocks) {
                             cb -= P.c_blocks;
-                            if (++t == ph.tap_count) {
-                                t = 0;
-                                ++pass;
-                            }
+                            ++t;
                         }
                     };
-                    advance(k_first + lane);
-                    for (int it = 0; it < k_iters; it += P.ka) {  // one stage per iteration
+                    advance(k_first + (P.planes == 2 ? lane >> 1 : lane));
+                    for (int it = 0; it < k_iters; it += ks) {  // one stage per iteration
                         // in a pair every load signals the LEADER's barrier, which expects both members' bytes
                         uint32_t fb = smem_u32(&full_bar[stage]);
                         if (kPair) fb = map_to_cta(fb, 0);
@@ -587,19 +594,16 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             ok = false;
                             break;
                         }
-                        const int n_in_stage = min(P.ka, k_iters - it);
+                        const int n_in_stage = min(P.ka, (k_iters - it) * P.planes);
                         if (lane == 0) {
                             if (!kPair) mbar_arrive_expect_tx(fb, n_in_stage * tx_bytes);
                             else if (leader) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * n_in_stage * tx_bytes);
                         }
                         __syncwarp(issue_mask);
-                        if (lane < n_in_stage) {  // this lane's atom: K iteration it + lane = (pass, tap, channel block)
+                        if (lane < n_in_stage) {
                             const Tap& tap = P.taps[ph.tap_begin + t];
-                            // 3xTF32 order: hi*lo, lo*hi, then hi*hi -- the small cross terms go in
-                            // while the accumulator is small, so the tensor core's truncating
-                            // accumulation costs them nothing
-                            const CUtensorMap* ta = &P.tmA[(P.passes == 3 && pass == 1) ? 1 : 0];
-                            const CUtensorMap* tb = &P.tmB[(P.passes == 3 && pass == 0) ? 1 : 0];
+                            const CUtensorMap* ta = &P.tmA[plane];
+                            const CUtensorMap* tb = &P.tmB[plane];
                             const uint32_t sa = smem_u32(smem + stage * stage_bytes) + lane * kStageABytes;
                             const uint32_t sb = smem_u32(smem + stage * stage_bytes) + b_off + lane * stage_b_bytes;
                             if (kPair) {
@@ -615,7 +619,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                                 load_b(sb, tb, fb, tap, cb, ntile, n0);
                             }
                         }
-                        advance(P.ka);
+                        advance(ks);
                         ++issued;
                         if (++stage == P.stages) {
                             stage = 0;
@@ -670,105 +674,60 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     int kb_begin = z * per;
                     int kb_end = min(kb_begin + per, P.kblocks_total);
                     int g_per_tile = kTileM / P.kb;
-                    int na = g_per_tile, nb = P.bn / P.kb;
                     if (kPair) {
-                    // one K block and one box per stage: the single issuing lane has ~500 clocks per
-                    // stage, so its loop carries nothing but counters
-                    int left = P.passes * max(kb_end - kb_begin, 0);  // K iterations still to load for this tile
-                    int slot = 0, n_in_stage = 0;
-                    for (int pass = 0; ok && pass < P.passes; ++pass) {
-                        const CUtensorMap* ta = &P.tmA[(P.passes == 3 && pass == 1) ? 1 : 0];
-                        const CUtensorMap* tb = &P.tmB[(P.passes == 3 && pass == 0) ? 1 : 0];
-                        int tw = kb_begin % P.ktiles_w;
-                        int th = (kb_begin / P.ktiles_w) % P.ktiles_h;
-                        int tn = kb_begin / (P.ktiles_w * P.ktiles_h);
-                        // groups of this M tile: with a_grouped they share one tap
-                        const int g0 = min(mt * g_per_tile, P.groups_total - 1);
-                        const int t0 = g0 / P.c_blocks;
-                        const int cib0 = g0 - t0 * P.c_blocks;
-                        for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
-                            int w0 = tw << P.wb_log2, h0 = th << P.hb_log2, n0 = tn << P.nb_log2;
-                            uint32_t fb = smem_u32(&full_bar[stage]);
-                            if (kPair) fb = map_to_cta(fb, 0);
-                            if (slot == 0) {
-                                if (!mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag,
-                                               P.err, ERR_WAIT_EMPTY)) {
-                                    ok = false;
-                                    break;
-                                }
-                                n_in_stage = min(P.ka, left);
-                                if (!kPair) mbar_arrive_expect_tx(fb, n_in_stage * tx_bytes);
-                                else if (leader) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * n_in_stage * tx_bytes);
-                            }
-                            --left;
-                            uint32_t sa = smem_u32(smem + stage * stage_bytes) + slot * kStageABytes;
-                            uint32_t sb = smem_u32(smem + stage * stage_bytes) + b_off + slot * stage_b_bytes;
-                            if (kPair) {  // pairs are only planned for grouped operands
-                                const Tap& tap = P.taps[t0];
-                                if (do_a)
-                                    tma_load_5d_pair(sa, ta, fb, 0, w0 * P.a_stride_w + tap.dw, h0 * P.a_stride_h + tap.dh, n0,
-                                                     cib0);
-                                if (do_b)
-                                    tma_load_5d_pair(sb, tb, fb, 0, w0, h0, n0,
-                                                     (ntile * P.bn) / P.kb + static_cast<int>(cta_rank) * (P.bn / 2 / P.kb));
-                            } else
-                            if (!do_a) {
-                            } else if (P.a_grouped) {
-                                const Tap& tap = P.taps[t0];
-                                tma_load_5d(sa, ta, fb, 0, w0 * P.a_stride_w + tap.dw, h0 * P.a_stride_h + tap.dh, n0,
-                                            cib0);
-                            } else {
-                                for (int g = 0; g < na; ++g) {
-                                    int gi = min(mt * g_per_tile + g, P.groups_total - 1);
-                                    int t = gi / P.c_blocks;
-                                    int cib = gi - t * P.c_blocks;
-                                    const Tap& tap = P.taps[t];
-                                    tma_load_4d(sa + g * box_bytes, ta, fb, cib * P.kb,
-                                                w0 * P.a_stride_w + tap.dw, h0 * P.a_stride_h + tap.dh, n0);
-                                }
-                            }
-                            if (kPair || !do_b) {
-                            } else if (P.b_grouped) {
-                                tma_load_5d(sb, tb, fb, 0, w0, h0, n0, (ntile * P.bn) / P.kb);
-                            } else {
-                                for (int j = 0; j < nb; ++j)
-                                    tma_load_4d(sb + j * box_bytes, tb, fb, ntile * P.bn + j * P.kb, w0,
-                                                h0, n0);
-                            }
-                            if (++slot == n_in_stage) {
-                                slot = 0;
-                                ++issued;
-                                if (++stage == P.stages) {
-                                    stage = 0;
-                                    parity ^= 1;
-                                }
-                            }
-                            if (++tw == P.ktiles_w) {
-                                tw = 0;
-                                if (++th == P.ktiles_h) {
-                                    th = 0;
-                                    ++tn;
-                                }
+                    // one K block per stage, one box per plane: the single issuing lane has ~500 clocks per stage, so its
+                    // loop carries nothing but counters
+                    int tw = kb_begin % P.ktiles_w;
+                    int th = (kb_begin / P.ktiles_w) % P.ktiles_h;
+                    int tn = kb_begin / (P.ktiles_w * P.ktiles_h);
+                    // groups of this M tile: with a_grouped they share one tap
+                    const int g0 = min(mt * g_per_tile, P.groups_total - 1);
+                    const int t0 = g0 / P.c_blocks;
+                    const int cib0 = g0 - t0 * P.c_blocks;
+                    const Tap& tap = P.taps[t0];
+                    for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
+                        const int w0 = tw << P.wb_log2, h0 = th << P.hb_log2, n0 = tn << P.nb_log2;
+                        const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
+                        if (!mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
+                            ok = false;
+                            break;
+                        }
+                        if (leader) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * P.planes * tx_bytes);
+                        const uint32_t sa = smem_u32(smem + stage * stage_bytes);
+                        for (int pl = 0; pl < P.planes; ++pl)
+                        if (do_a)
+                            tma_load_5d_pair(sa + pl * kStageABytes, &P.tmA[pl], fb, 0, w0 * P.a_stride_w + tap.dw, h0 * P.a_stride_h + tap.dh, n0, cib0);
+                        else
+                            tma_load_5d_pair(sa + b_off + pl * stage_b_bytes, &P.tmB[pl], fb, 0, w0, h0, n0,
+                                             (ntile * P.bn) / P.kb + static_cast<int>(cta_rank) * (P.bn / 2 / P.kb));
+                        ++issued;
+                        if (++stage == P.stages) {
+                            stage = 0;
+                            parity ^= 1;
+                        }
+                        if (++tw == P.ktiles_w) {
+                            tw = 0;
+                            if (++th == P.ktiles_h) {
+                                th = 0;
+                                ++tn;
                             }
                         }
                     }
                     } else {
                     const int nkb = max(kb_end - kb_begin, 0);
-                    const int k_total = P.passes * nkb;  // K iterations of this tile: (pass, K block)
                     // groups of this M tile: with a_grouped they share one tap
                     const int g0 = min(mt * g_per_tile, P.groups_total - 1);
                     const int t0 = g0 / P.c_blocks;
                     const int cib0 = g0 - t0 * P.c_blocks;
-                    // this lane's K iteration (it + lane) as (pass, K block -> pixel box), kept by counting
+                    // this lane's atom of a stage (slice and plane) and box; its K iteration as a pixel box, kept by counting
                     const int tw0 = kb_begin % P.ktiles_w;
                     const int th0 = (kb_begin / P.ktiles_w) % P.ktiles_h;
                     const int tn0 = kb_begin / (P.ktiles_w * P.ktiles_h);
-                    int pass = 0, rel = 0, tw = tw0, th = th0, tn = tn0;
+                    int rel = 0, tw = tw0, th = th0, tn = tn0;
                     auto advance = [&](int steps) {
                         for (int i = 0; i < steps; ++i) {
                             if (++rel >= nkb) {
                                 rel = 0;
-                                ++pass;
                                 tw = tw0;
                                 th = th0;
                                 tn = tn0;
@@ -782,8 +741,9 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         }
                     };
                     const int my_atom = lane / boxes_per_atom, my_box = lane - my_atom * boxes_per_atom;
-                    if (nkb > 0) advance(my_atom);
-                    for (int it = 0; it < k_total; it += P.ka) {  // one stage per iteration
+                    const int plane = P.planes == 2 ? (my_atom & 1) : 0;
+                    if (nkb > 0) advance(P.planes == 2 ? my_atom >> 1 : my_atom);
+                    for (int it = 0; it < nkb; it += ks) {  // one stage per iteration
                         uint32_t fb = smem_u32(&full_bar[stage]);
                         if (kPair) fb = map_to_cta(fb, 0);
                         if (!__all_sync(issue_mask, mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
@@ -791,15 +751,15 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             ok = false;
                             break;
                         }
-                        const int n_in_stage = min(P.ka, k_total - it);
+                        const int n_in_stage = min(P.ka, (nkb - it) * P.planes);
                         if (lane == 0) {
                             if (!kPair) mbar_arrive_expect_tx(fb, n_in_stage * tx_bytes);
                             else if (leader) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * n_in_stage * tx_bytes);
                         }
                         __syncwarp(issue_mask);
                         if (my_atom < n_in_stage) {
-                            const CUtensorMap* ta = &P.tmA[(P.passes == 3 && pass == 1) ? 1 : 0];
-                            const CUtensorMap* tb = &P.tmB[(P.passes == 3 && pass == 0) ? 1 : 0];
+                            const CUtensorMap* ta = &P.tmA[plane];
+                            const CUtensorMap* tb = &P.tmB[plane];
                             const int w0 = tw << P.wb_log2, h0 = th << P.hb_log2, n0 = tn << P.nb_log2;
                             const uint32_t sa = smem_u32(smem + stage * stage_bytes) + my_atom * kStageABytes;
                             const uint32_t sb = smem_u32(smem + stage * stage_bytes) + b_off + my_atom * stage_b_bytes;
@@ -831,7 +791,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                                 tma_load_4d(sb + my_box * box_bytes, tb, fb, ntile * P.bn + my_box * P.kb, w0, h0, n0);
                             }
                         }
-                        advance(P.ka);
+                        advance(ks);
                         ++issued;
                         if (++stage == P.stages) {
                             stage = 0;
@@ -906,7 +866,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             if (kMode == MODE_FPROP) {
                 int p = 0;
                 while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
-                k_iters = P.passes * P.phases[p].tap_count * P.c_blocks;
+                k_iters = P.phases[p].tap_count * P.c_blocks;
                 if (P.fsplit > 1) {
                     const int per = (k_iters + P.fsplit - 1) / P.fsplit;
                     const int k_first = min(kz * per, k_iters);
@@ -919,10 +879,10 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
                 int kb_begin = z * per;
                 int kb_end = min(kb_begin + per, P.kblocks_total);
-                k_iters = P.passes * max(kb_end - kb_begin, 0);
+                k_iters = max(kb_end - kb_begin, 0);
             }
-            const int buf = titer & 1;
-            const uint32_t tpar = (titer >> 1) & 1;
+            const int buf = P.tbufs == 2 ? (titer & 1) : 0;
+            const uint32_t tpar = P.tbufs == 2 ? (titer >> 1) & 1 : titer & 1;
             if (kMode == MODE_WGRAD && !kPair && P.wpatch) {
                 // all row tiles at once, accumulator i in columns [i * bn, (i + 1) * bn); no second TMEM buffer, so
                 // the epilogue of the previous tile (if this CTA has one) must be over
@@ -989,66 +949,92 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 break;
             }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + buf * P.bn;
+            const uint32_t d_tmem = tmem_base + buf * P.bn * P.planes;  // the split's cross products: bn columns further on
             uint32_t acc = 0;
+            // one K slice of the 3xTF32 split: hi*lo and lo*hi into the cross accumulator, hi*hi into the main one
+            auto issue_split = [&](uint64_t ah, uint64_t al, uint64_t bh, uint64_t bl, uint32_t aa, uint32_t ab) {
+                const uint32_t d_cross = d_tmem + P.bn;
+                auto product = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t first) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (kPair) umma_tf32_pair(d, a, b, idesc, first);
+                        else umma_tf32(d, a, b, idesc, first);
+                        first = 1u;
+                        a += aa;
+                        b += ab;
+                    }
+                };
+                product(d_cross, ah, bl, acc);
+                product(d_cross, al, bh, 1u);
+                product(d_tmem, ah, bh, acc);
+            };
             if (kMode == MODE_FPROP && !kPair && P.patch) {
                 int pp = 0;
                 while (pp + 1 < P.n_phases && tile >= P.phases[pp + 1].tile_begin) ++pp;
                 const Phase& ph = P.phases[pp];
                 const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h) * 128u;  // 8-row groups: one output row = a_stride_h patch rows apart
                 const uint64_t bdesc_ring0 = make_smem_desc(smem_u32(smem), lbo_b, b32 ? 512 : 1024, b32 ? 1 : 2);  // B ring starts the region
-                for (int pass = 0; ok && pass < P.passes; ++pass)
-                    for (int cb = 0; ok && cb < P.c_blocks; ++cb) {
+                for (int cb = 0; ok && cb < P.c_blocks; ++cb) {
+                    uint64_t adesc[2];
+                    int used[2];
+                    for (int pl = 0; pl < P.planes; ++pl) {
                         if (!mbar_wait(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) {
                             ok = false;
                             break;
                         }
-                        tc_fence_after();
-                        const uint32_t patch_addr = smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes;
-                        const uint64_t adesc0 = make_smem_desc(patch_addr, 16, sbo_a, 2);
-                        for (int t = 0; t < ph.tap_count; t += P.ka) {
-                            if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
-                                ok = false;
-                                break;
-                            }
-                            tc_fence_after();
-                            const int n = min(P.ka, ph.tap_count - t);
-                            if (elect_one()) {
-                                uint64_t bdesc = bdesc_ring0 + static_cast<uint64_t>(stage * P.ka * b_atom_step);
-                                for (int j = 0; j < n; ++j) {
-                                    const uint64_t adesc = adesc0 + static_cast<uint32_t>(P.taps[ph.tap_begin + t + j].aoff);
-                                    if (f16) {
-                                        umma_f16(d_tmem, adesc, bdesc, idesc, acc);
-                                        umma_f16(d_tmem, adesc + 2, bdesc + adv_b, idesc, 1u);
-                                        umma_f16(d_tmem, adesc + 4, bdesc + 2 * adv_b, idesc, 1u);
-                                        umma_f16(d_tmem, adesc + 6, bdesc + 3 * adv_b, idesc, 1u);
-                                    } else {
-                                        umma_tf32(d_tmem, adesc, bdesc, idesc, acc);
-                                        umma_tf32(d_tmem, adesc + 2, bdesc + adv_b, idesc, 1u);
-                                        umma_tf32(d_tmem, adesc + 4, bdesc + 2 * adv_b, idesc, 1u);
-                                        umma_tf32(d_tmem, adesc + 6, bdesc + 3 * adv_b, idesc, 1u);
-                                    }
-                                    acc = 1u;
-                                    bdesc += b_atom_step;
-                                }
-                                umma_commit(smem_u32(&empty_bar[stage]));
-                            }
-                            acc = 1u;
-                            if (++stage == P.stages) {
-                                stage = 0;
-                                parity ^= 1;
-                            }
-                        }
-                        if (!ok) break;
-                        if (elect_one()) umma_commit(smem_u32(&aempty_bar[pstage]));
+                        adesc[pl] = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, 2);
+                        used[pl] = pstage;
                         if (++pstage == P.a_stages) {
                             pstage = 0;
                             pparity ^= 1;
                         }
                     }
+                    if (!ok) break;
+                    tc_fence_after();
+                    for (int t = 0; t < ph.tap_count; t += ks) {
+                        if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const int n = min(ks, ph.tap_count - t);
+                        if (elect_one()) {
+                            uint64_t bdesc = bdesc_ring0 + static_cast<uint64_t>(stage * P.ka * b_atom_step);
+                            if (P.planes == 2) {
+                                const uint32_t off = static_cast<uint32_t>(P.taps[ph.tap_begin + t].aoff);
+                                issue_split(adesc[0] + off, adesc[1] + off, bdesc, bdesc + b_atom_step, 2, adv_b);
+                            } else
+                            for (int j = 0; j < n; ++j) {
+                                const uint64_t ad = adesc[0] + static_cast<uint32_t>(P.taps[ph.tap_begin + t + j].aoff);
+                                if (f16) {
+                                    umma_f16(d_tmem, ad, bdesc, idesc, acc);
+                                    umma_f16(d_tmem, ad + 2, bdesc + adv_b, idesc, 1u);
+                                    umma_f16(d_tmem, ad + 4, bdesc + 2 * adv_b, idesc, 1u);
+                                    umma_f16(d_tmem, ad + 6, bdesc + 3 * adv_b, idesc, 1u);
+                                } else {
+                                    umma_tf32(d_tmem, ad, bdesc, idesc, acc);
+                                    umma_tf32(d_tmem, ad + 2, bdesc + adv_b, idesc, 1u);
+                                    umma_tf32(d_tmem, ad + 4, bdesc + 2 * adv_b, idesc, 1u);
+                                    umma_tf32(d_tmem, ad + 6, bdesc + 3 * adv_b, idesc, 1u);
+                                }
+                                acc = 1u;
+                                bdesc += b_atom_step;
+                            }
+                            umma_commit(smem_u32(&empty_bar[stage]));
+                        }
+                        acc = 1u;
+                        if (++stage == P.stages) {
+                            stage = 0;
+                            parity ^= 1;
+                        }
+                    }
+                    if (!ok) break;
+                    if (elect_one())
+                        for (int pl = 0; pl < P.planes; ++pl) umma_commit(smem_u32(&aempty_bar[used[pl]]));
+                }
             } else
-            for (int it = 0; it < k_iters; it += P.ka) {
-                const int n_atoms = min(P.ka, k_iters - it);
+            for (int it = 0; it < k_iters; it += ks) {
+                const int n_atoms = min(ks, k_iters - it);
                 if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
                     ok = false;
                     break;
@@ -1058,6 +1044,9 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     uint64_t adesc = adesc0 + static_cast<uint64_t>(stage * stage_step);
                     uint64_t bdesc = bdesc0 + static_cast<uint64_t>(stage * stage_step);
                     uint32_t first = acc;
+                    if (P.planes == 2)  // (one slice per stage)
+                        issue_split(adesc, adesc + a_atom_step, bdesc, bdesc + b_atom_step, adv_a, adv_b);
+                    else
                     for (int a = 0; a < n_atoms; ++a) {
                         if (kPair) {
                             if (f16) {
@@ -1237,8 +1226,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[0]));
                 continue;
             }
-            const int buf = titer & 1;
-            const uint32_t tpar = (titer >> 1) & 1;
+            const int buf = P.tbufs == 2 ? (titer & 1) : 0;
+            const uint32_t tpar = P.tbufs == 2 ? (titer >> 1) & 1 : titer & 1;
             // tile decode
             int ntile, k_iters;
             bool row_valid;
@@ -1264,7 +1253,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 int oh = ph.ph + P.out_stride_h * ih;
                 k_iters = ph.tap_count;
                 if (P.fsplit > 1) {  // K iterations of this slice (0: nothing to add)
-                    const int full = P.passes * ph.tap_count * P.c_blocks;
+                    const int full = ph.tap_count * P.c_blocks;
                     const int per = (full + P.fsplit - 1) / P.fsplit;
                     const int k_first = min(kz * per, full);
                     k_iters = min(k_first + per, full) - k_first;
@@ -1355,7 +1344,16 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 break;
             }
             tc_fence_after();
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn;
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * P.planes;
+            const uint32_t cross = P.planes == 2 ? P.bn : 0;  // the split's second accumulator, this many columns further on
+            // r += columns [c, c + 32) of the second accumulator
+            auto add_cross = [&](uint32_t c, uint32_t (&r)[32]) {
+                uint32_t x[32];
+                tmem_ld_32x32(t_row + cross + c, x);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
+            };
             const int col_base = ntile * P.bn;
             if (kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode)) {
                 // Row-major output through TMA: each warp converts 128-byte row pieces of its 32 rows into a
@@ -1395,6 +1393,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (live && c_begin < c_end && col_base + c_begin < P.c_out) {
                     tmem_ld_32x32(t_row + c_begin, r0);
                     if (cpi == 64) tmem_ld_32x32(t_row + c_begin + 32, r1);
+                    else if (cross) tmem_ld_32x32(t_row + cross + c_begin, r1);
                     tmem_ld_wait();
                 }
                 for (int c0 = c_begin; c0 < c_end; c0 += cpi) {
@@ -1403,6 +1402,15 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     const int cn = c0 + cpi;
                     const bool more = live && cn < c_end && col_base + cn < P.c_out;
                     const uint32_t buf_addr = stg0 + ((P.stg_bufs == 2) ? (store_seq & 1) * kStagingBufBytes : 0);
+                    if (cross && live) {
+                        if (cpi == 64) {
+                            add_cross(c0, r0);
+                            add_cross(c0 + 32, r1);
+                        } else {  // (fetched along with r0)
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) r0[j] = __float_as_uint(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+                        }
+                    }
                     // the store that last read this buffer must be done reading it
                     if (lane == 0) {
                         if (P.stg_bufs == 2) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
@@ -1469,6 +1477,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     if (more) {  // registers are free again: start the next TMEM load now
                         tmem_ld_32x32(t_row + cn, r0);
                         if (cpi == 64) tmem_ld_32x32(t_row + cn + 32, r1);
+                        else if (cross) tmem_ld_32x32(t_row + cross + cn, r1);
                     }
                     fence_proxy_async();  // make the generic-proxy writes visible to the TMA engine
                     __syncwarp();
@@ -1532,6 +1541,13 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (k_iters > 0) {
                     tmem_ld_32x8(t_row, r);
                     tmem_ld_wait();
+                    if (cross) {
+                        uint32_t x[8];
+                        tmem_ld_32x8(t_row + cross, x);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
+                    }
                 }
                 if (row_valid) {
 #pragma unroll
@@ -1582,6 +1598,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (live && col_base < P.c_out) {
                     tmem_ld_32x32(t_row, r0);
                     if (cpi == 64 && 32 < P.bn) tmem_ld_32x32(t_row + 32, r1);
+                    if (cpi == 32 && cross) tmem_ld_32x32(t_row + cross, r1);
                     tmem_ld_wait();
                 }
                 for (int c0 = 0; c0 < P.bn; c0 += cpi) {
@@ -1590,6 +1607,15 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     const int ncols = min(min(cpi, P.bn - c0), P.c_out - cg);  // (a tail of the tile or of the row)
                     const int cn = c0 + cpi;   // next piece
                     const bool more = live && cn < P.bn && col_base + cn < P.c_out;
+                    if (cross && live) {
+                        if (cpi == 64) {
+                            add_cross(c0, r0);
+                            if (c0 + 32 < P.bn) add_cross(c0 + 32, r1);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) r0[j] = __float_as_uint(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+                        }
+                    }
                     if (ncols == cpi && aligned) {
 #pragma unroll
                         for (int qq = 0; qq < 8; ++qq) {
@@ -1608,6 +1634,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         if (more) {  // registers are free again: start the next TMEM load now
                             tmem_ld_32x32(t_row + cn, r0);
                             if (cpi == 64 && cn + 32 < P.bn) tmem_ld_32x32(t_row + cn + 32, r1);
+                            if (cpi == 32 && cross) tmem_ld_32x32(t_row + cross + cn, r1);
                         }
                         __syncwarp();
                         // this lane's slice of the bias: columns cg + q*8 .. +7 (fp16) or cg + q*4 .. +3 (fp32)
@@ -1681,6 +1708,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         if (more) {
                             tmem_ld_32x32(t_row + cn, r0);
                             if (cpi == 64 && cn + 32 < P.bn) tmem_ld_32x32(t_row + cn + 32, r1);
+                            if (cpi == 32 && cross) tmem_ld_32x32(t_row + cross + cn, r1);
                         }
                         __syncwarp();
 #pragma unroll 1
@@ -1723,6 +1751,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (k_iters > 0) {
                     tmem_ld_32x32(t_row + c0, r);
                     tmem_ld_wait();
+                    if (cross) add_cross(c0, r);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) r[j] = 0u;

@@ -83,8 +83,8 @@ struct KParams {
     int fastdiv;         // 1: tile ids and divisors are small enough for the multiply-and-shift division to be exact
     int bn;              // UMMA N of one tile
     int tbufs;           // accumulator buffers in TMEM: 2, or 1 where planes * bn takes more than half of it (256-column
-                         // pair tiles of the 3xTF32 split: their K loops are long, and what they save in operand feed is
-                         // more than the epilogue they do not overlap)
+                         // pair tiles of a 3xTF32 weight gradient: what they save in operand feed is more than the
+                         // epilogue they do not overlap; forward walks measured the other way round and stay at 128)
     int stages;
     int cm_bw_log2, cm_bh_log2;  // OUT_NCHW_TMA: pixel sub-box (w, h) of one epilogue warp's 32 rows
     int epi_warps;       // 4, or 8 on the TMA-store instances when the epilogue is the critical path

@@ -79,7 +79,7 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_STAGES   cap on the ring depth            NML_TUNE_BN        forced tile width (64 / 128 / 256)
 //   NML_TUNE_KA       K atoms per stage (1 or 2)       NML_TUNE_L2PROMO   TMA L2 promotion (0..3)
 //   NML_TUNE_PAIR     0: no CTA pairs                  NML_TUNE_TMASTORE  0: no TMA-store epilogues
-//   NML_TUNE_EPI8     0: never a second epilogue group NML_TUNE_EPI8_K    K slices up to which it is used
+//   NML_TUNE_EPI8     0: never a second epilogue group
 //   NML_TUNE_PATCH    0: no forward patch walk, 2: wherever it is legal, 3: also with streamed weights
 //   NML_TUNE_BRES     0: patch walk streams its weights NML_TUNE_SHUFFLE  0: no phase-packed gather walk
 //   NML_TUNE_FSPLIT   0: no K split of the forward walk
@@ -87,7 +87,7 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_WTRANS   0: Linear input-gradients never take a transposed copy of the weights
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, epi8_k, patch, bres, shuffle, fsplit, wpatch, wcoal, wtrans, pair128;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, bres, shuffle, fsplit, wpatch, wcoal, wtrans, pair128;
 };
 static const Tune& tune() {
     static Tune t;
@@ -104,7 +104,6 @@ static const Tune& tune() {
         t.pair = env("NML_TUNE_PAIR", 1);
         t.tmastore = env("NML_TUNE_TMASTORE", 1);
         t.epi8 = env("NML_TUNE_EPI8", 1);
-        t.epi8_k = env("NML_TUNE_EPI8_K", 8);
         t.patch = env("NML_TUNE_PATCH", 1);
         t.bres = env("NML_TUNE_BRES", 1);
         t.shuffle = env("NML_TUNE_SHUFFLE", 1);
@@ -518,31 +517,42 @@ static int profile_open(cudaStream_t st) {
     return NML_OK;
 }
 
+// shared memory besides operands and staging: alignment slack, barriers, bias tiles
+constexpr int kFixedSmem = 1024 + 384 + kBiasTileBytes;
+
 static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open_slot = nullptr) {
     // Narrow tiles finish a 64-deep K slice in well under the barrier round trip of a stage, so they
     // take two slices per stage (8 MMAs per round trip); 256-wide tiles already fill 512 clocks.
     // The 3xTF32 split takes one slice: its two planes are 12 MMAs.
     P.ka = P.planes == 2 ? 2 : (P.pair && P.bn == 256) ? 1 : std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
-    P.tbufs = 2 * P.bn * P.planes <= 512 ? 2 : 1;
     const int stage_bytes = P.ka * (kStageABytes + (P.pair ? P.bn / 2 : P.bn) * 128);
     // Shared memory: the operand ring, then the epilogue's staging buffers (two per warp if that does not
     // cost a ring stage, else one), the per-warp bias tiles, and the barriers.
-    const int fixed = 1024 + 256 + kBiasTileBytes;
+    const int fixed = kFixedSmem;
     const bool tma_out = (P.mode == MODE_FPROP) && NML_IS_TMA_OUT(P.out_mode);
-    // A second group of four epilogue warps (TMA-store instances only) halves the drain time of a tile;
-    // it pays where the K loop is too short to hide the drain behind the next tile's MMAs.
-    {
-        const int cpi = P.out_f16 ? 64 : 32;
-        int k_slices = 0;  // 64-deep (fp16) K slices per tile, longest phase
+    // A second group of four epilogue warps (TMA-store instances only) where a tile's drain outlasts its MMAs.  Clocks,
+    // measured: one group needs ~800 per tile plus ~900 per 128-byte piece; four MMAs (one K slice) take 192 at 64 columns
+    // and below (shared-memory reads), 512 at 256.  With several tiles per CTA the groups take alternate tiles (one
+    // decode per two tiles); with one or two they share each tile, which shortens the last drain.
+    const int ctas = P.pair ? limited(ds->sms) / 2 : limited(ds->sms);
+    P.epi_warps = 4;
+    P.epi_alt = 0;
+    if (tma_out && tune().epi8) {
+        int k_slices = 0;  // longest phase
         for (int p = 0; p < P.n_phases; ++p) k_slices = std::max(k_slices, P.c_blocks * P.phases[p].tap_count);
-        const bool short_k = k_slices <= tune().epi8_k;
-        P.epi_warps = (tma_out && short_k && P.planes == 1 && P.bn / cpi >= 2 && tune().epi8) ? 8 : 4;
+        const int pieces = ceil_div(P.bn, P.out_f16 ? 64 : 32);
+        const int mma = k_slices * (P.planes == 2 ? 3 : 1) * (P.bn <= 64 ? 192 : P.bn <= 128 ? 288 : 512);
+        if (mma * 2 < (800 + 900 * pieces) * 3) {
+            P.epi_alt = P.num_tiles > 2 * ctas ? 1 : 0;
+            P.epi_warps = (P.epi_alt || pieces >= 2) ? 8 : 4;
+        }
     }
+    P.tbufs_log2 = 0;
+    while (P.tbufs_log2 < (P.epi_alt ? 2 : 1) && ((2 * P.bn * P.planes) << P.tbufs_log2) <= 512) ++P.tbufs_log2;
     size_t smem;
     if (P.wpatch) {
         // [stages x (patch, box of the other tensor)][staging (unused by this walk)][bias][barriers]
         P.ka = 1;
-        P.epi_warps = 4;
         P.stg_bufs = 1;
         const int w_stage = P.patch_bytes + P.bn * 128;
         const int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
@@ -558,7 +568,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         P.ka = 1;
         const int b_slice = P.bn * 128;
         const int res_bytes = P.c_blocks * P.n_taps * b_slice;  // the taps of every phase
-        P.stg_bufs = 2;
+        P.stg_bufs = P.epi_warps == 8 ? 1 : 2;  // (alternate groups return to a buffer after two tiles; patches need the room)
         int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
         const bool res_wanted = P.n_tiles == 1 && P.planes == 1 && tune().bres;
         if (res_wanted && res_bytes + 2 * P.patch_bytes > avail) {  // trade staging for residency
@@ -566,6 +576,8 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
             avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
             if (res_bytes + 2 * P.patch_bytes > avail) {
                 P.epi_warps = 4;
+                P.epi_alt = 0;
+                P.tbufs_log2 = std::min(P.tbufs_log2, 1);
                 avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
             }
         }
@@ -591,7 +603,8 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
             if (P.stages < 2) return NML_ERR_UNSUPPORTED;
             b_region = P.stages * b_stage;
         }
-        P.issuers = (P.b_resident && P.a_stages >= 2 * P.c_blocks) ? 2 : 1;
+        if (P.b_resident && P.a_stages < (P.c_blocks << P.tbufs_log2)) P.tbufs_log2 = std::min(P.tbufs_log2, 1);
+        P.issuers = (P.b_resident && P.tbufs_log2 >= 1 && P.a_stages >= (P.c_blocks << P.tbufs_log2)) ? 2 : 1;
         P.a_ring_off = static_cast<int>(round_up(b_region, 1024));
         P.ring_bytes = P.a_ring_off + P.a_stages * P.patch_bytes;
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
@@ -963,7 +976,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const int bn_res = (N <= 16 && !b_mn_major) ? 16 : static_cast<int>(round_up(N, 32));
         const long long res_need = 1ll * c_blocks * n_taps * bn_res * 128 + 2 * round_up(pw_ * ph_ * 128, 1024);
         const bool res_ok = P.planes == 1 && N <= 256 &&
-                            res_need <= 232448 - (1024 + 256 + kBiasTileBytes) - 4 * kStagingBufBytes;
+                            res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
         const bool streamed_ok = N <= 128 && (P.planes == 2 || mode >= 3);
         if (can && mode && (mode == 2 || (eff_patch >= 0.8 * eff_box && (res_ok || streamed_ok)))) {
             patch_resident = res_ok;
@@ -1111,18 +1124,18 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     }
     P.num_tiles = tiles;
     P.base_tiles = tiles;
-    {   // division by multiplication in the kernels' tile decode: exact while tile index x divisor < 2^40
-        const unsigned long long one40 = 1ull << 40;
+    {   // division by multiplication in the kernels' tile decode: exact while tile index x divisor < 2^32
+        auto reciprocal = [](int d) { return d > 1 ? static_cast<uint32_t>((1ull << 32) / static_cast<unsigned>(d) + 1) : 0u; };
         long long dmax = P.n_tiles;
-        P.mul_nt = one40 / static_cast<unsigned long long>(P.n_tiles) + 1;
+        P.mul_nt = reciprocal(P.n_tiles);
         for (int p = 0; p < n_phases; ++p) {
             Phase& ph = P.phases[p];
-            ph.mul_w = one40 / static_cast<unsigned long long>(std::max(1, ph.tiles_w)) + 1;
-            ph.mul_h = one40 / static_cast<unsigned long long>(std::max(1, ph.tiles_h)) + 1;
+            ph.mul_w = reciprocal(ph.tiles_w);
+            ph.mul_h = reciprocal(ph.tiles_h);
             dmax = std::max<long long>(dmax, std::max(ph.tiles_w, ph.tiles_h));
         }
         // (a pair doubles the row-tile index before it is divided)
-        P.fastdiv = (2ll * tiles < (1ll << 23) && 2ll * tiles * dmax < (1ll << 40)) ? 1 : 0;
+        P.fastdiv = (2ll * (tiles + 1) * dmax < (1ll << 32)) ? 1 : 0;
     }
     P.fsplit = 1;
     if (z_plan >= 2) {

@@ -69,7 +69,7 @@ struct Phase {
     int hq, wq;          // extent of the phase grid
     int tiles_h, tiles_w;
     int tile_begin;      // first tile id of this phase
-    unsigned long long mul_w, mul_h;  // 2^40 / tiles_w + 1, 2^40 / tiles_h + 1 (division by multiplication)
+    uint32_t mul_w, mul_h;  // for fast_div by tiles_w and tiles_h
 };
 
 struct KParams {
@@ -79,15 +79,17 @@ struct KParams {
     CUtensorMap tmC;     // OUT_NHWC_TMA: the output, box = the 32 rows x 128 bytes one epilogue warp owns
     int mode, out_mode;
     int num_tiles, n_tiles;
-    unsigned long long mul_nt;  // 2^40 / n_tiles + 1
+    uint32_t mul_nt;     // for fast_div by n_tiles
     int fastdiv;         // 1: tile ids and divisors are small enough for the multiply-and-shift division to be exact
     int bn;              // UMMA N of one tile
-    int tbufs;           // accumulator buffers in TMEM: 2, or 1 where planes * bn takes more than half of it (256-column
-                         // pair tiles of a 3xTF32 weight gradient: what they save in operand feed is more than the
-                         // epilogue they do not overlap; forward walks measured the other way round and stay at 128)
+    int tbufs_log2;      // accumulator buffers in TMEM: 2 (or 4 of narrow tiles, which lets the MMAs run ahead of two epilogue
+                         // groups), or 1 where planes * bn takes more than half of it (256-column pair tiles of a 3xTF32
+                         // weight gradient: what they save in operand feed is more than the epilogue they do not
+                         // overlap; forward walks measured the other way round and stay at 128)
     int stages;
     int cm_bw_log2, cm_bh_log2;  // OUT_NCHW_TMA: pixel sub-box (w, h) of one epilogue warp's 32 rows
     int epi_warps;       // 4, or 8 on the TMA-store instances when the epilogue is the critical path
+    int epi_alt;         // 8 warps: 1 = the two groups take alternate tiles, 0 = each takes half the columns of every tile
     int pair;            // 1: launched as clusters of two CTAs sharing 256x256 tiles (cta_group::2)
     int stg_bufs;        // staging buffers per epilogue warp (4 KB each): 2 when shared memory allows, else 1
     int ka;              // K atoms (128-byte-wide operand slices, times planes) per stage; narrow tiles take 2 to amortise
@@ -131,7 +133,7 @@ struct KParams {
     int patch_bytes;     // bytes one patch buffer occupies (multiple of 1024)
     int a_stages;        // patch buffers
     int b_resident;      // 1: every B slice of the launch is loaded once, at [pass plane][cb][tap] * bn * 128
-    int issuers;         // resident patch walk: 2 = the B producer issues the odd tiles (needs a_stages >= 2 * c_blocks)
+    int issuers;         // resident patch walk: 2 = the B producer issues the odd tiles (needs a_stages >= tbufs * c_blocks)
     int ring_bytes;      // bytes of the operand ring(s) in front of the staging buffers
     int a_ring_off;      // patch walk: offset of the patch buffers within the ring region
     int kind;            // KIND_F16 / KIND_TF32
@@ -176,10 +178,8 @@ struct KParams {
 
 // Tile decode runs once per tile in every role, and the epilogue warps in particular are bound by
 // instruction issue: a runtime integer division is ~25 instructions, the multiply-and-shift 4.
-// Exact for x * d < 2^40 (the host checks).
-__device__ __forceinline__ uint32_t fast_div(uint32_t x, unsigned long long mul) {
-    return static_cast<uint32_t>((static_cast<unsigned long long>(x) * mul) >> 40);
-}
+// mul = floor(2^32 / d) + 1, or 0 for d = 1.  Exact for x * d < 2^32 (the host checks).
+__device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t mul) { return mul ? __umulhi(x, mul) : x; }
 // Forward walk: tile index within its phase -> column tile and the (w, h, n) position of the row tile.
 template <bool kPair>
 __device__ __forceinline__ void decode_fprop_tile(const KParams& P, const Phase& ph, int local, uint32_t cta_rank,
@@ -276,18 +276,19 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     uint8_t* ctrl = staging + staging_bytes + kBiasTileBytes;
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);          // [stages]
     uint64_t* empty_bar = full_bar + 8;                               // [stages]
-    uint64_t* tfull_bar = empty_bar + 8;                              // [2]
-    uint64_t* tempty_bar = tfull_bar + 2;                             // [2]
-    uint64_t* afull_bar = tempty_bar + 2;                             // [4] patch walk: patch buffers
+    uint64_t* tfull_bar = empty_bar + 8;                              // [4]
+    uint64_t* tempty_bar = tfull_bar + 4;                             // [4]
+    uint64_t* afull_bar = tempty_bar + 4;                             // [4] patch walk: patch buffers
     uint64_t* aempty_bar = afull_bar + 4;                             // [4]
     uint64_t* bres_bar = aempty_bar + 4;                              // [1] patch walk: resident B has landed
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bres_bar + 1);
+    uint64_t* turn_bar = bres_bar + 1;                                // [2] patch walk, two issuers: whose turn it is
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(turn_bar + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);  // abort state: 4 ints, 8-byte aligned
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     // two accumulators; the epilogue reads 32 columns at a time, so a 16-column tile still needs 16 + 32
-    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : P.tbufs * P.bn * P.planes;
+    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : (P.bn * P.planes) << P.tbufs_log2;
     const uint32_t tmem_cols = (tmem_need <= 32) ? 32 : (tmem_need <= 64) ? 64 : (tmem_need <= 128) ? 128
                                : (tmem_need <= 256) ? 256 : 512;
 
@@ -296,15 +297,18 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             mbar_init(smem_u32(&full_bar[s]), P.patch ? 1 : 2);  // one arrival (with its byte count) per producer warp
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < 4; ++b) {
             mbar_init(smem_u32(&tfull_bar[b]), 1);
-            mbar_init(smem_u32(&tempty_bar[b]), (kPair ? 2 : 1) * P.epi_warps);  // the leader also hears the partner's epilogue warps
+            // the epilogue warps that drain one tile (the leader also hears the partner's)
+            mbar_init(smem_u32(&tempty_bar[b]), (kPair ? 2 : 1) * (P.epi_alt ? 4 : P.epi_warps));
         }
         for (int s = 0; s < 4; ++s) {
             mbar_init(smem_u32(&afull_bar[s]), P.wpatch ? 4 : 1);  // weight-gradient patch walk: the four epilogue warps meet here
             mbar_init(smem_u32(&aempty_bar[s]), 1);
         }
         mbar_init(smem_u32(bres_bar), 1);
+        mbar_init(smem_u32(&turn_bar[0]), 1);
+        mbar_init(smem_u32(&turn_bar[1]), 1);
         abort_state_init(abort_flag, P.wait_limit_ns);
         fence_mbar_init();
         tma_prefetch_desc(&P.tmA[0]);
@@ -339,9 +343,11 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     // (accumulator 0) and the B producer, idle once the weights have landed, the odd ones (accumulator 1).
     // One warp's per-tile bookkeeping (barrier waits, commits) then hides behind the other's MMAs.
     // A parity wait is only meaningful if the barrier's previous phase is known to be over.  An issuer waits
-    // for a patch only after the epilogue has drained tile t - 2 (the accumulator it reuses), i.e. after every
-    // patch up to that tile's last has landed; with a_stages >= 2 * c_blocks the patch that used the same
+    // for a patch only after the epilogue has drained tile t - tbufs (the accumulator it reuses), i.e. after every
+    // patch up to that tile's last has landed; with a_stages >= tbufs * c_blocks the patch that used the same
     // buffer before is among those (or is this issuer's own), so the host allows two issuers only then.
+    // They take turns: an issuer does its waiting ahead, but issues its tile only once the other has issued the one before.
+    // (MMAs of two tiles interleaved on the pipe took 67 clocks each, one tile's after the other's 56.)
     auto patch_resident_issue = [&](int t_first, int t_step) {
         const uint32_t idesc = make_instr_desc(P.kind, 0, P.b_mn_major, kTileM, P.bn);
         const bool b32 = P.b_mn_major && P.kind == KIND_TF32;
@@ -358,8 +364,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             const Tap* tp = &P.taps[P.phases[p].tap_begin];
             const int nt = P.phases[p].tap_count;
             const int tb0 = P.phases[p].tap_begin;
-            const int buf = P.tbufs == 2 ? (titer & 1) : 0;
-            const uint32_t tpar = P.tbufs == 2 ? (titer >> 1) & 1 : titer & 1;
+            const int buf = titer & ((1 << P.tbufs_log2) - 1);
+            const uint32_t tpar = (titer >> P.tbufs_log2) & 1;
             if (!mbar_wait(smem_u32(&tempty_bar[buf]), tpar ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) return;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + buf * P.bn;
@@ -370,6 +376,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 const uint32_t pparity = (pi / P.a_stages) & 1;
                 if (!mbar_wait(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) return;
                 tc_fence_after();
+                if (P.issuers == 2 && cb == 0 && titer > 0 &&
+                    !mbar_wait(smem_u32(&turn_bar[t_first]), ((titer - 1) >> 1) & 1, abort_flag, P.err, ERR_WAIT_EMPTY)) return;
                 if (elect_one()) {
                     const uint64_t adesc0 = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, 2);
                     uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, lbo_b, b32 ? 512 : 1024, b32 ? 1 : 2);
@@ -392,6 +400,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     }
                     umma_commit(smem_u32(&aempty_bar[pstage]));
                     if (cb + 1 == P.c_blocks) {
+                        if (P.issuers == 2) mbar_arrive(smem_u32(&turn_bar[t_first ^ 1]));
                         umma_commit(smem_u32(&tfull_bar[buf]));
                     }
                 }
@@ -881,8 +890,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 int kb_end = min(kb_begin + per, P.kblocks_total);
                 k_iters = max(kb_end - kb_begin, 0);
             }
-            const int buf = P.tbufs == 2 ? (titer & 1) : 0;
-            const uint32_t tpar = P.tbufs == 2 ? (titer >> 1) & 1 : titer & 1;
+            const int buf = titer & ((1 << P.tbufs_log2) - 1);
+            const uint32_t tpar = (titer >> P.tbufs_log2) & 1;
             if (kMode == MODE_WGRAD && !kPair && P.wpatch) {
                 // all row tiles at once, accumulator i in columns [i * bn, (i + 1) * bn); no second TMEM buffer, so
                 // the epilogue of the previous tile (if this CTA has one) must be over
@@ -1109,6 +1118,194 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         int titer = 0;
         uint32_t store_seq = 0;  // TMA-store pieces issued by this warp so far (selects the staging buffer)
         int bias_ntile = -1;     // column tile whose bias values sit in this warp's shared-memory copy
+        if constexpr (kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode)) {
+            // Output through TMA stores: each warp converts 128-byte pieces of its 32 rows into a swizzled 4 KB buffer and
+            // one lane hands the buffer to a TMA store, whose box is exactly those 32 rows; rows and columns outside the
+            // tensor are clipped by the hardware.
+            //
+            // A warp of its own on its scheduler runs at its instruction latencies, so what a tile costs here is the length of
+            // this chain: ~2400 clocks a tile of 64 columns when the decode was done twice and with 64-bit divisions, against
+            // 1728 clocks of MMAs for 3x3 64 -> 64 and 1344 for the 7x7 stem.  Hence one decode in 32-bit arithmetic before the
+            // wait, the accumulator handed back as soon as it is in registers, and two groups of four warps that take
+            // alternate tiles (epi_alt) where a tile's K loop is shorter than the chain.
+            constexpr int cpi = kOutF16 ? 64 : 32;  // columns of one 128-byte piece
+            const uint32_t stg0 = smem_u32(staging) + ew * P.stg_bufs * kStagingBufBytes;
+            const float* bt = bias_tile + ew * 256;
+            const bool has_bias = (P.bias != nullptr);
+            const uint32_t cross = P.planes == 2 ? P.bn : 0;  // the 3xTF32 split's second accumulator, this many columns further on
+            // position of this warp's first row within the tile's box
+            const int rw = (quarter * 32) & (wb - 1), rh = ((quarter * 32) >> P.wb_log2) & (hb - 1);
+            const int rn = (quarter * 32) >> (P.wb_log2 + P.hb_log2);
+            // channel-major output: where this lane's pixel starts in the staging tile, and the bytes between channels
+            uint32_t cm_pix = 0, cm_step = 0;
+            if (kOutMode == OUT_NCHW_TMA) {
+                const int bwl = P.cm_bw_log2, bhl = P.cm_bh_log2;
+                const int dwp = lane & ((1 << bwl) - 1), dhp = (lane >> bwl) & ((1 << bhl) - 1), dnp = lane >> (bwl + bhl);
+                const uint32_t esz = kOutF16 ? 2 : 4;
+                cm_pix = ((((dnp * cpi) << bhl) + dhp) << bwl) * esz + dwp * esz;
+                cm_step = esz << (bwl + bhl);
+            }
+            // two groups that share every tile: the first takes the low half of its pieces, the second the rest
+            int c_begin = 0, c_end = P.bn;
+            if (P.epi_warps == 8 && !P.epi_alt) {
+                const int half = ((P.bn / cpi + 1) / 2) * cpi;
+                if (ew < 4) c_end = min(half, P.bn); else c_begin = half;
+            }
+            const int t_step = P.epi_alt ? 2 : 1;
+            titer = (P.epi_alt && ew >= 4) ? 1 : 0;
+            int p = 0;  // phase of the tile (tile ids only grow)
+            for (int tile = tile_first + titer * tile_step; tile < P.num_tiles; tile += t_step * tile_step, titer += t_step) {
+                while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
+                const Phase& ph = P.phases[p];
+                int ntile, tw, th, tn;
+                decode_fprop_tile<kPair>(P, ph, tile - ph.tile_begin, cta_rank, ntile, tw, th, tn);
+                const int sw = ph.pw + P.out_stride_w * ((tw << P.wb_log2) + rw);
+                const int sh = ph.ph + P.out_stride_h * ((th << P.hb_log2) + rh);
+                const int sn = (tn << P.nb_log2) + rn;
+                const int col_base = ntile * P.bn;
+                const int c_stop = min(c_end, P.c_out - col_base);  // pieces start below this column
+                const bool live = ph.tap_count > 0;
+                if (has_bias && ntile != bias_ntile) {
+                    // this column tile's bias values, one copy per warp (no cross-warp barrier to get stuck on); all eight
+                    // loads of a lane are issued before the first is used, so the fill costs one memory latency, not eight
+                    bias_ntile = ntile;
+                    float* btw = bias_tile + ew * 256;
+                    float bv[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int j = lane + 32 * u;
+                        bv[u] = !(j < P.bn && col_base + j < P.c_out) ? 0.f
+                                : P.bias_f16 ? __half2float(__ldg(reinterpret_cast<const __half*>(P.bias) + col_base + j))
+                                             : __ldg(P.bias + col_base + j);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        if (lane + 32 * u < P.bn) btw[lane + 32 * u] = bv[u];
+                    __syncwarp();
+                }
+                const int buf = titer & ((1 << P.tbufs_log2) - 1);
+                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * P.planes;
+                if (!mbar_wait(smem_u32(&tfull_bar[buf]), (titer >> P.tbufs_log2) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) break;
+                tc_fence_after();
+                uint32_t r0[32], r1[32];
+                // (fp32 pieces are 32 columns: r1 then holds the second accumulator's)
+                auto fetch = [&](int c) {
+                    tmem_ld_32x32(t_row + c, r0);
+                    if (cpi == 64) tmem_ld_32x32(t_row + c + 32, r1);
+                    else if (cross) tmem_ld_32x32(t_row + cross + c, r1);
+                };
+                auto add_cross = [&](int c, uint32_t (&r)[32]) {
+                    uint32_t x[32];
+                    tmem_ld_32x32(t_row + cross + c, x);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
+                };
+                auto hand_back = [&]() {  // everything this warp reads of the accumulator is in registers
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (kPair && !leader) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), 0));
+                        else mbar_arrive(smem_u32(&tempty_bar[buf]));
+                    }
+                };
+                if (!live) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) r0[j] = r1[j] = 0u;
+                }
+                if (live && c_begin < c_stop) {
+                    fetch(c_begin);
+                    tmem_ld_wait();
+                } else {
+                    hand_back();
+                }
+                for (int c0 = c_begin; c0 < c_stop; c0 += cpi) {
+                    const int cn = c0 + cpi;
+                    const bool more = live && cn < c_stop;
+                    const uint32_t buf_addr = stg0 + ((P.stg_bufs == 2) ? (store_seq & 1) * kStagingBufBytes : 0);
+                    if (cross && live) {
+                        if (cpi == 64) {
+                            add_cross(c0, r0);
+                            add_cross(c0 + 32, r1);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) r0[j] = __float_as_uint(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
+                        }
+                    }
+                    if (live && !more) hand_back();
+                    // the store that last read this buffer must be done reading it
+                    if (lane == 0) {
+                        if (P.stg_bufs == 2) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
+                    }
+                    __syncwarp();
+                    if (kOutMode == OUT_NCHW_TMA) {
+                        // channel-major output: the staging tile is [image][channel][h][w] of this warp's
+                        // pixel sub-box, so lane (= pixel) l writes channel j at ((dn*cpi + j)*bh + dh)*bw + dw
+                        const uint32_t pix = buf_addr + cm_pix, cstep = cm_step;
+#pragma unroll
+                        for (int j = 0; j < cpi; ++j) {
+                            float xv = __uint_as_float(j < 32 ? r0[j & 31] : r1[j & 31]);
+                            if (has_bias) xv += bt[c0 + j];
+                            if (kOutF16) {
+                                const __half hv = __float2half_rn(xv);
+                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(pix + j * cstep), "h"(*reinterpret_cast<const uint16_t*>(&hv)) : "memory");
+                            } else {
+                                if (P.round_f16) xv = round_through_f16(xv);
+                                asm volatile("st.shared.b32 [%0], %1;" ::"r"(pix + j * cstep), "r"(__float_as_uint(xv)) : "memory");
+                            }
+                        }
+                    } else
+#pragma unroll
+                    for (int qq = 0; qq < 8; ++qq) {
+                        uint4 pk;
+                        if (kOutF16) {
+                            const uint32_t* src = (qq < 4) ? &r0[8 * qq] : &r1[8 * (qq - 4)];
+                            float v[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(src[j]);
+                            if (has_bias) {
+                                const float4 ba = *reinterpret_cast<const float4*>(bt + c0 + 8 * qq);
+                                const float4 bb = *reinterpret_cast<const float4*>(bt + c0 + 8 * qq + 4);
+                                v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w;
+                                v[4] += bb.x; v[5] += bb.y; v[6] += bb.z; v[7] += bb.w;
+                            }
+                            pk.x = pack_half2(v[0], v[1]);
+                            pk.y = pack_half2(v[2], v[3]);
+                            pk.z = pack_half2(v[4], v[5]);
+                            pk.w = pack_half2(v[6], v[7]);
+                        } else {
+                            float v[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r0[4 * qq + j]);
+                            if (has_bias) {
+                                const float4 ba = *reinterpret_cast<const float4*>(bt + c0 + 4 * qq);
+                                v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w;
+                            }
+                            if (P.round_f16) {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) v[j] = round_through_f16(v[j]);
+                            }
+                            pk.x = __float_as_uint(v[0]); pk.y = __float_as_uint(v[1]);
+                            pk.z = __float_as_uint(v[2]); pk.w = __float_as_uint(v[3]);
+                        }
+                        st_shared_v4(buf_addr + lane * 128 + ((qq ^ (lane & 7)) << 4), pk);
+                    }
+                    if (more) fetch(cn);  // registers are free again: start the next TMEM load now
+                    fence_proxy_async();  // make the generic-proxy writes visible to the TMA engine
+                    __syncwarp();
+                    if (lane == 0) {
+                        const int cg = col_base + c0;
+                        if (kOutMode == OUT_NCHW_TMA) tma_store_4d(&P.tmC, buf_addr, sw, sh, cg, sn);
+                        else tma_store_4d(&P.tmC, buf_addr, cg, sw, sh, sn);
+                        bulk_commit_group();
+                    }
+                    ++store_seq;
+                    if (more) tmem_ld_wait();
+                }
+            }
+            if (lane == 0) bulk_wait_group<0>();  // stores must land before the CTA ends
+        } else
         for (int tile_id = tile_first; ok && tile_id < P.num_tiles; tile_id += tile_step, ++titer) {
             int tile = tile_id, kz = 0;
             if (kMode == MODE_FPROP && P.fsplit > 1) {
@@ -1226,8 +1423,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[0]));
                 continue;
             }
-            const int buf = P.tbufs == 2 ? (titer & 1) : 0;
-            const uint32_t tpar = P.tbufs == 2 ? (titer >> 1) & 1 : titer & 1;
+            const int buf = titer & ((1 << P.tbufs_log2) - 1);
+            const uint32_t tpar = (titer >> P.tbufs_log2) & 1;
             // tile decode
             int ntile, k_iters;
             bool row_valid;
@@ -1258,7 +1455,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     const int k_first = min(kz * per, full);
                     k_iters = min(k_first + per, full) - k_first;
                 }
-                if (kOutMode != OUT_NCHW && kOutMode != OUT_NCHW_TMA) {
+                if (kOutMode != OUT_NCHW) {
                     row_off = ((static_cast<size_t>(n) * P.out_h + oh) * P.out_w + ow) * P.ld_out;
                     col_stride = 1;
                 } else {
@@ -1299,29 +1496,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     col_stride = static_cast<size_t>(P.ld_plane);
                 }
             }
-            if (kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode) && P.bias != nullptr) {
-                // this tile's bias values, one copy per warp (no cross-warp barrier to get stuck on)
-                // (skipped when the column tile is the one this warp loaded last; all eight loads of a lane are
-                // issued before the first is used, so the fill costs one memory latency, not eight)
-                if (ntile != bias_ntile) {
-                    bias_ntile = ntile;
-                    float* btw = bias_tile + ew * 256;
-                    const int cb0 = ntile * P.bn;
-                    float bv[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int j = lane + 32 * u;
-                        bv[u] = !(j < P.bn && cb0 + j < P.c_out) ? 0.f
-                                : P.bias_f16 ? __half2float(__ldg(reinterpret_cast<const __half*>(P.bias) + cb0 + j))
-                                             : __ldg(P.bias + cb0 + j);
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (lane + 32 * u < P.bn) btw[lane + 32 * u] = bv[u];
-                    __syncwarp();
-                }
-            }
             // Row-major epilogue: this lane's bias slice for the first 128-byte piece is fetched before
             // the wait, and each later slice one piece ahead, so the load latency never shows.
             float4 nb0 = make_float4(0.f, 0.f, 0.f, 0.f), nb1 = nb0;
@@ -1355,141 +1529,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(x[j]));
             };
             const int col_base = ntile * P.bn;
-            if (kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode)) {
-                // Row-major output through TMA: each warp converts 128-byte row pieces of its 32 rows into a
-                // swizzled 4 KB buffer and one lane hands the buffer to a TMA store, whose box is exactly
-                // those 32 rows; rows and columns outside the tensor are clipped by the hardware.  Two
-                // buffers alternate, so packing the next piece overlaps the store of the previous one.
-                constexpr int cpi = kOutF16 ? 64 : 32;
-                const uint32_t stg0 = smem_u32(staging) + ew * P.stg_bufs * kStagingBufBytes;
-                const float* bt = bias_tile + ew * 256;
-                const bool has_bias = (P.bias != nullptr);
-                // store coordinates of this warp's first row
-                int sw, sh, sn;
-                {
-                    int p = 0;
-                    while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
-                    const Phase& ph = P.phases[p];
-                    int local = tile - ph.tile_begin;
-                    int nt_unused, tw, th, tn;
-                    decode_fprop_tile<kPair>(P, ph, local, cta_rank, nt_unused, tw, th, tn);
-                    const int row0 = quarter * 32;
-                    sw = ph.pw + P.out_stride_w * ((tw << P.wb_log2) + (row0 & (wb - 1)));
-                    sh = ph.ph + P.out_stride_h * ((th << P.hb_log2) + ((row0 >> P.wb_log2) & (hb - 1)));
-                    sn = (tn << P.nb_log2) + (row0 >> (P.wb_log2 + P.hb_log2));
-                }
-                uint32_t r0[32], r1[32];
-                const bool live = (k_iters > 0);
-                if (!live) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) r0[j] = r1[j] = 0u;
-                }
-                // with two epilogue groups, the first takes the low half of the tile's pieces, the second the rest
-                int c_begin = 0, c_end = P.bn;
-                if (P.epi_warps == 8) {
-                    const int half = ((P.bn / cpi + 1) / 2) * cpi;
-                    if (ew < 4) c_end = min(half, P.bn); else c_begin = half;
-                }
-                if (live && c_begin < c_end && col_base + c_begin < P.c_out) {
-                    tmem_ld_32x32(t_row + c_begin, r0);
-                    if (cpi == 64) tmem_ld_32x32(t_row + c_begin + 32, r1);
-                    else if (cross) tmem_ld_32x32(t_row + cross + c_begin, r1);
-                    tmem_ld_wait();
-                }
-                for (int c0 = c_begin; c0 < c_end; c0 += cpi) {
-                    const int cg = col_base + c0;
-                    if (cg >= P.c_out) break;  // uniform across the warp
-                    const int cn = c0 + cpi;
-                    const bool more = live && cn < c_end && col_base + cn < P.c_out;
-                    const uint32_t buf_addr = stg0 + ((P.stg_bufs == 2) ? (store_seq & 1) * kStagingBufBytes : 0);
-                    if (cross && live) {
-                        if (cpi == 64) {
-                            add_cross(c0, r0);
-                            add_cross(c0 + 32, r1);
-                        } else {  // (fetched along with r0)
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) r0[j] = __float_as_uint(__uint_as_float(r0[j]) + __uint_as_float(r1[j]));
-                        }
-                    }
-                    // the store that last read this buffer must be done reading it
-                    if (lane == 0) {
-                        if (P.stg_bufs == 2) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
-                    }
-                    __syncwarp();
-                    if (kOutMode == OUT_NCHW_TMA) {
-                        // channel-major output: the staging tile is [image][channel][h][w] of this warp's
-                        // pixel sub-box, so lane (= pixel) l writes channel j at ((dn*cpi + j)*bh + dh)*bw + dw
-                        const int bwl = P.cm_bw_log2, bhl = P.cm_bh_log2;
-                        const int dwp = lane & ((1 << bwl) - 1);
-                        const int dhp = (lane >> bwl) & ((1 << bhl) - 1);
-                        const int dnp = lane >> (bwl + bhl);
-                        const uint32_t esz = kOutF16 ? 2 : 4;
-                        const uint32_t pix = buf_addr + ((((dnp * cpi) << bhl) + dhp) << bwl) * esz + dwp * esz;
-                        const uint32_t cstep = (esz << (bwl + bhl));  // bytes between consecutive channels
-#pragma unroll
-                        for (int j = 0; j < cpi; ++j) {
-                            float xv = __uint_as_float(j < 32 ? r0[j & 31] : r1[j & 31]);
-                            if (has_bias) xv += bt[c0 + j];
-                            if (kOutF16) {
-                                const __half hv = __float2half_rn(xv);
-                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(pix + j * cstep), "h"(*reinterpret_cast<const uint16_t*>(&hv)) : "memory");
-                            } else {
-                                if (P.round_f16) xv = round_through_f16(xv);
-                                asm volatile("st.shared.b32 [%0], %1;" ::"r"(pix + j * cstep), "r"(__float_as_uint(xv)) : "memory");
-                            }
-                        }
-                    } else
-#pragma unroll
-                    for (int qq = 0; qq < 8; ++qq) {
-                        uint4 pk;
-                        if (kOutF16) {
-                            const uint32_t* src = (qq < 4) ? &r0[8 * qq] : &r1[8 * (qq - 4)];
-                            float v[8];
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(src[j]);
-                            if (has_bias) {
-                                const float4 ba = *reinterpret_cast<const float4*>(bt + c0 + 8 * qq);
-                                const float4 bb = *reinterpret_cast<const float4*>(bt + c0 + 8 * qq + 4);
-                                v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w;
-                                v[4] += bb.x; v[5] += bb.y; v[6] += bb.z; v[7] += bb.w;
-                            }
-                            pk.x = pack_half2(v[0], v[1]);
-                            pk.y = pack_half2(v[2], v[3]);
-                            pk.z = pack_half2(v[4], v[5]);
-                            pk.w = pack_half2(v[6], v[7]);
-                        } else {
-                            float v[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) v[j] = __uint_as_float(r0[4 * qq + j]);
-                            if (has_bias) {
-                                const float4 ba = *reinterpret_cast<const float4*>(bt + c0 + 4 * qq);
-                                v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w;
-                            }
-                            if (P.round_f16) {
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) v[j] = round_through_f16(v[j]);
-                            }
-                            pk.x = __float_as_uint(v[0]); pk.y = __float_as_uint(v[1]);
-                            pk.z = __float_as_uint(v[2]); pk.w = __float_as_uint(v[3]);
-                        }
-                        st_shared_v4(buf_addr + lane * 128 + ((qq ^ (lane & 7)) << 4), pk);
-                    }
-                    if (more) {  // registers are free again: start the next TMEM load now
-                        tmem_ld_32x32(t_row + cn, r0);
-                        if (cpi == 64) tmem_ld_32x32(t_row + cn + 32, r1);
-                        else if (cross) tmem_ld_32x32(t_row + cross + cn, r1);
-                    }
-                    fence_proxy_async();  // make the generic-proxy writes visible to the TMA engine
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (kOutMode == OUT_NCHW_TMA) tma_store_4d(&P.tmC, buf_addr, sw, sh, cg, sn);
-                        else tma_store_4d(&P.tmC, buf_addr, cg, sw, sh, sn);
-                        bulk_commit_group();
-                    }
-                    ++store_seq;
-                    if (more) tmem_ld_wait();
-                }
-            } else
             if (kMode == MODE_FPROP && kOutMode == OUT_NHWC && P.shuf_sh > 0) {
                 // Phase-packed columns: this thread's pixel owns shuf_sh rows of shuf_sw * shuf_c consecutive
                 // output values.  Short on purpose, like the few-channel epilogue below.
@@ -1800,7 +1839,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 else mbar_arrive(smem_u32(&tempty_bar[buf]));
             }
         }
-        if (NML_IS_TMA_OUT(kOutMode) && lane == 0) bulk_wait_group<0>();  // stores must land before the CTA ends
     }
 
     // ------------------------------------------------------------ teardown --

@@ -86,8 +86,9 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_WPATCH   0: no weight-gradient patch walk NML_TUNE_WCOAL     0: its gradient leaves by scattered stores
 //   NML_TUNE_WTRANS   0: Linear input-gradients never take a transposed copy of the weights
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
+//   NML_TUNE_NARROW   0: few-channel layers always take eight channels per pixel
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, bres, shuffle, fsplit, wpatch, wcoal, wtrans, pair128;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, bres, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow;
 };
 static const Tune& tune() {
     static Tune t;
@@ -112,11 +113,12 @@ static const Tune& tune() {
         t.wcoal = env("NML_TUNE_WCOAL", 1);
         t.wtrans = env("NML_TUNE_WTRANS", 1);
         t.pair128 = env("NML_TUNE_PAIR128", 1);
+        t.narrow = env("NML_TUNE_NARROW", 1);
     });
     return t;
 }
 
-enum { SWZ_NONE = 0, SWZ_128B = 1, SWZ_128B_ATOM32 = 2 };
+enum { SWZ_NONE = 0, SWZ_128B = 1, SWZ_128B_ATOM32 = 2, SWZ_64B = 3 };
 
 // Tensor map over a dense tensor given fastest-first dims; strides are the dense ones.
 static int encode_map(CUtensorMap* tm, const void* ptr, int elem_bytes, int rank, const uint64_t* dims,
@@ -140,6 +142,7 @@ static int encode_map(CUtensorMap* tm, const void* ptr, int elem_bytes, int rank
     CUresult r = fn(tm, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                     rank, const_cast<void*>(ptr), gdim, gstr, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle == SWZ_128B ? CU_TENSOR_MAP_SWIZZLE_128B
+                    : swizzle == SWZ_64B ? CU_TENSOR_MAP_SWIZZLE_64B
                     : swizzle == SWZ_128B_ATOM32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
                                                  : CU_TENSOR_MAP_SWIZZLE_NONE,
                     static_cast<CUtensorMapL2promotion>(tune().l2promo),
@@ -222,8 +225,9 @@ static int load_helper_kernels() {
         (const void*)colsum_vectors_kernel<float>, (const void*)colsum_vectors_kernel<__half>,
         (const void*)repack_weight_tile_kernel<float>, (const void*)repack_weight_tile_kernel<__half>,
         (const void*)repack_weight_rows_kernel<float>, (const void*)repack_weight_rows_kernel<__half>,
-        (const void*)pad_pack_c8_kernel<float>, (const void*)pad_pack_c8_kernel<__half>,
-        (const void*)repack_weight_c8_kernel<float>, (const void*)repack_weight_c8_kernel<__half>,
+        (const void*)pad_pack_kernel<float, 4>, (const void*)pad_pack_kernel<__half, 4>,
+        (const void*)pad_pack_kernel<float, 8>, (const void*)pad_pack_kernel<__half, 8>,
+        (const void*)repack_weight_window_kernel<float>, (const void*)repack_weight_window_kernel<__half>,
         (const void*)finish_rows_kernel<float>, (const void*)finish_rows_kernel<__half>,
         (const void*)pack_phase_weights_kernel<float, float>, (const void*)pack_phase_weights_kernel<float, __half>,
         (const void*)pack_phase_weights_kernel<__half, float>, (const void*)pack_phase_weights_kernel<__half, __half>,
@@ -429,30 +433,36 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
     return NML_OK;
 }
 
-// Few-channel path: the activation as a zero-padded [N][Hp][Wp][8] fp16 image (see pad_pack_c8_kernel).
+// Few-channel path: the activation as a zero-padded [N][Hp][Wp][ch] fp16 image (see pad_pack_kernel).
 // Wp leaves room for the 8-pixel window of the last output column.
 struct WindowImage {
     const void* ptr;
     int hp, wp;
 };
 static bool window_eligible(int c, int kw, int d_w, int enc) { return c <= 8 && kw <= 8 && d_w == 1 && enc == ENC_F16; }
+// Four channels per pixel halve the MMAs, the patches and the padded image, but consecutive windows start 8 * stride_w
+// bytes apart, and TMA wants multiples of 16: odd strides keep eight.
+static bool narrow_eligible(int c, int s_w) { return c <= 4 && s_w % 2 == 0 && tune().narrow; }
 static int prepare_window(const void* src, int dtype, int layout, int batch, int c, int h, int w, int p_h, int p_w,
-                          int s_w, int out_w, Bump& ws, cudaStream_t st, WindowImage* img, float* colsum = nullptr) {
+                          int s_w, int out_w, int ch, Bump& ws, cudaStream_t st, WindowImage* img, float* colsum = nullptr) {
     img->hp = h + 2 * p_h;
-    img->wp = std::max(w + 2 * p_w, (out_w - 1) * s_w + 8);
-    const size_t pixels = static_cast<size_t>(batch) * img->hp * img->wp;
-    void* p = ws.take(pixels * 16);
+    img->wp = static_cast<int>(round_up(std::max(w + 2 * p_w, (out_w - 1) * s_w + 8), 2));
+    const size_t rows = static_cast<size_t>(batch) * img->hp;
+    if (rows >= (1u << 31)) return NML_ERR_UNSUPPORTED;
+    void* p = ws.take(rows * img->wp * ch * 2);
     img->ptr = p;
-    int blocks = static_cast<int>(std::min<size_t>((pixels + 255) / 256, 148 * 32));
+    int blocks = static_cast<int>(std::min<size_t>((rows + 7) / 8, 148 * 8));
     ColsumScratch cs;
-    if (colsum) cs = colsum_scratch(ws, blocks, 8);  // one row of 8 channel sums per block
+    if (colsum) cs = colsum_scratch(ws, blocks, 8);  // one row of up to 8 channel sums per block
     if (ws.dry) return NML_OK;
     if (!ws.fits()) return NML_ERR_WORKSPACE;
     const int nchw = (layout == NML_NCHW) ? 1 : 0;
-    if (dtype == NML_F32)
-        { launch(pad_pack_c8_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(src), nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial); ++g_launches; }
-    else
-        { launch(pad_pack_c8_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(src), nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial); ++g_launches; }
+    auto run = [&](auto kernel, auto* in) {
+        launch(kernel, blocks, 256, 0, st, in, nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial);
+    };
+    if (dtype == NML_F32) run(ch == 4 ? pad_pack_kernel<float, 4> : pad_pack_kernel<float, 8>, static_cast<const float*>(src));
+    else run(ch == 4 ? pad_pack_kernel<__half, 4> : pad_pack_kernel<__half, 8>, static_cast<const __half*>(src));
+    ++g_launches;
     NML_CUDA(cudaGetLastError());
     if (colsum) return colsum_finish(cs, c, colsum, st);
     return NML_OK;
@@ -566,7 +576,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     } else if (P.patch) {
         // [B: resident slices, or a ring of single-slice stages][patch buffers][staging][bias][barriers]
         P.ka = 1;
-        const int b_slice = P.bn * 128;
+        const int b_slice = P.bn * P.b_row_bytes;
         const int res_bytes = P.c_blocks * P.n_taps * b_slice;  // the taps of every phase
         P.stg_bufs = P.epi_warps == 8 ? 1 : 2;  // (alternate groups return to a buffer after two tiles; patches need the room)
         int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
@@ -662,6 +672,23 @@ struct FpropLike {
     int w_batched;  // every image has its own [d0][d1] weights, one after the other (batched matmul; kh = kw = 1)
 };
 
+// Whether a few-channel layer with N output channels takes the patch walk with resident weights when its rows are 64
+// bytes long (the conditions of run_fprop_like's own choice, which then makes the same one).
+static bool narrow_patch_walk(const FpropLike& f, int N) {
+    if (tune().patch != 1 || !tune().bres || N > 256) return false;
+    const int range_h = (f.kh - 1) * f.d_h, pw = 8, ph = 15 * f.s_h + range_h + 1;
+    if (f.kh < 2 || ph > 256 || pw * ph * 64 > 48 * 1024) return false;
+    int wl = 0, hl = 0, nl = 0;
+    const bool nchw = f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1);
+    choose_box(7, f.out_w, f.out_h, f.batch, 1, f.s_h, &wl, &hl, &nl, nchw ? 5 : 0);
+    const double area = static_cast<double>(f.out_w) * f.out_h;
+    const double eff_patch = area / (1.0 * round_up(f.out_w, 8) * round_up(f.out_h, 16));
+    const double eff_box = area * f.batch / (1.0 * round_up(f.out_w, 1 << wl) * round_up(f.out_h, 1 << hl) * round_up(f.batch, 1 << nl));
+    const int bn = N <= 16 ? 16 : static_cast<int>(round_up(N, 32));
+    const long long need = 1ll * f.kh * bn * 64 + 2 * round_up(pw * ph * 64, 1024);
+    return eff_patch >= 0.8 * eff_box && need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
+}
+
 static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     MathInfo mi;
     if (!math_info(f.math, &mi)) return NML_ERR_INVALID;
@@ -738,13 +765,16 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     // as overlapping 8-pixel windows of a padded 8-channel image -- instead of one mostly empty
     // 64-channel slice per tap.
     const bool window = !f.gather && !f.k_is_dim0 && T > 1 && window_eligible(f.a_c, f.kw, f.d_w, mi.enc);
+    // (narrow: with four channels per pixel, where the patch walk with resident weights will be taken)
+    const bool narrow = window && narrow_eligible(f.a_c, f.s_w) && narrow_patch_walk(f, N);
+    const int win_ch = narrow ? 4 : 8, row_bytes = narrow ? 64 : 128;
     WindowImage wimg = {nullptr, 0, 0};
     // activation operand
     const void* a_planes[2] = {nullptr, nullptr};
     int Cp = 0;
     int rc;
     if (window)
-        rc = prepare_window(f.a, f.a_dtype, f.a_layout, f.batch, f.a_c, f.a_h, f.a_w, f.p_h, f.p_w, f.s_w, f.out_w, ws, st,
+        rc = prepare_window(f.a, f.a_dtype, f.a_layout, f.batch, f.a_c, f.a_h, f.a_w, f.p_h, f.p_w, f.s_w, f.out_w, win_ch, ws, st,
                             &wimg);
     else
         rc = prepare_activation(f.a, f.a_dtype, f.a_layout, f.batch, f.a_c, f.a_h, f.a_w, mi, ws, st, a_planes, &Cp,
@@ -760,15 +790,16 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     const void* w_planes[2] = {f.w, nullptr};
     int b_mn_major = 0;
     if (window) {
-        void* p0 = ws.take(static_cast<size_t>(N) * f.kh * 64 * 2);
+        void* p0 = ws.take(static_cast<size_t>(N) * f.kh * 8 * win_ch * 2);
         w_planes[0] = p0;
         if (!ws.dry) {
             if (!ws.fits()) return NML_ERR_WORKSPACE;
-            int blocks = std::min(ceil_div(N * f.kh * 64, 256), 148 * 8);
+            const int blocks = std::min(ceil_div(N * f.kh * 8 * win_ch, 256), 148 * 8);
             if (f.w_dtype == NML_F32)
-                { launch_short(repack_weight_c8_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw); ++g_launches; }
+                launch_short(repack_weight_window_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw, narrow ? 2 : 3);
             else
-                { launch_short(repack_weight_c8_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw); ++g_launches; }
+                launch_short(repack_weight_window_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw, narrow ? 2 : 3);
+            ++g_launches;
             NML_CUDA(cudaGetLastError());
         }
     } else if (direct_w) {
@@ -838,6 +869,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     P.out_mode = (f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1)) ? OUT_NCHW : OUT_NHWC;
     P.kind = mi.kind;
     P.planes = mi.planes;
+    P.a_row_bytes = P.b_row_bytes = row_bytes;
     const int products = mi.planes == 2 ? 3 : 1;  // tensor-core products per K slice
     P.kb = mi.kb;
     P.c_blocks = c_blocks;
@@ -872,7 +904,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             Tap& t = P.taps[n_taps++];
             t.dh = static_cast<short>(kh * f.d_h);
             t.dw = 0;
-            t.wk = kh * 64;
+            t.wk = kh * 8 * win_ch;
         }
         ph.tap_count = static_cast<short>(n_taps);
         n_phases = 1;
@@ -970,11 +1002,11 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const double eff_box = static_cast<double>(wq) * hq * f.batch /
                                (1.0 * round_up(wq, 1 << P.wb_log2) * round_up(hq, 1 << P.hb_log2) * round_up(f.batch, 1 << P.nb_log2));
         const bool can = every_phase_has_taps && n_taps >= 2 && esw == 1 && pw_ <= 256 && ph_ <= 256 &&
-                         pw_ * ph_ * 128 <= 48 * 1024;
+                         pw_ * ph_ * row_bytes <= 48 * 1024;
         // B stays resident when every slice fits beside two patch buffers and the smallest epilogue staging;
         // streaming B tap by tap pays only for the 3xTF32 split (a barrier round trip per 4 short MMAs otherwise)
         const int bn_res = (N <= 16 && !b_mn_major) ? 16 : static_cast<int>(round_up(N, 32));
-        const long long res_need = 1ll * c_blocks * n_taps * bn_res * 128 + 2 * round_up(pw_ * ph_ * 128, 1024);
+        const long long res_need = 1ll * c_blocks * n_taps * bn_res * row_bytes + 2 * round_up(pw_ * ph_ * row_bytes, 1024);
         const bool res_ok = P.planes == 1 && N <= 256 &&
                             res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
         const bool streamed_ok = N <= 128 && (P.planes == 2 || mode >= 3);
@@ -983,11 +1015,11 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             P.patch = 1;
             P.patch_w = pw_;
             P.patch_h = ph_;
-            P.patch_bytes = static_cast<int>(round_up(pw_ * ph_ * 128, 1024));
+            P.patch_bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024));
             for (int p = 0; p < n_phases; ++p)
                 for (int t = 0; t < P.phases[p].tap_count; ++t) {
                     Tap& tp = P.taps[P.phases[p].tap_begin + t];
-                    tp.aoff = ((tp.dh - P.phases[p].org_h) * pw_ + (tp.dw - P.phases[p].org_w)) * 128 / 16;
+                    tp.aoff = ((tp.dh - P.phases[p].org_h) * pw_ + (tp.dw - P.phases[p].org_w)) * row_bytes / 16;
                 }
             P.n_taps = n_taps;
             P.wb_log2 = 3;
@@ -1166,12 +1198,13 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             aes[1] = aes[2] = 1;
         }
         if (window) {
-            // dims: (64 elements = 8 pixels x 8 channels, output column, padded row, image); consecutive
+            // dims: (8 pixels x 8 or 4 channels, output column, padded row, image); consecutive
             // output columns start s_w pixels apart, so the windows overlap
-            uint64_t wd[4] = {64, static_cast<uint64_t>(f.out_w), static_cast<uint64_t>(wimg.hp), static_cast<uint64_t>(f.batch)};
-            uint64_t wstr[3] = {static_cast<uint64_t>(f.s_w) * 16, static_cast<uint64_t>(wimg.wp) * 16,
-                                static_cast<uint64_t>(wimg.hp) * wimg.wp * 16};
-            rc = encode_map(&P.tmA[pl], a_planes[pl], 2, 4, wd, abox, aes, SWZ_128B, wstr);
+            const uint64_t pix = 2ull * win_ch;
+            uint64_t wd[4] = {8ull * win_ch, static_cast<uint64_t>(f.out_w), static_cast<uint64_t>(wimg.hp), static_cast<uint64_t>(f.batch)};
+            uint64_t wstr[3] = {f.s_w * pix, wimg.wp * pix, static_cast<uint64_t>(wimg.hp) * wimg.wp * pix};
+            abox[0] = static_cast<uint32_t>(8 * win_ch);
+            rc = encode_map(&P.tmA[pl], a_planes[pl], 2, 4, wd, abox, aes, narrow ? SWZ_64B : SWZ_128B, wstr);
         } else {
             rc = encode_map(&P.tmA[pl], a_planes[pl], mi.es, 4, adims, abox, aes, SWZ_128B);
         }
@@ -1197,9 +1230,9 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                 rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 3, d, box, one4, SWZ_128B);
             }
         } else if (!b_mn_major) {
-            uint64_t bdims[2] = {static_cast<uint64_t>(direct_w ? K : (window ? f.kh * 64 : T * kp)), static_cast<uint64_t>(N)};
-            uint32_t bbox[2] = {static_cast<uint32_t>(mi.kb), static_cast<uint32_t>(P.pair ? P.bn / 2 : P.bn)};
-            rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 2, bdims, bbox, one, SWZ_128B);
+            uint64_t bdims[2] = {static_cast<uint64_t>(direct_w ? K : (window ? f.kh * 8 * win_ch : T * kp)), static_cast<uint64_t>(N)};
+            uint32_t bbox[2] = {static_cast<uint32_t>(row_bytes / mi.es), static_cast<uint32_t>(P.pair ? P.bn / 2 : P.bn)};
+            rc = encode_map(&P.tmB[pl], w_planes[pl], mi.es, 2, bdims, bbox, one, narrow ? SWZ_64B : SWZ_128B);
         } else if (N % mi.kb == 0) {
             // one box per stage: the outermost dimension walks the 128-byte column groups
             P.b_grouped = 1;
@@ -1289,11 +1322,21 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     // Few-channel layer input (RGB stems): patches come as 8-pixel windows of the padded 8-channel image,
     // one kernel row per tap, (kw, c) packed in the 64 patch columns.
     const bool window = T > 1 && window_eligible(g.patch_c, g.kw, g.d_w, mi.enc);
+    // (narrow: with four channels per pixel, where the patch walk below will be taken: the same conditions)
+    bool narrow = window && narrow_eligible(g.patch_c, g.s_w) && tune().wpatch && round_up(g.plain_c, 8) % 64 == 0 && g.kh >= 2 && g.kh <= 32;
+    if (narrow) {
+        const int ph = 7 * g.s_h + (g.kh - 1) * g.d_h + 1;
+        const double eff = static_cast<double>(g.plain_w) * g.plain_h / (1.0 * round_up(g.plain_w, 8) * round_up(g.plain_h, 8));
+        // (a row tile always reads four kernel rows: the ones past the last have to stay within the stage's other box)
+        const int past = static_cast<int>(round_up(g.kh, 4) - g.kh) * g.d_h * 8 * 64;
+        narrow = ph <= 256 && 8 * ph * 64 <= 40 * 1024 && eff >= 0.7 && past <= 64 * 128;
+    }
+    const int win_ch = narrow ? 4 : 8, row_bytes = narrow ? 64 : 128;
     WindowImage wimg = {nullptr, 0, 0};
     int rc;
     if (window) {
         rc = prepare_window(g.patch, g.dtype, g.layout, g.batch, g.patch_c, g.patch_h, g.patch_w, g.p_h, g.p_w, g.s_w,
-                            g.plain_w, ws, st, &wimg, g.colsum_of_patch ? g.colsum : nullptr);
+                            g.plain_w, win_ch, ws, st, &wimg, g.colsum_of_patch ? g.colsum : nullptr);
         pa[0] = wimg.ptr;
         cpa = 8;
     } else {
@@ -1310,6 +1353,10 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     P.mode = MODE_WGRAD;
     P.kind = mi.kind;
     P.planes = mi.planes;
+    P.a_row_bytes = row_bytes;
+    P.b_row_bytes = 128;
+    P.a_cols_log2 = narrow ? 5 : 6;
+    P.ch_log2 = narrow ? 2 : 3;
     P.kb = mi.kb;
     P.a_mn_major = 1;
     P.b_mn_major = 1;
@@ -1348,7 +1395,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     // K blocks that do not waste much of the image, the other tensor fetched as grouped boxes.
     {
         const int groups = P.groups_total;
-        const int mt = ceil_div(groups, 2);
+        const int mt = ceil_div(groups, narrow ? 4 : 2);
         int dw_min = 0, dw_max = 0, dh_min = 0, dh_max = 0;
         for (int t = 0; t < P.n_taps; ++t) {
             dw_min = t ? std::min<int>(dw_min, P.taps[t].dw) : P.taps[t].dw;
@@ -1361,18 +1408,18 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         const double eff = static_cast<double>(g.plain_w) * g.plain_h / (1.0 * round_up(g.plain_w, 8) * round_up(g.plain_h, 8));
         if (tune().wpatch && mi.enc == ENC_F16 && P.c_blocks == 1 && groups >= 2 && mt <= 8 &&
             (window || g.s_w == 1) && bn_w >= 64 && cpb % 64 == 0 && pw_ <= 256 && ph_ <= 256 &&
-            pw_ * ph_ * 128 <= 40 * 1024 && eff >= 0.7) {
+            pw_ * ph_ * row_bytes <= 40 * 1024 && eff >= 0.7) {
             P.wpatch = 1;
             P.w_mtiles = mt;
             P.bn = std::min(bn_w, static_cast<int>(round_up(g.plain_c, 64)));
             P.n_tiles = ceil_div(g.plain_c, P.bn);
             P.patch_w = pw_;
             P.patch_h = ph_;
-            P.patch_bytes = static_cast<int>(round_up(pw_ * ph_ * 128, 1024));
+            P.patch_bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024));
             P.phases[0].org_w = static_cast<short>(dw_min);
             P.phases[0].org_h = static_cast<short>(dh_min);
             for (int t = 0; t < P.n_taps; ++t)
-                P.taps[t].aoff = ((P.taps[t].dh - dh_min) * pw_ + (P.taps[t].dw - dw_min)) * 128 / 16;
+                P.taps[t].aoff = ((P.taps[t].dh - dh_min) * pw_ + (P.taps[t].dw - dw_min)) * row_bytes / 16;
             P.wb_log2 = 3;
             P.hb_log2 = 3;
             P.nb_log2 = 0;
@@ -1467,10 +1514,10 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             aes[1] = aes[2] = 1;
         }
         if (window) {
-            uint64_t wd[4] = {64, static_cast<uint64_t>(g.plain_w), static_cast<uint64_t>(wimg.hp), static_cast<uint64_t>(g.batch)};
-            uint64_t wstr[3] = {static_cast<uint64_t>(g.s_w) * 16, static_cast<uint64_t>(wimg.wp) * 16,
-                                static_cast<uint64_t>(wimg.hp) * wimg.wp * 16};
-            uint32_t wbox[4] = {64, static_cast<uint32_t>(1 << P.wb_log2), static_cast<uint32_t>((1 << P.hb_log2) * g.s_h),
+            const uint64_t pix = 2ull * win_ch;
+            uint64_t wd[4] = {8ull * win_ch, static_cast<uint64_t>(g.plain_w), static_cast<uint64_t>(wimg.hp), static_cast<uint64_t>(g.batch)};
+            uint64_t wstr[3] = {g.s_w * pix, wimg.wp * pix, static_cast<uint64_t>(wimg.hp) * wimg.wp * pix};
+            uint32_t wbox[4] = {static_cast<uint32_t>(8 * win_ch), static_cast<uint32_t>(1 << P.wb_log2), static_cast<uint32_t>((1 << P.hb_log2) * g.s_h),
                                 static_cast<uint32_t>(1 << P.nb_log2)};
             uint32_t wes[4] = {1, 1, static_cast<uint32_t>(g.s_h), 1};
             if (P.wpatch) {
@@ -1479,7 +1526,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                 wbox[3] = 1;
                 wes[2] = 1;
             }
-            rc = encode_map(&P.tmA[pl], pa[pl], 2, 4, wd, wbox, wes, mn_swz, wstr);
+            rc = encode_map(&P.tmA[pl], pa[pl], 2, 4, wd, wbox, wes, narrow ? SWZ_64B : mn_swz, wstr);
         } else if (P.wpatch) {
             rc = encode_map(&P.tmA[pl], pa[pl], mi.es, 4, adims, abox, aes, mn_swz);
         } else if (cpa % mi.kb == 0 && P.c_blocks % G == 0) {

@@ -372,53 +372,61 @@ __global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __r
     }
 }
 
-// Few-channel activations (C <= 8, e.g. RGB stems): copy into a zero-padded NHWC image with exactly 8
-// fp16 channels per pixel, [N][Hp][Wp][8], the original at offset (pad_h, pad_w).  One thread per
-// padded pixel, one 16-byte store each.  A row of 8 consecutive pixels of this image is one 128-byte
-// K slice holding (kw, c) for 8 taps, which is what the small-channel contraction path reads.
-template <typename TIn>
-__global__ void __launch_bounds__(256) pad_pack_c8_kernel(const TIn* __restrict__ in, int nchw, __half* __restrict__ out,
-                                                          int N, int C, int H, int W, int pad_h, int pad_w, int Hp,
-                                                          int Wp, float* colsum) {
+// Few-channel activations (e.g. RGB stems): copy into a zero-padded NHWC image with exactly kCh (4 or 8) fp16 channels per
+// pixel, [N][Hp][Wp][kCh], the original at offset (pad_h, pad_w).  A row of 8 consecutive pixels of this image is one K
+// slice (64 or 128 bytes) holding (kw, c) for 8 taps, which is what the small-channel contraction path reads.
+// A warp takes a padded row at a time, four pixels per lane in flight; an index decoded with 64-bit divisions per
+// pixel ran at 2.1 TB/s.
+template <typename TIn, int kCh>
+__global__ void __launch_bounds__(256) pad_pack_kernel(const TIn* __restrict__ in, int nchw, __half* __restrict__ out,
+                                                       int N, int C, int H, int W, int pad_h, int pad_w, int Hp,
+                                                       int Wp, float* colsum) {
     pdl_enter();
-    const size_t total = static_cast<size_t>(N) * Hp * Wp;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // per-channel sums of the values read (bias gradient)
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const int wp = static_cast<int>(i % Wp);
-        const size_t r = i / Wp;
-        const int hp = static_cast<int>(r % Hp);
-        const int n = static_cast<int>(r / Hp);
-        const int h = hp - pad_h, w = wp - pad_w;
-        __half v[8];
+    struct alignas(2 * kCh) Pixel {
+        __half2 v[kCh / 2];
+    };
+    const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    const int rows = N * Hp;
+    const size_t px = nchw ? 1 : C, ch = nchw ? static_cast<size_t>(H) * W : 1;  // element strides of the source
+    float acc[kCh];  // per-channel sums of the values read (bias gradient)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] = __float2half_rn(0.f);
-        if (h >= 0 && h < H && w >= 0 && w < W) {
+    for (int c = 0; c < kCh; ++c) acc[c] = 0.f;
+    for (int r = blockIdx.x * 8 + wy; r < rows; r += gridDim.x * 8) {
+        const int n = r / Hp, h = r - n * Hp - pad_h;
+        const bool row_in = h >= 0 && h < H;
+        const TIn* src = in + (nchw ? (static_cast<size_t>(n) * C * H + h) * W : (static_cast<size_t>(n) * H + h) * W * C);
+        Pixel* dst = reinterpret_cast<Pixel*>(out) + static_cast<size_t>(r) * Wp;
+        for (int p0 = lane; p0 < Wp; p0 += 128) {
+            float v[4][kCh];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                if (c < C) {
-                    size_t src = nchw ? ((static_cast<size_t>(n) * C + c) * H + h) * W + w
-                                      : ((static_cast<size_t>(n) * H + h) * W + w) * C + c;
-                    const float xv = load_as_float(in, src);
-                    v[c] = __float2half_rn(xv);
-                    acc[c] += xv;  // the bias gradient sums the values as given, like every other column-sum path
-                }
+            for (int u = 0; u < 4; ++u) {
+                const int w = p0 + 32 * u - pad_w;
+                const bool inside = row_in && w >= 0 && w < W;
+#pragma unroll
+                for (int c = 0; c < kCh; ++c) v[u][c] = (c < C && inside) ? load_as_float(src, w * px + c * ch) : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                Pixel q;
+#pragma unroll
+                for (int c = 0; c < kCh; ++c) acc[c] += v[u][c];  // (the values as given, like every other column-sum path)
+#pragma unroll
+                for (int c = 0; c < kCh / 2; ++c) q.v[c] = __floats2half2_rn(v[u][2 * c], v[u][2 * c + 1]);
+                if (p0 + 32 * u < Wp) dst[p0 + 32 * u] = q;
             }
         }
-        reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(v);
     }
     if (colsum != nullptr) {  // uniform across the grid
         __shared__ float part[8][8];
-        const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < kCh; ++c) {
             float x = acc[c];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
             if (lane == 0) part[wy][c] = x;
         }
         __syncthreads();
-        if (threadIdx.x < 8) {  // row blockIdx.x of the [blocks][8] partial-sum matrix
+        if (threadIdx.x < kCh) {  // row blockIdx.x of the [blocks][8] partial-sum matrix
             float sum = 0.f;
 #pragma unroll
             for (int w8 = 0; w8 < 8; ++w8) sum += part[w8][threadIdx.x];
@@ -427,18 +435,18 @@ __global__ void __launch_bounds__(256) pad_pack_c8_kernel(const TIn* __restrict_
     }
 }
 
-// Weights [C_out][C][KH][KW] -> [C_out][KH][64] with k = kw*8 + c (zero where c >= C or kw >= KW):
-// the K-major operand matching pad_pack_c8's (kw, c) slices.
+// Weights [C_out][C][KH][KW] -> [C_out][KH][8 * ch] with k = kw * ch + c (zero where c >= C or kw >= KW):
+// the K-major operand matching pad_pack's (kw, c) slices.
 template <typename TIn>
-__global__ void __launch_bounds__(256) repack_weight_c8_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
-                                                               int Cout, int C, int KH, int KW) {
+__global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
+                                                                   int Cout, int C, int KH, int KW, int ch_log2) {
     pdl_enter();
-    const int total = Cout * KH * 64;
+    const int total = (Cout * KH) << (3 + ch_log2);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int k = i & 63;
-        const int kh = (i >> 6) % KH;
-        const int co = (i >> 6) / KH;
-        const int kw = k >> 3, c = k & 7;
+        const int k = i & ((8 << ch_log2) - 1);
+        const int row = i >> (3 + ch_log2);
+        const int kh = row % KH, co = row / KH;
+        const int kw = k >> ch_log2, c = k & ((1 << ch_log2) - 1);
         float v = 0.f;
         if (c < C && kw < KW) v = load_as_float(w, ((static_cast<size_t>(co) * C + c) * KH + kh) * KW + kw);
         out[i] = __float2half_rn(v);

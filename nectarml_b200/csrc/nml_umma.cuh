@@ -131,6 +131,9 @@ struct KParams {
     int patch;           // 1: patch walk
     int patch_w, patch_h;    // patch extent in pixels
     int patch_bytes;     // bytes one patch buffer occupies (multiple of 1024)
+    int a_row_bytes;     // bytes of one patch row: 128, or 64 in the narrow window walks (up to 4 image channels; 64-byte
+                         // swizzle, two MMAs per K slice instead of four)
+    int b_row_bytes;     // forward: bytes of one row of a weight slice, likewise
     int a_stages;        // patch buffers
     int b_resident;      // 1: every B slice of the launch is loaded once, at [pass plane][cb][tap] * bn * 128
     int issuers;         // resident patch walk: 2 = the B producer issues the odd tiles (needs a_stages >= tbufs * c_blocks)
@@ -153,7 +156,9 @@ struct KParams {
     int groups_total;    // taps * c_blocks column groups of kb patch channels
     int split_k, kblocks_total, ktiles_h, ktiles_w;
     int c_patch, c_plain, n_taps;
-    int kw_pack;         // wgrad, few-channel path: patch index j of a tap means (kw = j / 8, c = j % 8)
+    int a_cols_log2;     // wgrad patch walk: columns of one tap's group (64; 32 in the narrow window walk)
+    int ch_log2;         // few-channel path: channels per pixel of the padded image (8; 4 in the narrow walks)
+    int kw_pack;         // wgrad, few-channel path: patch index j of a tap means (kw = j >> ch_log2, c = the rest)
     int kw_count;        //   ... with kw_count valid kw per tap row; dW index = ((plain*C + c)*KH + kh)*KW + kw
     int m_fastest;       // wgrad tile order: consecutive CTAs share the plain operand's columns (re-read the smaller tensor)
     // epilogue
@@ -267,7 +272,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     const bool leader = (cta_rank == 0);
     const int tile_first = kPair ? (blockIdx.x >> 1) : blockIdx.x;
     const int tile_step = kPair ? (gridDim.x >> 1) : gridDim.x;
-    const int stage_b_bytes = (kPair ? P.bn / 2 : P.bn) * 128;   // one atom of B (a pair member holds half the columns)
+    const int stage_b_bytes = (kPair ? P.bn / 2 : P.bn) * P.b_row_bytes;   // one atom of B (a pair member holds half the columns)
     const int stage_bytes = P.ka * (kStageABytes + stage_b_bytes);  // [A atoms][B atoms]
     const int b_off = P.ka * kStageABytes;                        // first B atom within a stage
     uint8_t* staging = smem + P.ring_bytes;  // epilogue warps x 4 KB
@@ -354,8 +359,10 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         const uint32_t lbo_b = P.b_mn_major ? box_bytes : 16;
         const uint32_t adv_b = P.b_mn_major ? (((P.kind == KIND_F16) ? 16 : 8) * 128) >> 4 : 2;
         const uint32_t b_step = static_cast<uint32_t>(stage_b_bytes) >> 4;
-        const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h) * 128u;  // 8-row groups: one output row = a_stride_h patch rows apart
+        const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h * P.a_row_bytes);  // 8-row groups: one output row = a_stride_h patch rows apart
         const bool f16 = (P.kind == KIND_F16);
+        const bool narrow = P.a_row_bytes == 64;
+        const uint32_t layout_a = narrow ? 4 : 2;  // 64-byte or 128-byte swizzle
         if (!mbar_wait(smem_u32(bres_bar), 0, abort_flag, P.err, ERR_WAIT_FULL)) return;
         int titer = t_first;
         int p = 0;
@@ -379,8 +386,19 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (P.issuers == 2 && cb == 0 && titer > 0 &&
                     !mbar_wait(smem_u32(&turn_bar[t_first]), ((titer - 1) >> 1) & 1, abort_flag, P.err, ERR_WAIT_EMPTY)) return;
                 if (elect_one()) {
-                    const uint64_t adesc0 = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, 2);
-                    uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, lbo_b, b32 ? 512 : 1024, b32 ? 1 : 2);
+                    const uint64_t adesc0 = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, layout_a);
+                    uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, lbo_b,
+                                                    b32 ? 512 : 8 * P.b_row_bytes, b32 ? 1 : layout_a);
+                    if (narrow) {
+#pragma unroll 1
+                        for (int t = 0; t < nt; ++t) {
+                            const uint64_t adesc = adesc0 + static_cast<uint32_t>(tp[t].aoff);
+                            umma_f16(d_tmem, adesc, bdesc, idesc, acc);
+                            umma_f16(d_tmem, adesc + 2, bdesc + 2, idesc, 1u);
+                            acc = 1u;
+                            bdesc += b_step;
+                        }
+                    } else
 #pragma unroll 1
                     for (int t = 0; t < nt; ++t) {
                         const uint64_t adesc = adesc0 + static_cast<uint32_t>(tp[t].aoff);
@@ -468,7 +486,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             if (kMode == MODE_FPROP && !kPair && P.patch) {
                 if (do_a) {
                     const uint32_t a_base = smem_u32(smem + P.a_ring_off);
-                    const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * 128u;
+                    const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * P.a_row_bytes;
                     int abuf = 0;
                     uint32_t apar = 0;
                     int p = 0;
@@ -643,7 +661,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     int th = (kb_begin / P.ktiles_w) % P.ktiles_h;
                     int tn = kb_begin / (P.ktiles_w * P.ktiles_h);
                     const uint32_t w_stage = static_cast<uint32_t>(P.patch_bytes) + stage_b_bytes;
-                    const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * 128u;
+                    const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * P.a_row_bytes;
                     for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
                         if (!mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
                             ok = false;
@@ -904,15 +922,16 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 }
                 tc_fence_after();
                 const uint32_t w_stage = static_cast<uint32_t>(P.patch_bytes) + stage_b_bytes;
-                const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h) * 128u;  // next pixel row of the K block
-                // Row tile i = taps (2i, 2i+1): its descriptor relative to stage 0, built once (a 64-column MMA
+                const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h * P.a_row_bytes);  // next pixel row of the K block
+                // Row tile i = taps (2i, 2i+1), or 4i ... 4i+3 of the narrow window walk, evenly spaced: its descriptor relative to stage 0, built once (a 64-column MMA
                 // lasts 48 clocks: the K loop has no time to build descriptors).
                 uint64_t ad[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const int t0 = min(2 * i, P.groups_total - 1), t1 = min(2 * i + 1, P.groups_total - 1);
+                    const int first = i << (7 - P.a_cols_log2);
+                    const int t0 = min(first, P.groups_total - 1), t1 = min(first + 1, P.groups_total - 1);
                     const uint32_t a0 = static_cast<uint32_t>(P.taps[t0].aoff), a1 = static_cast<uint32_t>(P.taps[t1].aoff);
-                    ad[i] = make_smem_desc(smem_u32(smem) + (a0 << 4), (a1 - a0) << 4, sbo_a, 2);
+                    ad[i] = make_smem_desc(smem_u32(smem) + (a0 << 4), (a1 - a0) << 4, sbo_a, P.a_row_bytes == 64 ? 4 : 2);
                 }
                 const uint64_t bd0 = make_smem_desc(smem_u32(smem) + P.patch_bytes, box_bytes, 1024, 2);
                 const uint32_t a_step = (2u * sbo_a) >> 4;  // two pixel rows = 16 pixels = one MMA's K
@@ -1350,12 +1369,12 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         const int ncols = min(32, P.c_out - cg);
 #pragma unroll 1
                         for (int i = 0; i < P.w_mtiles; ++i) {
-                            const int gi = i * (kTileM / P.kb) + row / P.kb;
-                            const int pc = row % P.kb;
+                            const int gi = (i << (7 - P.a_cols_log2)) + (row >> P.a_cols_log2);
+                            const int pc = row & ((1 << P.a_cols_log2) - 1);
                             bool w_valid;
                             size_t w_off;
                             if (P.kw_pack) {
-                                const int kwi = pc >> 3, c = pc & 7;
+                                const int kwi = pc >> P.ch_log2, c = pc & ((1 << P.ch_log2) - 1);
                                 w_valid = (gi < P.groups_total) && (c < P.c_patch) && (kwi < P.kw_count);
                                 w_off = (static_cast<size_t>(c) * P.n_taps + gi) * P.kw_count + kwi;
                             } else {
@@ -1388,12 +1407,12 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 } else
 #pragma unroll 1
                 for (int i = 0; i < P.w_mtiles; ++i) {
-                    const int gi = i * (kTileM / P.kb) + row / P.kb;  // tap (kernel row with kw packing) of this row
-                    const int pc = row % P.kb;
+                    const int gi = (i << (7 - P.a_cols_log2)) + (row >> P.a_cols_log2);  // tap (kernel row with kw packing) of this row
+                    const int pc = row & ((1 << P.a_cols_log2) - 1);
                     bool w_valid;
                     size_t w_off, w_stride;
                     if (P.kw_pack) {
-                        const int kwi = pc >> 3, c = pc & 7;
+                        const int kwi = pc >> P.ch_log2, c = pc & ((1 << P.ch_log2) - 1);
                         w_valid = (gi < P.groups_total) && (c < P.c_patch) && (kwi < P.kw_count);
                         w_off = (static_cast<size_t>(c) * P.n_taps + gi) * P.kw_count + kwi;
                         w_stride = static_cast<size_t>(P.c_patch) * P.n_taps * P.kw_count;
@@ -1477,7 +1496,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 int pc = cib * P.kb + (row % P.kb);
                 if (P.kw_pack) {
                     // few-channel path: tap t is a kernel row kh, patch index pc packs (kw, c)
-                    const int kwi = pc >> 3, c = pc & 7;
+                    const int kwi = pc >> P.ch_log2, c = pc & ((1 << P.ch_log2) - 1);
                     row_valid = (gi < P.groups_total) && (c < P.c_patch) && (kwi < P.kw_count);
                     row_off = (static_cast<size_t>(c) * P.n_taps + t) * P.kw_count + kwi;
                     col_stride = static_cast<size_t>(P.c_patch) * P.n_taps * P.kw_count;

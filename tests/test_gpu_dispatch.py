@@ -87,3 +87,35 @@ def test_batch_norm_backward_with_and_without_y(rows, c, act, with_res):
     ops.device_status()
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("c,k,s,p,d,hw,c_out", [
+    (3, 7, 2, 3, 1, 37, 64), (4, 4, 2, 1, 1, 34, 64), (1, 5, 2, 2, 1, 33, 128), (3, 3, 2, 1, 1, 16, 192), (2, 2, 2, 0, 1, 32, 64),
+    (3, 8, 2, 3, 1, 40, 64), (3, 7, 4, 3, 1, 64, 96), (3, 7, 1, 3, 1, 24, 64), (5, 7, 2, 3, 1, 37, 64)])
+def test_few_channel_windows(c, k, s, p, d, hw, c_out, oracle):
+    """Image-like layers, four and eight channels per window pixel, through forward and weight gradient; the transposed layer
+    that produces such an image, through its weight gradient.  dw is summed over at most 2 * 64 * 64 fp16 products."""
+    rng = np.random.default_rng(c * 100 + k * 10 + s)
+    h, r = torch.float16, oracle.round_f16
+    g = ops.ConvGeometry(2, c, hw, hw, c_out, k, k, (s, s), (p, p), (d, d))
+    ho, wo = g.out_hw()
+    x = rng.standard_normal((2, c, hw, hw), dtype=np.float32)
+    w = (rng.standard_normal((c_out, c, k, k), dtype=np.float32) * 0.1).astype(np.float32)
+    b = rng.standard_normal(c_out, dtype=np.float32)
+    dy = rng.standard_normal((2, c_out, ho, wo), dtype=np.float32)
+    args = ((s, s), (p, p), (d, d))
+    y_o, dw_o, db_o = oracle.conv2d(r(x), r(w), r(b), *args), oracle.conv2d_backward_weight(r(dy), r(x), w.shape, *args), oracle.bias_grad(r(dy))
+    for layout in ("nhwc", "nchw"):
+        nhwc = layout == "nhwc"
+        xd, dyd = dev(x, h, nhwc=nhwc), dev(dy, h, nhwc=nhwc)
+        assert_f16(host(ops.conv_forward(g, xd, dev(w, h), dev(b, h), layout=layout), nhwc=nhwc), y_o, f"y {layout}")
+        dw, db = ops.conv_backward_weight(g, xd, dyd, layout=layout)
+        assert_f32(host(dw), dw_o, f"dw {layout}", tol=2e-5)
+        assert_f32(host(db), db_o, f"db {layout}", tol=2e-5)
+    assert_f16(host(ops.conv_forward(g, dev(x), dev(w), dev(b), math="f16")), y_o, "y, fp32 tensors")
+    # the transposed layer c_out -> c whose output gradient is the image
+    gt = ops.ConvGeometry(2, c_out, ho, wo, c, k, k, (s, s), (p, p), (d, d), (hw - ((ho - 1) * s - 2 * p + d * (k - 1) + 1),) * 2, True)
+    dw, db = ops.conv_backward_weight(gt, dev(dy, h, nhwc=True), dev(x, h, nhwc=True), layout="nhwc")
+    assert_f32(host(dw), oracle.conv_transpose2d_backward_weight(r(x), r(dy), (c_out, c, k, k), *args), "dw, transposed", tol=2e-5)
+    assert_f32(host(db), oracle.bias_grad(r(x)), "db, transposed", tol=2e-5)
+    ops.device_status()

@@ -1143,7 +1143,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     for (int p = 0; p < n_phases; ++p)
         if (P.phases[p].tap_count > 0) k_iters_all = std::min(k_iters_all, products * P.c_blocks * P.phases[p].tap_count);
     const bool pair_width = P.bn == 256 || (tune().pair128 && P.bn == 128 && k_iters_all >= 4 && tiles_single * 4 >= 3ll * limited(ds->sms));
-    P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && k_iters_min >= 4 &&
+    // Pairs save operand feed, which shows over a long K loop or many tiles: with 4 slices, or with 8 and one or two tiles per
+    // SM, single CTAs measured 3-14 % faster (they drain twice as many independent tiles).
+    const bool pair_k = k_iters_min >= 12 || (k_iters_min >= 5 && tiles_single > 2ll * limited(ds->sms));
+    P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && pair_k &&
               (P.out_mode == OUT_NHWC_TMA || P.out_mode == OUT_NCHW_TMA || P.out_mode == OUT_NCHW) && limited(ds->sms) >= 2) ? 1 : 0;
     int tiles = 0;
     for (int p = 0; p < n_phases; ++p) {
@@ -1428,19 +1431,19 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     P.ktiles_w = ceil_div(g.plain_w, 1 << P.wb_log2);
     P.ktiles_h = ceil_div(g.plain_h, 1 << P.hb_log2);
     P.kblocks_total = P.ktiles_w * P.ktiles_h * ceil_div(g.batch, 1 << P.nb_log2);
-    // Tile width and K split so that the CTAs finish together: the makespan is (rounds of tiles per CTA) x (K
-    // blocks per slice, plus a few blocks' worth of prologue / epilogue per tile), plus, for more than one slice,
-    // the second-stage reduction: it writes and re-reads one plane of dW per slice and then writes dW (~5 TB/s), plus its
-    // launch.  256-wide tiles whose operands both come as grouped boxes run as CTA pairs.  Narrower tiles are for gradients
-    // with few tiles over a short K (256 rows of a 2048 -> 1000 Linear layer: 64 tiles of 256 columns for 148 SMs).
+    // Tile width and K split so that the CTAs finish together.  Microseconds, measured over widths 64 / 128 / 256 and 1 ... 32
+    // slices on 18 layers: a K block costs the same at 64 and 128 columns (0.32; operand feed, not MMAs), little more as a
+    // 256-column CTA pair (0.36, 0.41 with the whole GPU busy); twice that for the 3xTF32 split's blocks of half the
+    // pixels.  A tile adds its prologue and drain, more than one slice (and any multi-tap gradient) the second-stage
+    // reduction, which writes and re-reads one plane of dW per slice and then writes dW, from L2 while the planes fit.
     const int G_ = kTileM / mi.kb;
     const bool a_grp = !window && (cpa % mi.kb == 0) && (P.c_blocks % G_ == 0);
     const bool b_grp = (cpb % mi.kb == 0);
     const int row_tiles = ceil_div(P.groups_total * mi.kb, kTileM);
     int split = 1, m_tiles = 1;
     if (!P.wpatch) {
-        const double dw_bytes = 4.0 * g.plain_c * g.patch_c * T;
-        const int max_split = std::min(P.kblocks_total, 64);
+        const double dw_us = 4.0 * g.plain_c * g.patch_c * T / 8e6;  // one pass over dW at 8 TB/s
+        const int max_split = std::min(P.kblocks_total, 192);
         double best = -1;
         for (int width = 256; width >= 64; width /= 2) {
             const int nt = ceil_div(g.plain_c, width);
@@ -1448,17 +1451,20 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             const bool pair = tune().pair && bn == 256 && a_grp && b_grp && sms >= 2;
             if ((width < 256 && bn > width) || (bn > 128 && P.planes == 2 && !pair)) continue;
             const int mt = pair ? ceil_div(row_tiles, 2) : row_tiles;
-            const double block_us = slice_us(bn) * (P.planes == 2 ? 3 : 1);
+            const int units = pair ? sms / 2 : sms;
             for (int sp = 1; sp <= max_split; ++sp) {
-                int per_sp = ceil_div(P.kblocks_total, sp);
+                const long long tiles = 1ll * mt * nt * sp;
+                if (best >= 0 && sp > 1 && tiles > 3ll * units) break;
+                const int per_sp = ceil_div(P.kblocks_total, sp);
+                // every slice gets at least one K block: the next split that leaves each one block less
+                if (ceil_div(P.kblocks_total, per_sp) != sp) continue;
                 // the tensor core truncates as it accumulates: at most 4096 terms per sum of the 3xTF32 split
                 if (P.planes == 2 && per_sp * mi.kb > 4096 && sp < max_split) continue;
-                int real = ceil_div(P.kblocks_total, per_sp);  // every slice gets at least one K block
-                if (real != sp) continue;
-                long long rounds = ceil_div(mt * nt * sp, pair ? sms / 2 : sms);
-                double cost = rounds * (per_sp + 4) * block_us;
-                if (sp > 1 || T > 1) cost += 3.0 + (2.0 * sp + 1.0) * dw_bytes / 5e6;
-                if (best < 0 || cost < best * (width == 256 ? 1.0 : 0.95)) {  // the wider tile unless the gain is clear
+                const double block_us = (pair ? (tiles * 8 >= units * 7ll ? 0.41 : 0.36) : 0.32) * (P.planes == 2 ? 2.3 : 1.0);
+                const double rounds = static_cast<double>((tiles + units - 1) / units);
+                double cost = rounds * (per_sp * block_us + 1.0 + bn / 128.0);
+                if (sp > 1 || T > 1) cost += 2.5 + (2.0 * sp + 1.0) * dw_us * (sp * dw_us > 8.0 ? 1.6 : 1.0);
+                if (best < 0 || cost < best * (width == 256 ? 1.0 : 0.98)) {
                     best = cost;
                     split = sp;
                     m_tiles = mt;

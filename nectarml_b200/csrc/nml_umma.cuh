@@ -366,6 +366,17 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         if (!mbar_wait(smem_u32(bres_bar), 0, abort_flag, P.err, ERR_WAIT_FULL)) return;
         int titer = t_first;
         int p = 0;
+        // the patch buffer of this issuer's next patch and its parity, by counting (patches are consumed in tile order)
+        int pstage = 0;
+        uint32_t pparity = 0;
+        auto skip = [&](int patches) {
+            pstage += patches;
+            while (pstage >= P.a_stages) {
+                pstage -= P.a_stages;
+                pparity ^= 1;
+            }
+        };
+        skip(t_first * P.c_blocks);
         for (int tile = tile_first + t_first * tile_step; tile < P.num_tiles; tile += t_step * tile_step, titer += t_step) {
             while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
             const Tap* tp = &P.taps[P.phases[p].tap_begin];
@@ -378,9 +389,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             const uint32_t d_tmem = tmem_base + buf * P.bn;
             uint32_t acc = 0;
             for (int cb = 0; cb < P.c_blocks; ++cb) {
-                const int pi = titer * P.c_blocks + cb;  // patches are consumed in tile order
-                const int pstage = pi % P.a_stages;
-                const uint32_t pparity = (pi / P.a_stages) & 1;
                 if (!mbar_wait(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) return;
                 tc_fence_after();
                 if (P.issuers == 2 && cb == 0 && titer > 0 &&
@@ -389,19 +397,25 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     const uint64_t adesc0 = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, layout_a);
                     uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, lbo_b,
                                                     b32 ? 512 : 8 * P.b_row_bytes, b32 ? 1 : layout_a);
-                    if (narrow) {
-#pragma unroll 1
+                    // (the next tap's offset is fetched while this one's MMAs are issued: a constant load per tap in the chain
+                    // costs as much as a narrow tap's MMAs)
+                    uint32_t off = static_cast<uint32_t>(tp[0].aoff);
+                    if (narrow) {  // kernel rows, evenly spaced
+                        const uint32_t a_step = nt > 1 ? static_cast<uint32_t>(tp[1].aoff) - off : 0u;
+                        uint64_t adesc = adesc0 + off;
+#pragma unroll 4
                         for (int t = 0; t < nt; ++t) {
-                            const uint64_t adesc = adesc0 + static_cast<uint32_t>(tp[t].aoff);
                             umma_f16(d_tmem, adesc, bdesc, idesc, acc);
                             umma_f16(d_tmem, adesc + 2, bdesc + 2, idesc, 1u);
                             acc = 1u;
+                            adesc += a_step;
                             bdesc += b_step;
                         }
                     } else
 #pragma unroll 1
                     for (int t = 0; t < nt; ++t) {
-                        const uint64_t adesc = adesc0 + static_cast<uint32_t>(tp[t].aoff);
+                        const uint64_t adesc = adesc0 + off;
+                        off = static_cast<uint32_t>(tp[min(t + 1, nt - 1)].aoff);
                         if (f16) {
                             umma_f16(d_tmem, adesc, bdesc, idesc, acc);
                             umma_f16(d_tmem, adesc + 2, bdesc + adv_b, idesc, 1u);
@@ -418,13 +432,16 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     }
                     umma_commit(smem_u32(&aempty_bar[pstage]));
                     if (cb + 1 == P.c_blocks) {
-                        if (P.issuers == 2) mbar_arrive(smem_u32(&turn_bar[t_first ^ 1]));
                         umma_commit(smem_u32(&tfull_bar[buf]));
+                        // (after the commits: one issued behind the other warp's MMAs waits for room on the pipe)
+                        if (P.issuers == 2) mbar_arrive(smem_u32(&turn_bar[t_first ^ 1]));
                     }
                 }
                 acc = 1u;
+                skip(1);
                 __syncwarp();
             }
+            skip((t_step - 1) * P.c_blocks);
         }
     };
 
@@ -849,10 +866,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 }
             }
         }
-        if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident && P.issuers == 2 && warp == 6) {
-            __syncwarp();
-            patch_resident_issue(1, 2);  // the weights are in: help with the odd tiles
-        }
     }
     // ---------------------------------------------------------- MMA issuer --
     else if (warp == 1) {
@@ -881,7 +894,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         bool ok = true;
         int titer = 0;
         if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident) {
-            patch_resident_issue(0, P.issuers);
+            // (issued below, by one copy of the loop for both issuers)
         } else
         for (int tile_id = tile_first; ok && (!kPair || leader) && tile_id < P.num_tiles; tile_id += tile_step, ++titer) {
             int tile = tile_id, kz = 0;
@@ -1858,6 +1871,11 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 else mbar_arrive(smem_u32(&tempty_bar[buf]));
             }
         }
+    }
+
+    if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident && (warp == 1 || (warp == 6 && P.issuers == 2))) {
+        __syncwarp();  // (warp 6 comes from a loop that one lane ran)
+        patch_resident_issue(warp == 6 ? 1 : 0, P.issuers);
     }
 
     // ------------------------------------------------------------ teardown --

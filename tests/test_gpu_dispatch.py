@@ -90,7 +90,7 @@ def test_batch_norm_backward_with_and_without_y(rows, c, act, with_res):
 
 
 @pytest.mark.parametrize("c,k,s,p,d,hw,c_out", [
-    (3, 7, 2, 3, 1, 37, 64), (4, 4, 2, 1, 1, 34, 64), (1, 5, 2, 2, 1, 33, 128), (3, 3, 2, 1, 1, 16, 192), (2, 2, 2, 0, 1, 32, 64),
+    (3, 7, 2, 3, 1, 37, 64), (3, 7, 2, 3, 1, 64, 64), (3, 3, 1, 1, 1, 16, 48), (7, 5, 1, 2, 1, 32, 64), (4, 4, 2, 1, 1, 34, 64), (1, 5, 2, 2, 1, 33, 128), (3, 3, 2, 1, 1, 16, 192), (2, 2, 2, 0, 1, 32, 64),
     (3, 8, 2, 3, 1, 40, 64), (3, 7, 4, 3, 1, 64, 96), (3, 7, 1, 3, 1, 24, 64), (5, 7, 2, 3, 1, 37, 64)])
 def test_few_channel_windows(c, k, s, p, d, hw, c_out, oracle):
     """Image-like layers, four and eight channels per window pixel, through forward and weight gradient; the transposed layer
@@ -119,3 +119,21 @@ def test_few_channel_windows(c, k, s, p, d, hw, c_out, oracle):
     assert_f32(host(dw), oracle.conv_transpose2d_backward_weight(r(x), r(dy), (c_out, c, k, k), *args), "dw, transposed", tol=2e-5)
     assert_f32(host(db), oracle.bias_grad(r(x)), "db, transposed", tol=2e-5)
     ops.device_status()
+
+
+@pytest.mark.parametrize("rows,fin,fout,math", [
+    (5541, 1776, 1008, "3xtf32"), (4128, 2064, 1000, "3xtf32"), (4096, 512, 2048, "f16"), (33, 64, 64, "f16"), (700, 200, 72, "f16"),
+    (700, 200, 72, "3xtf32"), (9000, 256, 256, "f16")])
+def test_weight_gradient_plans(rows, fin, fout, math):
+    """Tile width, pairs and K split of the weight gradient, against float64: every element within the rounding of a sum over
+    `rows` products (fp32 accumulation: 2.5e-9 of the sum of magnitudes per term and accumulator, 4096 terms at most)."""
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    dt = torch.float16 if math == "f16" else torch.float32
+    x = torch.randn(rows, fin, device="cuda", generator=gen).to(dt)
+    dy = torch.randn(rows, fout, device="cuda", generator=gen).to(dt)
+    dw, db = ops.linear_backward_weight(x, dy, math=math)
+    ops.device_status()
+    want = dy.double().T @ x.double()
+    assert float((dw.double() - want).norm() / want.norm()) < 2e-5
+    assert float((dw.double() - want).abs().max()) < 1e-4 * rows ** 0.5
+    assert float((db.double() - dy.double().sum(0)).abs().max()) < 1e-5 * rows ** 0.5 * 10

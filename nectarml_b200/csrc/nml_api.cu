@@ -300,6 +300,21 @@ static bool math_info(int math, MathInfo* m) {
     return false;
 }
 
+// Role (see nml_launch.cuh) of this thread's next helper launch; it falls back to PDL_NORMAL with that launch.
+static thread_local int t_role = PDL_NORMAL;
+template <typename... P, typename... A>
+static void helper_launch(unsigned single_wave_limit, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+    const int role = t_role;
+    t_role = PDL_NORMAL;
+    launch_with(role == PDL_SIBLING || overlaps(grid, single_wave_limit), 1, kernel, grid, block, smem, st, static_cast<A&&>(args)..., role);
+}
+// The helper launch after this one runs beside it, if both are made.
+struct SideBySide {
+    SideBySide() { t_role = PDL_LEADER; }
+    void second() { t_role = t_role == PDL_NORMAL ? PDL_SIBLING : PDL_NORMAL; }  // (the leader's role is used up once it was launched)
+    ~SideBySide() { t_role = PDL_NORMAL; }
+};
+
 // Bias gradient = column sums of dY, in two stages so that the result is bitwise repeatable: the pass
 // that reads dY writes rows of partial sums ([P][stride], one row per block), colsum_finish_kernel adds
 // the rows in a fixed order.  Both scratch matrices come from the workspace.
@@ -323,7 +338,7 @@ static int colsum_finish(const ColsumScratch& cs, int C, float* out, cudaStream_
     for (;;) {
         const int S = ceil_div(P, kColsumSegment);
         float* dst = (S == 1) ? out : (src == cs.partial ? cs.second : cs.partial);
-        launch_short(colsum_finish_kernel, dim3(ceil_div(C, 8), S), dim3(8, 128), 0, st, src, P, stride, C, dst, cs.stride, kColsumSegment);
+        helper_launch(4 * kSms, colsum_finish_kernel, dim3(ceil_div(C, 8), S), dim3(8, 128), 0, st, src, P, stride, C, dst, cs.stride, kColsumSegment);
         ++g_launches;
         if (S == 1) break;
         src = dst;
@@ -336,8 +351,8 @@ static int colsum_finish(const ColsumScratch& cs, int C, float* out, cudaStream_
 
 static void convert_rows(const void* src, int dtype, void* p0, void* p1, int enc, size_t rows, int c, int cp, cudaStream_t st) {
     const int blocks = static_cast<int>(std::min<size_t>((rows * (cp / 4) + 255) / 256, 148 * 16));
-    if (dtype == NML_F32) launch_short(convert_rows_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(src), p0, p1, enc, rows, c, cp);
-    else launch_short(convert_rows_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(src), p0, p1, enc, rows, c, cp);
+    if (dtype == NML_F32) helper_launch(4 * kSms, convert_rows_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(src), p0, p1, enc, rows, c, cp);
+    else helper_launch(4 * kSms, convert_rows_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(src), p0, p1, enc, rows, c, cp);
     ++g_launches;
 }
 
@@ -348,54 +363,74 @@ static bool repack_half(const void* src, void* dst, int B, int R, int Cc, int Rp
     if ((reinterpret_cast<uintptr_t>(src) & 15) || Rp % 8) return false;
     if (Cc > 64) {
         if (Cc % 8) return false;
-        launch_short(repack_half_tile_kernel, dim3(ceil_div(Cc, 64), ceil_div(Rp, 64), B), 256, 0, st, w, o, R, Cc, Rp);
+        helper_launch(4 * kSms, repack_half_tile_kernel, dim3(ceil_div(Cc, 64), ceil_div(Rp, 64), B), 256, 0, st, w, o, R, Cc, Rp);
     } else {
         if ((static_cast<size_t>(R) * Cc) % 8) return false;
-        launch_short(repack_half_rows_kernel, dim3(ceil_div(Rp, 256), B), 256, 256 * (Cc | 1) * sizeof(__half), st, w, o, R, Cc, Rp);
+        helper_launch(4 * kSms, repack_half_rows_kernel, dim3(ceil_div(Rp, 256), B), 256, 256 * (Cc | 1) * sizeof(__half), st, w, o, R, Cc, Rp);
     }
     ++g_launches;
     return true;
 }
 
+// Column sums of a row-major matrix: the first stage's launch, its scratch, and where the sums go.
+struct RowsColsum {
+    const void* src = nullptr;
+    int dtype = 0, c = 0, rows_per_block = 0;
+    bool vectors = false;
+    size_t pixels = 0;
+    dim3 grid;
+    ColsumScratch cs;
+    float* out = nullptr;  // null: nothing to do
+    void plan(const void* s, int dt, size_t px, int ch, float* o) {
+        src = s; dtype = dt; pixels = px; c = ch; out = o;
+        // enough row blocks to fill the GPU, few enough that the second stage stays negligible
+        // (the width of a column block has to follow from the shape alone: workspace queries pass no pointer)
+        const int vector = dtype == NML_F16 ? 8 : 4;
+        const int col_blocks = ceil_div(c, c % vector == 0 ? 32 * vector : 256);
+        vectors = c % vector == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+        rows_per_block = static_cast<int>(std::max<size_t>(64, round_up(ceil_div(static_cast<int>(std::min<size_t>(pixels, 1u << 30)), std::max(1, 1184 / col_blocks)), 8)));
+        grid = dim3(col_blocks, static_cast<unsigned>((pixels + rows_per_block - 1) / rows_per_block));
+    }
+    void first_stage(cudaStream_t st) const {
+        if (dtype == NML_F16) {
+            auto k = vectors ? colsum_vectors_kernel<__half> : colsum_rows_kernel<__half>;
+            helper_launch(kSms, k, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
+        } else {
+            auto k = vectors ? colsum_vectors_kernel<float> : colsum_rows_kernel<float>;
+            helper_launch(kSms, k, grid, 256, 0, st, static_cast<const float*>(src), cs.partial, pixels, c, rows_per_block);
+        }
+        ++g_launches;
+    }
+    int second_stage(cudaStream_t st) const { return colsum_finish(cs, c, out, st); }
+};
+
 // Converts an activation tensor into the NHWC operand encoding of `mi` unless it already is one.
 // planes[0..1] receive the operand pointers, *cp the padded channel count.  With `colsum` the
-// per-channel sums of the tensor (the bias gradient) are produced in the same pass where there is one.
+// per-channel sums of the tensor (the bias gradient) are produced in the same pass where there is one; for a tensor used
+// in place the caller may take them over (`later`) and run them beside the contraction.
 static int prepare_activation(const void* src, int dtype, int layout, int batch, int c, int h, int w,
                               const MathInfo& mi, Bump& ws, cudaStream_t st, const void* planes[2], int* cp,
-                              float* colsum) {
+                              float* colsum, RowsColsum* later = nullptr) {
     const int align = 16 / mi.es;
     const bool direct = (mi.enc == ENC_F16) && dtype == NML_F16 && (c % align == 0) &&
                         (layout == NML_NHWC || (h == 1 && w == 1) || c == 1);
     const size_t pixels = static_cast<size_t>(batch) * h * w;
-    // row-major column sums: enough row blocks to fill the GPU, few enough that the second stage stays negligible
-    // (the width of a column block has to follow from the shape alone: workspace queries pass no pointer)
-    const int vector = dtype == NML_F16 ? 8 : 4;
-    const int col_blocks = ceil_div(c, c % vector == 0 ? 32 * vector : 256);
-    const bool vectors = c % vector == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-    const int rows_per_block = static_cast<int>(std::max<size_t>(64, round_up(ceil_div(static_cast<int>(std::min<size_t>(pixels, 1u << 30)), std::max(1, 1184 / col_blocks)), 8)));
-    const size_t row_blocks = (pixels + rows_per_block - 1) / rows_per_block;
-    auto rows_colsum = [&](const ColsumScratch& cs) -> int {
-        dim3 grid(col_blocks, static_cast<unsigned>(row_blocks));
-        if (dtype == NML_F16 && vectors)
-            launch(colsum_vectors_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
-        else if (vectors)
-            launch(colsum_vectors_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), cs.partial, pixels, c, rows_per_block);
-        else if (dtype == NML_F16)
-            launch(colsum_rows_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), cs.partial, pixels, c, rows_per_block);
-        else
-            launch(colsum_rows_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), cs.partial, pixels, c, rows_per_block);
-        ++g_launches;
-        return colsum_finish(cs, c, colsum, st);
-    };
+    RowsColsum rows;
+    rows.plan(src, dtype, pixels, c, colsum);
     if (direct) {
         planes[0] = src;
         planes[1] = nullptr;
         *cp = c;
         if (colsum) {
-            ColsumScratch cs = colsum_scratch(ws, row_blocks, c);
+            rows.cs = colsum_scratch(ws, rows.grid.y, c);
             if (ws.dry) return NML_OK;
             if (!ws.fits()) return NML_ERR_WORKSPACE;
-            return rows_colsum(cs);
+            if (later) {
+                *later = rows;
+                return NML_OK;
+            }
+            rows.first_stage(st);
+            return rows.second_stage(st);
         }
         return NML_OK;
     }
@@ -407,16 +442,16 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
     planes[1] = p1;
     const bool transposing = layout == NML_NCHW && !(h == 1 && w == 1);
     ColsumScratch cs;
-    if (colsum) cs = transposing ? colsum_scratch(ws, static_cast<size_t>(batch) * ceil_div(h * w, 64), c) : colsum_scratch(ws, row_blocks, c);
+    if (colsum) cs = transposing ? colsum_scratch(ws, static_cast<size_t>(batch) * ceil_div(h * w, 64), c) : colsum_scratch(ws, rows.grid.y, c);
     if (ws.dry) return NML_OK;
     if (!ws.fits()) return NML_ERR_WORKSPACE;
     if (transposing) {
         dim3 grid(ceil_div(h * w, 64), ceil_div(Cp, 64), batch);
         if (dtype == NML_F32)
-            { launch(nchw_to_nhwc_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), p0, p1, mi.enc, c, Cp,
+            { helper_launch(kSms, nchw_to_nhwc_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), p0, p1, mi.enc, c, Cp,
                                                             h * w, cs.partial); ++g_launches; }
         else
-            { launch(nchw_to_nhwc_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), p0, p1, mi.enc, c,
+            { helper_launch(kSms, nchw_to_nhwc_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), p0, p1, mi.enc, c,
                                                              Cp, h * w, cs.partial); ++g_launches; }
         if (colsum) {
             int rc = colsum_finish(cs, c, colsum, st);
@@ -425,7 +460,9 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
     } else {
         convert_rows(src, dtype, p0, p1, mi.enc, pixels, c, Cp, st);
         if (colsum) {
-            int rc = rows_colsum(cs);
+            rows.cs = cs;
+            rows.first_stage(st);
+            int rc = rows.second_stage(st);
             if (rc) return rc;
         }
     }
@@ -458,7 +495,7 @@ static int prepare_window(const void* src, int dtype, int layout, int batch, int
     if (!ws.fits()) return NML_ERR_WORKSPACE;
     const int nchw = (layout == NML_NCHW) ? 1 : 0;
     auto run = [&](auto kernel, auto* in) {
-        launch(kernel, blocks, 256, 0, st, in, nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial);
+        helper_launch(kSms, kernel, blocks, 256, 0, st, in, nchw, static_cast<__half*>(p), batch, c, h, w, p_h, p_w, img->hp, img->wp, cs.partial);
     };
     if (dtype == NML_F32) run(ch == 4 ? pad_pack_kernel<float, 4> : pad_pack_kernel<float, 8>, static_cast<const float*>(src));
     else run(ch == 4 ? pad_pack_kernel<__half, 4> : pad_pack_kernel<__half, 8>, static_cast<const __half*>(src));
@@ -727,7 +764,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                 const int total = np * Kc * khp * kwp;
                 const int blocks = std::min(ceil_div(total, 256), 148 * 8);
 #define NML_PACK(TW, TB)                                                                                            \
-    launch_short(pack_phase_weights_kernel<TW, TB>, blocks, 256, 0, st, static_cast<const TW*>(f.w), wp,                      \
+    helper_launch(4 * kSms, pack_phase_weights_kernel<TW, TB>, blocks, 256, 0, st, static_cast<const TW*>(f.w), wp,                      \
                                                               static_cast<const TB*>(f.bias), bp, Kc, C, f.kh, f.kw, \
                                                               f.s_h, f.s_w, f.p_h, f.p_w, khp, kwp, dh_min, dw_min)
                 if (f.w_dtype == NML_F32) {
@@ -773,6 +810,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     const void* a_planes[2] = {nullptr, nullptr};
     int Cp = 0;
     int rc;
+    SideBySide operands;  // the two conversions do not depend on one another
     if (window)
         rc = prepare_window(f.a, f.a_dtype, f.a_layout, f.batch, f.a_c, f.a_h, f.a_w, f.p_h, f.p_w, f.s_w, f.out_w, win_ch, ws, st,
                             &wimg);
@@ -781,6 +819,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                                 nullptr);
     if (rc) return rc;
     if (window) a_planes[0] = wimg.ptr;
+    operands.second();
     // weight operand
     const int c_blocks = window ? 1 : ceil_div(K, mi.kb);
     const int kp = c_blocks * mi.kb;
@@ -796,9 +835,9 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             if (!ws.fits()) return NML_ERR_WORKSPACE;
             const int blocks = std::min(ceil_div(N * f.kh * 8 * win_ch, 256), 148 * 8);
             if (f.w_dtype == NML_F32)
-                launch_short(repack_weight_window_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw, narrow ? 2 : 3);
+                helper_launch(4 * kSms, repack_weight_window_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw, narrow ? 2 : 3);
             else
-                launch_short(repack_weight_window_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw, narrow ? 2 : 3);
+                helper_launch(4 * kSms, repack_weight_window_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(f.w), static_cast<__half*>(p0), N, K, f.kh, f.kw, narrow ? 2 : 3);
             ++g_launches;
             NML_CUDA(cudaGetLastError());
         }
@@ -822,10 +861,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
 #define NML_REPACK(T)                                                                                                           \
     do {                                                                                                                        \
         if (rC <= 64)                                                                                                           \
-            launch_short(repack_weight_rows_kernel<T>, dim3(ceil_div(kp, 64), rB), 256, 0, st, static_cast<const T*>(f.w), p0, p1, mi.enc, \
+            helper_launch(4 * kSms, repack_weight_rows_kernel<T>, dim3(ceil_div(kp, 64), rB), 256, 0, st, static_cast<const T*>(f.w), p0, p1, mi.enc, \
                                                                                      rR, rC, kp);                               \
         else                                                                                                                    \
-            launch_short(repack_weight_tile_kernel<T>, dim3(ceil_div(rC, 64), ceil_div(kp, 64), rB), 256, 0, st,                           \
+            helper_launch(4 * kSms, repack_weight_tile_kernel<T>, dim3(ceil_div(rC, 64), ceil_div(kp, 64), rB), 256, 0, st,                           \
                 static_cast<const T*>(f.w), p0, p1, mi.enc, rR, rC, kp);                                                         \
     } while (0)
             if (rows_only) convert_rows(f.w, f.w_dtype, p0, p1, mi.enc, static_cast<size_t>(rB) * f.d0, f.d1, kp, st);
@@ -838,6 +877,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             NML_CUDA(cudaGetLastError());
         }
     }
+    t_role = PDL_NORMAL;
     // Bias as fp32: the TMA-store epilogues read an fp16 bias as it is (they stage the tile's bias values in
     // shared memory once per column tile anyway); the other epilogues and the finishing pass of a K-split walk
     // take a widened copy, made just before the launch once the plan is known.
@@ -1267,7 +1307,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             P.bias = static_cast<const float*>(f.bias);  // read as __half by the kernel
             P.bias_f16 = 1;
         } else {
-            launch_short(to_float_kernel<__half>, ceil_div(N, 256), 256, 0, st, static_cast<const __half*>(f.bias), bias_widened, N);
+            helper_launch(4 * kSms, to_float_kernel<__half>, ceil_div(N, 256), 256, 0, st, static_cast<const __half*>(f.bias), bias_widened, N);
             ++g_launches;
         }
     }
@@ -1281,10 +1321,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const int nchw = (f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1)) ? 1 : 0;
         const int vec = (!nchw && N % 4 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0) ? 1 : 0;
         if (f.out_dtype == NML_F16)
-            { launch_short(finish_rows_kernel<__half>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<__half*>(f.out), out_pixels, N,
+            { helper_launch(4 * kSms, finish_rows_kernel<__half>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<__half*>(f.out), out_pixels, N,
                                                               f.out_h * f.out_w, nchw, 0, vec); ++g_launches; }
         else
-            { launch_short(finish_rows_kernel<float>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
+            { helper_launch(4 * kSms, finish_rows_kernel<float>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
                                                              f.out_h * f.out_w, nchw, f.round_f16, vec); ++g_launches; }
         NML_CUDA(cudaGetLastError());
     }
@@ -1337,6 +1377,13 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     const int win_ch = narrow ? 4 : 8, row_bytes = narrow ? 64 : 128;
     WindowImage wimg = {nullptr, 0, 0};
     int rc;
+    // (the two conversions do not depend on one another; column sums taken with the first would stand between them)
+    SideBySide operands;
+    if (g.colsum && g.colsum_of_patch) t_role = PDL_NORMAL;
+    RowsColsum later;
+    // Column sums of a tensor used in place run beside the contraction and its reduction (on the SMs these leave, or as
+    // their CTAs finish) -- not while launches are being timed, which would count them in.
+    RowsColsum* const defer = g_prof.on.load(std::memory_order_relaxed) ? nullptr : &later;
     if (window) {
         rc = prepare_window(g.patch, g.dtype, g.layout, g.batch, g.patch_c, g.patch_h, g.patch_w, g.p_h, g.p_w, g.s_w,
                             g.plain_w, win_ch, ws, st, &wimg, g.colsum_of_patch ? g.colsum : nullptr);
@@ -1344,12 +1391,14 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         cpa = 8;
     } else {
         rc = prepare_activation(g.patch, g.dtype, g.layout, g.batch, g.patch_c, g.patch_h, g.patch_w, mi, ws, st, pa,
-                                &cpa, g.colsum_of_patch ? g.colsum : nullptr);
+                                &cpa, g.colsum_of_patch ? g.colsum : nullptr, defer);
     }
     if (rc) return rc;
+    if (!(g.colsum && g.colsum_of_patch)) operands.second();
     rc = prepare_activation(g.plain, g.dtype, g.layout, g.batch, g.plain_c, g.plain_h, g.plain_w, mi, ws, st, pb, &cpb,
-                            g.colsum_of_patch ? nullptr : g.colsum);
+                            g.colsum_of_patch ? nullptr : g.colsum, defer);
     if (rc) return rc;
+    t_role = PDL_NORMAL;
 
     KParams P;
     memset(&P, 0, sizeof(P));
@@ -1566,31 +1615,43 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         if (rc) return rc;
     }
     int slot = -1;
+    P.pdl_role = later.out ? PDL_LEADER : PDL_NORMAL;
     rc = launch_kernel(P, ds, st, &slot);
     if (rc) return rc;
+    if (later.out) {
+        t_role = PDL_SIBLING;
+        later.first_stage(st);
+        if (staged) t_role = PDL_LEADER;  // the planes' reduction, with the sums' second stage beside it
+    }
     if (staged) {
         const bool vec_ok = (reinterpret_cast<uintptr_t>(g.dw) & 15) == 0;
         if (P.wpatch && vec_ok && dw_elems % 4 == 0 && split > 8) {
             const size_t total4 = dw_elems / 4;
-            launch_short(wgrad_reduce_deep4_kernel, static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st, planes, g.dw, split, plane_elems, total4);
+            helper_launch(4 * kSms, wgrad_reduce_deep4_kernel, static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st, planes, g.dw, split, plane_elems, total4);
         } else if (P.wpatch && vec_ok && dw_elems % 4 == 0) {
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems / 4 + 255) / 256, 148 * 8));
-            launch_short(wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, 1, static_cast<int>(dw_elems / 4), 0);
+            helper_launch(4 * kSms, wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, 1, static_cast<int>(dw_elems / 4), 0);
         } else if (!P.wpatch && !P.kw_pack && T == 1 && vec_ok && g.patch_c % 4 == 0) {
             const size_t total4 = dw_elems / 4;
             const int blocks = static_cast<int>(std::min<size_t>((total4 + 255) / 256, 148 * 16));
-            launch_short(wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
+            helper_launch(4 * kSms, wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
         } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535) {
-            launch_short(wgrad_reduce_taps_kernel, dim3(ceil_div(g.patch_c, 64), g.plain_c), 256, 64 * (P.n_taps | 1) * sizeof(float), st,
+            helper_launch(4 * kSms, wgrad_reduce_taps_kernel, dim3(ceil_div(g.patch_c, 64), g.plain_c), 256, 64 * (P.n_taps | 1) * sizeof(float), st,
                          planes, g.dw, split, plane_elems, g.patch_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
         } else {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + 255) / 256, 148 * 16));
-            launch_short(wgrad_reduce_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, dw_elems, layout, g.patch_c, P.n_taps,
+            helper_launch(4 * kSms, wgrad_reduce_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, dw_elems, layout, g.patch_c, P.n_taps,
                                                         P.kw_count, P.c_blocks, mi.kb, plane_rows);
         }
         ++g_launches;
         NML_CUDA(cudaGetLastError());
+    }
+    if (later.out) {
+        t_role = staged ? PDL_SIBLING : PDL_NORMAL;
+        rc = later.second_stage(st);
+        t_role = PDL_NORMAL;
+        if (rc) return rc;
     }
     return profile_stop(slot, st);
 }
@@ -1702,7 +1763,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
             if (rc) return rc;
             if (!repack_half(in1, wt, 1, d->out_features, d->in_features, d->out_features, st)) {
                 const dim3 grid(ceil_div(d->in_features, 64), ceil_div(d->out_features, 64), 1);
-                launch_short(repack_weight_tile_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in1), wt, nullptr, ENC_F16,
+                helper_launch(4 * kSms, repack_weight_tile_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in1), wt, nullptr, ENC_F16,
                              d->out_features, d->in_features, d->out_features);
                 ++g_launches;
             }

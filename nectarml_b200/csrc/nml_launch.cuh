@@ -20,6 +20,21 @@ __device__ __forceinline__ void pdl_enter() {
     cudaGridDependencySynchronize();
 }
 
+// Two neighbours in a stream that do not depend on one another (the conversions of a pass's two operands, a
+// contraction and the column sums of one of its operands) run side by side as a leader and a sibling.  The leader lets
+// the sibling start only after its own wait, so everything in front of the leader is over when the sibling starts
+// working without a wait; the sibling waits at its end, so that it ends after the leader and whoever waits for the
+// sibling has waited for both.  The sibling is always launched as an overlapping grid.
+enum { PDL_NORMAL = 0, PDL_LEADER = 1, PDL_SIBLING = 2 };
+__device__ __forceinline__ void pdl_enter(int role) {
+    if (role == PDL_LEADER) cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (role == PDL_NORMAL) cudaGridDependencySynchronize();
+}
+__device__ __forceinline__ void pdl_leave(int role) {
+    if (role == PDL_SIBLING) cudaGridDependencySynchronize();
+}
+
 constexpr unsigned kSms = 148;
 inline bool overlaps(dim3 grid, unsigned single_wave_limit) {
     const unsigned long long blocks = 1ull * grid.x * grid.y * grid.z;

@@ -44,8 +44,8 @@ __device__ __forceinline__ void store_enc(int enc, void* out0, void* out1, size_
 template <typename TIn>
 __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict__ in, void* out0,
                                                            void* out1, int enc, int C, int Cp, int HW,
-                                                           float* colsum) {
-    pdl_enter();
+                                                           float* colsum, int role) {
+    pdl_enter(role);
     __shared__ float tile[64][65];
     const int n = blockIdx.z;
     const int c0 = blockIdx.y * 64;
@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict
             for (int i = 0; i < 8 && cb + i < Cp; ++i) store_enc(enc, out0, out1, o + i, v[i]);
         }
     }
+    pdl_leave(role);
 }
 
 // Row-major [R][C] -> [R][Cp] with encoding change (fp32/fp16 -> fp16 / tf32 pair), zero pad; Cp is a multiple of 4.
@@ -132,8 +133,8 @@ __device__ __forceinline__ float4 load4(const __half* p) {
 }
 template <typename TIn>
 __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict__ in, void* out0,
-                                                           void* out1, int enc, size_t R, int C, int Cp) {
-    pdl_enter();
+                                                           void* out1, int enc, size_t R, int C, int Cp, int role) {
+    pdl_enter(role);
     const size_t per_row = Cp / 4, total = R * per_row;
     const bool dense = C == Cp;  // rows follow one another on both sides
     const bool vec = (dense || C % 4 == 0) && (reinterpret_cast<uintptr_t>(in) & (4 * sizeof(TIn) - 1)) == 0;
@@ -170,14 +171,15 @@ __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict
                                                                  to_tf32_rna(v.z - hi.z), to_tf32_rna(v.w - hi.w));
         }
     }
+    pdl_leave(role);
 }
 
 // Column sums of a row-major [R][C] matrix (bias gradient of Linear, or of an NHWC dY), first stage:
 // row block blockIdx.y writes its sums to row blockIdx.y of the [row blocks][C] partial-sum matrix.
 template <typename TIn>
 __global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* __restrict__ in, float* colsum,
-                                                          size_t R, int C, int rows_per_block) {
-    pdl_enter();
+                                                          size_t R, int C, int rows_per_block, int role) {
+    pdl_enter(role);
     size_t r0 = static_cast<size_t>(blockIdx.y) * rows_per_block;
     size_t r1 = r0 + rows_per_block < R ? r0 + rows_per_block : R;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* __restrict_
         for (size_t r = r0; r < r1; ++r) s += load_as_float(in, r * C + c);
         colsum[static_cast<size_t>(blockIdx.y) * C + c] = s;
     }
+    pdl_leave(role);
 }
 
 // Vectorised column sums for rows that are whole 16-byte vectors (8 fp16 or 4 fp32 columns each): every thread owns one
@@ -205,8 +208,8 @@ __device__ __forceinline__ void add_vector(float (&acc)[4], const uint4& v, cons
 }
 template <typename TIn>
 __global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* __restrict__ in, float* colsum,
-                                                             size_t R, int C, int rows_per_block) {
-    pdl_enter();
+                                                             size_t R, int C, int rows_per_block, int role) {
+    pdl_enter(role);
     constexpr int V = 16 / sizeof(TIn);
     __shared__ float part[8][32 * V];
     const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* __restri
         for (int w = 0; w < 8; ++w) sum += part[w][threadIdx.x];
         colsum[static_cast<size_t>(blockIdx.y) * C + c] = sum;
     }
+    pdl_leave(role);
 }
 
 // Weights [D0][D1][T] -> K-major operand dst[n][t][kp]:
@@ -264,8 +268,8 @@ __device__ __forceinline__ void store_enc2(int enc, void* out0, void* out1, size
 
 template <typename TIn>
 __global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* __restrict__ w, void* out0, void* out1, int enc,
-                                                                 int R, int Cc, int Rp) {
-    pdl_enter();
+                                                                 int R, int Cc, int Rp, int role) {
+    pdl_enter(role);
     __shared__ float tile[64][65];  // [r][c]
     const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
     const size_t b = blockIdx.z;
@@ -281,12 +285,13 @@ __global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* __re
         const int c = c0 + j, r = r0 + 2 * tx;  // Rp is a multiple of the K block, so r + 1 < Rp whenever r < Rp
         if (c < Cc && r < Rp) store_enc2(enc, out0, out1, (b * Cc + c) * Rp + r, tile[2 * tx][j], tile[2 * tx + 1][j]);
     }
+    pdl_leave(role);
 }
 
 template <typename TIn>
 __global__ void __launch_bounds__(256) repack_weight_rows_kernel(const TIn* __restrict__ w, void* out0, void* out1, int enc,
-                                                                 int R, int Cc, int Rp) {
-    pdl_enter();
+                                                                 int R, int Cc, int Rp, int role) {
+    pdl_enter(role);
     __shared__ float tile[64][65];  // [c][r]
     const int r0 = blockIdx.x * 64;
     const size_t b = blockIdx.y;
@@ -302,13 +307,14 @@ __global__ void __launch_bounds__(256) repack_weight_rows_kernel(const TIn* __re
         const int c = idx >> 5, r = (idx & 31) * 2;
         if (r0 + r < Rp) store_enc2(enc, out0, out1, (b * Cc + c) * Rp + r0 + r, tile[c][r], tile[c][r + 1]);
     }
+    pdl_leave(role);
 }
 
 // The same two for fp16 weights that stay fp16 (a training step repacks every layer's weights twice): 16-byte loads, more
 // work per block, and no detour through float.  Both want 16-byte aligned source rows and Rp a multiple of 8.
 //   [B][R][Cc] -> [B][Cc][Rp], 64 x 64 tiles; Cc a multiple of 8.  2048 x 8192: 29.6 -> 12 us (bytes: 10 us).
-__global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* __restrict__ w, __half* __restrict__ out, int R, int Cc, int Rp) {
-    pdl_enter();
+__global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* __restrict__ w, __half* __restrict__ out, int R, int Cc, int Rp, int role) {
+    pdl_enter(role);
     __shared__ __half tile[64][66];  // [r][c]; a pitch of 33 words spreads the column reads below over the banks
     const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
     const size_t b = blockIdx.z;
@@ -335,11 +341,12 @@ __global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* __r
         for (int i = 0; i < 8; ++i) e[i] = tile[r + i][c];
         *reinterpret_cast<uint4*>(out + (b * Cc + c0 + c) * Rp + r0 + r) = y;
     }
+    pdl_leave(role);
 }
 
 // Cc <= 64 (the taps of one kernel), R * Cc a multiple of 8: 256 source rows per block, one contiguous run.
-__global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __restrict__ w, __half* __restrict__ out, int R, int Cc, int Rp) {
-    pdl_enter();
+__global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __restrict__ w, __half* __restrict__ out, int R, int Cc, int Rp, int role) {
+    pdl_enter(role);
     extern __shared__ __half run[];  // [256][pitch], pitch odd: lanes two rows apart read different banks
     const int pitch = Cc | 1;
     const int r0 = blockIdx.x * 256;
@@ -370,6 +377,7 @@ __global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __r
         for (int c = threadIdx.x >> 7; c < Cc; c += 2)
             *reinterpret_cast<__half2*>(out + (b * Cc + c) * Rp + r0 + r) = __halves2half2(run[r * pitch + c], run[(r + 1) * pitch + c]);
     }
+    pdl_leave(role);
 }
 
 // Few-channel activations (e.g. RGB stems): copy into a zero-padded NHWC image with exactly kCh (4 or 8) fp16 channels per
@@ -380,8 +388,8 @@ __global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __r
 template <typename TIn, int kCh>
 __global__ void __launch_bounds__(256) pad_pack_kernel(const TIn* __restrict__ in, int nchw, __half* __restrict__ out,
                                                        int N, int C, int H, int W, int pad_h, int pad_w, int Hp,
-                                                       int Wp, float* colsum) {
-    pdl_enter();
+                                                       int Wp, float* colsum, int role) {
+    pdl_enter(role);
     struct alignas(2 * kCh) Pixel {
         __half2 v[kCh / 2];
     };
@@ -433,14 +441,15 @@ __global__ void __launch_bounds__(256) pad_pack_kernel(const TIn* __restrict__ i
             colsum[static_cast<size_t>(blockIdx.x) * 8 + threadIdx.x] = sum;
         }
     }
+    pdl_leave(role);
 }
 
 // Weights [C_out][C][KH][KW] -> [C_out][KH][8 * ch] with k = kw * ch + c (zero where c >= C or kw >= KW):
 // the K-major operand matching pad_pack's (kw, c) slices.
 template <typename TIn>
 __global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
-                                                                   int Cout, int C, int KH, int KW, int ch_log2) {
-    pdl_enter();
+                                                                   int Cout, int C, int KH, int KW, int ch_log2, int role) {
+    pdl_enter(role);
     const int total = (Cout * KH) << (3 + ch_log2);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int k = i & ((8 << ch_log2) - 1);
@@ -451,6 +460,7 @@ __global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* __
         if (c < C && kw < KW) v = load_as_float(w, ((static_cast<size_t>(co) * C + c) * KH + kh) * KW + kw);
         out[i] = __float2half_rn(v);
     }
+    pdl_leave(role);
 }
 
 // Partial sums of a K-split forward walk, `planes` fp32 planes of [pixels][C] (one per K slice) -> the
@@ -470,8 +480,8 @@ __device__ __forceinline__ float4 finish4(float4 v, const float* bias, int c, in
 template <typename TOut>
 __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restrict__ acc, int planes, const float* __restrict__ bias,
                                                           TOut* __restrict__ out, size_t pixels, int C, int hw, int nchw,
-                                                          int round_f16, int vec) {
-    pdl_enter();
+                                                          int round_f16, int vec, int role) {
+    pdl_enter(role);
     const size_t total = pixels * C;
     if (vec) {
         const uint32_t c4n = static_cast<uint32_t>(C / 4);
@@ -494,6 +504,7 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restric
                 reinterpret_cast<float4*>(out)[i] = v;
             }
         }
+        pdl_leave(role);
         return;
     }
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -512,6 +523,7 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restric
         }
         out[o] = static_cast<TOut>(v);
     }
+    pdl_leave(role);
 }
 
 // Phase-packed gather walk: the weights [K][C][KH][KW] of a strided gather (input gradient of a
@@ -524,8 +536,8 @@ template <typename TIn, typename TBias>
 __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
                                                                  const TBias* __restrict__ bias, float* __restrict__ bias_out,
                                                                  int K, int C, int KH, int KW, int s_h, int s_w, int p_h,
-                                                                 int p_w, int khp, int kwp, int dh_min, int dw_min) {
-    pdl_enter();
+                                                                 int p_w, int khp, int kwp, int dh_min, int dw_min, int role) {
+    pdl_enter(role);
     const int np = s_h * s_w * C;
     const int total = np * K * khp * kwp;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -547,6 +559,7 @@ __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __re
     }
     if (bias_out != nullptr && blockIdx.x == 0 && threadIdx.x < np)
         bias_out[threadIdx.x] = (bias != nullptr) ? load_as_float(bias, threadIdx.x % C) : 0.f;
+    pdl_leave(role);
 }
 
 // Second stage of the column sums: adds rows [blockIdx.y * rows_per_block, ...) of the [P][stride]
@@ -554,8 +567,8 @@ __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __re
 // `out` ([segments][out_stride]).  Launched again on its own output while more than one segment is left.
 // blockDim = (8, 128): few channels and a chain of load latencies, so many threads take few rows each.
 __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __restrict__ partial, int P, int stride, int C,
-                                                             float* __restrict__ out, int out_stride, int rows_per_block) {
-    pdl_enter();
+                                                             float* __restrict__ out, int out_stride, int rows_per_block, int role) {
+    pdl_enter(role);
     __shared__ float part[128][9];
     const int c = blockIdx.x * 8 + threadIdx.x;
     const int p0 = blockIdx.y * rows_per_block;
@@ -571,6 +584,7 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
         if (threadIdx.y < half) part[threadIdx.y][threadIdx.x] += part[threadIdx.y + half][threadIdx.x];
     }
     if (threadIdx.y == 0 && c < C) out[static_cast<size_t>(blockIdx.y) * out_stride + c] = part[0][threadIdx.x];
+    pdl_leave(role);
 }
 
 // Second stage of a split-K weight gradient: adds the K slices' planes in slice order (bitwise
@@ -578,8 +592,8 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 // plane z holds row r at planes + z * plane_elems + r * src_pitch (floats).
 __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __restrict__ planes, float* __restrict__ dw,
                                                                  int split, size_t plane_elems, size_t rows, int row_len4,
-                                                                 size_t src_pitch) {
-    pdl_enter();
+                                                                 size_t src_pitch, int role) {
+    pdl_enter(role);
     const size_t total = rows * row_len4;
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -595,6 +609,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __
         }
         reinterpret_cast<float4*>(dw)[i] = a;
     }
+    pdl_leave(role);
 }
 
 // The same for many planes over a small gradient (the patch walk cuts K into one slice per SM): a thread
@@ -602,8 +617,8 @@ __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __
 // planes ty, ty + 8, ... of its float4 in order, then the eight running sums are added in order -- a
 // fixed association, so still bitwise repeatable.  Planes are laid out like dW.
 __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __restrict__ planes, float* __restrict__ dw,
-                                                                 int split, size_t plane_elems, size_t total4) {
-    pdl_enter();
+                                                                 int split, size_t plane_elems, size_t total4, int role) {
+    pdl_enter(role);
     __shared__ float4 part[8][32];
     const size_t i = blockIdx.x * 32ull + threadIdx.x;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -627,6 +642,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __
         }
         reinterpret_cast<float4*>(dw)[i] = t;
     }
+    pdl_leave(role);
 }
 
 // Planes of the tap-by-tile walk ([plain channel][R rows], row (t * c_blocks + pc / kb) * kb + pc % kb = one tap's patch
@@ -634,8 +650,8 @@ __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __
 // run along the patch channels (float4), the tap-fastest order is made in shared memory, and 64 * taps consecutive floats
 // are written.  (A thread per element read with a stride of a whole tap row: 4x4 512->128 11 us.)
 __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* __restrict__ planes, float* __restrict__ dw, int split,
-                                                                size_t plane_elems, int c_patch, int n_taps, int c_blocks, int kb, int R) {
-    pdl_enter();
+                                                                size_t plane_elems, int c_patch, int n_taps, int c_blocks, int kb, int R, int role) {
+    pdl_enter(role);
     extern __shared__ float taps[];  // [64][n_taps | 1]
     const int pitch = n_taps | 1;
     const size_t plain = blockIdx.y;
@@ -662,6 +678,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* __r
         const int c = i / n_taps;
         out[i] = taps[c * pitch + i - c * n_taps];
     }
+    pdl_leave(role);
 }
 
 // General form, one thread per dW element.  layout 0: a plane is laid out like dW.  layout 1: a plane is
@@ -670,8 +687,8 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* __r
 // (plain, c, kh, kw) sits at row kh * kb + kw * 8 + c.
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ planes, float* __restrict__ dw, int split,
                                                            size_t plane_elems, size_t total, int layout, int c_patch,
-                                                           int n_taps, int kw_count, int c_blocks, int kb, int R) {
-    pdl_enter();
+                                                           int n_taps, int kw_count, int c_blocks, int kb, int R, int role) {
+    pdl_enter(role);
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         size_t src = i;
@@ -694,13 +711,15 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
         for (int z = 1; z < split; ++z) a += __ldg(planes + z * plane_elems + src);
         dw[i] = a;
     }
+    pdl_leave(role);
 }
 
 template <typename TIn>
-__global__ void __launch_bounds__(256) to_float_kernel(const TIn* __restrict__ in, float* out, int n) {
-    pdl_enter();
+__global__ void __launch_bounds__(256) to_float_kernel(const TIn* __restrict__ in, float* out, int n, int role) {
+    pdl_enter(role);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = load_as_float(in, i);
+    pdl_leave(role);
 }
 
 }  // namespace nml

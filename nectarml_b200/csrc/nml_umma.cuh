@@ -78,6 +78,7 @@ struct KParams {
     CUtensorMap tmB[2];  // fprop: weights; wgrad: the plainly indexed tensor
     CUtensorMap tmC;     // OUT_NHWC_TMA: the output, box = the 32 rows x 128 bytes one epilogue warp owns
     int mode, out_mode;
+    int pdl_role;        // PDL_NORMAL, or PDL_LEADER in front of column sums that run beside this launch
     int num_tiles, n_tiles;
     uint32_t mul_nt;     // for fast_div by n_tiles
     int fastdiv;         // 1: tile ids and divisors are small enough for the multiply-and-shift division to be exact
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     if (kPair) cluster_sync_all();  // the partner's barriers must be initialised before anything arrives on them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_enter();  // everything above overlaps the tail of the kernel in front
+    pdl_enter(P.pdl_role);  // everything above overlaps the tail of the kernel in front
 
     const int ks = P.ka / P.planes;    // K slices per stage
     const int box_bytes = P.kb * 128;  // one MN-major box: kb k-rows of 128 bytes

@@ -212,14 +212,30 @@ int nml_bn_backward(const void* dy, const void* y, const void* x, long long rows
 /* The same without the forward's output y in the backward.  Where nothing was added before the activation its
  * derivative follows from x (pass mask = NULL on both sides, and the forward's beta to the backward); where a residual
  * was added, `mask` holds one bit per element, set where y > 0 (rows * channels / 8 bytes, byte v the channels 8v ... 8v+7
- * of the row-major matrix; written by the forward). */
+ * of the row-major matrix; written by the forward).
+ * The output and its gradient may be part of the channels of a wider tensor, so that a concatenation needs no pass of its
+ * own: *_pitch is the distance of their rows in elements (a multiple of 8; 0: `channels`).  y2 (optional) is a second copy
+ * of the output, dy2 (optional) a second gradient that is added to dy in fp32. */
 int nml_bn_forward_masked(const void* x, long long rows, int channels, const float* gamma, const float* beta,
-                          const void* residual, int act, float slope, float eps, void* y, void* mask, float* mean,
-                          float* rstd, void* workspace, size_t workspace_bytes, void* stream);
-int nml_bn_backward_masked(const void* dy, const void* mask, const void* x, long long rows, int channels,
-                           const float* gamma, const float* beta, const float* mean, const float* rstd, int act,
-                           float slope, void* dx, void* dres, float* dgamma, float* dbeta, void* workspace,
-                           size_t workspace_bytes, void* stream);
+                          const void* residual, int act, float slope, float eps, void* y, int y_pitch, void* y2,
+                          int y2_pitch, void* mask, float* mean, float* rstd, void* workspace, size_t workspace_bytes,
+                          void* stream);
+int nml_bn_backward_masked(const void* dy, int dy_pitch, const void* dy2, int dy2_pitch, const void* mask, const void* x,
+                           long long rows, int channels, const float* gamma, const float* beta, const float* mean,
+                           const float* rstd, int act, float slope, void* dx, void* dres, float* dgamma, float* dbeta,
+                           void* workspace, size_t workspace_bytes, void* stream);
+
+/* ReLU (act 1) / LeakyReLU (act 2) with no normalisation in front, same conventions. */
+int nml_act_forward(const void* x, long long rows, int channels, int act, float slope, void* y, void* y2, int y2_pitch,
+                    void* stream);
+int nml_act_backward(const void* dy, int dy_pitch, const void* dy2, int dy2_pitch, const void* x, long long rows,
+                     int channels, int act, float slope, void* dx, void* stream);
+
+/* *loss = sum |a - b| / denom over n fp16 values (4-byte aligned); da = sign(a - b) * *dloss / denom. */
+int nml_l1_workspace_size(size_t* bytes);
+int nml_l1_forward(const void* a, const void* b, size_t n, float denom, float* loss, void* workspace,
+                   size_t workspace_bytes, void* stream);
+int nml_l1_backward(const void* a, const void* b, size_t n, const float* dloss, float denom, void* da, void* stream);
 
 /* Max pooling of an NHWC fp16 tensor (channels a multiple of 8), output size (h + 2 pad - k)/stride + 1.
  * The forward also writes one byte per output value naming the window tap that won (`index`,

@@ -56,8 +56,15 @@ SYMBOLS = {
     "nml_bn_workspace_size": (_I, [C.c_longlong, _I, C.POINTER(_SZ)]),
     "nml_bn_forward": (_I, [_VP, C.c_longlong, _I, _VP, _VP, _VP, _I, C.c_float, C.c_float, _VP, _VP, _VP, _VP, _SZ, _VP]),
     "nml_bn_backward": (_I, [_VP, _VP, _VP, C.c_longlong, _I, _VP, _VP, _VP, _I, C.c_float, _VP, _VP, _VP, _VP, _VP, _SZ, _VP]),
-    "nml_bn_forward_masked": (_I, [_VP, C.c_longlong, _I, _VP, _VP, _VP, _I, C.c_float, C.c_float, _VP, _VP, _VP, _VP, _VP, _SZ, _VP]),
-    "nml_bn_backward_masked": (_I, [_VP, _VP, _VP, C.c_longlong, _I, _VP, _VP, _VP, _VP, _I, C.c_float, _VP, _VP, _VP, _VP, _VP, _SZ, _VP]),
+    "nml_bn_forward_masked": (_I, [_VP, C.c_longlong, _I, _VP, _VP, _VP, _I, C.c_float, C.c_float, _VP, _I, _VP, _I, _VP, _VP, _VP, _VP,
+                                   _SZ, _VP]),
+    "nml_bn_backward_masked": (_I, [_VP, _I, _VP, _I, _VP, _VP, C.c_longlong, _I, _VP, _VP, _VP, _VP, _I, C.c_float, _VP, _VP, _VP, _VP,
+                                    _VP, _SZ, _VP]),
+    "nml_l1_forward": (_I, [_VP, _VP, _SZ, C.c_float, _VP, _VP, _SZ, _VP]),
+    "nml_l1_workspace_size": (_I, [C.POINTER(_SZ)]),
+    "nml_l1_backward": (_I, [_VP, _VP, _SZ, _VP, C.c_float, _VP, _VP]),
+    "nml_act_forward": (_I, [_VP, C.c_longlong, _I, _I, C.c_float, _VP, _VP, _I, _VP]),
+    "nml_act_backward": (_I, [_VP, _I, _VP, _I, _VP, C.c_longlong, _I, _I, C.c_float, _VP, _VP]),
     "nml_maxpool_forward": (_I, [_VP, _I, _I, _I, _I, _I, _I, _I, _VP, _VP, _VP]),
     "nml_maxpool_backward": (_I, [_VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP, _VP]),
     "nml_grads_check": (_I, [_VP, _SZ, C.c_float, _VP, _VP]),

@@ -122,6 +122,34 @@ __device__ __forceinline__ void act_backward(float (&df)[8], const float (&xf)[8
     }
 }
 
+// The gradient of a pass's output: one fp16 tensor, or the sum of two (the output was read by the next layer and, as part of
+// the channels of a concatenation, by a later one).  Either may be part of the channels of a wider tensor: rows are `row`
+// (`row2`) vectors apart.  Reading both here keeps the slice's copy and the sum out of memory.
+struct OutGrad {
+    const uint4 *a, *b;
+    int row, row2;
+};
+struct OutGradVector {
+    uint4 a, b;
+};
+template <bool kTwo>
+__device__ __forceinline__ OutGradVector load_grad(const OutGrad& g, size_t row, int col) {
+    OutGradVector v;
+    v.a = __ldg(g.a + row * g.row + col);
+    if (kTwo) v.b = __ldg(g.b + row * g.row2 + col);
+    return v;
+}
+template <bool kTwo>
+__device__ __forceinline__ void unpack_grad(const OutGradVector& v, float (&f)[8]) {
+    unpack8(v.a, f);
+    if (kTwo) {
+        float t[8];
+        unpack8(v.b, t);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += t[j];
+    }
+}
+
 // What a backward pass reads of the forward besides x: see the D_* above.  `below` is the derivative where y <= 0.
 struct BnForward {
     const uint4* y;
@@ -190,8 +218,8 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* __restrict__
 // Backward sums: with dz = dy * act'(.): a = sum dz, b = sum dz * x (the second stage turns b into
 // d gamma = rstd * (b - mean * a), so this pass needs no per-channel constants but those of D_X).  Two rows in flight per
 // thread.
-template <int kDeriv>
-__global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, const BnForward f,
+template <int kDeriv, bool kTwo>
+__global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restrict__ x, const OutGrad dy, const BnForward f,
                                                            float* __restrict__ partial, size_t M, int C) {
     pdl_enter();
     __shared__ float sm[256][17];
@@ -202,10 +230,10 @@ __global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restri
     if (kDeriv == D_X) bn_affine(col, f.gamma, f.beta, f.mean, f.rstd, sc, sh);
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
-    auto add = [&](const uint4& xv, const uint4& dv, const uint4& yv, unsigned bits) {
+    auto add = [&](const uint4& xv, const OutGradVector& dv, const uint4& yv, unsigned bits) {
         float xf[8], df[8];
         unpack8(xv, xf);
-        unpack8(dv, df);
+        unpack_grad<kTwo>(dv, df);
         act_backward<kDeriv>(df, xf, yv, bits, sc, sh, f.below);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -218,7 +246,8 @@ __global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restri
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     for (; row + stride < M; row += 2 * stride) {
         const size_t v0 = row * cpr + col, v1 = (row + stride) * cpr + col;
-        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1), d0 = __ldg(dy + v0), d1 = __ldg(dy + v1);
+        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
+        const OutGradVector d0 = load_grad<kTwo>(dy, row, col), d1 = load_grad<kTwo>(dy, row + stride, col);
         const uint4 y0 = kDeriv == D_Y ? __ldg(f.y + v0) : zero, y1 = kDeriv == D_Y ? __ldg(f.y + v1) : zero;
         const unsigned m0 = kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? __ldg(f.mask + v1) : 0u;
         add(x0, d0, y0, m0);
@@ -226,7 +255,7 @@ __global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restri
     }
     if (row < M) {
         const size_t v0 = row * cpr + col;
-        add(__ldg(x + v0), __ldg(dy + v0), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
+        add(__ldg(x + v0), load_grad<kTwo>(dy, row, col), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
     }
     bn_store_partial(sm, a, b, cpr, rpb, C, partial);
 }
@@ -275,8 +304,10 @@ __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict
 // y = act(gamma * (x - mean) * rstd + beta [+ residual]), fp16 in and out; two rows in flight per thread.  With `mask`
 // one bit per element, set where y > 0, for D_MASK.  The rows are walked from the last to the first: the statistics pass
 // has just read x in the other direction, so what of it is still in L2 (126 MB) is read first.
+// y (and y2, a second copy) may be part of the channels of a wider tensor: their rows are y_row and y2_row vectors apart.
 __global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res,
-                                                       uint4* __restrict__ y, uint8_t* __restrict__ mask, const float* __restrict__ gamma,
+                                                       uint4* __restrict__ y, int y_row, uint4* __restrict__ y2, int y2_row,
+                                                       uint8_t* __restrict__ mask, const float* __restrict__ gamma,
                                                        const float* __restrict__ beta, const float* __restrict__ mean,
                                                        const float* __restrict__ rstd, int act, float slope, size_t M, int C) {
     pdl_enter();
@@ -285,7 +316,7 @@ __global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restric
     const int col = threadIdx.x % cpr, rsub = threadIdx.x / cpr;
     float sc[8], sh[8];
     bn_affine(col, gamma, beta, mean, rstd, sc, sh);
-    auto one = [&](size_t v, const uint4& xv, const uint4& rv) {
+    auto one = [&](size_t row, const uint4& xv, const uint4& rv) {
         float xf[8], rf[8];
         unpack8(xv, xf);
         if (res) unpack8(rv, rf);
@@ -298,8 +329,10 @@ __global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restric
             if (act != 0 && t < 0.f) t = (act == 1) ? 0.f : t * slope;
             xf[j] = t;
         }
-        y[v] = pack8(xf);
-        if (mask) mask[v] = static_cast<uint8_t>(bits);
+        const uint4 out = pack8(xf);
+        y[row * y_row + col] = out;
+        if (y2) y2[row * y2_row + col] = out;
+        if (mask) mask[row * cpr + col] = static_cast<uint8_t>(bits);
     };
     const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
     size_t k = static_cast<size_t>(blockIdx.x) * rpb + rsub;  // rows counted from the end
@@ -308,20 +341,20 @@ __global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restric
         const size_t v0 = (M - 1 - k) * cpr + col, v1 = (M - 1 - k - stride) * cpr + col;
         const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
         const uint4 r0 = res ? __ldg(res + v0) : zero, r1 = res ? __ldg(res + v1) : zero;
-        one(v0, x0, r0);
-        one(v1, x1, r1);
+        one(M - 1 - k, x0, r0);
+        one(M - 1 - k - stride, x1, r1);
     }
     if (k < M) {
         const size_t v0 = (M - 1 - k) * cpr + col;
-        one(v0, __ldg(x + v0), res ? __ldg(res + v0) : zero);
+        one(M - 1 - k, __ldg(x + v0), res ? __ldg(res + v0) : zero);
     }
 }
 
 // dx = gamma * rstd * (dz - dbeta / M - xhat * dgamma / M) with dz = dy * act'(.), folded into
 // dx = A * dz + B * x + C per channel; optionally dres = dz (the gradient of the residual input that was
 // added before the activation).  Two rows in flight per thread, from the last row to the first as in bn_apply_kernel.
-template <int kDeriv>
-__global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, const BnForward f,
+template <int kDeriv, bool kTwo>
+__global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__ x, const OutGrad dy, const BnForward f,
                                                     uint4* __restrict__ dx, uint4* __restrict__ dres, const float* __restrict__ dbeta,
                                                     const float* __restrict__ dgamma, float inv_M, size_t M, int C) {
     pdl_enter();
@@ -345,10 +378,10 @@ __global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__
             kc[j] = ka[j] * (mu[j] * rs[j] * k2 - k1);
         }
     }
-    auto one = [&](size_t v, const uint4& xv, const uint4& dv, const uint4& yv, unsigned bits) {
+    auto one = [&](size_t v, const uint4& xv, const OutGradVector& dv, const uint4& yv, unsigned bits) {
         float xf[8], df[8];
         unpack8(xv, xf);
-        unpack8(dv, df);
+        unpack_grad<kTwo>(dv, df);
         act_backward<kDeriv>(df, xf, yv, bits, sc, sh, f.below);
 #pragma unroll
         for (int j = 0; j < 8; ++j) xf[j] = ka[j] * df[j] + kb[j] * xf[j] + kc[j];
@@ -360,7 +393,8 @@ __global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     for (; k + stride < M; k += 2 * stride) {
         const size_t v0 = (M - 1 - k) * cpr + col, v1 = (M - 1 - k - stride) * cpr + col;
-        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1), d0 = __ldg(dy + v0), d1 = __ldg(dy + v1);
+        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
+        const OutGradVector d0 = load_grad<kTwo>(dy, M - 1 - k, col), d1 = load_grad<kTwo>(dy, M - 1 - k - stride, col);
         const uint4 y0 = kDeriv == D_Y ? __ldg(f.y + v0) : zero, y1 = kDeriv == D_Y ? __ldg(f.y + v1) : zero;
         const unsigned m0 = kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? __ldg(f.mask + v1) : 0u;
         one(v0, x0, d0, y0, m0);
@@ -368,8 +402,99 @@ __global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__
     }
     if (k < M) {
         const size_t v0 = (M - 1 - k) * cpr + col;
-        one(v0, __ldg(x + v0), __ldg(dy + v0), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
+        one(v0, __ldg(x + v0), load_grad<kTwo>(dy, M - 1 - k, col), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
     }
+}
+
+// An activation that no normalisation stands in front of: y = act(x), with a second copy as part of the channels of a wider
+// tensor.  rows x C, thread layout and grid as above.
+__global__ void __launch_bounds__(256, 4) act_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, uint4* __restrict__ y2,
+                                                     int y2_row, float below, size_t M, int C) {
+    pdl_enter();
+    const int cpr = C >> 3;
+    const int rpb = blockDim.x / cpr;
+    const int col = threadIdx.x % cpr;
+    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
+#pragma unroll 2
+    for (size_t row = static_cast<size_t>(blockIdx.x) * rpb + threadIdx.x / cpr; row < M; row += stride) {
+        float f[8];
+        unpack8(__ldg(x + row * cpr + col), f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] > 0.f ? f[j] : f[j] * below + 0.f;  // NaN stays NaN, -0 becomes 0
+        const uint4 out = pack8(f);
+        y[row * cpr + col] = out;
+        if (y2) y2[row * y2_row + col] = out;
+    }
+}
+// dx = dy * act'(x).
+template <bool kTwo>
+__global__ void __launch_bounds__(256, 4) act_backward_kernel(const uint4* __restrict__ x, const OutGrad dy, uint4* __restrict__ dx,
+                                                              float below, size_t M, int C) {
+    pdl_enter();
+    const int cpr = C >> 3;
+    const int rpb = blockDim.x / cpr;
+    const int col = threadIdx.x % cpr;
+    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
+#pragma unroll 2
+    for (size_t row = static_cast<size_t>(blockIdx.x) * rpb + threadIdx.x / cpr; row < M; row += stride) {
+        float f[8], d[8];
+        const OutGradVector g = load_grad<kTwo>(dy, row, col);
+        unpack8(__ldg(x + row * cpr + col), f);
+        unpack_grad<kTwo>(g, d);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) d[j] *= f[j] > 0.f ? 1.f : below;
+        dx[row * cpr + col] = pack8(d);
+    }
+}
+
+// L1 loss sum |a - b| / denom of two fp16 tensors, in fp32 within a thread's share and in double over the blocks, fixed order.
+// As separate passes (two conversions, difference, absolute value, sum; sign, product and conversion back) the loss of 16
+// images of 256 x 256 took 60 us of small kernels each way and twice as long to issue.
+__global__ void __launch_bounds__(256) l1_sum_kernel(const __half2* __restrict__ a, const __half2* __restrict__ b, size_t n, float* __restrict__ partial) {
+    pdl_enter();
+    float s = 0.f;
+    const size_t n2 = n / 2, step = static_cast<size_t>(gridDim.x) * blockDim.x;
+#pragma unroll 4
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n2; i += step) {
+        const float2 u = __half22float2(a[i]), v = __half22float2(b[i]);
+        s += fabsf(u.x - v.x) + fabsf(u.y - v.y);
+    }
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0)
+        s += fabsf(__half2float(reinterpret_cast<const __half*>(a)[n - 1]) - __half2float(reinterpret_cast<const __half*>(b)[n - 1]));
+    __shared__ float sm[8];
+#pragma unroll
+    for (int o = 16; o > 0; o /= 2) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x / 32] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s = 0.f;
+        for (int w = 0; w < 8; ++w) s += sm[w];
+        partial[blockIdx.x] = s;
+    }
+}
+__global__ void __launch_bounds__(32) l1_finish_kernel(const float* __restrict__ partial, int P, float denom, float* __restrict__ loss) {
+    pdl_enter();
+    double s = 0.0;
+    for (int p = threadIdx.x; p < P; p += 32) s += static_cast<double>(partial[p]);
+#pragma unroll
+    for (int o = 16; o > 0; o /= 2) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *loss = static_cast<float>(s) / denom;
+}
+// da = sign(a - b) * (*dloss / denom)
+__global__ void __launch_bounds__(256) l1_backward_kernel(const __half2* __restrict__ a, const __half2* __restrict__ b, size_t n,
+                                                          const float* __restrict__ dloss, float denom, __half2* __restrict__ da) {
+    pdl_enter();
+    const float g = __ldg(dloss) / denom;
+    auto one = [&](float d) { return d > 0.f ? g : d < 0.f ? -g : 0.f; };
+    const size_t n2 = n / 2, step = static_cast<size_t>(gridDim.x) * blockDim.x;
+#pragma unroll 4
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n2; i += step) {
+        const float2 u = __half22float2(__ldg(a + i)), v = __half22float2(__ldg(b + i));
+        da[i] = __floats2half2_rn(one(u.x - v.x), one(u.y - v.y));
+    }
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0)
+        reinterpret_cast<__half*>(da)[n - 1] = __float2half_rn(
+            one(__half2float(reinterpret_cast<const __half*>(a)[n - 1]) - __half2float(reinterpret_cast<const __half*>(b)[n - 1])));
 }
 
 // any(!isfinite(g * inv_scale)) over a flat fp32 buffer -> *found (set, never cleared, here)
@@ -516,6 +641,9 @@ static int bn_grid_elementwise(long long M, int C, int per_sm) {
     return static_cast<int>(want < 148 * per_sm ? want : 148 * per_sm);
 }
 static bool bn_shape_ok(long long M, int C) { return M > 0 && C > 0 && C % 8 == 0 && C <= 2048; }
+// A row pitch of a tensor of `channels` channels, in elements: 0 for a tensor of its own.
+static bool row_ok(int pitch, int channels) { return pitch == 0 || (pitch >= channels && pitch % 8 == 0); }
+static int row_vectors(int pitch, int channels) { return (pitch ? pitch : channels) / 8; }
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace nml_layers
@@ -535,16 +663,17 @@ int nml_bn_workspace_size(long long rows, int channels, size_t* bytes) {
 int nml_bn_forward(const void* x, long long rows, int channels, const float* gamma, const float* beta, const void* residual,
                    int act, float slope, float eps, void* y, float* mean, float* rstd, void* workspace,
                    size_t workspace_bytes, void* stream) {
-    return nml_bn_forward_masked(x, rows, channels, gamma, beta, residual, act, slope, eps, y, nullptr, mean, rstd, workspace,
-                                 workspace_bytes, stream);
+    return nml_bn_forward_masked(x, rows, channels, gamma, beta, residual, act, slope, eps, y, 0, nullptr, 0, nullptr, mean, rstd,
+                                 workspace, workspace_bytes, stream);
 }
 
 int nml_bn_forward_masked(const void* x, long long rows, int channels, const float* gamma, const float* beta, const void* residual,
-                          int act, float slope, float eps, void* y, void* mask, float* mean, float* rstd, void* workspace,
-                          size_t workspace_bytes, void* stream) {
+                          int act, float slope, float eps, void* y, int y_pitch, void* y2, int y2_pitch, void* mask, float* mean,
+                          float* rstd, void* workspace, size_t workspace_bytes, void* stream) {
     if (!x || !y || !mean || !rstd || act < 0 || act > 2) return NML_ERR_INVALID;
     if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
-    if (!aligned16(x) || !aligned16(y) || (residual && !aligned16(residual))) return NML_ERR_INVALID;
+    if (!aligned16(x) || !aligned16(y) || (residual && !aligned16(residual)) || (y2 && !aligned16(y2))) return NML_ERR_INVALID;
+    if (!row_ok(y_pitch, channels) || !row_ok(y2_pitch, channels)) return NML_ERR_INVALID;
     size_t need = 0;
     nml_bn_workspace_size(rows, channels, &need);
     if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
@@ -558,53 +687,124 @@ int nml_bn_forward_masked(const void* x, long long rows, int channels, const flo
     launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
            nullptr, nullptr, mean, rstd);
     launch(bn_apply_kernel, bn_grid_elementwise(rows, channels, kApplyBlocks), threads, 0, st, xv, static_cast<const uint4*>(residual),
-           static_cast<uint4*>(y), static_cast<uint8_t*>(mask), gamma, beta, mean, rstd, act, slope, M, channels);
+           static_cast<uint4*>(y), row_vectors(y_pitch, channels), static_cast<uint4*>(y2), row_vectors(y2_pitch, channels),
+           static_cast<uint8_t*>(mask), gamma, beta, mean, rstd, act, slope, M, channels);
     NMLL_CUDA(cudaGetLastError());
     g_layer_launches += 3;
     return NML_OK;
 }
 
-static int bn_backward(const void* dy, const void* x, long long rows, int channels, int deriv, const BnForward& f, void* dx, void* dres,
+}  // extern "C"
+
+template <bool kTwo>
+static void bn_backward_launch(const uint4* x, long long rows, int channels, int deriv, const OutGrad& dy, const BnForward& f, void* dx,
+                               void* dres, float* dgamma, float* dbeta, float* partial, cudaStream_t st) {
+    int threads;
+    const int P = bn_grid(rows, channels, &threads);
+    const size_t M = static_cast<size_t>(rows);
+    auto sums = deriv == D_NONE ? bn_grad_sums_kernel<D_NONE, kTwo> : deriv == D_Y ? bn_grad_sums_kernel<D_Y, kTwo>
+              : deriv == D_X ? bn_grad_sums_kernel<D_X, kTwo> : bn_grad_sums_kernel<D_MASK, kTwo>;
+    auto apply = deriv == D_NONE ? bn_dx_kernel<D_NONE, kTwo> : deriv == D_Y ? bn_dx_kernel<D_Y, kTwo>
+               : deriv == D_X ? bn_dx_kernel<D_X, kTwo> : bn_dx_kernel<D_MASK, kTwo>;
+    launch(sums, P, threads, 0, st, x, dy, f, partial, M, channels);
+    launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 1, 0.0, 0.f, f.mean, f.rstd, dbeta, dgamma);
+    launch(apply, bn_grid_elementwise(rows, channels, kDxBlocks), threads, 0, st, x, dy, f, static_cast<uint4*>(dx),
+           static_cast<uint4*>(dres), dbeta, dgamma, static_cast<float>(1.0 / static_cast<double>(rows)), M, channels);
+}
+static int bn_backward(const void* x, long long rows, int channels, int deriv, const OutGrad& dy, const BnForward& f, void* dx, void* dres,
                        float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, cudaStream_t st) {
     if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
-    if (!aligned16(dy) || !aligned16(x) || !aligned16(dx) || (f.y && !aligned16(f.y)) || (dres && !aligned16(dres))) return NML_ERR_INVALID;
+    if (!aligned16(dy.a) || (dy.b && !aligned16(dy.b)) || !aligned16(x) || !aligned16(dx) || (f.y && !aligned16(f.y)) ||
+        (dres && !aligned16(dres)))
+        return NML_ERR_INVALID;
     size_t need = 0;
     nml_bn_workspace_size(rows, channels, &need);
     if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
-    int threads;
-    const int P = bn_grid(rows, channels, &threads);
-    float* partial = static_cast<float*>(workspace);
-    const size_t M = static_cast<size_t>(rows);
-    const uint4 *xv = static_cast<const uint4*>(x), *dyv = static_cast<const uint4*>(dy);
-    auto sums = deriv == D_NONE ? bn_grad_sums_kernel<D_NONE> : deriv == D_Y ? bn_grad_sums_kernel<D_Y>
-              : deriv == D_X ? bn_grad_sums_kernel<D_X> : bn_grad_sums_kernel<D_MASK>;
-    auto apply = deriv == D_NONE ? bn_dx_kernel<D_NONE> : deriv == D_Y ? bn_dx_kernel<D_Y>
-               : deriv == D_X ? bn_dx_kernel<D_X> : bn_dx_kernel<D_MASK>;
-    launch(sums, P, threads, 0, st, xv, dyv, f, partial, M, channels);
-    launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 1, 0.0, 0.f, f.mean, f.rstd, dbeta, dgamma);
-    launch(apply, bn_grid_elementwise(rows, channels, kDxBlocks), threads, 0, st, xv, dyv, f, static_cast<uint4*>(dx), static_cast<uint4*>(dres),
-           dbeta, dgamma, static_cast<float>(1.0 / static_cast<double>(rows)), M, channels);
+    auto run = dy.b ? bn_backward_launch<true> : bn_backward_launch<false>;
+    run(static_cast<const uint4*>(x), rows, channels, deriv, dy, f, dx, dres, dgamma, dbeta, static_cast<float*>(workspace), st);
     NMLL_CUDA(cudaGetLastError());
     g_layer_launches += 3;
     return NML_OK;
 }
+static OutGrad out_grad(const void* dy, int pitch, const void* dy2, int pitch2, int channels) {
+    return {static_cast<const uint4*>(dy), static_cast<const uint4*>(dy2), row_vectors(pitch, channels), row_vectors(pitch2, channels)};
+}
+
+extern "C" {
 
 int nml_bn_backward(const void* dy, const void* y, const void* x, long long rows, int channels, const float* gamma,
                     const float* mean, const float* rstd, int act, float slope, void* dx, void* dres, float* dgamma,
                     float* dbeta, void* workspace, size_t workspace_bytes, void* stream) {
     if (!dy || !x || !mean || !rstd || !dx || !dgamma || !dbeta || act < 0 || act > 2 || (act != 0 && !y)) return NML_ERR_INVALID;
     const BnForward f = {act != 0 ? static_cast<const uint4*>(y) : nullptr, nullptr, gamma, nullptr, mean, rstd, act == 1 ? 0.f : slope};
-    return bn_backward(dy, x, rows, channels, act != 0 ? D_Y : D_NONE, f, dx, dres, dgamma, dbeta, workspace, workspace_bytes,
-                       static_cast<cudaStream_t>(stream));
+    return bn_backward(x, rows, channels, act != 0 ? D_Y : D_NONE, out_grad(dy, 0, nullptr, 0, channels), f, dx, dres, dgamma, dbeta,
+                       workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
 }
 
-int nml_bn_backward_masked(const void* dy, const void* mask, const void* x, long long rows, int channels, const float* gamma,
-                           const float* beta, const float* mean, const float* rstd, int act, float slope, void* dx, void* dres,
-                           float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, void* stream) {
+int nml_bn_backward_masked(const void* dy, int dy_pitch, const void* dy2, int dy2_pitch, const void* mask, const void* x, long long rows,
+                           int channels, const float* gamma, const float* beta, const float* mean, const float* rstd, int act, float slope,
+                           void* dx, void* dres, float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, void* stream) {
     if (!dy || !x || !mean || !rstd || !dx || !dgamma || !dbeta || act < 0 || act > 2) return NML_ERR_INVALID;
+    if (!row_ok(dy_pitch, channels) || !row_ok(dy2_pitch, channels)) return NML_ERR_INVALID;
     const BnForward f = {nullptr, static_cast<const uint8_t*>(mask), gamma, beta, mean, rstd, act == 1 ? 0.f : slope};
-    return bn_backward(dy, x, rows, channels, act == 0 ? D_NONE : mask ? D_MASK : D_X, f, dx, dres, dgamma, dbeta, workspace,
-                       workspace_bytes, static_cast<cudaStream_t>(stream));
+    return bn_backward(x, rows, channels, act == 0 ? D_NONE : mask ? D_MASK : D_X, out_grad(dy, dy_pitch, dy2, dy2_pitch, channels), f, dx,
+                       dres, dgamma, dbeta, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
+}
+
+int nml_act_forward(const void* x, long long rows, int channels, int act, float slope, void* y, void* y2, int y2_pitch, void* stream) {
+    if (!x || !y || act < 1 || act > 2 || !row_ok(y2_pitch, channels)) return NML_ERR_INVALID;
+    if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
+    if (!aligned16(x) || !aligned16(y) || (y2 && !aligned16(y2))) return NML_ERR_INVALID;
+    launch(act_kernel, bn_grid_elementwise(rows, channels, kApplyBlocks), 256 / (channels / 8) * (channels / 8), 0,
+           static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<uint4*>(y), static_cast<uint4*>(y2),
+           row_vectors(y2_pitch, channels), act == 1 ? 0.f : slope, static_cast<size_t>(rows), channels);
+    NMLL_CUDA(cudaGetLastError());
+    ++g_layer_launches;
+    return NML_OK;
+}
+
+int nml_act_backward(const void* dy, int dy_pitch, const void* dy2, int dy2_pitch, const void* x, long long rows, int channels, int act,
+                     float slope, void* dx, void* stream) {
+    if (!dy || !x || !dx || act < 1 || act > 2 || !row_ok(dy_pitch, channels) || !row_ok(dy2_pitch, channels)) return NML_ERR_INVALID;
+    if (!bn_shape_ok(rows, channels)) return NML_ERR_UNSUPPORTED;
+    if (!aligned16(dy) || (dy2 && !aligned16(dy2)) || !aligned16(x) || !aligned16(dx)) return NML_ERR_INVALID;
+    launch(dy2 ? act_backward_kernel<true> : act_backward_kernel<false>, bn_grid_elementwise(rows, channels, kApplyBlocks),
+           256 / (channels / 8) * (channels / 8), 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x),
+           out_grad(dy, dy_pitch, dy2, dy2_pitch, channels), static_cast<uint4*>(dx), act == 1 ? 0.f : slope, static_cast<size_t>(rows),
+           channels);
+    NMLL_CUDA(cudaGetLastError());
+    ++g_layer_launches;
+    return NML_OK;
+}
+
+constexpr int kL1Blocks = 4 * 148;
+int nml_l1_workspace_size(size_t* bytes) {
+    if (!bytes) return NML_ERR_INVALID;
+    *bytes = round_up(kL1Blocks * sizeof(float), 256);
+    return NML_OK;
+}
+static int l1_grid(size_t n) { return static_cast<int>(n / 512 + 1 < kL1Blocks ? n / 512 + 1 : kL1Blocks); }
+int nml_l1_forward(const void* a, const void* b, size_t n, float denom, float* loss, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!a || !b || !loss || n == 0 || (reinterpret_cast<uintptr_t>(a) & 3) || (reinterpret_cast<uintptr_t>(b) & 3)) return NML_ERR_INVALID;
+    size_t need = 0;
+    nml_l1_workspace_size(&need);
+    if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    float* partial = static_cast<float*>(workspace);
+    launch(l1_sum_kernel, l1_grid(n), 256, 0, st, static_cast<const __half2*>(a), static_cast<const __half2*>(b), n, partial);
+    launch(l1_finish_kernel, 1, 32, 0, st, partial, l1_grid(n), denom, loss);
+    NMLL_CUDA(cudaGetLastError());
+    g_layer_launches += 2;
+    return NML_OK;
+}
+int nml_l1_backward(const void* a, const void* b, size_t n, const float* dloss, float denom, void* da, void* stream) {
+    if (!a || !b || !dloss || !da || n == 0 || ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(da)) & 3))
+        return NML_ERR_INVALID;
+    launch(l1_backward_kernel, l1_grid(n), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const __half2*>(a),
+           static_cast<const __half2*>(b), n, dloss, denom, static_cast<__half2*>(da));
+    NMLL_CUDA(cudaGetLastError());
+    ++g_layer_launches;
+    return NML_OK;
 }
 
 long long nml_layers_launch_count(void) { return g_layer_launches.load(); }

@@ -371,66 +371,167 @@ PyObject* py_linear_backward_weight(PyObject*, PyObject* const* a, Py_ssize_t n)
     });
 }
 
-// ------------------------------------------------------------------ batch norm --
-// bn_forward(x, residual, gamma, beta, act, slope, eps, workspace) -> (y, mean, rstd, mask): the mask of y > 0 where the
-// backward cannot tell it from x, else None
+// ------------------------------------------------------------------ batch norm, activation --
+// Concatenations along the channels are not made by a pass of their own: the first of the two layers whose outputs meet
+// allocates the wide tensor and writes a second copy of its output into its last channels (`skip`), the other one writes its
+// output into the first channels (`join`).  In the backward each reads its part of the wide tensor's gradient in place.
+PyObject* wrap_or_none(const at::Tensor& t) { return t.defined() ? THPVariable_Wrap(t) : Py_NewRef(Py_None); }
+template <class... T>
+PyObject* tuple_of(const T&... t) {
+    PyObject* const items[] = {wrap_or_none(t)...};
+    PyObject* r = PyTuple_New(sizeof...(t));
+    for (size_t i = 0; i < sizeof...(t); ++i) PyTuple_SET_ITEM(r, i, items[i]);
+    return r;
+}
+at::Tensor wide_like(const at::Tensor& x) {
+    auto shape = x.sizes().vec();
+    shape.back() *= 2;
+    return at::empty(shape, x.options());
+}
+void* channels_from(const at::Tensor& wide, int64_t c) { return static_cast<char*>(ptr(wide)) + c * wide.element_size(); }
+void require_half_rows(const at::Tensor& t, const at::Tensor& x, int64_t c, const char* what) {
+    require(t.scalar_type() == at::kHalf && t.numel() / t.size(-1) == x.numel() / x.size(-1) && t.size(-1) == c, what);
+}
+
+// The gradient of an output: dy and, for an output that also is the last channels of a wide tensor, that tensor's
+// gradient; for an output that is the first channels of a wide tensor (join), that tensor's gradient alone.
+struct OutputGrad {
+    const void *a, *b = nullptr;
+    int pitch = 0, pitch2 = 0;
+};
+OutputGrad output_grad(const at::Tensor& dy, const at::Tensor* dskip, bool join, const at::Tensor& x) {
+    const int64_t c = x.size(-1);
+    require_half_rows(dy, x, join ? 2 * c : c, "dy does not have the output's shape");
+    OutputGrad g{ptr(dy)};
+    if (join) g.pitch = static_cast<int>(2 * c);
+    if (dskip) {
+        require_half_rows(*dskip, x, 2 * c, "the wide gradient has twice the channels");
+        g.b = channels_from(*dskip, c);
+        g.pitch2 = static_cast<int>(2 * c);
+    }
+    return g;
+}
+
+// bn_forward(x, residual, gamma, beta, act, slope, eps, join, skip, workspace) -> (y, wide, mean, rstd, mask): y is join's
+// storage where one is given; the mask of y > 0 where the backward cannot tell it from x, else None
 PyObject* py_bn_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (!arity(n, 8)) return nullptr;
+    if (!arity(n, 10)) return nullptr;
     return guarded([&]() -> PyObject* {
         const at::Tensor &x = tensor(a[0], "x"), &gamma = tensor(a[2], "gamma"), &beta = tensor(a[3], "beta");
-        const at::Tensor* res = tensor_or_none(a[1], "residual");
+        const at::Tensor *res = tensor_or_none(a[1], "residual"), *join = tensor_or_none(a[7], "join");
         const int64_t c = x.size(-1), rows = x.numel() / c;
         const int act = static_cast<int>(as_int(a[4]));
-        const at::Tensor y = at::empty(x.sizes(), x.options());
+        if (join) require_half_rows(*join, x, 2 * c, "join has twice the channels of x");
+        const at::Tensor y = join ? join->variable_data() : at::empty(x.sizes(), x.options());
         const auto fopt = at::TensorOptions().dtype(at::kFloat).device(x.device());
         const at::Tensor mean = at::empty({c}, fopt), rstd = at::empty({c}, fopt);
-        at::Tensor mask;
-        const bool has_mask = res != nullptr && act != 0;
-        if (has_mask) mask = at::empty({x.numel() / 8}, fopt.dtype(at::kByte));
+        at::Tensor mask, wide;
+        if (res != nullptr && act != 0) mask = at::empty({x.numel() / 8}, fopt.dtype(at::kByte));
+        if (as_int(a[8]) != 0) wide = wide_like(x);
+        const int pitch = static_cast<int>(2 * c);
         size_t need = 0;
         check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
-        const Scratch ws = scratch(a[7], need, x);
+        const Scratch ws = scratch(a[9], need, x);
         check(nml_bn_forward_masked(ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)),
                                     static_cast<const float*>(ptr(beta)), ptr_or_null(res), act, static_cast<float>(as_double(a[5])),
-                                    static_cast<float>(as_double(a[6])), ptr(y), has_mask ? ptr(mask) : nullptr,
+                                    static_cast<float>(as_double(a[6])), ptr(y), join ? pitch : 0,
+                                    wide.defined() ? channels_from(wide, c) : nullptr, pitch, mask.defined() ? ptr(mask) : nullptr,
                                     static_cast<float*>(ptr(mean)), static_cast<float*>(ptr(rstd)), ws.p, ws.bytes, stream()));
-        PyObject* t = PyTuple_New(4);
-        PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(y));
-        PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(mean));
-        PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(rstd));
-        PyTuple_SET_ITEM(t, 3, has_mask ? THPVariable_Wrap(mask) : Py_NewRef(Py_None));
-        return t;
+        return tuple_of(y, wide, mean, rstd, mask);
     });
 }
 
-// bn_backward(dy, mask, x, gamma, beta, mean, rstd, act, slope, want_residual_grad, dgamma, dbeta, workspace) -> (dx, dres)
+// bn_backward(dy, dwide, join, mask, x, gamma, beta, mean, rstd, act, slope, want_residual_grad, dgamma, dbeta, workspace)
+// -> (dx, dres)
 PyObject* py_bn_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (!arity(n, 13)) return nullptr;
+    if (!arity(n, 15)) return nullptr;
     return guarded([&]() -> PyObject* {
-        const at::Tensor &dy = tensor(a[0], "dy"), &x = tensor(a[2], "x"), &gamma = tensor(a[3], "gamma"), &beta = tensor(a[4], "beta"),
-                         &mean = tensor(a[5], "mean"), &rstd = tensor(a[6], "rstd"), &dgamma = tensor(a[10], "dgamma"), &dbeta = tensor(a[11], "dbeta");
-        const at::Tensor* mask = tensor_or_none(a[1], "mask");
+        const at::Tensor &dy = tensor(a[0], "dy"), &x = tensor(a[4], "x"), &gamma = tensor(a[5], "gamma"), &beta = tensor(a[6], "beta"),
+                         &mean = tensor(a[7], "mean"), &rstd = tensor(a[8], "rstd"), &dgamma = tensor(a[12], "dgamma"), &dbeta = tensor(a[13], "dbeta");
+        const at::Tensor* mask = tensor_or_none(a[3], "mask");
         const int64_t c = x.size(-1), rows = x.numel() / c;
+        const OutputGrad g = output_grad(dy, tensor_or_none(a[1], "dwide"), as_int(a[2]) != 0, x);
         const at::Tensor dx = at::empty(x.sizes(), x.options());
         at::Tensor dres;
-        const bool has_res = as_int(a[9]) != 0;
-        if (has_res) dres = at::empty(x.sizes(), x.options());
+        if (as_int(a[11]) != 0) dres = at::empty(x.sizes(), x.options());
         size_t need = 0;
         check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
-        const Scratch ws = scratch(a[12], need, x);
-        check(nml_bn_backward_masked(ptr(dy), ptr_or_null(mask), ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)),
-                                     static_cast<const float*>(ptr(beta)), static_cast<const float*>(ptr(mean)),
-                                     static_cast<const float*>(ptr(rstd)), static_cast<int>(as_int(a[7])),
-                                     static_cast<float>(as_double(a[8])), ptr(dx), has_res ? ptr(dres) : nullptr,
-                                     static_cast<float*>(ptr(dgamma)), static_cast<float*>(ptr(dbeta)), ws.p, ws.bytes, stream()));
-        return pair(dx, has_res ? &dres : nullptr);
+        const Scratch ws = scratch(a[14], need, x);
+        check(nml_bn_backward_masked(g.a, g.pitch, g.b, g.pitch2, ptr_or_null(mask), ptr(x), rows, static_cast<int>(c),
+                                     static_cast<const float*>(ptr(gamma)), static_cast<const float*>(ptr(beta)),
+                                     static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)),
+                                     static_cast<int>(as_int(a[9])), static_cast<float>(as_double(a[10])), ptr(dx),
+                                     dres.defined() ? ptr(dres) : nullptr, static_cast<float*>(ptr(dgamma)),
+                                     static_cast<float*>(ptr(dbeta)), ws.p, ws.bytes, stream()));
+        return tuple_of(dx, dres);
+    });
+}
+
+// act_forward(x, act, slope, skip) -> (y, wide)
+PyObject* py_act_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (!arity(n, 4)) return nullptr;
+    return guarded([&]() -> PyObject* {
+        const at::Tensor& x = tensor(a[0], "x");
+        const int64_t c = x.size(-1);
+        require_half_rows(x, x, c, "x is float16");
+        const at::Tensor y = at::empty(x.sizes(), x.options());
+        at::Tensor wide;
+        if (as_int(a[3]) != 0) wide = wide_like(x);
+        check(nml_act_forward(ptr(x), x.numel() / c, static_cast<int>(c), static_cast<int>(as_int(a[1])), static_cast<float>(as_double(a[2])),
+                              ptr(y), wide.defined() ? channels_from(wide, c) : nullptr, static_cast<int>(2 * c), stream()));
+        return tuple_of(y, wide);
+    });
+}
+
+// act_backward(dy, dwide, x, act, slope) -> dx
+PyObject* py_act_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (!arity(n, 5)) return nullptr;
+    return guarded([&]() -> PyObject* {
+        const at::Tensor &dy = tensor(a[0], "dy"), &x = tensor(a[2], "x");
+        const int64_t c = x.size(-1);
+        const OutputGrad g = output_grad(dy, tensor_or_none(a[1], "dwide"), false, x);
+        const at::Tensor dx = at::empty(x.sizes(), x.options());
+        check(nml_act_backward(g.a, g.pitch, g.b, g.pitch2, ptr(x), x.numel() / c, static_cast<int>(c), static_cast<int>(as_int(a[3])),
+                               static_cast<float>(as_double(a[4])), ptr(dx), stream()));
+        return THPVariable_Wrap(dx);
+    });
+}
+
+// ------------------------------------------------------------------ loss --
+// l1_forward(a, b, denom, workspace) -> loss
+PyObject* py_l1_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (!arity(n, 4)) return nullptr;
+    return guarded([&]() -> PyObject* {
+        const at::Tensor &a = tensor(args[0], "a"), &b = tensor(args[1], "b");
+        require(a.scalar_type() == at::kHalf && b.scalar_type() == at::kHalf && a.numel() == b.numel(), "two float16 tensors of one size");
+        const at::Tensor loss = at::empty({}, a.options().dtype(at::kFloat));
+        size_t need = 0;
+        check(nml_l1_workspace_size(&need));
+        const Scratch ws = scratch(args[3], need, a);
+        check(nml_l1_forward(ptr(a), ptr(b), a.numel(), static_cast<float>(as_double(args[2])), static_cast<float*>(ptr(loss)), ws.p, ws.bytes,
+                             stream()));
+        return THPVariable_Wrap(loss);
+    });
+}
+
+// l1_backward(a, b, dloss, denom) -> da
+PyObject* py_l1_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (!arity(n, 4)) return nullptr;
+    return guarded([&]() -> PyObject* {
+        const at::Tensor &a = tensor(args[0], "a"), &b = tensor(args[1], "b"), &dloss = tensor(args[2], "dloss");
+        require(dloss.scalar_type() == at::kFloat && dloss.numel() == 1, "the gradient of the loss is one float32");
+        const at::Tensor da = at::empty(a.sizes(), a.options());
+        check(nml_l1_backward(ptr(a), ptr(b), a.numel(), static_cast<const float*>(ptr(dloss)), static_cast<float>(as_double(args[3])), ptr(da),
+                              stream()));
+        return THPVariable_Wrap(da);
     });
 }
 
 #define NML_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {NML_FAST(geometry), NML_FAST(conv_forward), NML_FAST(conv_backward_data), NML_FAST(conv_backward_weight),
                           NML_FAST(linear_forward), NML_FAST(linear_backward_data), NML_FAST(linear_backward_weight),
-                          NML_FAST(bn_forward), NML_FAST(bn_backward), {nullptr, nullptr, 0, nullptr}};
+                          NML_FAST(bn_forward), NML_FAST(bn_backward), NML_FAST(act_forward), NML_FAST(act_backward),
+                          NML_FAST(l1_forward), NML_FAST(l1_backward), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

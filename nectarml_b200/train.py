@@ -8,10 +8,10 @@
 
 What runs where: every Conv2d / ConvTranspose2d / Linear, forward, input-gradient and weight-gradient, is the
 C ABI's descriptor API on fp16 NHWC tensors that stay in that layout between layers; BatchNorm with the
-activation and residual add that follow it, the finiteness check and the SGD-momentum update are the
-library's own kernels (``nml_bn_*``, ``nml_grads_check``, ``nml_sgd_momentum_step``).  torch supplies device
-memory, the autograd tape that orders the calls, and the few remaining small ops (pooling, concatenation,
-tanh, the loss).  Parameters live in ONE flat fp32 buffer with an fp16 copy for the kernels; their gradients
+activation, residual add and concatenation that follow it, the L1 loss, the finiteness check and the
+SGD-momentum update are the library's own kernels (``nml_bn_*``, ``nml_act_*``, ``nml_l1_*``,
+``nml_grads_check``, ``nml_sgd_momentum_step``).  torch supplies device memory, the autograd tape that orders
+the calls, and the few remaining small ops (the global average pool, tanh, the cross-entropy loss).  Parameters live in ONE flat fp32 buffer with an fp16 copy for the kernels; their gradients
 are written by the weight-gradient kernels straight into ONE flat fp32 buffer, whose buckets are
 all-reduced over NCCL as the backward pass completes them (weight gradient before input gradient in every
 layer, so the exchange starts as early as it can).
@@ -222,28 +222,65 @@ class _LinearFn(torch.autograd.Function):
 
 
 class _BnActFn(torch.autograd.Function):
-    """y = act(batchnorm(x) [+ residual]) over the rows of an NHWC tensor (training statistics)."""
+    """y = act(batchnorm(x) [+ residual]) over the rows of an NHWC tensor (training statistics).
+
+    A concatenation [a, b] along the channels is built by the two layers whose outputs it holds, without a pass of its own:
+    the layer of b returns the wide tensor as a second output (``skip``), with b already in its last channels; the layer of a
+    is given that tensor (``join``), fills its first channels and returns it.  Both read their part of its gradient in place."""
 
     @staticmethod
-    def forward(ctx, x, residual, token, layer, act):
-        y, mean, rstd, mask = ops._native.bn_forward(x, residual, layer.gamma, layer.beta, act, 0.2, layer.eps, _bn_ws)
-        ctx.layer, ctx.act, ctx.has_res = layer, act, residual is not None
+    def forward(ctx, x, residual, token, layer, act, join, skip):
+        y, wide, mean, rstd, mask = ops._native.bn_forward(x, residual, layer.gamma, layer.beta, act, 0.2, layer.eps, join, skip, _bn_ws)
+        ctx.layer, ctx.act, ctx.has_res, ctx.join = layer, act, residual is not None, join is not None
         ctx.save_for_backward(x, mean, rstd, mask)
-        return y
+        return (y, wide) if skip else y
 
     @staticmethod
-    def backward(ctx, dy):
+    def backward(ctx, dy, dwide=None):
         layer = ctx.layer
         x, mean, rstd, mask = ctx.saved_tensors
         dy = dy.contiguous()
+        if dwide is not None:
+            dwide = dwide.contiguous()
         grads = None
 
         def run(dgamma, dbeta):
             nonlocal grads
-            grads = ops._native.bn_backward(dy, mask, x, layer.gamma, layer.beta, mean, rstd, ctx.act, 0.2, int(ctx.has_res),
-                                            dgamma, dbeta, _bn_ws)
+            grads = ops._native.bn_backward(dy, dwide, ctx.join, mask, x, layer.gamma, layer.beta, mean, rstd, ctx.act, 0.2,
+                                            ctx.has_res, dgamma, dbeta, _bn_ws)
         layer.weight_gradient(run)
-        return grads[0], grads[1], None, None, None
+        return grads[0], grads[1], None, None, None, dy if ctx.join else None, None
+
+
+class _ActFn(torch.autograd.Function):
+    """y = act(x) where no normalisation stands in front; ``skip`` as in _BnActFn."""
+
+    @staticmethod
+    def forward(ctx, x, act, skip):
+        y, wide = ops._native.act_forward(x, act, 0.2, skip)
+        ctx.act = act
+        ctx.save_for_backward(x)
+        return (y, wide) if skip else y
+
+    @staticmethod
+    def backward(ctx, dy, dwide=None):
+        (x,) = ctx.saved_tensors
+        return ops._native.act_backward(dy.contiguous(), None if dwide is None else dwide.contiguous(), x, ctx.act, 0.2), None, None
+
+
+class _L1Fn(torch.autograd.Function):
+    """sum |out - target| / denom of two fp16 tensors."""
+
+    @staticmethod
+    def forward(ctx, out, target, denom):
+        ctx.denom = denom
+        ctx.save_for_backward(out, target)
+        return ops._native.l1_forward(out, target, denom, _bn_ws)
+
+    @staticmethod
+    def backward(ctx, dloss):
+        out, target = ctx.saved_tensors
+        return ops._native.l1_backward(out, target, dloss, ctx.denom), None, None
 
 
 class _MaxPoolFn(torch.autograd.Function):
@@ -359,8 +396,11 @@ class BatchNormAct(_Layer):
     @property
     def beta(self): return self.store.w32(self.ib)
 
-    def __call__(self, x, token, act=ACT_RELU, residual=None):
-        return self.store.record(_BnActFn.apply(x, residual, token, self, act))
+    def __call__(self, x, token, act=ACT_RELU, residual=None, join=None, skip=False):
+        out = _BnActFn.apply(x, residual, token, self, act, join, skip)
+        if self.store.trace is not None:
+            self.store.record(out[0] if skip else out if join is None else out[..., :x.shape[-1]])
+        return out
 
 
 # ------------------------------------------------------------------ models --
@@ -376,6 +416,7 @@ class _Net:
         # kept across steps: tensors of an earlier, uncaptured pass that die INSIDE a later stream capture
         # invalidate the capture (their allocator bookkeeping records events on the streams they crossed).
         self.frontier = None
+        self.wants_frontier = False   # set around a forward() whose backward is to be split
 
     def _finish(self, n_buckets):
         self.store.finalize(n_buckets)
@@ -468,6 +509,7 @@ class Pix2PixGenerator(_Net):
             self.up.append((Conv(s, ci, co, 4, 2, 1, transposed=True), BatchNormAct(s, co)))
             c = co
         self.final = Conv(s, c * 2, in_channels, 4, 2, 1, bias=True, transposed=True)
+        self.frontier_first_param = self.up[0][0].first   # decoder (and final layer) parameters start here
         self._finish(3)
 
     def init(self, seed=0):
@@ -484,30 +526,29 @@ class Pix2PixGenerator(_Net):
     def forward(self, x):
         """x: [N, H, W, 3] fp16 NHWC in [-1, 1] -> generated image, same shape."""
         t = self.token
-        skips = []
+        skips = []   # the tensors the decoder's convolutions read, the encoder's half of their channels filled in
         for i, (conv, bn) in enumerate(self.down):
             y = conv(x, t)
+            last = i == len(self.down) - 1   # the bottleneck: no concatenation reads it
             if bn is not None:
-                x = bn(y, t, ACT_LEAKY)
-            elif i == 0:
-                x = self.store.record(torch.nn.functional.leaky_relu(y, 0.2))
+                out = bn(y, t, ACT_LEAKY, skip=not last)
             else:
-                x = self.store.record(torch.relu(y))       # bottleneck
-            skips.append(x)
-        skips.pop()
-        # The frontier between decoder and encoder in the backward pass: the bottleneck's output as the decoder
-        # reads it and the encoder activations as the concatenations read them (views, so that each is its own
-        # autograd node).  A split backward (TrainStep.capture_split) stops here, sends the decoder's gradients
-        # off, and then continues into the encoder.
-        x = x.view_as(x)
-        skips = [d.view_as(d) for d in skips]
-        self.frontier = [x] + list(skips)   # (dropped again by whoever ran the backward pass: see TrainStep)
-        self.frontier_first_param = self.up[0][0].first   # decoder (and final layer) parameters start here
-        for i, (conv, bn) in enumerate(self.up):
-            if i > 0:
-                x = torch.cat((x, skips.pop()), dim=3)
-            x = bn(conv(x, t), t, ACT_RELU)
-        x = torch.cat((x, skips.pop()), dim=3)
+                out = _ActFn.apply(y, ACT_RELU if last else ACT_LEAKY, not last)
+                self.store.record(out if last else out[0])
+            if last:
+                x = out
+            else:
+                x, wide = out
+                skips.append(wide)
+        if self.wants_frontier:
+            # The frontier between decoder and encoder in the backward pass: the bottleneck's output as the decoder reads
+            # it and the wide tensors (views, so that each is its own autograd node).  A split backward
+            # (TrainStep.capture_split) stops here, sends the decoder's gradients off, and then continues into the encoder.
+            x = x.view_as(x)
+            skips = [d.view_as(d) for d in skips]
+            self.frontier = [x] + list(skips)   # (dropped again by whoever ran the backward pass: see TrainStep)
+        for conv, bn in self.up:
+            x = bn(conv(x, t), t, ACT_RELU, join=skips.pop())
         return self.store.record(torch.tanh(self.final(x, t)))
 
 
@@ -523,6 +564,9 @@ class TrainStep:
     def _loss(self, out, target, denom):
         if self.loss_kind == "cross_entropy":
             return torch.nn.functional.cross_entropy(out.float(), target, reduction="sum") / denom
+        if (out.is_cuda and out.dtype == target.dtype == torch.float16 and out.shape == target.shape and out.is_contiguous()
+                and target.is_contiguous() and not target.requires_grad and out.numel() > 0):
+            return _L1Fn.apply(out, target, float(denom))
         return (out.float() - target.float()).abs().sum() / denom     # L1 against the target image
 
     def micro_batch(self, x, target, global_count, first: bool, last: bool) -> torch.Tensor:
@@ -532,9 +576,8 @@ class TrainStep:
         store.begin_backward(last_micro_batch=last)
         out = self.net.forward(x)
         loss = self._loss(out, target, global_count)
-        (loss * self.loss_scale).backward()
+        loss.backward(torch.full_like(loss, self.loss_scale))
         store.accumulate = False
-        self.net.frontier = None
         return loss.detach()
 
     def capture(self, x, target, global_count: int, accumulate_variants=(False,)):
@@ -575,9 +618,13 @@ class TrainStep:
         def part_a():
             store.accumulate = False
             store.begin_backward(last_micro_batch=False)
-            out = net.forward(x)
+            net.wants_frontier = True
+            try:
+                out = net.forward(x)
+            finally:
+                net.wants_frontier = False
             loss = self._loss(out, target, global_count)
-            grads = torch.autograd.grad(loss * self.loss_scale, net.frontier)
+            grads = torch.autograd.grad(loss, net.frontier, torch.full_like(loss, self.loss_scale))
             return loss.detach(), grads
 
         def part_b(grads):
@@ -633,16 +680,16 @@ class TrainStep:
         """micro_batches: list of (input NHWC fp16, target); global_count: samples (cross-entropy) or elements (L1)
         of the GLOBAL batch, the divisor of the summed loss.  Returns this rank's share of the mean loss."""
         store = self.net.store
-        total = torch.zeros((), device=self.net.device)
+        total = None
         for i, (x, target) in enumerate(micro_batches):
             store.accumulate = i > 0
             store.begin_backward(last_micro_batch=(i == len(micro_batches) - 1))
             out = self.net.forward(x)
             loss = self._loss(out, target, global_count)
-            (loss * self.loss_scale).backward()
-            total += loss.detach()
+            loss.backward(torch.full_like(loss, self.loss_scale))
+            total = loss.detach() if total is None else total + loss.detach()
         store.accumulate = False
         store.wait_exchange()
         if optimize:
             store.sgd_step(self.lr, self.momentum, self.wd, 1.0 / self.loss_scale)
-        return total
+        return total if total is not None else torch.zeros((), device=self.net.device)

@@ -74,9 +74,9 @@ def test_batch_norm_backward_with_and_without_y(rows, c, act, with_res):
         mask = torch.zeros(rows * c // 8, dtype=torch.uint8, device="cuda") if with_res else None
         mean, rstd, dg, db = (torch.empty(c, device="cuda") for _ in range(4))
         if masked:
-            _lib.check(lib.nml_bn_forward_masked(p(x), rows, c, p(gamma), p(beta), p(res), act, 0.2, 1e-5, p(y), p(mask), p(mean), p(rstd),
-                                                 p(ws), need.value, st))
-            _lib.check(lib.nml_bn_backward_masked(p(dy), p(mask), p(x), rows, c, p(gamma), p(beta), p(mean), p(rstd), act, 0.2, p(dx),
+            _lib.check(lib.nml_bn_forward_masked(p(x), rows, c, p(gamma), p(beta), p(res), act, 0.2, 1e-5, p(y), 0, None, 0, p(mask),
+                                                 p(mean), p(rstd), p(ws), need.value, st))
+            _lib.check(lib.nml_bn_backward_masked(p(dy), 0, None, 0, p(mask), p(x), rows, c, p(gamma), p(beta), p(mean), p(rstd), act, 0.2, p(dx),
                                                   p(dres), p(dg), p(db), p(ws), need.value, st))
         else:
             _lib.check(lib.nml_bn_forward(p(x), rows, c, p(gamma), p(beta), p(res), act, 0.2, 1e-5, p(y), p(mean), p(rstd), p(ws),
@@ -137,3 +137,62 @@ def test_weight_gradient_plans(rows, fin, fout, math):
     assert float((dw.double() - want).norm() / want.norm()) < 2e-5
     assert float((dw.double() - want).abs().max()) < 1e-4 * rows ** 0.5
     assert float((db.double() - dy.double().sum(0)).abs().max()) < 1e-5 * rows ** 0.5 * 10
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (5, 64), (1000, 24), (37, 2048)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_outputs_as_channels_of_a_concatenation(rows, c, norm):
+    """Two layers whose outputs meet in a concatenation, written and differentiated in place: the values are the separate
+    layers' bits, the gradient of an output read twice is the sum of both (fp16 once at the end, and once in each of
+    the two parts of the normalisation's dx it is compared with, which may cancel: half an ulp, 2**-11, of all three).  The normalisation's dx is itself a difference of fp32
+    terms of at most gamma * rstd * max|dz| * (2 + |xhat|), |xhat| below 6 here: a few roundings of 8 times that (one row:
+    the terms cancel to nothing, rstd is 316)."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + c)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
+    x, z, dy, dcat = rnd(rows, c).half(), rnd(rows, c).half(), rnd(rows, c).half(), rnd(rows, 2 * c).half()
+    gamma, beta, ws, n = rnd(c), rnd(c), ops.Workspace(), ops._native
+    empty = lambda: (torch.empty(c, device="cuda"), torch.empty(c, device="cuda"))  # noqa: E731
+    dsum = (dy.float() + dcat[:, c:].float())
+    if norm:
+        y0, none, mean, rstd, _ = n.bn_forward(x, None, gamma, beta, 2, 0.2, 1e-5, None, False, ws)
+        assert none is None
+        y, wide, *_ = n.bn_forward(x, None, gamma, beta, 2, 0.2, 1e-5, None, True, ws)
+        (dg, db), (dg2, db2) = empty(), empty()
+        dx = n.bn_backward(dy, dcat, False, None, x, gamma, beta, mean, rstd, 2, 0.2, False, dg, db, ws)[0]
+        both = [n.bn_backward(d, None, False, None, x, gamma, beta, mean, rstd, 2, 0.2, False, dg2, db2, ws)[0].float()
+                for d in (dy, dcat[:, c:].contiguous())]
+        want, size = both[0] + both[1], both[0].abs() + both[1].abs()
+        terms = gamma.abs() * rstd * dsum.abs().max()
+        # the join: z's layer fills the first channels and reads its part of the gradient
+        a0, _, m2, r2, _ = n.bn_forward(z, None, gamma, beta, 1, 0.2, 1e-5, None, False, ws)
+        cat = n.bn_forward(z, None, gamma, beta, 1, 0.2, 1e-5, wide, False, ws)[0]
+        assert cat.data_ptr() == wide.data_ptr() and torch.equal(cat, torch.cat((a0, y0), dim=1))
+        got = n.bn_backward(dcat, None, True, None, z, gamma, beta, m2, r2, 1, 0.2, False, dg, db, ws)[0]
+        sep = n.bn_backward(dcat[:, :c].contiguous(), None, False, None, z, gamma, beta, m2, r2, 1, 0.2, False, dg2, db2, ws)[0]
+        assert torch.equal(got, sep) and torch.equal(dg, dg2) and torch.equal(db, db2)
+    else:
+        y0, _ = n.act_forward(x, 2, 0.2, False)
+        y, wide = n.act_forward(x, 2, 0.2, True)
+        assert torch.equal(y0, torch.nn.functional.leaky_relu(x, 0.2))
+        dx = n.act_backward(dy, dcat, x, 2, 0.2)
+        want = dsum * torch.where(x > 0, 1.0, 0.2)
+        size, terms = want.abs(), 0.0
+    ops.device_status()
+    assert torch.equal(y, y0) and torch.equal(wide[:, c:], y0)
+    assert bool(((dx.float() - want).abs() <= 2.0 ** -11 * (want.abs() + size) + 2.0 ** -23 + 64 * 2.0 ** -24 * terms).all())
+
+
+@pytest.mark.parametrize("n", [1, 2, 511, 4097, 3 * 64 * 64 * 5])
+def test_l1_loss(n):
+    """Sum in fp32 of n values below 8, in shares: n * 2**-24 relative at the very most."""
+    from nectarml_b200 import train
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.randn(n, device="cuda", generator=gen).half().requires_grad_()
+    b = torch.randn(n, device="cuda", generator=gen).half()
+    b[::3] = a.detach()[::3]
+    loss = train._L1Fn.apply(a, b, 7.0)
+    loss.backward(torch.full_like(loss, 16384.0))
+    d = a.detach().double() - b.double()
+    want = float(d.abs().sum() / 7.0)
+    assert abs(float(loss.detach()) - want) <= (n * 2.0 ** -24 + 2.0 ** -22) * want
+    assert torch.equal(a.grad, (torch.sign(d).float() * (torch.tensor(16384.0) / 7.0).item()).half())

@@ -63,7 +63,7 @@ class ParamStore:
         self.offsets: List[int] = []
         self.n = 0
         self.p32 = self.p16 = self.grad = self.vel = None
-        self.accumulate = False          # True from the second micro-batch of a step on
+        self.flags = bytearray(2)        # read by the layers' backward: see `accumulate` and `_exchange`
         self.scratch: Optional[torch.Tensor] = None
         self.layer_ranges: List[Tuple[int, int]] = []   # (first element, end) of every layer, forward order
         self.bucket_bounds: List[int] = []
@@ -73,6 +73,24 @@ class ParamStore:
         self.communicate = True
         self.flops = 0.0                 # algorithmic FLOPs of the contraction passes since it was last zeroed
         self.trace: Optional[list] = None  # when a list: every nonlinearity's output is appended (test support)
+
+    @property
+    def accumulate(self) -> bool:
+        """True from the second micro-batch of a step on: gradients add to the flat buffer."""
+        return bool(self.flags[0])
+
+    @accumulate.setter
+    def accumulate(self, value) -> None:
+        self.flags[0] = bool(value)
+
+    @property
+    def _exchange(self) -> bool:
+        """This backward pass sends the buckets off as its layers complete them."""
+        return bool(self.flags[1])
+
+    @_exchange.setter
+    def _exchange(self, value) -> None:
+        self.flags[1] = bool(value)
 
     def record(self, t):
         if self.trace is not None:
@@ -178,31 +196,7 @@ _bn_ws = ops.Workspace()
 
 
 # ------------------------------------------------------------------ autograd nodes --
-class _ConvFn(torch.autograd.Function):
-    """Conv2d / ConvTranspose2d on fp16 NHWC through the descriptor API; the weight gradient goes straight
-    into the flat gradient buffer (before the input gradient, so that its bucket can leave early)."""
-
-    @staticmethod
-    def forward(ctx, x, token, layer):
-        g = layer.geometry(x)
-        y = ops.conv_forward(g, x, layer.w16, layer.b16, layout="nhwc")
-        pix = x.shape[1] * x.shape[2] if layer.transposed else y.shape[1] * y.shape[2]  # a transposed layer multiplies per input pixel
-        layer.store.flops += (3 if layer.needs_dx else 2) * 2.0 * x.shape[0] * pix * g.c_out * g.c_in * g.kh * g.kw
-        ctx.layer, ctx.g = layer, g
-        ctx.save_for_backward(x)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        layer, g = ctx.layer, ctx.g
-        (x,) = ctx.saved_tensors
-        dy = dy.contiguous()
-        layer.weight_gradient(lambda dw, db: ops.conv_backward_weight(g, x, dy, layout="nhwc", dw=dw, db=db,
-                                                                        want_bias_grad=db is not None))
-        dx = ops.conv_backward_data(g, dy, layer.w16, layout="nhwc") if layer.needs_dx else None
-        return dx, None, None
-
-
+# (those of Conv and BatchNormAct are native: csrc/nml_torch.cpp)
 class _LinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, token, layer):
@@ -221,39 +215,8 @@ class _LinearFn(torch.autograd.Function):
         return ops.linear_backward_data(dy, layer.w16), None, None
 
 
-class _BnActFn(torch.autograd.Function):
-    """y = act(batchnorm(x) [+ residual]) over the rows of an NHWC tensor (training statistics).
-
-    A concatenation [a, b] along the channels is built by the two layers whose outputs it holds, without a pass of its own:
-    the layer of b returns the wide tensor as a second output (``skip``), with b already in its last channels; the layer of a
-    is given that tensor (``join``), fills its first channels and returns it.  Both read their part of its gradient in place."""
-
-    @staticmethod
-    def forward(ctx, x, residual, token, layer, act, join, skip):
-        y, wide, mean, rstd, mask = ops._native.bn_forward(x, residual, layer.gamma, layer.beta, act, 0.2, layer.eps, join, skip, _bn_ws)
-        ctx.layer, ctx.act, ctx.has_res, ctx.join = layer, act, residual is not None, join is not None
-        ctx.save_for_backward(x, mean, rstd, mask)
-        return (y, wide) if skip else y
-
-    @staticmethod
-    def backward(ctx, dy, dwide=None):
-        layer = ctx.layer
-        x, mean, rstd, mask = ctx.saved_tensors
-        dy = dy.contiguous()
-        if dwide is not None:
-            dwide = dwide.contiguous()
-        grads = None
-
-        def run(dgamma, dbeta):
-            nonlocal grads
-            grads = ops._native.bn_backward(dy, dwide, ctx.join, mask, x, layer.gamma, layer.beta, mean, rstd, ctx.act, 0.2,
-                                            ctx.has_res, dgamma, dbeta, _bn_ws)
-        layer.weight_gradient(run)
-        return grads[0], grads[1], None, None, None, dy if ctx.join else None, None
-
-
 class _ActFn(torch.autograd.Function):
-    """y = act(x) where no normalisation stands in front; ``skip`` as in _BnActFn."""
+    """y = act(x) where no normalisation stands in front; ``skip`` as in BatchNormAct."""
 
     @staticmethod
     def forward(ctx, x, act, skip):
@@ -342,6 +305,10 @@ class _Layer:
                 gb.add_(tb)
         s.layer_done(self.first)
 
+    def gradient_written(self) -> None:
+        """The native layers' report that their gradients are in the flat buffer (called while buckets are exchanged)."""
+        self.store.layer_done(self.first)
+
 
 class Conv(_Layer):
     def __init__(self, store, c_in, c_out, k, stride, pad, bias=False, transposed=False, needs_dx=True):
@@ -356,21 +323,32 @@ class Conv(_Layer):
     @property
     def b16(self): return self.store.w16(self.ib) if self.ib is not None else None
 
-    def geometry(self, x) -> ConvGeometry:
+    def geometry(self, x) -> Tuple[ConvGeometry, float]:
+        """The layer's geometry for this input, and the algorithmic FLOPs of its passes."""
         shape = tuple(x.shape)
-        g = self._geometries.get(shape)
-        if g is None:
+        hit = self._geometries.get(shape)
+        if hit is None:
             n, h, w, c = shape
             assert c == self.c_in, (c, self.c_in)
             g = ConvGeometry(n, c, h, w, self.c_out, self.k, self.k, (self.stride, self.stride), (self.pad, self.pad),
                              transposed=self.transposed)
+            ho, wo = g.out_hw()
+            pix = h * w if self.transposed else ho * wo  # a transposed layer multiplies per input pixel
+            flops = (3 if self.needs_dx else 2) * 2.0 * n * pix * self.c_out * self.c_in * self.k * self.k
             if len(self._geometries) >= 16:  # (a program with ever new image sizes)
                 self._geometries.clear()
-            self._geometries[shape] = g
-        return g
+            hit = self._geometries[shape] = (g, flops)
+        return hit
 
     def __call__(self, x, token):
-        return _ConvFn.apply(x, token, self)
+        """Conv2d / ConvTranspose2d on fp16 NHWC.  The weight gradient goes straight into the flat gradient buffer (before
+        the input gradient, so that its bucket can leave early)."""
+        g, flops = self.geometry(x)
+        s = self.store
+        y = ops._native.conv_layer(g.native(), x, token, self.w16, self.b16, s.g32(self.ia), s.g32(self.ib) if self.ib is not None else None,
+                                   self.needs_dx, self, s.flags, ops._default_ws)
+        s.flops += flops
+        return y
 
 
 class Linear(_Layer):
@@ -397,7 +375,15 @@ class BatchNormAct(_Layer):
     def beta(self): return self.store.w32(self.ib)
 
     def __call__(self, x, token, act=ACT_RELU, residual=None, join=None, skip=False):
-        out = _BnActFn.apply(x, residual, token, self, act, join, skip)
+        """y = act(batchnorm(x) [+ residual]) over the rows of an NHWC tensor (training statistics).
+
+        A concatenation [a, b] along the channels is built by the two layers whose outputs it holds, without a pass of its
+        own: the layer of b returns the wide tensor as a second output (``skip``), with b already in its last channels; the
+        layer of a is given that tensor (``join``), fills its first channels and returns it.  Both read their part of its
+        gradient in place."""
+        s = self.store
+        out = ops._native.bn_layer(x, residual, token, join, self.gamma, self.beta, s.g32(self.ia), s.g32(self.ib), act, 0.2, self.eps,
+                                   skip, self, s.flags, _bn_ws)
         if self.store.trace is not None:
             self.store.record(out[0] if skip else out if join is None else out[..., :x.shape[-1]])
         return out

@@ -366,7 +366,7 @@ static bool repack_half(const void* src, void* dst, int B, int R, int Cc, int Rp
         helper_launch(4 * kSms, repack_half_tile_kernel, dim3(ceil_div(Cc, 64), ceil_div(Rp, 64), B), 256, 0, st, w, o, R, Cc, Rp);
     } else {
         if ((static_cast<size_t>(R) * Cc) % 8) return false;
-        helper_launch(4 * kSms, repack_half_rows_kernel, dim3(ceil_div(Rp, 256), B), 256, 256 * (Cc | 1) * sizeof(__half), st, w, o, R, Cc, Rp);
+        helper_launch(4 * kSms, repack_half_rows_kernel, dim3(ceil_div(Rp, 256), B), 256, 256 * repack_rows_pitch(Cc) * sizeof(__half), st, w, o, R, Cc, Rp);
     }
     ++g_launches;
     return true;
@@ -1635,9 +1635,9 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             const size_t total4 = dw_elems / 4;
             const int blocks = static_cast<int>(std::min<size_t>((total4 + 255) / 256, 148 * 16));
             helper_launch(4 * kSms, wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
-        } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535) {
-            helper_launch(4 * kSms, wgrad_reduce_taps_kernel, dim3(ceil_div(g.patch_c, 64), g.plain_c), 256, 64 * (P.n_taps | 1) * sizeof(float), st,
-                         planes, g.dw, split, plane_elems, g.patch_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
+        } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535 && kReducePlain * 64 * (P.n_taps | 1) * sizeof(float) <= 48 * 1024) {
+            helper_launch(4 * kSms, wgrad_reduce_taps_kernel, dim3(ceil_div(g.patch_c, 64), ceil_div(g.plain_c, kReducePlain)), 256,
+                         kReducePlain * 64 * (P.n_taps | 1) * sizeof(float), st, planes, g.dw, split, plane_elems, g.patch_c, g.plain_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
         } else {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + 255) / 256, 148 * 16));

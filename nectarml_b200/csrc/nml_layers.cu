@@ -27,6 +27,7 @@ namespace nml_layers {
     } while (0)
 
 using nml::launch;
+using nml::launch_with;
 using nml::pdl_enter;
 
 static inline size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
@@ -686,7 +687,8 @@ int nml_bn_forward_masked(const void* x, long long rows, int channels, const flo
     launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels);
     launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
            nullptr, nullptr, mean, rstd);
-    launch(bn_apply_kernel, bn_grid_elementwise(rows, channels, kApplyBlocks), threads, 0, st, xv, static_cast<const uint4*>(residual),
+    // (overlapping, whatever its grid: the second stage in front of it leaves every SM room for four of its blocks)
+    launch_with(true, 1, bn_apply_kernel, bn_grid_elementwise(rows, channels, kApplyBlocks), threads, 0, st, xv, static_cast<const uint4*>(residual),
            static_cast<uint4*>(y), row_vectors(y_pitch, channels), static_cast<uint4*>(y2), row_vectors(y2_pitch, channels),
            static_cast<uint8_t*>(mask), gamma, beta, mean, rstd, act, slope, M, channels);
     NMLL_CUDA(cudaGetLastError());
@@ -708,7 +710,7 @@ static void bn_backward_launch(const uint4* x, long long rows, int channels, int
                : deriv == D_X ? bn_dx_kernel<D_X, kTwo> : bn_dx_kernel<D_MASK, kTwo>;
     launch(sums, P, threads, 0, st, x, dy, f, partial, M, channels);
     launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 1, 0.0, 0.f, f.mean, f.rstd, dbeta, dgamma);
-    launch(apply, bn_grid_elementwise(rows, channels, kDxBlocks), threads, 0, st, x, dy, f, static_cast<uint4*>(dx),
+    launch_with(true, 1, apply, bn_grid_elementwise(rows, channels, kDxBlocks), threads, 0, st, x, dy, f, static_cast<uint4*>(dx),
            static_cast<uint4*>(dres), dbeta, dgamma, static_cast<float>(1.0 / static_cast<double>(rows)), M, channels);
 }
 static int bn_backward(const void* x, long long rows, int channels, int deriv, const OutGrad& dy, const BnForward& f, void* dx, void* dres,

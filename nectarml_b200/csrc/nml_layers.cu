@@ -9,6 +9,7 @@
 //     nectarml/csrc/ops/amp/amp.cpp:18-37, and one update launch per parameter,
 //     nectarml/optim/sgd.py:75-90, nectarml/csrc/kernels/optim/sgd.cu).
 // Every reduction is two-stage with a fixed order (no atomics): results are bitwise repeatable.
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -407,6 +408,245 @@ __global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__
     }
 }
 
+// ---- Small tensors: a whole pass in one launch.
+// The three kernels of a pass spend 8 to 10 us on a tensor of a few KB: launches, drains and load latency.
+// Here a cluster of eight blocks owns 8 * gv channels: each block reads its eighth of the rows once into shared memory and sums
+// as it goes, the blocks exchange their sums through distributed shared memory, and every thread finishes its own vectors.
+// No second read, no partial sums in memory, and the order of every sum is fixed.
+constexpr int kClusterBlocks = 8, kClusterThreads = 256;
+constexpr int kMaxGv = 16;                       // channels: at most 2048, in about 16 clusters
+constexpr size_t kClusterShare = 32 * 1024;      // of each tensor per block
+
+// Sums of a thread's (a, b) over its block and the cluster; then finish(channel of the cluster's, sum a, sum b) once per
+// channel, before the block goes on.
+template <class F>
+__device__ __forceinline__ void cluster_sums(const float (&a)[8], const float (&b)[8], int gv, float (*part)[16 * kMaxGv], F&& finish) {
+    namespace cg = cooperative_groups;
+    auto cluster = cg::this_cluster();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = a[j], v[8 + j] = b[j];
+    for (int o = 16; o >= gv; o /= 2) {  // lanes of one vector column are gv apart
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+    }
+    if (lane < gv) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) part[warp][lane * 16 + j] = v[j];
+    }
+    __syncthreads();
+    const int n = 16 * gv;  // at most kClusterThreads
+    float* mine = part[kClusterThreads / 32];
+    if (threadIdx.x < n) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < kClusterThreads / 32; ++w) s += part[w][threadIdx.x];
+        mine[threadIdx.x] = s;
+    }
+    cluster.sync();
+    if (threadIdx.x < n / 2) {
+        const int i = threadIdx.x / 8 * 16 + threadIdx.x % 8;
+        double ta = 0.0, tb = 0.0;
+#pragma unroll
+        for (int r = 0; r < kClusterBlocks; ++r) {
+            const float* theirs = cluster.map_shared_rank(mine, r);
+            ta += static_cast<double>(theirs[i]);
+            tb += static_cast<double>(theirs[i + 8]);
+        }
+        finish(static_cast<int>(threadIdx.x), ta, tb);
+    }
+    __syncthreads();
+}
+
+struct ClusterShare {  // a block's share of the tensor and a thread's place in it
+    size_t first, last;
+    int col, lane, lanes;
+};
+__device__ __forceinline__ ClusterShare cluster_share(size_t M, int gv) {
+    ClusterShare s;
+    const int rank = blockIdx.x % kClusterBlocks;
+    const size_t per = (M + kClusterBlocks - 1) / kClusterBlocks;
+    s.first = min(M, rank * per);
+    s.last = min(M, s.first + per);
+    s.lanes = kClusterThreads / gv;
+    s.lane = threadIdx.x / gv;
+    s.col = blockIdx.x / kClusterBlocks * gv + threadIdx.x % gv;
+    return s;
+}
+
+__global__ void __launch_bounds__(kClusterThreads) bn_cluster_forward_kernel(
+    const uint4* __restrict__ x, const uint4* __restrict__ res, uint4* __restrict__ y, int y_row, uint4* __restrict__ y2, int y2_row,
+    uint8_t* __restrict__ mask, const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ mean,
+    float* __restrict__ rstd, int act, float slope, float eps, double inv_M, size_t M, int C, int gv) {
+    pdl_enter();
+    extern __shared__ uint4 keep[];
+    __shared__ float part[kClusterThreads / 32 + 1][16 * kMaxGv];
+    __shared__ float done[2][8 * kMaxGv];  // per channel of the cluster's
+    const int cpr = C >> 3;
+    const ClusterShare s = cluster_share(M, gv);
+    float a[8], b[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int kFlight = 8;  // rows a thread has in flight
+    int k = threadIdx.x;
+    for (size_t row = s.first + s.lane; row < s.last; row += kFlight * s.lanes, k += kFlight * kClusterThreads) {
+        uint4 v[kFlight];
+#pragma unroll
+        for (int i = 0; i < kFlight; ++i) v[i] = row + i * s.lanes < s.last ? __ldg(x + (row + i * s.lanes) * cpr + s.col) : zero;
+#pragma unroll
+        for (int i = 0; i < kFlight; ++i) {
+            float f[8];
+            unpack8(v[i], f);
+            if (row + i * s.lanes < s.last) keep[k + i * kClusterThreads] = v[i];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                a[j] += f[j];
+                b[j] += f[j] * f[j];
+            }
+        }
+    }
+    const int c0 = blockIdx.x / kClusterBlocks * gv * 8;
+    cluster_sums(a, b, gv, part, [&](int c, double ta, double tb) {
+        const double m = ta * inv_M;
+        double var = tb * inv_M - m * m;
+        if (var < 0.0) var = 0.0;
+        done[0][c] = static_cast<float>(m);
+        done[1][c] = static_cast<float>(1.0 / sqrt(var + static_cast<double>(eps)));
+        if (blockIdx.x % kClusterBlocks == 0) {
+            mean[c0 + c] = done[0][c];
+            rstd[c0 + c] = done[1][c];
+        }
+    });
+    float sc[8], sh[8];
+    load8_or(gamma, s.col, 1.f, sc);
+    load8_or(beta, s.col, 0.f, sh);
+    const int base = threadIdx.x % gv * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        sc[j] *= done[1][base + j];
+        sh[j] -= done[0][base + j] * sc[j];
+    }
+    k = threadIdx.x;
+#pragma unroll 2
+    for (size_t row = s.first + s.lane; row < s.last; row += s.lanes, k += kClusterThreads) {
+        float f[8], rf[8];
+        unpack8(keep[k], f);
+        if (res) unpack8(__ldg(res + row * cpr + s.col), rf);
+        unsigned bits = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float t = f[j] * sc[j] + sh[j];
+            if (res) t += rf[j];
+            bits |= (positive_as_half(t) ? 1u : 0u) << j;
+            if (act != 0 && t < 0.f) t = (act == 1) ? 0.f : t * slope;
+            f[j] = t;
+        }
+        const uint4 out = pack8(f);
+        y[row * y_row + s.col] = out;
+        if (y2) y2[row * y2_row + s.col] = out;
+        if (mask) mask[row * cpr + s.col] = static_cast<uint8_t>(bits);
+    }
+    cooperative_groups::this_cluster().sync();  // no block leaves while another reads its sums
+}
+
+template <int kDeriv, bool kTwo>
+__global__ void __launch_bounds__(kClusterThreads) bn_cluster_backward_kernel(
+    const uint4* __restrict__ x, const OutGrad dy, const BnForward f, uint4* __restrict__ dx, uint4* __restrict__ dres,
+    float* __restrict__ dbeta, float* __restrict__ dgamma, double inv_M, size_t M, int C, int gv) {
+    pdl_enter();
+    extern __shared__ uint4 keep[];  // [x, dy (, second dy)][share]
+    __shared__ float part[kClusterThreads / 32 + 1][16 * kMaxGv];
+    __shared__ float done[2][8 * kMaxGv];  // per channel of the cluster's
+    const int cpr = C >> 3;
+    const ClusterShare s = cluster_share(M, gv);
+    const size_t share = (M + kClusterBlocks - 1) / kClusterBlocks;
+    const int vectors = static_cast<int>((share + s.lanes - 1) / s.lanes) * kClusterThreads;
+    float a[8], b[8], sc[8], sh[8];
+    if (kDeriv == D_X) bn_affine(s.col, f.gamma, f.beta, f.mean, f.rstd, sc, sh);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = b[j] = 0.f;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int kFlight = kTwo ? 2 : 4;
+    int k = threadIdx.x;
+    for (size_t row = s.first + s.lane; row < s.last; row += kFlight * s.lanes, k += kFlight * kClusterThreads) {
+        uint4 xv[kFlight], yv[kFlight];
+        OutGradVector dv[kFlight];
+        unsigned bits[kFlight];
+#pragma unroll
+        for (int i = 0; i < kFlight; ++i) {
+            const size_t r = row + i * s.lanes, v = r * cpr + s.col;
+            const bool in = r < s.last;
+            xv[i] = in ? __ldg(x + v) : zero;
+            dv[i].a = dv[i].b = zero;
+            if (in) dv[i] = load_grad<kTwo>(dy, r, s.col);
+            yv[i] = kDeriv == D_Y && in ? __ldg(f.y + v) : zero;
+            bits[i] = kDeriv == D_MASK && in ? __ldg(f.mask + v) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < kFlight; ++i) {
+            if (row + i * s.lanes >= s.last) break;
+            float xf[8], df[8];
+            unpack8(xv[i], xf);
+            unpack_grad<kTwo>(dv[i], df);
+            act_backward<kDeriv>(df, xf, yv[i], bits[i], sc, sh, f.below);
+            const int at = k + i * kClusterThreads;
+            keep[at] = xv[i];
+            keep[vectors + at] = dv[i].a;
+            if (kTwo) keep[2 * vectors + at] = dv[i].b;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                a[j] += df[j];
+                b[j] += df[j] * xf[j];
+            }
+        }
+    }
+    const int c0 = blockIdx.x / kClusterBlocks * gv * 8;
+    cluster_sums(a, b, gv, part, [&](int c, double ta, double tb) {
+        done[0][c] = static_cast<float>(ta);
+        done[1][c] = static_cast<float>(static_cast<double>(f.rstd[c0 + c]) * (tb - static_cast<double>(f.mean[c0 + c]) * ta));
+        if (blockIdx.x % kClusterBlocks == 0) {
+            dbeta[c0 + c] = done[0][c];
+            dgamma[c0 + c] = done[1][c];
+        }
+    });
+    float ka[8], kb[8], kc[8];
+    {
+        float rs[8], mu[8];
+        load8_or(f.gamma, s.col, 1.f, ka);
+        load8(f.rstd, s.col, rs);
+        load8(f.mean, s.col, mu);
+        const int base = threadIdx.x % gv * 8;
+        const float inv = static_cast<float>(inv_M);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float k1 = done[0][base + j] * inv, k2 = done[1][base + j] * inv;
+            ka[j] *= rs[j];
+            kb[j] = -ka[j] * rs[j] * k2;
+            kc[j] = ka[j] * (mu[j] * rs[j] * k2 - k1);
+        }
+    }
+    k = threadIdx.x;
+    for (size_t row = s.first + s.lane; row < s.last; row += s.lanes, k += kClusterThreads) {
+        const size_t v = row * cpr + s.col;
+        OutGradVector dv;
+        dv.a = keep[vectors + k];
+        if (kTwo) dv.b = keep[2 * vectors + k];
+        const uint4 yv = kDeriv == D_Y ? __ldg(f.y + v) : zero;
+        const unsigned bits = kDeriv == D_MASK ? __ldg(f.mask + v) : 0u;
+        float xf[8], df[8];
+        unpack8(keep[k], xf);
+        unpack_grad<kTwo>(dv, df);
+        act_backward<kDeriv>(df, xf, yv, bits, sc, sh, f.below);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xf[j] = ka[j] * df[j] + kb[j] * xf[j] + kc[j];
+        dx[v] = pack8(xf);
+        if (dres) dres[v] = pack8(df);
+    }
+    cooperative_groups::this_cluster().sync();
+}
+
 // An activation that no normalisation stands in front of: y = act(x), with a second copy as part of the channels of a wider
 // tensor.  rows x C, thread layout and grid as above.
 __global__ void __launch_bounds__(256, 4) act_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, uint4* __restrict__ y2,
@@ -642,6 +882,39 @@ static int bn_grid_elementwise(long long M, int C, int per_sm) {
     return static_cast<int>(want < 148 * per_sm ? want : 148 * per_sm);
 }
 static bool bn_shape_ok(long long M, int C) { return M > 0 && C > 0 && C % 8 == 0 && C <= 2048; }
+// Whether a pass that keeps `tensors` tensors goes through the cluster kernels: gv > 0, and the shared memory of a block.
+// gv: so many vectors of a row per cluster that there are about 16 clusters (128 blocks), a power of two.  Above
+// kClusterShare a block the three kernels are as fast: their reads run on four blocks per SM.  (Forward / backward, three
+// kernels -> one: 64 x 512 7.9 / 9.7 -> 4.2 / 4.3 us, 1024 x 512 11.1 / 14.4 -> 5.8 / 5.9, 4096 x 512, the limit, 11.5 / 14.8 ->
+// 9.8 / 9.7, 16384 x 256, twice that, 15.1 / 18.3 -> 15.4 / 21.7; 5000 x 64 9.5 / 12.0 -> 5.1 / 6.2, 32768 x 64 12.3 -> 17.7.)
+struct ClusterPlan {
+    int gv = 0, grid = 0;
+    size_t smem = 0;
+};
+static ClusterPlan cluster_plan(long long M, int C, int tensors) {
+    const int cpr = C / 8;
+    int gv = 1;
+    while (gv < kMaxGv && cpr / gv > 16 && cpr % (2 * gv) == 0) gv *= 2;
+    const long long share = (M + kClusterBlocks - 1) / kClusterBlocks, lanes = kClusterThreads / gv;
+    const unsigned long long bytes = 16ull * kClusterThreads * ((share + lanes - 1) / lanes);
+    ClusterPlan p;
+    if (bytes > kClusterShare) return p;
+    p.gv = gv;
+    p.grid = cpr / gv * kClusterBlocks;
+    p.smem = bytes * tensors;
+    return p;
+}
+// Raises a cluster kernel's shared-memory limit on the current device, once.
+static int cluster_ready(const void* kernel, std::atomic<unsigned long long>& devices) {
+    int dev = 0;
+    NMLL_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (devices.load(std::memory_order_acquire) & bit) return NML_OK;
+    NMLL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(3 * kClusterShare)));
+    devices.fetch_or(bit, std::memory_order_release);
+    return NML_OK;
+}
+
 // A row pitch of a tensor of `channels` channels, in elements: 0 for a tensor of its own.
 static bool row_ok(int pitch, int channels) { return pitch == 0 || (pitch >= channels && pitch % 8 == 0); }
 static int row_vectors(int pitch, int channels) { return (pitch ? pitch : channels) / 8; }
@@ -679,11 +952,24 @@ int nml_bn_forward_masked(const void* x, long long rows, int channels, const flo
     nml_bn_workspace_size(rows, channels, &need);
     if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t M = static_cast<size_t>(rows);
+    const uint4* xv = static_cast<const uint4*>(x);
+    const ClusterPlan cp = cluster_plan(rows, channels, 1);
+    if (cp.gv) {
+        static std::atomic<unsigned long long> ready{0};
+        const int rc = cluster_ready(reinterpret_cast<const void*>(bn_cluster_forward_kernel), ready);
+        if (rc) return rc;
+        launch_with(true, kClusterBlocks, bn_cluster_forward_kernel, cp.grid, kClusterThreads, cp.smem, st, xv,
+                    static_cast<const uint4*>(residual), static_cast<uint4*>(y), row_vectors(y_pitch, channels), static_cast<uint4*>(y2),
+                    row_vectors(y2_pitch, channels), static_cast<uint8_t*>(mask), gamma, beta, mean, rstd, act, slope, eps,
+                    1.0 / static_cast<double>(rows), M, channels, cp.gv);
+        NMLL_CUDA(cudaGetLastError());
+        ++g_layer_launches;
+        return NML_OK;
+    }
     int threads;
     const int P = bn_grid(rows, channels, &threads);
     float* partial = static_cast<float*>(workspace);
-    const size_t M = static_cast<size_t>(rows);
-    const uint4* xv = static_cast<const uint4*>(x);
     launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels);
     launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
            nullptr, nullptr, mean, rstd);
@@ -698,20 +984,31 @@ int nml_bn_forward_masked(const void* x, long long rows, int channels, const flo
 
 }  // extern "C"
 
-template <bool kTwo>
-static void bn_backward_launch(const uint4* x, long long rows, int channels, int deriv, const OutGrad& dy, const BnForward& f, void* dx,
-                               void* dres, float* dgamma, float* dbeta, float* partial, cudaStream_t st) {
-    int threads;
-    const int P = bn_grid(rows, channels, &threads);
+template <int kDeriv, bool kTwo>
+static int bn_backward_launch(const uint4* x, long long rows, int channels, const OutGrad& dy, const BnForward& f, uint4* dx, uint4* dres,
+                              float* dgamma, float* dbeta, float* partial, cudaStream_t st) {
     const size_t M = static_cast<size_t>(rows);
-    auto sums = deriv == D_NONE ? bn_grad_sums_kernel<D_NONE, kTwo> : deriv == D_Y ? bn_grad_sums_kernel<D_Y, kTwo>
-              : deriv == D_X ? bn_grad_sums_kernel<D_X, kTwo> : bn_grad_sums_kernel<D_MASK, kTwo>;
-    auto apply = deriv == D_NONE ? bn_dx_kernel<D_NONE, kTwo> : deriv == D_Y ? bn_dx_kernel<D_Y, kTwo>
-               : deriv == D_X ? bn_dx_kernel<D_X, kTwo> : bn_dx_kernel<D_MASK, kTwo>;
-    launch(sums, P, threads, 0, st, x, dy, f, partial, M, channels);
-    launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 1, 0.0, 0.f, f.mean, f.rstd, dbeta, dgamma);
-    launch_with(true, 1, apply, bn_grid_elementwise(rows, channels, kDxBlocks), threads, 0, st, x, dy, f, static_cast<uint4*>(dx),
-           static_cast<uint4*>(dres), dbeta, dgamma, static_cast<float>(1.0 / static_cast<double>(rows)), M, channels);
+    const double inv_M = 1.0 / static_cast<double>(rows);
+    const ClusterPlan cp = cluster_plan(rows, channels, kTwo ? 3 : 2);
+    if (cp.gv) {
+        auto kernel = bn_cluster_backward_kernel<kDeriv, kTwo>;
+        static std::atomic<unsigned long long> ready{0};
+        const int rc = cluster_ready(reinterpret_cast<const void*>(kernel), ready);
+        if (rc) return rc;
+        launch_with(true, kClusterBlocks, kernel, cp.grid, kClusterThreads, cp.smem, st, x, dy, f, dx, dres, dbeta, dgamma, inv_M, M,
+                    channels, cp.gv);
+        ++g_layer_launches;
+    } else {
+        int threads;
+        const int P = bn_grid(rows, channels, &threads);
+        launch(bn_grad_sums_kernel<kDeriv, kTwo>, P, threads, 0, st, x, dy, f, partial, M, channels);
+        launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 1, 0.0, 0.f, f.mean, f.rstd, dbeta, dgamma);
+        launch_with(true, 1, bn_dx_kernel<kDeriv, kTwo>, bn_grid_elementwise(rows, channels, kDxBlocks), threads, 0, st, x, dy, f, dx, dres,
+                    dbeta, dgamma, static_cast<float>(inv_M), M, channels);
+        g_layer_launches += 3;
+    }
+    NMLL_CUDA(cudaGetLastError());
+    return NML_OK;
 }
 static int bn_backward(const void* x, long long rows, int channels, int deriv, const OutGrad& dy, const BnForward& f, void* dx, void* dres,
                        float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, cudaStream_t st) {
@@ -722,11 +1019,12 @@ static int bn_backward(const void* x, long long rows, int channels, int deriv, c
     size_t need = 0;
     nml_bn_workspace_size(rows, channels, &need);
     if (!workspace || workspace_bytes < need) return NML_ERR_WORKSPACE;
-    auto run = dy.b ? bn_backward_launch<true> : bn_backward_launch<false>;
-    run(static_cast<const uint4*>(x), rows, channels, deriv, dy, f, dx, dres, dgamma, dbeta, static_cast<float*>(workspace), st);
-    NMLL_CUDA(cudaGetLastError());
-    g_layer_launches += 3;
-    return NML_OK;
+    auto run = dy.b ? (deriv == D_NONE ? bn_backward_launch<D_NONE, true> : deriv == D_Y ? bn_backward_launch<D_Y, true>
+                       : deriv == D_X ? bn_backward_launch<D_X, true> : bn_backward_launch<D_MASK, true>)
+                    : (deriv == D_NONE ? bn_backward_launch<D_NONE, false> : deriv == D_Y ? bn_backward_launch<D_Y, false>
+                       : deriv == D_X ? bn_backward_launch<D_X, false> : bn_backward_launch<D_MASK, false>);
+    return run(static_cast<const uint4*>(x), rows, channels, dy, f, static_cast<uint4*>(dx), static_cast<uint4*>(dres), dgamma, dbeta,
+               static_cast<float*>(workspace), st);
 }
 static OutGrad out_grad(const void* dy, int pitch, const void* dy2, int pitch2, int channels) {
     return {static_cast<const uint4*>(dy), static_cast<const uint4*>(dy2), row_vectors(pitch, channels), row_vectors(pitch2, channels)};

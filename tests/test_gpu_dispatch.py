@@ -196,3 +196,38 @@ def test_l1_loss(n):
     want = float(d.abs().sum() / 7.0)
     assert abs(float(loss.detach()) - want) <= (n * 2.0 ** -24 + 2.0 ** -22) * want
     assert torch.equal(a.grad, (torch.sign(d).float() * (torch.tensor(16384.0) / 7.0).item()).half())
+
+
+@pytest.mark.parametrize("rows,c", [(7, 8), (8, 24), (9, 72), (2048, 136), (2049, 1024), (129, 2048), (4096, 512), (4097, 512),
+                                    (16384, 8), (16385, 8)])
+@pytest.mark.parametrize("with_res", [False, True])
+def test_batch_norm_in_one_launch_and_in_three(rows, c, with_res):
+    """Both sides of the line between the forms, and their remainders, against float64.  Unit-normal data: a thread and the tree
+    above it add at most 100 numbers in fp32, so mean and E[x^2] are off by 100 * 2**-24 = 6e-6, rstd by half as much times
+    (1 + mean^2 / var), and y by gamma * (2 + |xhat|) of that, below 1e-4 * gamma; the gradients' sums likewise, relative to
+    the sum of the magnitudes (the normalised input's |xhat| is below 6)."""
+    gen = torch.Generator(device="cuda").manual_seed(rows + c)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
+    x, dy, res = rnd(rows, c).half(), rnd(rows, c).half(), (rnd(rows, c).half() if with_res else None)
+    gamma, beta, ws, n = rnd(c).abs() + 0.1, rnd(c), ops.Workspace(), ops._native
+    dg, db = torch.empty(c, device="cuda"), torch.empty(c, device="cuda")
+    y, _, mean, rstd, mask = n.bn_forward(x, res, gamma, beta, 2, 0.2, 1e-5, None, False, ws)
+    dx, dres = n.bn_backward(dy, None, False, mask, x, gamma, beta, mean, rstd, 2, 0.2, with_res, dg, db, ws)
+    ops.device_status()
+    x64, dy64 = x.double(), dy.double()
+    m, var = x64.mean(0), x64.var(0, unbiased=False)
+    r = (var + 1e-5).rsqrt()
+    xhat = (x64 - m) * r
+    z = xhat * gamma + beta + (res.double() if with_res else 0.0)
+    want = torch.where(z > 0, z, 0.2 * z)
+    scale = 1.0 + m * m * r * r
+    assert bool(((mean - m).abs() <= 1e-5).all()) and bool(((rstd - r).abs() <= 1e-5 * r * scale).all())
+    assert bool(((y - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -24 + 1e-4 * gamma * scale).all())
+    dz = dy64 * torch.where(y > 0, 1.0, 0.2)  # (the kernel's own signs: a value that rounds to zero may have either)
+    wg, wb = (dz * xhat).sum(0), dz.sum(0)
+    assert bool(((db - wb).abs() <= 1e-5 * dz.abs().sum(0)).all())
+    assert bool(((dg - wg).abs() <= 1e-4 * scale * (dz.abs() * (1 + xhat.abs())).sum(0)).all())
+    wdx = gamma * r * (dz - wb / rows - xhat * wg / rows)
+    assert bool(((dx - wdx).abs() <= 2.0 ** -11 * wdx.abs() + 2.0 ** -24 + 1e-3 * scale * gamma * r * dz.abs().amax(0)).all())
+    if with_res:
+        assert torch.equal(dres, dz.half())

@@ -80,15 +80,15 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_KA       K atoms per stage (1 or 2)       NML_TUNE_L2PROMO   TMA L2 promotion (0..3)
 //   NML_TUNE_PAIR     0: no CTA pairs                  NML_TUNE_TMASTORE  0: no TMA-store epilogues
 //   NML_TUNE_EPI8     0: never a second epilogue group
-//   NML_TUNE_PATCH    0: no forward patch walk, 2: wherever it is legal, 3: also with streamed weights
-//   NML_TUNE_BRES     0: patch walk streams its weights NML_TUNE_SHUFFLE  0: no phase-packed gather walk
+//   NML_TUNE_PATCH    0: no forward patch walk, 2: wherever it is legal
+//   NML_TUNE_SHUFFLE  0: no phase-packed gather walk
 //   NML_TUNE_FSPLIT   0: no K split of the forward walk
 //   NML_TUNE_WPATCH   0: no weight-gradient patch walk NML_TUNE_WCOAL     0: its gradient leaves by scattered stores
 //   NML_TUNE_WTRANS   0: Linear input-gradients never take a transposed copy of the weights
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
 //   NML_TUNE_NARROW   0: few-channel layers always take eight channels per pixel
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, bres, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow;
 };
 static const Tune& tune() {
     static Tune t;
@@ -106,7 +106,6 @@ static const Tune& tune() {
         t.tmastore = env("NML_TUNE_TMASTORE", 1);
         t.epi8 = env("NML_TUNE_EPI8", 1);
         t.patch = env("NML_TUNE_PATCH", 1);
-        t.bres = env("NML_TUNE_BRES", 1);
         t.shuffle = env("NML_TUNE_SHUFFLE", 1);
         t.fsplit = env("NML_TUNE_FSPLIT", 1);
         t.wpatch = env("NML_TUNE_WPATCH", 1);
@@ -506,9 +505,9 @@ static int prepare_window(const void* src, int dtype, int layout, int batch, int
 }
 
 // Picks a power-of-two pixel box (w, h, n) with 2^bits pixels that covers the grid with the
-// fewest boxes; ties go to the wider box.  box extents times the element stride stay <= 256.
+// fewest boxes; ties go to the wider box.  box extents times the element stride stay <= 256.  n_tiles: tiles per box.
 static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* wl, int* hl, int* nl,
-                       int prefer_w_log2 = 0) {
+                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1) {
     long long best = -1, best_wide = -1;
     int ww = 0, wh = 0, wn = 0;
     for (int a = bits; a >= 0; --a) {
@@ -533,8 +532,10 @@ static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* 
         }
     }
     // A box at least 2^prefer_w_log2 pixels wide (whole 128-byte runs for pixel-major stores) is taken
-    // when it costs at most 15 % more tiles.
-    if (prefer_w_log2 > 0 && best_wide > 0 && best_wide * 100 <= best * 115) {
+    // when it costs at most 15 % more tiles and no further round of tiles: 3x3 96 -> 96 at 56 x 56, batch 16, fp16 31.1 -> 27.6 us
+    // with 392 tiles instead of 448; 128 -> 128 at 28 x 28, batch 16, 112 tiles instead of 98 in one round, 17.1 -> 15.9.
+    const auto rounds = [&](long long boxes) { return (boxes * n_tiles + sms - 1) / sms; };
+    if (prefer_w_log2 > 0 && best_wide > 0 && best_wide * 100 <= best * 115 && rounds(best_wide) <= rounds(best)) {
         *wl = ww;
         *hl = wh;
         *nl = wn;
@@ -611,14 +612,12 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         }
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
     } else if (P.patch) {
-        // [B: resident slices, or a ring of single-slice stages][patch buffers][staging][bias][barriers]
+        // [resident B slices][patch buffers][staging][bias][barriers]
         P.ka = 1;
-        const int b_slice = P.bn * P.b_row_bytes;
-        const int res_bytes = P.c_blocks * P.n_taps * b_slice;  // the taps of every phase
+        const int res_bytes = P.c_blocks * P.n_taps * P.bn * P.b_row_bytes;  // the taps of every phase
         P.stg_bufs = P.epi_warps == 8 ? 1 : 2;  // (alternate groups return to a buffer after two tiles; patches need the room)
         int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
-        const bool res_wanted = P.n_tiles == 1 && P.planes == 1 && tune().bres;
-        if (res_wanted && res_bytes + 2 * P.patch_bytes > avail) {  // trade staging for residency
+        if (res_bytes + 2 * P.patch_bytes > avail) {  // trade staging for residency
             P.stg_bufs = 1;
             avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
             if (res_bytes + 2 * P.patch_bytes > avail) {
@@ -628,31 +627,12 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
                 avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
             }
         }
-        int b_region;
-        if (res_wanted && res_bytes + 2 * P.patch_bytes <= avail) {
-            P.b_resident = 1;
-            P.stages = 1;
-            b_region = res_bytes;
-            P.a_stages = std::min(4, (avail - res_bytes) / P.patch_bytes);
-        } else {
-            P.b_resident = 0;
-            // B streams tap by tap; narrow tiles take two taps per stage (8 MMAs per barrier round trip)
-            P.ka = P.planes == 2 ? 2 : std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
-            const int b_stage = P.ka * b_slice;
-            P.a_stages = P.planes == 2 ? 4 : std::min(3, std::max(2, P.c_blocks));  // (the split takes its patches in pairs)
-            P.stages = std::min(8, (avail - P.a_stages * P.patch_bytes) / b_stage);
-            if (P.stages < 3) {  // wide tiles: give the B ring room
-                P.a_stages = 2;
-                P.stg_bufs = 1;
-                avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
-                P.stages = std::min(8, (avail - P.a_stages * P.patch_bytes) / b_stage);
-            }
-            if (P.stages < 2) return NML_ERR_UNSUPPORTED;
-            b_region = P.stages * b_stage;
-        }
-        if (P.b_resident && P.a_stages < (P.c_blocks << P.tbufs_log2)) P.tbufs_log2 = std::min(P.tbufs_log2, 1);
-        P.issuers = (P.b_resident && P.tbufs_log2 >= 1 && P.a_stages >= (P.c_blocks << P.tbufs_log2)) ? 2 : 1;
-        P.a_ring_off = static_cast<int>(round_up(b_region, 1024));
+        if (res_bytes + 2 * P.patch_bytes > avail) return NML_ERR_UNSUPPORTED;  // (run_fprop_like has checked that they fit)
+        P.stages = 1;
+        P.a_stages = std::min(4, (avail - res_bytes) / P.patch_bytes);
+        if (P.a_stages < (P.c_blocks << P.tbufs_log2)) P.tbufs_log2 = std::min(P.tbufs_log2, 1);
+        P.issuers = (P.tbufs_log2 >= 1 && P.a_stages >= (P.c_blocks << P.tbufs_log2)) ? 2 : 1;
+        P.a_ring_off = static_cast<int>(round_up(res_bytes, 1024));
         P.ring_bytes = P.a_ring_off + P.a_stages * P.patch_bytes;
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
     } else {
@@ -712,12 +692,12 @@ struct FpropLike {
 // Whether a few-channel layer with N output channels takes the patch walk with resident weights when its rows are 64
 // bytes long (the conditions of run_fprop_like's own choice, which then makes the same one).
 static bool narrow_patch_walk(const FpropLike& f, int N) {
-    if (tune().patch != 1 || !tune().bres || N > 256) return false;
+    if (tune().patch != 1 || N > 256) return false;
     const int range_h = (f.kh - 1) * f.d_h, pw = 8, ph = 15 * f.s_h + range_h + 1;
     if (f.kh < 2 || ph > 256 || pw * ph * 64 > 48 * 1024) return false;
     int wl = 0, hl = 0, nl = 0;
     const bool nchw = f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1);
-    choose_box(7, f.out_w, f.out_h, f.batch, 1, f.s_h, &wl, &hl, &nl, nchw ? 5 : 0);
+    choose_box(7, f.out_w, f.out_h, f.batch, 1, f.s_h, &wl, &hl, &nl, nchw ? 5 : 0, 1, planning_sms());
     const double area = static_cast<double>(f.out_w) * f.out_h;
     const double eff_patch = area / (1.0 * round_up(f.out_w, 8) * round_up(f.out_h, 16));
     const double eff_box = area * f.batch / (1.0 * round_up(f.out_w, 1 << wl) * round_up(f.out_h, 1 << hl) * round_up(f.batch, 1 << nl));
@@ -1005,9 +985,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         P.wb_log2 = 7;
     } else {
         choose_box(7, P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, &P.wb_log2, &P.hb_log2, &P.nb_log2,
-                   (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0);
+                   (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0, ceil_div(N, 256), limited(ds->sms));
     }
-    bool patch_resident = false;
     // Patch walk: unit-stride walks with several taps load one haloed patch per channel block instead of
     // one box per tap (8 x 16 pixel tiles of a single image).  Taken when the fixed tile shape does not
     // waste much more of the tile than the free-form box does.  Every phase of a gather walk has its own
@@ -1043,15 +1022,13 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                                (1.0 * round_up(wq, 1 << P.wb_log2) * round_up(hq, 1 << P.hb_log2) * round_up(f.batch, 1 << P.nb_log2));
         const bool can = every_phase_has_taps && n_taps >= 2 && esw == 1 && pw_ <= 256 && ph_ <= 256 &&
                          pw_ * ph_ * row_bytes <= 48 * 1024;
-        // B stays resident when every slice fits beside two patch buffers and the smallest epilogue staging;
-        // streaming B tap by tap pays only for the 3xTF32 split (a barrier round trip per 4 short MMAs otherwise)
-        const int bn_res = (N <= 16 && !b_mn_major) ? 16 : static_cast<int>(round_up(N, 32));
+        // Every weight slice stays in shared memory beside two patch buffers and the smallest epilogue staging.  (Weights
+        // streamed tap by tap cost a barrier round trip per four short MMAs; that form once paid for the 3xTF32 split and no
+        // longer does: 3x3 128 -> 128 at 56 x 56, batch 16 116 -> 71 us without it, 64 -> 64 at batch 8 30.2 -> 27.5.)
+        const int bn_res = N <= 16 ? 16 : static_cast<int>(round_up(N, 32));
         const long long res_need = 1ll * c_blocks * n_taps * bn_res * row_bytes + 2 * round_up(pw_ * ph_ * row_bytes, 1024);
-        const bool res_ok = P.planes == 1 && N <= 256 &&
-                            res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
-        const bool streamed_ok = N <= 128 && (P.planes == 2 || mode >= 3);
-        if (can && mode && (mode == 2 || (eff_patch >= 0.8 * eff_box && (res_ok || streamed_ok)))) {
-            patch_resident = res_ok;
+        const bool fits = P.planes == 1 && N <= 256 && !b_mn_major && res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
+        if (can && fits && mode && (mode == 2 || eff_patch >= 0.8 * eff_box)) {
             P.patch = 1;
             P.patch_w = pw_;
             P.patch_h = ph_;
@@ -1076,8 +1053,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         for (int p = 0; p < n_phases; ++p)
             m_tiles_all += 1ll * ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) *
                            ceil_div(f.batch, 1 << P.nb_log2);
-        const int forced = (P.patch && patch_resident) ? ((N <= 16 && !b_mn_major) ? 16 : static_cast<int>(round_up(N, 32)))
-                                                       : P.planes == 2 ? std::min(tune().bn, 128) : tune().bn;
+        const int forced = P.patch ? (N <= 16 ? 16 : static_cast<int>(round_up(N, 32)))
+                                   : P.planes == 2 ? std::min(tune().bn, 128) : tune().bn;
         const int cand[4] = {256, 128, 64, forced};
         const double cost[3] = {1.0, 1.28, 2.24};
         double best = -1;

@@ -129,15 +129,15 @@ struct KParams {
     int w_mtiles;        // row tiles (accumulators), w_mtiles * bn <= 512
     int w_coalesce;      // 1: the partial gradient leaves through shared memory as contiguous runs of stores
                          //    (needs 32 gradient columns, 32 * c_patch * taps floats, to fit in the operand ring)
-    int patch;           // 1: patch walk
+    int patch;           // 1: patch walk (one plane, one column tile; every B slice of the launch is loaded once, at
+                         //    [channel block][tap] * bn * b_row_bytes)
     int patch_w, patch_h;    // patch extent in pixels
     int patch_bytes;     // bytes one patch buffer occupies (multiple of 1024)
     int a_row_bytes;     // bytes of one patch row: 128, or 64 in the narrow window walks (up to 4 image channels; 64-byte
                          // swizzle, two MMAs per K slice instead of four)
     int b_row_bytes;     // forward: bytes of one row of a weight slice, likewise
     int a_stages;        // patch buffers
-    int b_resident;      // 1: every B slice of the launch is loaded once, at [pass plane][cb][tap] * bn * 128
-    int issuers;         // resident patch walk: 2 = the B producer issues the odd tiles (needs a_stages >= tbufs * c_blocks)
+    int issuers;         // patch walk: 2 = the B producer issues the odd tiles (needs a_stages >= tbufs * c_blocks)
     int ring_bytes;      // bytes of the operand ring(s) in front of the staging buffers
     int a_ring_off;      // patch walk: offset of the patch buffers within the ring region
     int kind;            // KIND_F16 / KIND_TF32
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.stages; ++s) {
-            mbar_init(smem_u32(&full_bar[s]), P.patch ? 1 : 2);  // one arrival (with its byte count) per producer warp
+            mbar_init(smem_u32(&full_bar[s]), 2);  // one arrival (with its byte count) per producer warp
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
         for (int b = 0; b < 4; ++b) {
@@ -456,9 +456,9 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         const int boxes_per_atom = (kMode != MODE_WGRAD || kPair) ? 1
                                    : do_a ? (P.a_grouped ? 1 : kTileM / P.kb) : (P.b_grouped ? 1 : P.bn / P.kb);
         const int issue_lanes = P.wpatch || (kMode == MODE_WGRAD && kPair) ? 1
-                                : P.patch ? ((do_a || P.b_resident) ? 1 : P.ka) : P.ka * boxes_per_atom;
+                                : P.patch ? 1 : P.ka * boxes_per_atom;
         const uint32_t issue_mask = (1u << issue_lanes) - 1u;
-        if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident && do_b) {
+        if (kMode == MODE_FPROP && !kPair && P.patch && do_b) {
             // Resident weights: every slice once, for the whole launch (one column tile, one pass plane, K-major
             // repacked weights).  The slices are spread over the lanes of the warp, so the dozens of TMA issues at
             // the start of the kernel cost one thread's worth of them, not their sum.
@@ -516,19 +516,17 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         const int w0 = (tw << P.wb_log2) * P.a_stride_w + pt.org_w;
                         const int h0 = (th << P.hb_log2) * P.a_stride_h + pt.org_h;
                         for (int cb = 0; ok && cb < P.c_blocks; ++cb) {
-                            for (int pl = 0; pl < P.planes; ++pl) {
-                                if (!mbar_wait(smem_u32(&aempty_bar[abuf]), apar ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
-                                    ok = false;
-                                    break;
-                                }
-                                const uint32_t fb = smem_u32(&afull_bar[abuf]);
-                                mbar_arrive_expect_tx(fb, patch_tx);
-                                tma_load_4d(a_base + abuf * P.patch_bytes, &P.tmA[pl], fb, cb * P.kb, w0, h0, tn);
-                                ++issued;
-                                if (++abuf == P.a_stages) {
-                                    abuf = 0;
-                                    apar ^= 1;
-                                }
+                            if (!mbar_wait(smem_u32(&aempty_bar[abuf]), apar ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
+                                ok = false;
+                                break;
+                            }
+                            const uint32_t fb = smem_u32(&afull_bar[abuf]);
+                            mbar_arrive_expect_tx(fb, patch_tx);
+                            tma_load_4d(a_base + abuf * P.patch_bytes, &P.tmA[0], fb, cb * P.kb, w0, h0, tn);
+                            ++issued;
+                            if (++abuf == P.a_stages) {
+                                abuf = 0;
+                                apar ^= 1;
                             }
                         }
                     }
@@ -550,7 +548,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     }
                     ok = true;   // nothing left for the common unwinding below
                     issued = 0;
-                } else if (P.b_resident) {
+                } else {
                     // (the slices were requested above, by the whole warp)
                     const uint32_t fb = smem_u32(bres_bar);
                     // the MMA warp waits for these before its first tile; if it gave up, wait here (bounded) so
@@ -561,35 +559,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             if (*abort_flag) atomicCAS(P.err, 0, ERR_WAIT_DRAIN);
                             break;
                         }
-                    }
-                } else {
-                    // B streams through the ring, ks tap slices (of every plane) per stage
-                    int p = 0;
-                    for (int tile = tile_first; ok && tile < P.num_tiles; tile += tile_step) {
-                        while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
-                        const Phase& pt = P.phases[p];
-                        const int ntile = (tile - pt.tile_begin) % P.n_tiles;
-                        for (int cb = 0; ok && cb < P.c_blocks; ++cb)
-                            for (int t = 0; t < pt.tap_count; t += ks) {
-                                // (one lane per atom: a second load from one thread costs what the stage's MMAs last)
-                                if (!__all_sync(issue_mask, mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
-                                                                      ERR_WAIT_EMPTY))) {
-                                    ok = false;
-                                    break;
-                                }
-                                const int n = min(ks, pt.tap_count - t) * P.planes;
-                                const uint32_t fb = smem_u32(&full_bar[stage]);
-                                if (lane == 0) mbar_arrive_expect_tx(fb, n * stage_b_bytes);
-                                __syncwarp(issue_mask);
-                                if (lane < n)
-                                    load_b(smem_u32(smem) + (stage * P.ka + lane) * stage_b_bytes, &P.tmB[P.planes == 2 ? (lane & 1) : 0], fb,
-                                           P.taps[pt.tap_begin + t + (P.planes == 2 ? lane >> 1 : lane)], cb, ntile, 0);
-                                ++issued;
-                                if (++stage == P.stages) {
-                                    stage = 0;
-                                    parity ^= 1;
-                                }
-                            }
                     }
                 }
             } else
@@ -890,11 +859,11 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         const uint32_t b_atom_step = static_cast<uint32_t>(stage_b_bytes) >> 4;
         const uint32_t stage_step = static_cast<uint32_t>(stage_bytes) >> 4;
         const bool f16 = (P.kind == KIND_F16);
-        int stage = 0, pstage = 0;
-        uint32_t parity = 0, pparity = 0;
+        int stage = 0;
+        uint32_t parity = 0;
         bool ok = true;
         int titer = 0;
-        if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident) {
+        if (kMode == MODE_FPROP && !kPair && P.patch) {
             // (issued below, by one copy of the loop for both issuers)
         } else
         for (int tile_id = tile_first; ok && (!kPair || leader) && tile_id < P.num_tiles; tile_id += tile_step, ++titer) {
@@ -1010,71 +979,6 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 product(d_cross, al, bh, 1u);
                 product(d_tmem, ah, bh, acc);
             };
-            if (kMode == MODE_FPROP && !kPair && P.patch) {
-                int pp = 0;
-                while (pp + 1 < P.n_phases && tile >= P.phases[pp + 1].tile_begin) ++pp;
-                const Phase& ph = P.phases[pp];
-                const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h) * 128u;  // 8-row groups: one output row = a_stride_h patch rows apart
-                const uint64_t bdesc_ring0 = make_smem_desc(smem_u32(smem), lbo_b, b32 ? 512 : 1024, b32 ? 1 : 2);  // B ring starts the region
-                for (int cb = 0; ok && cb < P.c_blocks; ++cb) {
-                    uint64_t adesc[2];
-                    int used[2];
-                    for (int pl = 0; pl < P.planes; ++pl) {
-                        if (!mbar_wait(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) {
-                            ok = false;
-                            break;
-                        }
-                        adesc[pl] = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, 2);
-                        used[pl] = pstage;
-                        if (++pstage == P.a_stages) {
-                            pstage = 0;
-                            pparity ^= 1;
-                        }
-                    }
-                    if (!ok) break;
-                    tc_fence_after();
-                    for (int t = 0; t < ph.tap_count; t += ks) {
-                        if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const int n = min(ks, ph.tap_count - t);
-                        if (elect_one()) {
-                            uint64_t bdesc = bdesc_ring0 + static_cast<uint64_t>(stage * P.ka * b_atom_step);
-                            if (P.planes == 2) {
-                                const uint32_t off = static_cast<uint32_t>(P.taps[ph.tap_begin + t].aoff);
-                                issue_split(adesc[0] + off, adesc[1] + off, bdesc, bdesc + b_atom_step, 2, adv_b);
-                            } else
-                            for (int j = 0; j < n; ++j) {
-                                const uint64_t ad = adesc[0] + static_cast<uint32_t>(P.taps[ph.tap_begin + t + j].aoff);
-                                if (f16) {
-                                    umma_f16(d_tmem, ad, bdesc, idesc, acc);
-                                    umma_f16(d_tmem, ad + 2, bdesc + adv_b, idesc, 1u);
-                                    umma_f16(d_tmem, ad + 4, bdesc + 2 * adv_b, idesc, 1u);
-                                    umma_f16(d_tmem, ad + 6, bdesc + 3 * adv_b, idesc, 1u);
-                                } else {
-                                    umma_tf32(d_tmem, ad, bdesc, idesc, acc);
-                                    umma_tf32(d_tmem, ad + 2, bdesc + adv_b, idesc, 1u);
-                                    umma_tf32(d_tmem, ad + 4, bdesc + 2 * adv_b, idesc, 1u);
-                                    umma_tf32(d_tmem, ad + 6, bdesc + 3 * adv_b, idesc, 1u);
-                                }
-                                acc = 1u;
-                                bdesc += b_atom_step;
-                            }
-                            umma_commit(smem_u32(&empty_bar[stage]));
-                        }
-                        acc = 1u;
-                        if (++stage == P.stages) {
-                            stage = 0;
-                            parity ^= 1;
-                        }
-                    }
-                    if (!ok) break;
-                    if (elect_one())
-                        for (int pl = 0; pl < P.planes; ++pl) umma_commit(smem_u32(&aempty_bar[used[pl]]));
-                }
-            } else
             for (int it = 0; it < k_iters; it += ks) {
                 const int n_atoms = min(ks, k_iters - it);
                 if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
@@ -1874,7 +1778,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         }
     }
 
-    if (kMode == MODE_FPROP && !kPair && P.patch && P.b_resident && (warp == 1 || (warp == 6 && P.issuers == 2))) {
+    if (kMode == MODE_FPROP && !kPair && P.patch && (warp == 1 || (warp == 6 && P.issuers == 2))) {
         __syncwarp();  // (warp 6 comes from a loop that one lane ran)
         patch_resident_issue(warp == 6 ? 1 : 0, P.issuers);
     }

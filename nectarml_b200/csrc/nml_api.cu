@@ -445,13 +445,17 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
     if (ws.dry) return NML_OK;
     if (!ws.fits()) return NML_ERR_WORKSPACE;
     if (transposing) {
-        dim3 grid(ceil_div(h * w, 64), ceil_div(Cp, 64), batch);
-        if (dtype == NML_F32)
-            { helper_launch(kSms, nchw_to_nhwc_kernel<float>, grid, 256, 0, st, static_cast<const float*>(src), p0, p1, mi.enc, c, Cp,
-                                                            h * w, cs.partial); ++g_launches; }
-        else
-            { helper_launch(kSms, nchw_to_nhwc_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(src), p0, p1, mi.enc, c,
-                                                             Cp, h * w, cs.partial); ++g_launches; }
+        const int tiles_p = ceil_div(h * w, 64), tiles_c = ceil_div(Cp, 64);
+        const long long tiles = 1ll * tiles_p * tiles_c * batch;
+        if (tiles > INT_MAX / 2) return NML_ERR_UNSUPPORTED;
+        const unsigned blocks = static_cast<unsigned>(std::min<long long>(tiles, 6 * kSms));  // (four of them resident)
+        auto convert = [&](auto* kernel, auto* in) {
+            helper_launch(6 * kSms, kernel, blocks, 256, 0, st, in, p0, p1, mi.enc, c, Cp, h * w, tiles_p, tiles_c, static_cast<int>(tiles),
+                          cs.partial);
+        };
+        if (dtype == NML_F32) convert(nchw_to_nhwc_kernel<float>, static_cast<const float*>(src));
+        else convert(nchw_to_nhwc_kernel<__half>, static_cast<const __half*>(src));
+        ++g_launches;
         if (colsum) {
             int rc = colsum_finish(cs, c, colsum, st);
             if (rc) return rc;

@@ -8,8 +8,9 @@
 //
 // Which grids overlap: those of at most one block per SM, and those of many waves.  In between, blocks that arrive while
 // the predecessor still fills some SMs pile up on the others, and a bandwidth-bound kernel of one or two waves then runs
-// on part of the GPU (an NCHW conversion of 392 blocks 6.5 -> 10 us, the batch-norm passes of a 56 x 56 x 256 block at batch
-// 256 +4 %); there only kernels whose blocks do a few KB of work each overlap (launch_short, up to 4 blocks per SM).
+// on part of the GPU (the batch-norm passes of a 56 x 56 x 256 block at batch 256 +4 %); there only kernels whose blocks do a
+// few KB of work each overlap (launch_short, up to 4 blocks per SM), and those of whose blocks no more fit an SM than the grid has
+// for it.
 #pragma once
 #include <cuda_runtime.h>
 

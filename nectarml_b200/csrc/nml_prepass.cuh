@@ -33,91 +33,122 @@ __device__ __forceinline__ void store_enc(int enc, void* out0, void* out1, size_
     }
 }
 
+__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load4(const __half* p) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
 // in  [N][C][HW] (NCHW)  ->  out [N][HW][Cp] (NHWC, channels zero-padded to Cp).
-// Tile of 64 channels x 64 pixels through shared memory.  Loads run along pixels (one 256-byte
-// row segment per 16 threads when the rows allow 16-byte loads), stores along channels: 8 threads
-// write the 64 channels of one pixel as 16-byte (fp16) or 2 x 16-byte (tf32 planes) pieces, so a
-// warp store covers four whole pixels.  When `colsum` is given, the per-channel sums over the tile's
-// pixels (a share of the bias gradient) go to row (n * gridDim.x + blockIdx.x) of that [tiles][C]
+// Tiles of 64 channels x 64 pixels through shared memory, several per block: the loads of the next tile are in flight while
+// this one is stored.  With one tile per block the last wave was half empty, and eight small blocks fitted an SM, so a grid
+// launched beside its predecessor's tail piled up on the SMs that were free first; these registers leave room for four.
+// fp32 3x3 64 -> 64 at 56 x 56, batch 8, three passes with four conversions 114.8 -> 108.4 us; 128 channels at 28 x 28, batch
+// 64, with three 136.0 -> 131.7.
+// Loads run along pixels (four per thread where the rows allow it), stores along channels: 8 threads write the 64 channels
+// of one pixel as 16-byte (fp16) or 2 x 16-byte (tf32 planes) pieces, so a warp store covers four whole pixels.  When
+// `colsum` is given, the per-channel sums over the tile's pixels (a share of the bias gradient) go to row
+// (n * pixel tiles + pixel tile) of that [tiles][C]
 // matrix of partial sums; colsum_finish_kernel adds the rows in a fixed order (no atomics, so the
 // bias gradient is bitwise repeatable).
 template <typename TIn>
 __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict__ in, void* out0,
-                                                           void* out1, int enc, int C, int Cp, int HW,
-                                                           float* colsum, int role) {
+                                                           void* out1, int enc, int C, int Cp, int HW, int tiles_p, int tiles_c,
+                                                           int tiles, float* colsum, int role) {
     pdl_enter(role);
     __shared__ float tile[64][65];
-    const int n = blockIdx.z;
-    const int c0 = blockIdx.y * 64;
-    const int p0 = blockIdx.x * 64;
-    const TIn* src = in + static_cast<size_t>(n) * C * HW;
-    const bool vec_ok = (sizeof(TIn) == 4) && (HW % 4 == 0) && ((reinterpret_cast<uintptr_t>(in) & 15) == 0);
-    if (vec_ok) {
-        const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16: four pixels per thread
-        for (int c = ty; c < 64; c += 16) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            const int p = p0 + 4 * tx;
-            if (c0 + c < C && p < HW)  // HW % 4 == 0, so a started quad is complete
-                v = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(src) +
-                                                          static_cast<size_t>(c0 + c) * HW + p));
-            tile[c][4 * tx + 0] = v.x;
-            tile[c][4 * tx + 1] = v.y;
-            tile[c][4 * tx + 2] = v.z;
-            tile[c][4 * tx + 3] = v.w;
+    const bool vec_ok = (HW % 4 == 0) && ((reinterpret_cast<uintptr_t>(in) & (4 * sizeof(TIn) - 1)) == 0);
+    const int tx = vec_ok ? (threadIdx.x & 15) * 4 : threadIdx.x & 63;      // 16 x 16 threads: four pixels each; or 64 x 4
+    const int ty = vec_ok ? threadIdx.x >> 4 : threadIdx.x >> 6;
+    int n, c0, p0;
+    auto decode = [&](int t) {
+        const int q = t / tiles_p;
+        n = q / tiles_c;
+        c0 = (q - n * tiles_c) * 64;
+        p0 = (t - q * tiles_p) * 64;
+    };
+    float4 next[4];
+    auto load = [&](int t) {
+        decode(t);
+        const int p = p0 + tx;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int c = c0 + ty + 16 * k;
+            next[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < C && p < HW) next[k] = load4(in + (static_cast<size_t>(n) * C + c) * HW + p);  // HW % 4 == 0: a started quad is complete
         }
-    } else {
-        const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;  // 64 x 4
-        for (int c = ty; c < 64; c += 4) {
-            float v = 0.f;
-            if (c0 + c < C && p0 + tx < HW) v = load_as_float(src, static_cast<size_t>(c0 + c) * HW + p0 + tx);
-            tile[c][tx] = v;
-        }
-    }
-    __syncthreads();
-    if (colsum != nullptr) {  // four threads per channel, 16 pixels each (all lanes of a warp on different banks)
-        const int c = threadIdx.x >> 2, q = threadIdx.x & 3;
-        float s = 0.f;
+    };
+    int t = blockIdx.x;
+    if (vec_ok && t < tiles) load(t);
+    for (; t < tiles; t += gridDim.x) {
+        decode(t);
+        if (vec_ok) {
 #pragma unroll
-        for (int p = 0; p < 16; ++p) s += tile[c][4 * p + q];
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (q == 0 && c0 + c < C) colsum[(static_cast<size_t>(n) * gridDim.x + blockIdx.x) * C + c0 + c] = s;
-    }
-    // store: 8 threads per pixel, 8 channels each
-    const int j = threadIdx.x & 7, pp = threadIdx.x >> 3;  // 8 x 32
-    const int cb = c0 + 8 * j;
-    const bool full8 = (cb + 8 <= Cp) && (Cp % 8 == 0);
-    for (int p = pp; p < 64; p += 32) {
-        if (p0 + p >= HW || cb >= Cp) continue;
-        const size_t o = (static_cast<size_t>(n) * HW + p0 + p) * Cp + cb;
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = tile[8 * j + i][p];
-        if (full8 && enc == ENC_F16) {
-            uint4 pk;
-            __half2 h;
-            h = __floats2half2_rn(v[0], v[1]); pk.x = *reinterpret_cast<uint32_t*>(&h);
-            h = __floats2half2_rn(v[2], v[3]); pk.y = *reinterpret_cast<uint32_t*>(&h);
-            h = __floats2half2_rn(v[4], v[5]); pk.z = *reinterpret_cast<uint32_t*>(&h);
-            h = __floats2half2_rn(v[6], v[7]); pk.w = *reinterpret_cast<uint32_t*>(&h);
-            *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out0) + o) = pk;
-        } else if (full8) {
-            float hi[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) hi[i] = to_tf32_rna(v[i]);
-            float4* d0 = reinterpret_cast<float4*>(reinterpret_cast<float*>(out0) + o);
-            d0[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
-            d0[1] = make_float4(hi[4], hi[5], hi[6], hi[7]);
-            if (enc == ENC_TF32_PAIR) {
-                float4* d1 = reinterpret_cast<float4*>(reinterpret_cast<float*>(out1) + o);
-                d1[0] = make_float4(to_tf32_rna(v[0] - hi[0]), to_tf32_rna(v[1] - hi[1]), to_tf32_rna(v[2] - hi[2]),
-                                    to_tf32_rna(v[3] - hi[3]));
-                d1[1] = make_float4(to_tf32_rna(v[4] - hi[4]), to_tf32_rna(v[5] - hi[5]), to_tf32_rna(v[6] - hi[6]),
-                                    to_tf32_rna(v[7] - hi[7]));
+            for (int k = 0; k < 4; ++k) {
+                float* o = &tile[ty + 16 * k][tx];
+                o[0] = next[k].x, o[1] = next[k].y, o[2] = next[k].z, o[3] = next[k].w;
             }
         } else {
-            for (int i = 0; i < 8 && cb + i < Cp; ++i) store_enc(enc, out0, out1, o + i, v[i]);
+            const TIn* src = in + static_cast<size_t>(n) * C * HW;
+#pragma unroll 8
+            for (int c = ty; c < 64; c += 4) {
+                float v = 0.f;
+                if (c0 + c < C && p0 + tx < HW) v = load_as_float(src, static_cast<size_t>(c0 + c) * HW + p0 + tx);
+                tile[c][tx] = v;
+            }
         }
+        __syncthreads();
+        if (vec_ok && t + static_cast<int>(gridDim.x) < tiles) {
+            load(t + gridDim.x);
+            decode(t);
+        }
+        if (colsum != nullptr) {  // four threads per channel, 16 pixels each (all lanes of a warp on different banks)
+            const int c = threadIdx.x >> 2, q = threadIdx.x & 3;
+            float s = 0.f;
+#pragma unroll
+            for (int p = 0; p < 16; ++p) s += tile[c][4 * p + q];
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if (q == 0 && c0 + c < C) colsum[(static_cast<size_t>(n) * tiles_p + p0 / 64) * C + c0 + c] = s;
+        }
+        // store: 8 threads per pixel, 8 channels each
+        const int j = threadIdx.x & 7, pp = threadIdx.x >> 3;  // 8 x 32
+        const int cb = c0 + 8 * j;
+        const bool full8 = (cb + 8 <= Cp) && (Cp % 8 == 0);
+        for (int p = pp; p < 64; p += 32) {
+            if (p0 + p >= HW || cb >= Cp) continue;
+            const size_t o = (static_cast<size_t>(n) * HW + p0 + p) * Cp + cb;
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = tile[8 * j + i][p];
+            if (full8 && enc == ENC_F16) {
+                uint4 pk;
+                __half2 h;
+                h = __floats2half2_rn(v[0], v[1]); pk.x = *reinterpret_cast<uint32_t*>(&h);
+                h = __floats2half2_rn(v[2], v[3]); pk.y = *reinterpret_cast<uint32_t*>(&h);
+                h = __floats2half2_rn(v[4], v[5]); pk.z = *reinterpret_cast<uint32_t*>(&h);
+                h = __floats2half2_rn(v[6], v[7]); pk.w = *reinterpret_cast<uint32_t*>(&h);
+                *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out0) + o) = pk;
+            } else if (full8) {
+                float hi[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) hi[i] = to_tf32_rna(v[i]);
+                float4* d0 = reinterpret_cast<float4*>(reinterpret_cast<float*>(out0) + o);
+                d0[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                d0[1] = make_float4(hi[4], hi[5], hi[6], hi[7]);
+                if (enc == ENC_TF32_PAIR) {
+                    float4* d1 = reinterpret_cast<float4*>(reinterpret_cast<float*>(out1) + o);
+                    d1[0] = make_float4(to_tf32_rna(v[0] - hi[0]), to_tf32_rna(v[1] - hi[1]), to_tf32_rna(v[2] - hi[2]),
+                                        to_tf32_rna(v[3] - hi[3]));
+                    d1[1] = make_float4(to_tf32_rna(v[4] - hi[4]), to_tf32_rna(v[5] - hi[5]), to_tf32_rna(v[6] - hi[6]),
+                                        to_tf32_rna(v[7] - hi[7]));
+                }
+            } else {
+                for (int i = 0; i < 8 && cb + i < Cp; ++i) store_enc(enc, out0, out1, o + i, v[i]);
+            }
+        }
+        __syncthreads();
     }
     pdl_leave(role);
 }
@@ -125,12 +156,6 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict
 // Row-major [R][C] -> [R][Cp] with encoding change (fp32/fp16 -> fp16 / tf32 pair), zero pad; Cp is a multiple of 4.
 // Four outputs per thread: a 16-byte load where the rows allow it, one 8-byte (fp16) or one or two 16-byte stores.
 // An element per thread with a 64-bit division each ran at 1.8 TB/s on 2 MB; this is bound by the launch there.
-__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
-__device__ __forceinline__ float4 load4(const __half* p) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
-    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
-    return make_float4(a.x, a.y, b.x, b.y);
-}
 template <typename TIn>
 __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict__ in, void* out0,
                                                            void* out1, int enc, size_t R, int C, int Cp, int role) {

@@ -873,7 +873,11 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     // room for the fp32 partial sums of a K-split walk.
     const size_t out_pixels = static_cast<size_t>(f.batch) * f.out_h * f.out_w;
     const int k_slices = (mi.planes == 2 ? 3 : 1) * T * c_blocks;
-    const bool may_split = !window && !f.shuf_sh && !f.w_batched && out_pixels <= 8192 && k_slices >= 32 && tune().fsplit;
+    const double plane_us = static_cast<double>(out_pixels) * N * 4.0 / 6e6;  // one plane through memory
+    const auto split_cost_us = [&](int z) { return 3.0 + (2 * z + 1) * plane_us; };  // storing z planes and the finishing pass
+    // (the last condition: two slices, the cheapest split, could save at most the K loop itself; no plan below takes one else)
+    const bool may_split = !window && !f.shuf_sh && !f.w_batched && out_pixels <= 8192 && k_slices >= 32 && tune().fsplit &&
+                           k_slices * slice_us(256) > split_cost_us(2);
     // one fp32 plane per K slice; the bound on the slice count below holds for every plan made further down
     // (tiles >= tiles_lb, at least 4 K iterations per slice)
     int z_cap = 1;
@@ -1082,11 +1086,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             int k_min = 1 << 30;  // every slice of every phase gets at least 4 K iterations (2 of three products each)
             for (int p = 0; p < n_phases; ++p)
                 if (P.phases[p].tap_count > 0) k_min = std::min(k_min, P.c_blocks * P.phases[p].tap_count);
-            const double plane_us = static_cast<double>(out_pixels) * N * 4.0 / 6e6;
             auto cost_us = [&](int nt, int bn, int z) {
                 const long long tiles = m_tiles_all * nt;
                 const double rounds = static_cast<double>((tiles * z + limited(ds->sms) - 1) / limited(ds->sms));
-                return rounds * (ceil_div(k_min, z) * slice_us(bn) * products + 2.5) + (z > 1 ? 3.0 + (2 * z + 1) * plane_us : 0.0);
+                return rounds * (ceil_div(k_min, z) * slice_us(bn) * products + 2.5) + (z > 1 ? split_cost_us(z) : 0.0);
             };
             double best_us = cost_us(P.n_tiles, P.bn, 1);
             for (int i = 0; i < 4; ++i) {

@@ -219,6 +219,7 @@ static int raise_smem_limit() {
 static int load_helper_kernels() {
     const void* fns[] = {
         (const void*)nchw_to_nhwc_kernel<float>, (const void*)nchw_to_nhwc_kernel<__half>,
+        (const void*)nhwc_to_nchw_kernel<float>, (const void*)nhwc_to_nchw_kernel<__half>,
         (const void*)convert_rows_kernel<float>, (const void*)convert_rows_kernel<__half>,
         (const void*)colsum_rows_kernel<float>, (const void*)colsum_rows_kernel<__half>,
         (const void*)colsum_vectors_kernel<float>, (const void*)colsum_vectors_kernel<__half>,
@@ -713,6 +714,42 @@ static bool narrow_patch_walk(const FpropLike& f, int N) {
 static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     MathInfo mi;
     if (!math_info(f.math, &mi)) return NML_ERR_INVALID;
+    // A column-strided gather into an NCHW result stores single values a stride apart (4 of every 8 bytes, phase after
+    // phase).  Where the phases' rows are no multiple of eight pixels the tiles' boxes are at most four pixels wide and every
+    // store is a part of a sector; those go through an NHWC copy in the workspace (the walk's stores are TMA boxes then), which
+    // one pass of full-width stores turns round.  Input gradient of 3x3 s2, fp32 result of fp16 / 3xTF32 products: 128 channels at
+    // 28 x 28, batch 64 30.6 -> 28.4 / 48.4 -> 39.9 us; 256 at 28 x 28, batch 64 99.8 -> 54.4 / 131 -> 101; but 64 at 64 x 64 (whole
+    // rows of 32) 54.2 -> 49.6 / 68.9 -> 85.5.  Below four million values the extra pass costs more than it saves (64 at 56 x 56,
+    // batch 16 13.3 -> 16.9).  Where the caller's workspace has no room for the copy, the walk stores directly.
+    const long long out_values = 1ll * f.batch * f.out_h * f.out_w * f.out_c;
+    if (f.gather && f.s_w > 1 && f.out_layout == NML_NCHW && f.out_w > 1 && ceil_div(f.out_w, f.s_w) % 8 != 0 &&
+        out_values >= (1 << 22) && f.out_c % (f.out_dtype == NML_F16 ? 64 : 32) == 0) {
+        FpropLike f2 = f;
+        f2.out_layout = NML_NHWC;
+        const int hw = f.out_h * f.out_w;
+        const size_t bytes = static_cast<size_t>(out_values) * (f.out_dtype == NML_F16 ? 2 : 4);
+        Bump probe = ws;
+        probe.dry = true;
+        probe.take(bytes);
+        const int probe_rc = run_fprop_like(f2, probe, st);
+        const int tiles_p = ceil_div(hw, 64), tiles_c = ceil_div(f.out_c, 64);
+        const long long tiles = 1ll * tiles_p * tiles_c * f.batch;
+        if (probe_rc == NML_OK && (ws.dry || probe.off <= ws.cap) && tiles < INT_MAX / 2) {
+            f2.out = ws.take(bytes);
+            const int rc = run_fprop_like(f2, ws, st);
+            if (rc || ws.dry) return rc;
+            const unsigned blocks = static_cast<unsigned>(std::min<long long>(tiles, 6 * kSms));
+            if (f.out_dtype == NML_F16)
+                helper_launch(6 * kSms, nhwc_to_nchw_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(f2.out),
+                              static_cast<__half*>(f.out), f.out_c, hw, tiles_p, tiles_c, static_cast<int>(tiles));
+            else
+                helper_launch(6 * kSms, nhwc_to_nchw_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(f2.out),
+                              static_cast<float*>(f.out), f.out_c, hw, tiles_p, tiles_c, static_cast<int>(tiles));
+            ++g_launches;
+            NML_CUDA(cudaGetLastError());
+            return NML_OK;
+        }
+    }
     // A strided gather with very few output channels (input gradient of an RGB stem, image-producing
     // transposed layer) would run one mostly empty 16-column pass per output phase.  All phases are
     // packed into the columns instead: one unit-stride pass over the input with stride_h*stride_w*C

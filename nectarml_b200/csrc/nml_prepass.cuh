@@ -153,6 +153,68 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict
     pdl_leave(role);
 }
 
+// in [N][HW][C] (NHWC, C a multiple of 4) -> out [N][C][HW], no change of values: the way back, in the same manner.
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store4(__half* p, const float (&v)[4]) {
+    uint2 h;
+    *reinterpret_cast<__half2*>(&h.x) = __floats2half2_rn(v[0], v[1]);
+    *reinterpret_cast<__half2*>(&h.y) = __floats2half2_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = h;
+}
+template <typename T>
+__global__ void __launch_bounds__(256) nhwc_to_nchw_kernel(const T* __restrict__ in, T* __restrict__ out, int C, int HW, int tiles_p,
+                                                           int tiles_c, int tiles, int role) {
+    pdl_enter(role);
+    __shared__ float tile[64][65];  // [pixel][channel]
+    const bool vec_ok = (HW % 4 == 0) && ((reinterpret_cast<uintptr_t>(out) & (4 * sizeof(T) - 1)) == 0);
+    const int x4 = (threadIdx.x & 15) * 4, y16 = threadIdx.x >> 4;
+    int n, c0, p0;
+    auto decode = [&](int t) {
+        const int q = t / tiles_p;
+        n = q / tiles_c;
+        c0 = (q - n * tiles_c) * 64;
+        p0 = (t - q * tiles_p) * 64;
+    };
+    float4 next[4];
+    auto load = [&](int t) {
+        decode(t);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int p = p0 + y16 + 16 * k;
+            next[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p < HW && c0 + x4 < C) next[k] = load4(in + (static_cast<size_t>(n) * HW + p) * C + c0 + x4);
+        }
+    };
+    int t = blockIdx.x;
+    if (t < tiles) load(t);
+    for (; t < tiles; t += gridDim.x) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float* o = &tile[y16 + 16 * k][x4];
+            o[0] = next[k].x, o[1] = next[k].y, o[2] = next[k].z, o[3] = next[k].w;
+        }
+        __syncthreads();
+        if (t + static_cast<int>(gridDim.x) < tiles) load(t + gridDim.x);
+        decode(t);
+        if (vec_ok) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int c = y16 + 16 * k;
+                if (c0 + c < C && p0 + x4 < HW) {  // HW % 4 == 0: a started quad is complete
+                    const float v[4] = {tile[x4][c], tile[x4 + 1][c], tile[x4 + 2][c], tile[x4 + 3][c]};
+                    store4(out + (static_cast<size_t>(n) * C + c0 + c) * HW + p0 + x4, v);
+                }
+            }
+        } else {
+            const int px = threadIdx.x & 63;
+            for (int c = threadIdx.x >> 6; c < 64; c += 4)
+                if (c0 + c < C && p0 + px < HW) out[(static_cast<size_t>(n) * C + c0 + c) * HW + p0 + px] = static_cast<T>(tile[px][c]);
+        }
+        __syncthreads();
+    }
+    pdl_leave(role);
+}
+
 // Row-major [R][C] -> [R][Cp] with encoding change (fp32/fp16 -> fp16 / tf32 pair), zero pad; Cp is a multiple of 4.
 // Four outputs per thread: a 16-byte load where the rows allow it, one 8-byte (fp16) or one or two 16-byte stores.
 // An element per thread with a 64-bit division each ran at 1.8 TB/s on 2 MB; this is bound by the launch there.

@@ -231,3 +231,29 @@ def test_batch_norm_in_one_launch_and_in_three(rows, c, with_res):
     assert bool(((dx - wdx).abs() <= 2.0 ** -11 * wdx.abs() + 2.0 ** -24 + 1e-3 * scale * gamma * r * dz.abs().amax(0)).all())
     if with_res:
         assert torch.equal(dres, dz.half())
+
+
+@pytest.mark.parametrize("batch,c,hw,s,dtype", [(64, 128, 23, 2, torch.float32), (65, 64, 32, 3, torch.float16), (43, 96, 32, 3, torch.float32),
+                                               (64, 64, 33, 2, torch.float16)])
+def test_strided_input_gradient_into_nchw_through_a_copy(batch, c, hw, s, dtype):
+    """Sizes just above four million values, with planes that are and are not a multiple of four pixels: the bits of the same
+    gradient into NHWC; and with no room for the copy in the workspace, the direct stores' (the same sums, rounded once)."""
+    import ctypes as C
+    from nectarml_b200 import _lib
+    gen = torch.Generator(device="cuda").manual_seed(hw)
+    g = ops.ConvGeometry(batch, c, hw, hw, 64, 3, 3, (s, s), (1, 1))
+    ho, wo = g.out_hw()
+    dy = torch.randn(batch, 64, ho, wo, device="cuda", generator=gen).half()
+    w = torch.randn(64, c, 3, 3, device="cuda", generator=gen).half()
+    got = ops.conv_backward_data(g, dy, w, layout="nchw", out_dtype=dtype)
+    want = ops.conv_backward_data(g, dy.permute(0, 2, 3, 1).contiguous(), w, layout="nhwc", out_dtype=dtype)
+    assert torch.equal(got, want.permute(0, 3, 1, 2))
+    code = _lib.NML_F16 if dtype == torch.float16 else _lib.NML_F32
+    d, need, st = g.desc(_lib.NML_F16, "nchw", code, "nchw", _lib.NML_F16, "f16", False), C.c_size_t(), torch.cuda.current_stream().cuda_stream
+    lib = _lib.load()
+    _lib.check(lib.nml_conv_workspace_size(C.byref(d), 1, C.byref(need)))
+    room = need.value - got.numel() * got.element_size()
+    ws, direct = torch.empty(room + 256, dtype=torch.uint8, device="cuda"), torch.empty_like(got)
+    _lib.check(lib.nml_conv_backward_data(C.byref(d), dy.data_ptr(), w.data_ptr(), direct.data_ptr(), ws.data_ptr(), ws.numel(), st))
+    ops.device_status()
+    assert torch.equal(direct, got)

@@ -1513,7 +1513,9 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     int split = 1, m_tiles = 1;
     if (!P.wpatch) {
         const double dw_us = 4.0 * g.plain_c * g.patch_c * T / 8e6;  // one pass over dW at 8 TB/s
-        const int max_split = std::min(P.kblocks_total, 192);
+        // at most 192 slices, as many as leave each at least one block (a count that the loop below does not pass over, so
+        // that there is a plan whatever else is refused)
+        const int max_split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, std::min(P.kblocks_total, 192)));
         double best = -1;
         for (int width = 256; width >= 64; width /= 2) {
             const int nt = ceil_div(g.plain_c, width);
@@ -1528,7 +1530,8 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                 const int per_sp = ceil_div(P.kblocks_total, sp);
                 // every slice gets at least one K block: the next split that leaves each one block less
                 if (ceil_div(P.kblocks_total, per_sp) != sp) continue;
-                // the tensor core truncates as it accumulates: at most 4096 terms per sum of the 3xTF32 split
+                // the tensor core truncates as it accumulates: at most 4096 terms per sum of the 3xTF32 split, or as few
+                // as the most slices leave
                 if (P.planes == 2 && per_sp * mi.kb > 4096 && sp < max_split) continue;
                 const double block_us = (pair ? (tiles * 8 >= units * 7ll ? 0.41 : 0.36) : 0.32) * (P.planes == 2 ? 2.3 : 1.0);
                 const double rounds = static_cast<double>((tiles + units - 1) / units);

@@ -1,0 +1,22 @@
+"""Inputs at the far ends of what the entry points accept: very long sums, scratch limits, values and pointers that a fast path
+has to hand on."""
+import pytest
+import torch
+
+from gpu_util import assert_f32, host
+from nectarml_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def test_weight_gradient_of_more_rows_than_the_slices_halve():
+    """787000 rows in fp32: 24594 K blocks, where 192 slices no longer keep a sum within 4096 terms.  A term costs 2.5e-9 of
+    its sum (the tensor core truncates as it accumulates): 1e-5 at 4128 terms, of |dw| where the slices' signs agree; and
+    as much again for the fp32 additions."""
+    rows, fin, fout = 787000, 160, 64
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x, dy = (torch.randn(rows, f, device="cuda", generator=gen) for f in (fin, fout))
+    dw, db = ops.linear_backward_weight(x, dy, math="3xtf32")
+    ops.device_status()
+    assert_f32(host(dw), (dy.double().T @ x.double()).cpu().numpy(), "dw", 2e-5)
+    assert_f32(host(db), dy.double().sum(0).cpu().numpy(), "db", 2e-5)

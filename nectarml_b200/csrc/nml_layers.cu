@@ -661,7 +661,8 @@ __global__ void __launch_bounds__(256, 4) act_kernel(const uint4* __restrict__ x
         float f[8];
         unpack8(__ldg(x + row * cpr + col), f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = f[j] > 0.f ? f[j] : f[j] * below + 0.f;  // NaN stays NaN, -0 becomes 0
+        for (int j = 0; j < 8; ++j)  // NaN stays NaN, -0 becomes 0; below = 0 is a choice, not a product: of -inf too
+            f[j] = f[j] > 0.f ? f[j] : below != 0.f ? f[j] * below + 0.f : f[j] <= 0.f ? 0.f : f[j];
         const uint4 out = pack8(f);
         y[row * cpr + col] = out;
         if (y2) y2[row * y2_row + col] = out;
@@ -683,7 +684,8 @@ __global__ void __launch_bounds__(256, 4) act_backward_kernel(const uint4* __res
         unpack8(__ldg(x + row * cpr + col), f);
         unpack_grad<kTwo>(g, d);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) d[j] *= f[j] > 0.f ? 1.f : below;
+        for (int j = 0; j < 8; ++j)  // (an overflowed gradient does not pass where the ReLU is shut; NaN inputs let it pass)
+            d[j] = f[j] > 0.f ? d[j] : below != 0.f ? d[j] * below : f[j] <= 0.f ? 0.f : d[j];
         dx[row * cpr + col] = pack8(d);
     }
 }

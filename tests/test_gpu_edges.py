@@ -20,3 +20,21 @@ def test_weight_gradient_of_more_rows_than_the_slices_halve():
     ops.device_status()
     assert_f32(host(dw), (dy.double().T @ x.double()).cpu().numpy(), "dw", 2e-5)
     assert_f32(host(db), dy.double().sum(0).cpu().numpy(), "db", 2e-5)
+
+
+@pytest.mark.parametrize("act,slope", [(1, 0.0), (2, 0.2)])
+def test_activation_of_overflowed_values(act, slope):
+    """Infinities and NaN through the activation that stands alone, and overflowed gradients through its backward, as torch's
+    relu / leaky_relu treat them: nothing passes a ReLU that is shut, not even an infinity times zero."""
+    inf, nan = float("inf"), float("nan")
+    values = torch.tensor([inf, -inf, nan, 0.0, -0.0, 1.0, -1.0, 65504.0, -65504.0, 6e-8, -6e-8], device="cuda").half()
+    x = values.repeat_interleave(len(values)).repeat(8).view(-1, 8).contiguous()
+    dy = values.repeat(len(values)).repeat(8).view(-1, 8).contiguous()
+    want_x = x.clone().requires_grad_()
+    want = torch.relu(want_x) if act == 1 else torch.nn.functional.leaky_relu(want_x, slope)
+    want.backward(dy)
+    y, wide = ops._native.act_forward(x, act, slope, True)
+    dx = ops._native.act_backward(dy, None, x, act, slope)
+    ops.device_status()
+    for got, ref in ((y, want.detach()), (wide[:, 8:], want.detach()), (dx, want_x.grad)):
+        assert torch.allclose(got.float(), ref.float(), rtol=0, atol=0, equal_nan=True)

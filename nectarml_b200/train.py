@@ -550,8 +550,10 @@ class TrainStep:
     def _loss(self, out, target, denom):
         if self.loss_kind == "cross_entropy":
             return torch.nn.functional.cross_entropy(out.float(), target, reduction="sum") / denom
+        # (the kernels read pairs of values, so a view that starts on an odd one is left to torch, as is a count on the device)
         if (out.is_cuda and out.dtype == target.dtype == torch.float16 and out.shape == target.shape and out.is_contiguous()
-                and target.is_contiguous() and not target.requires_grad and out.numel() > 0):
+                and target.is_contiguous() and not target.requires_grad and out.numel() > 0
+                and out.data_ptr() % 4 == 0 and target.data_ptr() % 4 == 0 and not torch.is_tensor(denom)):
             return _L1Fn.apply(out, target, float(denom))
         return (out.float() - target.float()).abs().sum() / denom     # L1 against the target image
 

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from gpu_util import assert_f32, host
-from nectarml_b200 import ops
+from nectarml_b200 import ops, train
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,22 @@ def test_activation_of_overflowed_values(act, slope):
     ops.device_status()
     for got, ref in ((y, want.detach()), (wide[:, 8:], want.detach()), (dx, want_x.grad)):
         assert torch.allclose(got.float(), ref.float(), rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("device_count", [False, True])
+def test_l1_loss_of_views(offset, device_count):
+    """A target that starts anywhere in its storage, and a divisor that is a tensor: torch's formula, gradient included."""
+    gen = torch.Generator(device="cuda").manual_seed(offset)
+    flat = torch.randn(4 + 5 * 7 * 3, device="cuda", generator=gen).half()
+    target = flat[offset:offset + 5 * 7 * 3].view(1, 5, 7, 3)
+    out = torch.randn(1, 5, 7, 3, device="cuda", generator=gen).half()
+    count = torch.tensor(315.0, device="cuda") if device_count else 315
+    got_out, want_out = out.clone().requires_grad_(), out.clone().requires_grad_()
+    got = train.TrainStep(None, "l1")._loss(got_out, target, count)
+    want = (want_out.float() - target.float()).abs().sum() / 315
+    got.backward()
+    want.backward()
+    ops.device_status()
+    assert abs(float(got.detach()) - float(want.detach())) <= 1e-6 * float(want.detach())
+    assert torch.equal(got_out.grad, want_out.grad)

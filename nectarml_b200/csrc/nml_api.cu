@@ -1806,6 +1806,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
 }
 
 // Grow-only per-device workspace for the reference-shaped entry points.
+constexpr size_t kRefScratchLimit = 1ull << 30;  // what a batched product takes of it at most
 struct RefWorkspace {
     void* ptr = nullptr;
     size_t bytes = 0;
@@ -2329,11 +2330,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
     const long long tiles = 1ll * ceil_div(M, 128) * ceil_div(N, 256);
     const size_t c_entry = static_cast<size_t>(M) * N * es, a_entry = static_cast<size_t>(M) * K * es, b_entry = static_cast<size_t>(K) * N * es;
     size_t per_call = 1;  // entries per launch
-    if (!shared_b && b_batch != 1 && tiles < 2ll * planning_sms()) {
-        // bounded by the scratch of the converted operands (1 GB) and by the grid of the weight repack
-        const size_t scratch = (a_entry + b_entry) * 2 + 4096;
-        per_call = std::max<size_t>(1, std::min<size_t>({batch, 32768, (1ull << 30) / scratch}));
-    }
+    if (!shared_b && b_batch != 1 && tiles < 2ll * planning_sms()) per_call = std::min<size_t>(batch, 32768);  // (the grid of the weight repack)
     auto entries = [&](const uint8_t* A, const uint8_t* B, uint8_t* C, size_t n, Bump& bump) -> int {
         if (per_call == 1 || shared_b) {
             nml_linear_desc d;
@@ -2353,10 +2350,18 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
         return run_fprop_like(f, bump, nullptr);
     };
     if (shared_b) per_call = batch;
-    Bump dry{nullptr, 0, 0, true};
-    int rc = entries(nullptr, nullptr, nullptr, per_call, dry);
-    if (rc) return rc;
-    const size_t need = round_up(dry.off, 256);
+    // The converted operands of many small entries can be far larger than the operands (K is padded to a slice of 32 or 64, fp32
+    // becomes two planes), and the workspace stays for good: at most 1 GB of it, or one entry's.
+    size_t need = 0;
+    int rc;
+    for (;;) {
+        Bump dry{nullptr, 0, 0, true};
+        rc = entries(nullptr, nullptr, nullptr, per_call, dry);
+        if (rc) return rc;
+        need = round_up(dry.off, 256);
+        if (shared_b || per_call == 1 || need <= kRefScratchLimit) break;
+        per_call = std::max<size_t>(1, std::min(per_call - 1, static_cast<size_t>(static_cast<double>(per_call) * kRefScratchLimit / need)));
+    }
     void* ws = nullptr;
     rc = ref_workspace(need, &ws);
     if (rc) return rc;

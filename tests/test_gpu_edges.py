@@ -3,8 +3,8 @@ has to hand on."""
 import pytest
 import torch
 
-from gpu_util import assert_f32, host
-from nectarml_b200 import ops, train
+from gpu_util import F32, assert_f32, fetch, host
+from nectarml_b200 import _nectarml, ops, train
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,21 @@ def test_l1_loss_of_views(offset, device_count):
     ops.device_status()
     assert abs(float(got.detach()) - float(want.detach())) <= 1e-6 * float(want.detach())
     assert torch.equal(got_out.grad, want_out.grad)
+
+
+def test_batched_matmul_of_many_thin_entries_keeps_its_scratch():
+    """Entries with one or a few products per value: the converted operands are up to 32 times the operands (K is padded to a
+    slice), 2 GB here, and go through the workspace in shares of at most 1 GB (a quarter more is allocated)."""
+    batch, m, k, n = 8192, 8, 1, 1024
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    a, b = torch.randn(batch, m, k, device="cuda", generator=gen), torch.randn(batch, k, n, device="cuda", generator=gen)
+    torch.cuda.synchronize()
+    before, launches = torch.cuda.mem_get_info()[0], ops.launch_count()
+    ptr = _nectarml.tensor.matmul(a.data_ptr(), b.data_ptr(), a.shape, b.shape, F32)
+    torch.cuda.synchronize()
+    grown, launches = before - torch.cuda.mem_get_info()[0], ops.launch_count() - launches
+    got = fetch(ptr, (batch, m, n))
+    ops.device_status()
+    assert grown <= 1.25 * 2 ** 30 + got.nbytes + (64 << 20), grown
+    assert launches <= 16  # (shares, not entries)
+    assert_f32(got, (a.double() * b.double()).cpu().numpy(), "products")

@@ -47,6 +47,7 @@ struct Bump {
     size_t off, cap;
     bool dry;
     DeviceState* ds = nullptr;  // when set, used instead of the lazily allocated per-device state
+    size_t limit = SIZE_MAX;    // what a plan may ask for in all: regions that only buy speed are left out above it
     void* take(size_t bytes) {
         off = round_up(off, 256);
         void* p = dry ? nullptr : base + off;
@@ -54,6 +55,10 @@ struct Bump {
         return p;
     }
     bool fits() const { return dry || off <= cap; }
+    size_t room() const {  // left below the limit, for a region taken next
+        const size_t o = round_up(off, 256);
+        return o < limit ? limit - o : 0;
+    }
 };
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -720,7 +725,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     // one pass of full-width stores turns round.  Input gradient of 3x3 s2, fp32 result of fp16 / 3xTF32 products: 128 channels at
     // 28 x 28, batch 64 30.6 -> 28.4 / 48.4 -> 39.9 us; 256 at 28 x 28, batch 64 99.8 -> 54.4 / 131 -> 101; but 64 at 64 x 64 (whole
     // rows of 32) 54.2 -> 49.6 / 68.9 -> 85.5.  Below four million values the extra pass costs more than it saves (64 at 56 x 56,
-    // batch 16 13.3 -> 16.9).  Where the caller's workspace has no room for the copy, the walk stores directly.
+    // batch 16 13.3 -> 16.9).  Where the caller's workspace has no room for the copy, the walk stores directly; and above 1 GB,
+    // because callers keep their workspace and this would double what the result takes.
     const long long out_values = 1ll * f.batch * f.out_h * f.out_w * f.out_c;
     if (f.gather && f.s_w > 1 && f.out_layout == NML_NCHW && f.out_w > 1 && ceil_div(f.out_w, f.s_w) % 8 != 0 &&
         out_values >= (1 << 22) && f.out_c % (f.out_dtype == NML_F16 ? 64 : 32) == 0) {
@@ -734,7 +740,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const int probe_rc = run_fprop_like(f2, probe, st);
         const int tiles_p = ceil_div(hw, 64), tiles_c = ceil_div(f.out_c, 64);
         const long long tiles = 1ll * tiles_p * tiles_c * f.batch;
-        if (probe_rc == NML_OK && (ws.dry || probe.off <= ws.cap) && tiles < INT_MAX / 2) {
+        if (probe_rc == NML_OK && bytes <= (1ull << 30) && probe.off <= ws.limit && (ws.dry || probe.off <= ws.cap) && tiles < INT_MAX / 2) {
             f2.out = ws.take(bytes);
             const int rc = run_fprop_like(f2, ws, st);
             if (rc || ws.dry) return rc;
@@ -922,6 +928,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const long long tiles_lb = 1ll * ((out_pixels + 127) / 128) * ceil_div(N, 256);
         const int sms = ds ? limited(ds->sms) : planning_sms();
         z_cap = static_cast<int>(std::max<long long>(1, std::min<long long>(sms / tiles_lb, k_slices / 4)));
+        z_cap = static_cast<int>(std::min<size_t>(z_cap, ws.room() / (out_pixels * N * sizeof(float))));
     }
     const bool can_split = may_split && z_cap >= 2;
     float* split_acc = can_split ? static_cast<float*>(ws.take(static_cast<size_t>(z_cap) * out_pixels * N * sizeof(float))) : nullptr;
@@ -2103,7 +2110,8 @@ int nml_conv_forward_static(const nml_conv_desc* d, const void* x, const void* w
         return read_status_word(ss->ds.err, nullptr);  // the code is in nml_status_string(NML_ERR_DEVICE)
     }
     if (!x || !w || !y) return NML_ERR_INVALID;
-    Bump dry{nullptr, 0, 0, true};
+    // (both runs plan within the array: a K split or an output copy that does not fit is left out)
+    Bump dry{nullptr, 0, 0, true, nullptr, kStaticScratchBytes};
     int rc = conv_pass(d, NML_PASS_FORWARD, nullptr, nullptr, bias ? d : nullptr, nullptr, nullptr, dry, nullptr);
     if (rc) return rc;
     const size_t need = round_up(dry.off, 256);
@@ -2117,7 +2125,7 @@ int nml_conv_forward_static(const nml_conv_desc* d, const void* x, const void* w
     if (rc) return rc;
     // Every region of the scratch that the contraction reads is rewritten in full by the conversion
     // passes of this call (channel and K padding included), so nothing from the last call survives.
-    Bump ws{static_cast<uint8_t*>(ss->scratch), 0, kStaticScratchBytes, false, &ss->ds};
+    Bump ws{static_cast<uint8_t*>(ss->scratch), 0, kStaticScratchBytes, false, &ss->ds, kStaticScratchBytes};
     return conv_pass(d, NML_PASS_FORWARD, x, w, bias, y, nullptr, ws, static_cast<cudaStream_t>(stream));
 }
 

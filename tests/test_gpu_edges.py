@@ -75,3 +75,25 @@ def test_batched_matmul_of_many_thin_entries_keeps_its_scratch():
     assert grown <= 1.25 * 2 ** 30 + got.nbytes + (64 << 20), grown
     assert launches <= 16  # (shares, not entries)
     assert_f32(got, (a.double() * b.double()).cpu().numpy(), "products")
+
+
+@pytest.mark.parametrize("case", [(10, 64, 91, 108, 256, 4, 2, 1, True, "f16", "nchw"), (102, 512, 5, 32, 8, 1, 2, 0, False, "3xtf32", "nchw"),
+                                  (1, 512, 26, 17, 256, 7, 2, 3, False, "3xtf32", "nhwc")])
+def test_static_entry_point_without_optional_scratch(case):
+    """Layers whose full plan (a copy of the result, planes of a K split) does not fit the built-in scratch: the plan without
+    gives the result of the call with a workspace.  The fp32 sums differ in order alone: 2.5e-9 of the result per term."""
+    import ctypes as C
+    from nectarml_b200 import _lib
+    b, ci, h, w, co, k, s, p, tr, math, lay = case
+    g = ops.ConvGeometry(b, ci, h, w, co, k, k, (s, s), (p, p), transposed=tr)
+    gen = torch.Generator(device="cuda").manual_seed(b)
+    x = torch.randn(g.act_shape("in", lay), device="cuda", generator=gen)
+    wt = torch.randn(g.weight_shape(), device="cuda", generator=gen) * 0.1
+    bias = torch.randn(co, device="cuda", generator=gen)
+    want = ops.conv_forward(g, x, wt, bias, layout=lay, math=math)
+    got = torch.empty_like(want)
+    d = g.desc(_lib.NML_F32, lay, _lib.NML_F32, lay, _lib.NML_F32, math, False)
+    _lib.check(_lib.load().nml_conv_forward_static(C.byref(d), x.data_ptr(), wt.data_ptr(), bias.data_ptr(), got.data_ptr(),
+                                                   torch.cuda.current_stream().cuda_stream))
+    _lib.check(_lib.load().nml_conv_forward_static(None, None, None, None, None, None))
+    assert_f32(host(got), host(want), "static", 1e-6 + 2.5e-9 * ci * k * k)

@@ -26,3 +26,36 @@ def test_every_3xtf32_weight_gradient_has_a_plan(lib):
         if need.value < 2 * 4 * 32 * k * (fin + fout) + planes:
             missing.append(k)
     assert not missing, (len(missing), missing[:5])
+
+
+# (batch, c_in, h, w, c_out, kernel, stride, padding, transposed, math, out layout): scratch without the regions that only buy speed
+# fits the static entry point's array, with them it does not
+STATIC = [
+    (10, 64, 91, 108, 256, 4, 2, 1, True, "f16", "nchw"),       # NHWC copy of a ragged strided result
+    (108, 64, 19, 7, 512, 7, 2, 3, True, "3xtf32", "nchw"),
+    (1, 512, 26, 17, 256, 7, 2, 3, False, "3xtf32", "nhwc"),    # planes of a K split
+    (102, 512, 5, 32, 8, 1, 2, 0, False, "3xtf32", "nchw"),
+]
+
+
+@pytest.mark.parametrize("case", STATIC)
+def test_static_entry_point_takes_what_fits_without_optional_scratch(lib, case):
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("stands in for pointers with numbers; the GPU suite runs such a layer")
+    b, ci, h, w, co, k, s, p, tr, math, lay = case
+    g = ops.ConvGeometry(b, ci, h, w, co, k, k, (s, s), (p, p), transposed=tr)
+    d = g.desc(NML_F32, lay, NML_F32, lay, NML_F32, math, False)
+    st = lib.nml_conv_forward_static(C.byref(d), 256, 256, None, 256, None)
+    assert st == _lib.NML_OK + 3, lib.nml_status_string(st)  # (CUDA: no device here; not "needs N bytes of scratch")
+
+
+def test_output_copy_is_bounded(lib):
+    """Above 1 GB the strided result is stored directly: a workspace is kept by its caller and stays this large."""
+    need = C.c_size_t()
+    for batch, copied in ((12, True), (55, False)):
+        g = ops.ConvGeometry(batch, 8, 87, 113, 512, 4, 4, (2, 2), (1, 1), transposed=True)
+        ho, wo = g.out_hw()
+        d = g.desc(NML_F32, "nchw", NML_F32, "nchw", NML_F32, "f16", False)
+        assert lib.nml_conv_workspace_size(C.byref(d), 0, C.byref(need)) == _lib.NML_OK
+        assert (need.value > batch * 512 * ho * wo * 4) == copied

@@ -21,7 +21,6 @@
 #include <torch/csrc/autograd/saved_variable.h>
 
 #include <cstring>
-#include <exception>
 #include <initializer_list>
 #include <memory>
 #include <string>
@@ -68,11 +67,14 @@ int dtype_of(const at::Tensor& t) {
     if (s == at::kHalf) return NML_F16;
     fail("only float32 and float16 tensors are supported");
 }
+// (Callers take every pointer before they ask for the stream: a tensor in the wrong place is reported as such even where there
+// is no GPU to have a stream on.)
 void* ptr(const at::Tensor& t) {
     if (!t.is_cuda()) fail("tensors must live on a CUDA device (there is no CPU path)");
     if (!t.is_contiguous()) fail("tensors must be contiguous");
     return t.data_ptr();
 }
+inline float* floats(const at::Tensor& t) { return static_cast<float*>(ptr(t)); }
 inline void* ptr_or_null(const at::Tensor* t) { return t ? ptr(*t) : nullptr; }
 inline void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
@@ -132,16 +134,17 @@ Scratch scratch(PyObject* ws, size_t need, const at::Tensor& like) {
     fail("the workspace object did not grow");
 }
 
-// Runs a function body with C++ exceptions turned into Python ones.
+// Runs a function body with C++ exceptions turned into the Python ones torch's own functions raise (out of memory and index
+// errors have types of their own).
 template <class F>
 PyObject* guarded(F&& f) {
+    HANDLE_TH_ERRORS
     try {
         return f();
     } catch (const Fail&) {
-    } catch (const std::exception& e) {
-        if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
     }
-    return nullptr;
+    END_HANDLE_TH_ERRORS
 }
 PyObject* pair(const at::Tensor& a, const at::Tensor* b) {
     PyObject* pa = THPVariable_Wrap(a);
@@ -240,7 +243,8 @@ at::Tensor run_conv_forward(const Geometry& g, const at::Tensor& x, const at::Te
     size_t need = 0;
     check(nml_conv_workspace_size(&d, NML_PASS_FORWARD, &need));
     const Scratch ws = scratch(workspace, need, x);
-    check(nml_conv_forward(&d, ptr(x), ptr(w), ptr_or_null(bias), ptr(out), ws.p, ws.bytes, stream()));
+    void *const px = ptr(x), *const pw = ptr(w), *const pb = ptr_or_null(bias), *const po = ptr(out);
+    check(nml_conv_forward(&d, px, pw, pb, po, ws.p, ws.bytes, stream()));
     return out;
 }
 
@@ -261,7 +265,8 @@ at::Tensor run_conv_backward_data(const Geometry& g, const at::Tensor& dy, const
     size_t need = 0;
     check(nml_conv_workspace_size(&d, NML_PASS_BACKWARD_DATA, &need));
     const Scratch ws = scratch(workspace, need, dy);
-    check(nml_conv_backward_data(&d, ptr(dy), ptr(w), ptr(out), ws.p, ws.bytes, stream()));
+    void *const pd = ptr(dy), *const pw = ptr(w), *const po = ptr(out);
+    check(nml_conv_backward_data(&d, pd, pw, po, ws.p, ws.bytes, stream()));
     return out;
 }
 
@@ -282,8 +287,9 @@ void run_conv_backward_weight(const Geometry& g, const at::Tensor& x, const at::
     size_t need = 0;
     check(nml_conv_workspace_size(&d, NML_PASS_BACKWARD_WEIGHT, &need));
     const Scratch ws = scratch(workspace, need, x);
-    check(nml_conv_backward_weight(&d, ptr(x), ptr(dy), static_cast<float*>(ptr(dw)), db.defined() ? static_cast<float*>(ptr(db)) : nullptr,
-                                   ws.p, ws.bytes, stream()));
+    void *const px = ptr(x), *const pd = ptr(dy);
+    float *const pdw = floats(dw), *const pdb = db.defined() ? floats(db) : nullptr;
+    check(nml_conv_backward_weight(&d, px, pd, pdw, pdb, ws.p, ws.bytes, stream()));
 }
 
 // conv_forward(geometry, x, w, bias, out, layout, out_layout, math, out_dtype, round_f16, workspace)
@@ -350,7 +356,8 @@ PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         size_t need = 0;
         check(nml_linear_workspace_size(&d, NML_PASS_FORWARD, &need));
         const Scratch ws = scratch(a[7], need, x);
-        check(nml_linear_forward(&d, ptr(x), ptr(w), ptr_or_null(bias), ptr(out), ws.p, ws.bytes, stream()));
+        void *const px = ptr(x), *const pw = ptr(w), *const pb = ptr_or_null(bias), *const po = ptr(out);
+        check(nml_linear_forward(&d, px, pw, pb, po, ws.p, ws.bytes, stream()));
         return THPVariable_Wrap(out);
     });
 }
@@ -369,7 +376,8 @@ PyObject* py_linear_backward_data(PyObject*, PyObject* const* a, Py_ssize_t n) {
         size_t need = 0;
         check(nml_linear_workspace_size(&d, NML_PASS_BACKWARD_DATA, &need));
         const Scratch ws = scratch(a[5], need, dy);
-        check(nml_linear_backward_data(&d, ptr(dy), ptr(w), ptr(out), ws.p, ws.bytes, stream()));
+        void *const pd = ptr(dy), *const pw = ptr(w), *const po = ptr(out);
+        check(nml_linear_backward_data(&d, pd, pw, po, ws.p, ws.bytes, stream()));
         return THPVariable_Wrap(out);
     });
 }
@@ -391,8 +399,9 @@ PyObject* py_linear_backward_weight(PyObject*, PyObject* const* a, Py_ssize_t n)
         size_t need = 0;
         check(nml_linear_workspace_size(&d, NML_PASS_BACKWARD_WEIGHT, &need));
         const Scratch ws = scratch(a[6], need, x);
-        check(nml_linear_backward_weight(&d, ptr(x), ptr(dy), static_cast<float*>(ptr(dw)),
-                                         has_db ? static_cast<float*>(ptr(db)) : nullptr, ws.p, ws.bytes, stream()));
+        void *const px = ptr(x), *const pd = ptr(dy);
+        float *const pdw = floats(dw), *const pdb = has_db ? floats(db) : nullptr;
+        check(nml_linear_backward_weight(&d, px, pd, pdw, pdb, ws.p, ws.bytes, stream()));
         return pair(dw, has_db ? &db : nullptr);
     });
 }
@@ -409,6 +418,11 @@ PyObject* tuple_of(const T&... t) {
     for (size_t i = 0; i < sizeof...(t); ++i) PyTuple_SET_ITEM(r, i, items[i]);
     return r;
 }
+int64_t channels(const at::Tensor& x) {
+    const int64_t c = x.size(-1);
+    require(c > 0, "a tensor without channels");
+    return c;
+}
 at::Tensor wide_like(const at::Tensor& x) {
     auto shape = x.sizes().vec();
     shape.back() *= 2;
@@ -416,7 +430,7 @@ at::Tensor wide_like(const at::Tensor& x) {
 }
 void* channels_from(const at::Tensor& wide, int64_t c) { return static_cast<char*>(ptr(wide)) + c * wide.element_size(); }
 void require_half_rows(const at::Tensor& t, const at::Tensor& x, int64_t c, const char* what) {
-    require(t.scalar_type() == at::kHalf && t.numel() / t.size(-1) == x.numel() / x.size(-1) && t.size(-1) == c, what);
+    require(t.scalar_type() == at::kHalf && t.size(-1) == c && t.numel() / c == x.numel() / channels(x), what);
 }
 
 // The gradient of an output: dy and, for an output that also is the last channels of a wide tensor, that tensor's
@@ -426,7 +440,7 @@ struct OutputGrad {
     int pitch = 0, pitch2 = 0;
 };
 OutputGrad output_grad(const at::Tensor& dy, const at::Tensor* dskip, bool join, const at::Tensor& x) {
-    const int64_t c = x.size(-1);
+    const int64_t c = channels(x);
     require_half_rows(dy, x, join ? 2 * c : c, "dy does not have the output's shape");
     OutputGrad g{ptr(dy)};
     if (join) g.pitch = static_cast<int>(2 * c);
@@ -443,7 +457,7 @@ struct BnSaved {
 };
 BnSaved run_bn_forward(const at::Tensor& x, const at::Tensor* res, const at::Tensor& gamma, const at::Tensor& beta, int act, float slope,
                        float eps, const at::Tensor* join, bool skip, PyObject* workspace) {
-    const int64_t c = x.size(-1), rows = x.numel() / c;
+    const int64_t c = channels(x), rows = x.numel() / c;
     if (join) require_half_rows(*join, x, 2 * c, "join has twice the channels of x");
     BnSaved r;
     r.y = join ? join->variable_data() : at::empty(x.sizes(), x.options());
@@ -456,10 +470,11 @@ BnSaved run_bn_forward(const at::Tensor& x, const at::Tensor* res, const at::Ten
     size_t need = 0;
     check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
     const Scratch ws = scratch(workspace, need, x);
-    check(nml_bn_forward_masked(ptr(x), rows, static_cast<int>(c), static_cast<const float*>(ptr(gamma)), static_cast<const float*>(ptr(beta)),
-                                ptr_or_null(res), act, slope, eps, ptr(r.y), join ? pitch : 0,
-                                skip ? channels_from(r.wide, c) : nullptr, pitch, r.mask.defined() ? ptr(r.mask) : nullptr,
-                                static_cast<float*>(ptr(r.mean)), static_cast<float*>(ptr(r.rstd)), ws.p, ws.bytes, stream()));
+    void *const px = ptr(x), *const pres = ptr_or_null(res), *const py = ptr(r.y);
+    void *const py2 = skip ? channels_from(r.wide, c) : nullptr, *const pmask = r.mask.defined() ? ptr(r.mask) : nullptr;
+    float *const pg = floats(gamma), *const pb = floats(beta), *const pm = floats(r.mean), *const pr = floats(r.rstd);
+    check(nml_bn_forward_masked(px, rows, static_cast<int>(c), pg, pb, pres, act, slope, eps, py, join ? pitch : 0, py2, pitch, pmask, pm, pr,
+                                ws.p, ws.bytes, stream()));
     return r;
 }
 
@@ -467,16 +482,16 @@ BnSaved run_bn_forward(const at::Tensor& x, const at::Tensor* res, const at::Ten
 at::Tensor run_bn_backward(const OutputGrad& g, const at::Tensor* mask, const at::Tensor& x, const at::Tensor& gamma, const at::Tensor& beta,
                            const at::Tensor& mean, const at::Tensor& rstd, int act, float slope, const at::Tensor& dres,
                            const at::Tensor& dgamma, const at::Tensor& dbeta, PyObject* workspace) {
-    const int64_t c = x.size(-1), rows = x.numel() / c;
+    const int64_t c = channels(x), rows = x.numel() / c;
     const at::Tensor dx = at::empty(x.sizes(), x.options());
     size_t need = 0;
     check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
     const Scratch ws = scratch(workspace, need, x);
-    check(nml_bn_backward_masked(g.a, g.pitch, g.b, g.pitch2, ptr_or_null(mask), ptr(x), rows, static_cast<int>(c),
-                                 static_cast<const float*>(ptr(gamma)), static_cast<const float*>(ptr(beta)),
-                                 static_cast<const float*>(ptr(mean)), static_cast<const float*>(ptr(rstd)), act, slope, ptr(dx),
-                                 dres.defined() ? ptr(dres) : nullptr, static_cast<float*>(ptr(dgamma)), static_cast<float*>(ptr(dbeta)),
-                                 ws.p, ws.bytes, stream()));
+    void *const px = ptr(x), *const pmask = ptr_or_null(mask), *const pdx = ptr(dx), *const pdres = dres.defined() ? ptr(dres) : nullptr;
+    float *const pg = floats(gamma), *const pb = floats(beta), *const pm = floats(mean), *const pr = floats(rstd);
+    float *const pdg = floats(dgamma), *const pdb = floats(dbeta);
+    check(nml_bn_backward_masked(g.a, g.pitch, g.b, g.pitch2, pmask, px, rows, static_cast<int>(c), pg, pb, pm, pr, act, slope, pdx, pdres, pdg,
+                                 pdb, ws.p, ws.bytes, stream()));
     return dx;
 }
 
@@ -514,13 +529,15 @@ PyObject* py_act_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!arity(n, 4)) return nullptr;
     return guarded([&]() -> PyObject* {
         const at::Tensor& x = tensor(a[0], "x");
-        const int64_t c = x.size(-1);
+        const int64_t c = channels(x);
         require_half_rows(x, x, c, "x is float16");
         const at::Tensor y = at::empty(x.sizes(), x.options());
         at::Tensor wide;
         if (as_int(a[3]) != 0) wide = wide_like(x);
-        check(nml_act_forward(ptr(x), x.numel() / c, static_cast<int>(c), static_cast<int>(as_int(a[1])), static_cast<float>(as_double(a[2])),
-                              ptr(y), wide.defined() ? channels_from(wide, c) : nullptr, static_cast<int>(2 * c), stream()));
+        const int act = static_cast<int>(as_int(a[1]));
+        const float slope = static_cast<float>(as_double(a[2]));
+        void *const px = ptr(x), *const py = ptr(y), *const py2 = wide.defined() ? channels_from(wide, c) : nullptr;
+        check(nml_act_forward(px, x.numel() / c, static_cast<int>(c), act, slope, py, py2, static_cast<int>(2 * c), stream()));
         return tuple_of(y, wide);
     });
 }
@@ -530,11 +547,13 @@ PyObject* py_act_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!arity(n, 5)) return nullptr;
     return guarded([&]() -> PyObject* {
         const at::Tensor &dy = tensor(a[0], "dy"), &x = tensor(a[2], "x");
-        const int64_t c = x.size(-1);
+        const int64_t c = channels(x);
         const OutputGrad g = output_grad(dy, tensor_or_none(a[1], "dwide"), false, x);
         const at::Tensor dx = at::empty(x.sizes(), x.options());
-        check(nml_act_backward(g.a, g.pitch, g.b, g.pitch2, ptr(x), x.numel() / c, static_cast<int>(c), static_cast<int>(as_int(a[3])),
-                               static_cast<float>(as_double(a[4])), ptr(dx), stream()));
+        const int act = static_cast<int>(as_int(a[3]));
+        const float slope = static_cast<float>(as_double(a[4]));
+        void *const px = ptr(x), *const pdx = ptr(dx);
+        check(nml_act_backward(g.a, g.pitch, g.b, g.pitch2, px, x.numel() / c, static_cast<int>(c), act, slope, pdx, stream()));
         return THPVariable_Wrap(dx);
     });
 }
@@ -753,8 +772,10 @@ PyObject* py_l1_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
         size_t need = 0;
         check(nml_l1_workspace_size(&need));
         const Scratch ws = scratch(args[3], need, a);
-        check(nml_l1_forward(ptr(a), ptr(b), a.numel(), static_cast<float>(as_double(args[2])), static_cast<float*>(ptr(loss)), ws.p, ws.bytes,
-                             stream()));
+        const float denom = static_cast<float>(as_double(args[2]));
+        void *const pa = ptr(a), *const pb = ptr(b);
+        float* const pl = floats(loss);
+        check(nml_l1_forward(pa, pb, a.numel(), denom, pl, ws.p, ws.bytes, stream()));
         return THPVariable_Wrap(loss);
     });
 }
@@ -766,8 +787,10 @@ PyObject* py_l1_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
         const at::Tensor &a = tensor(args[0], "a"), &b = tensor(args[1], "b"), &dloss = tensor(args[2], "dloss");
         require(dloss.scalar_type() == at::kFloat && dloss.numel() == 1, "the gradient of the loss is one float32");
         const at::Tensor da = at::empty(a.sizes(), a.options());
-        check(nml_l1_backward(ptr(a), ptr(b), a.numel(), static_cast<const float*>(ptr(dloss)), static_cast<float>(as_double(args[3])), ptr(da),
-                              stream()));
+        const float denom = static_cast<float>(as_double(args[3]));
+        void *const pa = ptr(a), *const pb = ptr(b), *const pda = ptr(da);
+        float* const pl = floats(dloss);
+        check(nml_l1_backward(pa, pb, a.numel(), pl, denom, pda, stream()));
         return THPVariable_Wrap(da);
     });
 }

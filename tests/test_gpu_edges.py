@@ -97,3 +97,11 @@ def test_static_entry_point_without_optional_scratch(case):
                                                    torch.cuda.current_stream().cuda_stream))
     _lib.check(_lib.load().nml_conv_forward_static(None, None, None, None, None, None))
     assert_f32(host(got), host(want), "static", 1e-6 + 2.5e-9 * ci * k * k)
+
+
+def test_out_of_memory_has_torchs_type():
+    """A result that no GPU holds: torch.OutOfMemoryError (what programs catch to try again with a smaller batch)."""
+    x = torch.zeros(1, 8, device="cuda").expand(1 << 28, 8)
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.linear_forward(x, torch.zeros(1 << 20, 8, device="cuda"))
+    ops.device_status()

@@ -7,12 +7,12 @@
 // on the GPU.  Here the same work is about 2 us: linear 32 x 512 -> 2048 forward 16.2 -> 7 us per call.
 //
 // Nothing is kept between calls except the parsed geometry of a layer (a capsule owned by the Python
-// ConvGeometry object).  The GIL stays held: every function returns within a few microseconds.
+// ConvGeometry object).  The GIL is released while memory is allocated and while kernels are launched: an allocation may
+// synchronise the device, and a launch waits where the stream's queue is full, for as long as the GPU is behind.
 #include <Python.h>
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
-#include <ATen/ops/empty_like.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -23,6 +23,7 @@
 #include <cstring>
 #include <initializer_list>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -76,7 +77,36 @@ void* ptr(const at::Tensor& t) {
 }
 inline float* floats(const at::Tensor& t) { return static_cast<float*>(ptr(t)); }
 inline void* ptr_or_null(const at::Tensor* t) { return t ? ptr(*t) : nullptr; }
-inline void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+
+struct NoGil {
+    PyThreadState* const state = PyEval_SaveThread();
+    NoGil() = default;
+    NoGil(const NoGil&) = delete;
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+template <class F>
+auto without_gil(F&& f) {
+    NoGil off;
+    return f();
+}
+at::Tensor new_empty(at::IntArrayRef shape, const at::TensorOptions& options) {
+    return without_gil([&] { return at::empty(shape, options); });
+}
+
+// Launches a pass, f(stream) -> status, on the current stream.  A pass is several kernels that share the workspace, so the
+// passes that threads issue on one stream follow one another whole: a lock per stream (streams that share one by their hash only
+// take turns), taken without the GIL and given back before it.
+template <class F>
+void issue(F&& f) {
+    static std::mutex order[64];
+    const auto s = c10::cuda::getCurrentCUDAStream();
+    const int status = without_gil([&] {
+        const size_t key = reinterpret_cast<size_t>(s.stream()) / 64 + 7u * static_cast<size_t>(s.device_index());
+        std::lock_guard<std::mutex> turn(order[(key ^ key >> 6 ^ key >> 12) % 64]);
+        return f(static_cast<void*>(s.stream()));
+    });
+    check(status);
+}
 
 long as_int(PyObject* o) {
     const long v = PyLong_AsLong(o);
@@ -93,7 +123,7 @@ double as_double(PyObject* o) {
 at::Tensor output(PyObject* given, at::IntArrayRef shape, long dtype_code, const at::Tensor& like) {
     if (given != Py_None) return tensor(given, "out");
     const auto st = dtype_code < 0 ? like.scalar_type() : dtype_code == NML_F16 ? at::kHalf : at::kFloat;
-    return at::empty(shape, at::TensorOptions().dtype(st).device(like.device()));
+    return new_empty(shape, at::TensorOptions().dtype(st).device(like.device()));
 }
 
 // Scratch from the caller's Workspace object (a grow-only buffer, see ops.Workspace): its tensor as it is while it is
@@ -101,6 +131,7 @@ at::Tensor output(PyObject* given, at::IntArrayRef shape, long dtype_code, const
 struct Scratch {
     void* p = nullptr;
     size_t bytes = 0;
+    at::Tensor hold;  // until the pass is launched: another thread may make the workspace grow meanwhile
 };
 Scratch scratch(PyObject* ws, size_t need, const at::Tensor& like) {
     static PyObject* const kBuf = PyUnicode_InternFromString("buf");
@@ -115,6 +146,7 @@ Scratch scratch(PyObject* ws, size_t need, const at::Tensor& like) {
             if (static_cast<size_t>(t.numel()) >= need && t.device() == like.device()) {
                 s.p = t.data_ptr();
                 s.bytes = t.numel();
+                s.hold = t;
                 Py_DECREF(buf);
                 return s;
             }
@@ -244,7 +276,9 @@ at::Tensor run_conv_forward(const Geometry& g, const at::Tensor& x, const at::Te
     check(nml_conv_workspace_size(&d, NML_PASS_FORWARD, &need));
     const Scratch ws = scratch(workspace, need, x);
     void *const px = ptr(x), *const pw = ptr(w), *const pb = ptr_or_null(bias), *const po = ptr(out);
-    check(nml_conv_forward(&d, px, pw, pb, po, ws.p, ws.bytes, stream()));
+    issue([&](void* st) {
+        return nml_conv_forward(&d, px, pw, pb, po, ws.p, ws.bytes, st);
+    });
     return out;
 }
 
@@ -266,7 +300,9 @@ at::Tensor run_conv_backward_data(const Geometry& g, const at::Tensor& dy, const
     check(nml_conv_workspace_size(&d, NML_PASS_BACKWARD_DATA, &need));
     const Scratch ws = scratch(workspace, need, dy);
     void *const pd = ptr(dy), *const pw = ptr(w), *const po = ptr(out);
-    check(nml_conv_backward_data(&d, pd, pw, po, ws.p, ws.bytes, stream()));
+    issue([&](void* st) {
+        return nml_conv_backward_data(&d, pd, pw, po, ws.p, ws.bytes, st);
+    });
     return out;
 }
 
@@ -289,7 +325,9 @@ void run_conv_backward_weight(const Geometry& g, const at::Tensor& x, const at::
     const Scratch ws = scratch(workspace, need, x);
     void *const px = ptr(x), *const pd = ptr(dy);
     float *const pdw = floats(dw), *const pdb = db.defined() ? floats(db) : nullptr;
-    check(nml_conv_backward_weight(&d, px, pd, pdw, pdb, ws.p, ws.bytes, stream()));
+    issue([&](void* st) {
+        return nml_conv_backward_weight(&d, px, pd, pdw, pdb, ws.p, ws.bytes, st);
+    });
 }
 
 // conv_forward(geometry, x, w, bias, out, layout, out_layout, math, out_dtype, round_f16, workspace)
@@ -357,7 +395,9 @@ PyObject* py_linear_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         check(nml_linear_workspace_size(&d, NML_PASS_FORWARD, &need));
         const Scratch ws = scratch(a[7], need, x);
         void *const px = ptr(x), *const pw = ptr(w), *const pb = ptr_or_null(bias), *const po = ptr(out);
-        check(nml_linear_forward(&d, px, pw, pb, po, ws.p, ws.bytes, stream()));
+        issue([&](void* st) {
+            return nml_linear_forward(&d, px, pw, pb, po, ws.p, ws.bytes, st);
+        });
         return THPVariable_Wrap(out);
     });
 }
@@ -377,7 +417,9 @@ PyObject* py_linear_backward_data(PyObject*, PyObject* const* a, Py_ssize_t n) {
         check(nml_linear_workspace_size(&d, NML_PASS_BACKWARD_DATA, &need));
         const Scratch ws = scratch(a[5], need, dy);
         void *const pd = ptr(dy), *const pw = ptr(w), *const po = ptr(out);
-        check(nml_linear_backward_data(&d, pd, pw, po, ws.p, ws.bytes, stream()));
+        issue([&](void* st) {
+            return nml_linear_backward_data(&d, pd, pw, po, ws.p, ws.bytes, st);
+        });
         return THPVariable_Wrap(out);
     });
 }
@@ -401,7 +443,9 @@ PyObject* py_linear_backward_weight(PyObject*, PyObject* const* a, Py_ssize_t n)
         const Scratch ws = scratch(a[6], need, x);
         void *const px = ptr(x), *const pd = ptr(dy);
         float *const pdw = floats(dw), *const pdb = has_db ? floats(db) : nullptr;
-        check(nml_linear_backward_weight(&d, px, pd, pdw, pdb, ws.p, ws.bytes, stream()));
+        issue([&](void* st) {
+            return nml_linear_backward_weight(&d, px, pd, pdw, pdb, ws.p, ws.bytes, st);
+        });
         return pair(dw, has_db ? &db : nullptr);
     });
 }
@@ -426,7 +470,7 @@ int64_t channels(const at::Tensor& x) {
 at::Tensor wide_like(const at::Tensor& x) {
     auto shape = x.sizes().vec();
     shape.back() *= 2;
-    return at::empty(shape, x.options());
+    return new_empty(shape, x.options());
 }
 void* channels_from(const at::Tensor& wide, int64_t c) { return static_cast<char*>(ptr(wide)) + c * wide.element_size(); }
 void require_half_rows(const at::Tensor& t, const at::Tensor& x, int64_t c, const char* what) {
@@ -460,11 +504,11 @@ BnSaved run_bn_forward(const at::Tensor& x, const at::Tensor* res, const at::Ten
     const int64_t c = channels(x), rows = x.numel() / c;
     if (join) require_half_rows(*join, x, 2 * c, "join has twice the channels of x");
     BnSaved r;
-    r.y = join ? join->variable_data() : at::empty(x.sizes(), x.options());
+    r.y = join ? join->variable_data() : new_empty(x.sizes(), x.options());
     const auto fopt = at::TensorOptions().dtype(at::kFloat).device(x.device());
-    r.mean = at::empty({c}, fopt);
-    r.rstd = at::empty({c}, fopt);
-    if (res != nullptr && act != 0) r.mask = at::empty({x.numel() / 8}, fopt.dtype(at::kByte));
+    r.mean = new_empty({c}, fopt);
+    r.rstd = new_empty({c}, fopt);
+    if (res != nullptr && act != 0) r.mask = new_empty({x.numel() / 8}, fopt.dtype(at::kByte));
     if (skip) r.wide = wide_like(x);
     const int pitch = static_cast<int>(2 * c);
     size_t need = 0;
@@ -473,8 +517,10 @@ BnSaved run_bn_forward(const at::Tensor& x, const at::Tensor* res, const at::Ten
     void *const px = ptr(x), *const pres = ptr_or_null(res), *const py = ptr(r.y);
     void *const py2 = skip ? channels_from(r.wide, c) : nullptr, *const pmask = r.mask.defined() ? ptr(r.mask) : nullptr;
     float *const pg = floats(gamma), *const pb = floats(beta), *const pm = floats(r.mean), *const pr = floats(r.rstd);
-    check(nml_bn_forward_masked(px, rows, static_cast<int>(c), pg, pb, pres, act, slope, eps, py, join ? pitch : 0, py2, pitch, pmask, pm, pr,
-                                ws.p, ws.bytes, stream()));
+    issue([&](void* st) {
+        return nml_bn_forward_masked(px, rows, static_cast<int>(c), pg, pb, pres, act, slope, eps, py, join ? pitch : 0, py2, pitch, pmask,
+                                     pm, pr, ws.p, ws.bytes, st);
+    });
     return r;
 }
 
@@ -483,15 +529,17 @@ at::Tensor run_bn_backward(const OutputGrad& g, const at::Tensor* mask, const at
                            const at::Tensor& mean, const at::Tensor& rstd, int act, float slope, const at::Tensor& dres,
                            const at::Tensor& dgamma, const at::Tensor& dbeta, PyObject* workspace) {
     const int64_t c = channels(x), rows = x.numel() / c;
-    const at::Tensor dx = at::empty(x.sizes(), x.options());
+    const at::Tensor dx = new_empty(x.sizes(), x.options());
     size_t need = 0;
     check(nml_bn_workspace_size(rows, static_cast<int>(c), &need));
     const Scratch ws = scratch(workspace, need, x);
     void *const px = ptr(x), *const pmask = ptr_or_null(mask), *const pdx = ptr(dx), *const pdres = dres.defined() ? ptr(dres) : nullptr;
     float *const pg = floats(gamma), *const pb = floats(beta), *const pm = floats(mean), *const pr = floats(rstd);
     float *const pdg = floats(dgamma), *const pdb = floats(dbeta);
-    check(nml_bn_backward_masked(g.a, g.pitch, g.b, g.pitch2, pmask, px, rows, static_cast<int>(c), pg, pb, pm, pr, act, slope, pdx, pdres, pdg,
-                                 pdb, ws.p, ws.bytes, stream()));
+    issue([&](void* st) {
+        return nml_bn_backward_masked(g.a, g.pitch, g.b, g.pitch2, pmask, px, rows, static_cast<int>(c), pg, pb, pm, pr, act, slope, pdx,
+                                      pdres, pdg, pdb, ws.p, ws.bytes, st);
+    });
     return dx;
 }
 
@@ -515,7 +563,7 @@ PyObject* py_bn_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor& x = tensor(a[4], "x");
         const OutputGrad g = output_grad(tensor(a[0], "dy"), tensor_or_none(a[1], "dwide"), as_int(a[2]) != 0, x);
         at::Tensor dres;
-        if (as_int(a[11]) != 0) dres = at::empty(x.sizes(), x.options());
+        if (as_int(a[11]) != 0) dres = new_empty(x.sizes(), x.options());
         const at::Tensor dx = run_bn_backward(g, tensor_or_none(a[3], "mask"), x, tensor(a[5], "gamma"), tensor(a[6], "beta"),
                                               tensor(a[7], "mean"), tensor(a[8], "rstd"), static_cast<int>(as_int(a[9])),
                                               static_cast<float>(as_double(a[10])), dres, tensor(a[12], "dgamma"), tensor(a[13], "dbeta"),
@@ -531,13 +579,15 @@ PyObject* py_act_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor& x = tensor(a[0], "x");
         const int64_t c = channels(x);
         require_half_rows(x, x, c, "x is float16");
-        const at::Tensor y = at::empty(x.sizes(), x.options());
+        const at::Tensor y = new_empty(x.sizes(), x.options());
         at::Tensor wide;
         if (as_int(a[3]) != 0) wide = wide_like(x);
         const int act = static_cast<int>(as_int(a[1]));
         const float slope = static_cast<float>(as_double(a[2]));
         void *const px = ptr(x), *const py = ptr(y), *const py2 = wide.defined() ? channels_from(wide, c) : nullptr;
-        check(nml_act_forward(px, x.numel() / c, static_cast<int>(c), act, slope, py, py2, static_cast<int>(2 * c), stream()));
+        issue([&](void* st) {
+            return nml_act_forward(px, x.numel() / c, static_cast<int>(c), act, slope, py, py2, static_cast<int>(2 * c), st);
+        });
         return tuple_of(y, wide);
     });
 }
@@ -549,11 +599,13 @@ PyObject* py_act_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor &dy = tensor(a[0], "dy"), &x = tensor(a[2], "x");
         const int64_t c = channels(x);
         const OutputGrad g = output_grad(dy, tensor_or_none(a[1], "dwide"), false, x);
-        const at::Tensor dx = at::empty(x.sizes(), x.options());
+        const at::Tensor dx = new_empty(x.sizes(), x.options());
         const int act = static_cast<int>(as_int(a[3]));
         const float slope = static_cast<float>(as_double(a[4]));
         void *const px = ptr(x), *const pdx = ptr(dx);
-        check(nml_act_backward(g.a, g.pitch, g.b, g.pitch2, px, x.numel() / c, static_cast<int>(c), act, slope, pdx, stream()));
+        issue([&](void* st) {
+            return nml_act_backward(g.a, g.pitch, g.b, g.pitch2, px, x.numel() / c, static_cast<int>(c), act, slope, pdx, st);
+        });
         return THPVariable_Wrap(dx);
     });
 }
@@ -594,12 +646,14 @@ struct Owner {
         if (!flag(0)) {
             run(a, b);
         } else {
-            const at::Tensor ta = at::empty_like(a);
+            const at::Tensor ta = new_empty(a.sizes(), a.options());
             at::Tensor tb;
-            if (b.defined()) tb = at::empty_like(b);
+            if (b.defined()) tb = new_empty(b.sizes(), b.options());
             run(ta, tb);
-            a.add_(ta);
-            if (b.defined()) b.add_(tb);
+            without_gil([&] {
+                a.add_(ta);
+                if (b.defined()) b.add_(tb);
+            });
         }
         if (flag(1)) {
             PyObject* r = PyObject_CallMethod(layer, "gradient_written", nullptr);
@@ -643,7 +697,7 @@ autograd::Edge edge_of(const at::Tensor* t) {
 }
 // An output nobody differentiated through has no gradient: zeros.
 at::Tensor grad_or_zeros(const at::Tensor& g, at::IntArrayRef shape, const at::Tensor& like) {
-    return g.defined() ? g.contiguous() : at::zeros(shape, like.options());
+    return without_gil([&] { return g.defined() ? g.contiguous() : at::zeros(shape, like.options()); });
 }
 
 struct ConvNode : LayerNode {
@@ -712,10 +766,10 @@ struct BnNode : LayerNode {
             if (join) shape.back() *= 2;
             const at::Tensor dy = grad_or_zeros(grads[0], shape, in);
             at::Tensor dwide;
-            if (grads.size() > 1 && grads[1].defined()) dwide = grads[1].contiguous();
+            if (grads.size() > 1 && grads[1].defined()) dwide = without_gil([&] { return grads[1].contiguous(); });
             const OutputGrad g = output_grad(dy, dwide.defined() ? &dwide : nullptr, join, in);
             autograd::variable_list out(4);
-            if (residual) out[1] = at::empty(in.sizes(), in.options());
+            if (residual) out[1] = new_empty(in.sizes(), in.options());
             owner->weight_gradient(grad_a, grad_b, [&](const at::Tensor& dgamma, const at::Tensor& dbeta) {
                 out[0] = run_bn_backward(g, mask.defined() ? &mask : nullptr, in, gamma, beta, mean, rstd, act, slope, out[1], dgamma, dbeta,
                                          owner->workspace);
@@ -768,14 +822,16 @@ PyObject* py_l1_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         const at::Tensor &a = tensor(args[0], "a"), &b = tensor(args[1], "b");
         require(a.scalar_type() == at::kHalf && b.scalar_type() == at::kHalf && a.numel() == b.numel(), "two float16 tensors of one size");
-        const at::Tensor loss = at::empty({}, a.options().dtype(at::kFloat));
+        const at::Tensor loss = new_empty({}, a.options().dtype(at::kFloat));
         size_t need = 0;
         check(nml_l1_workspace_size(&need));
         const Scratch ws = scratch(args[3], need, a);
         const float denom = static_cast<float>(as_double(args[2]));
         void *const pa = ptr(a), *const pb = ptr(b);
         float* const pl = floats(loss);
-        check(nml_l1_forward(pa, pb, a.numel(), denom, pl, ws.p, ws.bytes, stream()));
+        issue([&](void* st) {
+            return nml_l1_forward(pa, pb, a.numel(), denom, pl, ws.p, ws.bytes, st);
+        });
         return THPVariable_Wrap(loss);
     });
 }
@@ -786,11 +842,13 @@ PyObject* py_l1_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         const at::Tensor &a = tensor(args[0], "a"), &b = tensor(args[1], "b"), &dloss = tensor(args[2], "dloss");
         require(dloss.scalar_type() == at::kFloat && dloss.numel() == 1, "the gradient of the loss is one float32");
-        const at::Tensor da = at::empty(a.sizes(), a.options());
+        const at::Tensor da = new_empty(a.sizes(), a.options());
         const float denom = static_cast<float>(as_double(args[3]));
         void *const pa = ptr(a), *const pb = ptr(b), *const pda = ptr(da);
         float* const pl = floats(dloss);
-        check(nml_l1_backward(pa, pb, a.numel(), pl, denom, pda, stream()));
+        issue([&](void* st) {
+            return nml_l1_backward(pa, pb, a.numel(), pl, denom, pda, st);
+        });
         return THPVariable_Wrap(da);
     });
 }

@@ -1,5 +1,8 @@
 """Inputs at the far ends of what the entry points accept: very long sums, scratch limits, values and pointers that a fast path
 has to hand on."""
+import threading
+import time
+
 import pytest
 import torch
 
@@ -105,3 +108,57 @@ def test_out_of_memory_has_torchs_type():
     with pytest.raises(torch.OutOfMemoryError):
         ops.linear_forward(x, torch.zeros(1 << 20, 8, device="cuda"))
     ops.device_status()
+
+
+def test_other_threads_run_while_a_call_waits_for_the_queue():
+    """The GPU is kept busy for about half a second while more launches are issued than its queue holds: the call that waits
+    for room must not keep Python's lock, so another thread's clock has no gap of that length."""
+    x, w, out = torch.zeros(8, 64, device="cuda").half(), torch.zeros(64, 64, device="cuda").half(), torch.empty(8, 64, device="cuda").half()
+    ops.linear_forward(x, w, out=out)
+    torch.cuda.synchronize()
+    gaps, stop = [0.0], threading.Event()
+
+    def clock():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps[0] = max(gaps[0], now - last)
+            last = now
+
+    t = threading.Thread(target=clock)
+    t.start()
+    torch.cuda._sleep(1_000_000_000)
+    begin = time.perf_counter()
+    for _ in range(4000):
+        ops.linear_forward(x, w, out=out)
+    waited = time.perf_counter() - begin
+    stop.set()
+    t.join()
+    ops.device_status()
+    assert waited > 0.2, "the queue never filled"
+    assert gaps[0] < 0.5 * waited, (gaps[0], waited)
+
+
+def test_passes_of_two_threads_on_one_stream_do_not_mix():
+    """Both share the default workspace: a pass's kernels are issued together, so each gets its own result, to the bit."""
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    data = []
+    for rows in (96, 352):
+        x, dy = (torch.randn(rows, f, device="cuda", generator=gen) for f in (160, 72))
+        data.append((x, dy, ops.linear_backward_weight(x, dy, math="3xtf32")))
+    wrong = []
+
+    def work(x, dy, want):
+        for _ in range(400):
+            dw, db = ops.linear_backward_weight(x, dy, math="3xtf32")
+            if not (torch.equal(dw, want[0]) and torch.equal(db, want[1])):
+                wrong.append(x.shape)
+
+    threads = [threading.Thread(target=work, args=d) for d in data for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    ops.device_status()
+    assert not wrong, wrong

@@ -695,6 +695,14 @@ std::shared_ptr<N> make_node(PyObject* layer, PyObject* flags, PyObject* workspa
 autograd::Edge edge_of(const at::Tensor* t) {
     return t && t->defined() && t->requires_grad() ? autograd::impl::gradient_edge(*t) : autograd::Edge();
 }
+// The layers have no forward-mode derivative: a tangent would be dropped in silence.
+void require_no_tangent(std::initializer_list<const at::Tensor*> inputs) {
+    for (const at::Tensor* t : inputs)
+        if (t && t->defined() && t->_fw_grad(0).defined()) {
+            PyErr_SetString(PyExc_NotImplementedError, "this layer has no forward-mode derivative");
+            throw Fail();
+        }
+}
 // An output nobody differentiated through has no gradient: zeros.
 at::Tensor grad_or_zeros(const at::Tensor& g, at::IntArrayRef shape, const at::Tensor& like) {
     return without_gil([&] { return g.defined() ? g.contiguous() : at::zeros(shape, like.options()); });
@@ -732,6 +740,7 @@ PyObject* py_conv_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor* db = tensor_or_none(a[6], "db");
         const bool needs_dx = as_int(a[7]) != 0;
         require_flags(a[9]);
+        require_no_tangent({&x, &token});
         at::Tensor y = run_conv_forward(g, x, w, tensor_or_none(a[4], "bias"), Py_None, NML_NHWC, NML_NHWC, NML_MATH_F16, -1, 0, a[10]);
         if (at::GradMode::is_enabled() && (x.requires_grad() || token.requires_grad())) {
             auto node = make_node<ConvNode>(a[8], a[9], a[10]);
@@ -791,6 +800,7 @@ PyObject* py_bn_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const float slope = static_cast<float>(as_double(a[9]));
         const bool skip = as_int(a[11]) != 0;
         require_flags(a[13]);
+        require_no_tangent({&x, res, &token, join});
         BnSaved r = run_bn_forward(x, res, gamma, beta, act, slope, static_cast<float>(as_double(a[10])), join, skip, a[14]);
         const bool differentiable = x.requires_grad() || token.requires_grad() || (res && res->requires_grad()) || (join && join->requires_grad());
         if (at::GradMode::is_enabled() && differentiable) {

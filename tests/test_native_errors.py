@@ -3,7 +3,7 @@ gives them, and never end the process."""
 import pytest
 import torch
 
-from nectarml_b200 import ops
+from nectarml_b200 import ops, train
 
 
 @pytest.fixture(autouse=True)
@@ -42,3 +42,19 @@ def test_unsupported_tensors():
 def _error():
     from nectarml_b200 import _lib
     return _lib.NectarB200Error
+
+
+def test_layers_refuse_forward_mode():
+    """A layer without a forward-mode derivative says so, as an autograd function without one does; it must not return a value
+    whose tangent is missing."""
+    import torch.autograd.forward_ad as fwd
+    store = train.ParamStore("cpu")
+    conv, bn = train.Conv(store, 8, 8, 3, 1, 1), train.BatchNormAct(store, 8)
+    store.finalize(1)
+    x, token = torch.zeros(1, 4, 4, 8, dtype=torch.float16), torch.zeros((), requires_grad=True)
+    with fwd.dual_level():
+        dual = fwd.make_dual(x, torch.ones_like(x))
+        for call in (lambda: conv(dual, token), lambda: bn(dual, token), lambda: bn(x, token, residual=dual),
+                     lambda: bn(x, token, join=dual)):
+            with pytest.raises(NotImplementedError):
+                call()

@@ -758,19 +758,25 @@ PyObject* py_conv_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 struct BnNode : LayerNode {
-    at::Tensor gamma, beta, mean, rstd, mask;
+    at::Tensor gamma, beta;
+    autograd::SavedVariable mean, rstd, mask;  // (saved like x, so that hooks on saved tensors see all a layer keeps)
+    bool masked = false;
     int act = 0;
     float slope = 0.f;
     bool residual = false, join = false;
 
     void release_variables() override {
         LayerNode::release_variables();
-        mean = rstd = mask = at::Tensor();
+        mean.reset_data();
+        rstd.reset_data();
+        mask.reset_data();
     }
     std::string name() const override { return "BatchNormBackward"; }
     autograd::variable_list apply(autograd::variable_list&& grads) override {
         return guarded_backward([&]() -> autograd::variable_list {
-            const at::Tensor in = x.unpack();
+            const at::Tensor in = x.unpack(), mu = mean.unpack(), rs = rstd.unpack();
+            at::Tensor positive;
+            if (masked) positive = mask.unpack();
             auto shape = in.sizes().vec();
             if (join) shape.back() *= 2;
             const at::Tensor dy = grad_or_zeros(grads[0], shape, in);
@@ -780,7 +786,7 @@ struct BnNode : LayerNode {
             autograd::variable_list out(4);
             if (residual) out[1] = new_empty(in.sizes(), in.options());
             owner->weight_gradient(grad_a, grad_b, [&](const at::Tensor& dgamma, const at::Tensor& dbeta) {
-                out[0] = run_bn_backward(g, mask.defined() ? &mask : nullptr, in, gamma, beta, mean, rstd, act, slope, out[1], dgamma, dbeta,
+                out[0] = run_bn_backward(g, masked ? &positive : nullptr, in, gamma, beta, mu, rs, act, slope, out[1], dgamma, dbeta,
                                          owner->workspace);
             });
             if (join) out[3] = dy;
@@ -807,9 +813,10 @@ PyObject* py_bn_layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
             auto node = make_node<BnNode>(a[12], a[13], a[14]);
             node->gamma = gamma;
             node->beta = beta;
-            node->mean = r.mean;
-            node->rstd = r.rstd;
-            node->mask = r.mask;
+            node->mean = autograd::SavedVariable(r.mean, false);
+            node->rstd = autograd::SavedVariable(r.rstd, false);
+            node->masked = r.mask.defined();
+            if (node->masked) node->mask = autograd::SavedVariable(r.mask, false);
             node->act = act;
             node->slope = slope;
             node->residual = res != nullptr;

@@ -1,5 +1,6 @@
 """Inputs at the far ends of what the entry points accept: very long sums, scratch limits, values and pointers that a fast path
 has to hand on."""
+import contextlib
 import threading
 import time
 
@@ -162,3 +163,34 @@ def test_passes_of_two_threads_on_one_stream_do_not_mix():
         t.join()
     ops.device_status()
     assert not wrong, wrong
+
+
+def test_saved_tensor_hooks_see_what_the_layers_keep():
+    """Everything a layer saves for its backward passes through the hooks on saved tensors (which move it to the host here),
+    and the gradients are the same bits; a second backward through freed tensors is refused."""
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    store = train.ParamStore("cuda")
+    conv, bn = train.Conv(store, 8, 16, 3, 1, 1), train.BatchNormAct(store, 16)
+    store.finalize(1)
+    store.p32.copy_(torch.randn(store.n, device="cuda", generator=gen))
+    store.sync_half()
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen).half()  # noqa: E731
+    x, res, dy, token = rnd(2, 6, 6, 8), rnd(2, 6, 6, 16), rnd(2, 6, 6, 16), torch.zeros((), device="cuda", requires_grad=True)
+    results, packed = [], []
+
+    def pack(t):
+        packed.append(tuple(t.shape))
+        return t.cpu()
+
+    for hooked in (False, True):
+        leaf = x.clone().requires_grad_()
+        store.begin_backward(False)
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()) if hooked else contextlib.nullcontext():
+            y = bn(conv(leaf, token), token, train.ACT_RELU, residual=res)
+        y.backward(dy)
+        results.append((leaf.grad, store.grad.clone()))
+        with pytest.raises(RuntimeError, match="second time"):
+            y.backward(dy)
+    ops.device_status()
+    assert sorted(packed) == sorted([(2, 6, 6, 8), (2, 6, 6, 16), (16,), (16,), (2 * 6 * 6 * 16 // 8,)])
+    assert all(torch.equal(a, b) for a, b in zip(*results))

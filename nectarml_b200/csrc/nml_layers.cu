@@ -29,6 +29,8 @@ namespace nml_layers {
 
 using nml::launch;
 using nml::launch_with;
+using nml::load_global;
+using nml::load_streaming;
 using nml::pdl_enter;
 
 static inline size_t round_up(size_t v, size_t m) { return (v + m - 1) / m * m; }
@@ -72,17 +74,17 @@ __device__ __forceinline__ bool positive_as_half(float t) { return t > 2.9802322
 // The eight values of a vector's channels from a per-channel array, in two loads.  A thread owns its channels for good, so a
 // block pays for its constants once, but with one 4-byte load per value (32 bytes apart in a warp) that was eight times
 // the L1 wavefronts and cost a block as much as several rows of the tensor.  Callers' arrays may start anywhere.
-__device__ __forceinline__ void load8(const float* __restrict__ p, int col, float (&f)[8]) {
+__device__ __forceinline__ void load8(const float* p, int col, float (&f)[8]) {
     p += col * 8;
     if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+        const float4 a = load_global(reinterpret_cast<const float4*>(p)), b = load_global(reinterpret_cast<const float4*>(p) + 1);
         f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
     } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = __ldg(p + j);
+        for (int j = 0; j < 8; ++j) f[j] = load_global(p + j);
     }
 }
-__device__ __forceinline__ void load8_or(const float* __restrict__ p, int col, float otherwise, float (&f)[8]) {
+__device__ __forceinline__ void load8_or(const float* p, int col, float otherwise, float (&f)[8]) {
     if (p) {
         load8(p, col, f);
     } else {
@@ -92,8 +94,8 @@ __device__ __forceinline__ void load8_or(const float* __restrict__ p, int col, f
 }
 
 // Per-channel constants of the forward's y = act(sc * x + sh), as the forward computes them.
-__device__ __forceinline__ void bn_affine(int col, const float* __restrict__ gamma, const float* __restrict__ beta,
-                                          const float* __restrict__ mean, const float* __restrict__ rstd, float (&sc)[8], float (&sh)[8]) {
+__device__ __forceinline__ void bn_affine(int col, const float* gamma, const float* beta,
+                                          const float* mean, const float* rstd, float (&sc)[8], float (&sh)[8]) {
     float r[8], m[8];
     load8_or(gamma, col, 1.f, sc);
     load8_or(beta, col, 0.f, sh);
@@ -137,8 +139,8 @@ struct OutGradVector {
 template <bool kTwo>
 __device__ __forceinline__ OutGradVector load_grad(const OutGrad& g, size_t row, int col) {
     OutGradVector v;
-    v.a = __ldg(g.a + row * g.row + col);
-    if (kTwo) v.b = __ldg(g.b + row * g.row2 + col);
+    v.a = load_global(g.a + row * g.row + col);
+    if (kTwo) v.b = load_global(g.b + row * g.row2 + col);
     return v;
 }
 template <bool kTwo>
@@ -185,7 +187,7 @@ __device__ __forceinline__ void bn_store_partial(float (*sm)[17], const float (&
 }
 
 // Forward statistics: a = sum x, b = sum x^2; four rows in flight per thread.
-__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* __restrict__ x, float* __restrict__ partial, size_t M, int C) {
+__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __restrict__ partial, size_t M, int C) {
     pdl_enter();
     __shared__ float sm[256][17];
     const int cpr = C >> 3;
@@ -206,14 +208,14 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* __restrict__
     const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
     size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
     for (; row + 3 * stride < M; row += 4 * stride) {
-        const uint4 x0 = __ldg(x + row * cpr + col), x1 = __ldg(x + (row + stride) * cpr + col);
-        const uint4 x2 = __ldg(x + (row + 2 * stride) * cpr + col), x3 = __ldg(x + (row + 3 * stride) * cpr + col);
+        const uint4 x0 = load_global(x + row * cpr + col), x1 = load_global(x + (row + stride) * cpr + col);
+        const uint4 x2 = load_global(x + (row + 2 * stride) * cpr + col), x3 = load_global(x + (row + 3 * stride) * cpr + col);
         add(x0);
         add(x1);
         add(x2);
         add(x3);
     }
-    for (; row < M; row += stride) add(__ldg(x + row * cpr + col));
+    for (; row < M; row += stride) add(load_global(x + row * cpr + col));
     bn_store_partial(sm, a, b, cpr, rpb, C, partial);
 }
 
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* __restrict__
 // d gamma = rstd * (b - mean * a), so this pass needs no per-channel constants but those of D_X).  Two rows in flight per
 // thread.
 template <int kDeriv, bool kTwo>
-__global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restrict__ x, const OutGrad dy, const BnForward f,
+__global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* x, const OutGrad dy, const BnForward f,
                                                            float* __restrict__ partial, size_t M, int C) {
     pdl_enter();
     __shared__ float sm[256][17];
@@ -248,16 +250,16 @@ __global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restri
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     for (; row + stride < M; row += 2 * stride) {
         const size_t v0 = row * cpr + col, v1 = (row + stride) * cpr + col;
-        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
+        const uint4 x0 = load_global(x + v0), x1 = load_global(x + v1);
         const OutGradVector d0 = load_grad<kTwo>(dy, row, col), d1 = load_grad<kTwo>(dy, row + stride, col);
-        const uint4 y0 = kDeriv == D_Y ? __ldg(f.y + v0) : zero, y1 = kDeriv == D_Y ? __ldg(f.y + v1) : zero;
-        const unsigned m0 = kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? __ldg(f.mask + v1) : 0u;
+        const uint4 y0 = kDeriv == D_Y ? load_global(f.y + v0) : zero, y1 = kDeriv == D_Y ? load_global(f.y + v1) : zero;
+        const unsigned m0 = kDeriv == D_MASK ? load_global(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? load_global(f.mask + v1) : 0u;
         add(x0, d0, y0, m0);
         add(x1, d1, y1, m1);
     }
     if (row < M) {
         const size_t v0 = row * cpr + col;
-        add(__ldg(x + v0), load_grad<kTwo>(dy, row, col), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
+        add(load_global(x + v0), load_grad<kTwo>(dy, row, col), kDeriv == D_Y ? load_global(f.y + v0) : zero, kDeriv == D_MASK ? load_global(f.mask + v0) : 0u);
     }
     bn_store_partial(sm, a, b, cpr, rpb, C, partial);
 }
@@ -267,8 +269,8 @@ __global__ void __launch_bounds__(256) bn_grad_sums_kernel(const uint4* __restri
 // mode 1: out0 = sum a (d beta), out1 = rstd * (sum b - mean * sum a) (d gamma).  blockDim = (8, 128): the pass is a chain of
 // load latencies, so it is spread over many blocks and a thread's few loads are all in flight (32 channels a block and
 // 19 rows a thread took 6 us; a U-Net step runs it 26 times).
-__global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict__ partial, int P, int C, int mode, double inv_M,
-                                                        float eps, const float* __restrict__ mean, const float* __restrict__ rstd,
+__global__ void __launch_bounds__(1024) bn_finish_kernel(const float* partial, int P, int C, int mode, double inv_M,
+                                                        float eps, const float* mean, const float* rstd,
                                                         float* __restrict__ out0, float* __restrict__ out1) {
     pdl_enter();
     __shared__ double pa[128][9], pb[128][9];
@@ -276,8 +278,8 @@ __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict
     double sa = 0.0, sb = 0.0;
 #pragma unroll 5
     for (int p = threadIdx.y; p < P; p += 128) {
-        sa += static_cast<double>(__ldg(partial + static_cast<size_t>(p) * 2 * C + c));
-        sb += static_cast<double>(__ldg(partial + static_cast<size_t>(p) * 2 * C + C + c));
+        sa += static_cast<double>(load_global(partial + static_cast<size_t>(p) * 2 * C + c));
+        sb += static_cast<double>(load_global(partial + static_cast<size_t>(p) * 2 * C + C + c));
     }
     pa[threadIdx.y][threadIdx.x] = sa;
     pb[threadIdx.y][threadIdx.x] = sb;
@@ -298,7 +300,7 @@ __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict
             out1[c] = static_cast<float>(1.0 / sqrt(var + static_cast<double>(eps)));
         } else {
             out0[c] = static_cast<float>(ta);
-            out1[c] = static_cast<float>(static_cast<double>(rstd[c]) * (tb - static_cast<double>(mean[c]) * ta));
+            out1[c] = static_cast<float>(static_cast<double>(load_global(rstd + c)) * (tb - static_cast<double>(load_global(mean + c)) * ta));
         }
     }
 }
@@ -307,11 +309,11 @@ __global__ void __launch_bounds__(1024) bn_finish_kernel(const float* __restrict
 // one bit per element, set where y > 0, for D_MASK.  The rows are walked from the last to the first: the statistics pass
 // has just read x in the other direction, so what of it is still in L2 (126 MB) is read first.
 // y (and y2, a second copy) may be part of the channels of a wider tensor: their rows are y_row and y2_row vectors apart.
-__global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res,
+__global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* x, const uint4* res,
                                                        uint4* __restrict__ y, int y_row, uint4* __restrict__ y2, int y2_row,
-                                                       uint8_t* __restrict__ mask, const float* __restrict__ gamma,
-                                                       const float* __restrict__ beta, const float* __restrict__ mean,
-                                                       const float* __restrict__ rstd, int act, float slope, size_t M, int C) {
+                                                       uint8_t* __restrict__ mask, const float* gamma,
+                                                       const float* beta, const float* mean,
+                                                       const float* rstd, int act, float slope, size_t M, int C) {
     pdl_enter();
     const int cpr = C >> 3;
     const int rpb = blockDim.x / cpr;
@@ -341,14 +343,14 @@ __global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restric
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     for (; k + stride < M; k += 2 * stride) {
         const size_t v0 = (M - 1 - k) * cpr + col, v1 = (M - 1 - k - stride) * cpr + col;
-        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
-        const uint4 r0 = res ? __ldg(res + v0) : zero, r1 = res ? __ldg(res + v1) : zero;
+        const uint4 x0 = load_global(x + v0), x1 = load_global(x + v1);
+        const uint4 r0 = res ? load_global(res + v0) : zero, r1 = res ? load_global(res + v1) : zero;
         one(M - 1 - k, x0, r0);
         one(M - 1 - k - stride, x1, r1);
     }
     if (k < M) {
         const size_t v0 = (M - 1 - k) * cpr + col;
-        one(M - 1 - k, __ldg(x + v0), res ? __ldg(res + v0) : zero);
+        one(M - 1 - k, load_global(x + v0), res ? load_global(res + v0) : zero);
     }
 }
 
@@ -356,9 +358,9 @@ __global__ void __launch_bounds__(256, 4) bn_apply_kernel(const uint4* __restric
 // dx = A * dz + B * x + C per channel; optionally dres = dz (the gradient of the residual input that was
 // added before the activation).  Two rows in flight per thread, from the last row to the first as in bn_apply_kernel.
 template <int kDeriv, bool kTwo>
-__global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__ x, const OutGrad dy, const BnForward f,
-                                                    uint4* __restrict__ dx, uint4* __restrict__ dres, const float* __restrict__ dbeta,
-                                                    const float* __restrict__ dgamma, float inv_M, size_t M, int C) {
+__global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* x, const OutGrad dy, const BnForward f,
+                                                    uint4* __restrict__ dx, uint4* __restrict__ dres, const float* dbeta,
+                                                    const float* dgamma, float inv_M, size_t M, int C) {
     pdl_enter();
     const int cpr = C >> 3;
     const int rpb = blockDim.x / cpr;
@@ -395,16 +397,16 @@ __global__ void __launch_bounds__(256, 3) bn_dx_kernel(const uint4* __restrict__
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     for (; k + stride < M; k += 2 * stride) {
         const size_t v0 = (M - 1 - k) * cpr + col, v1 = (M - 1 - k - stride) * cpr + col;
-        const uint4 x0 = __ldg(x + v0), x1 = __ldg(x + v1);
+        const uint4 x0 = load_global(x + v0), x1 = load_global(x + v1);
         const OutGradVector d0 = load_grad<kTwo>(dy, M - 1 - k, col), d1 = load_grad<kTwo>(dy, M - 1 - k - stride, col);
-        const uint4 y0 = kDeriv == D_Y ? __ldg(f.y + v0) : zero, y1 = kDeriv == D_Y ? __ldg(f.y + v1) : zero;
-        const unsigned m0 = kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? __ldg(f.mask + v1) : 0u;
+        const uint4 y0 = kDeriv == D_Y ? load_global(f.y + v0) : zero, y1 = kDeriv == D_Y ? load_global(f.y + v1) : zero;
+        const unsigned m0 = kDeriv == D_MASK ? load_global(f.mask + v0) : 0u, m1 = kDeriv == D_MASK ? load_global(f.mask + v1) : 0u;
         one(v0, x0, d0, y0, m0);
         one(v1, x1, d1, y1, m1);
     }
     if (k < M) {
         const size_t v0 = (M - 1 - k) * cpr + col;
-        one(v0, __ldg(x + v0), load_grad<kTwo>(dy, M - 1 - k, col), kDeriv == D_Y ? __ldg(f.y + v0) : zero, kDeriv == D_MASK ? __ldg(f.mask + v0) : 0u);
+        one(v0, load_global(x + v0), load_grad<kTwo>(dy, M - 1 - k, col), kDeriv == D_Y ? load_global(f.y + v0) : zero, kDeriv == D_MASK ? load_global(f.mask + v0) : 0u);
     }
 }
 
@@ -476,8 +478,8 @@ __device__ __forceinline__ ClusterShare cluster_share(size_t M, int gv) {
 }
 
 __global__ void __launch_bounds__(kClusterThreads) bn_cluster_forward_kernel(
-    const uint4* __restrict__ x, const uint4* __restrict__ res, uint4* __restrict__ y, int y_row, uint4* __restrict__ y2, int y2_row,
-    uint8_t* __restrict__ mask, const float* __restrict__ gamma, const float* __restrict__ beta, float* __restrict__ mean,
+    const uint4* x, const uint4* res, uint4* __restrict__ y, int y_row, uint4* __restrict__ y2, int y2_row,
+    uint8_t* __restrict__ mask, const float* gamma, const float* beta, float* __restrict__ mean,
     float* __restrict__ rstd, int act, float slope, float eps, double inv_M, size_t M, int C, int gv) {
     pdl_enter();
     extern __shared__ uint4 keep[];
@@ -494,7 +496,7 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_forward_kernel(
     for (size_t row = s.first + s.lane; row < s.last; row += kFlight * s.lanes, k += kFlight * kClusterThreads) {
         uint4 v[kFlight];
 #pragma unroll
-        for (int i = 0; i < kFlight; ++i) v[i] = row + i * s.lanes < s.last ? __ldg(x + (row + i * s.lanes) * cpr + s.col) : zero;
+        for (int i = 0; i < kFlight; ++i) v[i] = row + i * s.lanes < s.last ? load_global(x + (row + i * s.lanes) * cpr + s.col) : zero;
 #pragma unroll
         for (int i = 0; i < kFlight; ++i) {
             float f[8];
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_forward_kernel(
     for (size_t row = s.first + s.lane; row < s.last; row += s.lanes, k += kClusterThreads) {
         float f[8], rf[8];
         unpack8(keep[k], f);
-        if (res) unpack8(__ldg(res + row * cpr + s.col), rf);
+        if (res) unpack8(load_global(res + row * cpr + s.col), rf);
         unsigned bits = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -553,7 +555,7 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_forward_kernel(
 
 template <int kDeriv, bool kTwo>
 __global__ void __launch_bounds__(kClusterThreads) bn_cluster_backward_kernel(
-    const uint4* __restrict__ x, const OutGrad dy, const BnForward f, uint4* __restrict__ dx, uint4* __restrict__ dres,
+    const uint4* x, const OutGrad dy, const BnForward f, uint4* __restrict__ dx, uint4* __restrict__ dres,
     float* __restrict__ dbeta, float* __restrict__ dgamma, double inv_M, size_t M, int C, int gv) {
     pdl_enter();
     extern __shared__ uint4 keep[];  // [x, dy (, second dy)][share]
@@ -578,11 +580,11 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_backward_kernel(
         for (int i = 0; i < kFlight; ++i) {
             const size_t r = row + i * s.lanes, v = r * cpr + s.col;
             const bool in = r < s.last;
-            xv[i] = in ? __ldg(x + v) : zero;
+            xv[i] = in ? load_global(x + v) : zero;
             dv[i].a = dv[i].b = zero;
             if (in) dv[i] = load_grad<kTwo>(dy, r, s.col);
-            yv[i] = kDeriv == D_Y && in ? __ldg(f.y + v) : zero;
-            bits[i] = kDeriv == D_MASK && in ? __ldg(f.mask + v) : 0u;
+            yv[i] = kDeriv == D_Y && in ? load_global(f.y + v) : zero;
+            bits[i] = kDeriv == D_MASK && in ? load_global(f.mask + v) : 0u;
         }
 #pragma unroll
         for (int i = 0; i < kFlight; ++i) {
@@ -605,7 +607,7 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_backward_kernel(
     const int c0 = blockIdx.x / kClusterBlocks * gv * 8;
     cluster_sums(a, b, gv, part, [&](int c, double ta, double tb) {
         done[0][c] = static_cast<float>(ta);
-        done[1][c] = static_cast<float>(static_cast<double>(f.rstd[c0 + c]) * (tb - static_cast<double>(f.mean[c0 + c]) * ta));
+        done[1][c] = static_cast<float>(static_cast<double>(load_global(f.rstd + c0 + c)) * (tb - static_cast<double>(load_global(f.mean + c0 + c)) * ta));
         if (blockIdx.x % kClusterBlocks == 0) {
             dbeta[c0 + c] = done[0][c];
             dgamma[c0 + c] = done[1][c];
@@ -633,8 +635,8 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_backward_kernel(
         OutGradVector dv;
         dv.a = keep[vectors + k];
         if (kTwo) dv.b = keep[2 * vectors + k];
-        const uint4 yv = kDeriv == D_Y ? __ldg(f.y + v) : zero;
-        const unsigned bits = kDeriv == D_MASK ? __ldg(f.mask + v) : 0u;
+        const uint4 yv = kDeriv == D_Y ? load_global(f.y + v) : zero;
+        const unsigned bits = kDeriv == D_MASK ? load_global(f.mask + v) : 0u;
         float xf[8], df[8];
         unpack8(keep[k], xf);
         unpack_grad<kTwo>(dv, df);
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(kClusterThreads) bn_cluster_backward_kernel(
 
 // An activation that no normalisation stands in front of: y = act(x), with a second copy as part of the channels of a wider
 // tensor.  rows x C, thread layout and grid as above.
-__global__ void __launch_bounds__(256, 4) act_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, uint4* __restrict__ y2,
+__global__ void __launch_bounds__(256, 4) act_kernel(const uint4* x, uint4* __restrict__ y, uint4* __restrict__ y2,
                                                      int y2_row, float below, size_t M, int C) {
     pdl_enter();
     const int cpr = C >> 3;
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(256, 4) act_kernel(const uint4* __restrict__ x
 #pragma unroll 2
     for (size_t row = static_cast<size_t>(blockIdx.x) * rpb + threadIdx.x / cpr; row < M; row += stride) {
         float f[8];
-        unpack8(__ldg(x + row * cpr + col), f);
+        unpack8(load_global(x + row * cpr + col), f);
 #pragma unroll
         for (int j = 0; j < 8; ++j)  // NaN stays NaN, -0 becomes 0; below = 0 is a choice, not a product: of -inf too
             f[j] = f[j] > 0.f ? f[j] : below != 0.f ? f[j] * below + 0.f : f[j] <= 0.f ? 0.f : f[j];
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(256, 4) act_kernel(const uint4* __restrict__ x
 }
 // dx = dy * act'(x).
 template <bool kTwo>
-__global__ void __launch_bounds__(256, 4) act_backward_kernel(const uint4* __restrict__ x, const OutGrad dy, uint4* __restrict__ dx,
+__global__ void __launch_bounds__(256, 4) act_backward_kernel(const uint4* x, const OutGrad dy, uint4* __restrict__ dx,
                                                               float below, size_t M, int C) {
     pdl_enter();
     const int cpr = C >> 3;
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(256, 4) act_backward_kernel(const uint4* __res
     for (size_t row = static_cast<size_t>(blockIdx.x) * rpb + threadIdx.x / cpr; row < M; row += stride) {
         float f[8], d[8];
         const OutGradVector g = load_grad<kTwo>(dy, row, col);
-        unpack8(__ldg(x + row * cpr + col), f);
+        unpack8(load_global(x + row * cpr + col), f);
         unpack_grad<kTwo>(g, d);
 #pragma unroll
         for (int j = 0; j < 8; ++j)  // (an overflowed gradient does not pass where the ReLU is shut; NaN inputs let it pass)
@@ -693,17 +695,17 @@ __global__ void __launch_bounds__(256, 4) act_backward_kernel(const uint4* __res
 // L1 loss sum |a - b| / denom of two fp16 tensors, in fp32 within a thread's share and in double over the blocks, fixed order.
 // As separate passes (two conversions, difference, absolute value, sum; sign, product and conversion back) the loss of 16
 // images of 256 x 256 took 60 us of small kernels each way and twice as long to issue.
-__global__ void __launch_bounds__(256) l1_sum_kernel(const __half2* __restrict__ a, const __half2* __restrict__ b, size_t n, float* __restrict__ partial) {
+__global__ void __launch_bounds__(256) l1_sum_kernel(const __half2* a, const __half2* b, size_t n, float* __restrict__ partial) {
     pdl_enter();
     float s = 0.f;
     const size_t n2 = n / 2, step = static_cast<size_t>(gridDim.x) * blockDim.x;
 #pragma unroll 4
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n2; i += step) {
-        const float2 u = __half22float2(a[i]), v = __half22float2(b[i]);
+        const float2 u = __half22float2(load_global(a + i)), v = __half22float2(load_global(b + i));
         s += fabsf(u.x - v.x) + fabsf(u.y - v.y);
     }
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0)
-        s += fabsf(__half2float(reinterpret_cast<const __half*>(a)[n - 1]) - __half2float(reinterpret_cast<const __half*>(b)[n - 1]));
+        s += fabsf(__half2float(load_global(reinterpret_cast<const __half*>(a) + n - 1)) - __half2float(load_global(reinterpret_cast<const __half*>(b) + n - 1)));
     __shared__ float sm[8];
 #pragma unroll
     for (int o = 16; o > 0; o /= 2) s += __shfl_down_sync(0xffffffffu, s, o);
@@ -715,34 +717,34 @@ __global__ void __launch_bounds__(256) l1_sum_kernel(const __half2* __restrict__
         partial[blockIdx.x] = s;
     }
 }
-__global__ void __launch_bounds__(32) l1_finish_kernel(const float* __restrict__ partial, int P, float denom, float* __restrict__ loss) {
+__global__ void __launch_bounds__(32) l1_finish_kernel(const float* partial, int P, float denom, float* __restrict__ loss) {
     pdl_enter();
     double s = 0.0;
-    for (int p = threadIdx.x; p < P; p += 32) s += static_cast<double>(partial[p]);
+    for (int p = threadIdx.x; p < P; p += 32) s += static_cast<double>(load_global(partial + p));
 #pragma unroll
     for (int o = 16; o > 0; o /= 2) s += __shfl_down_sync(0xffffffffu, s, o);
     if (threadIdx.x == 0) *loss = static_cast<float>(s) / denom;
 }
 // da = sign(a - b) * (*dloss / denom)
-__global__ void __launch_bounds__(256) l1_backward_kernel(const __half2* __restrict__ a, const __half2* __restrict__ b, size_t n,
-                                                          const float* __restrict__ dloss, float denom, __half2* __restrict__ da) {
+__global__ void __launch_bounds__(256) l1_backward_kernel(const __half2* a, const __half2* b, size_t n,
+                                                          const float* dloss, float denom, __half2* __restrict__ da) {
     pdl_enter();
-    const float g = __ldg(dloss) / denom;
+    const float g = load_global(dloss) / denom;
     auto one = [&](float d) { return d > 0.f ? g : d < 0.f ? -g : 0.f; };
     const size_t n2 = n / 2, step = static_cast<size_t>(gridDim.x) * blockDim.x;
 #pragma unroll 4
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n2; i += step) {
-        const float2 u = __half22float2(__ldg(a + i)), v = __half22float2(__ldg(b + i));
+        const float2 u = __half22float2(load_global(a + i)), v = __half22float2(load_global(b + i));
         da[i] = __floats2half2_rn(one(u.x - v.x), one(u.y - v.y));
     }
     if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0)
         reinterpret_cast<__half*>(da)[n - 1] = __float2half_rn(
-            one(__half2float(reinterpret_cast<const __half*>(a)[n - 1]) - __half2float(reinterpret_cast<const __half*>(b)[n - 1])));
+            one(__half2float(load_global(reinterpret_cast<const __half*>(a) + n - 1)) - __half2float(load_global(reinterpret_cast<const __half*>(b) + n - 1))));
 }
 
 // any(!isfinite(g * inv_scale)) over a flat fp32 buffer -> *found (set, never cleared, here).  Four loads in flight per
 // thread; 54 million values 46 -> 45 us.
-__global__ void __launch_bounds__(256) grads_check_kernel(const float4* __restrict__ g, size_t n4, float inv_scale, int* found) {
+__global__ void __launch_bounds__(256) grads_check_kernel(const float4* g, size_t n4, float inv_scale, int* found) {
     pdl_enter();
     bool bad = false;
     auto one = [&](const float4& v) {
@@ -751,13 +753,13 @@ __global__ void __launch_bounds__(256) grads_check_kernel(const float4* __restri
     const size_t step = static_cast<size_t>(gridDim.x) * blockDim.x;
     size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     for (; i + 3 * step < n4; i += 4 * step) {
-        const float4 v0 = __ldg(g + i), v1 = __ldg(g + i + step), v2 = __ldg(g + i + 2 * step), v3 = __ldg(g + i + 3 * step);
+        const float4 v0 = load_global(g + i), v1 = load_global(g + i + step), v2 = load_global(g + i + 2 * step), v3 = load_global(g + i + 3 * step);
         one(v0);
         one(v1);
         one(v2);
         one(v3);
     }
-    for (; i < n4; i += step) one(__ldg(g + i));
+    for (; i < n4; i += step) one(load_global(g + i));
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *found = 1;  // every writer writes the same value
 }
 
@@ -767,11 +769,11 @@ __global__ void __launch_bounds__(256) grads_check_kernel(const float4* __restri
 // Bound by memory (22 bytes a value).  Walked from the end to the start: the finiteness check has just read the gradients in
 // the other direction, so those of the last parameters are in L2, and the fp16 copies of the first layers stay there for the next
 // forward; parameters and velocity are streamed past (evict first).  54 million values 190 -> 184 us.
-__global__ void __launch_bounds__(256) sgd_momentum_kernel(float4* __restrict__ p, const float4* __restrict__ g, float4* __restrict__ vel,
+__global__ void __launch_bounds__(256) sgd_momentum_kernel(float4* __restrict__ p, const float4* g, float4* __restrict__ vel,
                                                            uint2* __restrict__ p16, size_t n4, float lr, float momentum, float dampening,
-                                                           float wd, float inv_scale, const int* __restrict__ found_inf) {
+                                                           float wd, float inv_scale, const int* found_inf) {
     pdl_enter();
-    if (found_inf && *found_inf) return;
+    if (found_inf && load_global(found_inf)) return;
     auto one = [&](size_t i, float4 pv, float4 vv, const float4& gv) {
         float* pp = reinterpret_cast<float*>(&pv);
         float* vp = reinterpret_cast<float*>(&vv);
@@ -795,14 +797,14 @@ __global__ void __launch_bounds__(256) sgd_momentum_kernel(float4* __restrict__ 
     size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;  // counted from the end
     for (; k + step < n4; k += 2 * step) {
         const size_t i0 = n4 - 1 - k, i1 = i0 - step;
-        const float4 p0 = __ldcs(p + i0), p1 = __ldcs(p + i1), v0 = __ldcs(vel + i0), v1 = __ldcs(vel + i1);
-        const float4 g0 = __ldg(g + i0), g1 = __ldg(g + i1);
+        const float4 p0 = load_streaming(p + i0), p1 = load_streaming(p + i1), v0 = load_streaming(vel + i0), v1 = load_streaming(vel + i1);
+        const float4 g0 = load_global(g + i0), g1 = load_global(g + i1);
         one(i0, p0, v0, g0);
         one(i1, p1, v1, g1);
     }
     if (k < n4) {
         const size_t i = n4 - 1 - k;
-        one(i, __ldcs(p + i), __ldcs(vel + i), __ldg(g + i));
+        one(i, load_streaming(p + i), load_streaming(vel + i), load_global(g + i));
     }
 }
 
@@ -810,7 +812,7 @@ __global__ void __launch_bounds__(256) sgd_momentum_kernel(float4* __restrict__ 
 // the window won (kh * k + kw, one byte); backward is a GATHER over the <= ceil(k/s)^2 windows that cover an
 // input pixel -- no atomics, so it is bitwise repeatable, and every input gradient is written exactly once
 // (no zero-fill pass).  Out-of-image taps are skipped (i.e. padded with -inf).
-__global__ void __launch_bounds__(256) maxpool_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, uint2* __restrict__ idx,
+__global__ void __launch_bounds__(256) maxpool_fwd_kernel(const uint4* x, uint4* __restrict__ y, uint2* __restrict__ idx,
                                                           int N, int H, int W, int C, int k, int s, int p, int Ho, int Wo) {
     pdl_enter();
     const int cpr = C >> 3;
@@ -836,7 +838,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const uint4* __restric
                 const int iw = ow * s - p + kw;
                 if (iw < 0 || iw >= W) continue;
                 float f[8];
-                unpack8(__ldg(x + ((static_cast<size_t>(n) * H + ih) * W + iw) * cpr + cv), f);
+                unpack8(load_global(x + ((static_cast<size_t>(n) * H + ih) * W + iw) * cpr + cv), f);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     if (f[j] > best[j]) {
@@ -853,7 +855,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(const uint4* __restric
     }
 }
 
-__global__ void __launch_bounds__(256) maxpool_bwd_kernel(const uint4* __restrict__ dy, const uint2* __restrict__ idx, uint4* __restrict__ dx,
+__global__ void __launch_bounds__(256) maxpool_bwd_kernel(const uint4* dy, const uint2* idx, uint4* __restrict__ dx,
                                                           int N, int H, int W, int C, int k, int s, int p, int Ho, int Wo) {
     pdl_enter();
     const int cpr = C >> 3;
@@ -873,9 +875,9 @@ __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const uint4* __restric
             for (int ow = ow_hi; ow >= 0 && iw + p - ow * s < k; --ow) {
                 const int me = kh * k + (iw + p - ow * s);
                 const size_t o = ((static_cast<size_t>(n) * Ho + oh) * Wo + ow) * cpr + cv;
-                const uint2 w2 = __ldg(idx + o);
+                const uint2 w2 = load_global(idx + o);
                 float g[8];
-                unpack8(__ldg(dy + o), g);
+                unpack8(load_global(dy + o), g);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const unsigned who = ((j < 4 ? w2.x : w2.y) >> (8 * (j & 3))) & 0xffu;

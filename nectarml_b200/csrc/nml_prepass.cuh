@@ -17,8 +17,8 @@ __device__ __forceinline__ float to_tf32_rna(float x) {
     return __uint_as_float(r);
 }
 
-__device__ __forceinline__ float load_as_float(const float* p, size_t i) { return p[i]; }
-__device__ __forceinline__ float load_as_float(const __half* p, size_t i) { return __half2float(p[i]); }
+__device__ __forceinline__ float load_as_float(const float* p, size_t i) { return load_global(p + i); }
+__device__ __forceinline__ float load_as_float(const __half* p, size_t i) { return __half2float(load_global(p + i)); }
 
 // Output encodings of the conversion kernels.
 enum { ENC_F16 = 0, ENC_TF32_PAIR = 1, ENC_TF32_HI = 2 };
@@ -33,9 +33,9 @@ __device__ __forceinline__ void store_enc(int enc, void* out0, void* out1, size_
     }
 }
 
-__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load4(const float* p) { return load_global(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 load4(const __half* p) {
-    const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 v = load_global(reinterpret_cast<const uint2*>(p));
     const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
     return make_float4(a.x, a.y, b.x, b.y);
 }
@@ -53,7 +53,7 @@ __device__ __forceinline__ float4 load4(const __half* p) {
 // matrix of partial sums; colsum_finish_kernel adds the rows in a fixed order (no atomics, so the
 // bias gradient is bitwise repeatable).
 template <typename TIn>
-__global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* __restrict__ in, void* out0,
+__global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const TIn* in, void* out0,
                                                            void* out1, int enc, int C, int Cp, int HW, int tiles_p, int tiles_c,
                                                            int tiles, float* colsum, int role) {
     pdl_enter(role);
@@ -162,7 +162,7 @@ __device__ __forceinline__ void store4(__half* p, const float (&v)[4]) {
     *reinterpret_cast<uint2*>(p) = h;
 }
 template <typename T>
-__global__ void __launch_bounds__(256) nhwc_to_nchw_kernel(const T* __restrict__ in, T* __restrict__ out, int C, int HW, int tiles_p,
+__global__ void __launch_bounds__(256) nhwc_to_nchw_kernel(const T* in, T* __restrict__ out, int C, int HW, int tiles_p,
                                                            int tiles_c, int tiles, int role) {
     pdl_enter(role);
     __shared__ float tile[64][65];  // [pixel][channel]
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) nhwc_to_nchw_kernel(const T* __restrict__
 // Four outputs per thread: a 16-byte load where the rows allow it, one 8-byte (fp16) or one or two 16-byte stores.
 // An element per thread with a 64-bit division each ran at 1.8 TB/s on 2 MB; this is bound by the launch there.
 template <typename TIn>
-__global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict__ in, void* out0,
+__global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* in, void* out0,
                                                            void* out1, int enc, size_t R, int C, int Cp, int role) {
     pdl_enter(role);
     const size_t per_row = Cp / 4, total = R * per_row;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) convert_rows_kernel(const TIn* __restrict
 // Column sums of a row-major [R][C] matrix (bias gradient of Linear, or of an NHWC dY), first stage:
 // row block blockIdx.y writes its sums to row blockIdx.y of the [row blocks][C] partial-sum matrix.
 template <typename TIn>
-__global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* __restrict__ in, float* colsum,
+__global__ void __launch_bounds__(256) colsum_rows_kernel(const TIn* in, float* colsum,
                                                           size_t R, int C, int rows_per_block, int role) {
     pdl_enter(role);
     size_t r0 = static_cast<size_t>(blockIdx.y) * rows_per_block;
@@ -294,7 +294,7 @@ __device__ __forceinline__ void add_vector(float (&acc)[4], const uint4& v, cons
     acc[0] += __uint_as_float(v.x); acc[1] += __uint_as_float(v.y); acc[2] += __uint_as_float(v.z); acc[3] += __uint_as_float(v.w);
 }
 template <typename TIn>
-__global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* __restrict__ in, float* colsum,
+__global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* in, float* colsum,
                                                              size_t R, int C, int rows_per_block, int role) {
     pdl_enter(role);
     constexpr int V = 16 / sizeof(TIn);
@@ -312,11 +312,11 @@ __global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* __restri
         for (; r + 56 < r1; r += 64) {
             uint4 v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(p + (r + 8 * i) * C));
+            for (int i = 0; i < 8; ++i) v[i] = load_global(reinterpret_cast<const uint4*>(p + (r + 8 * i) * C));
 #pragma unroll
             for (int i = 0; i < 8; ++i) add_vector(acc, v[i], p);
         }
-        for (; r < r1; r += 8) add_vector(acc, __ldg(reinterpret_cast<const uint4*>(p + r * C)), p);
+        for (; r < r1; r += 8) add_vector(acc, load_global(reinterpret_cast<const uint4*>(p + r * C)), p);
     }
 #pragma unroll
     for (int j = 0; j < V; ++j) part[wy][lane * V + j] = acc[j];
@@ -354,7 +354,7 @@ __device__ __forceinline__ void store_enc2(int enc, void* out0, void* out1, size
 }
 
 template <typename TIn>
-__global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* __restrict__ w, void* out0, void* out1, int enc,
+__global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* w, void* out0, void* out1, int enc,
                                                                  int R, int Cc, int Rp, int role) {
     pdl_enter(role);
     __shared__ float tile[64][65];  // [r][c]
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(256) repack_weight_tile_kernel(const TIn* __re
 }
 
 template <typename TIn>
-__global__ void __launch_bounds__(256) repack_weight_rows_kernel(const TIn* __restrict__ w, void* out0, void* out1, int enc,
+__global__ void __launch_bounds__(256) repack_weight_rows_kernel(const TIn* w, void* out0, void* out1, int enc,
                                                                  int R, int Cc, int Rp, int role) {
     pdl_enter(role);
     __shared__ float tile[64][65];  // [c][r]
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) repack_weight_rows_kernel(const TIn* __re
 // The same two for fp16 weights that stay fp16 (a training step repacks every layer's weights twice): 16-byte loads, more
 // work per block, and no detour through float.  Both want 16-byte aligned source rows and Rp a multiple of 8.
 //   [B][R][Cc] -> [B][Cc][Rp], 64 x 64 tiles; Cc a multiple of 8.  2048 x 8192: 29.6 -> 12 us (bytes: 10 us).
-__global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* __restrict__ w, __half* __restrict__ out, int R, int Cc, int Rp, int role) {
+__global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* w, __half* __restrict__ out, int R, int Cc, int Rp, int role) {
     pdl_enter(role);
     __shared__ __half tile[64][66];  // [r][c]; a pitch of 33 words spreads the column reads below over the banks
     const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* __r
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int r = r0 + q + 32 * h, c = c0 + 8 * v;
-        x[h] = (r < R && c < Cc) ? __ldg(reinterpret_cast<const uint4*>(w + (b * R + r) * Cc + c)) : make_uint4(0u, 0u, 0u, 0u);
+        x[h] = (r < R && c < Cc) ? load_global(reinterpret_cast<const uint4*>(w + (b * R + r) * Cc + c)) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(256) repack_half_tile_kernel(const __half* __r
 // in 16-byte vectors of eight rows.  A warp takes 8 taps x 4 row groups (4 x 8 where Cc is no multiple of 8): with a pitch of
 // Cc + 2 (odd) halves its reads fall on different banks.  512 x 1024 x 16: 9.9 -> 8.7 us.
 __host__ __device__ inline int repack_rows_pitch(int Cc) { return Cc % 8 == 0 ? Cc + 2 : (Cc | 1); }
-__global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __restrict__ w, __half* __restrict__ out, int R, int Cc, int Rp, int role) {
+__global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* w, __half* __restrict__ out, int R, int Cc, int Rp, int role) {
     pdl_enter(role);
     extern __shared__ __half run[];  // [256][pitch]
     const int pitch = repack_rows_pitch(Cc);
@@ -453,10 +453,10 @@ __global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __r
             const int i = i0 + h * 256 * 8;
             x[h] = make_uint4(0u, 0u, 0u, 0u);
             __half* e = reinterpret_cast<__half*>(&x[h]);
-            if (i + 8 <= n_valid) x[h] = __ldg(reinterpret_cast<const uint4*>(src + i));
+            if (i + 8 <= n_valid) x[h] = load_global(reinterpret_cast<const uint4*>(src + i));
             else
                 for (int k = 0; k < 8; ++k)
-                    if (i + k < n_valid) e[k] = src[i + k];
+                    if (i + k < n_valid) e[k] = load_global(src + i + k);
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(256) repack_half_rows_kernel(const __half* __r
 // A warp takes a padded row at a time, four pixels per lane in flight; an index decoded with 64-bit divisions per
 // pixel ran at 2.1 TB/s.
 template <typename TIn, int kCh>
-__global__ void __launch_bounds__(256) pad_pack_kernel(const TIn* __restrict__ in, int nchw, __half* __restrict__ out,
+__global__ void __launch_bounds__(256) pad_pack_kernel(const TIn* in, int nchw, __half* __restrict__ out,
                                                        int N, int C, int H, int W, int pad_h, int pad_w, int Hp,
                                                        int Wp, float* colsum, int role) {
     pdl_enter(role);
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(256) pad_pack_kernel(const TIn* __restrict__ i
 // Weights [C_out][C][KH][KW] -> [C_out][KH][8 * ch] with k = kw * ch + c (zero where c >= C or kw >= KW):
 // the K-major operand matching pad_pack's (kw, c) slices.
 template <typename TIn>
-__global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
+__global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* w, __half* __restrict__ out,
                                                                    int Cout, int C, int KH, int KW, int ch_log2, int role) {
     pdl_enter(role);
     const int total = (Cout * KH) << (3 + ch_log2);
@@ -583,9 +583,9 @@ __global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* __
 // output tensor: the planes are added in slice order (so the result is bitwise repeatable), then bias,
 // optional rounding through fp16, cast, and the caller's layout (nchw: out[n][c][pixel of the image]).
 // Row-major outputs whose channel count is a multiple of 4 take four values per thread (`vec`).
-__device__ __forceinline__ float4 finish4(float4 v, const float* bias, int c, int round_f16) {
-    if (bias != nullptr) {
-        v.x += bias[c]; v.y += bias[c + 1]; v.z += bias[c + 2]; v.w += bias[c + 3];
+__device__ __forceinline__ float4 finish4(float4 v, bool has_bias, const float4& b, int round_f16) {
+    if (has_bias) {
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
     }
     if (round_f16) {
         v.x = __half2float(__float2half_rn(v.x)); v.y = __half2float(__float2half_rn(v.y));
@@ -594,7 +594,7 @@ __device__ __forceinline__ float4 finish4(float4 v, const float* bias, int c, in
     return v;
 }
 template <typename TOut>
-__global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restrict__ acc, int planes, const float* __restrict__ bias,
+__global__ void __launch_bounds__(256) finish_rows_kernel(const float* acc, int planes, const float* bias,
                                                           TOut* __restrict__ out, size_t pixels, int C, int hw, int nchw,
                                                           int round_f16, int vec, int role) {
     pdl_enter(role);
@@ -604,13 +604,17 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restric
         const size_t total4 = total / 4;
         const float4* src = reinterpret_cast<const float4*>(acc);
         for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total4; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-            float4 v = __ldg(src + i);
+            float4 v = load_global(src + i), bv = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (bias != nullptr) {  // (in flight with the planes)
+                const float* b = bias + static_cast<uint32_t>(i) % c4n * 4;
+                bv = make_float4(load_global(b), load_global(b + 1), load_global(b + 2), load_global(b + 3));
+            }
 #pragma unroll 8
             for (int z = 1; z < planes; ++z) {
-                const float4 b = __ldg(src + static_cast<size_t>(z) * total4 + i);
+                const float4 b = load_global(src + static_cast<size_t>(z) * total4 + i);
                 v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
             }
-            v = finish4(v, bias, static_cast<int>(static_cast<uint32_t>(i) % c4n) * 4, round_f16);
+            v = finish4(v, bias != nullptr, bv, round_f16);
             if (sizeof(TOut) == 2) {
                 uint2 h;
                 *reinterpret_cast<__half2*>(&h.x) = __floats2half2_rn(v.x, v.y);
@@ -627,10 +631,10 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restric
          i += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const size_t p = i / C;
         const int c = static_cast<int>(i - p * C);
-        float v = acc[i];
+        float v = load_global(acc + i);
 #pragma unroll 4
-        for (int z = 1; z < planes; ++z) v += __ldg(acc + static_cast<size_t>(z) * total + i);
-        if (bias != nullptr) v += bias[c];
+        for (int z = 1; z < planes; ++z) v += load_global(acc + static_cast<size_t>(z) * total + i);
+        if (bias != nullptr) v += load_global(bias + c);
         if (round_f16) v = __half2float(__float2half_rn(v));
         size_t o = i;
         if (nchw) {
@@ -649,8 +653,8 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* __restric
 // which phase ph reaches through kernel row kh = ph + p_h - (kh' + dh_min) * s_h (zero weight if that
 // is no kernel row).  Also replicates the bias per phase.
 template <typename TIn, typename TBias>
-__global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __restrict__ w, __half* __restrict__ out,
-                                                                 const TBias* __restrict__ bias, float* __restrict__ bias_out,
+__global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* w, __half* __restrict__ out,
+                                                                 const TBias* bias, float* __restrict__ bias_out,
                                                                  int K, int C, int KH, int KW, int s_h, int s_w, int p_h,
                                                                  int p_w, int khp, int kwp, int dh_min, int dw_min, int role) {
     pdl_enter(role);
@@ -682,7 +686,7 @@ __global__ void __launch_bounds__(256) pack_phase_weights_kernel(const TIn* __re
 // partial-sum matrix in a fixed order (128 interleaved running sums, then those in a tree) and writes row blockIdx.y of
 // `out` ([segments][out_stride]).  Launched again on its own output while more than one segment is left.
 // blockDim = (8, 128): few channels and a chain of load latencies, so many threads take few rows each.
-__global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __restrict__ partial, int P, int stride, int C,
+__global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* partial, int P, int stride, int C,
                                                              float* __restrict__ out, int out_stride, int rows_per_block, int role) {
     pdl_enter(role);
     __shared__ float part[128][9];
@@ -692,7 +696,7 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
     float s = 0.f;
     if (c < C) {
 #pragma unroll 8
-        for (int p = p0 + threadIdx.y; p < p1; p += 128) s += __ldg(partial + static_cast<size_t>(p) * stride + c);
+        for (int p = p0 + threadIdx.y; p < p1; p += 128) s += load_global(partial + static_cast<size_t>(p) * stride + c);
     }
     part[threadIdx.y][threadIdx.x] = s;
     for (int half = 64; half > 0; half /= 2) {
@@ -706,7 +710,7 @@ __global__ void __launch_bounds__(1024) colsum_finish_kernel(const float* __rest
 // Second stage of a split-K weight gradient: adds the K slices' planes in slice order (bitwise
 // repeatable, unlike atomics) and writes dW once.  Row form: dW is `rows` rows of `row_len4` float4,
 // plane z holds row r at planes + z * plane_elems + r * src_pitch (floats).
-__global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __restrict__ planes, float* __restrict__ dw,
+__global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* planes, float* __restrict__ dw,
                                                                  int split, size_t plane_elems, size_t rows, int row_len4,
                                                                  size_t src_pitch, int role) {
     pdl_enter(role);
@@ -716,11 +720,11 @@ __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __
         const size_t r = i / row_len4;
         const int c4 = static_cast<int>(i - r * row_len4);
         const float4* src = reinterpret_cast<const float4*>(planes + r * src_pitch) + c4;
-        float4 a = __ldg(src);
+        float4 a = load_global(src);
         const size_t step = plane_elems / 4;
 #pragma unroll 4
         for (int z = 1; z < split; ++z) {
-            const float4 b = __ldg(src + z * step);
+            const float4 b = load_global(src + z * step);
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
         }
         reinterpret_cast<float4*>(dw)[i] = a;
@@ -732,7 +736,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* __
 // per element would walk ~150 planes one load latency at a time.  blockDim = (32, 8): lane ty adds
 // planes ty, ty + 8, ... of its float4 in order, then the eight running sums are added in order -- a
 // fixed association, so still bitwise repeatable.  Planes are laid out like dW.
-__global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __restrict__ planes, float* __restrict__ dw,
+__global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* planes, float* __restrict__ dw,
                                                                  int split, size_t plane_elems, size_t total4, int role) {
     pdl_enter(role);
     __shared__ float4 part[8][32];
@@ -743,7 +747,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __
         const size_t step = plane_elems / 4;
 #pragma unroll 4
         for (int z = threadIdx.y; z < split; z += 8) {
-            const float4 b = __ldg(src + z * step);
+            const float4 b = load_global(src + z * step);
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
         }
     }
@@ -767,7 +771,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* __
 // are written.  (A thread per element read with a stride of a whole tap row: 4x4 512->128 11 us.)  kPlain plain channels a
 // block, their loads in flight together, and 16-byte stores: 4x4 512 x 1024, one plane, 18.8 -> 14 us (bytes: 10 us).
 constexpr int kReducePlain = 2;
-__global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* __restrict__ planes, float* __restrict__ dw, int split,
+__global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* planes, float* __restrict__ dw, int split,
                                                                 size_t plane_elems, int c_patch, int c_plain, int n_taps, int c_blocks, int kb,
                                                                 int R, int role) {
     pdl_enter(role);
@@ -783,13 +787,13 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* __r
             float4 a[kReducePlain];
 #pragma unroll
             for (int q = 0; q < kReducePlain; ++q)
-                if (q < n_plain) a[q] = __ldg(reinterpret_cast<const float4*>(p + static_cast<size_t>(q) * R));
+                if (q < n_plain) a[q] = load_global(reinterpret_cast<const float4*>(p + static_cast<size_t>(q) * R));
 #pragma unroll 4
             for (int z = 1; z < split; ++z) {
 #pragma unroll
                 for (int q = 0; q < kReducePlain; ++q)
                     if (q < n_plain) {
-                        const float4 v = __ldg(reinterpret_cast<const float4*>(p + z * plane_elems + static_cast<size_t>(q) * R));
+                        const float4 v = load_global(reinterpret_cast<const float4*>(p + z * plane_elems + static_cast<size_t>(q) * R));
                         a[q].x += v.x; a[q].y += v.y; a[q].z += v.z; a[q].w += v.w;
                     }
             }
@@ -832,7 +836,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* __r
 // [plain channel][R rows of the tile walk] and dW element (plain, pc, t) sits at row
 // (t * c_blocks + pc / kb) * kb + pc % kb.  layout 2 (few-channel window walk): dW element
 // (plain, c, kh, kw) sits at row kh * kb + kw * 8 + c.
-__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ planes, float* __restrict__ dw, int split,
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* planes, float* __restrict__ dw, int split,
                                                            size_t plane_elems, size_t total, int layout, int c_patch,
                                                            int n_taps, int kw_count, int c_blocks, int kb, int R, int role) {
     pdl_enter(role);
@@ -854,15 +858,15 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
             const size_t plain = q / c_patch;
             src = plain * R + static_cast<size_t>(kh) * kb + kw * 8 + c;
         }
-        float a = __ldg(planes + src);
-        for (int z = 1; z < split; ++z) a += __ldg(planes + z * plane_elems + src);
+        float a = load_global(planes + src);
+        for (int z = 1; z < split; ++z) a += load_global(planes + z * plane_elems + src);
         dw[i] = a;
     }
     pdl_leave(role);
 }
 
 template <typename TIn>
-__global__ void __launch_bounds__(256) to_float_kernel(const TIn* __restrict__ in, float* out, int n, int role) {
+__global__ void __launch_bounds__(256) to_float_kernel(const TIn* in, float* out, int n, int role) {
     pdl_enter(role);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = load_as_float(in, i);

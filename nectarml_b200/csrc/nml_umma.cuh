@@ -1112,8 +1112,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     for (int u = 0; u < 8; ++u) {
                         const int j = lane + 32 * u;
                         bv[u] = !(j < P.bn && col_base + j < P.c_out) ? 0.f
-                                : P.bias_f16 ? __half2float(__ldg(reinterpret_cast<const __half*>(P.bias) + col_base + j))
-                                             : __ldg(P.bias + col_base + j);
+                                : P.bias_f16 ? __half2float(load_global(reinterpret_cast<const __half*>(P.bias) + col_base + j))
+                                             : load_global(P.bias + col_base + j);
                     }
                     __syncwarp();
 #pragma unroll
@@ -1443,10 +1443,10 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 if (cgf + cpi0 <= P.c_out) {
                     const int ql = lane & 7;
                     if (kOutF16) {
-                        nb0 = __ldg(reinterpret_cast<const float4*>(P.bias + cgf + 8 * ql));
-                        nb1 = __ldg(reinterpret_cast<const float4*>(P.bias + cgf + 8 * ql + 4));
+                        nb0 = load_global(reinterpret_cast<const float4*>(P.bias + cgf + 8 * ql));
+                        nb1 = load_global(reinterpret_cast<const float4*>(P.bias + cgf + 8 * ql + 4));
                     } else {
-                        nb0 = __ldg(reinterpret_cast<const float4*>(P.bias + cgf + 4 * ql));
+                        nb0 = load_global(reinterpret_cast<const float4*>(P.bias + cgf + 4 * ql));
                     }
                 }
             }
@@ -1487,7 +1487,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         if (j < P.c_out) {
                             if (oh0 + phs < P.shuf_oh && ow0 + pw < P.shuf_ow) {
                                 float xv = (k_iters > 0) ? __uint_as_float(r[j]) : 0.f;
-                                if (P.bias != nullptr) xv += __ldg(P.bias + j);
+                                if (P.bias != nullptr) xv += load_global(P.bias + j);
                                 if (kOutF16) {
                                     reinterpret_cast<__half*>(P.out)[o_row + q] = __float2half_rn(xv);
                                 } else {
@@ -1530,7 +1530,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     for (int j = 0; j < 8; ++j) {
                         if (j < P.c_out) {
                             float xv = (k_iters > 0) ? __uint_as_float(r[j]) : 0.f;
-                            if (P.bias != nullptr) xv += __ldg(P.bias + j);
+                            if (P.bias != nullptr) xv += load_global(P.bias + j);
                             if (kOutF16) {
                                 reinterpret_cast<__half*>(P.out)[row_off + j] = __float2half_rn(xv);
                             } else {
@@ -1619,10 +1619,10 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             const int cgn = cg + cpi;
                             if (c0 + cpi < P.bn && cgn + cpi <= P.c_out) {
                                 if (kOutF16) {
-                                    nb0 = __ldg(reinterpret_cast<const float4*>(P.bias + cgn + 8 * q));
-                                    nb1 = __ldg(reinterpret_cast<const float4*>(P.bias + cgn + 8 * q + 4));
+                                    nb0 = load_global(reinterpret_cast<const float4*>(P.bias + cgn + 8 * q));
+                                    nb1 = load_global(reinterpret_cast<const float4*>(P.bias + cgn + 8 * q + 4));
                                 } else {
-                                    nb0 = __ldg(reinterpret_cast<const float4*>(P.bias + cgn + 4 * q));
+                                    nb0 = load_global(reinterpret_cast<const float4*>(P.bias + cgn + 4 * q));
                                 }
                             }
                         }
@@ -1662,8 +1662,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         // Ragged tail, or rows that do not start on 16 bytes: the piece goes through the staging tile as
                         // above and leaves row by row, the lanes along the row.  (A thread storing its own row touches
                         // 32 sectors per instruction: 333 x 64 x 333 matmuls spent 22 us each in it.)
-                        const float bias_lo = (has_bias && lane < ncols) ? __ldg(P.bias + cg + lane) : 0.f;
-                        const float bias_hi = (kOutF16 && has_bias && lane + 32 < ncols) ? __ldg(P.bias + cg + 32 + lane) : 0.f;
+                        const float bias_lo = (has_bias && lane < ncols) ? load_global(P.bias + cg + lane) : 0.f;
+                        const float bias_hi = (kOutF16 && has_bias && lane + 32 < ncols) ? load_global(P.bias + cg + 32 + lane) : 0.f;
                         if (kOutF16) {
 #pragma unroll
                             for (int j = 0; j < 32; ++j) {  // one bank per lane: word (lane, j) of a 33-word pitch
@@ -1752,7 +1752,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 } else {
                     // channel-major output
                     if (P.bias != nullptr) {
-                        const float bl = lane < ncols ? __ldg(P.bias + cg + lane) : 0.f;  // one load, handed round
+                        const float bl = lane < ncols ? load_global(P.bias + cg + lane) : 0.f;  // one load, handed round
 #pragma unroll
                         for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __shfl_sync(0xffffffffu, bl, j));
                     }

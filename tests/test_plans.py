@@ -59,3 +59,18 @@ def test_output_copy_is_bounded(lib):
         d = g.desc(NML_F32, "nchw", NML_F32, "nchw", NML_F32, "f16", False)
         assert lib.nml_conv_workspace_size(C.byref(d), 0, C.byref(need)) == _lib.NML_OK
         assert (need.value > batch * 512 * ho * wo * 4) == copied
+
+
+def test_no_read_only_loads_in_the_kernels():
+    """Grids become resident before the ones in front have written what they read, so no kernel may use read-only loads: neither
+    the intrinsics nor const __restrict__ pointers, which the compiler reads through the same path."""
+    import glob
+    import os
+    import re
+    csrc = os.path.join(os.path.dirname(_lib.__file__), "csrc")
+    files = glob.glob(os.path.join(csrc, "*.cu")) + glob.glob(os.path.join(csrc, "*.cuh"))
+    assert len(files) >= 6
+    for path in files:
+        code = re.sub(r"//[^\n]*", "", open(path).read())
+        found = re.findall(r"__ldg\s*\(|__ldc[gsavl]+\s*\(|__ldlu\s*\(|global\.nc|const\s+\w+\s*\*\s*__restrict__", code)
+        assert not found, (os.path.basename(path), found[:3])

@@ -669,7 +669,9 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     }
     const bool rec = rec_slot >= 0;
     if (rec && !pre_opened) NML_CUDA(cudaEventRecord(g_prof.start[rec_slot], st));
-    launch_with(true, P.pair ? 2 : 1, kernel_for(P), grid, threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st, P);
+    // (under an SM limit not before its predecessor has ended: blocks that wait would sit on the SMs that are to stay free, and
+    // a block of this kernel leaves no room beside it)
+    launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st, P);
     NML_CUDA(cudaGetLastError());
     if (open_slot) *open_slot = rec_slot;
     else if (rec) NML_CUDA(cudaEventRecord(g_prof.stop[rec_slot], st));

@@ -194,3 +194,40 @@ def test_saved_tensor_hooks_see_what_the_layers_keep():
     ops.device_status()
     assert sorted(packed) == sorted([(2, 6, 6, 8), (2, 6, 6, 16), (16,), (16,), (2 * 6 * 6 * 16 // 8,)])
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_sm_limit_holds_for_the_next_launch_too():
+    """Two long products in a stream under a limit of half the SMs: the second must not take the other half while it waits for
+    the first, so a small product on another stream (a collective, in earnest) runs at once and not after the first."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    x, w = torch.zeros(32768, 8192, device="cuda").half(), torch.zeros(8192, 8192, device="cuda").half()
+    out = [torch.empty(32768, 8192, device="cuda").half() for _ in range(2)]
+    a, b, ws = torch.zeros(128, 512, device="cuda").half(), torch.zeros(512, 512, device="cuda").half(), ops.Workspace()
+    side, event = torch.cuda.Stream(), lambda: torch.cuda.Event(enable_timing=True)  # noqa: E731
+    ops.set_sm_limit(sms // 2)
+    try:
+        for _ in range(2):  # (once to warm up)
+            torch.cuda.synchronize()
+            begin, first, small = event(), event(), event()
+            begin.record()
+            ops.linear_forward(x, w, out=out[0])
+            first.record()
+            torch.cuda.synchronize()
+            alone = begin.elapsed_time(first)
+            with torch.cuda.stream(side):
+                c = torch.empty(128, 512, device="cuda").half()
+            torch.cuda.synchronize()
+            begin.record()
+            for o in out:
+                ops.linear_forward(x, w, out=o)
+            time.sleep(0.001)
+            with torch.cuda.stream(side):
+                ops.linear_forward(a, b, out=c, ws=ws)
+                small.record()
+            torch.cuda.synchronize()
+            ended = begin.elapsed_time(small)
+    finally:
+        ops.set_sm_limit(0)
+    ops.device_status()
+    assert alone > 3.0, alone
+    assert ended < 0.7 * alone, (ended, alone)

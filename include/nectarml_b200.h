@@ -182,7 +182,9 @@ long long nml_launch_count(void);
 
 /* Per-launch device timing of the contraction kernel.  After nml_profile_begin(n) each of the
  * next n contraction launches is bracketed by CUDA events on its own stream; nml_profile_end
- * synchronises, writes the durations in milliseconds in launch order and stops recording.
+ * synchronises, writes the durations in milliseconds in launch order and stops recording.  The
+ * second stage of a launch (sums of K slices, the turn of a result into NCHW) counts in; the sums of
+ * a bias gradient do not, and run in front of the contraction instead of beside it meanwhile.
  * Measurement support only: nothing else in the library depends on it. */
 int nml_profile_begin(int max_records);
 int nml_profile_end(float* ms_out, int capacity, int* count);

@@ -718,7 +718,8 @@ static bool narrow_patch_walk(const FpropLike& f, int N) {
     return eff_patch >= 0.8 * eff_box && need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
 }
 
-static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
+// With `open_slot` the timing bracket of a recorded launch is left open, for a caller that launches more of the pass.
+static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* open_slot = nullptr) {
     MathInfo mi;
     if (!math_info(f.math, &mi)) return NML_ERR_INVALID;
     // A column-strided gather into an NCHW result stores single values a stride apart (4 of every 8 bytes, phase after
@@ -744,7 +745,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
         const long long tiles = 1ll * tiles_p * tiles_c * f.batch;
         if (probe_rc == NML_OK && bytes <= (1ull << 30) && probe.off <= ws.limit && (ws.dry || probe.off <= ws.cap) && tiles < INT_MAX / 2) {
             f2.out = ws.take(bytes);
-            const int rc = run_fprop_like(f2, ws, st);
+            int slot = -1;
+            const int rc = run_fprop_like(f2, ws, st, &slot);
             if (rc || ws.dry) return rc;
             const unsigned blocks = static_cast<unsigned>(std::min<long long>(tiles, 6 * kSms));
             if (f.out_dtype == NML_F16)
@@ -755,7 +757,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
                               static_cast<float*>(f.out), f.out_c, hw, tiles_p, tiles_c, static_cast<int>(tiles));
             ++g_launches;
             NML_CUDA(cudaGetLastError());
-            return NML_OK;
+            return profile_stop(slot, st);
         }
     }
     // A strided gather with very few output channels (input gradient of an RGB stem, image-producing
@@ -811,7 +813,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             f2.out_c = np; f2.out_h = ceil_div(f.out_h, f.s_h); f2.out_w = ceil_div(f.out_w, f.s_w);
             f2.bias = bp; f2.bias_dtype = NML_F32;
             f2.shuf_sh = f.s_h; f2.shuf_sw = f.s_w; f2.shuf_c = C; f2.shuf_oh = f.out_h; f2.shuf_ow = f.out_w;
-            return run_fprop_like(f2, ws, st);
+            return run_fprop_like(f2, ws, st, open_slot);
         }
     }
     const int T = f.kh * f.kw;
@@ -1344,8 +1346,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
     int slot = -1;
     rc = launch_kernel(P, ds, st, &slot);
     if (rc) return rc;
-    if (P.fsplit <= 1) return profile_stop(slot, st);
-    {
+    if (P.fsplit > 1) {
         const size_t total = out_pixels * N;
         const int blocks = static_cast<int>(std::min<size_t>((total + 1023) / 1024, 148 * 8));
         const int nchw = (f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1)) ? 1 : 0;
@@ -1357,6 +1358,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st) {
             { helper_launch(4 * kSms, finish_rows_kernel<float>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
                                                              f.out_h * f.out_w, nchw, f.round_f16, vec); ++g_launches; }
         NML_CUDA(cudaGetLastError());
+    }
+    if (open_slot) {
+        *open_slot = slot;
+        return NML_OK;
     }
     return profile_stop(slot, st);
 }

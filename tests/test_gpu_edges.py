@@ -231,3 +231,23 @@ def test_sm_limit_holds_for_the_next_launch_too():
     ops.device_status()
     assert alone > 3.0, alone
     assert ended < 0.7 * alone, (ended, alone)
+
+
+def test_profile_counts_the_turn_into_nchw():
+    """A strided gradient into NCHW through a copy: the recorded duration holds the copy's turn.  The 205 MB are read and written
+    once more, 50 us at 8 TB/s; half of that tells the two apart."""
+    g = ops.ConvGeometry(256, 256, 28, 28, 64, 3, 3, (2, 2), (1, 1))
+    best = {}
+    for layout in ("nchw", "nhwc"):
+        dy = torch.zeros(g.act_shape("out", layout), device="cuda").half()
+        w = torch.zeros(g.weight_shape(), device="cuda").half()
+        out = torch.empty(g.act_shape("in", layout), device="cuda")
+        ops.conv_backward_data(g, dy, w, layout=layout, out=out)
+        ops.profile_begin(5)
+        for _ in range(5):
+            ops.conv_backward_data(g, dy, w, layout=layout, out=out)
+        times = ops.profile_end(5)
+        assert len(times) == 5
+        best[layout] = min(times)
+    ops.device_status()
+    assert best["nchw"] - best["nhwc"] > 0.025, best

@@ -1159,8 +1159,9 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         }
     }
     // Row-major output through TMA stores when the geometry allows: the box is the 32 consecutive tile
-    // rows one epilogue warp owns (a sub-box of the tile's pixel box), 128 bytes of columns wide.
-    if (P.out_mode == OUT_NHWC && tune().tmastore) {
+    // rows one epilogue warp owns (a sub-box of the tile's pixel box), 128 bytes of columns wide.  (Never phase-packed columns:
+    // they belong to several output pixels, and the packed image may be larger than the output.)
+    if (P.out_mode == OUT_NHWC && !P.shuf_sh && tune().tmastore) {
         const int esz = P.out_f16 ? 2 : 4;
         const int cpi = 128 / esz;
         if (P.bn % cpi == 0 && (static_cast<size_t>(N) * esz) % 16 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0) {

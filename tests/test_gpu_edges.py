@@ -251,3 +251,42 @@ def test_profile_counts_the_turn_into_nchw():
         best[layout] = min(times)
     ops.device_status()
     assert best["nchw"] - best["nhwc"] > 0.025, best
+
+
+# input gradients (or transposed forwards) with a handful of channels at strides above one, into fp32 NHWC: kernels, strides and
+# paddings whose images do not suit the patch walk; (batch, channels in, h, w, channels out, kernel, stride, padding,
+# output padding, transposed)
+PACKED = [
+    (5, 4, 1, 45, 1, (1, 3), (2, 1), (0, 1), (0, 0), False), (9, 3, 15, 4, 8, (3, 3), (2, 2), (0, 0), (0, 0), False),
+    (18, 1, 7, 13, 192, (3, 1), (2, 2), (2, 0), (0, 0), False), (22, 4, 2, 40, 3, (4, 4), (2, 2), (3, 2), (0, 0), False),
+    (4, 2, 14, 28, 8, (3, 1), (2, 2), (2, 0), (0, 0), False), (11, 1, 3, 4, 4, (3, 3), (2, 2), (0, 2), (0, 0), False),
+    (11, 1, 12, 32, 3, (7, 7), (2, 2), (5, 4), (1, 1), True), (22, 64, 4, 5, 4, (1, 1), (2, 2), (0, 0), (0, 1), True),
+    (2, 8, 12, 17, 4, (1, 3), (1, 2), (0, 1), (0, 0), True), (3, 16, 16, 16, 3, (4, 4), (2, 2), (1, 1), (0, 0), True),
+]
+
+
+@pytest.mark.parametrize("case", PACKED)
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.float16])
+def test_phase_packed_columns(case, out_dtype):
+    """All output phases in the columns of one walk, each value to its own pixel and nothing beside the result: against float64
+    on fp16 operands (fp32 sums of at most 200 * 49 products, 1e-6 of the result's norm; half an ulp of fp16 where it is stored
+    so), with a canary on both sides of the output."""
+    b, ci, h, w, co, k, s, p, op, tr = case
+    g = ops.ConvGeometry(b, ci, h, w, co, *k, s, p, (1, 1), op, tr)
+    gen = torch.Generator(device="cuda").manual_seed(h * w)
+    wt = (torch.randn(g.weight_shape(), device="cuda", generator=gen) * 0.2).half()
+    src = torch.randn(g.act_shape("in" if tr else "out", "nhwc"), device="cuda", generator=gen).half()
+    shape = g.act_shape("out" if tr else "in", "nhwc")
+    n = shape[0] * shape[1] * shape[2] * shape[3]
+    flat = torch.full((n + 2 * 4096,), 7.0, device="cuda", dtype=out_dtype)
+    out = flat[4096:4096 + n].view(shape)
+    if tr:
+        ops.conv_forward(g, src, wt, layout="nhwc", out=out)
+    else:
+        ops.conv_backward_data(g, src, wt, layout="nhwc", out=out)
+    ops.device_status()
+    x, wd = src.double().permute(0, 3, 1, 2), wt.double()
+    pad = op if tr else [(e + 2 * q - kk) % ss for e, q, kk, ss in zip((h, w), p, k, s)]
+    want = torch.nn.functional.conv_transpose2d(x, wd, None, s, p, pad).permute(0, 2, 3, 1)
+    assert float((out.double() - want).norm() / want.norm()) <= (1e-6 if out_dtype == torch.float32 else 5e-4)
+    assert bool((flat[:4096] == 7).all()) and bool((flat[4096 + n:] == 7).all())

@@ -517,7 +517,7 @@ static int prepare_window(const void* src, int dtype, int layout, int batch, int
 // Picks a power-of-two pixel box (w, h, n) with 2^bits pixels that covers the grid with the
 // fewest boxes; ties go to the wider box.  box extents times the element stride stay <= 256.  n_tiles: tiles per box.
 static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* wl, int* hl, int* nl,
-                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1) {
+                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1, bool split = false) {
     long long best = -1, best_wide = -1;
     int ww = 0, wh = 0, wn = 0;
     for (int a = bits; a >= 0; --a) {
@@ -544,8 +544,12 @@ static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* 
     // A box at least 2^prefer_w_log2 pixels wide (whole 128-byte runs for pixel-major stores) is taken
     // when it costs at most 15 % more tiles and no further round of tiles: 3x3 96 -> 96 at 56 x 56, batch 16, fp16 31.1 -> 27.6 us
     // with 392 tiles instead of 448; 128 -> 128 at 28 x 28, batch 16, 112 tiles instead of 98 in one round, 17.1 -> 15.9.
+    // 3xTF32 tiles are 128 columns wide: 256 -> 256 at 56 x 56, batch 8, 392 tiles instead of 448 154 -> 124 us.  Their narrow
+    // boxes have to save a round of several, though: where all run at once nothing overlaps the drain (`split`; 128 -> 384 at
+    // 28 x 28, batch 8, 49.1 us in two rounds of wide boxes, 54.2 in one of narrow ones).
     const auto rounds = [&](long long boxes) { return (boxes * n_tiles + sms - 1) / sms; };
-    if (prefer_w_log2 > 0 && best_wide > 0 && best_wide * 100 <= best * 115 && rounds(best_wide) <= rounds(best)) {
+    if (prefer_w_log2 > 0 && best_wide > 0 && best_wide * 100 <= best * 115 &&
+        (rounds(best_wide) <= rounds(best) || (split && rounds(best) == 1))) {
         *wl = ww;
         *hl = wh;
         *nl = wn;
@@ -1041,7 +1045,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         P.wb_log2 = 7;
     } else {
         choose_box(7, P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, &P.wb_log2, &P.hb_log2, &P.nb_log2,
-                   (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0, ceil_div(N, 256), limited(ds->sms));
+                   (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0, ceil_div(N, P.planes == 2 ? 128 : 256), limited(ds->sms), P.planes == 2);
     }
     // Patch walk: unit-stride walks with several taps load one haloed patch per channel block instead of
     // one box per tap (8 x 16 pixel tiles of a single image).  Taken when the fixed tile shape does not

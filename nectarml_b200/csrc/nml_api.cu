@@ -727,7 +727,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     MathInfo mi;
     if (!math_info(f.math, &mi)) return NML_ERR_INVALID;
     // A column-strided gather into an NCHW result stores single values a stride apart (4 of every 8 bytes, phase after
-    // phase).  Where the phases' rows are no multiple of eight pixels the tiles' boxes are at most four pixels wide and every
+    // phase).  Where the first (widest) phase's rows are no multiple of eight pixels the tiles' boxes are at most four pixels wide and every
     // store is a part of a sector; those go through an NHWC copy in the workspace (the walk's stores are TMA boxes then), which
     // one pass of full-width stores turns round.  Input gradient of 3x3 s2, fp32 result of fp16 / 3xTF32 products: 128 channels at
     // 28 x 28, batch 64 30.6 -> 28.4 / 48.4 -> 39.9 us; 256 at 28 x 28, batch 64 99.8 -> 54.4 / 131 -> 101; but 64 at 64 x 64 (whole
@@ -834,7 +834,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         if (rc) return rc;
     }
     // Few input channels (RGB stems): one K slice per kernel ROW, holding (kw, c) for 8 taps, read
-    // as overlapping 8-pixel windows of a padded 8-channel image -- instead of one mostly empty
+    // as overlapping 8-pixel windows of a padded image of four or eight channels -- instead of one mostly empty
     // 64-channel slice per tap.
     const bool window = !f.gather && !f.k_is_dim0 && T > 1 && window_eligible(f.a_c, f.kw, f.d_w, mi.enc);
     // (narrow: with four channels per pixel, where the patch walk with resident weights will be taken)
@@ -1402,7 +1402,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     const void* pa[2] = {nullptr, nullptr};
     const void* pb[2];
     int cpa = 0, cpb = 0;
-    // Few-channel layer input (RGB stems): patches come as 8-pixel windows of the padded 8-channel image,
+    // Few-channel layer input (RGB stems): patches come as 8-pixel windows of the padded image,
     // one kernel row per tap, (kw, c) packed in the 64 patch columns.
     const bool window = T > 1 && window_eligible(g.patch_c, g.kw, g.d_w, mi.enc);
     // (narrow: with four channels per pixel, where the patch walk below will be taken: the same conditions)

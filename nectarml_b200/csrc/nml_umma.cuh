@@ -6,7 +6,7 @@
 //                                operand, warp 6 the B operand (issuing a TMA costs its thread a
 //                                few hundred clocks, so one thread cannot feed narrow tiles)
 //   warp 1      MMA issuer     : one thread issues tcgen05.mma, accumulators live in TMEM,
-//                                two TMEM buffers so the epilogue of tile i overlaps tile i+1
+//                                two or four TMEM buffers so the epilogue of tile i overlaps tile i+1
 //   warps 2..5  epilogue       : tcgen05.ld -> bias / rounding / cast -> TMA or plain global stores
 //   warps 7..10 epilogue       : second group, TMA-store instances only, used on short-K tiles
 //
@@ -105,8 +105,8 @@ struct KParams {
     // of every tap, and the MMA of tap (dh, dw) reads its 128 rows straight out of that patch: its
     // descriptor starts (dh * patch_w + dw) rows in, and 8-row groups are patch_w rows apart.  (The swizzle
     // is a function of the shared-memory address, so a descriptor may start on any 128-byte row.)
-    // A is then read from L2 about once instead of once per tap.  B slices stream through the stage ring,
-    // or stay resident in shared memory for the whole launch when all of them fit.
+    // A is then read from L2 about once instead of once per tap.  Every B slice is loaded once and stays in shared memory for
+    // the whole launch (the walk is taken only where all of them fit).
     // Forward walk, few tiles and a long K loop (U-Net bottleneck layers): the K iterations of a tile are
     // cut into fsplit slices that run as separate tiles; slice z stores its partial sums into plane z
     // of a row-major scratch, and a small pass adds the planes in order and produces the output.
@@ -355,10 +355,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     // They take turns: an issuer does its waiting ahead, but issues its tile only once the other has issued the one before.
     // (MMAs of two tiles interleaved on the pipe took 67 clocks each, one tile's after the other's 56.)
     auto patch_resident_issue = [&](int t_first, int t_step) {
-        const uint32_t idesc = make_instr_desc(P.kind, 0, P.b_mn_major, kTileM, P.bn);
-        const bool b32 = P.b_mn_major && P.kind == KIND_TF32;
-        const uint32_t lbo_b = P.b_mn_major ? box_bytes : 16;
-        const uint32_t adv_b = P.b_mn_major ? (((P.kind == KIND_F16) ? 16 : 8) * 128) >> 4 : 2;
+        const uint32_t idesc = make_instr_desc(P.kind, 0, 0, kTileM, P.bn);  // (both operands K-major)
         const uint32_t b_step = static_cast<uint32_t>(stage_b_bytes) >> 4;
         const uint32_t sbo_a = static_cast<uint32_t>(P.patch_w * P.a_stride_h * P.a_row_bytes);  // 8-row groups: one output row = a_stride_h patch rows apart
         const bool f16 = (P.kind == KIND_F16);
@@ -396,8 +393,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     !mbar_wait(smem_u32(&turn_bar[t_first]), ((titer - 1) >> 1) & 1, abort_flag, P.err, ERR_WAIT_EMPTY)) return;
                 if (elect_one()) {
                     const uint64_t adesc0 = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, layout_a);
-                    uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, lbo_b,
-                                                    b32 ? 512 : 8 * P.b_row_bytes, b32 ? 1 : layout_a);
+                    uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, 16, 8 * P.b_row_bytes, layout_a);
                     // (the next tap's offset is fetched while this one's MMAs are issued: a constant load per tap in the chain
                     // costs as much as a narrow tap's MMAs)
                     uint32_t off = static_cast<uint32_t>(tp[0].aoff);
@@ -419,14 +415,14 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         off = static_cast<uint32_t>(tp[min(t + 1, nt - 1)].aoff);
                         if (f16) {
                             umma_f16(d_tmem, adesc, bdesc, idesc, acc);
-                            umma_f16(d_tmem, adesc + 2, bdesc + adv_b, idesc, 1u);
-                            umma_f16(d_tmem, adesc + 4, bdesc + 2 * adv_b, idesc, 1u);
-                            umma_f16(d_tmem, adesc + 6, bdesc + 3 * adv_b, idesc, 1u);
+                            umma_f16(d_tmem, adesc + 2, bdesc + 2, idesc, 1u);
+                            umma_f16(d_tmem, adesc + 4, bdesc + 4, idesc, 1u);
+                            umma_f16(d_tmem, adesc + 6, bdesc + 6, idesc, 1u);
                         } else {
                             umma_tf32(d_tmem, adesc, bdesc, idesc, acc);
-                            umma_tf32(d_tmem, adesc + 2, bdesc + adv_b, idesc, 1u);
-                            umma_tf32(d_tmem, adesc + 4, bdesc + 2 * adv_b, idesc, 1u);
-                            umma_tf32(d_tmem, adesc + 6, bdesc + 3 * adv_b, idesc, 1u);
+                            umma_tf32(d_tmem, adesc + 2, bdesc + 2, idesc, 1u);
+                            umma_tf32(d_tmem, adesc + 4, bdesc + 4, idesc, 1u);
+                            umma_tf32(d_tmem, adesc + 6, bdesc + 6, idesc, 1u);
                         }
                         acc = 1u;
                         bdesc += b_step;
@@ -688,7 +684,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     int kb_begin = z * per;
                     int kb_end = min(kb_begin + per, P.kblocks_total);
                     int g_per_tile = kTileM / P.kb;
-                    if (kPair) {
+                    if (kPair) {  // (pairs are only planned for grouped operands)
                     // one K block per stage, one box per plane: the single issuing lane has ~500 clocks per stage, so its
                     // loop carries nothing but counters
                     int tw = kb_begin % P.ktiles_w;
@@ -758,18 +754,14 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     const int plane = P.planes == 2 ? (my_atom & 1) : 0;
                     if (nkb > 0) advance(P.planes == 2 ? my_atom >> 1 : my_atom);
                     for (int it = 0; it < nkb; it += ks) {  // one stage per iteration
-                        uint32_t fb = smem_u32(&full_bar[stage]);
-                        if (kPair) fb = map_to_cta(fb, 0);
+                        const uint32_t fb = smem_u32(&full_bar[stage]);
                         if (!__all_sync(issue_mask, mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
                                                               ERR_WAIT_EMPTY))) {
                             ok = false;
                             break;
                         }
                         const int n_in_stage = min(P.ka, (nkb - it) * P.planes);
-                        if (lane == 0) {
-                            if (!kPair) mbar_arrive_expect_tx(fb, n_in_stage * tx_bytes);
-                            else if (leader) mbar_arrive_expect_tx(smem_u32(&full_bar[stage]), 2 * n_in_stage * tx_bytes);
-                        }
+                        if (lane == 0) mbar_arrive_expect_tx(fb, n_in_stage * tx_bytes);
                         __syncwarp(issue_mask);
                         if (my_atom < n_in_stage) {
                             const CUtensorMap* ta = &P.tmA[plane];
@@ -777,15 +769,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                             const int w0 = tw << P.wb_log2, h0 = th << P.hb_log2, n0 = tn << P.nb_log2;
                             const uint32_t sa = smem_u32(smem + stage * stage_bytes) + my_atom * kStageABytes;
                             const uint32_t sb = smem_u32(smem + stage * stage_bytes) + b_off + my_atom * stage_b_bytes;
-                            if (kPair) {  // pairs are only planned for grouped operands
-                                const Tap& tap = P.taps[t0];
-                                if (do_a)
-                                    tma_load_5d_pair(sa, ta, fb, 0, w0 * P.a_stride_w + tap.dw, h0 * P.a_stride_h + tap.dh, n0,
-                                                     cib0);
-                                if (do_b)
-                                    tma_load_5d_pair(sb, tb, fb, 0, w0, h0, n0,
-                                                     (ntile * P.bn) / P.kb + static_cast<int>(cta_rank) * (P.bn / 2 / P.kb));
-                            } else if (do_a) {
+                            if (do_a) {
                                 if (P.a_grouped) {
                                     const Tap& tap = P.taps[t0];
                                     tma_load_5d(sa, ta, fb, 0, w0 * P.a_stride_w + tap.dw, h0 * P.a_stride_h + tap.dh, n0,

@@ -29,7 +29,7 @@ import torch
 
 from . import _lib
 from ._lib import (NML_F16, NML_F32, NML_MATH_3XTF32, NML_MATH_F16, NML_MATH_TF32, NML_NCHW,
-                   NML_NHWC, ConvDesc, LinearDesc, check)
+                   NML_NHWC, ConvDesc, check)
 
 _MATH = {"f16": NML_MATH_F16, "3xtf32": NML_MATH_3XTF32, "tf32": NML_MATH_TF32}
 _LAYOUT = {"nchw": NML_NCHW, "nhwc": NML_NHWC}
@@ -189,15 +189,6 @@ def conv_backward_weight(g: ConvGeometry, x: torch.Tensor, dy: torch.Tensor, *, 
     into the views of a flat gradient bucket."""
     return _native.conv_backward_weight(g.native(), x, dy, dw, db, _LAYOUT[layout], _MATH[math], 1 if want_bias_grad else 0,
                                         ws or _default_ws)
-
-
-def _linear_desc(rows, fin, fout, in_dtype, out_dtype, w_dtype, math, round_out_f16) -> LinearDesc:
-    d = LinearDesc()
-    d.rows, d.in_features, d.out_features = rows, fin, fout
-    d.in_dtype, d.out_dtype, d.w_dtype = in_dtype, out_dtype, w_dtype
-    d.math = _MATH[math]
-    d.round_out_f16 = int(bool(round_out_f16))
-    return d
 
 
 def linear_forward(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, *, math: str = "f16",

@@ -64,7 +64,6 @@ class ParamStore:
         self.n = 0
         self.p32 = self.p16 = self.grad = self.vel = None
         self.flags = bytearray(2)        # read by the layers' backward: see `accumulate` and `_exchange`
-        self.scratch: Optional[torch.Tensor] = None
         self.layer_ranges: List[Tuple[int, int]] = []   # (first element, end) of every layer, forward order
         self.bucket_bounds: List[int] = []
         self.world = dist.get_world_size() if dist.is_available() and dist.is_initialized() else 1
@@ -110,8 +109,6 @@ class ParamStore:
     def finalize(self, n_buckets: int = 4) -> None:
         mk = lambda dt: torch.zeros(self.n, dtype=dt, device=self.device)
         self.p32, self.p16, self.grad, self.vel = mk(torch.float32), mk(torch.float16), mk(torch.float32), mk(torch.float32)
-        biggest = max(int(torch.tensor(s).prod()) for s in self.shapes)
-        self.scratch = torch.empty(biggest, dtype=torch.float32, device=self.device)
         # buckets: contiguous ranges of the flat gradient, cut at layer boundaries into n_buckets of similar size
         starts = sorted(a for a, _ in self.layer_ranges)
         self.bucket_bounds = [0]
@@ -297,7 +294,7 @@ class _Layer:
         if not s.accumulate:
             run(ga, gb)
         else:
-            ta = s.scratch[:ga.numel()].view(ga.shape)
+            ta = torch.empty_like(ga)
             tb = torch.empty_like(gb) if gb is not None else None
             run(ta, tb)
             ga.add_(ta)

@@ -19,7 +19,7 @@ def test_every_3xtf32_weight_gradient_has_a_plan(lib):
     need = C.c_size_t()
     missing = []
     for k in range(1, 40001):
-        d = ops._linear_desc(32 * k, fin, fout, NML_F32, NML_F32, NML_F32, "3xtf32", False)
+        d = _lib.LinearDesc(32 * k, fin, fout, NML_F32, NML_F32, NML_F32, _lib.NML_MATH_3XTF32, 0)
         assert lib.nml_linear_workspace_size(C.byref(d), NML_PASS_BACKWARD_WEIGHT, C.byref(need)) == _lib.NML_OK
         slices = min(ceil_div(k, 128), 190)
         planes = slices * fout * row_tiles * 128 * 4 if slices > 1 else 0

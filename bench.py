@@ -5,11 +5,13 @@ One "step" = forward + input-gradient + weight-gradient (with bias gradient) of 
 workload, inputs resident in HBM.  The headline workload (`value`) is the Linear projection sweep
 (X[B*T, d] @ W^T[d, 4d] + b for d in {512, 1024, 2048}, B*T in {4096, 16384}; fp16 storage, fp32
 accumulation; synthetic N(0,1) activations, Xavier-uniform weights).  The same JSON line carries,
-under `workloads`, the ResNet-style conv shapes at batch 256, the 16 convolutions of the Pix2Pix
-U-Net generator at batch 64 and the fp32 (3xTF32) Conv2d of configuration 1, each with its own
-roofline block, per-layer table and CPU baseline.  Prints ONE JSON line.
+under `workloads`, the results of the ResNet-style conv shapes at batch 256, the 16 convolutions of
+the Pix2Pix U-Net generator at batch 64, the fp32 (3xTF32) Conv2d of configuration 1 and the two
+training steps.  Prints ONE JSON line on stdout, short enough to be read from the end of a log; the
+full record (per-layer tables, every roofline block, CPU baselines) goes to a file with `--details FILE`.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--workload linear|resnet|pix2pix|config1]
+                    [--details FILE]
 
 N > 1 is launched with torch.distributed.run; every rank owns its own shard of the rows / batch (weak
 scaling: per-GPU work fixed); the weight and bias gradients are written straight into flat fp32
@@ -607,6 +609,43 @@ def measure_train(kind, args, peaks, sampler, torch, dist, dev, rank, world):
                     "counts only the Conv2d / ConvTranspose2d / Linear passes' algorithmic FLOPs over the whole step time"}
 
 
+LINE_LIMIT = 2600  # characters of the JSON line on stdout
+
+
+def _short(v):
+    """Six significant digits are more than any of these measurements has."""
+    if isinstance(v, float):
+        return float(f"{v:.6g}")
+    if isinstance(v, dict):
+        return {k: _short(x) for k, x in v.items()}
+    return [_short(x) for x in v] if isinstance(v, (list, tuple)) else v
+
+
+def summary(record):
+    """The record's line: the headline workload without its per-layer table, one result per other workload."""
+    pick = lambda d, *keys: {k: d[k] for k in keys if d.get(k) is not None}  # noqa: E731
+    cut = {"roofline": ("bound", "achieved", "peak", "unit", "frac", "peak_source", "traffic", "algorithmic_bytes_per_launch"),
+           "sustained": ("value", "ms_per_step", "frac_of_sustained_peak"), "cpu_baseline": ("value", "unit", "cores", "kind"),
+           "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"),
+           "e2e_all_results": ("value", "d2h_bytes_per_step"), "clocks": ("sm_mhz", "sm_max_mhz", "reasons", "samples")}
+    line = {}
+    for key, v in record.items():
+        if key in cut:
+            line[key] = pick(v, *cut[key]) if v else v
+        elif key == "workloads":
+            line[key] = {name: dict(pick(w, "value", "unit", "ms_per_step"), **pick(w.get("roofline") or {}, "frac")) for name, w in v.items()}
+        elif key not in ("per_layer", "detail"):
+            line[key] = v
+    return _short(line)
+
+
+def emit(record, details):
+    if details:
+        with open(details, "w") as f:
+            f.write(json.dumps(record) + "\n")
+    print(json.dumps(summary(record)), flush=True)
+
+
 def pin_to_gpu_numa_node(index: int):
     """Binds this process to the CPUs NVML lists as local to GPU `index` (a read-only NVML query), so that the
     pinned host buffers of the end-to-end leg are allocated on, and driven from, the GPU's own NUMA node.
@@ -660,13 +699,13 @@ def run_gpu(args):
         if sampler:
             sampler.stop()
         if rank == 0:
-            print(json.dumps({"metric": "conv-net train img/s", "value": r["value"], "unit": "img/s", "n_gpus": world,
+            emit({"metric": "conv-net train img/s", "value": r["value"], "unit": "img/s", "n_gpus": world,
                               "steps": r["steps"], "warmup": 2, "ms_per_step": r["ms_per_step"], "higher_is_better": True,
                               "scaling": "strong", "vs_baseline": None, "dtype": "f16 (fp32 accumulate, fp32 master weights)",
                               "data": "synthetic", "impl": "nectarml_b200",
                               "config": {"workload": TRAIN_NAMES[args.workload], "global_batch": r["global_batch"],
                                          "parallelism": f"dp{world}" if world > 1 else "1 GPU"},
-                              "e2e": None, "gpu_launches": r["gpu_launches"], "clocks": r["clocks"], "detail": r}), flush=True)
+                              "e2e": None, "gpu_launches": r["gpu_launches"], "clocks": r["clocks"], "detail": r}, args.details)
         if world > 1:
             dist.barrier()
             dist.destroy_process_group()
@@ -789,8 +828,8 @@ def run_gpu(args):
                                        f"NCCL_MAX_CTAS={os.environ.get('NCCL_MAX_CTAS')}, {head['sm_reserve']} SMs left to it while in flight)")
                        if world > 1 else "1 GPU",
                        "host_cpus_bound": numa, "launch": head["launch"],
-                       "l2": "inputs and outputs of one step exceed the 126 MB L2 several times over; every step cycles through it",
-                       "timing": f"every timed region is a burst of `steps` steps from an idle GPU ({args.idle_s} s pause); `sustained` is the same step for >= {args.sustain_s} s"},
+                       "l2": "inputs and outputs of one step exceed the 126 MB L2 several times over",
+                       "timing": f"burst of `steps` steps from an idle GPU ({args.idle_s} s pause); `sustained`: the same step for >= {args.sustain_s} s"},
             "e2e": e2e, "e2e_all_results": e2e_legs.get("e2e_all_results") if e2e else None, "gpu_launches": head["gpu_launches"], "clocks": head["clocks"], "roofline": head["roofline"],
             "per_layer": head.get("per_layer"),
         }
@@ -802,7 +841,7 @@ def run_gpu(args):
             out["workloads"] = others
         if world == 1 and not args.no_cpu_baseline:
             out["cpu_baseline"] = cpu_baseline(args.workload, budget_s=12.0)
-        print(json.dumps(out), flush=True)
+        emit(out, args.details)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
@@ -926,6 +965,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--cpu-budget", type=float, default=0.0,
                     help="seconds of CPU work per step of the reference arm (default: sized from --steps)")
+    ap.add_argument("--details", default="", help="file for the full record (per-layer tables, roofline blocks)")
     ap.add_argument("--only", default="", help="profiling aid: restrict the linear sweep to ROWSxD, or a conv sweep to the layer with this index")
     args = ap.parse_args()
     if args.impl == "reference":

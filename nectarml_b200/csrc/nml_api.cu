@@ -92,8 +92,9 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_WTRANS   0: Linear input-gradients never take a transposed copy of the weights
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
 //   NML_TUNE_NARROW   0: few-channel layers always take eight channels per pixel
+//   NML_TUNE_DOUBLE   0: no double tiles, 2: wherever they are legal
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow, dbl;
 };
 static const Tune& tune() {
     static Tune t;
@@ -118,6 +119,7 @@ static const Tune& tune() {
         t.wtrans = env("NML_TUNE_WTRANS", 1);
         t.pair128 = env("NML_TUNE_PAIR128", 1);
         t.narrow = env("NML_TUNE_NARROW", 1);
+        t.dbl = env("NML_TUNE_DOUBLE", 1);
     });
     return t;
 }
@@ -192,6 +194,8 @@ static UmmaKernel fprop_instance(bool f16) {
     return f16 ? umma_conv_kernel<MODE_FPROP, kOut, true, kPair> : umma_conv_kernel<MODE_FPROP, kOut, false, kPair>;
 }
 static UmmaKernel kernel_for(const KParams& P) {
+    if (P.dbl)
+        return P.mode == MODE_WGRAD ? umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true> : umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>;
     if (P.mode == MODE_WGRAD)
         return P.pair ? umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true> : umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>;
     const bool h = P.out_f16 != 0;
@@ -206,7 +210,8 @@ static UmmaKernel kernel_for(const KParams& P) {
     return fprop_instance<OUT_NCHW, false>(h);
 }
 static int raise_smem_limit() {
-    UmmaKernel all[16] = {umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true>,
+    UmmaKernel all[18] = {umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
+                          umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true>,
                           fprop_instance<OUT_NHWC_TMA, false>(true), fprop_instance<OUT_NHWC_TMA, false>(false),
                           fprop_instance<OUT_NCHW_TMA, false>(true), fprop_instance<OUT_NCHW_TMA, false>(false),
                           fprop_instance<OUT_NHWC, false>(true), fprop_instance<OUT_NHWC, false>(false),
@@ -587,10 +592,11 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     // take two slices per stage (8 MMAs per round trip); 256-wide tiles already fill 512 clocks.
     // The 3xTF32 split takes one slice: its two planes are 12 MMAs.
     P.ka = P.planes == 2 ? 2 : (P.pair && P.bn == 256) ? 1 : std::max(1, std::min(2, tune().ka ? tune().ka : (P.bn >= 192 ? 1 : 2)));
-    const int stage_bytes = P.ka * (kStageABytes + (P.pair ? P.bn / 2 : P.bn) * 128);
+    if (P.dbl) P.ka = 1;
+    const int stage_bytes = P.ka * ((P.dbl ? 2 : 1) * kStageABytes + (P.pair ? P.bn / 2 : P.bn) * 128);
     // Shared memory: the operand ring, then the epilogue's staging buffers (two per warp if that does not
     // cost a ring stage, else one), the per-warp bias tiles, and the barriers.
-    const int fixed = kFixedSmem;
+    const int fixed = kFixedSmem - (P.dbl ? kBiasTileBytes : 0);
     const bool tma_out = (P.mode == MODE_FPROP) && NML_IS_TMA_OUT(P.out_mode);
     // A second group of four epilogue warps (TMA-store instances only) where a tile's drain outlasts its MMAs.  Clocks,
     // measured: one group needs ~800 per tile plus ~900 per 128-byte piece; four MMAs (one K slice) take 192 at 64 columns
@@ -599,7 +605,9 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     const int ctas = P.pair ? limited(ds->sms) / 2 : limited(ds->sms);
     P.epi_warps = 4;
     P.epi_alt = 0;
-    if (tma_out && tune().epi8) {
+    if (P.dbl) {
+        P.epi_warps = 8;
+    } else if (tma_out && tune().epi8) {
         int k_slices = 0;  // longest phase
         for (int p = 0; p < P.n_phases; ++p) k_slices = std::max(k_slices, P.c_blocks * P.phases[p].tap_count);
         const int pieces = ceil_div(P.bn, P.out_f16 ? 64 : 32);
@@ -610,7 +618,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         }
     }
     P.tbufs_log2 = 0;
-    while (P.tbufs_log2 < (P.epi_alt ? 2 : 1) && ((2 * P.bn * P.planes) << P.tbufs_log2) <= 512) ++P.tbufs_log2;
+    while (P.tbufs_log2 < (P.epi_alt ? 2 : 1) && ((2 * P.bn * P.planes * (P.dbl ? 2 : 1)) << P.tbufs_log2) <= 512) ++P.tbufs_log2;
     size_t smem;
     if (P.wpatch) {
         // [stages x (patch, box of the other tensor)][staging (unused by this walk)][bias][barriers]
@@ -650,9 +658,11 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         P.ring_bytes = P.a_ring_off + P.a_stages * P.patch_bytes;
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
     } else {
-    int stages2 = (232448 - fixed - P.epi_warps * 2 * kStagingBufBytes) / stage_bytes;
-    int stages1 = (232448 - fixed - P.epi_warps * 1 * kStagingBufBytes) / stage_bytes;
-    P.stg_bufs = (stages2 >= std::min(stages1, 8)) ? 2 : 1;
+    // (a double tile's warps have one buffer each, or none where they store from registers)
+    int stages2 = P.dbl ? 0 : (232448 - fixed - P.epi_warps * 2 * kStagingBufBytes) / stage_bytes;
+    const int bufs1 = P.dbl && !tma_out ? 0 : 1;
+    int stages1 = (232448 - fixed - P.epi_warps * bufs1 * kStagingBufBytes) / stage_bytes;
+    P.stg_bufs = (stages2 >= std::min(stages1, 8)) ? 2 : bufs1;
     int stages = std::min(8, P.stg_bufs == 2 ? stages2 : stages1);
     stages = std::max(2, std::min(stages, tune().stages));
     P.stages = stages;
@@ -675,7 +685,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     if (rec && !pre_opened) NML_CUDA(cudaEventRecord(g_prof.start[rec_slot], st));
     // (under an SM limit not before its predecessor has ended: blocks that wait would sit on the SMs that are to stay free, and
     // a block of this kernel leaves no room beside it)
-    launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st, P);
+    launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, P.dbl ? kThreadsWide : threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st, P);
     NML_CUDA(cudaGetLastError());
     if (open_slot) *open_slot = rec_slot;
     else if (rec) NML_CUDA(cudaEventRecord(g_prof.stop[rec_slot], st));
@@ -686,6 +696,46 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
 // Microseconds one 128-byte-deep K slice of a 128-row tile keeps an SM busy, by tile width: 512 clocks of MMA at 256
 // columns; narrower tiles cost more per column (measured: 1.28x at 128, 2.24x at 64).
 static double slice_us(int bn) { return 0.27 * (bn / 256.0) * (bn > 128 ? 1.0 : bn > 64 ? 1.28 : 2.24); }
+
+// Double tiles (see umma_conv_kernel): clocks of a K slice of a pair's tile, one row tile high and two, and what a 256-column
+// double tile adds, whose drain nothing overlaps.  Measured on Linear layers: 16384 x 512 -> 2048 (8 slices, 7 rounds of single
+// tiles, 4 of double ones) 36.9 us single, 44.3 double; 16384 x 1024 -> 4096 (16; 14 and 7) 110.6 and 116.4; 16384 x 2048 -> 8192
+// (32; 28 and 14) 408 and 383; its input gradient (128 slices, 7 rounds of single tiles; three double ones and a single
+// one) 421 and 384; 4096 x 2048 -> 8192's (64 tiles in one round of double ones) 123 and 98.
+struct PairCost {
+    double one, two, drain;
+};
+static PairCost pair_cost(int bn) { return bn == 256 ? PairCost{575.0, 1060.0, 2000.0} : PairCost{430.0, 690.0, 0.0}; }
+// The plan of a launch of `rows` x n_tiles pair tiles of k slices on `units` pairs: 0 double rows, all of them (INT_MAX), or as
+// many as fill whole rounds, with single tiles behind them where their last round would be half empty.
+static int plan_double_rows(int rows, int n_tiles, int k, int bn, int units, bool may_mix) {
+    if (tune().dbl == 0) return 0;
+    if (tune().dbl == 2) return may_mix && rows > 2 ? (rows / 2 + 1) / 2 : INT_MAX;
+    const PairCost c = pair_cost(bn);
+    const double one = k * c.one, two = k * c.two + c.drain;
+    const long long single = 1ll * rows * n_tiles, dbl = 1ll * ((rows + 1) / 2) * n_tiles;
+    const double all_single = static_cast<double>((single + units - 1) / units) * one;
+    const double all_double = static_cast<double>((dbl + units - 1) / units) * two;
+    double best = all_single * 0.985;
+    int plan = 0;
+    if (all_double < best) {
+        best = all_double;
+        plan = INT_MAX;
+    }
+    if (may_mix) {
+        const int big_rows = static_cast<int>(dbl / units * units / n_tiles);
+        const long long big = 1ll * big_rows * n_tiles, total = big + 1ll * (rows - 2 * big_rows) * n_tiles;
+        if (big_rows > 0 && rows > 2 * big_rows) {
+            double cost = 0;
+            for (const long long j : {0ll, big % units}) {  // the first pair, and the first with one double tile less
+                const long long b = (big - j + units - 1) / units, t = (total - j + units - 1) / units;
+                cost = std::max(cost, b * two + (t - b) * one);
+            }
+            if (cost < best) plan = big_rows;
+        }
+    }
+    return plan;
+}
 
 // ------------------------------------------------------- fprop-like problems --
 struct FpropLike {
@@ -1225,6 +1275,17 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     const bool pair_k = k_iters_min >= 12 || (k_iters_min >= 5 && tiles_single > 2ll * limited(ds->sms));
     P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && pair_k &&
               (P.out_mode == OUT_NHWC_TMA || P.out_mode == OUT_NCHW_TMA || P.out_mode == OUT_NCHW) && limited(ds->sms) >= 2) ? 1 : 0;
+    // Double tiles: pairs that write fp16 rows by TMA stores.  The phases of a gather are planned by their sum.
+    if (P.pair && P.out_mode == OUT_NHWC_TMA && P.out_f16 && P.planes == 1 && (P.bn == 256 || P.bn == 128)) {
+        int rows = 0, slices = 0;
+        for (int p = 0; p < n_phases; ++p) {
+            rows += ceil_div(ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) * ceil_div(f.batch, 1 << P.nb_log2), 2);
+            slices += P.c_blocks * P.phases[p].tap_count;
+        }
+        P.big_rows = plan_double_rows(rows, P.n_tiles, slices / n_phases, P.bn, limited(ds->sms) / 2, n_phases == 1);
+        P.dbl = P.big_rows > 0 ? 1 : 0;
+        P.big_tiles = P.big_rows == INT_MAX ? INT_MAX : P.big_rows * P.n_tiles;
+    }
     int tiles = 0;
     for (int p = 0; p < n_phases; ++p) {
         Phase& ph = P.phases[p];
@@ -1232,7 +1293,9 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         ph.tiles_h = ceil_div(ph.hq, 1 << P.hb_log2);
         ph.tile_begin = tiles;
         int m_tiles = ph.tiles_w * ph.tiles_h * ceil_div(f.batch, 1 << P.nb_log2);
-        tiles += (P.pair ? ceil_div(m_tiles, 2) : m_tiles) * P.n_tiles;
+        if (P.pair) m_tiles = ceil_div(m_tiles, 2);
+        if (P.dbl) m_tiles = P.big_rows == INT_MAX ? ceil_div(m_tiles, 2) : m_tiles - P.big_rows;
+        tiles += m_tiles * P.n_tiles;
     }
     P.num_tiles = tiles;
     P.base_tiles = tiles;
@@ -1246,8 +1309,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             ph.mul_h = reciprocal(ph.tiles_h);
             dmax = std::max<long long>(dmax, std::max(ph.tiles_w, ph.tiles_h));
         }
-        // (a pair doubles the row-tile index before it is divided)
-        P.fastdiv = (2ll * (tiles + 1) * dmax < (1ll << 32)) ? 1 : 0;
+        // (a pair doubles the row-tile index before it is divided, a double tile once more)
+        P.fastdiv = ((P.dbl ? 4ll : 2ll) * (tiles + 1) * dmax < (1ll << 32)) ? 1 : 0;
     }
     P.fsplit = 1;
     if (z_plan >= 2) {
@@ -1384,6 +1447,11 @@ struct WgradLike {
     int colsum_of_patch;
     int math;
 };
+
+// Microseconds of a K block (64 pixels) of a double 256-column pair tile, and of its prologue and drain (256 KB of fp32 per SM,
+// all SMs at once).  Measured: 16384 x 2048 -> 8192, 256 blocks, four rounds of single tiles 468 us, two of double ones 422;
+// transposed 4x4 512 -> 128 at 32 x 32, batch 64 110 -> 99; but 16384 x 512 -> 2048 cut into nine slices of 29 blocks 48 -> 52.
+constexpr double kDoubleBlockUs = 0.57, kDoubleTileUs = 8.0;
 
 static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     MathInfo mi;
@@ -1530,6 +1598,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     const bool b_grp = (cpb % mi.kb == 0);
     const int row_tiles = ceil_div(P.groups_total * mi.kb, kTileM);
     int split = 1, m_tiles = 1;
+    long long launch_tiles = 0;
     if (!P.wpatch) {
         const double dw_us = 4.0 * g.plain_c * g.patch_c * T / 8e6;  // one pass over dW at 8 TB/s
         // at most 192 slices, as many as leave each at least one block (a count that the loop below does not pass over, so
@@ -1553,27 +1622,49 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                 // as the most slices leave
                 if (P.planes == 2 && per_sp * mi.kb > 4096 && sp < max_split) continue;
                 const double block_us = (pair ? (tiles * 8 >= units * 7ll ? 0.41 : 0.36) : 0.32) * (P.planes == 2 ? 2.3 : 1.0);
-                const double rounds = static_cast<double>((tiles + units - 1) / units);
-                double cost = rounds * (per_sp * block_us + 1.0 + bn / 128.0);
-                if (sp > 1 || T > 1) cost += 2.5 + (2.0 * sp + 1.0) * dw_us * (sp * dw_us > 8.0 ? 1.6 : 1.0);
-                if (best < 0 || cost < best * (width == 256 ? 1.0 : 0.98)) {
-                    best = cost;
+                const double tile_us = per_sp * block_us + 1.0 + bn / 128.0;
+                const double reduce_us = sp > 1 || T > 1 ? 2.5 + (2.0 * sp + 1.0) * dw_us * (sp * dw_us > 8.0 ? 1.6 : 1.0) : 0.0;
+                const auto rounds = [&](long long n) { return static_cast<double>((n + units - 1) / units); };
+                const auto consider = [&](double us, int big_rows, long long n, int rows) {
+                    if (best >= 0 && us >= best * (width == 256 ? 1.0 : 0.98)) return;
+                    best = us;
                     split = sp;
-                    m_tiles = mt;
+                    m_tiles = rows;
+                    launch_tiles = n;
                     P.n_tiles = nt;
                     P.bn = bn;
                     P.pair = pair ? 1 : 0;
+                    P.big_rows = big_rows;
+                };
+                if (tune().dbl != 2 || !pair || P.planes == 2) consider(rounds(tiles) * tile_us + reduce_us, 0, tiles, mt);
+                // double tiles, with single ones behind them where K is whole (for 3 % and more)
+                if (pair && P.planes == 1 && tune().dbl) {
+                    const double double_us = per_sp * kDoubleBlockUs + kDoubleTileUs;
+                    const int rows2 = ceil_div(mt, 2);
+                    const long long dbl = 1ll * rows2 * nt * sp;
+                    consider((rounds(dbl) * double_us + reduce_us) * 1.03, INT_MAX, dbl, 2 * rows2);
+                    const int big_rows = tune().dbl == 2 ? (mt / 2 + 1) / 2 : static_cast<int>(dbl / units * units / nt);
+                    if (sp == 1 && big_rows > 0 && mt > 2 * big_rows) {
+                        const long long big = 1ll * big_rows * nt, total = big + 1ll * (mt - 2 * big_rows) * nt;
+                        double us = 0;
+                        for (const long long j : {0ll, big % units}) {  // the first pair, and the first with one double tile less
+                            const double b = rounds(big - j), t = rounds(total - j);
+                            us = std::max(us, b * double_us + (t - b) * tile_us);
+                        }
+                        consider((us + reduce_us) * 1.03, big_rows, total, mt);
+                    }
                 }
             }
         }
     }
-    const int mn_tiles = m_tiles * P.n_tiles;
+    P.dbl = P.big_rows > 0 ? 1 : 0;
+    P.big_tiles = P.big_rows == INT_MAX ? INT_MAX : P.big_rows * P.n_tiles;
     if (P.wpatch) {  // one tile per CTA, no empty slice
         split = std::max(1, std::min(P.kblocks_total, sms / std::max(1, P.n_tiles)));
         split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, split));
     }
     P.split_k = split;
-    P.num_tiles = mn_tiles * split;
+    P.num_tiles = P.wpatch ? P.n_tiles * split : static_cast<int>(launch_tiles);
     // One K slice of a one-tap layer writes dW itself.  With several taps the rows of a tile are 4 * taps bytes apart in dW
     // (a store instruction would touch 32 sectors: 4x4 512->512 on 4x4 images took 29 us for its 17 MB of gradient), so
     // they go through a plane even when there is one slice.  Several slices store their partial sums into one fp32 plane each

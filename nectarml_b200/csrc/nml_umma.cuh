@@ -92,6 +92,9 @@ struct KParams {
     int epi_warps;       // 4, or 8 on the TMA-store instances when the epilogue is the critical path
     int epi_alt;         // 8 warps: 1 = the two groups take alternate tiles, 0 = each takes half the columns of every tile
     int pair;            // 1: launched as clusters of two CTAs sharing 256x256 tiles (cta_group::2)
+    // Double tiles (a pair instance of their own, see the kernel's comment): rows [0, big_rows) of the tile grid (per phase /
+    // K slice) are two row tiles high, the rows behind them one; big_tiles = big_rows * n_tiles.
+    int dbl, big_rows, big_tiles;
     int stg_bufs;        // staging buffers per epilogue warp (4 KB each): 2 when shared memory allows, else 1
     int ka;              // K atoms (128-byte-wide operand slices, times planes) per stage; narrow tiles take 2 to amortise
                          // the per-stage barrier round trip over 8 MMAs
@@ -187,11 +190,13 @@ struct KParams {
 // mul = floor(2^32 / d) + 1, or 0 for d = 1.  Exact for x * d < 2^32 (the host checks).
 __device__ __forceinline__ uint32_t fast_div(uint32_t x, uint32_t mul) { return mul ? __umulhi(x, mul) : x; }
 // Forward walk: tile index within its phase -> column tile and the (w, h, n) position of the row tile.
-template <bool kPair>
+// half: which of a double tile's two row tiles.
+template <bool kPair, bool kDbl = false>
 __device__ __forceinline__ void decode_fprop_tile(const KParams& P, const Phase& ph, int local, uint32_t cta_rank,
-                                                  int& ntile, int& tw, int& th, int& tn) {
+                                                  int& ntile, int& tw, int& th, int& tn, int half = 0) {
     uint32_t m = P.fastdiv ? fast_div(local, P.mul_nt) : static_cast<uint32_t>(local) / P.n_tiles;
     ntile = local - static_cast<int>(m) * P.n_tiles;
+    if (kDbl) m = static_cast<int>(m) < P.big_rows ? 2 * m + half : m + P.big_rows;
     if (kPair) m = 2 * m + cta_rank;  // the pair's two row tiles
     const uint32_t q = P.fastdiv ? fast_div(m, ph.mul_w) : m / ph.tiles_w;
     tw = static_cast<int>(m - q * ph.tiles_w);
@@ -200,8 +205,24 @@ __device__ __forceinline__ void decode_fprop_tile(const KParams& P, const Phase&
     tn = static_cast<int>(n);
 }
 
-// Tile id -> (column tile, row tile, K slice) of a weight-gradient launch.
-__device__ __forceinline__ void decode_wgrad_tile(const KParams& P, int tile, int m_tiles, int& ntile, int& mt, int& z) {
+// Tile id -> (column tile, row tile, K slice) of a weight-gradient launch.  Rows are row tiles, pairs of them where CTAs are paired.
+// -> row tiles (or pairs) of the tile: 2 of a double one.
+template <bool kPair, bool kDbl>
+__device__ __forceinline__ int decode_wgrad_tile(const KParams& P, int tile, int& ntile, int& mt, int& z) {
+    int m_tiles = (P.groups_total * P.kb + kTileM - 1) / kTileM;
+    if (kPair) m_tiles = (m_tiles + 1) / 2;
+    int halves = 1, first = 0;
+    z = 0;
+    if (kDbl) {
+        if (tile >= P.big_tiles) {  // (one K slice)
+            tile -= P.big_tiles;
+            first = 2 * P.big_rows;
+            m_tiles -= first;
+        } else {
+            m_tiles = min(P.big_rows, (m_tiles + 1) / 2);
+            halves = 2;
+        }
+    }
     const int mn = m_tiles * P.n_tiles;
     z = tile / mn;
     const int r = tile - z * mn;
@@ -212,6 +233,8 @@ __device__ __forceinline__ void decode_wgrad_tile(const KParams& P, int tile, in
         mt = r / P.n_tiles;
         ntile = r - mt * P.n_tiles;
     }
+    mt = mt * halves + first;
+    return halves;
 }
 
 __device__ __forceinline__ float round_through_f16(float v) {
@@ -263,8 +286,16 @@ __device__ __forceinline__ void store_columns(T* o, size_t stride, const uint32_
 // kPair: two CTAs of a cluster compute one 256-row x 256-column tile with cta_group::2 MMAs issued by
 // the rank-0 CTA; each CTA loads its own 128 rows of A and its own 128-column half of B (no multicast),
 // which halves the B traffic and the MMA issue cost per SM and leaves room for 6 stages.
-template <int kMode, int kOutMode, bool kOutF16, bool kPair>
-__global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(const __grid_constant__ KParams P) {
+// kDbl: a pair's tile is two row tiles high (512 x bn), two accumulators that share every B slice.  An SM takes in at most 64
+// bytes a clock from L2 (TMA loads of any shape: 18.9 TB/s over 148 SMs, wherever the lines are shared), and a 256-column pair
+// tile wants 32 KB per K slice of 512 clocks, all of it: a slice takes 570 to 700 clocks.  A double tile wants 48 KB per 1024
+// clocks and takes 1045 to 1060 (Linear; convolutions, whose slices arrive in more pieces, 720 and 1350).  At 256 columns the two
+// accumulators fill TMEM, so nothing overlaps the drain: the epilogue takes a tile into registers as fp16 and hands the
+// accumulators back before it stores anything, one group of four warps to a row tile.
+template <int kMode, int kOutMode, bool kOutF16, bool kPair, bool kDbl = false>
+__global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1) umma_conv_kernel(const __grid_constant__ KParams P) {
+    static_assert(!kDbl || kPair, "double tiles are tiles of CTA pairs");
+    constexpr int kRowTiles = kDbl ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     // stages need 1024-byte alignment for the 128-byte swizzle pattern
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -274,12 +305,12 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     const int tile_first = kPair ? (blockIdx.x >> 1) : blockIdx.x;
     const int tile_step = kPair ? (gridDim.x >> 1) : gridDim.x;
     const int stage_b_bytes = (kPair ? P.bn / 2 : P.bn) * P.b_row_bytes;   // one atom of B (a pair member holds half the columns)
-    const int stage_bytes = P.ka * (kStageABytes + stage_b_bytes);  // [A atoms][B atoms]
-    const int b_off = P.ka * kStageABytes;                        // first B atom within a stage
+    const int b_off = P.ka * kRowTiles * kStageABytes;            // first B atom within a stage
+    const int stage_bytes = b_off + P.ka * stage_b_bytes;         // [A atoms][B atoms]
     uint8_t* staging = smem + P.ring_bytes;  // epilogue warps x 4 KB
     const int staging_bytes = P.epi_warps * P.stg_bufs * kStagingBufBytes;
     float* bias_tile = reinterpret_cast<float*>(staging + staging_bytes);
-    uint8_t* ctrl = staging + staging_bytes + kBiasTileBytes;
+    uint8_t* ctrl = staging + staging_bytes + (kDbl ? 0 : kBiasTileBytes);  // (double tiles keep bias values in the staging buffers)
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(ctrl);          // [stages]
     uint64_t* empty_bar = full_bar + 8;                               // [stages]
     uint64_t* tfull_bar = empty_bar + 8;                              // [4]
@@ -294,7 +325,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     // two accumulators; the epilogue reads 32 columns at a time, so a 16-column tile still needs 16 + 32
-    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : (P.bn * P.planes) << P.tbufs_log2;
+    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : (P.bn * P.planes * kRowTiles) << P.tbufs_log2;
     const uint32_t tmem_cols = (tmem_need <= 32) ? 32 : (tmem_need <= 64) ? 64 : (tmem_need <= 128) ? 128
                                : (tmem_need <= 256) ? 256 : 512;
 
@@ -442,8 +473,128 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         }
     };
 
+    // A producer that gave up: copies already issued get a bounded chance to land before the CTA's shared memory goes away.
+    auto drain_ring = [&](int s, uint32_t par, int issued) {
+        for (int back = issued < P.stages ? issued : P.stages; back > 0; --back) {
+            if (--s < 0) {
+                s = P.stages - 1;
+                par ^= 1;
+            }
+            uint64_t t0 = globaltimer_ns();
+            while (!mbar_try_wait(smem_u32(&full_bar[s]), par)) {
+                if (globaltimer_ns() - t0 > 2000000ull) {
+                    atomicCAS(P.err, 0, ERR_WAIT_DRAIN);
+                    break;
+                }
+            }
+        }
+    };
+
     // ------------------------------------------------------------ producer --
-    if (warp == 0 || warp == 6) {
+    if (kDbl && (warp == 0 || warp == 6)) {
+        // Double tiles: one K slice per stage, one thread per operand, whose loop carries nothing but counters (a K slice
+        // lasts about 1024 clocks, an iteration with its wait 300 and more).
+        if (lane == 0) {
+            const bool do_a = (warp == 0);
+            int stage = 0;
+            uint32_t parity = 0;
+            bool ok = true;
+            int issued = 0;
+            // every load signals the LEADER's barrier, which expects both members' bytes
+            const uint32_t full0 = smem_u32(full_bar), empty0 = smem_u32(empty_bar);
+            const uint32_t signal0 = map_to_cta(full0, 0);
+            const uint32_t dst0 = smem_u32(smem) + (do_a ? 0 : b_off);
+            // waits for the stage and announces this producer's bytes
+            auto open_stage = [&](uint32_t bytes) -> bool {
+                ok = mbar_wait(empty0 + 8 * stage, parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY);
+                if (ok && leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * bytes);
+                return ok;
+            };
+            auto next_stage = [&]() {
+                ++issued;
+                if (++stage == P.stages) {
+                    stage = 0;
+                    parity ^= 1;
+                }
+            };
+            for (int tile = tile_first; ok && tile < P.num_tiles; tile += tile_step) {
+                if (kMode == MODE_FPROP) {
+                    int p = 0;
+                    while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
+                    const Phase& ph = P.phases[p];
+                    const int local = tile - ph.tile_begin;
+                    const bool two = local < P.big_tiles;
+                    int ntile, tw, th, tn;
+                    int w0[2], h0[2], n0[2];  // boxes of the row tiles
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        decode_fprop_tile<kPair, kDbl>(P, ph, local, cta_rank, ntile, tw, th, tn, h);
+                        w0[h] = (tw << P.wb_log2) * P.a_stride_w;
+                        h0[h] = (th << P.hb_log2) * P.a_stride_h;
+                        n0[h] = tn << P.nb_log2;
+                    }
+                    const int ncol = ntile * P.bn + static_cast<int>(cta_rank) * (P.bn / 2);  // this member's half of B
+                    const uint32_t bytes = do_a ? (two ? 2 : 1) * kStageABytes : stage_b_bytes;
+                    for (int t = ph.tap_begin; ok && t < ph.tap_begin + ph.tap_count; ++t) {
+                        const int dw = P.taps[t].dw, dh = P.taps[t].dh, wk = P.taps[t].wk;
+                        for (int c = 0; c < P.c_blocks * P.kb; c += P.kb) {
+                            if (!open_stage(bytes)) break;
+                            const uint32_t dst = dst0 + stage * stage_bytes, signal = signal0 + 8 * stage;
+                            if (do_a) {
+                                tma_load_4d_pair(dst, &P.tmA[0], signal, c, w0[0] + dw, h0[0] + dh, n0[0]);
+                                if (two) tma_load_4d_pair(dst + kStageABytes, &P.tmA[0], signal, c, w0[1] + dw, h0[1] + dh, n0[1]);
+                            } else if (!P.b_mn_major) {
+                                tma_load_2d_pair(dst, &P.tmB[0], signal, wk + c, ncol);
+                            } else {
+                                tma_load_3d_pair(dst, &P.tmB[0], signal, 0, wk + c, ncol / P.kb);
+                            }
+                            next_stage();
+                        }
+                    }
+                } else {
+                    int ntile, mt, z;
+                    const int halves = decode_wgrad_tile<kPair, kDbl>(P, tile, ntile, mt, z);
+                    const int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
+                    const int kb_begin = z * per, kb_end = min(kb_begin + per, P.kblocks_total);
+                    int tw = kb_begin % P.ktiles_w;
+                    int th = (kb_begin / P.ktiles_w) % P.ktiles_h;
+                    int tn = kb_begin / (P.ktiles_w * P.ktiles_h);
+                    int a_dw[2], a_dh[2], a_c[2];  // tap and channel group of the row tiles (the partner's first lies between them)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int g = min((2 * (mt + h) + static_cast<int>(cta_rank)) * (kTileM / P.kb), P.groups_total - 1);
+                        const int t = g / P.c_blocks;
+                        a_dw[h] = P.taps[t].dw;
+                        a_dh[h] = P.taps[t].dh;
+                        a_c[h] = g - t * P.c_blocks;
+                    }
+                    const int b_group = (ntile * P.bn) / P.kb + static_cast<int>(cta_rank) * (P.bn / 2 / P.kb);
+                    const uint32_t bytes = do_a ? halves * kStageABytes : stage_b_bytes;
+                    for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
+                        if (!open_stage(bytes)) break;
+                        const uint32_t dst = dst0 + stage * stage_bytes, signal = signal0 + 8 * stage;
+                        const int w = tw << P.wb_log2, h = th << P.hb_log2, n = tn << P.nb_log2;
+                        if (do_a) {
+                            const int wa = w * P.a_stride_w, ha = h * P.a_stride_h;
+                            tma_load_5d_pair(dst, &P.tmA[0], signal, 0, wa + a_dw[0], ha + a_dh[0], n, a_c[0]);
+                            if (halves == 2) tma_load_5d_pair(dst + kStageABytes, &P.tmA[0], signal, 0, wa + a_dw[1], ha + a_dh[1], n, a_c[1]);
+                        } else {
+                            tma_load_5d_pair(dst, &P.tmB[0], signal, 0, w, h, n, b_group);
+                        }
+                        next_stage();
+                        if (++tw == P.ktiles_w) {
+                            tw = 0;
+                            if (++th == P.ktiles_h) {
+                                th = 0;
+                                ++tn;
+                            }
+                        }
+                    }
+                }
+            }
+            if (!ok) drain_ring(stage, parity, issued);
+        }
+    } else if (warp == 0 || warp == 6) {
         const bool do_a = (warp == 0), do_b = (warp == 6);
         // Issuing one TMA keeps its thread busy for ~300 clocks, more than the MMAs of a narrow K atom last.
         // The atoms of a stage are therefore issued by one lane each, in the same instruction (patches, one box per
@@ -675,10 +826,8 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                         }
                     }
                 } else {  // MODE_WGRAD
-                    int m_tiles = (P.groups_total * P.kb + kTileM - 1) / kTileM;
-                if (kPair) m_tiles = (m_tiles + 1) / 2;  // tile ids name pairs of row tiles
                     int ntile, mt, z;
-                    decode_wgrad_tile(P, tile, m_tiles, ntile, mt, z);
+                    decode_wgrad_tile<kPair, false>(P, tile, ntile, mt, z);
                     if (kPair) mt = 2 * mt + static_cast<int>(cta_rank);
                     int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
                     int kb_begin = z * per;
@@ -799,26 +948,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     }
                 }
             }
-            if (!ok && lane == 0) {
-                // Unwinding: give copies already issued a bounded chance to land before the
-                // CTA's shared memory goes away.
-                int back = issued < P.stages ? issued : P.stages;
-                int s = stage;
-                uint32_t par = parity;
-                for (int i = 0; i < back; ++i) {
-                    if (--s < 0) {
-                        s = P.stages - 1;
-                        par ^= 1;
-                    }
-                    uint64_t t0 = globaltimer_ns();
-                    while (!mbar_try_wait(smem_u32(&full_bar[s]), par)) {
-                        if (globaltimer_ns() - t0 > 2000000ull) {
-                            atomicCAS(P.err, 0, ERR_WAIT_DRAIN);
-                            break;
-                        }
-                    }
-                }
-            }
+            if (!ok && lane == 0) drain_ring(stage, parity, issued);
         }
     }
     // ---------------------------------------------------------- MMA issuer --
@@ -856,20 +986,20 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 kz = tile_id / P.base_tiles;
                 tile = tile_id - kz * P.base_tiles;
             }
-            int k_iters;
+            int k_iters, halves = 1;
             if (kMode == MODE_FPROP) {
                 int p = 0;
                 while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
                 k_iters = P.phases[p].tap_count * P.c_blocks;
+                if (kDbl && tile - P.phases[p].tile_begin < P.big_tiles) halves = 2;
                 if (P.fsplit > 1) {
                     const int per = (k_iters + P.fsplit - 1) / P.fsplit;
                     const int k_first = min(kz * per, k_iters);
                     k_iters = min(k_first + per, k_iters) - k_first;
                 }
             } else {
-                int m_tiles = (P.groups_total * P.kb + kTileM - 1) / kTileM;
-                if (kPair) m_tiles = (m_tiles + 1) / 2;  // tile ids name pairs of row tiles
-                int z = tile / (P.n_tiles * m_tiles);
+                int ntile, mt, z;
+                halves = decode_wgrad_tile<kPair, kDbl>(P, tile, ntile, mt, z);
                 int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
                 int kb_begin = z * per;
                 int kb_end = min(kb_begin + per, P.kblocks_total);
@@ -944,7 +1074,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 break;
             }
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + buf * P.bn * P.planes;  // the split's cross products: bn columns further on
+            const uint32_t d_tmem = tmem_base + buf * P.bn * P.planes * kRowTiles;  // the split's cross products: bn columns further on
             uint32_t acc = 0;
             // one K slice of the 3xTF32 split: hi*lo and lo*hi into the cross accumulator, hi*hi into the main one
             auto issue_split = [&](uint64_t ah, uint64_t al, uint64_t bh, uint64_t bl, uint32_t aa, uint32_t ab) {
@@ -977,6 +1107,18 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     if (P.planes == 2)  // (one slice per stage)
                         issue_split(adesc, adesc + a_atom_step, bdesc, bdesc + b_atom_step, adv_a, adv_b);
                     else
+                    if (kDbl) {  // (fp16, one slice per stage; a double tile's row tiles share its B)
+                        uint32_t d = d_tmem;
+#pragma unroll 1
+                        for (int h = 0; h < halves; ++h) {
+                            umma_f16_pair(d, adesc, bdesc, idesc, first);
+                            umma_f16_pair(d, adesc + adv_a, bdesc + adv_b, idesc, 1u);
+                            umma_f16_pair(d, adesc + 2 * adv_a, bdesc + 2 * adv_b, idesc, 1u);
+                            umma_f16_pair(d, adesc + 3 * adv_a, bdesc + 3 * adv_b, idesc, 1u);
+                            adesc += a_atom_step;
+                            d += P.bn;
+                        }
+                    } else
                     for (int a = 0; a < n_atoms; ++a) {
                         if (kPair) {
                             if (f16) {
@@ -1039,7 +1181,103 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
         int titer = 0;
         uint32_t store_seq = 0;  // TMA-store pieces issued by this warp so far (selects the staging buffer)
         int bias_ntile = -1;     // column tile whose bias values sit in this warp's shared-memory copy
-        if constexpr (kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode)) {
+        if constexpr (kMode == MODE_FPROP && kDbl) {
+            // Double tiles (fp16, row-major output through TMA stores): this group's row tile goes into registers whole, bias
+            // added and rounded, so that the next tile's MMAs wait for the drain of TMEM alone.  A tile of one row tile is
+            // shared by column halves.  The bias values lie in the warp's staging buffer until the pieces need it.
+            static_assert(kOutMode == OUT_NHWC_TMA && kOutF16, "");
+            const uint32_t stg = smem_u32(staging) + ew * kStagingBufBytes;
+            float* const bt = reinterpret_cast<float*>(staging + ew * kStagingBufBytes);
+            const int rw = (quarter * 32) & (wb - 1), rh = ((quarter * 32) >> P.wb_log2) & (hb - 1);
+            const int rn = (quarter * 32) >> (P.wb_log2 + P.hb_log2);
+            const int group = ew >> 2;
+            const bool has_bias = (P.bias != nullptr);
+            int p = 0;
+            for (int tile = tile_first; tile < P.num_tiles; tile += tile_step, ++titer) {
+                while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
+                const Phase& ph = P.phases[p];
+                const int local = tile - ph.tile_begin;
+                const bool two = local < P.big_tiles;
+                int ntile, tw, th, tn;
+                decode_fprop_tile<kPair, kDbl>(P, ph, local, cta_rank, ntile, tw, th, tn, group);
+                const int sw = ph.pw + P.out_stride_w * ((tw << P.wb_log2) + rw);
+                const int sh = ph.ph + P.out_stride_h * ((th << P.hb_log2) + rh);
+                const int sn = (tn << P.nb_log2) + rn;
+                const int half = ((P.bn / 64 + 1) / 2) * 64;
+                const int col_base = ntile * P.bn + (!two && group ? half : 0);
+                const int cols = min(two ? P.bn : group ? P.bn - half : half, P.c_out - col_base);  // this warp's, from col_base
+                const bool live = ph.tap_count > 0;
+                if (has_bias) {
+                    if (lane == 0) bulk_wait_group_read<0>();  // the last tile's stores are done with the buffer
+                    float bv[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const int j = lane + 32 * u;
+                        bv[u] = j >= cols ? 0.f : P.bias_f16 ? __half2float(load_global(reinterpret_cast<const __half*>(P.bias) + col_base + j))
+                                                             : load_global(P.bias + col_base + j);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) bt[lane + 32 * u] = bv[u];
+                    __syncwarp();
+                }
+                const int buf = titer & ((1 << P.tbufs_log2) - 1);
+                const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * kRowTiles +
+                                       (two ? group * P.bn : group * half);
+                if (!mbar_wait(smem_u32(&tfull_bar[buf]), (titer >> P.tbufs_log2) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) break;
+                tc_fence_after();
+                uint32_t pk[4][32];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (64 * q >= cols) continue;
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        uint32_t r[32];
+                        if (live) {
+                            tmem_ld_32x32(t_row + 64 * q + 32 * u, r);
+                            tmem_ld_wait();
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) r[j] = 0u;
+                        }
+                        if (has_bias) {
+#pragma unroll
+                            for (int j = 0; j < 32; j += 4) {
+                                const float4 b = *reinterpret_cast<const float4*>(bt + 64 * q + 32 * u + j);
+                                r[j] = __float_as_uint(__uint_as_float(r[j]) + b.x);
+                                r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + b.y);
+                                r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + b.z);
+                                r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + b.w);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) pk[q][16 * u + j] = pack_half2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (!leader) mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[buf]), 0));
+                    else mbar_arrive(smem_u32(&tempty_bar[buf]));
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (64 * q >= cols) continue;
+                    if (lane == 0) bulk_wait_group_read<0>();
+                    __syncwarp();
+#pragma unroll
+                    for (int v = 0; v < 8; ++v)
+                        st_shared_v4(stg + lane * 128 + ((v ^ (lane & 7)) << 4), make_uint4(pk[q][4 * v], pk[q][4 * v + 1], pk[q][4 * v + 2], pk[q][4 * v + 3]));
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_4d(&P.tmC, stg, col_base + 64 * q, sw, sh, sn);
+                        bulk_commit_group();
+                    }
+                }
+            }
+            if (lane == 0) bulk_wait_group<0>();  // stores must land before the CTA ends
+        } else if constexpr (kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode)) {
             // Output through TMA stores: each warp converts 128-byte pieces of its 32 rows into a swizzled 4 KB buffer and
             // one lane hands the buffer to a TMA store, whose box is exactly those 32 rows; rows and columns outside the
             // tensor are clipped by the hardware.
@@ -1347,6 +1585,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
             const int buf = titer & ((1 << P.tbufs_log2) - 1);
             const uint32_t tpar = (titer >> P.tbufs_log2) & 1;
             // tile decode
+            int t_half = 0, c_first = 0, c_last = P.bn;  // this warp's accumulator (double tiles) and columns
             int ntile, k_iters;
             bool row_valid;
             int pix_n = 0, pix_h = 0, pix_w = 0;  // forward walk: this row's pixel within its phase grid
@@ -1384,10 +1623,14 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     col_stride = static_cast<size_t>(P.out_h) * P.out_w;
                 }
             } else {
-                int m_tiles = (P.groups_total * P.kb + kTileM - 1) / kTileM;
-                if (kPair) m_tiles = (m_tiles + 1) / 2;  // tile ids name pairs of row tiles
                 int mt, z;
-                decode_wgrad_tile(P, tile, m_tiles, ntile, mt, z);
+                const int halves = decode_wgrad_tile<kPair, kDbl>(P, tile, ntile, mt, z);
+                if (kDbl) {  // a group to a row tile, or to half the columns of one
+                    const int group = ew >> 2;
+                    if (halves == 2) mt += group, t_half = group * P.bn;
+                    else if (group) c_first = P.bn / 2;
+                    else c_last = P.bn / 2;
+                }
                 if (kPair) mt = 2 * mt + static_cast<int>(cta_rank);
                 int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
                 k_iters = max(min(z * per + per, P.kblocks_total) - z * per, 0);
@@ -1439,7 +1682,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                 break;
             }
             tc_fence_after();
-            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * P.planes;
+            const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * P.planes * kRowTiles + t_half;
             const uint32_t cross = P.planes == 2 ? P.bn : 0;  // the split's second accumulator, this many columns further on
             // r += columns [c, c + 32) of the second accumulator
             auto add_cross = [&](uint32_t c, uint32_t (&r)[32]) {
@@ -1705,7 +1948,7 @@ __global__ void __launch_bounds__(threads_for(kOutMode), 1) umma_conv_kernel(con
                     }
                 }
             } else
-            for (int c0 = 0; c0 < P.bn; c0 += 32) {
+            for (int c0 = kDbl ? c_first : 0; c0 < (kDbl ? c_last : P.bn); c0 += 32) {
                 if (col_base + c0 >= P.c_out) break;  // uniform across the warp
                 uint32_t r[32];
                 if (k_iters > 0) {

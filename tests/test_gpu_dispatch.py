@@ -48,6 +48,73 @@ def test_rows_that_do_not_start_on_16_bytes(rows, fout, oracle):
     ops.device_status()
 
 
+@pytest.fixture
+def four_pairs():
+    """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all."""
+    ops.set_sm_limit(8)
+    yield
+    ops.set_sm_limit(0)
+
+
+# pair tiles are 256 x 256 and four run at a time: five to eight of them in one round of double tiles (the last row tile missing
+# from 1100 rows, the last columns from 1000), and nine rows as four double tiles with a single one behind them.  K is summed
+# in fp32 (errors of sqrt(K) * 2^-24 of the terms' size), the result rounded to fp16: 1e-2 rel holds that many times over, and
+# the absolute bound is 1e-3 of the results' size, sqrt(K) * 0.2.
+@pytest.mark.parametrize("rows,fin,fout", [(1100, 1600, 256), (1280, 1984, 200), (512, 2048, 1000), (2300, 3200, 256), (2304, 3136, 232)])
+def test_double_tiles_linear(rows, fin, fout, oracle, four_pairs):
+    rng = np.random.default_rng(rows + fin)
+    h, r = torch.float16, oracle.round_f16
+    x = rng.standard_normal((rows, fin), dtype=np.float32)
+    w = (rng.standard_normal((fout, fin), dtype=np.float32) * 0.2).astype(np.float32)
+    b = rng.standard_normal(fout, dtype=np.float32)
+    want = oracle.linear_forward(r(x), r(w), r(b))
+    atol = 1e-3 * 0.2 * fin ** 0.5
+    assert_f16(host(ops.linear_forward(dev(x, h), dev(w, h), dev(b, h))), want, "bias", atol=atol)
+    assert_f16(host(ops.linear_forward(dev(x, h), dev(w, h))), oracle.linear_forward(r(x), r(w), None), "no bias", atol=atol)
+    # the same product as an input gradient (W read in place, columns inner) of the layer fout <- fin
+    assert_f16(host(ops.linear_backward_data(dev(x, h), dev(w.T, h))), oracle.linear_forward(r(x), r(w), None), "dx", atol=atol)
+    ops.device_status()
+
+
+@pytest.mark.parametrize("rows,fin,fout", [(4096, 640, 512), (4096, 1280, 512), (4100, 1280, 456), (2048, 256, 2304)])
+def test_double_tiles_linear_weight_gradient(rows, fin, fout, oracle, four_pairs):
+    rng = np.random.default_rng(rows + fin)
+    h, r = torch.float16, oracle.round_f16
+    x, dy = rng.standard_normal((rows, fin), dtype=np.float32), rng.standard_normal((rows, fout), dtype=np.float32)
+    dw, db = ops.linear_backward_weight(dev(x, h), dev(dy, h))
+    assert_f32(host(dw), r(dy).T.astype(np.float64) @ r(x).astype(np.float64), "dw")
+    assert_f32(host(db), r(dy).astype(np.float64).sum(0), "db")
+    ops.device_status()
+
+
+@pytest.mark.parametrize("n,c_in,hw,c_out,k,s,p,tr", [
+    (5, 128, 16, 256, 3, 1, 1, False), (3, 128, 21, 256, 5, 1, 2, False), (3, 256, 18, 256, 4, 2, 1, False), (3, 384, 16, 128, 4, 2, 1, True), (2, 256, 15, 256, 4, 2, 1, True)])
+def test_double_tiles_convolutions(n, c_in, hw, c_out, k, s, p, tr, oracle, four_pairs):
+    """Boxes of pixels, the phases of a gather, 128-column tiles, and row tiles of a weight gradient that belong to
+    different taps."""
+    rng = np.random.default_rng(c_in + hw)
+    h, r = torch.float16, oracle.round_f16
+    g = ops.ConvGeometry(n, c_in, hw, hw, c_out, k, k, (s, s), (p, p), transposed=tr)
+    x = rng.standard_normal((n, c_in, hw, hw), dtype=np.float32)
+    w = (rng.standard_normal(g.weight_shape(), dtype=np.float32) * 0.05).astype(np.float32)
+    dy = rng.standard_normal((n, c_out, *g.out_hw()), dtype=np.float32)
+    xd, wd, dyd = dev(x, h, nhwc=True), dev(w, h), dev(dy, h, nhwc=True)
+    # (float64 convolutions on the GPU: the oracle's loops would take minutes)
+    f = torch.nn.functional
+    x64, w64, dy64 = (torch.from_numpy(r(a)).cuda().double() for a in (x, w, dy))
+    x64.requires_grad_()
+    w64.requires_grad_()
+    y64 = (f.conv_transpose2d if tr else f.conv2d)(x64, w64, stride=s, padding=p)
+    y64.backward(dy64)
+    atol = 1e-3 * 0.05 * (max(c_in, c_out) * k * k) ** 0.5
+    assert_f16(host(ops.conv_forward(g, xd, wd, layout="nhwc"), nhwc=True), y64.detach().cpu().numpy(), "y", atol=atol)
+    assert_f16(host(ops.conv_backward_data(g, dyd, wd, layout="nhwc"), nhwc=True), x64.grad.cpu().numpy(), "dx", atol=atol)
+    dw, db = ops.conv_backward_weight(g, xd, dyd, layout="nhwc")
+    assert_f32(host(dw), w64.grad.cpu().numpy(), "dw")
+    assert_f32(host(db), dy64.sum((0, 2, 3)).cpu().numpy(), "db")
+    ops.device_status()
+
+
 @pytest.mark.parametrize("rows,c", [(1, 8), (3, 64), (1000, 24), (37, 2048)])
 @pytest.mark.parametrize("act", [0, 1, 2])
 @pytest.mark.parametrize("with_res", [False, True])

@@ -296,6 +296,7 @@ template <int kMode, int kOutMode, bool kOutF16, bool kPair, bool kDbl = false>
 __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1) umma_conv_kernel(const __grid_constant__ KParams P) {
     static_assert(!kDbl || kPair, "double tiles are tiles of CTA pairs");
     constexpr int kRowTiles = kDbl ? 2 : 1;
+    constexpr bool kPoll = kMode == MODE_FPROP && kOutF16 && !kDbl;  // how waits begin, see mbar_poll
     extern __shared__ uint8_t smem_raw[];
     // stages need 1024-byte alignment for the 128-byte swizzle pattern
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -392,7 +393,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
         const bool f16 = (P.kind == KIND_F16);
         const bool narrow = P.a_row_bytes == 64;
         const uint32_t layout_a = narrow ? 4 : 2;  // 64-byte or 128-byte swizzle
-        if (!mbar_wait(smem_u32(bres_bar), 0, abort_flag, P.err, ERR_WAIT_FULL)) return;
+        if (!mbar_wait<kPoll>(smem_u32(bres_bar), 0, abort_flag, P.err, ERR_WAIT_FULL)) return;
         int titer = t_first;
         int p = 0;
         // the patch buffer of this issuer's next patch and its parity, by counting (patches are consumed in tile order)
@@ -413,15 +414,15 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
             const int tb0 = P.phases[p].tap_begin;
             const int buf = titer & ((1 << P.tbufs_log2) - 1);
             const uint32_t tpar = (titer >> P.tbufs_log2) & 1;
-            if (!mbar_wait(smem_u32(&tempty_bar[buf]), tpar ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) return;
+            if (!mbar_wait<kPoll>(smem_u32(&tempty_bar[buf]), tpar ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) return;
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + buf * P.bn;
             uint32_t acc = 0;
             for (int cb = 0; cb < P.c_blocks; ++cb) {
-                if (!mbar_wait(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) return;
+                if (!mbar_wait<kPoll>(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) return;
                 tc_fence_after();
                 if (P.issuers == 2 && cb == 0 && titer > 0 &&
-                    !mbar_wait(smem_u32(&turn_bar[t_first]), ((titer - 1) >> 1) & 1, abort_flag, P.err, ERR_WAIT_EMPTY)) return;
+                    !mbar_wait<kPoll>(smem_u32(&turn_bar[t_first]), ((titer - 1) >> 1) & 1, abort_flag, P.err, ERR_WAIT_EMPTY)) return;
                 if (elect_one()) {
                     const uint64_t adesc0 = make_smem_desc(smem_u32(smem + P.a_ring_off) + pstage * P.patch_bytes, 16, sbo_a, layout_a);
                     uint64_t bdesc = make_smem_desc(smem_u32(smem) + (cb * P.n_taps + tb0) * stage_b_bytes, 16, 8 * P.b_row_bytes, layout_a);
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
             const uint32_t dst0 = smem_u32(smem) + (do_a ? 0 : b_off);
             // waits for the stage and announces this producer's bytes
             auto open_stage = [&](uint32_t bytes) -> bool {
-                ok = mbar_wait(empty0 + 8 * stage, parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY);
+                ok = mbar_wait<kPoll>(empty0 + 8 * stage, parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY);
                 if (ok && leader) mbar_arrive_expect_tx(full0 + 8 * stage, 2 * bytes);
                 return ok;
             };
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         const int w0 = (tw << P.wb_log2) * P.a_stride_w + pt.org_w;
                         const int h0 = (th << P.hb_log2) * P.a_stride_h + pt.org_h;
                         for (int cb = 0; ok && cb < P.c_blocks; ++cb) {
-                            if (!mbar_wait(smem_u32(&aempty_bar[abuf]), apar ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
+                            if (!mbar_wait<kPoll>(smem_u32(&aempty_bar[abuf]), apar ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
                                 ok = false;
                                 break;
                             }
@@ -750,7 +751,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         uint32_t fb = smem_u32(&full_bar[stage]);
                         if (kPair) fb = map_to_cta(fb, 0);
                         // (the issuing lanes leave together: a lane must never wait in __syncwarp for one that gave up)
-                        if (!__all_sync(issue_mask, mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
+                        if (!__all_sync(issue_mask, mbar_wait<kPoll>(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
                                                               ERR_WAIT_EMPTY))) {
                             ok = false;
                             break;
@@ -797,7 +798,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                     const uint32_t w_stage = static_cast<uint32_t>(P.patch_bytes) + stage_b_bytes;
                     const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * P.a_row_bytes;
                     for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
-                        if (!mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
+                        if (!mbar_wait<kPoll>(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
                             ok = false;
                             break;
                         }
@@ -847,7 +848,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                     for (int kbi = kb_begin; kbi < kb_end; ++kbi) {
                         const int w0 = tw << P.wb_log2, h0 = th << P.hb_log2, n0 = tn << P.nb_log2;
                         const uint32_t fb = map_to_cta(smem_u32(&full_bar[stage]), 0);
-                        if (!mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
+                        if (!mbar_wait<kPoll>(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY)) {
                             ok = false;
                             break;
                         }
@@ -904,7 +905,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                     if (nkb > 0) advance(P.planes == 2 ? my_atom >> 1 : my_atom);
                     for (int it = 0; it < nkb; it += ks) {  // one stage per iteration
                         const uint32_t fb = smem_u32(&full_bar[stage]);
-                        if (!__all_sync(issue_mask, mbar_wait(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
+                        if (!__all_sync(issue_mask, mbar_wait<kPoll>(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err,
                                                               ERR_WAIT_EMPTY))) {
                             ok = false;
                             break;
@@ -1013,7 +1014,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 const int z = tile / P.n_tiles;
                 const int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
                 const int nkb = max(min(z * per + per, P.kblocks_total) - z * per, 0);
-                if (!mbar_wait(smem_u32(&tempty_bar[0]), (titer & 1) ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) {
+                if (!mbar_wait<kPoll>(smem_u32(&tempty_bar[0]), (titer & 1) ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) {
                     ok = false;
                     break;
                 }
@@ -1035,7 +1036,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 const uint32_t stage_step16 = w_stage >> 4;
                 uint32_t accw = 0;
                 for (int kbi = 0; kbi < nkb; ++kbi) {
-                    if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
+                    if (!mbar_wait<kPoll>(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
                         ok = false;
                         break;
                     }
@@ -1069,7 +1070,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 }
                 continue;
             }
-            if (!mbar_wait(smem_u32(&tempty_bar[buf]), tpar ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) {
+            if (!mbar_wait<kPoll>(smem_u32(&tempty_bar[buf]), tpar ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) {
                 ok = false;
                 break;
             }
@@ -1095,7 +1096,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
             };
             for (int it = 0; it < k_iters; it += ks) {
                 const int n_atoms = min(ks, k_iters - it);
-                if (!mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
+                if (!mbar_wait<kPoll>(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) {
                     ok = false;
                     break;
                 }
@@ -1224,7 +1225,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 const int buf = titer & ((1 << P.tbufs_log2) - 1);
                 const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * kRowTiles +
                                        (two ? group * P.bn : group * half);
-                if (!mbar_wait(smem_u32(&tfull_bar[buf]), (titer >> P.tbufs_log2) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) break;
+                if (!mbar_wait<kPoll>(smem_u32(&tfull_bar[buf]), (titer >> P.tbufs_log2) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) break;
                 tc_fence_after();
                 uint32_t pk[4][32];
 #pragma unroll
@@ -1345,7 +1346,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 }
                 const int buf = titer & ((1 << P.tbufs_log2) - 1);
                 const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * P.planes;
-                if (!mbar_wait(smem_u32(&tfull_bar[buf]), (titer >> P.tbufs_log2) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) break;
+                if (!mbar_wait<kPoll>(smem_u32(&tfull_bar[buf]), (titer >> P.tbufs_log2) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) break;
                 tc_fence_after();
                 uint32_t r0[32], r1[32];
                 // (fp32 pieces are 32 columns: r1 then holds the second accumulator's)
@@ -1476,7 +1477,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 const int w_ntile = tile % P.n_tiles, w_z = tile / P.n_tiles;
                 const int per = (P.kblocks_total + P.split_k - 1) / P.split_k;
                 const int nkb = max(min(w_z * per + per, P.kblocks_total) - w_z * per, 0);
-                if (!mbar_wait(smem_u32(&tfull_bar[0]), titer & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) {
+                if (!mbar_wait<kPoll>(smem_u32(&tfull_bar[0]), titer & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) {
                     ok = false;
                     break;
                 }
@@ -1498,7 +1499,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         __syncwarp();
                         const uint32_t bar = smem_u32(&afull_bar[syncs & 1]);
                         if (lane == 0) mbar_arrive(bar);
-                        const bool met = mbar_wait(bar, (syncs >> 1) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL);
+                        const bool met = mbar_wait<kPoll>(bar, (syncs >> 1) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL);
                         ++syncs;
                         return met;
                     };
@@ -1677,7 +1678,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                     }
                 }
             }
-            if (!mbar_wait(smem_u32(&tfull_bar[buf]), tpar, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) {
+            if (!mbar_wait<kPoll>(smem_u32(&tfull_bar[buf]), tpar, abort_flag, P.err, ERR_WAIT_TMEM_FULL)) {
                 ok = false;
                 break;
             }

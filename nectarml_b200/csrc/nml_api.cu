@@ -522,16 +522,27 @@ static int prepare_window(const void* src, int dtype, int layout, int batch, int
 // Picks a power-of-two pixel box (w, h, n) with 2^bits pixels that covers the grid with the
 // fewest boxes; ties go to the wider box.  box extents times the element stride stay <= 256.  n_tiles: tiles per box.
 static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* wl, int* hl, int* nl,
-                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1, bool split = false) {
-    long long best = -1, best_wide = -1;
-    int ww = 0, wh = 0, wn = 0;
+                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1, bool split = false, double k_us = 0, double tile_kb = 0) {
+    const auto rounds = [&](long long boxes) { return (boxes * n_tiles + sms - 1) / sms; };
+    long long best = -1, best_wide = -1, best_narrow = -1;
+    int ww = 0, wh = 0, wn = 0, nw = 0, nh = 0, nn = 0;
     for (int a = bits; a >= 0; --a) {
         if ((1 << a) * s_w > 256) continue;
+        const bool narrow = prefer_w_log2 > 0 && a < 3 && (1 << a) < gw;  // (see below)
         for (int b = bits - a; b >= 0; --b) {
             if ((1 << b) * s_h > 256) continue;
             int c = bits - a - b;
             if ((1 << c) > 256) continue;
             long long tiles = 1ll * ceil_div(gw, 1 << a) * ceil_div(gh, 1 << b) * ceil_div(gn, 1 << c);
+            if (narrow) {
+                if (best_narrow < 0 || tiles < best_narrow) {
+                    best_narrow = tiles;
+                    nw = a;
+                    nh = b;
+                    nn = c;
+                }
+                continue;
+            }
             if (best < 0 || tiles < best) {
                 best = tiles;
                 *wl = a;
@@ -552,12 +563,24 @@ static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* 
     // 3xTF32 tiles are 128 columns wide: 256 -> 256 at 56 x 56, batch 8, 392 tiles instead of 448 154 -> 124 us.  Their narrow
     // boxes have to save a round of several, though: where all run at once nothing overlaps the drain (`split`; 128 -> 384 at
     // 28 x 28, batch 8, 49.1 us in two rounds of wide boxes, 54.2 in one of narrow ones).
-    const auto rounds = [&](long long boxes) { return (boxes * n_tiles + sms - 1) / sms; };
     if (prefer_w_log2 > 0 && best_wide > 0 && best_wide * 100 <= best * 115 &&
         (rounds(best_wide) <= rounds(best) || (split && rounds(best) == 1))) {
         *wl = ww;
         *hl = wh;
         *nl = wn;
+        best = best_wide;
+    }
+    // Boxes of fewer than eight pixels of a wider row may save rounds (62 x 62 pixels of 64 images are 1922 boxes of 2 x 1 x 64 and 1984
+    // of 64 x 2 x 1), but their pixel-major stores reach 1 TB/s and less (two pixels 0.63) where eight and more reach 3.7: only
+    // where the K loop outlasts the stores.  k_us: a tile's K loop, tile_kb: its result.  1x1 64 -> 200 at 62 x 62, batch 64, fp32
+    // result of fp16 products 314 -> 54 us without them; 5x5 96 -> 64 at 21 x 21, batch 128, 3xTF32 162 us without, 141 with them.
+    if (best_narrow > 0) {
+        const auto tile_us = [&](double store_us) { return std::max(k_us, store_us) + 0.25 * std::min(k_us, store_us); };  // (mostly overlapped)
+        if (rounds(best_narrow) * tile_us(tile_kb / (2.4 * (1 << nw))) < 0.97 * rounds(best) * tile_us(tile_kb / 25.0)) {
+            *wl = nw;
+            *hl = nh;
+            *nl = nn;
+        }
     }
 }
 
@@ -598,7 +621,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     // cost a ring stage, else one), the per-warp bias tiles, and the barriers.
     const int fixed = kFixedSmem - (P.dbl ? kBiasTileBytes : 0);
     const bool tma_out = (P.mode == MODE_FPROP) && NML_IS_TMA_OUT(P.out_mode);
-    // A second group of four epilogue warps (TMA-store instances only) where a tile's drain outlasts its MMAs.  Clocks,
+    // A second group of four epilogue warps (TMA-store and channel-major instances) where a tile's drain outlasts its MMAs.  Clocks,
     // measured: one group needs ~800 per tile plus ~900 per 128-byte piece; four MMAs (one K slice) take 192 at 64 columns
     // and below (shared-memory reads), 512 at 256.  With several tiles per CTA the groups take alternate tiles (one
     // decode per two tiles); with one or two they share each tile, which shortens the last drain.
@@ -607,14 +630,16 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     P.epi_alt = 0;
     if (P.dbl) {
         P.epi_warps = 8;
-    } else if (tma_out && tune().epi8) {
+    } else if ((tma_out || (P.mode == MODE_FPROP && P.out_mode == OUT_NCHW)) && tune().epi8) {
         int k_slices = 0;  // longest phase
         for (int p = 0; p < P.n_phases; ++p) k_slices = std::max(k_slices, P.c_blocks * P.phases[p].tap_count);
         const int pieces = ceil_div(P.bn, P.out_f16 ? 64 : 32);
         const int mma = k_slices * (P.planes == 2 ? 3 : 1) * (P.bn <= 64 ? 192 : P.bn <= 128 ? 288 : 512);
         if (mma * 2 < (800 + 900 * pieces) * 3) {
-            P.epi_alt = P.num_tiles > 2 * ctas ? 1 : 0;
-            P.epi_warps = (P.epi_alt || pieces >= 2) ? 8 : 4;
+            // (channel-major stores alternate or have one group; 128 x 300 x 128 x 300 fp16 products 23.7 -> 21.6 us, 8 x 1000 x 64 x
+            // 999 fp32 22.9 -> 20.0)
+            P.epi_alt = P.num_tiles > (tma_out ? 2 * ctas : ctas) ? 1 : 0;
+            P.epi_warps = (P.epi_alt || (tma_out && pieces >= 2)) ? 8 : 4;
         }
     }
     P.tbufs_log2 = 0;
@@ -683,9 +708,12 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     }
     const bool rec = rec_slot >= 0;
     if (rec && !pre_opened) NML_CUDA(cudaEventRecord(g_prof.start[rec_slot], st));
+    // No idle second group (352 -> 224 threads: Linear 700 x 300 -> 200 forward 9.0 -> 8.7 us, 32 x 512 -> 2048 input gradient 10.5 -> 9.9),
+    // but for the patch walk, which measured 3 % slower without (3x3 64 at 56 x 56, batch 8, channel-major fp16 13.2 -> 13.7).
+    const int threads = P.epi_warps == 8 ? kThreadsWide : P.patch ? threads_for(P.out_mode) : kThreads;
     // (under an SM limit not before its predecessor has ended: blocks that wait would sit on the SMs that are to stay free, and
     // a block of this kernel leaves no room beside it)
-    launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, P.dbl ? kThreadsWide : threads_for(P.mode == MODE_FPROP ? P.out_mode : OUT_NHWC), smem, st, P);
+    launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, threads, smem, st, P);
     NML_CUDA(cudaGetLastError());
     if (open_slot) *open_slot = rec_slot;
     else if (rec) NML_CUDA(cudaEventRecord(g_prof.stop[rec_slot], st));
@@ -755,6 +783,13 @@ struct FpropLike {
     int w_batched;  // every image has its own [d0][d1] weights, one after the other (batched matmul; kh = kw = 1)
 };
 
+// choose_box for the tiles of a forward walk: N columns, `slices` K slices (of three products each for the 3xTF32 split).
+static void choose_tile_box(int gw, int gh, int gn, int s_w, int s_h, int N, int planes, int slices, int out_bytes, int prefer_w_log2, int sms,
+                            int* wl, int* hl, int* nl) {
+    const int n_tiles = ceil_div(N, planes == 2 ? 128 : 256), bn = ceil_div(N, n_tiles);
+    choose_box(7, gw, gh, gn, s_w, s_h, wl, hl, nl, prefer_w_log2, n_tiles, sms, planes == 2, slices * slice_us(bn) * (planes == 2 ? 3 : 1), bn * out_bytes / 8.0);
+}
+
 // Whether a few-channel layer with N output channels takes the patch walk with resident weights when its rows are 64
 // bytes long (the conditions of run_fprop_like's own choice, which then makes the same one).
 static bool narrow_patch_walk(const FpropLike& f, int N) {
@@ -763,7 +798,7 @@ static bool narrow_patch_walk(const FpropLike& f, int N) {
     if (f.kh < 2 || ph > 256 || pw * ph * 64 > 48 * 1024) return false;
     int wl = 0, hl = 0, nl = 0;
     const bool nchw = f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1);
-    choose_box(7, f.out_w, f.out_h, f.batch, 1, f.s_h, &wl, &hl, &nl, nchw ? 5 : 0, 1, planning_sms());
+    choose_tile_box(f.out_w, f.out_h, f.batch, 1, f.s_h, N, 1, f.kh, f.out_dtype == NML_F16 ? 2 : 4, nchw ? 5 : 0, planning_sms(), &wl, &hl, &nl);
     const double area = static_cast<double>(f.out_w) * f.out_h;
     const double eff_patch = area / (1.0 * round_up(f.out_w, 8) * round_up(f.out_h, 16));
     const double eff_box = area * f.batch / (1.0 * round_up(f.out_w, 1 << wl) * round_up(f.out_h, 1 << hl) * round_up(f.batch, 1 << nl));
@@ -1094,8 +1129,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         P.b_batched = 1;
         P.wb_log2 = 7;
     } else {
-        choose_box(7, P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, &P.wb_log2, &P.hb_log2, &P.nb_log2,
-                   (P.out_mode == OUT_NCHW && !f.gather) ? 5 : 0, ceil_div(N, P.planes == 2 ? 128 : 256), limited(ds->sms), P.planes == 2);
+        choose_tile_box(P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, N, P.planes, c_blocks * P.phases[0].tap_count, P.out_f16 ? 2 : 4,
+                        P.out_mode != OUT_NCHW ? 0 : f.gather && f.s_w > 1 ? 1 : 5, limited(ds->sms), &P.wb_log2, &P.hb_log2, &P.nb_log2);
     }
     // Patch walk: unit-stride walks with several taps load one haloed patch per channel block instead of
     // one box per tap (8 x 16 pixel tiles of a single image).  Taken when the fixed tile shape does not

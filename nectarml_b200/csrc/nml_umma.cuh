@@ -8,7 +8,7 @@
 //   warp 1      MMA issuer     : one thread issues tcgen05.mma, accumulators live in TMEM,
 //                                two or four TMEM buffers so the epilogue of tile i overlaps tile i+1
 //   warps 2..5  epilogue       : tcgen05.ld -> bias / rounding / cast -> TMA or plain global stores
-//   warps 7..10 epilogue       : second group, TMA-store instances only, used on short-K tiles
+//   warps 7..10 epilogue       : second group, TMA-store and channel-major instances only, used on short-K tiles
 //
 // Two tile walks share the pipeline:
 //   MODE_FPROP  rows of the tile are output pixels (n, h, w) taken as one TMA box of the
@@ -50,9 +50,9 @@ constexpr int kMaxTaps = 128;
 constexpr int kTileM = 128;
 constexpr int kStageABytes = kTileM * 128;
 constexpr int kThreads = 224;      // warp 0: A loads, warp 1: MMA issue, warps 2-5: epilogue, warp 6: B loads
-constexpr int kThreadsWide = 352;  // TMA-store instances: warps 7-10 are a second epilogue group (used when the
-                                   // K loop is short and the epilogue is the critical path; they need few registers)
-__host__ __device__ constexpr int threads_for(int out_mode) { return (out_mode == 2 || out_mode == 3) ? kThreadsWide : kThreads; }
+constexpr int kThreadsWide = 352;  // TMA-store and channel-major instances: warps 7-10 are a second epilogue group (used when
+                                   // the K loop is short and the epilogue is the critical path; they need few registers)
+__host__ __device__ constexpr int threads_for(int out_mode) { return out_mode != 0 ? kThreadsWide : kThreads; }
 constexpr int kStagingBufBytes = 4096;         // one staging buffer: 32 rows x 128 bytes of output
 constexpr int kBiasTileBytes = 8 * 256 * 4;   // per epilogue warp (up to 8): the current tile's bias values
 
@@ -1466,7 +1466,9 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
             }
             if (lane == 0) bulk_wait_group<0>();  // stores must land before the CTA ends
         } else
-        for (int tile_id = tile_first; ok && tile_id < P.num_tiles; tile_id += tile_step, ++titer) {
+        // (two groups of channel-major stores take alternate tiles; those of a double tile share each)
+        for (int alt = kMode == MODE_FPROP && P.epi_alt ? 1 : 0, tile_id = tile_first + (titer = alt & (ew >> 2)) * tile_step;
+             ok && tile_id < P.num_tiles; tile_id += (1 + alt) * tile_step, titer += 1 + alt) {
             int tile = tile_id, kz = 0;
             if (kMode == MODE_FPROP && P.fsplit > 1) {
                 kz = tile_id / P.base_tiles;

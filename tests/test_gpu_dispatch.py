@@ -48,6 +48,26 @@ def test_rows_that_do_not_start_on_16_bytes(rows, fout, oracle):
     ops.device_status()
 
 
+# pixel boxes of channel-major results: the fewest boxes are 2 x 1 x 64 and 1 x 1 x 128 pixels, taken only where the K loop outlasts
+# their stores; images narrower than eight pixels; both groups of epilogue warps (more tiles than SMs)
+@pytest.mark.parametrize("n,c_in,h,w,c_out,k,s", [
+    (64, 8, 62, 62, 24, 1, 1), (64, 8, 30, 62, 24, 3, 1), (128, 40, 5, 21, 24, 5, 1), (70, 16, 9, 5, 40, 3, 1), (128, 8, 7, 7, 72, 1, 1), (130, 16, 31, 3, 33, 3, 2), (9, 8, 131, 61, 40, 3, 2)])
+def test_channel_major_results_of_any_width(n, c_in, h, w, c_out, k, s):
+    gen = torch.Generator(device="cuda").manual_seed(n + w)
+    g = ops.ConvGeometry(n, c_in, h, w, c_out, k, k, (s, s), (k // 2, k // 2))
+    x = torch.randn(n, c_in, h, w, device="cuda", generator=gen)
+    wt = torch.randn(c_out, c_in, k, k, device="cuda", generator=gen) * 0.1
+    dy = torch.randn(n, c_out, *g.out_hw(), device="cuda", generator=gen)
+    for dt, math, check in ((torch.float32, "3xtf32", assert_f32), (torch.float16, "f16", assert_f16)):
+        xd, wd, dyd = x.to(dt), wt.to(dt), dy.to(dt)
+        x64 = xd.double().requires_grad_()
+        y64 = torch.nn.functional.conv2d(x64, wd.double(), stride=s, padding=k // 2)
+        (dx64,) = torch.autograd.grad(y64, (x64,), dyd.double())
+        check(host(ops.conv_forward(g, xd, wd, math=math)), y64.detach().cpu().numpy(), f"y {dt}")
+        check(host(ops.conv_backward_data(g, dyd, wd, math=math)), dx64.cpu().numpy(), f"dx {dt}")
+    ops.device_status()
+
+
 @pytest.fixture
 def four_pairs():
     """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all."""

@@ -14,7 +14,7 @@ import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = [os.path.join(_HERE, "csrc", "nml_api.cu"), os.path.join(_HERE, "csrc", "nml_layers.cu")]
-HEADERS = [os.path.join(_HERE, "csrc", n) for n in ("nml_launch.cuh", "nml_ptx.cuh", "nml_umma.cuh", "nml_prepass.cuh")] + [
+HEADERS = [os.path.join(_HERE, "csrc", n) for n in ("nml_launch.cuh", "nml_ptx.cuh", "nml_umma.cuh", "nml_prepass.cuh", "nml_gemm.cuh")] + [
     os.path.join(os.path.dirname(_HERE), "include", "nectarml_b200.h")]
 OUTPUT = os.path.join(_HERE, "libnectarml_b200.so")
 NATIVE_SOURCE = os.path.join(_HERE, "csrc", "nml_torch.cpp")

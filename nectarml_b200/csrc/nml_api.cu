@@ -4,6 +4,7 @@
 // points; the reference-shaped entry points allocate their result as the reference does.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -16,6 +17,7 @@
 #include "../../include/nectarml_b200.h"
 #include "nml_prepass.cuh"
 #include "nml_umma.cuh"
+#include "nml_gemm.cuh"
 
 namespace nml {
 
@@ -93,8 +95,9 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
 //   NML_TUNE_NARROW   0: few-channel layers always take eight channels per pixel
 //   NML_TUNE_DOUBLE   0: no double tiles, 2: wherever they are legal
+//   NML_TUNE_GEMM     0: no strided products
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow, dbl;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow, dbl, gemm;
 };
 static const Tune& tune() {
     static Tune t;
@@ -120,6 +123,7 @@ static const Tune& tune() {
         t.pair128 = env("NML_TUNE_PAIR128", 1);
         t.narrow = env("NML_TUNE_NARROW", 1);
         t.dbl = env("NML_TUNE_DOUBLE", 1);
+        t.gemm = env("NML_TUNE_GEMM", 1);
     });
     return t;
 }
@@ -209,7 +213,17 @@ static UmmaKernel kernel_for(const KParams& P) {
     if (P.out_mode == OUT_NHWC) return fprop_instance<OUT_NHWC, false>(h);
     return fprop_instance<OUT_NCHW, false>(h);
 }
+typedef void (*GemmKernel)(const GemmParams);
+template <typename T>
+static GemmKernel gemm_instance(bool a_contiguous, bool b_contiguous) {
+    return a_contiguous ? (b_contiguous ? gemm_strided_kernel<T, true, true> : gemm_strided_kernel<T, true, false>)
+                        : (b_contiguous ? gemm_strided_kernel<T, false, true> : gemm_strided_kernel<T, false, false>);
+}
 static int raise_smem_limit() {
+    for (int i = 0; i < 4; ++i) {
+        NML_CUDA(cudaFuncSetAttribute(gemm_instance<float>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+        NML_CUDA(cudaFuncSetAttribute(gemm_instance<__half>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
+    }
     UmmaKernel all[18] = {umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
                           umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true>,
                           fprop_instance<OUT_NHWC_TMA, false>(true), fprop_instance<OUT_NHWC_TMA, false>(false),
@@ -1825,6 +1839,95 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     return profile_stop(slot, st);
 }
 
+// ------------------------------------------------------------ strided products --
+// out[m + n * out_ns] (+ entry * out_batch) = sum over k of a(m, k) * b(n, k) [+ bias[m]]: see nml_gemm.cuh.
+struct StridedProduct {
+    int M, N, K, batch;
+    int dtype;  // of both operands; fp32 runs as 3xTF32
+    const void *a, *b;
+    bool a_contiguous, b_contiguous;  // k is the inner dimension (else m or n is)
+    long long a_stride, b_stride, out_ns, a_batch, b_batch, out_batch;
+    void* out;
+    int out_dtype;
+    const void* bias;
+    int bias_dtype, round_f16;
+};
+
+struct StridedPlan {
+    int bn = 0, splits = 1;
+    double us = 0;
+};
+// Tile width and blocks per tile by estimated time: 6.6 us for launch, set-up and drain, then a K slice by how full the SMs are
+// (alone 0.5 us at 32 columns, 0.6 at 64; with two blocks to every SM 1.1 and 1.3; 30 % more for an operand whose rows are the
+// inner dimension, which is four loads a chunk), and for every further wave of blocks its own set-up and drain.
+static StridedPlan plan_strided(const StridedProduct& g, int sms) {
+    const int slices = ceil_div(g.K, g.dtype == NML_F32 ? 32 : 64);
+    StridedPlan best;
+    for (int bn = 64; bn >= 32; bn /= 2) {
+        const long long tiles = 1ll * ceil_div(g.M, kTileM) * ceil_div(g.N, bn) * g.batch;
+        for (int z = 1; z <= kGemmMaxSplits && (z == 1 || slices >= 2 * z); z *= 2) {
+            const double blocks = static_cast<double>(tiles) * z, waves = std::ceil(blocks / (2.0 * sms));
+            const double slice_us = (bn == 32 ? 0.5 : 0.6) * (1.0 + 0.6 * std::min(2.0, blocks / sms)) * (g.a_contiguous ? 1.0 : 1.3) *
+                                    (g.b_contiguous ? 1.0 : 1.3);
+            const double us = 6.6 + waves * ceil_div(slices, z) * slice_us + (waves - 1.0) * 4.0;
+            if (best.bn == 0 || us < best.us) {
+                best.bn = bn;
+                best.splits = z;
+                best.us = us;
+            }
+        }
+    }
+    return best;
+}
+
+static int run_strided(const StridedProduct& g, int role, DeviceState* ds, cudaStream_t st) {
+    const bool f32 = g.dtype == NML_F32;
+    const int es = f32 ? 4 : 2, slice = f32 ? 32 : 64;
+    if (!ds) {
+        const int rc = device_state(&ds);
+        if (rc) return rc;
+    }
+    const StridedPlan plan = plan_strided(g, planning_sms());
+    GemmParams P;
+    memset(&P, 0, sizeof(P));
+    P.a = g.a; P.b = g.b; P.bias = g.bias; P.out = g.out;
+    P.a_stride = g.a_stride; P.b_stride = g.b_stride; P.out_ns = g.out_ns;
+    P.a_batch = g.a_batch; P.b_batch = g.b_batch; P.out_batch = g.out_batch;
+    P.M = g.M; P.N = g.N; P.K = g.K;
+    P.bn = plan.bn;
+    P.tiles_m = ceil_div(g.M, kTileM);
+    P.tiles_n = ceil_div(g.N, plan.bn);
+    P.splits = plan.splits;
+    P.per = ceil_div(ceil_div(g.K, slice), plan.splits);
+    const int stage_bytes = (f32 ? 2 : 1) * (kStageABytes + plan.bn * 128);
+    P.stages = f32 ? 2 : 4;  // (80 to 96 KB: two blocks to an SM)
+    const auto vec = [&](const void* p, long long stride, long long batch) {
+        return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && stride * es % 16 == 0 && batch * es % 16 == 0 ? 1 : 0;
+    };
+    P.a_vec = vec(g.a, g.a_stride, g.a_batch);
+    P.b_vec = vec(g.b, g.b_stride, g.b_batch);
+    P.bias_f16 = g.bias_dtype == NML_F16;
+    P.out_f16 = g.out_dtype == NML_F16;
+    P.round_f16 = g.round_f16;
+    P.role = role;
+    P.err = ds->err;
+    P.wait_limit_ns = g_dbg_wait_limit_ns;
+    const long long blocks = 1ll * P.tiles_m * P.tiles_n * g.batch * plan.splits;
+    if (blocks > INT_MAX) return NML_ERR_UNSUPPORTED;
+    int rc = profile_open(st);
+    if (rc) return rc;
+    const int slot = g_bracket_slot;
+    g_bracket_slot = -1;
+    // Two blocks to an SM, and none beside a block of the contraction kernel (120 KB and more): blocks of clusters that wait for
+    // TMEM columns behind one another on two SMs would wait for good.
+    const size_t smem = std::max<size_t>(static_cast<size_t>(P.stages) * stage_bytes + 1024 + 256, 110 * 1024);
+    launch_with(true, plan.splits, f32 ? gemm_instance<float>(g.a_contiguous, g.b_contiguous) : gemm_instance<__half>(g.a_contiguous, g.b_contiguous),
+                static_cast<unsigned>(blocks), kGemmThreads, smem, st, P);
+    NML_CUDA(cudaGetLastError());
+    ++g_launches;
+    return profile_stop(slot, st);
+}
+
 // --------------------------------------------------------- layer -> problems --
 static bool conv_out_size(const nml_conv_desc* d, int* ho, int* wo) {
     if (!d || d->stride_h <= 0 || d->stride_w <= 0 || d->dil_h <= 0 || d->dil_w <= 0 || d->kh <= 0 || d->kw <= 0 ||
@@ -1900,6 +2003,61 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
                        void* out, float* db, Bump& ws, cudaStream_t st) {
     if (!d || d->rows <= 0 || d->in_features <= 0 || d->out_features <= 0) return NML_ERR_INVALID;
     g_last_scratch_error[0] = 0;
+    if (tune().gemm && d->math == NML_MATH_3XTF32 && d->in_dtype == NML_F32 && (pass == NML_PASS_BACKWARD_WEIGHT || d->w_dtype == NML_F32) &&
+        g_sm_limit.load(std::memory_order_relaxed) == 0) {
+        const int R = d->rows, I = d->in_features, O = d->out_features;
+        StridedProduct g;
+        memset(&g, 0, sizeof(g));
+        g.dtype = NML_F32;
+        g.batch = 1;
+        g.out = out;
+        g.out_dtype = pass == NML_PASS_BACKWARD_WEIGHT ? NML_F32 : d->out_dtype;
+        if (pass == NML_PASS_FORWARD) {          // y[r][o] = x[r][i] * w[o][i]
+            g.M = O; g.N = R; g.K = I;
+            g.a = in1; g.a_contiguous = true; g.a_stride = I;
+            g.b = in0; g.b_contiguous = true; g.b_stride = I;
+            g.out_ns = O;
+            g.bias = bias; g.bias_dtype = d->w_dtype; g.round_f16 = d->round_out_f16;
+        } else if (pass == NML_PASS_BACKWARD_DATA) {  // dx[r][i] = dy[r][o] * w[o][i]
+            g.M = I; g.N = R; g.K = O;
+            g.a = in1; g.a_contiguous = false; g.a_stride = I;
+            g.b = in0; g.b_contiguous = true; g.b_stride = O;
+            g.out_ns = I;
+        } else {                                 // dw[o][i] = dy[r][o] * x[r][i]
+            g.M = I; g.N = O; g.K = R;
+            g.a = in0; g.a_contiguous = false; g.a_stride = I;
+            g.b = in1; g.b_contiguous = false; g.b_stride = O;
+            g.out_ns = I;
+        }
+        // The conversions and the contraction kernel take (forward / input gradient / weight gradient, us, with this path in
+        // brackets) 64 x 512 -> 512 12.0 / 13.6 / 12.3 (7.6 / 8.1 / 8.5), 128 x 768 -> 256 12.5 / 13.6 / 12.3 (8.6 / 7.8 / 10.4), 300 x 1500 ->
+        // 300 20.7 / 16.1 / 18.7 (15.7 / 12.6 / 17.0), 256 x 2048 -> 1000 22.4 / 24.3 / 18.9 (20.1 / 20.9 / 24.7), 2000 x 90 -> 400
+        // 10.2 / 25.0 / 18.4 (9.6 / 12.9 / 21.9), 20 x 4000 -> 200 17.4 / 13.6 / 12.5 (18.3 / 9.3 / 7.8): the estimates up to which
+        // this path was the faster.
+        // (a weight gradient of fewer than eight tiles is the contraction kernel's: it cuts K into up to 192 shares)
+        const StridedPlan plan = plan_strided(g, planning_sms());
+        const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
+        if (!few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0)) {
+            RowsColsum sums;
+            if (pass == NML_PASS_BACKWARD_WEIGHT && db) {
+                sums.plan(in1, NML_F32, R, O, db);
+                sums.cs = colsum_scratch(ws, sums.grid.y, O);
+            }
+            if (ws.dry) return NML_OK;
+            if (!ws.fits()) return NML_ERR_WORKSPACE;
+            const bool beside = sums.out && !g_prof.on.load(std::memory_order_relaxed);
+            if (sums.out && !beside) {
+                sums.first_stage(st);
+                const int rc = sums.second_stage(st);
+                if (rc) return rc;
+            }
+            const int rc = run_strided(g, beside ? PDL_LEADER : PDL_NORMAL, nullptr, st);
+            if (rc || !beside) return rc;
+            t_role = PDL_SIBLING;
+            sums.first_stage(st);
+            return sums.second_stage(st);
+        }
+    }
     if (pass == NML_PASS_BACKWARD_WEIGHT) {
         WgradLike g;
         memset(&g, 0, sizeof(g));
@@ -2493,6 +2651,19 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             d.in_dtype = d.out_dtype = d.w_dtype = dtype;
             d.math = math;
             return linear_pass(&d, NML_PASS_BACKWARD_DATA, A, B, nullptr, C, nullptr, bump, nullptr);
+        }
+        if (turned && tune().gemm && n <= 65535 && g_sm_limit.load(std::memory_order_relaxed) == 0) {
+            StridedProduct g;
+            memset(&g, 0, sizeof(g));
+            g.M = N; g.N = M; g.K = K; g.batch = static_cast<int>(n);
+            g.dtype = g.out_dtype = dtype;
+            g.a = B; g.a_contiguous = false; g.a_stride = N; g.a_batch = 1ll * K * N;
+            g.b = A; g.b_contiguous = true; g.b_stride = K; g.b_batch = 1ll * M * K;
+            g.out = C; g.out_ns = N; g.out_batch = 1ll * M * N;
+            // Products of few blocks, in place: 128 x 33 x 64 x 33 fp16 10.0 -> 6.4 us, fp32 12.9 -> 7.3; 3 x 800 x 96 x 801 fp16 10.9 ->
+            // 9.4, fp32 16.3 -> 10.4; 64 x 45 x 64 x 1001 fp32, two waves, 25.0 -> 15.6; more of them are the contraction kernel's: 64 x 333
+            // x 64 x 333 fp32 25.1 against 28.7, 20 x 777 x 64 x 140 fp16, two waves, 9.3 against 12.9.
+            if (plan_strided(g, planning_sms()).us <= (es == 4 ? 18.0 : 10.5)) return bump.dry ? NML_OK : run_strided(g, PDL_NORMAL, nullptr, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));

@@ -68,6 +68,38 @@ def test_channel_major_results_of_any_width(n, c_in, h, w, c_out, k, s):
     ops.device_status()
 
 
+# operands read in place: one row, one column, K of one value and of no whole slice, rows that start anywhere, K loops shared by the
+# blocks of a cluster (the last of them with nothing to do), two waves of blocks
+@pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (1, 70, 33), (129, 33, 130), (64, 513, 127), (33, 288, 65), (5, 2049, 3), (300, 36, 1025)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_fp32_products_in_place(rows, fin, fout, shift, oracle):
+    rng = np.random.default_rng(rows + fin)
+    sizes = {"x": (rows, fin), "w": (fout, fin), "dy": (rows, fout), "b": (fout,)}
+    host_of = {k: rng.standard_normal(s, dtype=np.float32) for k, s in sizes.items()}
+    x, w, dy, b = (torch.cat([torch.zeros(shift, device="cuda"), dev(v).flatten()])[shift:].view(v.shape) for v in host_of.values())
+    xh, wh, dyh, bh = host_of.values()
+    launches = ops.launch_count()
+    y = ops.linear_forward(x, w, b, math="3xtf32")
+    dx = ops.linear_backward_data(dy, w, math="3xtf32")
+    assert ops.launch_count() - launches == 2
+    assert_f32(host(y), oracle.linear_forward(xh, wh, bh), "y")
+    assert_f32(host(dx), dyh.astype(np.float64) @ wh.astype(np.float64), "dx")
+    dw, db = ops.linear_backward_weight(x, dy, math="3xtf32")
+    assert_f32(host(dw), dyh.T.astype(np.float64) @ xh.astype(np.float64), "dw")
+    assert_f32(host(db), dyh.astype(np.float64).sum(0), "db")
+    half = host(ops.linear_forward(x, w, b, math="3xtf32", out_dtype=torch.float16))
+    assert_f16(half, oracle.linear_forward(xh, wh, bh), "fp16 result")
+    rounded = host(ops.linear_forward(x, w, b, math="3xtf32", round_out_f16=True))
+    assert np.array_equal(rounded, half)
+    assert torch.equal(y, ops.linear_forward(x, w, b, math="3xtf32"))
+    ops.set_sm_limit(140)  # (contraction kernel: these blocks do not keep to a limit)
+    try:
+        assert_f32(host(ops.linear_forward(x, w, b, math="3xtf32")), oracle.linear_forward(xh, wh, bh), "y, limited")
+    finally:
+        ops.set_sm_limit(0)
+    ops.device_status()
+
+
 @pytest.fixture
 def four_pairs():
     """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all."""

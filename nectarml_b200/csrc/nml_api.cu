@@ -2003,12 +2003,13 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
                        void* out, float* db, Bump& ws, cudaStream_t st) {
     if (!d || d->rows <= 0 || d->in_features <= 0 || d->out_features <= 0) return NML_ERR_INVALID;
     g_last_scratch_error[0] = 0;
-    if (tune().gemm && d->math == NML_MATH_3XTF32 && d->in_dtype == NML_F32 && (pass == NML_PASS_BACKWARD_WEIGHT || d->w_dtype == NML_F32) &&
+    const int operands = d->math == NML_MATH_3XTF32 ? NML_F32 : d->math == NML_MATH_F16 ? NML_F16 : -1;
+    if (tune().gemm && d->in_dtype == operands && (pass == NML_PASS_BACKWARD_WEIGHT || d->w_dtype == operands) &&
         g_sm_limit.load(std::memory_order_relaxed) == 0) {
         const int R = d->rows, I = d->in_features, O = d->out_features;
         StridedProduct g;
         memset(&g, 0, sizeof(g));
-        g.dtype = NML_F32;
+        g.dtype = operands;
         g.batch = 1;
         g.out = out;
         g.out_dtype = pass == NML_PASS_BACKWARD_WEIGHT ? NML_F32 : d->out_dtype;
@@ -2035,12 +2036,24 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
         // 10.2 / 25.0 / 18.4 (9.6 / 12.9 / 21.9), 20 x 4000 -> 200 17.4 / 13.6 / 12.5 (18.3 / 9.3 / 7.8): the estimates up to which
         // this path was the faster.
         // (a weight gradient of fewer than eight tiles is the contraction kernel's: it cuts K into up to 192 shares)
+        // fp16 operands that are read in place by TMA need no conversions in the first place, and an operand whose rows are the inner
+        // dimension is eight 2-byte loads a chunk here: forward only, with one or two K slices (500 x 128 -> 512 5.8 -> 4.7 us, 2000 x
+        // 90 -> 400 9.1 -> 7.8; four slices, 4000 x 256 -> 100, 8.4 and 8.5; 32 x 512 -> 2048, whose loop blocks would share, 6.8 and
+        // 6.5 from L2 but 6.4 and 6.6 from HBM).  Rows that TMA is to read and cannot, because the matrix does not start on 16 bytes,
+        // stay refused.
         const StridedPlan plan = plan_strided(g, planning_sms());
-        const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
-        if (!few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0)) {
+        bool in_place;
+        if (operands == NML_F32) {
+            const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
+            in_place = !few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0);
+        } else {
+            const bool starts = ((reinterpret_cast<uintptr_t>(in0) | reinterpret_cast<uintptr_t>(in1)) & 15) == 0;
+            in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms() && (starts || I % 8 != 0);
+        }
+        if (in_place) {
             RowsColsum sums;
             if (pass == NML_PASS_BACKWARD_WEIGHT && db) {
-                sums.plan(in1, NML_F32, R, O, db);
+                sums.plan(in1, operands, R, O, db);
                 sums.cs = colsum_scratch(ws, sums.grid.y, O);
             }
             if (ws.dry) return NML_OK;
@@ -2663,7 +2676,9 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             // Products of few blocks, in place: 128 x 33 x 64 x 33 fp16 10.0 -> 6.4 us, fp32 12.9 -> 7.3; 3 x 800 x 96 x 801 fp16 10.9 ->
             // 9.4, fp32 16.3 -> 10.4; 64 x 45 x 64 x 1001 fp32, two waves, 25.0 -> 15.6; more of them are the contraction kernel's: 64 x 333
             // x 64 x 333 fp32 25.1 against 28.7, 20 x 777 x 64 x 140 fp16, two waves, 9.3 against 12.9.
-            if (plan_strided(g, planning_sms()).us <= (es == 4 ? 18.0 : 10.5)) return bump.dry ? NML_OK : run_strided(g, PDL_NORMAL, nullptr, nullptr);
+            // (fp16 rows that TMA was to read and cannot stay refused)
+            const bool refused = es == 2 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) != 0;
+            if (!refused && plan_strided(g, planning_sms()).us <= (es == 4 ? 18.0 : 10.5)) return bump.dry ? NML_OK : run_strided(g, PDL_NORMAL, nullptr, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));

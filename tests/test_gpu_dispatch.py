@@ -70,9 +70,9 @@ def test_channel_major_results_of_any_width(n, c_in, h, w, c_out, k, s):
 
 # operands read in place: one row, one column, K of one value and of no whole slice, rows that start anywhere, K loops shared by the
 # blocks of a cluster (the last of them with nothing to do), two waves of blocks
-@pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (1, 70, 33), (129, 33, 130), (64, 513, 127), (33, 288, 65), (5, 2049, 3), (300, 36, 1025)])
+@pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (1, 70, 33), (129, 33, 130), (64, 513, 127), (33, 288, 65), (5, 2049, 3), (300, 36, 1025), (40, 96, 130)])
 @pytest.mark.parametrize("shift", [0, 1])
-def test_fp32_products_in_place(rows, fin, fout, shift, oracle):
+def test_products_in_place(rows, fin, fout, shift, oracle):
     rng = np.random.default_rng(rows + fin)
     sizes = {"x": (rows, fin), "w": (fout, fin), "dy": (rows, fout), "b": (fout,)}
     host_of = {k: rng.standard_normal(s, dtype=np.float32) for k, s in sizes.items()}
@@ -87,8 +87,13 @@ def test_fp32_products_in_place(rows, fin, fout, shift, oracle):
     dw, db = ops.linear_backward_weight(x, dy, math="3xtf32")
     assert_f32(host(dw), dyh.T.astype(np.float64) @ xh.astype(np.float64), "dw")
     assert_f32(host(db), dyh.astype(np.float64).sum(0), "db")
+    r = oracle.round_f16
+    atol = 1e-3 * max(1.0, fin ** 0.5)  # (of the results' size)
+    if shift == 0 or fin % 8:  # (rows that TMA would read have to start on 16 bytes)
+        x16, w16, b16 = (torch.cat([torch.zeros(shift, device="cuda"), dev(v).flatten()]).half()[shift:].view(v.shape) for v in (xh, wh, bh))
+        assert_f16(host(ops.linear_forward(x16, w16, b16)), oracle.linear_forward(r(xh), r(wh), r(bh)), "fp16 operands", atol=atol)
     half = host(ops.linear_forward(x, w, b, math="3xtf32", out_dtype=torch.float16))
-    assert_f16(half, oracle.linear_forward(xh, wh, bh), "fp16 result")
+    assert_f16(half, oracle.linear_forward(xh, wh, bh), "fp16 result", atol=atol)
     rounded = host(ops.linear_forward(x, w, b, math="3xtf32", round_out_f16=True))
     assert np.array_equal(rounded, half)
     assert torch.equal(y, ops.linear_forward(x, w, b, math="3xtf32"))

@@ -2091,11 +2091,16 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     f.w = in1; f.w_dtype = d->w_dtype; f.d0 = d->out_features; f.d1 = d->in_features; f.kh = f.kw = 1;
     f.k_is_dim0 = forward ? 0 : 1;
     f.w_direct = 1;
-    // Input gradient of a tall layer: W [out][in] read in place is an MN-major B operand, which the tensor core
-    // consumes ~10 % slower than a K-major one.  From 8192 rows on, a transposed fp16 copy W^T [in][out] (one
-    // coalesced pass over the weights, counted in the pass's duration) pays for itself.
-    if (!forward && d->rows >= 8192 && d->math == NML_MATH_F16 && d->w_dtype == NML_F16 && d->in_features % 8 == 0 &&
-        d->out_features % 64 == 0 && tune().wtrans) {
+    // Input gradient: W [out][in] read in place is an MN-major B operand.  Where its rows are no whole groups of 64 it takes a load per
+    // group and excludes CTA pairs, and a transposed fp16 copy W^T [in][out] (one coalesced pass over the weights, counted in the
+    // pass's duration) pays from 3e9 products on: 12000 x 520 -> 2048 55.6 -> 36.4 us, 10000 x 1000 -> 3000 116 -> 64, 5000 x 2040 -> 1000 45
+    // -> 36; 2000 x 2040 -> 1000 20.2 and 20.2, 2000 x 1000 -> 640 10.6 -> 12.7.  Whole groups are read almost as fast as a K-major
+    // operand: only very wide layers of many rows gain a little (16384 x 3072 -> 1024 93.5 -> 88.5, 8192 x 4096 -> 4096 213 -> 205;
+    // but 16384 x 512 -> 2048 33.3 -> 37.2, 16384 x 2048 -> 8192 360 -> 371).
+    const bool pays = d->in_features % 64 != 0 ? 1ll * d->rows * d->in_features * d->out_features >= 3000000000ll
+                                               : d->in_features >= 3072 && d->rows >= 8192;
+    if (!forward && d->math == NML_MATH_F16 && d->w_dtype == NML_F16 && d->in_features % 8 == 0 && d->out_features % 8 == 0 && pays &&
+        tune().wtrans) {
         __half* wt = static_cast<__half*>(ws.take(static_cast<size_t>(d->in_features) * d->out_features * sizeof(__half)));
         if (!ws.dry) {
             if (!ws.fits()) return NML_ERR_WORKSPACE;

@@ -133,6 +133,17 @@ def test_double_tiles_linear(rows, fin, fout, oracle, four_pairs):
     ops.device_status()
 
 
+# the transposed copy of the weights: widths of no whole groups on both sides of its limit, and very wide layers of many rows
+@pytest.mark.parametrize("rows,fin,fout", [(3000, 1000, 1000), (2900, 1000, 1000), (5003, 776, 1000), (8192, 3072, 128), (8200, 3080, 136)])
+def test_linear_input_gradient_with_transposed_weights(rows, fin, fout):
+    gen = torch.Generator(device="cuda").manual_seed(rows + fin)
+    dy = torch.randn(rows, fout, device="cuda", generator=gen).half()
+    w = (torch.randn(fout, fin, device="cuda", generator=gen) * 0.2).half()
+    want = dy.double() @ w.double()
+    assert_f16(host(ops.linear_backward_data(dy, w)), want.cpu().numpy(), "dx", atol=1e-3 * 0.2 * fout ** 0.5)
+    ops.device_status()
+
+
 @pytest.mark.parametrize("rows,fin,fout", [(4096, 640, 512), (4096, 1280, 512), (4100, 1280, 456), (2048, 256, 2304)])
 def test_double_tiles_linear_weight_gradient(rows, fin, fout, oracle, four_pairs):
     rng = np.random.default_rng(rows + fin)

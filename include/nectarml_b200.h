@@ -139,6 +139,14 @@ int nml_conv_forward_static(const nml_conv_desc* d, const void* x, const void* w
 int nml_conv_backward_data(const nml_conv_desc* d, const void* dy, const void* w, void* dx,
                            void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same with a second gradient of the layer's input added before the result is rounded: dx += add * (bit ? 1 : add_below),
+ * where add is fp16 NHWC like dx and add_mask holds one bit per element (bit j of byte i: element 8 * i + j; NULL: all set).
+ * With the output gradient and the mask of the normalisation that ends a residual block, this is the whole gradient of
+ * the block's input, in one pass over it; the reference adds the two in a pass of its own.  fp16 math, fp16 NHWC result,
+ * c_in a multiple of 8 and more than 16 / (stride_h * stride_w); dx and add 16-byte aligned. */
+int nml_conv_backward_data_add(const nml_conv_desc* d, const void* dy, const void* w, const void* add, const void* add_mask,
+                               float add_below, void* dx, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Weight gradient (overwrites dw, fp32, weight-shaped) and, when db != NULL, the bias gradient
  * db[c] = sum over batch and pixels of dy (fp32).  dw is bitwise repeatable from run to run: K
  * slices store partial sums into planes of the workspace that a second kernel adds in a fixed

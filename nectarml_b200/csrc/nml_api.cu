@@ -198,6 +198,7 @@ static UmmaKernel fprop_instance(bool f16) {
     return f16 ? umma_conv_kernel<MODE_FPROP, kOut, true, kPair> : umma_conv_kernel<MODE_FPROP, kOut, false, kPair>;
 }
 static UmmaKernel kernel_for(const KParams& P) {
+    if (P.add) return umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, false, false, true>;
     if (P.dbl)
         return P.mode == MODE_WGRAD ? umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true> : umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>;
     if (P.mode == MODE_WGRAD)
@@ -224,7 +225,7 @@ static int raise_smem_limit() {
         NML_CUDA(cudaFuncSetAttribute(gemm_instance<float>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
         NML_CUDA(cudaFuncSetAttribute(gemm_instance<__half>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
     }
-    UmmaKernel all[18] = {umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
+    UmmaKernel all[19] = {umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, false, false, true>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
                           umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true>,
                           fprop_instance<OUT_NHWC_TMA, false>(true), fprop_instance<OUT_NHWC_TMA, false>(false),
                           fprop_instance<OUT_NCHW_TMA, false>(true), fprop_instance<OUT_NCHW_TMA, false>(false),
@@ -256,7 +257,7 @@ static int load_helper_kernels() {
         (const void*)pack_phase_weights_kernel<float, float>, (const void*)pack_phase_weights_kernel<float, __half>,
         (const void*)pack_phase_weights_kernel<__half, float>, (const void*)pack_phase_weights_kernel<__half, __half>,
         (const void*)to_float_kernel<__half>, (const void*)colsum_finish_kernel,
-        (const void*)repack_half_tile_kernel, (const void*)repack_half_rows_kernel, (const void*)wgrad_reduce_taps_kernel,
+        (const void*)add_masked_kernel, (const void*)repack_half_tile_kernel, (const void*)repack_half_rows_kernel, (const void*)wgrad_reduce_taps_kernel,
         (const void*)wgrad_reduce_rows4_kernel, (const void*)wgrad_reduce_kernel, (const void*)wgrad_reduce_deep4_kernel,
     };
     for (const void* f : fns) {
@@ -701,7 +702,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     int stages2 = P.dbl ? 0 : (232448 - fixed - P.epi_warps * 2 * kStagingBufBytes) / stage_bytes;
     const int bufs1 = P.dbl && !tma_out ? 0 : 1;
     int stages1 = (232448 - fixed - P.epi_warps * bufs1 * kStagingBufBytes) / stage_bytes;
-    P.stg_bufs = (stages2 >= std::min(stages1, 8)) ? 2 : bufs1;
+    P.stg_bufs = (stages2 >= std::min(stages1, 8) || (P.add && stages2 >= 3)) ? 2 : bufs1;
     int stages = std::min(8, P.stg_bufs == 2 ? stages2 : stages1);
     stages = std::max(2, std::min(stages, tune().stages));
     P.stages = stages;
@@ -794,6 +795,9 @@ struct FpropLike {
     int math, round_f16;
     // phase-packed gather walk (set by run_fprop_like itself): the real output behind the packed columns
     int shuf_sh, shuf_sw, shuf_c, shuf_oh, shuf_ow;
+    const void* add;  // fp16, laid out like the (fp16 NHWC) result, added to it: see KParams::add
+    const void* add_mask;
+    float add_below;
     int w_batched;  // every image has its own [d0][d1] weights, one after the other (batched matmul; kh = kw = 1)
 };
 
@@ -1275,7 +1279,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             uint32_t cb[4] = {static_cast<uint32_t>(cpi), static_cast<uint32_t>(bw * P.out_stride_w),
                               static_cast<uint32_t>(bh * P.out_stride_h), static_cast<uint32_t>(bnn)};
             uint32_t ce[4] = {1, static_cast<uint32_t>(P.out_stride_w), static_cast<uint32_t>(P.out_stride_h), 1};
-            if (cb[1] <= 256 && cb[2] <= 256 && encode_map(&P.tmC, f.out, esz, 4, cd, cb, ce, SWZ_128B) == NML_OK)
+            if (cb[1] <= 256 && cb[2] <= 256 && encode_map(&P.tmC, f.out, esz, 4, cd, cb, ce, SWZ_128B) == NML_OK &&
+                (!f.add || encode_map(&P.tmD, f.add, esz, 4, cd, cb, ce, SWZ_128B) == NML_OK))
                 P.out_mode = OUT_NHWC_TMA;
         }
     }
@@ -1322,7 +1327,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     // Pairs save operand feed, which shows over a long K loop or many tiles: with 4 slices, or with 8 and one or two tiles per
     // SM, single CTAs measured 3-14 % faster (they drain twice as many independent tiles).
     const bool pair_k = k_iters_min >= 12 || (k_iters_min >= 5 && tiles_single > 2ll * limited(ds->sms));
-    P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && pair_k &&
+    P.pair = (tune().pair && !P.patch && !f.add && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && pair_k &&
               (P.out_mode == OUT_NHWC_TMA || P.out_mode == OUT_NCHW_TMA || P.out_mode == OUT_NCHW) && limited(ds->sms) >= 2) ? 1 : 0;
     // Double tiles: pairs that write fp16 rows by TMA stores.  The phases of a gather are planned by their sum.
     if (P.pair && P.out_mode == OUT_NHWC_TMA && P.out_f16 && P.planes == 1 && (P.bn == 256 || P.bn == 128)) {
@@ -1460,6 +1465,11 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             ++g_launches;
         }
     }
+    if (f.add && P.out_mode == OUT_NHWC_TMA) {
+        P.add = 1;
+        P.add_mask = static_cast<const uint8_t*>(f.add_mask);
+        P.add_below = f.add_below;
+    }
     int slot = -1;
     rc = launch_kernel(P, ds, st, &slot);
     if (rc) return rc;
@@ -1474,6 +1484,14 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         else
             { helper_launch(4 * kSms, finish_rows_kernel<float>, blocks, 256, 0, st, split_acc, P.fsplit, bias32, static_cast<float*>(f.out), out_pixels, N,
                                                              f.out_h * f.out_w, nchw, f.round_f16, vec); ++g_launches; }
+        NML_CUDA(cudaGetLastError());
+    }
+    if (f.add && !P.add) {  // a K-split walk, few channels, a result that TMA does not store
+        const size_t vectors = out_pixels * N / 8;
+        const int blocks = static_cast<int>(std::min<size_t>((vectors + 255) / 256, 148 * 16));
+        helper_launch(4 * kSms, add_masked_kernel, blocks, 256, 0, st, static_cast<uint4*>(f.out), static_cast<const uint4*>(f.add),
+                      static_cast<const uint8_t*>(f.add_mask), f.add_below, vectors);
+        ++g_launches;
         NML_CUDA(cudaGetLastError());
     }
     if (open_slot) {
@@ -1947,7 +1965,7 @@ static bool conv_out_size(const nml_conv_desc* d, int* ho, int* wo) {
 }
 
 static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const void* in1, const void* bias, void* out,
-                     float* db, Bump& ws, cudaStream_t st) {
+                     float* db, Bump& ws, cudaStream_t st, const void* add = nullptr, const void* add_mask = nullptr, float add_below = 0.f) {
     int ho, wo;
     g_last_scratch_error[0] = 0;  // a workspace error reported from here on is not the static entry point's
     if (!conv_out_size(d, &ho, &wo)) return NML_ERR_INVALID;
@@ -1996,6 +2014,7 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
     f.bias = forward ? bias : nullptr; f.bias_dtype = d->w_dtype;
     f.math = d->math;
     f.round_f16 = forward ? d->round_out_f16 : 0;
+    f.add = add; f.add_mask = add_mask; f.add_below = add_below;
     return run_fprop_like(f, ws, st);
 }
 
@@ -2280,6 +2299,16 @@ int nml_conv_backward_data(const nml_conv_desc* d, const void* dy, const void* w
     if (!d || !dy || !w || !dx) return NML_ERR_INVALID;
     Bump ws{static_cast<uint8_t*>(workspace), 0, workspace ? workspace_bytes : 0, false};
     return conv_pass(d, NML_PASS_BACKWARD_DATA, dy, w, nullptr, dx, nullptr, ws, static_cast<cudaStream_t>(stream));
+}
+
+int nml_conv_backward_data_add(const nml_conv_desc* d, const void* dy, const void* w, const void* add, const void* add_mask, float add_below,
+                               void* dx, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!d || !dy || !w || !dx || !add || ((reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(dx)) & 15)) return NML_ERR_INVALID;
+    // (phase-packed columns have their own stores, which do not add)
+    if (d->out_dtype != NML_F16 || d->out_layout != NML_NHWC || d->math != NML_MATH_F16 || d->c_in % 8 || d->stride_h * d->stride_w * d->c_in <= 16)
+        return NML_ERR_UNSUPPORTED;
+    Bump ws{static_cast<uint8_t*>(workspace), 0, workspace ? workspace_bytes : 0, false};
+    return conv_pass(d, NML_PASS_BACKWARD_DATA, dy, w, nullptr, dx, nullptr, ws, static_cast<cudaStream_t>(stream), add, add_mask, add_below);
 }
 
 int nml_conv_backward_weight(const nml_conv_desc* d, const void* x, const void* dy, float* dw, float* db,

@@ -865,6 +865,28 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* planes, 
     pdl_leave(role);
 }
 
+// out += add, scaled by `below` where the mask has no bit (null: nowhere), in vectors of eight fp16 values; summed in fp32.
+__global__ void __launch_bounds__(256) add_masked_kernel(uint4* out, const uint4* add, const uint8_t* mask, float below, size_t n, int role) {
+    pdl_enter(role);
+    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        uint4 a = load_global(out + i);
+        const uint4 b = load_global(add + i);
+        const unsigned bits = mask ? load_global(mask + i) : 0xffu;
+        __half2* x = reinterpret_cast<__half2*>(&a);
+        const __half2* y = reinterpret_cast<const __half2*>(&b);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float2 s = __half22float2(x[j]);
+            const float2 t = __half22float2(y[j]);
+            s.x += (bits >> (2 * j)) & 1u ? t.x : t.x * below;
+            s.y += (bits >> (2 * j + 1)) & 1u ? t.y : t.y * below;
+            x[j] = __floats2half2_rn(s.x, s.y);
+        }
+        out[i] = a;
+    }
+    pdl_leave(role);
+}
+
 template <typename TIn>
 __global__ void __launch_bounds__(256) to_float_kernel(const TIn* in, float* out, int n, int role) {
     pdl_enter(role);

@@ -77,6 +77,7 @@ struct KParams {
                          // wgrad: the tensor patches are cut from
     CUtensorMap tmB[2];  // fprop: weights; wgrad: the plainly indexed tensor
     CUtensorMap tmC;     // OUT_NHWC_TMA: the output, box = the 32 rows x 128 bytes one epilogue warp owns
+    CUtensorMap tmD;     // the same of `add`
     int mode, out_mode;
     int pdl_role;        // PDL_NORMAL, or PDL_LEADER in front of column sums that run beside this launch
     int num_tiles, n_tiles;
@@ -121,6 +122,11 @@ struct KParams {
     // (n, i, j) scatters to out[n][shuf_sh*i + ph][shuf_sw*j + pw][c] (row-major output only).
     int shuf_sh, shuf_sw;  // 0 = off
     int shuf_c, shuf_oh, shuf_ow;
+    // Added to the result before it is rounded (kAdd): a tensor of its shape, scaled by add_below where the mask has no bit (one bit
+    // per element; null: nowhere).  The gradient that reaches a layer's input by another way, see nml_conv_backward_data_add.
+    int add;
+    const uint8_t* add_mask;
+    float add_below;
     // Weight-gradient patch walk (unit column stride, one 64-channel group per tap): a CTA owns a slice of
     // the K blocks (8 x 8 pixels of one image) and ALL row tiles of the gradient at once.  Per K block it
     // loads one haloed patch of the tensor the taps are cut from and one box of the other tensor; row tile
@@ -292,9 +298,10 @@ __device__ __forceinline__ void store_columns(T* o, size_t stride, const uint32_
 // clocks and takes 1045 to 1060 (Linear; convolutions, whose slices arrive in more pieces, 720 and 1350).  At 256 columns the two
 // accumulators fill TMEM, so nothing overlaps the drain: the epilogue takes a tile into registers as fp16 and hands the
 // accumulators back before it stores anything, one group of four warps to a row tile.
-template <int kMode, int kOutMode, bool kOutF16, bool kPair, bool kDbl = false>
+template <int kMode, int kOutMode, bool kOutF16, bool kPair, bool kDbl = false, bool kAdd = false>
 __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1) umma_conv_kernel(const __grid_constant__ KParams P) {
     static_assert(!kDbl || kPair, "double tiles are tiles of CTA pairs");
+    static_assert(!kAdd || (kMode == MODE_FPROP && kOutMode == OUT_NHWC_TMA && kOutF16 && !kPair), "sums are fp16 rows of single CTAs");
     constexpr int kRowTiles = kDbl ? 2 : 1;
     constexpr bool kPoll = kMode == MODE_FPROP && kOutF16 && !kDbl;  // how waits begin, see mbar_poll
     extern __shared__ uint8_t smem_raw[];
@@ -320,7 +327,8 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
     uint64_t* aempty_bar = afull_bar + 4;                             // [4]
     uint64_t* bres_bar = aempty_bar + 4;                              // [1] patch walk: resident B has landed
     uint64_t* turn_bar = bres_bar + 1;                                // [2] patch walk, two issuers: whose turn it is
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(turn_bar + 2);
+    uint64_t* add_bar = turn_bar + 2;                                 // [8] sums: an epilogue warp's addend has landed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(add_bar + 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);  // abort state: 4 ints, 8-byte aligned
 
     const int warp = threadIdx.x >> 5;
@@ -347,6 +355,8 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
         mbar_init(smem_u32(bres_bar), 1);
         mbar_init(smem_u32(&turn_bar[0]), 1);
         mbar_init(smem_u32(&turn_bar[1]), 1);
+        if (kAdd)
+            for (int w = 0; w < 8; ++w) mbar_init(smem_u32(&add_bar[w]), 1);
         abort_state_init(abort_flag, P.wait_limit_ns);
         fence_mbar_init();
         tma_prefetch_desc(&P.tmA[0]);
@@ -1311,6 +1321,8 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                 const int half = ((P.bn / cpi + 1) / 2) * cpi;
                 if (ew < 4) c_end = min(half, P.bn); else c_begin = half;
             }
+            uint32_t add_parity = 0;
+            bool add_flying = false;
             const int t_step = P.epi_alt ? 2 : 1;
             titer = (P.epi_alt && ew >= 4) ? 1 : 0;
             int p = 0;  // phase of the tile (tile ids only grow)
@@ -1343,6 +1355,27 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                     for (int u = 0; u < 8; ++u)
                         if (lane + 32 * u < P.bn) btw[lane + 32 * u] = bv[u];
                     __syncwarp();
+                }
+                // A sum's other addend: the box of a piece is loaded into the staging buffer it will leave from, one piece ahead
+                // where there are two buffers, and each lane adds its row in place.  A 256-channel 56 x 56 block at batch 256: 2048 us
+                // with the two gradients stored and added by torch, 1952 with the addend loaded by each lane from its own row (32
+                // lines an instruction), 1861 so.
+                auto load_addend = [&](int c, uint32_t seq) {
+                    if (lane == 0) {
+                        bulk_wait_group_read<0>();  // the store that last read this buffer
+                        mbar_arrive_expect_tx(smem_u32(&add_bar[ew]), kStagingBufBytes);
+                        tma_load_4d(stg0 + (P.stg_bufs == 2 ? (seq & 1) * kStagingBufBytes : 0), &P.tmD, smem_u32(&add_bar[ew]), col_base + c, sw, sh, sn);
+                    }
+                    add_flying = true;
+                };
+                size_t add_at = 0;  // this lane's row, for its bits
+                bool add_ok = false;
+                if constexpr (kAdd) {
+                    const int iw = (tw << P.wb_log2) + (row & (wb - 1)), ih = (th << P.hb_log2) + ((row >> P.wb_log2) & (hb - 1));
+                    const int n = (tn << P.nb_log2) + (row >> (P.wb_log2 + P.hb_log2));
+                    add_ok = iw < ph.wq && ih < ph.hq && n < P.batch;
+                    add_at = ((static_cast<size_t>(n) * P.out_h + ph.ph + P.out_stride_h * ih) * P.out_w + ph.pw + P.out_stride_w * iw) * P.ld_out + col_base;
+                    if (c_begin < c_stop) load_addend(c_begin, store_seq);
                 }
                 const int buf = titer & ((1 << P.tbufs_log2) - 1);
                 const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * P.bn * P.planes;
@@ -1394,6 +1427,30 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         }
                     }
                     if (live && !more) hand_back();
+                    uint32_t add_bits[2] = {0xffffffffu, 0xffffffffu};
+                    if constexpr (kAdd) {
+                        if (P.add_mask != nullptr) {
+                            const uint8_t* m = P.add_mask + (add_at + c0) / 8;
+                            add_bits[0] = add_bits[1] = 0u;
+                            if ((P.ld_out & 63) == 0) {
+                                if (add_ok) {
+                                    const uint2 b = load_global(reinterpret_cast<const uint2*>(m));
+                                    add_bits[0] = b.x, add_bits[1] = b.y;
+                                }
+                            } else {
+#pragma unroll
+                                for (int q = 0; q < 8; ++q)
+                                    if (add_ok && col_base + c0 + 8 * q < P.c_out) add_bits[q >> 2] |= load_global(m + q) << (8 * (q & 3));
+                            }
+                        }
+                        if (!__all_sync(0xffffffffu, mbar_wait<kPoll>(smem_u32(&add_bar[ew]), add_parity, abort_flag, P.err, ERR_WAIT_FULL))) {
+                            ok = false;
+                            break;
+                        }
+                        add_parity ^= 1;
+                        add_flying = false;
+                        if (cn < c_stop && P.stg_bufs == 2) load_addend(cn, store_seq + 1);
+                    } else
                     // the store that last read this buffer must be done reading it
                     if (lane == 0) {
                         if (P.stg_bufs == 2) bulk_wait_group_read<1>(); else bulk_wait_group_read<0>();
@@ -1430,6 +1487,17 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                                 v[0] += ba.x; v[1] += ba.y; v[2] += ba.z; v[3] += ba.w;
                                 v[4] += bb.x; v[5] += bb.y; v[6] += bb.z; v[7] += bb.w;
                             }
+                            if constexpr (kAdd) {
+                                const uint4 addend = ld_shared_v4(buf_addr + lane * 128 + ((qq ^ (lane & 7)) << 4));
+                                const __half2* g = reinterpret_cast<const __half2*>(&addend);
+                                const uint32_t bits = add_bits[qq >> 2] >> (8 * (qq & 3));
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const float2 t = __half22float2(g[j]);
+                                    v[2 * j] += (bits >> (2 * j)) & 1u ? t.x : t.x * P.add_below;
+                                    v[2 * j + 1] += (bits >> (2 * j + 1)) & 1u ? t.y : t.y * P.add_below;
+                                }
+                            }
                             pk.x = pack_half2(v[0], v[1]);
                             pk.y = pack_half2(v[2], v[3]);
                             pk.z = pack_half2(v[4], v[5]);
@@ -1461,8 +1529,20 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         bulk_commit_group();
                     }
                     ++store_seq;
+                    if constexpr (kAdd) {
+                        if (cn < c_stop && P.stg_bufs == 1) load_addend(cn, store_seq);
+                    }
                     if (more) tmem_ld_wait();
                 }
+                if (kAdd && !ok) break;
+            }
+            if (kAdd && add_flying) {  // (gave up: a bounded chance to land, as for the operands)
+                const uint64_t t0 = globaltimer_ns();
+                while (!mbar_try_wait(smem_u32(&add_bar[ew]), add_parity))
+                    if (globaltimer_ns() - t0 > 2000000ull) {
+                        atomicCAS(P.err, 0, ERR_WAIT_DRAIN);
+                        break;
+                    }
             }
             if (lane == 0) bulk_wait_group<0>();  // stores must land before the CTA ends
         } else

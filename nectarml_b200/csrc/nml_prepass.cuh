@@ -3,6 +3,7 @@
 // 3xTF32 split, with the bias-gradient column sum folded into the same pass over dY),
 // weight repacking into the K-major [n][tap][k] operand, and small utilities.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -328,6 +329,59 @@ __global__ void __launch_bounds__(256) colsum_vectors_kernel(const TIn* in, floa
         for (int w = 0; w < 8; ++w) sum += part[w][threadIdx.x];
         colsum[static_cast<size_t>(blockIdx.y) * C + c] = sum;
     }
+    pdl_leave(role);
+}
+
+// The same in one launch, for matrices of few enough rows: the row blocks of a column block form a cluster, which adds their
+// sums through distributed shared memory, in order.  Eight rows are added up by themselves before they join a thread's sum,
+// so no chain of additions is longer than in the two stages.
+constexpr int kColsumCluster = 8;
+template <typename TIn>
+__global__ void __launch_bounds__(256) colsum_cluster_kernel(const TIn* in, float* __restrict__ out, int R, int C, int rows_per_block, int role) {
+    pdl_enter(role);
+    constexpr int V = 16 / sizeof(TIn), kCols = 32 * V, kShare = kCols / kColsumCluster;
+    __shared__ float part[8][kCols];
+    __shared__ float sum[kCols];
+    const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    const int rank = blockIdx.x % kColsumCluster, col0 = blockIdx.x / kColsumCluster * kCols, c0 = col0 + lane * V;
+    const int r0 = rank * rows_per_block, r1 = min(R, r0 + rows_per_block);
+    float acc[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] = 0.f;
+    if (c0 < C) {
+        const TIn* p = in + c0;
+        for (int r = r0 + wy; r < r1; r += 64) {
+            uint4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                v[i] = r + 8 * i < r1 ? load_global(reinterpret_cast<const uint4*>(p + static_cast<size_t>(r + 8 * i) * C)) : make_uint4(0u, 0u, 0u, 0u);
+            float eight[V];
+#pragma unroll
+            for (int j = 0; j < V; ++j) eight[j] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) add_vector(eight, v[i], p);
+#pragma unroll
+            for (int j = 0; j < V; ++j) acc[j] += eight[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < V; ++j) part[wy][lane * V + j] = acc[j];
+    __syncthreads();
+    if (threadIdx.x < kCols) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += part[w][threadIdx.x];
+        sum[threadIdx.x] = s;
+    }
+    cooperative_groups::this_cluster().sync();
+    const int c = rank * kShare + threadIdx.x;
+    if (threadIdx.x < kShare && col0 + c < C) {
+        float s = 0.f;
+#pragma unroll
+        for (int r = 0; r < kColsumCluster; ++r) s += cooperative_groups::this_cluster().map_shared_rank(sum, r)[c];
+        out[col0 + c] = s;
+    }
+    cooperative_groups::this_cluster().sync();  // no block leaves while another reads its sums
     pdl_leave(role);
 }
 

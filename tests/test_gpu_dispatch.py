@@ -105,6 +105,21 @@ def test_products_in_place(rows, fin, fout, shift, oracle):
     ops.device_status()
 
 
+# column sums in one launch up to 1024 rows: fewer rows than blocks of a cluster, a share that is no multiple of eight, the last
+# vector of the last column block, both sides of the limit
+@pytest.mark.parametrize("rows", [1, 7, 9, 64, 65, 519, 1024, 1025])
+@pytest.mark.parametrize("fout", [8, 264, 520])
+def test_bias_gradient_sums(rows, fout):
+    gen = torch.Generator(device="cuda").manual_seed(rows + fout)
+    for dt, math in ((torch.float16, "f16"), (torch.float32, "3xtf32")):
+        x = torch.randn(rows, 64, device="cuda", generator=gen).to(dt)
+        dy = (torch.randn(rows, fout, device="cuda", generator=gen) + 0.5).to(dt)
+        _, db = ops.linear_backward_weight(x, dy, math=math)
+        assert_f32(host(db), dy.double().sum(0).cpu().numpy(), f"db {dt}", tol=1e-6)
+        assert torch.equal(db, ops.linear_backward_weight(x, dy, math=math)[1])
+    ops.device_status()
+
+
 @pytest.fixture
 def four_pairs():
     """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all."""

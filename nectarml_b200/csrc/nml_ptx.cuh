@@ -72,9 +72,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 }
 
 // The same without the hint, which costs a wait that finds its phase over 35 clocks (117 instead of 82).  As the first poll of
-// every wait it makes forward walks of single tiles with fp16 results 2 to 4 % faster (3x3 64 -> 64 at 56 x 56, batch 256 75.6 -> 72 us, 4096 x
-// 2048 -> 8192 106 -> 103), weight gradients 4 to 5 % slower (16384 x 2048 -> 8192 466 -> 486), double tiles 2 % (3x3 512 at
-// 7 x 7, batch 256 57.5 -> 58.8) and fp32 results 1 % (3x3 64 at 56 x 56, batch 8 30.7 -> 31.1), whose waits mostly find their phase not over: those begin with the hint.
+// every wait it makes forward walks of single tiles with fp16 results 2 to 4 % faster (3x3 64 -> 64 at 56 x 56, batch 256 75.6 ->
+// 72 us, 4096 x 2048 -> 8192 106 -> 103), weight gradients 4 to 5 % slower (16384 x 2048 -> 8192 466 -> 486), double tiles 2 % (3x3
+// 512 at 7 x 7, batch 256 57.5 -> 58.8) and fp32 results 1 % (3x3 64 at 56 x 56, batch 8 30.7 -> 31.1), whose waits mostly find their
+// phase not over: those begin with the hint.
 __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(

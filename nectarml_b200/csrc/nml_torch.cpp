@@ -738,14 +738,21 @@ at::Tensor grad_or_zeros(const at::Tensor& g, at::IntArrayRef shape, const at::T
 // That is sound where both nodes are run whenever one is, the normalisation first: the convolution's input and the residual
 // are one output of the graph (equal edges, so the engine needs both gradients or neither), and the way from the
 // normalisation back to the convolution leads through input edges of nodes of this file alone (ancestors, so run later).
-// All of this is read off the graph when it is built.  What is left is kept per backward pass (its task's id), so passes over one
-// graph, one after another or in several threads, do not meet.
+// All of this is read off the graph when it is built; that no hook waits for either node's own gradients, when the
+// normalisation runs.  What is left is kept per backward pass (its task's id), so passes over one graph, one after another or in
+// several threads, do not meet.  (A pass that raises between the two leaves its part until the graph goes or runs to its end.)
 struct Handoff {
     struct Part {
         int task;
         at::Tensor dy, mask;  // no mask: no activation
         float below;
     };
+    std::weak_ptr<autograd::Node> taker;  // the convolution's node
+    // (its hooks are given the input gradient it returns, which has to be its own)
+    bool wanted() const {
+        const auto node = taker.lock();
+        return node && node->post_hooks().empty();
+    }
     std::mutex lock;
     std::vector<Part> parts;
     void leave(Part p) {
@@ -846,8 +853,10 @@ struct BnNode : LayerNode {
                 const auto& e = c->next_edge(0);
                 if (e.function == res_edge.function && e.input_nr == res_edge.input_nr) {
                     const auto& d = c->g.d;
-                    if (!c->incoming && c->needs_dx && c->made_on == here && d.c_in % 8 == 0 && d.stride_h * d.stride_w * d.c_in > 16)
+                    if (!c->incoming && c->needs_dx && c->made_on == here && d.c_in % 8 == 0 && d.stride_h * d.stride_w * d.c_in > 16) {
                         outgoing = c->incoming = std::make_shared<Handoff>();
+                        outgoing->taker = c->getptr();
+                    }
                     return;
                 }
                 n = e.function.get();
@@ -879,7 +888,7 @@ struct BnNode : LayerNode {
             const OutputGrad g = output_grad(dy, dwide.defined() ? &dwide : nullptr, join, in);
             autograd::variable_list out(4);
             // (a hook on this node would miss the gradient it returns)
-            const bool leave = outgoing && !join && !dwide.defined() && task_should_compute_output(1) && post_hooks().empty() &&
+            const bool leave = outgoing && !join && !dwide.defined() && task_should_compute_output(1) && post_hooks().empty() && outgoing->wanted() &&
                                (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15) == 0;
             if (residual && !leave) out[1] = new_empty(in.sizes(), in.options());
             owner->weight_gradient(grad_a, grad_b, [&](const at::Tensor& dgamma, const at::Tensor& dbeta) {

@@ -138,6 +138,35 @@ def test_block_input_gradient_reaches_whoever_asks():
     assert got[0] is not None and close(dx, fused)
 
 
+# a hook on the first convolution's node is given that convolution's input gradient, and what it puts in its place is all it
+# replaces: the residual's share is neither shown to it nor scaled by it
+@pytest.mark.parametrize("act", [train.ACT_NONE, train.ACT_RELU])
+def test_hook_on_the_first_convolution(act):
+    x0, dy = tensors()
+    block, x = Block(act=act), x0.clone().requires_grad_()
+    (fused,) = torch.autograd.grad(block(x), (x,), dy)
+
+    def first_convolution(node):
+        while node.name() != "ConvBackward" or node.next_functions[0][0].name() != "torch::autograd::AccumulateGrad":
+            node = node.next_functions[0][0]
+        return node
+
+    y = block(x)
+    residual = torch.where(y > 0, dy, torch.zeros_like(dy)) if act == train.ACT_RELU else dy
+    for scale in (None, 0.0):
+        seen = []
+
+        def hook(gi, go):
+            seen.append(gi[0].clone())
+            return None if scale is None else (gi[0] * scale, gi[1])
+
+        y = block(x)
+        first_convolution(y.grad_fn).register_hook(hook)
+        (dx,) = torch.autograd.grad(y, (x,), dy)
+        assert close(seen[0].double() + residual.double(), fused) and not close(seen[0], fused)
+        assert close(dx, fused) if scale is None else torch.equal(dx, residual)
+
+
 def test_block_input_gradient_on_two_streams_and_in_a_graph():
     x0, dy = tensors()
     block, x = Block(), x0.clone().requires_grad_()

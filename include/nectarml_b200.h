@@ -140,8 +140,8 @@ int nml_conv_backward_data(const nml_conv_desc* d, const void* dy, const void* w
                            void* workspace, size_t workspace_bytes, void* stream);
 
 /* The same with a second gradient of the layer's input added before the result is rounded: dx += add * (bit ? 1 : add_below),
- * where add is fp16 NHWC like dx and add_mask holds one bit per element (bit j of byte i: element 8 * i + j; NULL: all set).
- * With the output gradient and the mask of the normalisation that ends a residual block, this is the whole gradient of
+ * where add is fp16 NHWC like dx and add_mask holds one bit per element (bit j of byte i: element 8 * i + j; NULL: all set; any
+ * alignment).  With the output gradient and the mask of the normalisation that ends a residual block, this is the whole gradient of
  * the block's input, in one pass over it; the reference adds the two in a pass of its own.  fp16 math, fp16 NHWC result,
  * c_in a multiple of 8 and more than 16 / (stride_h * stride_w); dx and add 16-byte aligned. */
 int nml_conv_backward_data_add(const nml_conv_desc* d, const void* dy, const void* w, const void* add, const void* add_mask,

@@ -1432,7 +1432,8 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         if (P.add_mask != nullptr) {
                             const uint8_t* m = P.add_mask + (add_at + c0) / 8;
                             add_bits[0] = add_bits[1] = 0u;
-                            if ((P.ld_out & 63) == 0) {
+                            // (whole pieces of 64 columns are eight bytes of the mask, which may start anywhere)
+                            if ((P.ld_out & 63) == 0 && (reinterpret_cast<uintptr_t>(P.add_mask) & 7) == 0) {
                                 if (add_ok) {
                                     const uint2 b = load_global(reinterpret_cast<const uint2*>(m));
                                     add_bits[0] = b.x, add_bits[1] = b.y;

@@ -42,6 +42,28 @@ def test_input_gradient_with_an_addend(n, c_in, hw, c_out, k, s, masked):
     ops.device_status()
 
 
+# the mask's bytes may start anywhere: widths whose pieces are whole groups of eight bytes, and one whose are not
+@pytest.mark.parametrize("c_in", [64, 256, 72])
+@pytest.mark.parametrize("shift", [1, 4, 7])
+def test_mask_at_any_offset(c_in, shift):
+    gen = torch.Generator(device="cuda").manual_seed(c_in + shift)
+    rnd = lambda *shape: torch.randn(shape, device="cuda", generator=gen)  # noqa: E731
+    g = ConvGeometry(3, c_in, 10, 10, 64, 1, 1)
+    dy, w, add = rnd(3, 10, 10, 64).half(), (rnd(64, c_in, 1, 1) * 0.1).half(), rnd(3, 10, 10, c_in).half()
+    bits = torch.randint(0, 256, (add.numel() // 8,), device="cuda", generator=gen).to(torch.uint8)
+    moved = torch.cat([torch.zeros(shift, device="cuda", dtype=torch.uint8), bits])[shift:]
+    d = g.desc(_lib.NML_F16, "nhwc", _lib.NML_F16, "nhwc", _lib.NML_F16, "f16", False)
+    lib, need = _lib.load(), C.c_size_t()
+    _lib.check(lib.nml_conv_workspace_size(C.byref(d), 1, C.byref(need)))
+    ws, got = torch.empty(max(need.value, 1), dtype=torch.uint8, device="cuda"), []
+    for mask in (bits, moved):
+        got.append(torch.empty_like(add))
+        _lib.check(lib.nml_conv_backward_data_add(C.byref(d), dy.data_ptr(), w.data_ptr(), add.data_ptr(), mask.data_ptr(), 0.25,
+                                                  got[-1].data_ptr(), ws.data_ptr(), need.value, torch.cuda.current_stream().cuda_stream))
+    assert moved.data_ptr() % 8 == shift and torch.equal(*got)
+    ops.device_status()
+
+
 def test_input_gradient_with_an_addend_refuses():
     lib = _lib.load()
     t = torch.zeros(4096, device="cuda", dtype=torch.float16)

@@ -2039,6 +2039,14 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
     return run_fprop_like(f, ws, st);
 }
 
+// Whether TMA takes an fp16 matrix of `rows` rows of `inner` values, as the contraction kernel's own maps of it would find.
+static int rows_for_tma(const void* p, int inner, int rows) {
+    CUtensorMap tm;
+    const uint64_t dims[2] = {static_cast<uint64_t>(inner), static_cast<uint64_t>(rows)};
+    const uint32_t box[2] = {8, 1}, steps[2] = {1, 1};
+    return encode_map(&tm, p, 2, 2, dims, box, steps, SWZ_NONE);
+}
+
 static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, const void* in1, const void* bias,
                        void* out, float* db, Bump& ws, cudaStream_t st) {
     if (!d || d->rows <= 0 || d->in_features <= 0 || d->out_features <= 0) return NML_ERR_INVALID;
@@ -2080,15 +2088,19 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
         // dimension is eight 2-byte loads a chunk here: forward only, with one or two K slices (500 x 128 -> 512 5.8 -> 4.7 us, 2000 x
         // 90 -> 400 9.1 -> 7.8; four slices, 4000 x 256 -> 100, 8.4 and 8.5; 32 x 512 -> 2048, whose loop blocks would share, 6.8 and
         // 6.5 from L2 but 6.4 and 6.6 from HBM).  Rows that TMA is to read and cannot, because the matrix does not start on 16 bytes,
-        // stay refused.
+        // stay refused, by the map's own error (the plan's scratch, none, is no room for the contraction kernel to find out).
         const StridedPlan plan = plan_strided(g, planning_sms());
         bool in_place;
         if (operands == NML_F32) {
             const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
             in_place = !few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0);
         } else {
-            const bool starts = ((reinterpret_cast<uintptr_t>(in0) | reinterpret_cast<uintptr_t>(in1)) & 15) == 0;
-            in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms() && (starts || I % 8 != 0);
+            in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms();
+            if (in_place && !ws.dry && I % 8 == 0) {
+                int rc = rows_for_tma(in0, I, R);
+                if (!rc) rc = rows_for_tma(in1, I, O);
+                if (rc) return rc;
+            }
         }
         if (in_place) {
             RowsColsum sums;
@@ -2732,8 +2744,11 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             // 9.4, fp32 16.3 -> 10.4; 64 x 45 x 64 x 1001 fp32, two waves, 25.0 -> 15.6; more of them are the contraction kernel's: 64 x 333
             // x 64 x 333 fp32 25.1 against 28.7, 20 x 777 x 64 x 140 fp16, two waves, 9.3 against 12.9.
             // (fp16 rows that TMA was to read and cannot stay refused)
-            const bool refused = es == 2 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) != 0;
-            if (!refused && plan_strided(g, planning_sms()).us <= (es == 4 ? 18.0 : 10.5)) return bump.dry ? NML_OK : run_strided(g, PDL_NORMAL, nullptr, nullptr);
+            if (es == 2 && K % 8 == 0 && !bump.dry) {
+                const int rc = rows_for_tma(A, K, M);
+                if (rc) return rc;
+            }
+            if (plan_strided(g, planning_sms()).us <= (es == 4 ? 18.0 : 10.5)) return bump.dry ? NML_OK : run_strided(g, PDL_NORMAL, nullptr, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from gpu_util import F16, F32, assert_f16, assert_f32, dev, fetch, host
-from nectarml_b200 import _nectarml, ops
+from nectarml_b200 import _lib, _nectarml, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -102,6 +102,28 @@ def test_products_in_place(rows, fin, fout, shift, oracle):
         assert_f32(host(ops.linear_forward(x, w, b, math="3xtf32")), oracle.linear_forward(xh, wh, bh), "y, limited")
     finally:
         ops.set_sm_limit(0)
+    ops.device_status()
+
+
+# fp16 rows that TMA reads have to start on 16 bytes.  Where they do not, the call says so by the map that was refused, also at
+# sizes that are read in place and have no scratch.
+@pytest.mark.parametrize("rows,fin,fout", [(32, 56, 8), (11, 8, 22), (535, 128, 16), (300, 512, 256)])
+@pytest.mark.parametrize("which", ["x", "w"])
+def test_unaligned_rows_are_refused_by_name(rows, fin, fout, which):
+    t = {"x": (rows, fin), "w": (fout, fin)}
+    x, w = (torch.zeros(a * b + 1, device="cuda", dtype=torch.float16)[int(k == which):][:a * b].view(a, b) for k, (a, b) in t.items())
+    for bias in (None, torch.zeros(fout, device="cuda", dtype=torch.float16)):
+        with pytest.raises(_lib.NectarB200Error, match="cuTensorMapEncodeTiled"):
+            ops.linear_forward(x, w, bias)
+    ops.device_status()
+
+
+@pytest.mark.parametrize("batch,m,k,n", [(2, 4, 64, 7), (5, 300, 64, 301), (3, 700, 512, 264)])
+def test_unaligned_batched_rows_are_refused_by_name(batch, m, k, n):
+    a = torch.zeros(batch * m * k + 1, device="cuda", dtype=torch.float16)[1:]
+    b = torch.zeros(batch, k, n, device="cuda", dtype=torch.float16)
+    with pytest.raises(RuntimeError, match="cuTensorMapEncodeTiled"):
+        _nectarml.tensor.matmul(a.data_ptr(), b.data_ptr(), (batch, m, k), (batch, k, n), F16)
     ops.device_status()
 
 

@@ -2151,8 +2151,12 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     // but 16384 x 512 -> 2048 33.3 -> 37.2, 16384 x 2048 -> 8192 360 -> 371).
     const bool pays = d->in_features % 64 != 0 ? 1ll * d->rows * d->in_features * d->out_features >= 3000000000ll
                                                : d->in_features >= 3072 && d->rows >= 8192;
-    if (!forward && d->math == NML_MATH_F16 && d->w_dtype == NML_F16 && d->in_features % 8 == 0 && d->out_features % 8 == 0 && pays &&
-        tune().wtrans) {
+    // Weights that do not start on 16 bytes are no operand for TMA, but the copy's kernel takes them: from 8192 rows on, with whole groups
+    // of outputs, such a layer has its copy (and a workspace query, which sees no pointer, counts it); elsewhere it is refused.
+    const bool any_start = d->rows >= 8192 && d->out_features % 64 == 0;
+    const bool starts = (reinterpret_cast<uintptr_t>(in1) & 15) == 0;
+    if (!forward && d->math == NML_MATH_F16 && d->w_dtype == NML_F16 && d->in_features % 8 == 0 && d->out_features % 8 == 0 &&
+        (ws.dry ? pays || any_start : starts ? pays : any_start) && tune().wtrans) {
         __half* wt = static_cast<__half*>(ws.take(static_cast<size_t>(d->in_features) * d->out_features * sizeof(__half)));
         if (!ws.dry) {
             if (!ws.fits()) return NML_ERR_WORKSPACE;

@@ -181,6 +181,23 @@ def test_linear_input_gradient_with_transposed_weights(rows, fin, fout):
     ops.device_status()
 
 
+# weights that do not start on 16 bytes: through the copy from 8192 rows on with whole groups of 64 outputs, whether or not aligned ones
+# would take it, and refused elsewhere
+@pytest.mark.parametrize("rows,fin,fout,taken", [(8192, 512, 128, True), (8195, 520, 64, True), (8192, 3072, 64, True), (8192, 512, 136, False), (4096, 512, 128, False), (3000, 1000, 1000, False)])
+def test_linear_input_gradient_with_unaligned_weights(rows, fin, fout, taken):
+    gen = torch.Generator(device="cuda").manual_seed(rows + fin)
+    dy = torch.randn(rows, fout, device="cuda", generator=gen).half()
+    w = (torch.randn(fout * fin + 1, device="cuda", generator=gen) * 0.2).half()[1:].view(fout, fin)
+    if not taken:
+        with pytest.raises(_lib.NectarB200Error, match="cuTensorMapEncodeTiled"):
+            ops.linear_backward_data(dy, w)
+    else:
+        assert torch.equal(ops.linear_backward_data(dy, w), ops.linear_backward_data(dy, w.clone()))
+        want = dy.double() @ w.double()
+        assert_f16(host(ops.linear_backward_data(dy, w)), want.cpu().numpy(), "dx", atol=1e-3 * 0.2 * fout ** 0.5)
+    ops.device_status()
+
+
 @pytest.mark.parametrize("rows,fin,fout", [(4096, 640, 512), (4096, 1280, 512), (4100, 1280, 456), (2048, 256, 2304)])
 def test_double_tiles_linear_weight_gradient(rows, fin, fout, oracle, four_pairs):
     rng = np.random.default_rng(rows + fin)

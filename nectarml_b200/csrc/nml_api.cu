@@ -2095,7 +2095,8 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
             const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
             in_place = !few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0);
         } else {
-            in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms();
+            // (a launch that is to stall is the contraction kernel's)
+            in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms() && !g_dbg_short_a_box;
             if (in_place && !ws.dry && I % 8 == 0) {
                 int rc = rows_for_tma(in0, I, R);
                 if (!rc) rc = rows_for_tma(in1, I, O);

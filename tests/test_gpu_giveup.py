@@ -91,3 +91,19 @@ def test_contraction_kernel_unwinds_when_its_operands_never_land():
     ops.device_status()
     ref = torch.nn.functional.conv2d(xc.permute(0, 3, 1, 2).float(), wc.float(), padding=1).permute(0, 2, 3, 1)
     assert torch.allclose(yc.float(), ref, rtol=1e-2, atol=1e-3)
+
+
+def test_short_layers_stall_as_well():
+    """Layers of one or two K slices run in a kernel of their own, but not where the call asks for a stalled contraction."""
+    lib = _lib.load()
+    for fin in (64, 128):
+        x, w = torch.randn(512, fin, device=DEV).half(), torch.randn(128, fin, device=DEV).half()
+        y = torch.full((512, 128), 7.0, device=DEV, dtype=torch.float16)
+        d = _lib.LinearDesc(512, fin, 128, _lib.NML_F16, _lib.NML_F16, _lib.NML_F16, _lib.NML_MATH_F16, 0)
+        assert _status() == (0, 0)
+        assert lib.nml_debug_stalled_linear_forward(C.byref(d), x.data_ptr(), w.data_ptr(), y.data_ptr(), None, 0, 2_000_000,
+                                                    torch.cuda.current_stream().cuda_stream) == 0
+        st, code = _status()
+        assert st == NML_ERR_DEVICE and code in WAIT_CODES, (st, code)
+        assert bool((y == 7.0).all())
+    _linear_still_correct()

@@ -2342,6 +2342,10 @@ int nml_conv_backward_data(const nml_conv_desc* d, const void* dy, const void* w
 int nml_conv_backward_data_add(const nml_conv_desc* d, const void* dy, const void* w, const void* add, const void* add_mask, float add_below,
                                void* dx, void* workspace, size_t workspace_bytes, void* stream) {
     if (!d || !dy || !w || !dx || !add || ((reinterpret_cast<uintptr_t>(add) | reinterpret_cast<uintptr_t>(dx)) & 15)) return NML_ERR_INVALID;
+    // dx is written before add is read where the sum is a pass of its own
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(add), d0 = reinterpret_cast<uintptr_t>(dx);
+    const uintptr_t bytes = 2ull * std::max(d->batch, 0) * std::max(d->h, 0) * std::max(d->w, 0) * std::max(d->c_in, 0);
+    if (a0 < d0 + bytes && d0 < a0 + bytes) return NML_ERR_INVALID;
     // (phase-packed columns have their own stores, which do not add)
     if (d->out_dtype != NML_F16 || d->out_layout != NML_NHWC || d->math != NML_MATH_F16 || d->c_in % 8 || d->stride_h * d->stride_w * d->c_in <= 16)
         return NML_ERR_UNSUPPORTED;

@@ -64,13 +64,27 @@ def test_mask_at_any_offset(c_in, shift):
     ops.device_status()
 
 
+# (with all the scratch the call could want, so that nothing but the refusal in question stops it)
 def test_input_gradient_with_an_addend_refuses():
     lib = _lib.load()
-    t = torch.zeros(4096, device="cuda", dtype=torch.float16)
-    for layout, channels in (("nhwc", 12), ("nchw", 16)):
-        g = ConvGeometry(1, channels, 8, 8, 16, 3, 3, (1, 1), (1, 1))
+    dy, w, add, dx = (torch.zeros(8192, device="cuda", dtype=torch.float16) for _ in range(4))
+    ws = torch.empty(1 << 24, device="cuda", dtype=torch.uint8)
+    INVALID, UNSUPPORTED = 1, 4
+
+    def call(layout="nhwc", channels=16, stride=1, add=add, dx=dx, add_shift=0, dx_shift=0):
+        g = ConvGeometry(1, channels, 8, 8, 16, 3, 3, (stride, stride), (1, 1))
         d = g.desc(_lib.NML_F16, layout, _lib.NML_F16, layout, _lib.NML_F16, "f16", False)
-        assert lib.nml_conv_backward_data_add(C.byref(d), t.data_ptr(), t.data_ptr(), t.data_ptr(), None, 0.0, t.data_ptr(), None, 0, None) != _lib.NML_OK
+        return lib.nml_conv_backward_data_add(C.byref(d), dy.data_ptr(), w.data_ptr(), add.data_ptr() + add_shift, None, 0.0, dx.data_ptr() + dx_shift,
+                                              ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+
+    assert call(channels=24) == _lib.NML_OK and call(channels=8, stride=2) == _lib.NML_OK
+    assert call(channels=12) == UNSUPPORTED and call(channels=24, layout="nchw") == UNSUPPORTED
+    assert call(channels=16) == UNSUPPORTED and call(channels=8) == UNSUPPORTED  # (no more than 16 columns over all phases)
+    assert call(channels=24, add_shift=8) == INVALID and call(channels=24, dx_shift=2) == INVALID
+    for shift in (0, 16, 2 * 8 * 8 * 24 - 16):  # whole and partial overlap
+        assert call(channels=24, add=dx, add_shift=shift) == INVALID and call(channels=24, dx=add, dx_shift=shift) == INVALID
+    assert call(channels=24, add=dx, add_shift=2 * 8 * 8 * 24) == _lib.NML_OK
+    ops.device_status()
 
 
 class Block:

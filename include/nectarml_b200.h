@@ -143,9 +143,9 @@ int nml_conv_backward_data(const nml_conv_desc* d, const void* dy, const void* w
  * and add_mask holds one bit per element (bit j of byte i: element 8 * i + j; NULL: all set; any alignment).  With the output
  * gradient and the mask of the normalisation that ends a residual block, this is the whole gradient of the block's
  * input; the reference adds the two in a pass of its own.  Most plans add in fp32 before they round; where the sum is a pass of
- * its own (a K loop split over the SMs, c_in whose tiles no TMA store takes) the product is rounded to fp16 first and the sum,
- * taken in fp32, again.  fp16 math, fp16 NHWC result, c_in a multiple of 8 and more than 16 / (stride_h * stride_w); dx and
- * add 16-byte aligned and not overlapping. */
+ * its own (a K loop split over the SMs, pairs of SMs under a long K loop, c_in whose tiles no TMA store takes) the product is
+ * rounded to fp16 first and the sum, taken in fp32, again.  fp16 math, fp16 NHWC result, c_in a multiple of 8 and more than
+ * 16 / (stride_h * stride_w); dx and add 16-byte aligned and not overlapping. */
 int nml_conv_backward_data_add(const nml_conv_desc* d, const void* dy, const void* w, const void* add, const void* add_mask,
                                float add_below, void* dx, void* workspace, size_t workspace_bytes, void* stream);
 

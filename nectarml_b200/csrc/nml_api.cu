@@ -1348,8 +1348,20 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     // Pairs save operand feed, which shows over a long K loop or many tiles: with 4 slices, or with 8 and one or two tiles per
     // SM, single CTAs measured 3-14 % faster (they drain twice as many independent tiles).
     const bool pair_k = k_iters_min >= 12 || (k_iters_min >= 5 && tiles_single > 2ll * limited(ds->sms));
-    P.pair = (tune().pair && !P.patch && !f.add && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && pair_k &&
+    P.pair = (tune().pair && !P.patch && !P.b_batched && z_plan == 1 && pair_width && (!b_mn_major || N % mi.kb == 0) && pair_k &&
               (P.out_mode == OUT_NHWC_TMA || P.out_mode == OUT_NCHW_TMA || P.out_mode == OUT_NCHW) && limited(ds->sms) >= 2) ? 1 : 0;
+    // A sum is taken by single CTAs, whose staging buffers have room for the addend.  Under a long K loop pairs (and double tiles) save
+    // more than the pass costs that adds behind them: per million values 5.3e-4 us a K term at 256 columns (7.5e-4 at 128, where
+    // single CTAs are slower) against 0.92 us, and 2 us for its launch.  Single CTAs / pairs and the pass, us: 3x3 512 at 28 x 28, batch 16
+    // 69 / 64; at 7 x 7, batch 256 79 / 69; at 14 x 14, batch 64 79 / 66; 5x5 256 at 28 x 28, batch 64 138 / 122; 1x1 2048 -> 512 at 28 x 28,
+    // batch 64 117 / 109; even 3x3 256 at 14 x 14, batch 256 73 / 73; 3x3 128 at 56 x 56, batch 64 90 / 91; but 3x3 256 at 28 x 28, batch 16
+    // 30 / 34; 3x3 128 at 28 x 28, batch 64 27 / 29; 1x1 1024 -> 512 at 28 x 28, batch 64 70 / 72; 3x3 stride 2 512 at 28 x 28 69 / 76.
+    if (f.add && P.pair) {
+        long long slices = 0;
+        for (int p = 0; p < n_phases; ++p) slices += P.c_blocks * P.phases[p].tap_count;
+        const double mvalues = static_cast<double>(out_pixels) * N * 1e-6, terms = static_cast<double>(slices) * P.kb / n_phases;
+        P.pair = mvalues * terms * (P.bn == 256 ? 5.3e-4 : 7.5e-4) > 2.0 + 0.92 * mvalues ? 1 : 0;
+    }
     // Double tiles: pairs that write fp16 rows by TMA stores.  The phases of a gather are planned by their sum.
     if (P.pair && P.out_mode == OUT_NHWC_TMA && P.out_f16 && P.planes == 1 && (P.bn == 256 || P.bn == 128)) {
         int rows = 0, slices = 0;
@@ -1486,7 +1498,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             ++g_launches;
         }
     }
-    if (f.add && P.out_mode == OUT_NHWC_TMA) {
+    if (f.add && P.out_mode == OUT_NHWC_TMA && !P.pair) {
         P.add = 1;
         P.add_mask = static_cast<const uint8_t*>(f.add_mask);
         P.add_below = f.add_below;
@@ -1507,7 +1519,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                                                              f.out_h * f.out_w, nchw, f.round_f16, vec); ++g_launches; }
         NML_CUDA(cudaGetLastError());
     }
-    if (f.add && !P.add) {  // a K-split walk, few channels, a result that TMA does not store
+    if (f.add && !P.add) {  // a K-split walk, pairs, a result that TMA does not store
         const size_t vectors = out_pixels * N / 8;
         const int blocks = static_cast<int>(std::min<size_t>((vectors + 255) / 256, 148 * 16));
         helper_launch(4 * kSms, add_masked_kernel, blocks, 256, 0, st, static_cast<uint4*>(f.out), static_cast<const uint4*>(f.add),

@@ -42,6 +42,16 @@ def test_input_gradient_with_an_addend(n, c_in, hw, c_out, k, s, masked):
     ops.device_status()
 
 
+# which plan takes the sum, by its kernels (weights' repack, product, pass of the sum): pairs under a long K loop and many values leave
+# it to a pass, single CTAs add in the epilogue
+@pytest.mark.parametrize("n,c_in,hw,c_out,k,s,kernels", [
+    (11, 512, 28, 512, 3, 1, 3), (16, 256, 27, 1024, 3, 1, 3), (16, 128, 56, 512, 3, 1, 3), (3, 256, 56, 256, 3, 1, 2), (16, 512, 28, 128, 1, 1, 2), (13, 512, 27, 256, 4, 2, 2)])
+def test_sums_beside_pairs(n, c_in, hw, c_out, k, s, kernels):
+    before = ops.launch_count()
+    test_input_gradient_with_an_addend(n, c_in, hw, c_out, k, s, True)
+    assert ops.launch_count() - before == kernels
+
+
 # the mask's bytes may start anywhere: widths whose pieces are whole groups of eight bytes, and one whose are not
 @pytest.mark.parametrize("c_in", [64, 256, 72])
 @pytest.mark.parametrize("shift", [1, 4, 7])

@@ -1906,7 +1906,7 @@ struct StridedProduct {
 
 struct StridedPlan {
     int bn = 0, splits = 1;
-    double us = 0;
+    double us = 0, waves = 0, loop_us = 0;  // in all, waves of blocks, the K loops of all of them
 };
 // Tile width and blocks per tile by estimated time: 6.6 us for launch, set-up and drain, then a K slice by how full the SMs are
 // (alone 0.5 us at 32 columns, 0.6 at 64; with two blocks to every SM 1.1 and 1.3; 30 % more for an operand whose rows are the
@@ -1920,12 +1920,8 @@ static StridedPlan plan_strided(const StridedProduct& g, int sms) {
             const double blocks = static_cast<double>(tiles) * z, waves = std::ceil(blocks / (2.0 * sms));
             const double slice_us = (bn == 32 ? 0.5 : 0.6) * (1.0 + 0.6 * std::min(2.0, blocks / sms)) * (g.a_contiguous ? 1.0 : 1.3) *
                                     (g.b_contiguous ? 1.0 : 1.3);
-            const double us = 6.6 + waves * ceil_div(slices, z) * slice_us + (waves - 1.0) * 4.0;
-            if (best.bn == 0 || us < best.us) {
-                best.bn = bn;
-                best.splits = z;
-                best.us = us;
-            }
+            const double loop_us = waves * ceil_div(slices, z) * slice_us, us = 6.6 + loop_us + (waves - 1.0) * 4.0;
+            if (best.bn == 0 || us < best.us) best = {bn, z, us, waves, loop_us};
         }
     }
     return best;
@@ -1977,6 +1973,37 @@ static int run_strided(const StridedProduct& g, int role, DeviceState* ds, cudaS
     NML_CUDA(cudaGetLastError());
     ++g_launches;
     return profile_stop(slot, st);
+}
+
+// Estimated microseconds of n products [M][K] x [K][N], as images of one launch of the contraction kernel, by rows of the result or
+// turned round (see nml_ref_matmul): what starts and ends it, the conversions of both operands (per million values written), the
+// K loops and, per 32 columns, the drains of the rounds of tiles, and the result; no less than the host takes for the launches.
+// Fitted to 1372 random fp32 products and 944 of fp16 with N not of whole vectors, of 7 to 500 us: a standard error of 9 to 22 %.
+// The fastest of the two and of the in-place kernel by these estimates took 13.2 us in the (geometric) mean where the best takes 13.1,
+// always by rows 20.5, always turned 20.8, always in place 14.3; fp16 11.7, 11.6, 17.5, 15.4 and 14.6.
+static double batched_us(bool turned, double n, int M, int K, int N, int es, int sms) {
+    struct Cost { double fixed, a, b, loop, drain, ragged_round, ragged, result; };
+    static constexpr Cost kCost[2][2] = {{{8.3, 2.4, 2.6, 0.86, 0.27, 0.69, 0.91, 0.27}, {9.8, 2.35, 3.6, 0.77, 0.07, 0.0, 0.0, 0.69}},
+                                         {{7.7, 1.2, 1.05, 1.33, 0.55, 2.0, 0.0, 0.27}, {9.1, 0.87, 1.55, 1.37, 0.165, 0.0, 0.0, 0.24}}};
+    const bool f32 = es == 4;
+    const Cost& c = kCost[f32 ? 0 : 1][turned ? 1 : 0];
+    const int kb = f32 ? 32 : 64, vector = 16 / es, slices = ceil_div(K, kb) * (f32 ? 3 : 1);
+    const double row_tiles = n * ceil_div(turned ? N : M, kTileM);
+    const int columns = turned ? M : N;
+    double best = 0, rounds = 0, bn = 0;
+    for (int width = f32 ? 128 : 256; width >= 64; width /= 2) {  // (as run_fprop_like chooses)
+        const int nt = ceil_div(columns, width);
+        const double b = static_cast<double>(round_up(ceil_div(columns, nt), 32)), r = std::ceil(row_tiles * nt / sms);
+        const double t = r * b * (b > 128 ? 1.0 : b > 64 ? 1.28 : 2.24);
+        if (bn == 0 || t < best * 0.97) best = t, rounds = r, bn = b;
+    }
+    const double a_values = f32 || K % 8 ? n * M * round_up(K, turned ? kb : vector) * 1e-6 : 0.0;
+    const double b_values = n * N * round_up(K, turned ? vector : kb) * 1e-6;
+    const double drains = rounds * std::ceil(bn / 32);
+    const double ragged = !turned && N > 8 && N % vector ? 1.0 : 0.0;
+    const double us = c.fixed + c.a * a_values + c.b * b_values + c.loop * rounds * slices * slice_us(std::max(64, static_cast<int>(bn))) + c.drain * drains +
+                      ragged * (c.ragged_round * rounds + c.ragged * drains) + c.result * n * M * N * 1e-6;
+    return std::max(f32 || K % 8 ? 13.0 : 10.0, us);
 }
 
 // --------------------------------------------------------- layer -> problems --
@@ -2734,16 +2761,42 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
     const bool shared_b = b_batch == 1 && batch * static_cast<size_t>(M) < (1u << 30);
     const long long tiles = 1ll * ceil_div(M, 128) * ceil_div(N, 256);
     const size_t c_entry = static_cast<size_t>(M) * N * es, a_entry = static_cast<size_t>(M) * K * es, b_entry = static_cast<size_t>(K) * N * es;
-    // Rows of the result that do not start on 16 bytes cannot leave by TMA stores, and row by row through the staging tile they
-    // took five times as long as the product.  Those run turned round: the columns of the result are the pixels of
-    // an image whose channels are its rows (B [K][N] is that image's input, channel-major, and A its weights), so that the
-    // lanes of the epilogue are consecutive columns and store from their registers, on any alignment.  fp32 always: the
-    // transposing conversion is then the one for activations, which is the faster.  64 x 333 x 64 x 333 fp16 25.7 -> 16.0 us, fp32 43.9 ->
-    // 25.4; 128 x 300 x 128 x 300 fp16 47.6 -> 23.4; 128 x 33 x 64 x 33 15.6 -> 9.8; whole vectors: 64 x 512 x 64 x 512 fp32 41.3 -> 36.9,
-    // fp16 11.1 -> 19.8.
-    const bool turned = es == 4 || N % 8 != 0;
     size_t per_call = 1;  // entries per launch
     if (!shared_b && b_batch != 1 && tiles < 2ll * planning_sms()) per_call = std::min<size_t>(batch, 32768);  // (the grid of the weight repack)
+    auto in_place = [&](const uint8_t* A, const uint8_t* B, uint8_t* C, size_t n) {
+        StridedProduct g;
+        memset(&g, 0, sizeof(g));
+        g.M = N; g.N = M; g.K = K; g.batch = static_cast<int>(n);
+        g.dtype = g.out_dtype = dtype;
+        g.a = B; g.a_contiguous = false; g.a_stride = N; g.a_batch = 1ll * K * N;
+        g.b = A; g.b_contiguous = true; g.b_stride = K; g.b_batch = 1ll * M * K;
+        g.out = C; g.out_ns = N; g.out_batch = 1ll * M * N;
+        return g;
+    };
+    // The way `n` entries of one launch go, by estimated time.  By rows, as the layer above; turned round, the columns of the
+    // result being the pixels of an image whose channels are its rows (B [K][N] is that image's input, channel-major, and A its
+    // weights), so that the lanes of the epilogue are consecutive columns and store from their registers, on any alignment;
+    // in place (see nml_gemm.cuh).  fp16 rows of whole vectors leave by TMA stores and go by rows (64 x 512 x 64 x 512 11.1 us, turned 19.8).
+    // Turned round, results of eight columns and fewer store a few bytes a line (64 x 18571 x 8 x 1 fp16 55 us by rows, 244 turned).
+    // Us by rows / turned / in place: fp16 24 x 192 x 471 x 33 18.7 / 13.3 / 21.0; 64 x 333 x 64 x 333 25.7 / 16.0 / -; 128 x 33 x 64 x 33
+    // 15.6 / 9.8 / 6.4; fp32 64 x 333 x 64 x 333 43.9 / 25.4 / 28.7; 3 x 800 x 96 x 801 - / 16.3 / 10.4; 85 x 12 x 284 x 1200 127 / 337 / 52;
+    // 20 x 19698 x 6 x 1 29 / 166 / 91; 103 x 14010 x 2 x 39 323 / 191 / 341.
+    enum Way { BY_ROWS, TURNED, IN_PLACE };
+    auto way_of = [&](size_t n) -> Way {
+        if (es == 2 && N % 8 == 0) return BY_ROWS;
+        const int sms = planning_sms();
+        const double rows_us = batched_us(false, n, M, K, N, es, sms);
+        const double turned_us = N <= 8 ? 1e30 : batched_us(true, n, M, K, N, es, sms);
+        double place_us = 1e30;
+        if (tune().gemm && g_sm_limit.load(std::memory_order_relaxed) == 0) {
+            const StridedPlan plan = plan_strided(in_place(nullptr, nullptr, nullptr, n), sms);
+            const double result = n * static_cast<double>(M) * N * 1e-6;
+            place_us = es == 4 ? 5.9 + 0.92 * plan.loop_us + 2.0 * (plan.waves - 1.0) + 0.32 * result
+                               : 5.65 + 1.4 * plan.loop_us + 1.8 * (plan.waves - 1.0) + 0.28 * result;
+        }
+        return place_us < std::min(rows_us, turned_us) ? IN_PLACE : turned_us < rows_us ? TURNED : BY_ROWS;
+    };
+    Way way = BY_ROWS;
     auto entries = [&](const uint8_t* A, const uint8_t* B, uint8_t* C, size_t n, Bump& bump) -> int {
         if (per_call == 1 || shared_b) {
             nml_linear_desc d;
@@ -2753,27 +2806,15 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             d.math = math;
             return linear_pass(&d, NML_PASS_BACKWARD_DATA, A, B, nullptr, C, nullptr, bump, nullptr);
         }
-        if (turned && tune().gemm && n <= 65535 && g_sm_limit.load(std::memory_order_relaxed) == 0) {
-            StridedProduct g;
-            memset(&g, 0, sizeof(g));
-            g.M = N; g.N = M; g.K = K; g.batch = static_cast<int>(n);
-            g.dtype = g.out_dtype = dtype;
-            g.a = B; g.a_contiguous = false; g.a_stride = N; g.a_batch = 1ll * K * N;
-            g.b = A; g.b_contiguous = true; g.b_stride = K; g.b_batch = 1ll * M * K;
-            g.out = C; g.out_ns = N; g.out_batch = 1ll * M * N;
-            // Products of few blocks, in place: 128 x 33 x 64 x 33 fp16 10.0 -> 6.4 us, fp32 12.9 -> 7.3; 3 x 800 x 96 x 801 fp16 10.9 ->
-            // 9.4, fp32 16.3 -> 10.4; 64 x 45 x 64 x 1001 fp32, two waves, 25.0 -> 15.6; more of them are the contraction kernel's: 64 x 333
-            // x 64 x 333 fp32 25.1 against 28.7, 20 x 777 x 64 x 140 fp16, two waves, 9.3 against 12.9.
+        if (way == IN_PLACE) {
+            if (bump.dry) return NML_OK;
             // (fp16 rows that TMA was to read and cannot stay refused)
-            if (es == 2 && K % 8 == 0 && !bump.dry) {
-                const int rc = rows_for_tma(A, K, M);
-                if (rc) return rc;
-            }
-            if (plan_strided(g, planning_sms()).us <= (es == 4 ? 18.0 : 10.5)) return bump.dry ? NML_OK : run_strided(g, PDL_NORMAL, nullptr, nullptr);
+            const int rc = es == 2 && K % 8 == 0 ? rows_for_tma(A, K, M) : NML_OK;
+            return rc ? rc : run_strided(in_place(A, B, C, n), PDL_NORMAL, nullptr, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));
-        if (turned) {
+        if (way == TURNED) {
             f.a = B; f.a_dtype = dtype; f.a_layout = NML_NCHW; f.batch = static_cast<int>(n); f.a_h = 1; f.a_w = N; f.a_c = K;
             f.w = A; f.w_dtype = dtype; f.d0 = M; f.d1 = K; f.kh = f.kw = 1; f.k_is_dim0 = 0; f.w_direct = 1; f.w_batched = 1;
             f.s_h = f.s_w = f.d_h = f.d_w = 1;
@@ -2795,6 +2836,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
     int rc;
     for (;;) {
         Bump dry{nullptr, 0, 0, true};
+        way = way_of(per_call);  // (for all launches: a last one of fewer entries has this one's scratch)
         rc = entries(nullptr, nullptr, nullptr, per_call, dry);
         if (rc) return rc;
         need = round_up(dry.off, 256);

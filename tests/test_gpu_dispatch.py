@@ -30,6 +30,30 @@ def test_batched_matmul_entries_share_a_launch(batch, m, k, n, oracle):
     ops.device_status()
 
 
+# tall and narrow, short and wide: what the conversions cost decides whether the operands are read in place (one launch, else
+# three)
+@pytest.mark.parametrize("batch,m,k,n,launches32,launches16", [
+    (40, 15001, 6, 1, 3, 3), (9, 3000, 16, 8, None, None), (30, 12000, 40, 9, 3, None), (17, 1367, 72, 40, None, None), (70, 12, 284, 1199, 1, None),
+    (90, 4, 129, 602, 1, 1), (24, 190, 471, 33, None, None), (64, 45, 64, 1001, 1, None), (300, 1, 40, 77, 1, 1)])
+def test_batched_matmul_tall_and_wide(batch, m, k, n, launches32, launches16):
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(batch, m, k, device="cuda", generator=gen)
+    b = torch.randn(batch, k, n, device="cuda", generator=gen)
+    for dt, code, want_launches in ((torch.float32, F32, launches32), (torch.float16, F16, launches16)):
+        ad, bd = a.to(dt), b.to(dt)
+        torch.cuda.synchronize()
+        before = ops.launch_count()
+        ptr = _nectarml.tensor.matmul(ad.data_ptr(), bd.data_ptr(), a.shape, b.shape, code)
+        launched = ops.launch_count() - before
+        want = (ad.double() @ bd.double()).cpu().numpy()
+        if dt == torch.float32:
+            assert_f32(fetch(ptr, (batch, m, n)), want, "fp32")
+        else:  # (an absolute bound of the results' size)
+            assert_f16(fetch(ptr, (batch, m, n), np.float16), want, "fp16", atol=1e-3 * max(1.0, k ** 0.5))
+        assert want_launches is None or launched == want_launches, (dt, launched)
+    ops.device_status()
+
+
 @pytest.mark.parametrize("fout", [1, 2, 9, 31, 33, 63, 65, 127, 257, 333])
 @pytest.mark.parametrize("rows", [1, 130])
 def test_rows_that_do_not_start_on_16_bytes(rows, fout, oracle):

@@ -558,7 +558,7 @@ static int prepare_window(const void* src, int dtype, int layout, int batch, int
 // Picks a power-of-two pixel box (w, h, n) with 2^bits pixels that covers the grid with the
 // fewest boxes; ties go to the wider box.  box extents times the element stride stay <= 256.  n_tiles: tiles per box.
 static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* wl, int* hl, int* nl,
-                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1, bool split = false, double k_us = 0, double tile_kb = 0) {
+                       int prefer_w_log2 = 0, int n_tiles = 1, int sms = 1, bool split = false, double k_us = 0, double tile_kb = 0, int z_cap = 1) {
     const auto rounds = [&](long long boxes) { return (boxes * n_tiles + sms - 1) / sms; };
     long long best = -1, best_wide = -1, best_narrow = -1;
     int ww = 0, wh = 0, wn = 0, nw = 0, nh = 0, nn = 0;
@@ -609,17 +609,21 @@ static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* 
     // Boxes of fewer than eight pixels of a wider row may save rounds (62 x 62 pixels of 64 images are 1922 boxes of 2 x 1 x 64 and 1984
     // of 64 x 2 x 1), but their pixel-major stores reach 1 TB/s and less (two pixels 0.63) where eight and more reach 3.7: only
     // where the K loop outlasts the stores.  k_us: a tile's K loop, tile_kb: its result.  1x1 64 -> 200 at 62 x 62, batch 64, fp32
-    // result of fp16 products 314 -> 54 us without them; 5x5 96 -> 64 at 21 x 21, batch 128, 3xTF32 162 us without, 141 with them.
+    // result of fp16 products 314 -> 54 us without them; 5x5 96 -> 64 at 21 x 21, batch 128, 3xTF32 162 us without, 141 with them; 4x4
+    // stride 2 14 -> 3 at 64 x 19, batch 64 23.9 without (two rounds), 15.8 with.  Where fewer boxes leave SMs for a K split (up to z_cap
+    // slices) they win by it, and its planes are row-major: input gradient of 4x4 64 -> 200 at 48 x 9, batch 16, 3xTF32 60.8 without, 46.4 with.
     if (best_narrow > 0) {
-        const auto tile_us = [&](double store_us) { return std::max(k_us, store_us) + 0.25 * std::min(k_us, store_us); };  // (mostly overlapped)
-        if (rounds(best_narrow) * tile_us(tile_kb / (2.4 * (1 << nw))) < 0.97 * rounds(best) * tile_us(tile_kb / 25.0)) {
+        const auto launch_us = [&](long long boxes, double store_us) {
+            const long long z = z_cap > 1 ? std::min<long long>(z_cap, sms / (boxes * n_tiles)) : 1;
+            return z >= 2 ? k_us / z + 3.0 : rounds(boxes) * (std::max(k_us, store_us) + 0.25 * std::min(k_us, store_us));  // (mostly overlapped)
+        };
+        if (launch_us(best_narrow, tile_kb / (2.4 * (1 << nw))) < 0.97 * launch_us(best, tile_kb / 25.0)) {
             *wl = nw;
             *hl = nh;
             *nl = nn;
         }
     }
 }
-
 
 // Closes the timing bracket of a recorded launch (see nml_profile_begin).
 static int profile_stop(int slot, cudaStream_t st) {
@@ -822,11 +826,15 @@ struct FpropLike {
     int w_batched;  // every image has its own [d0][d1] weights, one after the other (batched matmul; kh = kw = 1)
 };
 
-// choose_box for the tiles of a forward walk: N columns, `slices` K slices (of three products each for the 3xTF32 split).
-static void choose_tile_box(int gw, int gh, int gn, int s_w, int s_h, int N, int planes, int slices, int out_bytes, int prefer_w_log2, int sms,
-                            int* wl, int* hl, int* nl) {
+// choose_box for the tiles of a forward walk: N columns, `slices` K slices (of three products each for the 3xTF32 split) on the
+// average of `phases` of as many boxes.  A slice of fewer than 64 columns takes as long as one of 64; where the patch walk could
+// take the layer (patch) it counts by its columns all the same: wide boxes leave the layer to that walk, which is worth
+// more than a round (7x7 4 -> 2 at 16 x 12, batch 65, input gradient 14.5 us, 26.3 with narrow boxes).
+static void choose_tile_box(int gw, int gh, int gn, int s_w, int s_h, int N, int planes, double slices, int phases, int z_cap, bool patch, int out_bytes,
+                            int prefer_w_log2, int sms, int* wl, int* hl, int* nl) {
     const int n_tiles = ceil_div(N, planes == 2 ? 128 : 256), bn = ceil_div(N, n_tiles);
-    choose_box(7, gw, gh, gn, s_w, s_h, wl, hl, nl, prefer_w_log2, n_tiles, sms, planes == 2, slices * slice_us(bn) * (planes == 2 ? 3 : 1), bn * out_bytes / 8.0);
+    choose_box(7, gw, gh, gn, s_w, s_h, wl, hl, nl, prefer_w_log2, n_tiles * phases, sms, planes == 2,
+               slices * slice_us(patch ? bn : std::max(64, bn)) * (planes == 2 ? 3 : 1), bn * out_bytes / 8.0, z_cap);
 }
 
 // Whether a few-channel layer with N output channels takes the patch walk with resident weights when its rows are 64
@@ -837,7 +845,7 @@ static bool narrow_patch_walk(const FpropLike& f, int N) {
     if (f.kh < 2 || ph > 256 || pw * ph * 64 > 48 * 1024) return false;
     int wl = 0, hl = 0, nl = 0;
     const bool nchw = f.out_layout == NML_NCHW && !(f.out_h == 1 && f.out_w == 1);
-    choose_tile_box(f.out_w, f.out_h, f.batch, 1, f.s_h, N, 1, f.kh, f.out_dtype == NML_F16 ? 2 : 4, nchw ? 5 : 0, planning_sms(), &wl, &hl, &nl);
+    choose_tile_box(f.out_w, f.out_h, f.batch, 1, f.s_h, N, 1, f.kh, 1, 1, true, f.out_dtype == NML_F16 ? 2 : 4, nchw ? 5 : 0, planning_sms(), &wl, &hl, &nl);
     const double area = static_cast<double>(f.out_w) * f.out_h;
     const double eff_patch = area / (1.0 * round_up(f.out_w, 8) * round_up(f.out_h, 16));
     const double eff_box = area * f.batch / (1.0 * round_up(f.out_w, 1 << wl) * round_up(f.out_h, 1 << hl) * round_up(f.batch, 1 << nl));
@@ -1164,19 +1172,14 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     P.n_phases = n_phases;
     // M-tile box from the largest phase grid
     const int esw = (f.gather || window) ? 1 : f.s_w, esh = f.gather ? 1 : f.s_h;
-    if (f.w_batched) {  // a tile never straddles two images
-        P.b_batched = 1;
-        P.wb_log2 = 7;
-    } else {
-        choose_tile_box(P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, N, P.planes, c_blocks * P.phases[0].tap_count, P.out_f16 ? 2 : 4,
-                        P.out_mode != OUT_NCHW ? 0 : f.gather && f.s_w > 1 ? 1 : 5, limited(ds->sms), &P.wb_log2, &P.hb_log2, &P.nb_log2);
-    }
     // Patch walk: unit-stride walks with several taps load one haloed patch per channel block instead of
     // one box per tap (8 x 16 pixel tiles of a single image).  Taken when the fixed tile shape does not
     // waste much more of the tile than the free-form box does.  Every phase of a gather walk has its own
     // taps and patch origin; the box is sized for the widest phase.
+    const int patch_mode = tune().patch;
+    int pw_ = 0, ph_ = 0;
+    bool patch_fits = false;
     {
-        const int mode = tune().patch;
         int range_w = 0, range_h = 0;
         bool every_phase_has_taps = true;
         for (int p = 0; p < n_phases; ++p) {
@@ -1199,11 +1202,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             range_h = std::max(range_h, dh_max - dh_min);
         }
         // (a row stride of the walk only stretches the patch: consecutive output rows are esh patch rows apart)
-        const int pw_ = 8 + range_w, ph_ = 15 * esh + range_h + 1;
-        const int wq = P.phases[0].wq, hq = P.phases[0].hq;
-        const double eff_patch = static_cast<double>(wq) * hq / (1.0 * round_up(wq, 8) * round_up(hq, 16));
-        const double eff_box = static_cast<double>(wq) * hq * f.batch /
-                               (1.0 * round_up(wq, 1 << P.wb_log2) * round_up(hq, 1 << P.hb_log2) * round_up(f.batch, 1 << P.nb_log2));
+        pw_ = 8 + range_w;
+        ph_ = 15 * esh + range_h + 1;
         const bool can = every_phase_has_taps && n_taps >= 2 && esw == 1 && pw_ <= 256 && ph_ <= 256 &&
                          pw_ * ph_ * row_bytes <= 48 * 1024;
         // Every weight slice stays in shared memory beside two patch buffers and the smallest epilogue staging.  (Weights
@@ -1211,8 +1211,22 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         // longer does: 3x3 128 -> 128 at 56 x 56, batch 16 116 -> 71 us without it, 64 -> 64 at batch 8 30.2 -> 27.5.)
         const int bn_res = N <= 16 ? 16 : static_cast<int>(round_up(N, 32));
         const long long res_need = 1ll * c_blocks * n_taps * bn_res * row_bytes + 2 * round_up(pw_ * ph_ * row_bytes, 1024);
-        const bool fits = P.planes == 1 && N <= 256 && !b_mn_major && res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
-        if (can && fits && mode && (mode == 2 || eff_patch >= 0.8 * eff_box)) {
+        patch_fits = can && patch_mode && P.planes == 1 && N <= 256 && !b_mn_major && res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
+    }
+    if (f.w_batched) {  // a tile never straddles two images
+        P.b_batched = 1;
+        P.wb_log2 = 7;
+    } else {
+        choose_tile_box(P.phases[0].wq, P.phases[0].hq, f.batch, esw, esh, N, P.planes, static_cast<double>(c_blocks) * n_taps / n_phases, n_phases,
+                        can_split ? std::min(z_cap, 8) : 1, patch_fits, P.out_f16 ? 2 : 4, P.out_mode != OUT_NCHW ? 0 : f.gather && f.s_w > 1 ? 1 : 5,
+                        limited(ds->sms), &P.wb_log2, &P.hb_log2, &P.nb_log2);
+    }
+    {
+        const int wq = P.phases[0].wq, hq = P.phases[0].hq;
+        const double eff_patch = static_cast<double>(wq) * hq / (1.0 * round_up(wq, 8) * round_up(hq, 16));
+        const double eff_box = static_cast<double>(wq) * hq * f.batch /
+                               (1.0 * round_up(wq, 1 << P.wb_log2) * round_up(hq, 1 << P.hb_log2) * round_up(f.batch, 1 << P.nb_log2));
+        if (patch_fits && (patch_mode == 2 || eff_patch >= 0.8 * eff_box)) {
             P.patch = 1;
             P.patch_w = pw_;
             P.patch_h = ph_;

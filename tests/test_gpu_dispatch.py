@@ -92,6 +92,12 @@ def test_channel_major_results_of_any_width(n, c_in, h, w, c_out, k, s):
     ops.device_status()
 
 
+# few columns, whose slices cost as much as those of 64; boxes of a K split; boxes of several phases
+@pytest.mark.parametrize("n,c_in,h,w,c_out,k,s", [(64, 14, 64, 19, 3, 4, 2), (16, 200, 50, 11, 64, 4, 1), (40, 3, 76, 28, 320, 7, 3)])
+def test_channel_major_boxes_by_time(n, c_in, h, w, c_out, k, s):
+    test_channel_major_results_of_any_width(n, c_in, h, w, c_out, k, s)
+
+
 # operands read in place: one row, one column, K of one value and of no whole slice, rows that start anywhere, K loops shared by the
 # blocks of a cluster (the last of them with nothing to do), two waves of blocks
 @pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (1, 70, 33), (129, 33, 130), (64, 513, 127), (33, 288, 65), (5, 2049, 3), (300, 36, 1025), (40, 96, 130)])

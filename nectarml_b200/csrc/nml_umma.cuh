@@ -1547,9 +1547,10 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
             }
             if (lane == 0) bulk_wait_group<0>();  // stores must land before the CTA ends
         } else
-        // (two groups of channel-major stores take alternate tiles; those of a double tile share each.  Row-major instances have one group and
-        // keep the plain loop: with this one's step in registers 10194 x 24 -> 3271, fp16 products, fp32 result 65 -> 70 us)
-        for (int alt = kMode == MODE_FPROP && kOutMode == OUT_NCHW && P.epi_alt ? 1 : 0, tile_id = tile_first + (titer = alt & (ew >> 2)) * tile_step;
+        // (two groups of channel-major stores take alternate tiles; those of a double tile share each.  Row-major instances have one group;
+        // a constant step makes those of fp16 results 5-8 % faster, 12792 x 31 -> 1423 43.6 -> 40.1 us, and those of fp32 results up to 5 %
+        // slower, 16256 x 1882 -> 7 input gradient 94.7 -> 98.6)
+        for (int alt = kMode == MODE_FPROP && (kOutMode == OUT_NCHW || !kOutF16) && P.epi_alt ? 1 : 0, tile_id = tile_first + (titer = alt & (ew >> 2)) * tile_step;
              ok && tile_id < P.num_tiles; tile_id += (1 + alt) * tile_step, titer += 1 + alt) {
             int tile = tile_id, kz = 0;
             if (kMode == MODE_FPROP && P.fsplit > 1) {

@@ -1718,11 +1718,13 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         // at most 192 slices, as many as leave each at least one block (a count that the loop below does not pass over, so
         // that there is a plan whatever else is refused)
         const int max_split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, std::min(P.kblocks_total, 192)));
+        const bool may_pair = tune().pair;  // (read once: the loop runs up to 500 times per plan)
+        const int dbl = tune().dbl;
         double best = -1;
         for (int width = 256; width >= 64; width /= 2) {
             const int nt = ceil_div(g.plain_c, width);
             const int bn = static_cast<int>(round_up(ceil_div(g.plain_c, nt), 64));
-            const bool pair = tune().pair && bn == 256 && a_grp && b_grp && sms >= 2;
+            const bool pair = may_pair && bn == 256 && a_grp && b_grp && sms >= 2;
             if ((width < 256 && bn > width) || (bn > 128 && P.planes == 2 && !pair)) continue;
             const int mt = pair ? ceil_div(row_tiles, 2) : row_tiles;
             const int units = pair ? sms / 2 : sms;
@@ -1750,14 +1752,14 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                     P.pair = pair ? 1 : 0;
                     P.big_rows = big_rows;
                 };
-                if (tune().dbl != 2 || !pair || P.planes == 2) consider(rounds(tiles) * tile_us + reduce_us, 0, tiles, mt);
+                if (dbl != 2 || !pair || P.planes == 2) consider(rounds(tiles) * tile_us + reduce_us, 0, tiles, mt);
                 // double tiles, with single ones behind them where K is whole (for 3 % and more)
-                if (pair && P.planes == 1 && tune().dbl) {
+                if (pair && P.planes == 1 && dbl) {
                     const double double_us = per_sp * kDoubleBlockUs + kDoubleTileUs;
                     const int rows2 = ceil_div(mt, 2);
-                    const long long dbl = 1ll * rows2 * nt * sp;
-                    consider((rounds(dbl) * double_us + reduce_us) * 1.03, INT_MAX, dbl, 2 * rows2);
-                    const int big_rows = tune().dbl == 2 ? (mt / 2 + 1) / 2 : static_cast<int>(dbl / units * units / nt);
+                    const long long doubles = 1ll * rows2 * nt * sp;
+                    consider((rounds(doubles) * double_us + reduce_us) * 1.03, INT_MAX, doubles, 2 * rows2);
+                    const int big_rows = dbl == 2 ? (mt / 2 + 1) / 2 : static_cast<int>(doubles / units * units / nt);
                     if (sp == 1 && big_rows > 0 && mt > 2 * big_rows) {
                         const long long big = 1ll * big_rows * nt, total = big + 1ll * (mt - 2 * big_rows) * nt;
                         double us = 0;
@@ -1941,14 +1943,12 @@ static StridedPlan plan_strided(const StridedProduct& g, int sms) {
     return best;
 }
 
-static int run_strided(const StridedProduct& g, int role, DeviceState* ds, cudaStream_t st) {
+static int run_strided(const StridedProduct& g, const StridedPlan& plan, int role, cudaStream_t st) {
     const bool f32 = g.dtype == NML_F32;
     const int es = f32 ? 4 : 2, slice = f32 ? 32 : 64;
-    if (!ds) {
-        const int rc = device_state(&ds);
-        if (rc) return rc;
-    }
-    const StridedPlan plan = plan_strided(g, planning_sms());
+    DeviceState* ds = nullptr;
+    int rc = device_state(&ds);
+    if (rc) return rc;
     GemmParams P;
     memset(&P, 0, sizeof(P));
     P.a = g.a; P.b = g.b; P.bias = g.bias; P.out = g.out;
@@ -1975,7 +1975,7 @@ static int run_strided(const StridedProduct& g, int role, DeviceState* ds, cudaS
     P.wait_limit_ns = g_dbg_wait_limit_ns;
     const long long blocks = 1ll * P.tiles_m * P.tiles_n * g.batch * plan.splits;
     if (blocks > INT_MAX) return NML_ERR_UNSUPPORTED;
-    int rc = profile_open(st);
+    rc = profile_open(st);
     if (rc) return rc;
     const int slot = g_bracket_slot;
     g_bracket_slot = -1;
@@ -2142,15 +2142,16 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
         // 90 -> 400 9.1 -> 7.8; four slices, 4000 x 256 -> 100, 8.4 and 8.5; 32 x 512 -> 2048, whose loop blocks would share, 6.8 and
         // 6.5 from L2 but 6.4 and 6.6 from HBM).  Rows that TMA is to read and cannot, because the matrix does not start on 16 bytes,
         // stay refused, by the map's own error (the plan's scratch, none, is no room for the contraction kernel to find out).
-        const StridedPlan plan = plan_strided(g, planning_sms());
+        StridedPlan plan;
         bool in_place;
         if (operands == NML_F32) {
+            plan = plan_strided(g, planning_sms());
             const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
             in_place = !few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0);
         } else {
             // (a launch that is to stall is the contraction kernel's)
             in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms() && !g_dbg_short_a_box;
-            if (in_place && !ws.dry && I % 8 == 0) {
+            if (in_place && !ws.dry && I % 8 == 0 && ((reinterpret_cast<uintptr_t>(in0) | reinterpret_cast<uintptr_t>(in1)) & 15) != 0) {
                 int rc = rows_for_tma(in0, I, R);
                 if (!rc) rc = rows_for_tma(in1, I, O);
                 if (rc) return rc;
@@ -2164,13 +2165,14 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
             }
             if (ws.dry) return NML_OK;
             if (!ws.fits()) return NML_ERR_WORKSPACE;
+            if (operands == NML_F16) plan = plan_strided(g, planning_sms());
             const bool beside = sums.out && !g_prof.on.load(std::memory_order_relaxed);
             if (sums.out && !beside) {
                 sums.first_stage(st);
                 const int rc = sums.second_stage(st);
                 if (rc) return rc;
             }
-            const int rc = run_strided(g, beside ? PDL_LEADER : PDL_NORMAL, nullptr, st);
+            const int rc = run_strided(g, plan, beside ? PDL_LEADER : PDL_NORMAL, st);
             if (rc || !beside) return rc;
             t_role = PDL_SIBLING;
             sums.first_stage(st);
@@ -2823,8 +2825,9 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
         if (way == IN_PLACE) {
             if (bump.dry) return NML_OK;
             // (fp16 rows that TMA was to read and cannot stay refused)
-            const int rc = es == 2 && K % 8 == 0 ? rows_for_tma(A, K, M) : NML_OK;
-            return rc ? rc : run_strided(in_place(A, B, C, n), PDL_NORMAL, nullptr, nullptr);
+            const int rc = es == 2 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) != 0 ? rows_for_tma(A, K, M) : NML_OK;
+            const StridedProduct g = in_place(A, B, C, n);
+            return rc ? rc : run_strided(g, plan_strided(g, planning_sms()), PDL_NORMAL, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));

@@ -2201,12 +2201,18 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     f.w_direct = 1;
     // Input gradient: W [out][in] read in place is an MN-major B operand.  Where its rows are no whole groups of 64 it takes a load per
     // group and excludes CTA pairs, and a transposed fp16 copy W^T [in][out] (one coalesced pass over the weights, counted in the
-    // pass's duration) pays from 3e9 products on: 12000 x 520 -> 2048 55.6 -> 36.4 us, 10000 x 1000 -> 3000 116 -> 64, 5000 x 2040 -> 1000 45
-    // -> 36; 2000 x 2040 -> 1000 20.2 and 20.2, 2000 x 1000 -> 640 10.6 -> 12.7.  Whole groups are read almost as fast as a K-major
+    // pass's duration) pays from 2.2e9 products on, with 128 outputs (two K slices) and more: 12000 x 520 -> 2048 55.6 -> 36.4 us, 8192 x 328
+    // -> 1024 18.7 -> 16.0, 4096 x 520 -> 1024 18.6 -> 15.0, 16384 x 520 -> 320 18.6 -> 16.9; 4096 x 1000 -> 512 12.6 -> 13.5; 65536 x 1000 -> 64
+    // 36.5 -> 42.2.  Less than one group is mostly fill: from 8192 rows on for up to 32 inputs, 16384 x 8 -> 512 15.9 -> 8.3, 81664 x 40 -> 320
+    // 20.3 -> 16.0, 16384 x 40 -> 1024 13.0 -> 12.0, -> 512 10.1 -> 10.2.  Whole groups are read almost as fast as a K-major
     // operand: only very wide layers of many rows gain a little (16384 x 3072 -> 1024 93.5 -> 88.5, 8192 x 4096 -> 4096 213 -> 205;
-    // but 16384 x 512 -> 2048 33.3 -> 37.2, 16384 x 2048 -> 8192 360 -> 371).
-    const bool pays = d->in_features % 64 != 0 ? 1ll * d->rows * d->in_features * d->out_features >= 3000000000ll
-                                               : d->in_features >= 3072 && d->rows >= 8192;
+    // but 16384 x 3072 -> 512 52.1 -> 54.3, 16384 x 512 -> 2048 33.3 -> 37.2, 16384 x 2048 -> 8192 360 -> 371).
+    const long long out_rows = 1ll * d->rows * d->out_features;
+    const bool pays = d->in_features % 64 == 0 ? d->in_features >= 3072 && d->rows >= 8192 && d->out_features >= 1024
+                      : d->out_features < 128 ? false
+                      : d->in_features <= 32 ? d->rows >= 8192
+                      : d->in_features < 64 ? out_rows >= 16000000ll
+                                            : out_rows * d->in_features >= 2200000000ll;
     // Weights that do not start on 16 bytes are no operand for TMA, but the copy's kernel takes them: from 8192 rows on, with whole groups
     // of outputs, such a layer has its copy (and a workspace query, which sees no pointer, counts it); elsewhere it is refused.
     const bool any_start = d->rows >= 8192 && d->out_features % 64 == 0;

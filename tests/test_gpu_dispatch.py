@@ -211,6 +211,18 @@ def test_linear_input_gradient_with_transposed_weights(rows, fin, fout):
     ops.device_status()
 
 
+# both sides of each of its limits, by the launches (the copy is one more)
+@pytest.mark.parametrize("rows,fin,fout,copied", [
+    (8192, 8, 128, 1), (8191, 8, 128, 0), (8192, 8, 120, 0), (8192, 40, 1960, 1), (8192, 40, 1944, 0), (2200, 1000, 1000, 1), (2199, 1000, 1000, 0),
+    (8192, 3072, 1024, 1), (8192, 3072, 1016, 0), (8184, 3072, 1024, 0)])
+def test_where_the_weights_are_transposed(rows, fin, fout, copied):
+    dy, w = torch.zeros(rows, fout, device="cuda", dtype=torch.float16), torch.zeros(fout, fin, device="cuda", dtype=torch.float16)
+    launches = ops.launch_count()
+    ops.linear_backward_data(dy, w)
+    assert ops.launch_count() - launches == 1 + copied
+    test_linear_input_gradient_with_transposed_weights(rows, fin, fout)
+
+
 # weights that do not start on 16 bytes: through the copy from 8192 rows on with whole groups of 64 outputs, whether or not aligned ones
 # would take it, and refused elsewhere
 @pytest.mark.parametrize("rows,fin,fout,taken", [(8192, 512, 128, True), (8195, 520, 64, True), (8192, 3072, 64, True), (8192, 512, 136, False), (4096, 512, 128, False), (3000, 1000, 1000, False)])

@@ -419,7 +419,11 @@ struct RowsColsum {
     }
     // Both stages in one launch of eight blocks per column block, up to 1024 rows: a weight gradient with its bias gradient of 64 x
     // 512 -> 512 8.2 -> 6.0 us, 1000 x 304 -> 776 13.7 -> 11.4; more rows are too many for so few blocks (2000 x 512 -> 128 10.5 -> 12.9).
-    bool one_launch() const { return vectors && pixels <= 1024; }
+    // On their own between the conversions and the contraction (`serial`: fp32) wide rows are too many from 512 on: 848 x 4 -> 1216 21.4 us in two
+    // launches, 23.3 in one; 640 x 512 -> 1216 7 % slower, 1024 x 2048 -> 512 5 %; up to 256 columns 10 to 15 % faster all the way, and beside
+    // a product that reads its operands in place, too (824 x 1 -> 348 13.0 and 11.1, 640 x 7 -> 1560 16.5 and 14.3).
+    bool serial = false;
+    bool one_launch() const { return vectors && pixels <= (serial && dtype == NML_F32 && c > 256 ? 512 : 1024); }
     void first_stage(cudaStream_t st) const {
         if (one_launch()) {
             const int role = t_role, rpb = static_cast<int>(round_up(ceil_div(static_cast<int>(pixels), kColsumCluster), 8));
@@ -511,6 +515,7 @@ static int prepare_activation(const void* src, int dtype, int layout, int batch,
         convert_rows(src, dtype, p0, p1, mi.enc, pixels, c, Cp, st);
         if (colsum) {
             rows.cs = cs;
+            rows.serial = true;
             rows.first_stage(st);
             int rc = rows.second_stage(st);
             if (rc) return rc;

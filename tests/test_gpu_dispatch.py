@@ -172,6 +172,25 @@ def test_bias_gradient_sums(rows, fout):
     ops.device_status()
 
 
+# between conversions and contraction, fp32 rows of more than 256 columns up to 512 of them; beside a product in place up to 1024 (the
+# launches of a weight gradient that are its sums')
+@pytest.mark.parametrize("fin,fout,sums", [(1024, 256, [1, 1, 1, 2]), (1024, 772, [1, 2, 2, 2]), (16, 260, [1, 1, 1, 2])])
+def test_wide_bias_gradient_sums(fin, fout, sums):
+    gen = torch.Generator(device="cuda").manual_seed(fout)
+    launches = []
+    for rows in (512, 513, 1024, 1025):
+        x, dy = torch.randn(rows, fin, device="cuda", generator=gen), torch.randn(rows, fout, device="cuda", generator=gen) + 0.5
+        before = ops.launch_count()
+        _, db = ops.linear_backward_weight(x, dy, math="3xtf32")
+        with_sums = ops.launch_count() - before
+        assert_f32(host(db), dy.double().sum(0).cpu().numpy(), "db", tol=1e-6)
+        before = ops.launch_count()
+        ops.linear_backward_weight(x, dy, math="3xtf32", want_bias_grad=False)
+        launches.append(with_sums - (ops.launch_count() - before))
+    assert launches == sums
+    ops.device_status()
+
+
 @pytest.fixture
 def four_pairs():
     """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all."""

@@ -2152,7 +2152,11 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
         if (operands == NML_F32) {
             plan = plan_strided(g, planning_sms());
             const bool few = pass == NML_PASS_BACKWARD_WEIGHT && ceil_div(I, kTileM) * ceil_div(O, 32) < 8;
-            in_place = !few && plan.us <= (pass == NML_PASS_FORWARD ? 14.0 : pass == NML_PASS_BACKWARD_DATA ? 20.0 : 13.0);
+            // (of one to four tiles, which the contraction kernel cuts over all SMs and eight blocks each take long for: 1 x 3456 -> 6 forward
+            // 12.4 us there and 15.6 here, input gradient of 2 x 3 -> 3877 12.5 and 19.8, of 85 x 1 -> 3328 12.8 and 17.9)
+            const double tiles = static_cast<double>(ceil_div(g.M, kTileM)) * ceil_div(g.N, plan.bn);
+            const double limit_us = pass == NML_PASS_BACKWARD_WEIGHT ? 13.0 : tiles <= 4 ? 12.5 : pass == NML_PASS_FORWARD ? 14.0 : 20.0;
+            in_place = !few && plan.us <= limit_us;
         } else {
             // (a launch that is to stall is the contraction kernel's)
             in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms() && !g_dbg_short_a_box;

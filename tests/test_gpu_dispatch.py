@@ -135,6 +135,19 @@ def test_products_in_place(rows, fin, fout, shift, oracle):
     ops.device_status()
 
 
+# long fp32 K loops of few tiles are the contraction kernel's: both sides of the limit, by the launches (one in place)
+@pytest.mark.parametrize("rows,fin,fout,forward,in_place", [
+    (1, 2000, 6, True, True), (1, 3456, 6, True, False), (130, 2600, 100, True, False), (2, 3, 1800, False, True), (2, 3, 3877, False, False), (85, 1, 3328, False, False)])
+def test_long_products_of_few_tiles(rows, fin, fout, forward, in_place, oracle):
+    rng = np.random.default_rng(fin + fout)
+    xh, wh = rng.standard_normal((rows, fin if forward else fout), dtype=np.float32), rng.standard_normal((fout, fin), dtype=np.float32)
+    launches = ops.launch_count()
+    got = ops.linear_forward(dev(xh), dev(wh), math="3xtf32") if forward else ops.linear_backward_data(dev(xh), dev(wh), math="3xtf32")
+    assert (ops.launch_count() - launches == 1) == in_place
+    assert_f32(host(got), oracle.linear_forward(xh, wh, None) if forward else xh.astype(np.float64) @ wh.astype(np.float64), "result")
+    ops.device_status()
+
+
 # fp16 rows that TMA reads have to start on 16 bytes.  Where they do not, the call says so by the map that was refused, also at
 # sizes that are read in place and have no scratch.
 @pytest.mark.parametrize("rows,fin,fout", [(32, 56, 8), (11, 8, 22), (535, 128, 16), (300, 512, 256)])

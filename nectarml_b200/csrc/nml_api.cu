@@ -94,10 +94,8 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_WTRANS   0: Linear input-gradients never take a transposed copy of the weights
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
 //   NML_TUNE_NARROW   0: few-channel layers always take eight channels per pixel
-//   NML_TUNE_DOUBLE   0: no double tiles, 2: wherever they are legal
-//   NML_TUNE_GEMM     0: no strided products
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow, dbl, gemm;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow;
 };
 static const Tune& tune() {
     static Tune t;
@@ -122,8 +120,6 @@ static const Tune& tune() {
         t.wtrans = env("NML_TUNE_WTRANS", 1);
         t.pair128 = env("NML_TUNE_PAIR128", 1);
         t.narrow = env("NML_TUNE_NARROW", 1);
-        t.dbl = env("NML_TUNE_DOUBLE", 1);
-        t.gemm = env("NML_TUNE_GEMM", 1);
     });
     return t;
 }
@@ -782,8 +778,6 @@ static PairCost pair_cost(int bn) { return bn == 256 ? PairCost{575.0, 1060.0, 2
 // The plan of a launch of `rows` x n_tiles pair tiles of k slices on `units` pairs: 0 double rows, all of them (INT_MAX), or as
 // many as fill whole rounds, with single tiles behind them where their last round would be half empty.
 static int plan_double_rows(int rows, int n_tiles, int k, int bn, int units, bool may_mix) {
-    if (tune().dbl == 0) return 0;
-    if (tune().dbl == 2) return may_mix && rows > 2 ? (rows / 2 + 1) / 2 : INT_MAX;
     const PairCost c = pair_cost(bn);
     const double one = k * c.one, two = k * c.two + c.drain;
     const long long single = 1ll * rows * n_tiles, dbl = 1ll * ((rows + 1) / 2) * n_tiles;
@@ -1724,7 +1718,6 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         // that there is a plan whatever else is refused)
         const int max_split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, std::min(P.kblocks_total, 192)));
         const bool may_pair = tune().pair;  // (read once: the loop runs up to 500 times per plan)
-        const int dbl = tune().dbl;
         double best = -1;
         for (int width = 256; width >= 64; width /= 2) {
             const int nt = ceil_div(g.plain_c, width);
@@ -1757,14 +1750,14 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                     P.pair = pair ? 1 : 0;
                     P.big_rows = big_rows;
                 };
-                if (dbl != 2 || !pair || P.planes == 2) consider(rounds(tiles) * tile_us + reduce_us, 0, tiles, mt);
+                consider(rounds(tiles) * tile_us + reduce_us, 0, tiles, mt);
                 // double tiles, with single ones behind them where K is whole (for 3 % and more)
-                if (pair && P.planes == 1 && dbl) {
+                if (pair && P.planes == 1) {
                     const double double_us = per_sp * kDoubleBlockUs + kDoubleTileUs;
                     const int rows2 = ceil_div(mt, 2);
                     const long long doubles = 1ll * rows2 * nt * sp;
                     consider((rounds(doubles) * double_us + reduce_us) * 1.03, INT_MAX, doubles, 2 * rows2);
-                    const int big_rows = dbl == 2 ? (mt / 2 + 1) / 2 : static_cast<int>(doubles / units * units / nt);
+                    const int big_rows = static_cast<int>(doubles / units * units / nt);
                     if (sp == 1 && big_rows > 0 && mt > 2 * big_rows) {
                         const long long big = 1ll * big_rows * nt, total = big + 1ll * (mt - 2 * big_rows) * nt;
                         double us = 0;
@@ -2110,7 +2103,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     if (!d || d->rows <= 0 || d->in_features <= 0 || d->out_features <= 0) return NML_ERR_INVALID;
     g_last_scratch_error[0] = 0;
     const int operands = d->math == NML_MATH_3XTF32 ? NML_F32 : d->math == NML_MATH_F16 ? NML_F16 : -1;
-    if (tune().gemm && d->in_dtype == operands && (pass == NML_PASS_BACKWARD_WEIGHT || d->w_dtype == operands) &&
+    if (d->in_dtype == operands && (pass == NML_PASS_BACKWARD_WEIGHT || d->w_dtype == operands) &&
         g_sm_limit.load(std::memory_order_relaxed) == 0) {
         const int R = d->rows, I = d->in_features, O = d->out_features;
         StridedProduct g;
@@ -2819,7 +2812,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
         const double rows_us = batched_us(false, n, M, K, N, es, sms);
         const double turned_us = N <= 8 ? 1e30 : batched_us(true, n, M, K, N, es, sms);
         double place_us = 1e30;
-        if (tune().gemm && g_sm_limit.load(std::memory_order_relaxed) == 0) {
+        if (g_sm_limit.load(std::memory_order_relaxed) == 0) {
             const StridedPlan plan = plan_strided(in_place(nullptr, nullptr, nullptr, n), sms);
             const double result = n * static_cast<double>(M) * N * 1e-6;
             place_us = es == 4 ? 5.9 + 0.92 * plan.loop_us + 2.0 * (plan.waves - 1.0) + 0.32 * result

@@ -91,6 +91,7 @@ SYMBOLS = {
     "nml_ref_conv_transpose1d_backward_weight": (_I, [_UP, _UP] + [_I] * 10 + [C.POINTER(_UP)]),
     "nml_ref_matmul": (_I, [_UP, _UP, C.POINTER(_I), _I, C.POINTER(_I), _I, _I, C.POINTER(_UP)]),
     "nml_ref_free": (_I, [_UP]),
+    "nml_debug_launch_count": (C.c_longlong, [_I]),
     "nml_debug_copy_to_host": (_I, [_VP, _UP, _SZ]),
     "nml_debug_wait_timeout": (_I, [C.c_ulonglong, _I, _VP]),
     "nml_debug_stalled_linear_forward": (_I, [C.POINTER(LinearDesc), _VP, _VP, _VP, _VP, _SZ, C.c_ulonglong, _VP]),

@@ -173,6 +173,7 @@ struct DeviceState {
 static DeviceState g_dev[64];
 static std::mutex g_dev_mutex;   // guards g_dev, g_static, g_prof and g_ref_ws
 static std::atomic<long long> g_launches{0};
+static std::atomic<long long> g_launches_of[4];  // by kind, see nml_debug_launch_count
 // Where kernels report an abandoned wait.  The words live in the library image, so set-up needs no
 // allocation: their device addresses come from cudaGetSymbolAddress, once per device.
 static __device__ int g_status_word;
@@ -754,6 +755,8 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     const int threads = P.epi_warps == 8 ? kThreadsWide : P.patch ? threads_for(P.out_mode) : kThreads;
     // (under an SM limit not before its predecessor has ended: blocks that wait would sit on the SMs that are to stay free, and
     // a block of this kernel leaves no room beside it)
+    if (P.dbl) ++g_launches_of[NML_DEBUG_DOUBLE_TILES];
+    if (P.add) ++g_launches_of[NML_DEBUG_SUMS];
     launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, threads, smem, st, P);
     NML_CUDA(cudaGetLastError());
     if (open_slot) *open_slot = rec_slot;
@@ -1984,6 +1987,7 @@ static int run_strided(const StridedProduct& g, const StridedPlan& plan, int rol
                 static_cast<unsigned>(blocks), kGemmThreads, smem, st, P);
     NML_CUDA(cudaGetLastError());
     ++g_launches;
+    ++g_launches_of[NML_DEBUG_IN_PLACE];
     return profile_stop(slot, st);
 }
 
@@ -2481,6 +2485,8 @@ int nml_device_status(int* code) {
 
 long long nml_launch_count(void) { return g_launches.load() + nml_layers_launch_count(); }
 
+long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 4 ? g_launches_of[kind].load() : -1; }
+
 int nml_profile_begin(int max_records) {
     if (max_records <= 0 || max_records > 1 << 16) return NML_ERR_INVALID;
     while (static_cast<int>(g_prof.start.size()) < max_records) {
@@ -2840,6 +2846,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
         FpropLike f;
         memset(&f, 0, sizeof(f));
         if (way == TURNED) {
+            if (!bump.dry) ++g_launches_of[NML_DEBUG_TURNED];
             f.a = B; f.a_dtype = dtype; f.a_layout = NML_NCHW; f.batch = static_cast<int>(n); f.a_h = 1; f.a_w = N; f.a_c = K;
             f.w = A; f.w_dtype = dtype; f.d0 = M; f.d1 = K; f.kh = f.kw = 1; f.k_is_dim0 = 0; f.w_direct = 1; f.w_batched = 1;
             f.s_h = f.s_w = f.d_h = f.d_w = 1;

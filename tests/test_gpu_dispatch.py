@@ -99,7 +99,7 @@ def test_channel_major_boxes_by_time(n, c_in, h, w, c_out, k, s):
 
 
 # operands read in place: one row, one column, K of one value and of no whole slice, rows that start anywhere, K loops shared by the
-# blocks of a cluster (the last of them with nothing to do), two waves of blocks
+# blocks of a cluster (the last of them with nothing to do)
 @pytest.mark.parametrize("rows,fin,fout", [(1, 1, 1), (1, 70, 33), (129, 33, 130), (64, 513, 127), (33, 288, 65), (5, 2049, 3), (300, 36, 1025), (40, 96, 130)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_products_in_place(rows, fin, fout, shift, oracle):
@@ -108,10 +108,10 @@ def test_products_in_place(rows, fin, fout, shift, oracle):
     host_of = {k: rng.standard_normal(s, dtype=np.float32) for k, s in sizes.items()}
     x, w, dy, b = (torch.cat([torch.zeros(shift, device="cuda"), dev(v).flatten()])[shift:].view(v.shape) for v in host_of.values())
     xh, wh, dyh, bh = host_of.values()
-    launches = ops.launch_count()
+    launches, in_place = ops.launch_count(), launches_of(IN_PLACE)
     y = ops.linear_forward(x, w, b, math="3xtf32")
     dx = ops.linear_backward_data(dy, w, math="3xtf32")
-    assert ops.launch_count() - launches == 2
+    assert ops.launch_count() - launches == 2 and launches_of(IN_PLACE) - in_place == 2
     assert_f32(host(y), oracle.linear_forward(xh, wh, bh), "y")
     assert_f32(host(dx), dyh.astype(np.float64) @ wh.astype(np.float64), "dx")
     dw, db = ops.linear_backward_weight(x, dy, math="3xtf32")
@@ -135,9 +135,11 @@ def test_products_in_place(rows, fin, fout, shift, oracle):
     ops.device_status()
 
 
-# long fp32 K loops of few tiles are the contraction kernel's: both sides of the limit, by the launches (one in place)
+# long fp32 K loops of few tiles are the contraction kernel's: both sides of the limit, by the launches (one in place); in place with two
+# waves of blocks (570 of 296 at a time), and with clusters of two on SMs that hold two blocks (224 on 148)
 @pytest.mark.parametrize("rows,fin,fout,forward,in_place", [
-    (1, 2000, 6, True, True), (1, 3456, 6, True, False), (130, 2600, 100, True, False), (2, 3, 1800, False, True), (2, 3, 3877, False, False), (85, 1, 3328, False, False)])
+    (1, 2000, 6, True, True), (1, 3456, 6, True, False), (60, 3456, 100, True, False), (2, 3, 1800, False, True), (2, 3, 3877, False, False), (85, 1, 3328, False, False),
+    (12160, 5, 336, True, True), (1003, 249, 824, True, True)])
 def test_long_products_of_few_tiles(rows, fin, fout, forward, in_place, oracle):
     rng = np.random.default_rng(fin + fout)
     xh, wh = rng.standard_normal((rows, fin if forward else fout), dtype=np.float32), rng.standard_normal((fout, fin), dtype=np.float32)
@@ -204,19 +206,50 @@ def test_wide_bias_gradient_sums(fin, fout, sums):
     ops.device_status()
 
 
+DOUBLE_TILES, IN_PLACE, TURNED = 0, 2, 3  # kinds of nml_debug_launch_count
+
+
+def launches_of(kind):
+    return _lib.load().nml_debug_launch_count(kind)
+
+
+# turned round, in fp16 and where the sizes say so in fp32: one row tile and several, columns of one pixel tile and of three, K of no whole
+# vector, entries of one column tile and of more
+@pytest.mark.parametrize("batch,m,k,n,fp32_too", [
+    (100, 129, 96, 65, False), (300, 127, 64, 63, False), (64, 333, 64, 333, False), (40, 257, 130, 257, True), (103, 3010, 2, 39, True), (64, 130, 72, 261, False)])
+def test_batched_matmul_turned_round(batch, m, k, n, fp32_too):
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    a, b = torch.randn(batch, m, k, device="cuda", generator=gen), torch.randn(batch, k, n, device="cuda", generator=gen)
+    for dt, code in ((torch.float16, F16),) + (((torch.float32, F32),) if fp32_too else ()):
+        ad, bd = a.to(dt), b.to(dt)
+        torch.cuda.synchronize()
+        before = launches_of(TURNED)
+        ptr = _nectarml.tensor.matmul(ad.data_ptr(), bd.data_ptr(), a.shape, b.shape, code)
+        assert launches_of(TURNED) - before == 1
+        want = (ad.double() @ bd.double()).cpu().numpy()
+        if dt == torch.float32:
+            assert_f32(fetch(ptr, (batch, m, n)), want, "fp32")
+        else:  # (an absolute bound of the results' size)
+            assert_f16(fetch(ptr, (batch, m, n), np.float16), want, "fp16", atol=1e-3 * k ** 0.5)
+    ops.device_status()
+
+
 @pytest.fixture
 def four_pairs():
-    """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all."""
+    """Plans for eight SMs, on which small layers have as many rounds of tiles as large ones on all; some launch of the test
+    has to have had double tiles."""
     ops.set_sm_limit(8)
+    before = launches_of(DOUBLE_TILES)
     yield
     ops.set_sm_limit(0)
+    assert launches_of(DOUBLE_TILES) > before
 
 
 # pair tiles are 256 x 256 and four run at a time: five to eight of them in one round of double tiles (the last row tile missing
 # from 1100 rows, the last columns from 1000), and nine rows as four double tiles with a single one behind them.  K is summed
 # in fp32 (errors of sqrt(K) * 2^-24 of the terms' size), the result rounded to fp16: 1e-2 rel holds that many times over, and
 # the absolute bound is 1e-3 of the results' size, sqrt(K) * 0.2.
-@pytest.mark.parametrize("rows,fin,fout", [(1100, 1600, 256), (1280, 1984, 200), (512, 2048, 1000), (2300, 3200, 256), (2304, 3136, 232)])
+@pytest.mark.parametrize("rows,fin,fout", [(1100, 1600, 256), (1280, 1984, 248), (512, 2048, 1000), (2300, 3200, 256), (2304, 3136, 232)])
 def test_double_tiles_linear(rows, fin, fout, oracle, four_pairs):
     rng = np.random.default_rng(rows + fin)
     h, r = torch.float16, oracle.round_f16
@@ -272,7 +305,7 @@ def test_linear_input_gradient_with_unaligned_weights(rows, fin, fout, taken):
     ops.device_status()
 
 
-@pytest.mark.parametrize("rows,fin,fout", [(4096, 640, 512), (4096, 1280, 512), (4100, 1280, 456), (2048, 256, 2304)])
+@pytest.mark.parametrize("rows,fin,fout", [(4096, 640, 512), (4096, 1280, 512), (4100, 1280, 448), (2048, 1024, 2304)])
 def test_double_tiles_linear_weight_gradient(rows, fin, fout, oracle, four_pairs):
     rng = np.random.default_rng(rows + fin)
     h, r = torch.float16, oracle.round_f16
@@ -284,7 +317,7 @@ def test_double_tiles_linear_weight_gradient(rows, fin, fout, oracle, four_pairs
 
 
 @pytest.mark.parametrize("n,c_in,hw,c_out,k,s,p,tr", [
-    (5, 128, 16, 256, 3, 1, 1, False), (3, 128, 21, 256, 5, 1, 2, False), (3, 256, 18, 256, 4, 2, 1, False), (3, 384, 16, 128, 4, 2, 1, True), (2, 256, 15, 256, 4, 2, 1, True)])
+    (5, 128, 16, 256, 3, 1, 1, False), (3, 128, 21, 256, 5, 1, 2, False), (5, 256, 18, 512, 4, 2, 1, False), (2, 384, 16, 128, 4, 2, 1, True), (5, 512, 9, 256, 4, 2, 1, True)])
 def test_double_tiles_convolutions(n, c_in, hw, c_out, k, s, p, tr, oracle, four_pairs):
     """Boxes of pixels, the phases of a gather, 128-column tiles, and row tiles of a weight gradient that belong to
     different taps."""

@@ -97,6 +97,10 @@ def test_input_gradient_with_an_addend_refuses():
     ops.device_status()
 
 
+def sums_in_epilogues():
+    return _lib.load().nml_debug_launch_count(1)
+
+
 class Block:
     """x -> conv, norm, ReLU, conv, norm + x, ReLU; ``through`` is what the residual passes on its way."""
 
@@ -131,10 +135,12 @@ def close(a, b):
 def test_block_input_gradient(act):
     x0, dy = tensors()
     block, x = Block(act=act), x0.clone().requires_grad_()
-    launches = ops.launch_count()
+    sums = sums_in_epilogues()
     (fused,) = torch.autograd.grad(block(x), (x,), dy)
     grads = block.store.grad.clone()
+    assert sums_in_epilogues() - sums == 1
     (engine,) = torch.autograd.grad(block(x, lambda r: r.view_as(r)), (x,), dy)  # (another edge: the engine adds)
+    assert sums_in_epilogues() - sums == 1
     assert torch.equal(grads, block.store.grad)
     assert close(fused, engine) and not torch.equal(fused, torch.zeros_like(fused))
     # a graph kept for a second pass, with another gradient, and then again the first
@@ -143,7 +149,7 @@ def test_block_input_gradient(act):
     twice = torch.autograd.grad(y, (x,), 2 * dy, retain_graph=True)[0]
     again = torch.autograd.grad(y, (x,), dy)[0]
     assert torch.equal(first, fused) and torch.equal(again, fused) and close(twice, 2 * fused)
-    assert launches < ops.launch_count()
+    assert sums_in_epilogues() - sums == 4
 
 
 def test_block_input_gradient_reaches_whoever_asks():
@@ -208,7 +214,9 @@ def test_hook_on_the_first_convolution(act):
 
         y = block(x)
         first_convolution(y.grad_fn).register_hook(hook)
+        sums = sums_in_epilogues()
         (dx,) = torch.autograd.grad(y, (x,), dy)
+        assert sums_in_epilogues() == sums
         assert close(seen[0].double() + residual.double(), fused) and not close(seen[0], fused)
         assert close(dx, fused) if scale is None else torch.equal(dx, residual)
 

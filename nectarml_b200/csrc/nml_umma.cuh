@@ -292,8 +292,8 @@ __device__ __forceinline__ void store_columns(T* o, size_t stride, const uint32_
 // kPair: two CTAs of a cluster compute one 256-row x 256-column tile with cta_group::2 MMAs issued by
 // the rank-0 CTA; each CTA loads its own 128 rows of A and its own 128-column half of B (no multicast),
 // which halves the B traffic and the MMA issue cost per SM and leaves room for 6 stages.
-// kDbl: a pair's tile is two row tiles high (512 x bn), two accumulators that share every B slice.  An SM takes in at most 64
-// bytes a clock from L2 (TMA loads of any shape: 18.9 TB/s over 148 SMs, wherever the lines are shared), and a 256-column pair
+// kDbl: a pair's tile is two row tiles high (512 x bn), two accumulators that share every B slice.  An SM takes in about 64
+// bytes a clock from L2 (TMA loads of any shape: 18.9 TB/s over 148 SMs, 65 bytes at 1965 MHz, wherever the lines are shared), and a 256-column pair
 // tile wants 32 KB per K slice of 512 clocks, all of it: a slice takes 570 to 700 clocks.  A double tile wants 48 KB per 1024
 // clocks and takes 1045 to 1060 (Linear; convolutions, whose slices arrive in more pieces, 720 and 1350).  At 256 columns the two
 // accumulators fill TMEM, so nothing overlaps the drain: the epilogue takes a tile into registers as fp16 and hands the

@@ -1244,6 +1244,11 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             P.nb_log2 = 0;
         }
     }
+    // Row-major results by TMA stores (see below), where the geometry allows them: up to eight columns have a short epilogue of their own.
+    // (Never phase-packed columns: they belong to several output pixels, and the packed image may be larger than the output.)
+    const int out_es = P.out_f16 ? 2 : 4;
+    const bool rows_by_tma = P.out_mode == OUT_NHWC && !P.shuf_sh && tune().tmastore && N > 8 && (static_cast<size_t>(N) * out_es) % 16 == 0 &&
+                             (reinterpret_cast<uintptr_t>(f.out) & 15) == 0;
     int z_plan = 1;  // K slices per tile
     // Tile width: 256 columns run the tensor pipe best, but when that leaves SMs idle (few row tiles,
     // narrow N) a narrower tile wins.  Cost per column relative to a 256-wide tile, measured on B200:
@@ -1261,7 +1266,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         for (int i = 0; i < 4; ++i) {
             if (forced ? i != 3 : i == 3) continue;
             int nt = ceil_div(N, cand[i]);
-            int bn = static_cast<int>(round_up(ceil_div(N, nt), b_mn_major ? 64 : (forced == 16 ? 16 : 32)));
+            // (TMA stores take whole pieces of columns, and only a row's last one may be cut off: 354 x 512 -> 192 in two tiles of 96 columns
+            // by the plain epilogue 9.3 us, in three of 64 by TMA stores 6.5)
+            const int unit = b_mn_major ? 64 : forced == 16 ? 16 : nt > 1 && rows_by_tma ? std::max(32, 128 / out_es) : 32;
+            int bn = static_cast<int>(round_up(ceil_div(N, nt), unit));
             // (the split keeps two accumulators per tile; 256 columns would leave one buffer: 16384 x 1024 -> 1024 125 -> 150 us)
             if (bn > 256 || (bn > 128 && P.planes == 2)) continue;
             double rounds = static_cast<double>(ceil_div(static_cast<int>(std::min<long long>(m_tiles_all * nt, 1 << 30)), limited(ds->sms)));
@@ -1302,13 +1310,14 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             }
         }
     }
-    // Row-major output through TMA stores when the geometry allows: the box is the 32 consecutive tile
-    // rows one epilogue warp owns (a sub-box of the tile's pixel box), 128 bytes of columns wide.  (Never phase-packed columns:
-    // they belong to several output pixels, and the packed image may be larger than the output.)
-    if (P.out_mode == OUT_NHWC && !P.shuf_sh && tune().tmastore) {
-        const int esz = P.out_f16 ? 2 : 4;
+    // Row-major output through TMA stores: the box is the 32 consecutive tile rows one epilogue warp owns (a sub-box of the tile's pixel
+    // box), 128 bytes of columns wide.  Columns past the row's end are clipped, so the one tile of a narrow result may end anywhere within
+    // a piece (its epilogue then stores accumulator columns of nobody's into the clipped part).  354 x 512 -> 80 forward, whose
+    // 96-column tile went through the plain epilogue and took a widened copy of the bias, 9.2 -> 6.3 us.
+    if (rows_by_tma) {
+        const int esz = out_es;
         const int cpi = 128 / esz;
-        if (P.bn % cpi == 0 && (static_cast<size_t>(N) * esz) % 16 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0) {
+        if (P.bn % cpi == 0 || P.n_tiles == 1) {
             const int wbx = 1 << P.wb_log2, hbx = 1 << P.hb_log2;
             const int bw = std::min(wbx, 32), bh = std::min(hbx, 32 / bw), bnn = 32 / (bw * bh);
             uint64_t cd[4] = {static_cast<uint64_t>(N), static_cast<uint64_t>(f.out_w), static_cast<uint64_t>(f.out_h),

@@ -333,8 +333,12 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    // two accumulators; the epilogue reads 32 columns at a time, so a 16-column tile still needs 16 + 32
-    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn : (P.bn < 32) ? P.bn + 32 : (P.bn * P.planes * kRowTiles) << P.tbufs_log2;
+    // two accumulators; the epilogue reads 32 columns at a time, so a 16-column tile still needs 16 + 32.  TMA-store epilogues read
+    // whole pieces: the last one of a tile that ends within it reads on behind the last accumulator.
+    constexpr uint32_t kPiece = kMode == MODE_FPROP && NML_IS_TMA_OUT(kOutMode) ? (kOutF16 ? 64 : 32) : 1;
+    const uint32_t tmem_need = P.wpatch ? P.w_mtiles * P.bn
+                               : (P.bn < 32 && kPiece == 1) ? P.bn + 32
+                               : ((P.bn * P.planes * kRowTiles) << P.tbufs_log2) + ((0u - static_cast<uint32_t>(P.bn)) & (kPiece - 1));
     const uint32_t tmem_cols = (tmem_need <= 32) ? 32 : (tmem_need <= 64) ? 64 : (tmem_need <= 128) ? 128
                                : (tmem_need <= 256) ? 256 : 512;
 

@@ -1,0 +1,59 @@
+"""Row-major results whose width is no multiple of a 128-byte piece of columns: they leave by TMA stores whose last piece hangs over the
+end of the row and is clipped there.  Widths around the pieces and the tiles, against float64, with guards around the result."""
+import pytest
+import torch
+
+from nectarml_b200 import ops
+from nectarml_b200.ops import ConvGeometry
+
+pytestmark = pytest.mark.gpu
+
+
+def guarded(*shape, dtype=torch.float16):
+    """A tensor inside a larger one of NaNs; check() says whether they are all still there."""
+    n = 1
+    for s in shape:
+        n *= s
+    whole = torch.full((n + 2048,), float("nan"), device="cuda", dtype=dtype)
+    return whole[1024:1024 + n].view(shape), lambda: bool(whole[:1024].isnan().all() and whole[1024 + n:].isnan().all())
+
+
+def assert_rounded(got, want):
+    """fp16 results of fp32 sums: one rounding (2^-11), the sums' own error below 2^-13 of the largest term."""
+    bound = want.abs() * 2.0 ** -11 + 2.0 ** -13 * want.abs().amax()
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+# one tile of 16 ... 224 columns, tiles whose width is rounded up to a piece (320: two of 192), few and many tiles per CTA
+@pytest.mark.parametrize("rows", [3, 129, 40001])
+@pytest.mark.parametrize("fout", [16, 24, 32, 40, 72, 96, 104, 160, 192, 224, 320, 328])
+def test_linear_rows(rows, fout):
+    gen = torch.Generator(device="cuda").manual_seed(rows + fout)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen).half()  # noqa: E731
+    x, w, b, dy = rnd(rows, 200), rnd(fout, 200), rnd(fout), rnd(rows, 200)
+    y, clean = guarded(rows, fout)
+    ops.linear_forward(x, w, b, out=y)
+    assert_rounded(y, x.double() @ w.double().t() + b.double())
+    assert clean()
+    dx, clean = guarded(rows, fout)  # the input gradient of a layer of `fout` inputs
+    ops.linear_backward_data(dy, w.t().contiguous(), out=dx)
+    assert_rounded(dx, dy.double() @ w.double().t())
+    assert clean()
+    ops.device_status()
+
+
+# patch walk with 16- and 32-column tiles (four accumulators behind one another), its phases, and fp32 rows of 16 columns
+@pytest.mark.parametrize("n,c_in,hw,c_out,k,s,transposed", [
+    (3, 64, 19, 16, 3, 1, False), (40, 64, 28, 24, 3, 1, False), (40, 32, 33, 96, 5, 1, False), (5, 64, 17, 48, 4, 2, True), (3, 40, 15, 80, 3, 2, False)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_convolution_rows(n, c_in, hw, c_out, k, s, transposed, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(c_in + c_out)
+    g = ConvGeometry(n, c_in, hw, hw, c_out, k, k, (s, s), (1, 1), transposed=transposed)
+    x = torch.randn(g.act_shape("in", "nhwc"), device="cuda", generator=gen).half()
+    w = (torch.randn(g.weight_shape(), device="cuda", generator=gen) * 0.1).half()
+    y, clean = guarded(*g.act_shape("out", "nhwc"), dtype=dtype)
+    ops.conv_forward(g, x, w, None, layout="nhwc", math="f16", out=y)
+    conv = torch.nn.functional.conv_transpose2d if transposed else torch.nn.functional.conv2d
+    assert_rounded(y, conv(x.permute(0, 3, 1, 2).double(), w.double(), stride=s, padding=1).permute(0, 2, 3, 1))
+    assert clean()
+    ops.device_status()

@@ -2,7 +2,8 @@
 
 ``python -m nectarml_b200.build`` compiles ``csrc/nml_api.cu`` (which includes the contraction
 kernels) and ``csrc/nml_layers.cu`` (normalisation / optimizer kernels of the training step) into ``nectarml_b200/libnectarml_b200.so``,
-and ``csrc/nml_torch.cpp`` (the tensor-level host path on top of that library's C ABI) into ``nectarml_b200/_native.so``.
+``csrc/nml_torch.cpp`` (the tensor-level host path on top of that library's C ABI) into ``nectarml_b200/_native.so``, and
+``csrc/nml_dropin.cpp`` (the drop-in's calls of the same ABI) into ``nectarml_b200/_dropin.so``.
 nvcc cross-compiles without a GPU.
 """
 from __future__ import annotations
@@ -19,6 +20,8 @@ HEADERS = [os.path.join(_HERE, "csrc", n) for n in ("nml_launch.cuh", "nml_ptx.c
 OUTPUT = os.path.join(_HERE, "libnectarml_b200.so")
 NATIVE_SOURCE = os.path.join(_HERE, "csrc", "nml_torch.cpp")
 NATIVE_OUTPUT = os.path.join(_HERE, "_native.so")
+DROPIN_SOURCE = os.path.join(_HERE, "csrc", "nml_dropin.cpp")
+DROPIN_OUTPUT = os.path.join(_HERE, "_dropin.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC"]
@@ -39,7 +42,8 @@ def _fresh(output: str, sources) -> bool:
 
 
 def up_to_date() -> bool:
-    return _fresh(OUTPUT, SOURCES + HEADERS) and _fresh(NATIVE_OUTPUT, [NATIVE_SOURCE, HEADERS[-1]])
+    return (_fresh(OUTPUT, SOURCES + HEADERS) and _fresh(NATIVE_OUTPUT, [NATIVE_SOURCE, HEADERS[-1]]) and
+            _fresh(DROPIN_OUTPUT, [DROPIN_SOURCE, HEADERS[-1]]))
 
 
 def _native_command():
@@ -55,6 +59,11 @@ def _native_command():
         f"-L{os.path.join(root, 'lib')}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
 
 
+def _dropin_command():
+    return ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-I{sysconfig.get_paths()['include']}", DROPIN_SOURCE,
+            "-o", DROPIN_OUTPUT, f"-L{_HERE}", "-l:libnectarml_b200.so", "-Wl,-rpath,$ORIGIN"]
+
+
 def _run(cmd, verbose: bool) -> None:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if verbose or res.returncode != 0:
@@ -64,11 +73,13 @@ def _run(cmd, verbose: bool) -> None:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Builds the library and the tensor-level module on top of it where their sources are newer; returns the library's path."""
+    """Builds the library and the two modules on top of it where their sources are newer; returns the library's path."""
     if force or not _fresh(OUTPUT, SOURCES + HEADERS):
         _run([_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", OUTPUT] + SOURCES, verbose)
     if force or not _fresh(NATIVE_OUTPUT, [NATIVE_SOURCE, HEADERS[-1]]):
         _run(_native_command(), verbose)
+    if force or not _fresh(DROPIN_OUTPUT, [DROPIN_SOURCE, HEADERS[-1]]):
+        _run(_dropin_command(), verbose)
     return OUTPUT
 
 

@@ -222,6 +222,7 @@ static int raise_smem_limit() {
         NML_CUDA(cudaFuncSetAttribute(gemm_instance<float>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
         NML_CUDA(cudaFuncSetAttribute(gemm_instance<__half>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
     }
+    NML_CUDA(cudaFuncSetAttribute(gemm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
     UmmaKernel all[19] = {umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, false, false, true>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
                           umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true>,
                           fprop_instance<OUT_NHWC_TMA, false>(true), fprop_instance<OUT_NHWC_TMA, false>(false),
@@ -1953,36 +1954,41 @@ static StridedPlan plan_strided(const StridedProduct& g, int sms) {
     return best;
 }
 
+static void fill_strided(GemmParams* P, const StridedProduct& g, const DeviceState* ds, int role) {
+    memset(P, 0, sizeof(*P));
+    P->a = g.a; P->b = g.b; P->bias = g.bias; P->out = g.out;
+    P->a_stride = g.a_stride; P->b_stride = g.b_stride; P->out_ns = g.out_ns;
+    P->a_batch = g.a_batch; P->b_batch = g.b_batch; P->out_batch = g.out_batch;
+    P->M = g.M; P->N = g.N; P->K = g.K;
+    P->tiles_m = ceil_div(g.M, kTileM);
+    const int es = g.dtype == NML_F32 ? 4 : 2;
+    const auto vec = [&](const void* p, long long stride, long long batch) {
+        return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && stride * es % 16 == 0 && batch * es % 16 == 0 ? 1 : 0;
+    };
+    P->a_vec = vec(g.a, g.a_stride, g.a_batch);
+    P->b_vec = vec(g.b, g.b_stride, g.b_batch);
+    P->bias_f16 = g.bias_dtype == NML_F16;
+    P->out_f16 = g.out_dtype == NML_F16;
+    P->round_f16 = g.round_f16;
+    P->role = role;
+    P->err = ds->err;
+    P->wait_limit_ns = g_dbg_wait_limit_ns;
+}
+
 static int run_strided(const StridedProduct& g, const StridedPlan& plan, int role, cudaStream_t st) {
     const bool f32 = g.dtype == NML_F32;
-    const int es = f32 ? 4 : 2, slice = f32 ? 32 : 64;
+    const int slice = f32 ? 32 : 64;
     DeviceState* ds = nullptr;
     int rc = device_state(&ds);
     if (rc) return rc;
     GemmParams P;
-    memset(&P, 0, sizeof(P));
-    P.a = g.a; P.b = g.b; P.bias = g.bias; P.out = g.out;
-    P.a_stride = g.a_stride; P.b_stride = g.b_stride; P.out_ns = g.out_ns;
-    P.a_batch = g.a_batch; P.b_batch = g.b_batch; P.out_batch = g.out_batch;
-    P.M = g.M; P.N = g.N; P.K = g.K;
+    fill_strided(&P, g, ds, role);
     P.bn = plan.bn;
-    P.tiles_m = ceil_div(g.M, kTileM);
     P.tiles_n = ceil_div(g.N, plan.bn);
     P.splits = plan.splits;
     P.per = ceil_div(ceil_div(g.K, slice), plan.splits);
     const int stage_bytes = (f32 ? 2 : 1) * (kStageABytes + plan.bn * 128);
     P.stages = f32 ? 2 : 4;  // (80 to 96 KB: two blocks to an SM)
-    const auto vec = [&](const void* p, long long stride, long long batch) {
-        return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && stride * es % 16 == 0 && batch * es % 16 == 0 ? 1 : 0;
-    };
-    P.a_vec = vec(g.a, g.a_stride, g.a_batch);
-    P.b_vec = vec(g.b, g.b_stride, g.b_batch);
-    P.bias_f16 = g.bias_dtype == NML_F16;
-    P.out_f16 = g.out_dtype == NML_F16;
-    P.round_f16 = g.round_f16;
-    P.role = role;
-    P.err = ds->err;
-    P.wait_limit_ns = g_dbg_wait_limit_ns;
     const long long blocks = 1ll * P.tiles_m * P.tiles_n * g.batch * plan.splits;
     if (blocks > INT_MAX) return NML_ERR_UNSUPPORTED;
     rc = profile_open(st);
@@ -1997,6 +2003,50 @@ static int run_strided(const StridedProduct& g, const StridedPlan& plan, int rol
     NML_CUDA(cudaGetLastError());
     ++g_launches;
     ++g_launches_of[NML_DEBUG_IN_PLACE];
+    return profile_stop(slot, st);
+}
+
+// A batched fp16 product with K <= kRowsMaxK by gemm_rows_kernel: b's rows are contiguous along k, a's columns along m.
+struct RowsPlan {
+    int splits = 1, per = 0;
+    double us = 0;
+};
+// Blocks that share a strip of 128 columns, by estimated time: two blocks to an SM, what starts and ends one, and its groups of 64 rows.
+// (By the groups of the busiest SM, which asks for fewer and longer blocks: 25 x 464 x 32 x 170 7.3 -> 9.5 us, 108 x 443 x 32 x 51 9.4 -> 13.0.)
+static RowsPlan plan_rows(const StridedProduct& g, int sms) {
+    const int groups = ceil_div(g.N, kRowsBn), slices = ceil_div(g.K, 64);
+    const double strips = static_cast<double>(g.batch) * ceil_div(g.M, kTileM);
+    RowsPlan best;
+    for (int z = 1; z <= groups; ++z) {
+        const int per = ceil_div(groups, z);
+        if (ceil_div(groups, per) != z) continue;
+        const double blocks = strips * z, waves = std::ceil(blocks / (2.0 * sms));
+        const double us = 2.5 + waves * (2.0 + 0.7 * slices) + waves * per * (blocks > sms ? 0.6 : 0.4);
+        if (best.per == 0 || us < best.us) best = {z, per, us};
+    }
+    return best;
+}
+static int run_rows(const StridedProduct& g, cudaStream_t st) {
+    DeviceState* ds = nullptr;
+    int rc = device_state(&ds);
+    if (rc) return rc;
+    const RowsPlan plan = plan_rows(g, limited(ds->sms));
+    GemmParams P;
+    fill_strided(&P, g, ds, PDL_NORMAL);
+    P.bn = kRowsBn;
+    P.tiles_n = ceil_div(g.N, kRowsBn);
+    P.splits = plan.splits;
+    P.per = plan.per;
+    const long long blocks = 1ll * P.tiles_m * g.batch * plan.splits;
+    if (blocks > INT_MAX) return NML_ERR_UNSUPPORTED;
+    rc = profile_open(st);
+    if (rc) return rc;
+    const int slot = g_bracket_slot;
+    g_bracket_slot = -1;
+    // (two blocks to an SM and none beside a block of the contraction kernel, as in run_strided)
+    launch_with(true, 1, gemm_rows_kernel, static_cast<unsigned>(blocks), kGemmThreads, 110 * 1024, st, P);
+    NML_CUDA(cudaGetLastError());
+    ++g_launches;
     return profile_stop(slot, st);
 }
 
@@ -2820,7 +2870,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
     // Us by rows / turned / in place: fp16 24 x 192 x 471 x 33 18.7 / 13.3 / 21.0; 64 x 333 x 64 x 333 25.7 / 16.0 / -; 128 x 33 x 64 x 33
     // 15.6 / 9.8 / 6.4; fp32 64 x 333 x 64 x 333 43.9 / 25.4 / 28.7; 3 x 800 x 96 x 801 - / 16.3 / 10.4; 85 x 12 x 284 x 1200 127 / 337 / 52;
     // 20 x 19698 x 6 x 1 29 / 166 / 91; 103 x 14010 x 2 x 39 323 / 191 / 341.
-    enum Way { BY_ROWS, TURNED, IN_PLACE };
+    enum Way { BY_ROWS, TURNED, IN_PLACE, STRIPS };
     auto way_of = [&](size_t n) -> Way {
         if (es == 2 && N % 8 == 0) return BY_ROWS;
         const int sms = planning_sms();
@@ -2828,6 +2878,11 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
         const double turned_us = N <= 8 ? 1e30 : batched_us(true, n, M, K, N, es, sms);
         double place_us = 1e30;
         if (g_sm_limit.load(std::memory_order_relaxed) == 0) {
+            // Strips of 128 columns, read in place (gemm_rows_kernel), for K loops of one or two slices.  Stores of 64 bytes that start anywhere bound
+            // large results whichever way they go, and two slices of both operands then cost more here than a conversion (28 x 726 x 96 x 844
+            // 24.6 us, turned 19.6; 128 x 511 x 128 x 513 57 and 51); very large ones are equal or up to 3 % slower (60 x 900 x 32 x 999 50.1 and 48.5).
+            const double groups = static_cast<double>(n) * ceil_div(N, kTileM) * ceil_div(M, kRowsBn) / sms;
+            if (es == 2 && K <= kRowsMaxK && N >= 32 && M >= 32 && groups <= (K <= 64 ? 32.0 : 8.0)) return STRIPS;
             const StridedPlan plan = plan_strided(in_place(nullptr, nullptr, nullptr, n), sms);
             const double result = n * static_cast<double>(M) * N * 1e-6;
             place_us = es == 4 ? 5.9 + 0.92 * plan.loop_us + 2.0 * (plan.waves - 1.0) + 0.32 * result
@@ -2845,12 +2900,13 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             d.math = math;
             return linear_pass(&d, NML_PASS_BACKWARD_DATA, A, B, nullptr, C, nullptr, bump, nullptr);
         }
-        if (way == IN_PLACE) {
+        if (way == IN_PLACE || way == STRIPS) {
             if (bump.dry) return NML_OK;
             // (fp16 rows that TMA was to read and cannot stay refused)
             const int rc = es == 2 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) != 0 ? rows_for_tma(A, K, M) : NML_OK;
             const StridedProduct g = in_place(A, B, C, n);
-            return rc ? rc : run_strided(g, plan_strided(g, planning_sms()), PDL_NORMAL, nullptr);
+            if (way == STRIPS && !rc) ++g_launches_of[NML_DEBUG_TURNED];
+            return rc ? rc : way == STRIPS ? run_rows(g, nullptr) : run_strided(g, plan_strided(g, planning_sms()), PDL_NORMAL, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));

@@ -343,4 +343,165 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_strided_kernel(const __g
     }
 }
 
+// ---- Batched fp16 products of short K loops (attention scores) whose rows are no whole vectors.
+// A block owns 128 columns of one entry's result and walks down its rows, 64 at a time.  Its columns of B (K x 128, at most two K slices)
+// are read once and stay in shared memory; the rows of A come 64 at a time, two groups ahead in registers, three in shared memory, two
+// accumulators in TMEM, so that the loads of a group, the MMAs of the one before and the stores of the one before that overlap.  The lanes of
+// the epilogue are consecutive columns, as above.  Bound by these stores, 64 bytes of a row that starts anywhere (about eight clocks each), and
+// for small products by launch and set-up.  By a conversion that turns B round, and the contraction kernel: 64 x 333 x 64 x 333 14.9 us, here
+// 13.1; 25 x 464 x 32 x 170 10.3, 7.3; 49 x 368 x 96 x 230 12.1, 9.3; 128 x 700 x 64 x 41 14.4, 11.3.  Put together in shared memory and stored as
+// whole 16-byte vectors, four warps meeting once a group, the same rows left more slowly (18.9 us instead of 13.1).
+constexpr int kRowsBn = 64, kRowsStages = 3, kRowsMaxK = 128;
+
+// P: M columns of the result, N rows, per groups of rows a block, splits blocks that share a 128-column strip.
+__global__ void __launch_bounds__(kGemmThreads, 2) gemm_rows_kernel(const __grid_constant__ GemmParams P) {
+    using X = GemmType<__half>;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    const int slices = (P.K + X::kSlice - 1) / X::kSlice;  // 1 or 2
+    constexpr uint32_t kGroupBytes = kRowsBn * 128;        // one K slice of a group of rows
+    const uint32_t rows_at = slices * kStageABytes, stage_bytes = slices * kGroupBytes;
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + rows_at + kRowsStages * stage_bytes);  // [3]
+    uint64_t* empty_bar = full_bar + kRowsStages;                                                  // [3]
+    uint64_t* tfull_bar = empty_bar + kRowsStages;                                                 // [2]
+    uint64_t* tempty_bar = tfull_bar + 2;                                                          // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr uint32_t tmem_cols = 2 * kRowsBn;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kRowsStages; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), kGemmProducers / 32);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&tfull_bar[b]), 1);
+            mbar_init(smem_u32(&tempty_bar[b]), kGemmProducers / 32);
+        }
+        abort_state_init(abort_flag, P.wait_limit_ns);
+        fence_mbar_init();
+    }
+    if (warp == 8) {
+        tmem_alloc(smem_u32(tmem_slot), tmem_cols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_enter(P.role);  // (behind the allocation, as above)
+
+    int strip = blockIdx.x / P.splits;
+    const int first = (blockIdx.x - strip * P.splits) * P.per;
+    const int batch = strip / P.tiles_m, m0 = (strip - batch * P.tiles_m) * kTileM;
+    const int groups = max(min(P.tiles_n, first + P.per) - first, 0);
+    bool ok = true;
+    if (warp < 8) {
+        const __half* const rows = static_cast<const __half*>(P.b) + batch * P.b_batch;
+        const int row0 = threadIdx.x >> 3, chunk0 = threadIdx.x & 7;
+        uint4 v0[4], v1[4];  // [slice][row half] of a group of rows
+        auto load = [&](uint4 (&v)[4], int group) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = (first + group) * kRowsBn + row0 + 32 * (i & 1), k = (i >> 1) * X::kSlice + chunk0 * X::kChunk;
+                if ((i >> 1) >= slices) break;
+                const int n = row < P.N && group < groups ? P.K - k : 0;
+                const __half* const q = rows + row * P.b_stride + k;
+                if (P.b_vec && n >= X::kChunk) v[i] = load_global(reinterpret_cast<const uint4*>(q));
+                else v[i] = gemm_gather(q, 1, n);
+            }
+        };
+        {
+            GemmOperand<__half, false> A(static_cast<const __half*>(P.a) + batch * P.a_batch, P.a_stride, m0, P.M, kTileM, 0, 0);
+            uint4 a[4];
+            A.load(a, P.K);
+            load(v0, 0);
+            load(v1, 1);
+            A.store(a, smem_u32(smem), 0);
+            if (slices == 2) {
+                A.load(a, P.K - X::kSlice);
+                A.store(a, smem_u32(smem) + kStageABytes, 0);
+            }
+        }
+        // ---------------------------------------------------------- epilogue of a group --
+        const int quarter = warp & 3, half = warp >> 2, m = m0 + quarter * 32 + lane;
+        auto drain = [&](int group) -> bool {
+            const int buf = group & 1, n = (first + group) * kRowsBn + 32 * half;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&tfull_bar[buf]), (group >> 1) & 1, abort_flag, P.err, ERR_WAIT_TMEM_FULL))) return false;
+            tc_fence_after();
+            uint32_t r[32];
+            tmem_ld_32x32(tmem + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kRowsBn + 32 * half, r);
+            tmem_ld_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&tempty_bar[buf]));
+            if (m < P.M && n < P.N)
+                store_columns(static_cast<__half*>(P.out) + batch * P.out_batch + m + n * P.out_ns, P.out_ns, r, min(32, P.N - n));
+            __syncwarp();
+            return true;
+        };
+        int stage = 0;
+        uint32_t parity = 1;
+        auto step = [&](uint4 (&v)[4], int group) -> bool {
+            if (group < groups) {
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&empty_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_EMPTY))) return false;
+                const uint32_t at = smem_u32(smem) + rows_at + stage * stage_bytes;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if ((i >> 1) >= slices) break;
+                    const int r = row0 + 32 * (i & 1);
+                    st_shared_v4(at + (i >> 1) * kGroupBytes + r * 128 + ((chunk0 ^ (r & 7)) << 4), v[i]);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&full_bar[stage]));
+                if (++stage == kRowsStages) {
+                    stage = 0;
+                    parity ^= 1;
+                }
+                load(v, group + 2);
+            }
+            return group == 0 || drain(group - 1);
+        };
+        for (int g = 0; ok && g <= groups && groups > 0; g += 2) {
+            ok = step(v0, g);
+            if (ok && g + 1 <= groups) ok = step(v1, g + 1);
+        }
+    } else {
+        const uint32_t idesc = make_instr_desc(X::kKind, 0, 0, kTileM, kRowsBn);
+        int stage = 0;
+        uint32_t parity = 0;
+        for (int g = 0; g < groups; ++g) {
+            const int buf = g & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&tempty_bar[buf]), ((g >> 1) & 1) ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) ||
+                !__all_sync(0xffffffffu, mbar_wait(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)))
+                break;
+            tc_fence_after();
+            if (elect_one()) {
+                for (int s = 0; s < slices; ++s) {
+                    const uint64_t a = make_smem_desc(smem_u32(smem) + s * kStageABytes, 16, 1024, 2);
+                    const uint64_t b = make_smem_desc(smem_u32(smem) + rows_at + stage * stage_bytes + s * kGroupBytes, 16, 1024, 2);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) umma_f16(tmem + buf * kRowsBn, a + 2 * k, b + 2 * k, idesc, k || s ? 1u : 0u);
+                }
+                umma_commit(smem_u32(&empty_bar[stage]));
+                umma_commit(smem_u32(&tfull_bar[buf]));
+            }
+            __syncwarp();
+            if (++stage == kRowsStages) {
+                stage = 0;
+                parity ^= 1;
+            }
+        }
+    }
+    pdl_leave(P.role);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 8) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem, tmem_cols);
+    }
+}
+
 }  // namespace nml

@@ -173,7 +173,7 @@ struct DeviceState {
 static DeviceState g_dev[64];
 static std::mutex g_dev_mutex;   // guards g_dev, g_static, g_prof and g_ref_ws
 static std::atomic<long long> g_launches{0};
-static std::atomic<long long> g_launches_of[4];  // by kind, see nml_debug_launch_count
+static std::atomic<long long> g_launches_of[5];  // by kind, see nml_debug_launch_count
 // Where kernels report an abandoned wait.  The words live in the library image, so set-up needs no
 // allocation: their device addresses come from cudaGetSymbolAddress, once per device.
 static __device__ int g_status_word;
@@ -194,7 +194,16 @@ template <int kOut, bool kPair>
 static UmmaKernel fprop_instance(bool f16) {
     return f16 ? umma_conv_kernel<MODE_FPROP, kOut, true, kPair> : umma_conv_kernel<MODE_FPROP, kOut, false, kPair>;
 }
+template <int kOut>
+static UmmaKernel stream_instance(bool f16) {
+    return f16 ? umma_conv_kernel<MODE_FPROP, kOut, true, false, false, false, true> : umma_conv_kernel<MODE_FPROP, kOut, false, false, false, false, true>;
+}
 static UmmaKernel kernel_for(const KParams& P) {
+    if (P.b_taps) {
+        if (P.out_mode == OUT_NHWC_TMA) return stream_instance<OUT_NHWC_TMA>(P.out_f16);
+        if (P.out_mode == OUT_NCHW_TMA) return stream_instance<OUT_NCHW_TMA>(P.out_f16);
+        return P.out_mode == OUT_NHWC ? stream_instance<OUT_NHWC>(P.out_f16) : stream_instance<OUT_NCHW>(P.out_f16);
+    }
     if (P.add) return umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, false, false, true>;
     if (P.dbl)
         return P.mode == MODE_WGRAD ? umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true> : umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>;
@@ -223,7 +232,10 @@ static int raise_smem_limit() {
         NML_CUDA(cudaFuncSetAttribute(gemm_instance<__half>(i & 1, i & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
     }
     NML_CUDA(cudaFuncSetAttribute(gemm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448));
-    UmmaKernel all[19] = {umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, false, false, true>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
+    UmmaKernel all[27] = {stream_instance<OUT_NHWC_TMA>(true), stream_instance<OUT_NHWC_TMA>(false), stream_instance<OUT_NCHW_TMA>(true),
+                          stream_instance<OUT_NCHW_TMA>(false), stream_instance<OUT_NHWC>(true), stream_instance<OUT_NHWC>(false),
+                          stream_instance<OUT_NCHW>(true), stream_instance<OUT_NCHW>(false),
+                          umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, false, false, true>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true, true>, umma_conv_kernel<MODE_FPROP, OUT_NHWC_TMA, true, true, true>,
                           umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, false>, umma_conv_kernel<MODE_WGRAD, OUT_NHWC, false, true>,
                           fprop_instance<OUT_NHWC_TMA, false>(true), fprop_instance<OUT_NHWC_TMA, false>(false),
                           fprop_instance<OUT_NCHW_TMA, false>(true), fprop_instance<OUT_NCHW_TMA, false>(false),
@@ -704,6 +716,30 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     } else if (P.patch) {
         // [resident B slices][patch buffers][staging][bias][barriers]
         P.ka = 1;
+        if (P.b_taps) {
+            // [B stages][patch buffers]: two channel blocks' patches, and the taps of as much of a channel block to a stage as two stages
+            // have room for.  (What a stage costs besides its MMAs, about 400 clocks, is spread over its taps: 3x3 256 -> 64 at 32 x 32, batch 64,
+            // two taps to a stage 44 us, three 38, five 35, nine 33.)
+            const int slice = P.planes * P.bn * 128, patches = P.planes * P.patch_bytes;
+            P.stg_bufs = 1;
+            int avail = 232448 - fixed - P.epi_warps * kStagingBufBytes - 2 * patches;
+            if (avail < 3 * slice && P.epi_warps == 8) {
+                P.epi_warps = 4;
+                P.epi_alt = 0;
+                P.tbufs_log2 = std::min(P.tbufs_log2, 1);
+                avail += 4 * kStagingBufBytes;
+            }
+            if (avail < 2 * slice) return NML_ERR_UNSUPPORTED;  // (two patches of 130 KB at most leave more)
+            const int most = std::max(1, std::min(P.planes == 2 ? kStreamTapsSplit : kStreamTaps, avail / slice / 2));
+            P.b_taps = ceil_div(P.b_taps, ceil_div(P.b_taps, most));
+            P.stages = std::min(8, avail / (P.b_taps * slice));
+            avail -= P.stages * P.b_taps * slice;
+            P.a_stages = std::min(4, 2 + avail / patches);
+            P.a_ring_off = P.stages * P.b_taps * slice;
+            P.ring_bytes = P.a_ring_off + P.a_stages * patches;
+            P.issuers = 1;
+            smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
+        } else {
         const int res_bytes = P.c_blocks * P.n_taps * P.bn * P.b_row_bytes;  // the taps of every phase
         P.stg_bufs = P.epi_warps == 8 ? 1 : 2;  // (alternate groups return to a buffer after two tiles; patches need the room)
         int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
@@ -725,6 +761,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         P.a_ring_off = static_cast<int>(round_up(res_bytes, 1024));
         P.ring_bytes = P.a_ring_off + P.a_stages * P.patch_bytes;
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
+        }
     } else {
     // (a double tile's warps have one buffer each, or none where they store from registers)
     int stages2 = P.dbl ? 0 : (232448 - fixed - P.epi_warps * 2 * kStagingBufBytes) / stage_bytes;
@@ -758,6 +795,7 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
     // a block of this kernel leaves no room beside it)
     if (P.dbl) ++g_launches_of[NML_DEBUG_DOUBLE_TILES];
     if (P.add) ++g_launches_of[NML_DEBUG_SUMS];
+    if (P.mode == MODE_FPROP && P.b_taps) ++g_launches_of[NML_DEBUG_STREAMED];
     launch_with(g_sm_limit.load(std::memory_order_relaxed) == 0, P.pair ? 2 : 1, kernel_for(P), grid, threads, smem, st, P);
     NML_CUDA(cudaGetLastError());
     if (open_slot) *open_slot = rec_slot;
@@ -1181,7 +1219,8 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     // taps and patch origin; the box is sized for the widest phase.
     const int patch_mode = tune().patch;
     int pw_ = 0, ph_ = 0;
-    bool patch_fits = false;
+    bool patch_fits = false, can_patch = false;
+    int taps_max = 0;
     {
         int range_w = 0, range_h = 0;
         bool every_phase_has_taps = true;
@@ -1191,6 +1230,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                 every_phase_has_taps = false;
                 continue;
             }
+            taps_max = std::max<int>(taps_max, ph.tap_count);
             int dw_min = 0, dw_max = 0, dh_min = 0, dh_max = 0;
             for (int t = 0; t < ph.tap_count; ++t) {
                 const Tap& tp = P.taps[ph.tap_begin + t];
@@ -1207,14 +1247,12 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         // (a row stride of the walk only stretches the patch: consecutive output rows are esh patch rows apart)
         pw_ = 8 + range_w;
         ph_ = 15 * esh + range_h + 1;
-        const bool can = every_phase_has_taps && n_taps >= 2 && esw == 1 && pw_ <= 256 && ph_ <= 256 &&
+        can_patch = every_phase_has_taps && n_taps >= 2 && esw == 1 && pw_ <= 256 && ph_ <= 256 &&
                          pw_ * ph_ * row_bytes <= 48 * 1024;
-        // Every weight slice stays in shared memory beside two patch buffers and the smallest epilogue staging.  (Weights
-        // streamed tap by tap cost a barrier round trip per four short MMAs; that form once paid for the 3xTF32 split and no
-        // longer does: 3x3 128 -> 128 at 56 x 56, batch 16 116 -> 71 us without it, 64 -> 64 at batch 8 30.2 -> 27.5.)
+        // Every weight slice stays in shared memory beside two patch buffers and the smallest epilogue staging (else they are streamed, below).
         const int bn_res = N <= 16 ? 16 : static_cast<int>(round_up(N, 32));
         const long long res_need = 1ll * c_blocks * n_taps * bn_res * row_bytes + 2 * round_up(pw_ * ph_ * row_bytes, 1024);
-        patch_fits = can && patch_mode && P.planes == 1 && N <= 256 && !b_mn_major && res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
+        patch_fits = can_patch && patch_mode && P.planes == 1 && N <= 256 && !b_mn_major && res_need <= 232448 - kFixedSmem - 4 * kStagingBufBytes;
     }
     if (f.w_batched) {  // a tile never straddles two images
         P.b_batched = 1;
@@ -1234,6 +1272,34 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             P.patch_w = pw_;
             P.patch_h = ph_;
             P.patch_bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024));
+        }
+        // The patch walk with streamed weights, where they do not stay: for tiles that do not pair up (pairs of 128 and 256 columns are as
+        // fast or faster by boxes: 3x3 128 -> 128 at 64 x 64, batch 64, 72 us, 73 so), which wait for their operands.  A patch is read once for all
+        // taps, but its tiles are 8 x 16 pixels of one image; so by rounds of tiles and the measured ratio of a slice's time, which falls with the
+        // taps that share a patch.  By boxes / so, us: fp16 3x3 256 -> 64 at 32 x 32, batch 64, 39.2 / 32.7; 256 -> 192 at 64 x 64 222 / 179; 64 -> 144
+        // at 31 x 31, batch 87, 28.5 / 23.1; 5x5 192 -> 24 at 99 x 99, batch 4, 61.0 / 40.7; transposed 4x4 512 -> 64 at 64 x 64, batch 16, 114 / 102; fp32
+        // 3x3 128 -> 32 at 64 x 64, batch 16, 88.8 / 75.4; input gradient of 3 -> 234 at 145 x 145, batch 14, 966 / 766.  One tap a phase gains nothing
+        // (2x2 s2 transposed 960 -> 40 149 / 182).  Of 90 random passes 24 take it, with 0.85 of the time in the mean.
+        if (!P.patch && can_patch && patch_mode && taps_max >= 2 && !b_mn_major && !window && !f.w_batched && !f.shuf_sh && !f.add && !can_split &&
+            (P.planes == 2 ? N <= 64 : P.kind == KIND_F16 && (N <= 64 || (N > 128 && N <= 224)))) {
+            const int bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024)), sms = limited(ds->sms);
+            const double slice = (P.planes == 2 ? (N <= 32 ? 0.83 : 0.92) : N <= 32 ? 0.75 : N <= 64 ? 0.86 : 0.82) * (taps_max >= 12 ? 0.85 : 1.0);
+            long long patches = 0, boxes = 0;
+            for (int p = 0; p < n_phases; ++p) {
+                const Phase& ph = P.phases[p];
+                patches += 1ll * ceil_div(ph.wq, 8) * ceil_div(ph.hq, 16) * f.batch;
+                boxes += 1ll * ceil_div(ph.wq, 1 << P.wb_log2) * ceil_div(ph.hq, 1 << P.hb_log2) * ceil_div(f.batch, 1 << P.nb_log2);
+            }
+            const auto rounds = [&](long long n) { return static_cast<double>((n + sms - 1) / sms); };
+            if (rounds(patches) * slice <= rounds(boxes) * 0.95 && 2ll * P.planes * bytes <= 130 * 1024) {
+                P.patch = 1;
+                P.patch_w = pw_;
+                P.patch_h = ph_;
+                P.patch_bytes = bytes;
+                P.b_taps = taps_max;  // (how many there is room for: launch_kernel)
+            }
+        }
+        if (P.patch) {
             for (int p = 0; p < n_phases; ++p)
                 for (int t = 0; t < P.phases[p].tap_count; ++t) {
                     Tap& tp = P.taps[P.phases[p].tap_begin + t];
@@ -1259,7 +1325,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         for (int p = 0; p < n_phases; ++p)
             m_tiles_all += 1ll * ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) *
                            ceil_div(f.batch, 1 << P.nb_log2);
-        const int forced = P.patch ? (N <= 16 ? 16 : static_cast<int>(round_up(N, 32)))
+        const int forced = P.patch && !P.b_taps ? (N <= 16 ? 16 : static_cast<int>(round_up(N, 32)))
                                    : P.planes == 2 ? std::min(tune().bn, 128) : tune().bn;
         const int cand[4] = {256, 128, 64, forced};
         const double cost[3] = {1.0, 1.28, 2.24};
@@ -2544,7 +2610,7 @@ int nml_device_status(int* code) {
 
 long long nml_launch_count(void) { return g_launches.load() + nml_layers_launch_count(); }
 
-long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 4 ? g_launches_of[kind].load() : -1; }
+long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 5 ? g_launches_of[kind].load() : -1; }
 
 int nml_profile_begin(int max_records) {
     if (max_records <= 0 || max_records > 1 << 16) return NML_ERR_INVALID;

@@ -26,6 +26,8 @@
 //               Covers Conv2d / ConvTranspose2d weight-gradient and Linear weight-gradient.
 // 256-wide tiles of long-K problems run as CTA pairs (cta_group::2, see the kernel's comment).
 #pragma once
+#include <type_traits>
+
 #include "nml_launch.cuh"
 #include "nml_ptx.cuh"
 
@@ -47,6 +49,7 @@ enum {
 
 constexpr int kMaxPhases = 16;
 constexpr int kMaxTaps = 128;
+constexpr int kStreamTaps = 9, kStreamTapsSplit = 5;  // patch walk with streamed weights: taps of a stage, at most
 constexpr int kTileM = 128;
 constexpr int kStageABytes = kTileM * 128;
 constexpr int kThreads = 224;      // warp 0: A loads, warp 1: MMA issue, warps 2-5: epilogue, warp 6: B loads
@@ -110,7 +113,7 @@ struct KParams {
     // descriptor starts (dh * patch_w + dw) rows in, and 8-row groups are patch_w rows apart.  (The swizzle
     // is a function of the shared-memory address, so a descriptor may start on any 128-byte row.)
     // A is then read from L2 about once instead of once per tap.  Every B slice is loaded once and stays in shared memory for
-    // the whole launch (the walk is taken only where all of them fit).
+    // the whole launch where all of them fit, else they are streamed (b_taps).
     // Forward walk, few tiles and a long K loop (U-Net bottleneck layers): the K iterations of a tile are
     // cut into fsplit slices that run as separate tiles; slice z stores its partial sums into plane z
     // of a row-major scratch, and a small pass adds the planes in order and produces the output.
@@ -138,8 +141,10 @@ struct KParams {
     int w_mtiles;        // row tiles (accumulators), w_mtiles * bn <= 512
     int w_coalesce;      // 1: the partial gradient leaves through shared memory as contiguous runs of stores
                          //    (needs 32 gradient columns, 32 * c_patch * taps floats, to fit in the operand ring)
-    int patch;           // 1: patch walk (one plane, one column tile; every B slice of the launch is loaded once, at
-                         //    [channel block][tap] * bn * b_row_bytes)
+    int patch;           // 1: patch walk
+    int b_taps;          // 0: every B slice of the launch is loaded once, at [channel block][tap] * bn * b_row_bytes (one plane, one
+                         //    column tile).  Else B slices are streamed through the ring of `stages`, so many taps to a stage, each
+                         //    [tap][plane] * bn * b_row_bytes
     int patch_w, patch_h;    // patch extent in pixels
     int patch_bytes;     // bytes one patch buffer occupies (multiple of 1024)
     int a_row_bytes;     // bytes of one patch row: 128, or 64 in the narrow window walks (up to 4 image channels; 64-byte
@@ -298,9 +303,12 @@ __device__ __forceinline__ void store_columns(T* o, size_t stride, const uint32_
 // clocks and takes 1045 to 1060 (Linear; convolutions, whose slices arrive in more pieces, 720 and 1350).  At 256 columns the two
 // accumulators fill TMEM, so nothing overlaps the drain: the epilogue takes a tile into registers as fp16 and hands the
 // accumulators back before it stores anything, one group of four warps to a row tile.
-template <int kMode, int kOutMode, bool kOutF16, bool kPair, bool kDbl = false, bool kAdd = false>
+// kStream: the patch walk with streamed weights, an instance of its own (in the others its unrolled issue loop, never run, cost a Linear
+// layer of 4096 rows 1.6 %).
+template <int kMode, int kOutMode, bool kOutF16, bool kPair, bool kDbl = false, bool kAdd = false, bool kStream = false>
 __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1) umma_conv_kernel(const __grid_constant__ KParams P) {
     static_assert(!kDbl || kPair, "double tiles are tiles of CTA pairs");
+    static_assert(!kStream || (kMode == MODE_FPROP && !kPair && !kAdd), "streamed patch walks are forward walks of single CTAs");
     static_assert(!kAdd || (kMode == MODE_FPROP && kOutMode == OUT_NHWC_TMA && kOutF16 && !kPair), "sums are fp16 rows of single CTAs");
     constexpr int kRowTiles = kDbl ? 2 : 1;
     constexpr bool kPoll = kMode == MODE_FPROP && kOutF16 && !kDbl;  // how waits begin, see mbar_poll
@@ -344,7 +352,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < P.stages; ++s) {
-            mbar_init(smem_u32(&full_bar[s]), 2);  // one arrival (with its byte count) per producer warp
+            mbar_init(smem_u32(&full_bar[s]), kStream ? 1 : 2);  // one arrival (with its byte count) per producer warp
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
         for (int b = 0; b < 4; ++b) {
@@ -488,6 +496,77 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
         }
     };
 
+    // Patch walk with streamed B: the MMA issue loop.  The taps of a channel block read the patch that lies there; their B slices come
+    // through the ring, b_taps (at most kStreamTaps) to a stage: a barrier round trip per tap would outlast four MMAs of 64 columns.  One
+    // thread's instructions bound it, so what a stage's MMAs need is worked out before the wait for it, and the taps are unrolled.
+    auto patch_streamed_issue = [&](auto split) {
+        constexpr bool kSplit = decltype(split)::value;
+        constexpr int kTaps = kSplit ? kStreamTapsSplit : kStreamTaps;
+        const uint32_t idesc = make_instr_desc(P.kind, 0, 0, kTileM, P.bn);
+        const uint32_t b_step = static_cast<uint32_t>(stage_b_bytes) >> 4, tap_step = kSplit ? 2 * b_step : b_step, stage_step = P.b_taps * tap_step;
+        const uint32_t a_plane = static_cast<uint32_t>(P.patch_bytes) >> 4, patch_step = kSplit ? 2 * a_plane : a_plane;
+        const uint64_t b_first = make_smem_desc(smem_u32(smem), 16, 1024, 2);
+        const uint64_t a_first = make_smem_desc(smem_u32(smem + P.a_ring_off), 16, static_cast<uint32_t>(P.patch_w * P.a_stride_h * 128), 2);
+        int titer = 0, p = 0, stage = 0, pstage = 0;
+        uint32_t parity = 0, pparity = 0;
+        for (int tile = tile_first; tile < P.num_tiles; tile += tile_step, ++titer) {
+            while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
+            const Tap* tp = &P.taps[P.phases[p].tap_begin];
+            const int nt = P.phases[p].tap_count;
+            const int buf = titer & ((1 << P.tbufs_log2) - 1);
+            if (!mbar_wait<kPoll>(smem_u32(&tempty_bar[buf]), ((titer >> P.tbufs_log2) & 1) ^ 1, abort_flag, P.err, ERR_WAIT_TMEM_EMPTY)) return;
+            tc_fence_after();
+            const uint32_t d_main = tmem_base + buf * P.bn * P.planes, d_cross = d_main + P.bn;
+            uint32_t acc = 0;
+            for (int cb = 0; cb < P.c_blocks; ++cb) {
+                const uint64_t a0 = a_first + static_cast<uint64_t>(pstage * patch_step);
+                for (int t0 = 0; t0 < nt; t0 += P.b_taps) {
+                    const int n = min(P.b_taps, nt - t0);
+                    uint64_t a[kTaps];
+#pragma unroll
+                    for (int t = 0; t < kTaps; ++t) a[t] = a0 + static_cast<uint32_t>(tp[min(t0 + t, nt - 1)].aoff);
+                    const uint64_t b0 = b_first + static_cast<uint64_t>(stage * stage_step);
+                    if (t0 == 0 && !mbar_wait<kPoll>(smem_u32(&afull_bar[pstage]), pparity, abort_flag, P.err, ERR_WAIT_FULL)) return;
+                    if (!mbar_wait<kPoll>(smem_u32(&full_bar[stage]), parity, abort_flag, P.err, ERR_WAIT_FULL)) return;
+                    tc_fence_after();
+                    if (elect_one()) {
+#pragma unroll
+                        for (int t = 0; t < kTaps; ++t) {
+                            if (t >= n) break;
+                            const uint64_t b = b0 + t * tap_step;
+                            if (kSplit) {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_tf32(d_cross, a[t] + 2 * k, b + b_step + 2 * k, idesc, t || k ? 1u : acc);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_tf32(d_cross, a[t] + a_plane + 2 * k, b + 2 * k, idesc, 1u);
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_tf32(d_main, a[t] + 2 * k, b + 2 * k, idesc, t || k ? 1u : acc);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) umma_f16(d_main, a[t] + 2 * k, b + 2 * k, idesc, t || k ? 1u : acc);
+                            }
+                        }
+                        umma_commit(smem_u32(&empty_bar[stage]));
+                        if (t0 + n == nt) {
+                            umma_commit(smem_u32(&aempty_bar[pstage]));
+                            if (cb + 1 == P.c_blocks) umma_commit(smem_u32(&tfull_bar[buf]));
+                        }
+                    }
+                    acc = 1u;
+                    if (++stage == P.stages) {
+                        stage = 0;
+                        parity ^= 1;
+                    }
+                    __syncwarp();
+                }
+                if (++pstage == P.a_stages) {
+                    pstage = 0;
+                    pparity ^= 1;
+                }
+            }
+        }
+    };
+
     // A producer that gave up: copies already issued get a bounded chance to land before the CTA's shared memory goes away.
     auto drain_ring = [&](int s, uint32_t par, int issued) {
         for (int back = issued < P.stages ? issued : P.stages; back > 0; --back) {
@@ -618,9 +697,9 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
         const int boxes_per_atom = (kMode != MODE_WGRAD || kPair) ? 1
                                    : do_a ? (P.a_grouped ? 1 : kTileM / P.kb) : (P.b_grouped ? 1 : P.bn / P.kb);
         const int issue_lanes = P.wpatch || (kMode == MODE_WGRAD && kPair) ? 1
-                                : P.patch ? 1 : P.ka * boxes_per_atom;
+                                : kStream && do_b ? P.b_taps * P.planes : P.patch ? 1 : P.ka * boxes_per_atom;
         const uint32_t issue_mask = (1u << issue_lanes) - 1u;
-        if (kMode == MODE_FPROP && !kPair && P.patch && do_b) {
+        if (kMode == MODE_FPROP && !kPair && !kStream && P.patch && do_b) {
             // Resident weights: every slice once, for the whole launch (one column tile, one pass plane, K-major
             // repacked weights).  The slices are spread over the lanes of the warp, so the dozens of TMA issues at
             // the start of the kernel cost one thread's worth of them, not their sum.
@@ -663,7 +742,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         tma_load_2d(sb + j * box_bytes, tb, fb, ntile * P.bn + j * P.kb, tap.wk + cb * P.kb);
                 }
             };
-            if (kMode == MODE_FPROP && !kPair && P.patch) {
+            if (kMode == MODE_FPROP && !kPair && (kStream || P.patch)) {
                 if (do_a) {
                     const uint32_t a_base = smem_u32(smem + P.a_ring_off);
                     const uint32_t patch_tx = static_cast<uint32_t>(P.patch_w) * P.patch_h * P.a_row_bytes;
@@ -683,8 +762,10 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                                 break;
                             }
                             const uint32_t fb = smem_u32(&afull_bar[abuf]);
-                            mbar_arrive_expect_tx(fb, patch_tx);
-                            tma_load_4d(a_base + abuf * P.patch_bytes, &P.tmA[0], fb, cb * P.kb, w0, h0, tn);
+                            const int planes = kStream ? P.planes : 1;
+                            mbar_arrive_expect_tx(fb, patch_tx * planes);
+                            for (int pl = 0; pl < planes; ++pl)
+                                tma_load_4d(a_base + (abuf * planes + pl) * P.patch_bytes, &P.tmA[pl], fb, cb * P.kb, w0, h0, tn);
                             ++issued;
                             if (++abuf == P.a_stages) {
                                 abuf = 0;
@@ -710,6 +791,35 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                     }
                     ok = true;   // nothing left for the common unwinding below
                     issued = 0;
+                } else if constexpr (kStream) {
+                    // B slices of the taps of a stage, by one lane each
+                    const int my_tap = P.planes == 2 ? lane >> 1 : lane, plane = P.planes == 2 ? lane & 1 : 0;
+                    int p = 0;
+                    for (int tile = tile_first; ok && tile < P.num_tiles; tile += tile_step) {
+                        while (p + 1 < P.n_phases && tile >= P.phases[p + 1].tile_begin) ++p;
+                        const Phase& pt = P.phases[p];
+                        int ntile, tw, th, tn;
+                        decode_fprop_tile<false>(P, pt, tile - pt.tile_begin, 0u, ntile, tw, th, tn);
+                        for (int cb = 0; ok && cb < P.c_blocks; ++cb)
+                            for (int t0 = 0; t0 < pt.tap_count; t0 += P.b_taps) {
+                                const uint32_t fb = smem_u32(&full_bar[stage]);
+                                if (!__all_sync(issue_mask, mbar_wait<kPoll>(smem_u32(&empty_bar[stage]), parity ^ 1, abort_flag, P.err, ERR_WAIT_EMPTY))) {
+                                    ok = false;
+                                    break;
+                                }
+                                const int n = min(P.b_taps, pt.tap_count - t0);
+                                if (lane == 0) mbar_arrive_expect_tx(fb, n * P.planes * stage_b_bytes);
+                                __syncwarp(issue_mask);
+                                if (my_tap < n)
+                                    tma_load_2d(smem_u32(smem) + (stage * P.b_taps * P.planes + lane) * stage_b_bytes, &P.tmB[plane], fb,
+                                                P.taps[pt.tap_begin + t0 + my_tap].wk + cb * P.kb, ntile * P.bn);
+                                ++issued;
+                                if (++stage == P.stages) {
+                                    stage = 0;
+                                    parity ^= 1;
+                                }
+                            }
+                    }
                 } else {
                     // (the slices were requested above, by the whole warp)
                     const uint32_t fb = smem_u32(bres_bar);
@@ -723,7 +833,7 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
                         }
                     }
                 }
-            } else
+            } else if constexpr (!kStream)
             for (int tile_id = tile_first; ok && tile_id < P.num_tiles; tile_id += tile_step) {
                 int tile = tile_id, kz = 0;
                 if (kMode == MODE_FPROP && P.fsplit > 1) {
@@ -992,9 +1102,9 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
         uint32_t parity = 0;
         bool ok = true;
         int titer = 0;
-        if (kMode == MODE_FPROP && !kPair && P.patch) {
+        if (kStream || (kMode == MODE_FPROP && !kPair && P.patch)) {
             // (issued below, by one copy of the loop for both issuers)
-        } else
+        } else if constexpr (!kStream)
         for (int tile_id = tile_first; ok && (!kPair || leader) && tile_id < P.num_tiles; tile_id += tile_step, ++titer) {
             int tile = tile_id, kz = 0;
             if (kMode == MODE_FPROP && P.fsplit > 1) {
@@ -2095,7 +2205,12 @@ __global__ void __launch_bounds__(kDbl ? kThreadsWide : threads_for(kOutMode), 1
         }
     }
 
-    if (kMode == MODE_FPROP && !kPair && P.patch && (warp == 1 || (warp == 6 && P.issuers == 2))) {
+    if constexpr (kStream) {
+        if (warp == 1) {
+            if (P.planes == 2) patch_streamed_issue(std::true_type());
+            else patch_streamed_issue(std::false_type());
+        }
+    } else if (kMode == MODE_FPROP && !kPair && P.patch && (warp == 1 || (warp == 6 && P.issuers == 2))) {
         __syncwarp();  // (warp 6 comes from a loop that one lane ran)
         patch_resident_issue(warp == 6 ? 1 : 0, P.issuers);
     }

@@ -1,0 +1,63 @@
+"""The patch walk whose weights do not stay in shared memory: the taps of a channel block read one patch, their weights come through a ring, a
+few taps to a stage."""
+import pytest
+import torch
+
+from gpu_util import assert_f32
+from nectarml_b200 import _lib, ops
+from nectarml_b200.ops import ConvGeometry
+
+pytestmark = pytest.mark.gpu
+STREAMED = 4  # kind of nml_debug_launch_count
+
+
+def streamed():
+    return _lib.load().nml_debug_launch_count(STREAMED)
+
+
+def conv(x, w, g):
+    f = torch.nn.functional.conv_transpose2d if g.transposed else torch.nn.functional.conv2d
+    return f(x, w, stride=g.stride, padding=g.padding)
+
+
+# one channel block and a broken one, taps in whole stages and not (9 of 9, 25 and 49 of fewer, 4 a phase), one column tile of 16 ... 224 columns,
+# tiles hanging over the image, several tiles per CTA
+@pytest.mark.parametrize("n,c_in,hw,c_out,k,s,transposed", [
+    (9, 256, 32, 64, 3, 1, False), (9, 200, 31, 24, 5, 1, False), (87, 64, 31, 144, 3, 1, False), (4, 136, 48, 224, 3, 1, False), (40, 520, 16, 9, 3, 1, True),
+    (3, 512, 32, 64, 4, 2, True), (3, 256, 61, 40, 7, 1, False), (9, 640, 47, 16, 3, 1, False)])
+def test_fp16(n, c_in, hw, c_out, k, s, transposed):
+    gen = torch.Generator(device="cuda").manual_seed(c_in + c_out)
+    g = ConvGeometry(n, c_in, hw, hw, c_out, k, k, (s, s), (k // 2 if s == 1 else 1,) * 2, transposed=transposed)
+    x = torch.randn(g.act_shape("in", "nhwc"), device="cuda", generator=gen).half()
+    w = (torch.randn(g.weight_shape(), device="cuda", generator=gen) * 0.05).half()
+    b = torch.randn(c_out, device="cuda", generator=gen).half()
+    before = streamed()
+    y = ops.conv_forward(g, x, w, b, layout="nhwc", math="f16")
+    assert streamed() == before + 1
+    want = (conv(x.permute(0, 3, 1, 2).double(), w.double(), g) + b.double().view(-1, 1, 1)).permute(0, 2, 3, 1)
+    # one rounding to fp16 (two where a ragged row's bias is added to the rounded sum), fp32 sums well below it
+    bound = (want.abs() + b.double().abs() + want.abs().amax() / 64) * 2.0 ** -10
+    assert ((y.double() - want).abs() <= bound).all()
+    ops.device_status()
+
+
+@pytest.mark.parametrize("n,c_in,hw,c_out,k,s,transposed", [
+    (9, 128, 33, 32, 3, 1, False), (14, 3, 73, 100, 3, 1, False), (33, 70, 31, 64, 3, 1, False), (3, 128, 64, 24, 5, 1, False), (8, 232, 30, 24, 4, 2, True)])
+def test_split_of_fp32(n, c_in, hw, c_out, k, s, transposed):
+    """Forward, or for an image's few channels the input gradient."""
+    gen = torch.Generator(device="cuda").manual_seed(c_in + c_out)
+    g = ConvGeometry(n, c_in, hw, hw, c_out, k, k, (s, s), (k // 2 if s == 1 else 1,) * 2, transposed=transposed)
+    w = torch.randn(g.weight_shape(), device="cuda", generator=gen)
+    x = torch.randn(g.act_shape("in", "nchw"), device="cuda", generator=gen)
+    before = streamed()
+    if c_in > 3:
+        got, want = ops.conv_forward(g, x, w, math="3xtf32"), conv(x.double(), w.double(), g)
+    else:
+        dy = torch.randn(g.act_shape("out", "nchw"), device="cuda", generator=gen)
+        got = ops.conv_backward_data(g, dy, w, math="3xtf32")
+        want = torch.nn.functional.conv_transpose2d(dy.double(), w.double(), padding=k // 2)
+    assert streamed() == before + 1
+    assert_f32(got.cpu(), want.cpu(), "fp32")
+    again = ops.conv_forward(g, x, w, math="3xtf32") if c_in > 3 else ops.conv_backward_data(g, dy, w, math="3xtf32")
+    assert torch.equal(got, again)
+    ops.device_status()

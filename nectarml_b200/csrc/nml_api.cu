@@ -268,8 +268,8 @@ static int load_helper_kernels() {
         (const void*)pack_phase_weights_kernel<float, float>, (const void*)pack_phase_weights_kernel<float, __half>,
         (const void*)pack_phase_weights_kernel<__half, float>, (const void*)pack_phase_weights_kernel<__half, __half>,
         (const void*)to_float_kernel<__half>, (const void*)colsum_finish_kernel,
-        (const void*)add_masked_kernel, (const void*)repack_half_tile_kernel, (const void*)repack_half_rows_kernel, (const void*)wgrad_reduce_taps_kernel,
-        (const void*)wgrad_reduce_rows4_kernel, (const void*)wgrad_reduce_kernel, (const void*)wgrad_reduce_deep4_kernel,
+        (const void*)add_masked_kernel, (const void*)repack_half_tile_kernel, (const void*)repack_half_rows_kernel, (const void*)wgrad_reduce_taps_kernel<1>, (const void*)wgrad_reduce_taps_kernel<kReduceGroups>,
+        (const void*)wgrad_reduce_rows4_kernel, (const void*)wgrad_reduce_kernel<1>, (const void*)wgrad_reduce_kernel<4>, (const void*)wgrad_reduce_deep4_kernel,
     };
     for (const void* f : fns) {
         cudaFuncAttributes a;
@@ -1952,24 +1952,30 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     }
     if (staged) {
         const bool vec_ok = (reinterpret_cast<uintptr_t>(g.dw) & 15) == 0;
-        if (P.wpatch && vec_ok && dw_elems % 4 == 0 && split > 8) {
-            const size_t total4 = dw_elems / 4;
-            helper_launch(4 * kSms, wgrad_reduce_deep4_kernel, static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st, planes, g.dw, split, plane_elems, total4);
-        } else if (P.wpatch && vec_ok && dw_elems % 4 == 0) {
-            const int blocks = static_cast<int>(std::min<size_t>((dw_elems / 4 + 255) / 256, 148 * 8));
-            helper_launch(4 * kSms, wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, 1, static_cast<int>(dw_elems / 4), 0);
-        } else if (!P.wpatch && !P.kw_pack && T == 1 && vec_ok && g.patch_c % 4 == 0) {
-            const size_t total4 = dw_elems / 4;
+        // planes whose rows are float4s of dW's, in order: of the patch walk (laid out like dW) and of one tap
+        const bool rows4 = vec_ok && (P.wpatch ? dw_elems % 4 == 0 : !P.kw_pack && T == 1 && g.patch_c % 4 == 0);
+        const size_t total4 = dw_elems / 4;
+        const int row_len4 = P.wpatch ? static_cast<int>(total4) : g.patch_c / 4;
+        const size_t group_bytes = kReducePlain * 64 * (P.n_taps | 1) * sizeof(float);
+        // Many planes of a small gradient: several threads an element, or a few blocks walk the planes one load latency at a time.
+        if (rows4 && split > 8 && (P.wpatch || total4 <= 16384)) {
+            helper_launch(4 * kSms, wgrad_reduce_deep4_kernel, static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st, planes, g.dw, split, plane_elems, total4,
+                          row_len4, static_cast<size_t>(plane_rows));
+        } else if (rows4) {
             const int blocks = static_cast<int>(std::min<size_t>((total4 + 255) / 256, 148 * 16));
-            helper_launch(4 * kSms, wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, g.plain_c, g.patch_c / 4, plane_rows);
-        } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535 && kReducePlain * 64 * (P.n_taps | 1) * sizeof(float) <= 48 * 1024) {
-            helper_launch(4 * kSms, wgrad_reduce_taps_kernel, dim3(ceil_div(g.patch_c, 64), ceil_div(g.plain_c, kReducePlain)), 256,
-                         kReducePlain * 64 * (P.n_taps | 1) * sizeof(float), st, planes, g.dw, split, plane_elems, g.patch_c, g.plain_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
+            helper_launch(4 * kSms, wgrad_reduce_rows4_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, total4 / row_len4, row_len4, plane_rows);
+        } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535 && group_bytes <= 48 * 1024) {
+            const dim3 blocks(ceil_div(g.patch_c, 64), ceil_div(g.plain_c, kReducePlain));
+            const bool deep = split >= 4 * kReduceGroups && blocks.x * blocks.y <= kSms && kReduceGroups * group_bytes <= 48 * 1024;
+            helper_launch(4 * kSms, deep ? wgrad_reduce_taps_kernel<kReduceGroups> : wgrad_reduce_taps_kernel<1>, blocks, dim3(256, deep ? kReduceGroups : 1),
+                         (deep ? kReduceGroups : 1) * group_bytes, st, planes, g.dw, split, plane_elems, g.patch_c, g.plain_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
         } else {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
-            const int blocks = static_cast<int>(std::min<size_t>((dw_elems + 255) / 256, 148 * 16));
-            helper_launch(4 * kSms, wgrad_reduce_kernel, blocks, 256, 0, st, planes, g.dw, split, plane_elems, dw_elems, layout, g.patch_c, P.n_taps,
-                                                        P.kw_count, P.c_blocks, mi.kb, plane_rows);
+            const bool deep = split >= 16 && dw_elems <= 65536;
+            const int elems = deep ? 64 : 256;
+            const int blocks = static_cast<int>(std::min<size_t>((dw_elems + elems - 1) / elems, 148 * 16));
+            helper_launch(4 * kSms, deep ? wgrad_reduce_kernel<4> : wgrad_reduce_kernel<1>, blocks, dim3(elems, deep ? 4 : 1), 0, st, planes, g.dw, split, plane_elems,
+                          dw_elems, layout, g.patch_c, P.n_taps, P.kw_count, P.c_blocks, mi.kb, plane_rows);
         }
         ++g_launches;
         NML_CUDA(cudaGetLastError());

@@ -799,18 +799,19 @@ __global__ void __launch_bounds__(256) wgrad_reduce_rows4_kernel(const float* pl
     pdl_leave(role);
 }
 
-// The same for many planes over a small gradient (the patch walk cuts K into one slice per SM): a thread
-// per element would walk ~150 planes one load latency at a time.  blockDim = (32, 8): lane ty adds
+// The same for many planes: a thread per element would walk them one load latency at a time (the patch walk cuts K into one slice per
+// SM; 1x1 40 -> 16 of 8619 pixels, 135 slices, 27.5 us so and 11.2 with eight lanes).  blockDim = (32, 8): lane ty adds
 // planes ty, ty + 8, ... of its float4 in order, then the eight running sums are added in order -- a
-// fixed association, so still bitwise repeatable.  Planes are laid out like dW.
+// fixed association, so still bitwise repeatable.
 __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* planes, float* __restrict__ dw,
-                                                                 int split, size_t plane_elems, size_t total4, int role) {
+                                                                 int split, size_t plane_elems, size_t total4, int row_len4, size_t src_pitch, int role) {
     pdl_enter(role);
     __shared__ float4 part[8][32];
     const size_t i = blockIdx.x * 32ull + threadIdx.x;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < total4) {
-        const float4* src = reinterpret_cast<const float4*>(planes) + i;
+        const size_t r = i / row_len4;
+        const float4* src = reinterpret_cast<const float4*>(planes + r * src_pitch) + (i - r * row_len4);
         const size_t step = plane_elems / 4;
 #pragma unroll 4
         for (int z = threadIdx.y; z < split; z += 8) {
@@ -837,13 +838,16 @@ __global__ void __launch_bounds__(256) wgrad_reduce_deep4_kernel(const float* pl
 // run along the patch channels (float4), the tap-fastest order is made in shared memory, and 64 * taps consecutive floats
 // are written.  (A thread per element read with a stride of a whole tap row: 4x4 512->128 11 us.)  kPlain plain channels a
 // block, their loads in flight together, and 16-byte stores: 4x4 512 x 1024, one plane, 18.8 -> 14 us (bytes: 10 us).
-constexpr int kReducePlain = 2;
-__global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* planes, float* __restrict__ dw, int split,
+// kGroups groups of threads take every so many planes each, so that no thread of a small gradient walks dozens of them one load latency
+// at a time; their sums are added in order.
+constexpr int kReducePlain = 2, kReduceGroups = 4;
+template <int kGroups>
+__global__ void __launch_bounds__(256 * kGroups) wgrad_reduce_taps_kernel(const float* planes, float* __restrict__ dw, int split,
                                                                 size_t plane_elems, int c_patch, int c_plain, int n_taps, int c_blocks, int kb,
                                                                 int R, int role) {
     pdl_enter(role);
-    extern __shared__ float taps[];  // [kReducePlain][64][n_taps | 1]
-    const int pitch = n_taps | 1;
+    extern __shared__ float taps[];  // [kGroups][kReducePlain][64][n_taps | 1]
+    const int pitch = n_taps | 1, group = kGroups > 1 ? threadIdx.y : 0, group_floats = kReducePlain * 64 * pitch;
     const int plain0 = blockIdx.y * kReducePlain, n_plain = min(kReducePlain, c_plain - plain0);
     const int pc0 = blockIdx.x * 64;
     const int pc = pc0 + 4 * (threadIdx.x & 15);
@@ -854,9 +858,9 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* pla
             float4 a[kReducePlain];
 #pragma unroll
             for (int q = 0; q < kReducePlain; ++q)
-                if (q < n_plain) a[q] = load_global(reinterpret_cast<const float4*>(p + static_cast<size_t>(q) * R));
+                if (q < n_plain) a[q] = load_global(reinterpret_cast<const float4*>(p + group * plane_elems + static_cast<size_t>(q) * R));
 #pragma unroll 4
-            for (int z = 1; z < split; ++z) {
+            for (int z = group + kGroups; z < split; z += kGroups) {  // (no more groups than planes)
 #pragma unroll
                 for (int q = 0; q < kReducePlain; ++q)
                     if (q < n_plain) {
@@ -866,7 +870,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* pla
             }
 #pragma unroll
             for (int q = 0; q < kReducePlain; ++q) {
-                float* o = taps + (q * 64 + pc - pc0) * pitch + t;
+                float* o = taps + group * group_floats + (q * 64 + pc - pc0) * pitch + t;
                 if (q < n_plain) o[0] = a[q].x, o[pitch] = a[q].y, o[2 * pitch] = a[q].z, o[3 * pitch] = a[q].w;
             }
         }
@@ -877,12 +881,14 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* pla
     for (int q = 0; q < n_plain; ++q) {
         float* out = dw + (static_cast<size_t>(plain0 + q) * c_patch + pc0) * n_taps;
         const float* in = taps + q * 64 * pitch;
-        for (int i = threadIdx.x * 4; i < n; i += 1024) {
+        for (int i = (threadIdx.x + 256 * group) * 4; i < n; i += 1024 * kGroups) {
             int c = i / n_taps, t = i - c * n_taps;
             float v[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 v[k] = in[c * pitch + t];
+#pragma unroll
+                for (int g = 1; g < kGroups; ++g) v[k] += in[g * group_floats + c * pitch + t];
                 if (++t == n_taps) {
                     t = 0;
                     ++c;
@@ -899,16 +905,20 @@ __global__ void __launch_bounds__(256) wgrad_reduce_taps_kernel(const float* pla
     pdl_leave(role);
 }
 
-// General form, one thread per dW element.  layout 0: a plane is laid out like dW.  layout 1: a plane is
+// General form, kLanes threads per dW element.  layout 0: a plane is laid out like dW.  layout 1: a plane is
 // [plain channel][R rows of the tile walk] and dW element (plain, pc, t) sits at row
 // (t * c_blocks + pc / kb) * kb + pc % kb.  layout 2 (few-channel window walk): dW element
 // (plain, c, kh, kw) sits at row kh * kb + kw * 8 + c.
+// blockDim = (256 / kLanes, kLanes): lane ty adds planes ty, ty + kLanes, ... in order, then the sums are added in order.
+template <int kLanes>
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* planes, float* __restrict__ dw, int split,
                                                            size_t plane_elems, size_t total, int layout, int c_patch,
                                                            int n_taps, int kw_count, int c_blocks, int kb, int R, int role) {
     pdl_enter(role);
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    constexpr unsigned long long kElems = 256 / kLanes;
+    __shared__ float part[kLanes][kElems];
+    for (size_t i0 = blockIdx.x * kElems; i0 < total; i0 += gridDim.x * kElems) {
+        const size_t i = i0 + threadIdx.x;
         size_t src = i;
         if (layout == 1) {
             const int t = static_cast<int>(i % n_taps);
@@ -925,9 +935,21 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* planes, 
             const size_t plain = q / c_patch;
             src = plain * R + static_cast<size_t>(kh) * kb + kw * 8 + c;
         }
-        float a = load_global(planes + src);
-        for (int z = 1; z < split; ++z) a += load_global(planes + z * plane_elems + src);
-        dw[i] = a;
+        const int first = kLanes > 1 ? threadIdx.y : 0;  // (no more lanes than planes)
+        float a = 0.f;
+        if (i < total) {
+            a = load_global(planes + first * plane_elems + src);
+            for (int z = first + kLanes; z < split; z += kLanes) a += load_global(planes + z * plane_elems + src);
+        }
+        if (kLanes > 1) {
+            part[threadIdx.y][threadIdx.x] = a;
+            __syncthreads();
+            if (threadIdx.y == 0)
+#pragma unroll
+                for (int k = 1; k < kLanes; ++k) a += part[k][threadIdx.x];
+            __syncthreads();
+        }
+        if ((kLanes == 1 || threadIdx.y == 0) && i < total) dw[i] = a;
     }
     pdl_leave(role);
 }

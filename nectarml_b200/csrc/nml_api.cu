@@ -609,13 +609,14 @@ static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* 
         }
     }
     // A box at least 2^prefer_w_log2 pixels wide (whole 128-byte runs for pixel-major stores) is taken
-    // when it costs at most 15 % more tiles and no further round of tiles: 3x3 96 -> 96 at 56 x 56, batch 16, fp16 31.1 -> 27.6 us
+    // when it costs at most 15 % more tiles and no further round of them (or 3 % more rounds:
+    // fp32 1x1 16 -> 832 at 54 x 54, batch 40, boxes of eight pixels in 43 rounds 442 us, of 32 in 44 105 us): 3x3 96 -> 96 at 56 x 56, batch 16, fp16 31.1 -> 27.6 us
     // with 392 tiles instead of 448; 128 -> 128 at 28 x 28, batch 16, 112 tiles instead of 98 in one round, 17.1 -> 15.9.
     // 3xTF32 tiles are 128 columns wide: 256 -> 256 at 56 x 56, batch 8, 392 tiles instead of 448 154 -> 124 us.  Their narrow
     // boxes have to save a round of several, though: where all run at once nothing overlaps the drain (`split`; 128 -> 384 at
     // 28 x 28, batch 8, 49.1 us in two rounds of wide boxes, 54.2 in one of narrow ones).
     if (prefer_w_log2 > 0 && best_wide > 0 && best_wide * 100 <= best * 115 &&
-        (rounds(best_wide) <= rounds(best) || (split && rounds(best) == 1))) {
+        (rounds(best_wide) * 32 <= rounds(best) * 33 || (split && rounds(best) == 1))) {
         *wl = ww;
         *hl = wh;
         *nl = wn;
@@ -851,7 +852,8 @@ struct FpropLike {
     const void* a;
     int a_dtype, a_layout, batch, a_c, a_h, a_w;
     const void* w;
-    int w_dtype, d0, d1, kh, kw, k_is_dim0, w_direct;
+    int w_dtype, d0, d1, kh, kw, k_is_dim0;
+    int w_direct;  // 0: repacked; 1: read in place where that can be; 2: so if they start on 16 bytes (scratch for a copy is taken anyway)
     int gather;  // 0: output pixel o reads input o*s - p + k*d; 1: output pixel o gathers from (o + p - k*d)/s
     int s_h, s_w, p_h, p_w, d_h, d_w;
     void* out;
@@ -1034,6 +1036,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     const int align = 16 / mi.es;
     bool direct_w = !window && f.w_direct && T == 1 && mi.enc == ENC_F16 && f.w_dtype == NML_F16 &&
                     ((f.k_is_dim0 ? N : K) % align == 0);
+    if (direct_w && f.w_direct == 2) {
+        if (ws.dry || (reinterpret_cast<uintptr_t>(f.w) & 15) == 0) ws.take(static_cast<size_t>(N) * kp * mi.es);
+        else direct_w = false;
+    }
     const void* w_planes[2] = {f.w, nullptr};
     int b_mn_major = 0;
     if (window) {
@@ -2171,13 +2177,47 @@ static bool conv_out_size(const nml_conv_desc* d, int* ho, int* wo) {
     return *ho > 0 && *wo > 0;
 }
 
+struct Pointwise {  // a 1x1 convolution as a Linear layer: its weights may start anywhere, and its input gradient may have an addend (KParams::add)
+    const void *add, *add_mask;
+    float add_below;
+};
+static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, const void* in1, const void* bias, void* out, float* db, Bump& ws,
+                       cudaStream_t st, const Pointwise* conv = nullptr);
+
 static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const void* in1, const void* bias, void* out,
                      float* db, Bump& ws, cudaStream_t st, const void* add = nullptr, const void* add_mask = nullptr, float add_below = 0.f) {
     int ho, wo;
+    nml_conv_desc flattened;
     g_last_scratch_error[0] = 0;  // a workspace error reported from here on is not the static entry point's
     if (!conv_out_size(d, &ho, &wo)) return NML_ERR_INVALID;
     const bool tr = d->transposed != 0;
-    if (pass == NML_PASS_BACKWARD_WEIGHT) {
+    // 1x1 layers of unit stride without padding have no geometry.  fp16 rows of pixels are a Linear layer's: its rules, weights read in place,
+    // no tile hanging over an image.  Forward / input gradient, us: 448 -> 192 at 5 x 5,
+    // batch 14, 9.3 -> 6.3 (forward); 1024 -> 256 at 9 x 9, batch 24, 10.0 / 9.5 -> 8.4 / 6.6; 512 -> 2048 at 7 x 7, batch 64, 16.8 / 16.6 -> 12.4 / 13.9;
+    // 256 -> 64 at 56 x 56, batch 256, 80.7 / 96.4 -> 79.0 / 95.0.
+    const bool pointwise = d->kh == 1 && d->kw == 1 && d->stride_h == 1 && d->stride_w == 1 && d->pad_h == 0 && d->pad_w == 0 && !tr;
+    const bool weights = pass == NML_PASS_BACKWARD_WEIGHT;
+    const long long pixels = 1ll * d->batch * d->h * d->w;
+    if (pointwise && d->batch > 0 && d->h > 0 && d->w > 0 && pixels <= INT_MAX / 2 && d->in_layout == NML_NHWC && (weights || d->out_layout == NML_NHWC) &&
+        d->math == NML_MATH_F16 && d->in_dtype == NML_F16 && (weights || d->w_dtype == NML_F16)) {
+        nml_linear_desc l;
+        memset(&l, 0, sizeof(l));
+        l.rows = static_cast<int>(pixels); l.in_features = d->c_in; l.out_features = d->c_out;
+        l.in_dtype = d->in_dtype; l.out_dtype = d->out_dtype; l.w_dtype = d->w_dtype; l.math = d->math; l.round_out_f16 = d->round_out_f16;
+        const Pointwise conv = {add, add_mask, add_below};
+        return linear_pass(&l, pass, in0, in1, bias, out, db, ws, st, &conv);
+    }
+    // Other tensors become images of one row, so that channel-major stores run on over the ends of the rows (small images find better
+    // boxes in two dimensions: fp32 96 -> 384 at 14 x 14, batch 60, 20.0 us, flat 22.3).
+    if (pointwise && d->batch > 0 && d->h > 0 && d->w > 0 && 1ll * d->h * d->w <= INT_MAX / 2 && (weights || 1ll * d->h * d->w >= 512)) {
+        flattened = *d;
+        flattened.w *= d->h;
+        flattened.h = 1;
+        d = &flattened;
+        wo *= ho;
+        ho = 1;
+    }
+    if (weights) {
         // in0 = x, in1 = dy
         WgradLike g;
         memset(&g, 0, sizeof(g));
@@ -2234,7 +2274,7 @@ static int rows_for_tma(const void* p, int inner, int rows) {
 }
 
 static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, const void* in1, const void* bias,
-                       void* out, float* db, Bump& ws, cudaStream_t st) {
+                       void* out, float* db, Bump& ws, cudaStream_t st, const Pointwise* conv) {
     if (!d || d->rows <= 0 || d->in_features <= 0 || d->out_features <= 0) return NML_ERR_INVALID;
     g_last_scratch_error[0] = 0;
     const int operands = d->math == NML_MATH_3XTF32 ? NML_F32 : d->math == NML_MATH_F16 ? NML_F16 : -1;
@@ -2290,7 +2330,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
             in_place = pass == NML_PASS_FORWARD && I <= 128 && 1ll * ceil_div(O, kTileM) * ceil_div(R, 64) <= 2 * planning_sms() && !g_dbg_short_a_box;
             if (in_place && !ws.dry && I % 8 == 0 && ((reinterpret_cast<uintptr_t>(in0) | reinterpret_cast<uintptr_t>(in1)) & 15) != 0) {
                 int rc = rows_for_tma(in0, I, R);
-                if (!rc) rc = rows_for_tma(in1, I, O);
+                if (!rc && !conv) rc = rows_for_tma(in1, I, O);
                 if (rc) return rc;
             }
         }
@@ -2335,7 +2375,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     f.a_c = forward ? d->in_features : d->out_features;
     f.w = in1; f.w_dtype = d->w_dtype; f.d0 = d->out_features; f.d1 = d->in_features; f.kh = f.kw = 1;
     f.k_is_dim0 = forward ? 0 : 1;
-    f.w_direct = 1;
+    f.w_direct = conv ? 2 : 1;
     // Input gradient: W [out][in] read in place is an MN-major B operand.  Where its rows are no whole groups of 64 it takes a load per
     // group and excludes CTA pairs, and a transposed fp16 copy W^T [in][out] (one coalesced pass over the weights, counted in the
     // pass's duration) pays from 2.2e9 products on, with 128 outputs (two K slices) and more: 12000 x 520 -> 2048 55.6 -> 36.4 us, 8192 x 328
@@ -2354,7 +2394,11 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     // of outputs, such a layer has its copy (and a workspace query, which sees no pointer, counts it); elsewhere it is refused.
     const bool any_start = d->rows >= 8192 && d->out_features % 64 == 0;
     const bool starts = (reinterpret_cast<uintptr_t>(in1) & 15) == 0;
-    if (!forward && d->math == NML_MATH_F16 && d->w_dtype == NML_F16 && d->in_features % 8 == 0 && d->out_features % 8 == 0 &&
+    if (conv && !forward && (pays || conv->add)) {
+        f.w_direct = 0;  // (repacked: that is the same copy)
+        f.add = conv->add; f.add_mask = conv->add_mask; f.add_below = conv->add_below;
+    } else
+    if (!forward && !conv && d->math == NML_MATH_F16 && d->w_dtype == NML_F16 && d->in_features % 8 == 0 && d->out_features % 8 == 0 &&
         (ws.dry ? pays || any_start : starts ? pays : any_start) && tune().wtrans) {
         __half* wt = static_cast<__half*>(ws.take(static_cast<size_t>(d->in_features) * d->out_features * sizeof(__half)));
         if (!ws.dry) {

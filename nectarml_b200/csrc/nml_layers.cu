@@ -171,23 +171,22 @@ __device__ __forceinline__ void bn_store_partial(float (*sm)[17], const float (&
         sm[threadIdx.x][8 + j] = b[j];
     }
     __syncthreads();
-    if (threadIdx.x < cpr) {  // fixed order over the block's row lanes
-        float* out = partial + static_cast<size_t>(blockIdx.x) * 2 * C;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float sa = 0.f, sb = 0.f;
-            for (int r = 0; r < rpb; ++r) {
-                sa += sm[r * cpr + threadIdx.x][j];
-                sb += sm[r * cpr + threadIdx.x][8 + j];
-            }
-            out[threadIdx.x * 8 + j] = sa;
-            out[C + threadIdx.x * 8 + j] = sb;
-        }
+    // fixed order over the block's row lanes, a thread to a sum (in the threads of the first row alone, sixteen sums each: 12544 x 1024 forward
+    // 28.8 us instead of 25.4, 262144 x 64 31.1 / 29.0, backward 41.0 / 38.9)
+    float* out = partial + static_cast<size_t>(blockIdx.x) * 2 * C;
+    for (int o = threadIdx.x; o < 16 * cpr; o += blockDim.x) {
+        const int col = o >> 4, j = o & 15;
+        float s = 0.f;
+#pragma unroll 4
+        for (int r = 0; r < rpb; ++r) s += sm[r * cpr + col][j];
+        out[(j < 8 ? 0 : C - 8) + col * 8 + j] = s;
     }
 }
 
 // Forward statistics: a = sum x, b = sum x^2; four rows in flight per thread.
-__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __restrict__ partial, size_t M, int C) {
+// `shares`: a block's rows follow one another, which HBM likes better than rows of all blocks in turn (802816 x 256, 411 MB, 85.8 -> 76.5 us;
+// the passes of two tensors are faster in turn, and so are tensors that L2 holds).
+__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __restrict__ partial, size_t M, int C, int shares) {
     pdl_enter();
     __shared__ float sm[256][17];
     const int cpr = C >> 3;
@@ -205,9 +204,10 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __
             b[j] += xf[j] * xf[j];
         }
     };
-    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
-    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
-    for (; row + 3 * stride < M; row += 4 * stride) {
+    const size_t share = shares ? (M + gridDim.x - 1) / gridDim.x : rpb, last = shares ? min(M, (blockIdx.x + 1) * share) : M;
+    const size_t stride = shares ? rpb : static_cast<size_t>(gridDim.x) * rpb;
+    size_t row = blockIdx.x * share + rsub;
+    for (; row + 3 * stride < last; row += 4 * stride) {
         const uint4 x0 = load_global(x + row * cpr + col), x1 = load_global(x + (row + stride) * cpr + col);
         const uint4 x2 = load_global(x + (row + 2 * stride) * cpr + col), x3 = load_global(x + (row + 3 * stride) * cpr + col);
         add(x0);
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __
         add(x2);
         add(x3);
     }
-    for (; row < M; row += stride) add(load_global(x + row * cpr + col));
+    for (; row < last; row += stride) add(load_global(x + row * cpr + col));
     bn_store_partial(sm, a, b, cpr, rpb, C, partial);
 }
 
@@ -998,7 +998,7 @@ int nml_bn_forward_masked(const void* x, long long rows, int channels, const flo
     int threads;
     const int P = bn_grid(rows, channels, &threads);
     float* partial = static_cast<float*>(workspace);
-    launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels);
+    launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels, M * channels >= (1u << 25) ? 1 : 0);  // (64 MB)
     launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
            nullptr, nullptr, mean, rstd);
     // (overlapping, whatever its grid: the second stage in front of it leaves every SM room for four of its blocks)

@@ -184,9 +184,9 @@ __device__ __forceinline__ void bn_store_partial(float (*sm)[17], const float (&
 }
 
 // Forward statistics: a = sum x, b = sum x^2; four rows in flight per thread.
-// `shares`: a block's rows follow one another, which HBM likes better than rows of all blocks in turn (802816 x 256, 411 MB, 85.8 -> 76.5 us;
-// the passes of two tensors are faster in turn, and so are tensors that L2 holds).
-__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __restrict__ partial, size_t M, int C, int shares) {
+// (Blocks whose rows follow one another read a tensor of 411 MB in 74 us instead of 83, but sum it in another order: a mean that rounds the
+// other way flips single ReLUs behind it, which is not worth half a percent of a block's step.)
+__global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __restrict__ partial, size_t M, int C) {
     pdl_enter();
     __shared__ float sm[256][17];
     const int cpr = C >> 3;
@@ -204,10 +204,9 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __
             b[j] += xf[j] * xf[j];
         }
     };
-    const size_t share = shares ? (M + gridDim.x - 1) / gridDim.x : rpb, last = shares ? min(M, (blockIdx.x + 1) * share) : M;
-    const size_t stride = shares ? rpb : static_cast<size_t>(gridDim.x) * rpb;
-    size_t row = blockIdx.x * share + rsub;
-    for (; row + 3 * stride < last; row += 4 * stride) {
+    const size_t stride = static_cast<size_t>(gridDim.x) * rpb;
+    size_t row = static_cast<size_t>(blockIdx.x) * rpb + rsub;
+    for (; row + 3 * stride < M; row += 4 * stride) {
         const uint4 x0 = load_global(x + row * cpr + col), x1 = load_global(x + (row + stride) * cpr + col);
         const uint4 x2 = load_global(x + (row + 2 * stride) * cpr + col), x3 = load_global(x + (row + 3 * stride) * cpr + col);
         add(x0);
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(256) bn_stats_kernel(const uint4* x, float* __
         add(x2);
         add(x3);
     }
-    for (; row < last; row += stride) add(load_global(x + row * cpr + col));
+    for (; row < M; row += stride) add(load_global(x + row * cpr + col));
     bn_store_partial(sm, a, b, cpr, rpb, C, partial);
 }
 
@@ -998,7 +997,7 @@ int nml_bn_forward_masked(const void* x, long long rows, int channels, const flo
     int threads;
     const int P = bn_grid(rows, channels, &threads);
     float* partial = static_cast<float*>(workspace);
-    launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels, M * channels >= (1u << 25) ? 1 : 0);  // (64 MB)
+    launch(bn_stats_kernel, P, threads, 0, st, xv, partial, M, channels);
     launch(bn_finish_kernel, channels / 8, dim3(8, 128), 0, st, partial, P, channels, 0, 1.0 / static_cast<double>(rows), eps,
            nullptr, nullptr, mean, rstd);
     // (overlapping, whatever its grid: the second stage in front of it leaves every SM room for four of its blocks)

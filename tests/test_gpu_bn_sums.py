@@ -1,5 +1,4 @@
-"""Sums of the normalisation's passes: blocks whose rows follow one another (tensors of 64 MB and more) and not, blocks of one row of channels and
-of many, rows that do not share out evenly."""
+"""Sums of the normalisation's passes: blocks of one row of channels and of many, rows that do not share out evenly."""
 import pytest
 import torch
 

@@ -1283,11 +1283,12 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         // fast or faster by boxes: 3x3 128 -> 128 at 64 x 64, batch 64, 72 us, 73 so), which wait for their operands.  A patch is read once for all
         // taps, but its tiles are 8 x 16 pixels of one image; so by rounds of tiles and the measured ratio of a slice's time, which falls with the
         // taps that share a patch.  By boxes / so, us: fp16 3x3 256 -> 64 at 32 x 32, batch 64, 39.2 / 32.7; 256 -> 192 at 64 x 64 222 / 179; 64 -> 144
-        // at 31 x 31, batch 87, 28.5 / 23.1; 5x5 192 -> 24 at 99 x 99, batch 4, 61.0 / 40.7; transposed 4x4 512 -> 64 at 64 x 64, batch 16, 114 / 102; fp32
+        // at 31 x 31, batch 87, 28.5 / 23.1; 5x5 192 -> 24 at 99 x 99, batch 4, 61.0 / 40.7; fp32
         // 3x3 128 -> 32 at 64 x 64, batch 16, 88.8 / 75.4; input gradient of 3 -> 234 at 145 x 145, batch 14, 966 / 766.  One tap a phase gains nothing
-        // (2x2 s2 transposed 960 -> 40 149 / 182).  Of 90 random passes 24 take it, with 0.85 of the time in the mean.
+        // (2x2 s2 transposed 960 -> 40 149 / 182); the four of a 4x4 s2 transposed layer a tenth in fp16 (512 -> 64 114 / 102), which is left: their sums
+        // then keep the order of boxes, and an image net's activations do not flip by rounding.  Of 90 random passes 24 take it, with 0.85 of the time in the mean.
         if (!P.patch && can_patch && patch_mode && taps_max >= 2 && !b_mn_major && !window && !f.w_batched && !f.shuf_sh && !f.add && !can_split &&
-            (P.planes == 2 ? N <= 64 : P.kind == KIND_F16 && (N <= 64 || (N > 128 && N <= 224)))) {
+            (P.planes == 2 ? N <= 64 : P.kind == KIND_F16 && taps_max >= 6 && (N <= 64 || (N > 128 && N <= 224)))) {
             const int bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024)), sms = limited(ds->sms);
             const double slice = (P.planes == 2 ? (N <= 32 ? 0.83 : 0.92) : N <= 32 ? 0.75 : N <= 64 ? 0.86 : 0.82) * (taps_max >= 12 ? 0.85 : 1.0);
             long long patches = 0, boxes = 0;

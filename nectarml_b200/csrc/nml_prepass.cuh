@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(256) repack_weight_window_kernel(const TIn* w,
 }
 
 // Partial sums of a K-split forward walk, `planes` fp32 planes of [pixels][C] (one per K slice) -> the
-// output tensor: the planes are added in a fixed order (so the result is bitwise repeatable), then bias,
+// output tensor: the planes are added in slice order (so the result is bitwise repeatable), then bias,
 // optional rounding through fp16, cast, and the caller's layout (nchw: out[n][c][pixel of the image]).
 // Row-major outputs whose channel count is a multiple of 4 take four values per thread (`vec`).
 __device__ __forceinline__ float4 finish4(float4 v, bool has_bias, const float4& b, int round_f16) {
@@ -729,59 +729,60 @@ __global__ void __launch_bounds__(256) finish_rows_kernel(const float* acc, int 
 }
 
 // The same for many planes of few elements, which a thread would walk one load latency at a time (fp32 4x4 s2 512 -> 64 at 4 x 4, batch 3,
-// forward 48.1 -> 14.0 us; linear 22 x 5248 -> 96 20.9 -> 12.2): blockDim = (32, 8), lane ty adds planes ty, ty + 8, ... in order, then the
-// eight sums are added in order.
-constexpr int kFinishLanes = 8;
+// forward 48.1 -> 16 us; linear 22 x 5248 -> 96 21 -> 13): blockDim = (32, 8), the lanes ty fetch 32 planes at a time into shared memory, where a
+// thread per value adds them in the planes' order: results are the same bits.  (Summed by lane instead, a value that rounds the other way in
+// an early layer of a net flips activations behind it.)
+constexpr int kFinishLanes = 8, kFinishChunk = 32;
 template <typename TOut>
 __global__ void __launch_bounds__(256) finish_rows_deep_kernel(const float* acc, int planes, const float* bias,
                                                                TOut* __restrict__ out, size_t pixels, int C, int hw, int nchw,
                                                                int round_f16, int vec, int role) {
     pdl_enter(role);
-    __shared__ float4 part[kFinishLanes][32];
+    __shared__ float part[kFinishChunk][128];  // [plane][value of the block: 32 vectors of four, or 32 values]
     const size_t total = pixels * C, items = vec ? total / 4 : total;
-    const uint32_t per_pixel = static_cast<uint32_t>(vec ? C / 4 : C);
+    const int t = threadIdx.y * 32 + threadIdx.x, values = vec ? 128 : 32;
     for (size_t i0 = blockIdx.x * 32ull; i0 < items; i0 += gridDim.x * 32ull) {
         const size_t i = i0 + threadIdx.x;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < items) {
-#pragma unroll 4
-            for (int z = threadIdx.y; z < planes; z += kFinishLanes) {
-                const size_t at = static_cast<size_t>(z) * items + i;
-                const float4 b = vec ? load_global(reinterpret_cast<const float4*>(acc) + at) : make_float4(load_global(acc + at), 0.f, 0.f, 0.f);
-                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-            }
-        }
-        part[threadIdx.y][threadIdx.x] = v;
-        __syncthreads();
-        if (threadIdx.y == 0 && i < items) {
+        float v = 0.f;
+        for (int z0 = 0; z0 < planes; z0 += kFinishChunk) {
+            float4 b[kFinishChunk / kFinishLanes];
 #pragma unroll
-            for (int k = 1; k < kFinishLanes; ++k) {
-                const float4 b = part[k][threadIdx.x];
-                v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-            }
-            const size_t p = i / per_pixel;
-            const int c = static_cast<int>(i - p * per_pixel) * (vec ? 4 : 1);
-            float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (bias != nullptr) bv = vec ? make_float4(load_global(bias + c), load_global(bias + c + 1), load_global(bias + c + 2), load_global(bias + c + 3))
-                                          : make_float4(load_global(bias + c), 0.f, 0.f, 0.f);
-            v = finish4(v, bias != nullptr, bv, round_f16);
-            if (!vec) {
-                size_t o = i;
-                if (nchw) {
-                    const size_t n = p / hw;
-                    o = (n * C + c) * hw + (p - n * hw);
+            for (int k = 0; k < kFinishChunk / kFinishLanes; ++k) {
+                const int z = z0 + threadIdx.y + kFinishLanes * k;
+                const size_t at = static_cast<size_t>(z) * items + i;
+                b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (z < planes && i < items) {
+                    if (vec) b[k] = load_global(reinterpret_cast<const float4*>(acc) + at);
+                    else b[k].x = load_global(acc + at);
                 }
-                out[o] = static_cast<TOut>(v.x);
-            } else if (sizeof(TOut) == 2) {
-                uint2 h;
-                *reinterpret_cast<__half2*>(&h.x) = __floats2half2_rn(v.x, v.y);
-                *reinterpret_cast<__half2*>(&h.y) = __floats2half2_rn(v.z, v.w);
-                reinterpret_cast<uint2*>(out)[i] = h;
-            } else {
-                reinterpret_cast<float4*>(out)[i] = v;
             }
+#pragma unroll
+            for (int k = 0; k < kFinishChunk / kFinishLanes; ++k) {
+                float* o = part[threadIdx.y + kFinishLanes * k];
+                if (vec) *reinterpret_cast<float4*>(o + 4 * threadIdx.x) = b[k];
+                else o[threadIdx.x] = b[k].x;
+            }
+            __syncthreads();
+            if (t < values) {
+                const int n = min(kFinishChunk, planes - z0);
+                if (z0 == 0) v = part[0][t];
+                for (int z = z0 == 0 ? 1 : 0; z < n; ++z) v += part[z][t];
+            }
+            __syncthreads();
         }
-        __syncthreads();
+        const size_t at = i0 * (vec ? 4 : 1) + t;  // this thread's value
+        if (t < values && at < total) {
+            const size_t p = at / C;
+            const int c = static_cast<int>(at - p * C);
+            if (bias != nullptr) v += load_global(bias + c);
+            if (round_f16) v = __half2float(__float2half_rn(v));
+            size_t o = at;
+            if (nchw) {
+                const size_t n = p / hw;
+                o = (n * C + c) * hw + (p - n * hw);
+            }
+            out[o] = static_cast<TOut>(v);
+        }
     }
     pdl_leave(role);
 }

@@ -20,11 +20,11 @@ def conv(x, w, g):
     return f(x, w, stride=g.stride, padding=g.padding)
 
 
-# one channel block and a broken one, taps in whole stages and not (9 of 9, 25 and 49 of fewer, 4 a phase), one column tile of 16 ... 224 columns,
+# one channel block and a broken one, taps in whole stages and not (9 of 9, 25 and 49 of fewer; 4 a phase in fp32), one column tile of 16 ... 224 columns,
 # tiles hanging over the image, several tiles per CTA
 @pytest.mark.parametrize("n,c_in,hw,c_out,k,s,transposed", [
     (9, 256, 32, 64, 3, 1, False), (9, 200, 31, 24, 5, 1, False), (87, 64, 31, 144, 3, 1, False), (4, 136, 48, 224, 3, 1, False), (40, 520, 16, 9, 3, 1, True),
-    (3, 512, 32, 64, 4, 2, True), (3, 256, 61, 40, 7, 1, False), (9, 640, 47, 16, 3, 1, False)])
+    (3, 256, 61, 40, 7, 1, False), (9, 640, 47, 16, 3, 1, False)])
 def test_fp16(n, c_in, hw, c_out, k, s, transposed):
     gen = torch.Generator(device="cuda").manual_seed(c_in + c_out)
     g = ConvGeometry(n, c_in, hw, hw, c_out, k, k, (s, s), (k // 2 if s == 1 else 1,) * 2, transposed=transposed)

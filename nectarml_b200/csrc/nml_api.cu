@@ -1613,7 +1613,11 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         const size_t items = vec ? total / 4 : total;
         // (from 64 x 2 x 2 pixels of 512 channels, 32768 items of 9 planes, a thread an item is as fast: 18.6 us, eight 19.5)
         const bool deep = P.fsplit >= kFinishLanes && items <= 16384;
-        const int blocks = static_cast<int>(std::min<size_t>(deep ? (items + 31) / 32 : (total + (vec ? 1023 : 255)) / (vec ? 1024 : 256), 148 * 8));
+        // (values one by one: a thread each while the grid still overlaps its predecessor; 3x3 s2 72 -> 77 at 58 x 58, batch 9, 34.1 us, a grid above
+        // that limit 38.3)
+        const size_t quarter = (total + 1023) / 1024;
+        const size_t wanted = deep ? (items + 31) / 32 : vec ? quarter : std::min<size_t>((total + 255) / 256, std::max<size_t>(4 * kSms, quarter));
+        const int blocks = static_cast<int>(std::min<size_t>(wanted, 148 * 8));
         const auto finish = [&](auto* kernel, auto* out, int round_f16) {
             helper_launch(4 * kSms, kernel, blocks, deep ? dim3(32, kFinishLanes) : dim3(256), 0, st, split_acc, P.fsplit, bias32, out, out_pixels, N,
                           f.out_h * f.out_w, nchw, round_f16, vec);

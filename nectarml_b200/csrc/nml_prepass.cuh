@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(256) finish_rows_deep_kernel(const float* acc,
                                                                TOut* __restrict__ out, size_t pixels, int C, int hw, int nchw,
                                                                int round_f16, int vec, int role) {
     pdl_enter(role);
-    __shared__ float part[kFinishChunk][128];  // [plane][value of the block: 32 vectors of four, or 32 values]
+    __shared__ __align__(16) float part[kFinishChunk][128];  // [plane][value of the block: 32 vectors of four, or 32 values]
     const size_t total = pixels * C, items = vec ? total / 4 : total;
     const int t = threadIdx.y * 32 + threadIdx.x, values = vec ? 128 : 32;
     for (size_t i0 = blockIdx.x * 32ull; i0 < items; i0 += gridDim.x * 32ull) {

@@ -2063,11 +2063,11 @@ static void fill_strided(GemmParams* P, const StridedProduct& g, const DeviceSta
     P->wait_limit_ns = g_dbg_wait_limit_ns;
 }
 
-static int run_strided(const StridedProduct& g, const StridedPlan& plan, int role, cudaStream_t st) {
+// ds: the state of the entry point (Bump::ds), nullptr for the device's own.
+static int run_strided(const StridedProduct& g, const StridedPlan& plan, DeviceState* ds, int role, cudaStream_t st) {
     const bool f32 = g.dtype == NML_F32;
     const int slice = f32 ? 32 : 64;
-    DeviceState* ds = nullptr;
-    int rc = device_state(&ds);
+    int rc = ds ? NML_OK : device_state(&ds);
     if (rc) return rc;
     GemmParams P;
     fill_strided(&P, g, ds, role);
@@ -2359,7 +2359,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
                 const int rc = sums.second_stage(st);
                 if (rc) return rc;
             }
-            const int rc = run_strided(g, plan, beside ? PDL_LEADER : PDL_NORMAL, st);
+            const int rc = run_strided(g, plan, ws.ds, beside ? PDL_LEADER : PDL_NORMAL, st);
             if (rc || !beside) return rc;
             t_role = PDL_SIBLING;
             sums.first_stage(st);
@@ -3032,7 +3032,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             const int rc = es == 2 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) != 0 ? rows_for_tma(A, K, M) : NML_OK;
             const StridedProduct g = in_place(A, B, C, n);
             if (way == STRIPS && !rc) ++g_launches_of[NML_DEBUG_TURNED];
-            return rc ? rc : way == STRIPS ? run_rows(g, nullptr) : run_strided(g, plan_strided(g, planning_sms()), PDL_NORMAL, nullptr);
+            return rc ? rc : way == STRIPS ? run_rows(g, nullptr) : run_strided(g, plan_strided(g, planning_sms()), bump.ds, PDL_NORMAL, nullptr);
         }
         FpropLike f;
         memset(&f, 0, sizeof(f));

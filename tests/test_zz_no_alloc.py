@@ -9,6 +9,9 @@ with the ordinary entry point's.  It also checks that a layer too large for the 
 is refused with a message instead of being run.  This file is named to be collected last.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -111,3 +114,48 @@ def test_layer_beyond_the_built_in_scratch_is_refused():
     assert st == 2
     msg = lib.nml_status_string(st).decode()
     assert "67108864" in msg and "scratch" in msg
+
+
+_CAPTURE = """
+import ctypes as C, torch
+from nectarml_b200 import _lib
+from nectarml_b200.ops import ConvGeometry
+lib, dev = _lib.load(), "cuda:0"
+
+def forward(g, x, w, out, stream):
+    d = g.desc(_lib.NML_F16, "nhwc", _lib.NML_F16, "nhwc", _lib.NML_F16, "f16", False)
+    st = lib.nml_conv_forward_static(C.byref(d), x.data_ptr(), w.data_ptr(), None, out.data_ptr(), stream.cuda_stream)
+    assert st == 0, lib.nml_status_string(st)
+
+first = ConvGeometry(1, 64, 8, 8, 32, 3, 3, (1, 1), (1, 1))  # the first call on the device, before the capture
+x = torch.zeros(first.act_shape("in", "nhwc"), device=dev).half()
+forward(first, x, torch.zeros(first.weight_shape(), device=dev).half(), torch.empty(first.act_shape("out", "nhwc"), device=dev).half(),
+        torch.cuda.current_stream())
+assert lib.nml_conv_forward_static(None, None, None, None, None, None) == 0
+handle = C.c_void_p()  # (a stream that waits for the legacy stream, as cudaStreamCreate makes it: nothing may go there during its capture)
+assert int(torch.cuda.cudart().cudaStreamCreate(C.addressof(handle))) == 0
+stream = torch.cuda.ExternalStream(handle.value)
+for c_in in (40, 64, 128, 256):  # (up to 128 channels: the kernel that reads its operands in place; above it the contraction kernel)
+    g = ConvGeometry(2, c_in, 9, 11, 48, 1, 1)
+    x = torch.randn(g.act_shape("in", "nhwc"), device=dev).half()
+    w = (torch.randn(g.weight_shape(), device=dev) * 0.1).half()
+    out = torch.full(g.act_shape("out", "nhwc"), float("nan"), device=dev).half()
+    torch.cuda.synchronize()
+    in_place, graph = lib.nml_debug_launch_count(2), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="global"):
+        forward(g, x, w, out, stream)
+    graph.replay()
+    assert lib.nml_conv_forward_static(None, None, None, None, None, None) == 0
+    want = x.double() @ w.view(48, c_in).double().t()
+    assert bool(((out.double() - want).abs() <= 1e-3 + 1e-2 * want.abs()).all()), c_in
+    assert lib.nml_debug_launch_count(2) - in_place == (c_in <= 128), c_in
+print("captured")
+"""
+
+
+def test_pointwise_layers_under_capture_after_the_first_static_call():
+    """In a process that has called no other entry point: what a 1x1 layer needs was set up by the first static call, so that a
+    capture may follow it, whichever kernel the layer runs in."""
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    res = subprocess.run([sys.executable, "-c", _CAPTURE], capture_output=True, text=True, timeout=300, env=env)
+    assert res.returncode == 0 and "captured" in res.stdout, res.stderr[-2000:]

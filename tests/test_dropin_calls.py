@@ -46,6 +46,37 @@ def test_integers_are_cut_to_the_width_of_the_parameter():
         _nectarml.tensor.matmul(-1, 1 << 70, (1 << 32, 4), (4, 4), F32)
 
 
+class _Stands:
+    def __init__(self, v):
+        self._as_parameter_ = v
+
+
+@pytest.mark.parametrize("wrap", [lambda t, v: v, lambda t, v: t(v), lambda t, v: _Stands(v), lambda t, v: _Stands(t(v)), lambda t, v: _Stands(_Stands(v))],
+                         ids=["int", "ctypes", "as_parameter", "as_parameter_ctypes", "as_parameter_twice"])
+def test_what_ctypes_takes_for_an_integer(wrap):
+    """The value arrives as well: two groups are refused in another way than one group of no channels."""
+    def call(groups):
+        names = list(inspect.signature(CONV.conv2d).parameters)
+        args = dict.fromkeys(names, wrap(C.c_int, 1))
+        args.update({n: wrap(C.c_size_t, 16) for n in names if n.endswith("_ptr") or n.endswith("_size")})
+        args.update(C_in=wrap(C.c_int, 0), groups=wrap(C.c_int, groups), dtype=F32, half_precision=False)
+        with pytest.raises(RuntimeError) as e:
+            CONV.conv2d(**args)
+        return str(e.value)
+    assert "invalid argument" in call(1) and call(1) != call(2)
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        _nectarml.tensor.matmul(wrap(C.c_size_t, 0), wrap(C.c_size_t, 0), (2, 0), (0, 2), F32)
+
+
+@pytest.mark.parametrize("bad", [_Stands("1"), _Stands(_Stands(None)), C.c_short(1), C.c_size_t(1)])
+def test_what_ctypes_refuses_for_an_int(bad):
+    names = list(inspect.signature(CONV.conv2d).parameters)
+    args = dict.fromkeys(names, 0)
+    args.update(B=bad, dtype=F32)
+    with pytest.raises(C.ArgumentError):
+        CONV.conv2d(**args)
+
+
 @pytest.mark.parametrize("a,b,error", [((2, 0), (0, 2), RuntimeError), ((2, 3), (4, 2), RuntimeError), ((2,), (2, 2), RuntimeError), (3, (2, 2), TypeError),
                                        (iter((2, 2)), (2, 2), TypeError), ((2, "x"), (2, 2), ValueError), ((2, None), (2, 2), TypeError)])
 def test_matmul_shapes(a, b, error):

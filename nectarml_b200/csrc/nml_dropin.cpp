@@ -8,6 +8,7 @@
 // ctypes type, objects that stand for one of these by `_as_parameter_`; anything else raises its ArgumentError.  The GIL is released for the call.
 #include <Python.h>
 
+#include <exception>
 #include <tuple>
 #include <type_traits>
 #include <utility>
@@ -87,15 +88,21 @@ struct Entry<kFn> {
     static PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t n) { return call(kFn, a, n, std::make_index_sequence<sizeof...(A) - 1>()); }
 };
 
+// (a copy of the sequence: an item's __int__ may change a list while it is read)
 bool shape(PyObject* o, std::vector<int>* dims) {
     if (PyObject_Size(o) < 0) return false;
-    PyObject* items = PySequence_Fast(o, "a shape is a sequence of integers");
+    PyObject* items = PySequence_Tuple(o);
     if (!items) return false;
-    const Py_ssize_t n = PySequence_Fast_GET_SIZE(items);
-    dims->resize(n);
+    const Py_ssize_t n = PyTuple_GET_SIZE(items);
     bool ok = true;
+    try {
+        dims->resize(n);
+    } catch (const std::exception&) {  // (none may leave a C entry)
+        PyErr_NoMemory();
+        ok = false;
+    }
     for (Py_ssize_t i = 0; ok && i < n; ++i) {
-        PyObject* v = PyNumber_Long(PySequence_Fast_GET_ITEM(items, i));
+        PyObject* v = PyNumber_Long(PyTuple_GET_ITEM(items, i));
         ok = v != nullptr;
         if (ok) (*dims)[i] = static_cast<int>(PyLong_AsUnsignedLongLongMask(v));
         Py_XDECREF(v);

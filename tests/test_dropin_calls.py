@@ -84,6 +84,18 @@ def test_matmul_shapes(a, b, error):
         _nectarml.tensor.matmul(0, 0, a, b, F32)
 
 
+def test_a_shape_that_changes_while_it_is_read():
+    """The sizes are those of the moment of the call."""
+    class Clears:
+        def __int__(self):
+            dims.clear()
+            return 1 << 31  # (as an int: negative, refused)
+    dims = [Clears()] + [2] * 1000
+    with pytest.raises(RuntimeError, match="invalid argument"):
+        _nectarml.tensor.matmul(0, 0, dims, (2, 2), F32)
+    assert dims == []
+
+
 def test_matmul_pointers():
     with pytest.raises(C.ArgumentError):
         _nectarml.tensor.matmul(None, 0, (2, 2), (2, 2), F32)

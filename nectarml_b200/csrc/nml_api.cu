@@ -1654,6 +1654,11 @@ struct WgradLike {
     float* colsum;
     int colsum_of_patch;
     int math;
+    // A 1x1 layer's images that are walked as one row: their own batch, height and width (0: as walked).  The tensor core truncates as it
+    // accumulates, so the error of a sum grows with its K blocks; fewer blocks, none of which hangs over an image, would be cut into fewer slices of
+    // the same length, or none.  So the slices are planned for the images' blocks, and each gets fewer: relative error against
+    // float64 of 126 -> 248 at 104 x 3, batch 2, 8.0e-7 in one slice of ten blocks, 1.2e-7 in the images' thirteen slices.
+    int plan_batch, plan_h, plan_w;
 };
 
 // Microseconds of a K block (64 pixels) of a double 256-column pair tile, and of its prologue and drain (256 KB of fp32 per SM,
@@ -1796,6 +1801,12 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     P.ktiles_w = ceil_div(g.plain_w, 1 << P.wb_log2);
     P.ktiles_h = ceil_div(g.plain_h, 1 << P.hb_log2);
     P.kblocks_total = P.ktiles_w * P.ktiles_h * ceil_div(g.batch, 1 << P.nb_log2);
+    int plan_blocks = P.kblocks_total;
+    if (g.plan_w) {
+        int wl, hl, nl;
+        choose_box(bits, g.plan_w, g.plan_h, g.plan_batch, 1, 1, &wl, &hl, &nl);
+        plan_blocks = std::max(plan_blocks, ceil_div(g.plan_w, 1 << wl) * ceil_div(g.plan_h, 1 << hl) * ceil_div(g.plan_batch, 1 << nl));
+    }
     // Tile width and K split so that the CTAs finish together.  Microseconds, measured over widths 64 / 128 / 256 and 1 ... 32
     // slices on 18 layers: a K block costs the same at 64 and 128 columns (0.32; operand feed, not MMAs), little more as a
     // 256-column CTA pair (0.36, 0.41 with the whole GPU busy); twice that for the 3xTF32 split's blocks of half the
@@ -1811,7 +1822,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         const double dw_us = 4.0 * g.plain_c * g.patch_c * T / 8e6;  // one pass over dW at 8 TB/s
         // at most 192 slices, as many as leave each at least one block (a count that the loop below does not pass over, so
         // that there is a plan whatever else is refused)
-        const int max_split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, std::min(P.kblocks_total, 192)));
+        const int max_split = ceil_div(plan_blocks, ceil_div(plan_blocks, std::min(plan_blocks, 192)));
         const bool may_pair = tune().pair;  // (read once: the loop runs up to 500 times per plan)
         double best = -1;
         for (int width = 256; width >= 64; width /= 2) {
@@ -1824,9 +1835,9 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             for (int sp = 1; sp <= max_split; ++sp) {
                 const long long tiles = 1ll * mt * nt * sp;
                 if (best >= 0 && sp > 1 && tiles > 3ll * units) break;
-                const int per_sp = ceil_div(P.kblocks_total, sp);
+                const int per_sp = ceil_div(plan_blocks, sp);
                 // every slice gets at least one K block: the next split that leaves each one block less
-                if (ceil_div(P.kblocks_total, per_sp) != sp) continue;
+                if (ceil_div(plan_blocks, per_sp) != sp) continue;
                 // the tensor core truncates as it accumulates: at most 4096 terms per sum of the 3xTF32 split, or as few
                 // as the most slices leave
                 if (P.planes == 2 && per_sp * mi.kb > 4096 && sp < max_split) continue;
@@ -1871,6 +1882,11 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
     if (P.wpatch) {  // one tile per CTA, no empty slice
         split = std::max(1, std::min(P.kblocks_total, sms / std::max(1, P.n_tiles)));
         split = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, split));
+    }
+    if (plan_blocks > P.kblocks_total) {  // as many slices of the blocks that there are, at least one block to each
+        const int slices = ceil_div(P.kblocks_total, ceil_div(P.kblocks_total, split));
+        launch_tiles = launch_tiles / split * slices;
+        split = slices;
     }
     P.split_k = split;
     P.num_tiles = P.wpatch ? P.n_tiles * split : static_cast<int>(launch_tiles);
@@ -2190,6 +2206,7 @@ static bool conv_out_size(const nml_conv_desc* d, int* ho, int* wo) {
 struct Pointwise {  // a 1x1 convolution as a Linear layer: its weights may start anywhere, and its input gradient may have an addend (KParams::add)
     const void *add, *add_mask;
     float add_below;
+    int batch, h, w;
 };
 static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, const void* in1, const void* bias, void* out, float* db, Bump& ws,
                        cudaStream_t st, const Pointwise* conv = nullptr);
@@ -2198,6 +2215,7 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
                      float* db, Bump& ws, cudaStream_t st, const void* add = nullptr, const void* add_mask = nullptr, float add_below = 0.f) {
     int ho, wo;
     nml_conv_desc flattened;
+    const nml_conv_desc* image = nullptr;  // of a layer that is walked as images of one row
     g_last_scratch_error[0] = 0;  // a workspace error reported from here on is not the static entry point's
     if (!conv_out_size(d, &ho, &wo)) return NML_ERR_INVALID;
     const bool tr = d->transposed != 0;
@@ -2214,13 +2232,14 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
         memset(&l, 0, sizeof(l));
         l.rows = static_cast<int>(pixels); l.in_features = d->c_in; l.out_features = d->c_out;
         l.in_dtype = d->in_dtype; l.out_dtype = d->out_dtype; l.w_dtype = d->w_dtype; l.math = d->math; l.round_out_f16 = d->round_out_f16;
-        const Pointwise conv = {add, add_mask, add_below};
+        const Pointwise conv = {add, add_mask, add_below, d->batch, d->h, d->w};
         return linear_pass(&l, pass, in0, in1, bias, out, db, ws, st, &conv);
     }
     // Other tensors become images of one row, so that channel-major stores run on over the ends of the rows (small images find better
     // boxes in two dimensions: fp32 96 -> 384 at 14 x 14, batch 60, 20.0 us, flat 22.3).
     if (pointwise && d->batch > 0 && d->h > 0 && d->w > 0 && 1ll * d->h * d->w <= INT_MAX / 2 && (weights || 1ll * d->h * d->w >= 512)) {
         flattened = *d;
+        image = d;
         flattened.w *= d->h;
         flattened.h = 1;
         d = &flattened;
@@ -2246,6 +2265,7 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
         g.dw = static_cast<float*>(out);
         g.colsum = db;
         g.math = d->math;
+        if (image) g.plan_batch = image->batch, g.plan_h = image->h, g.plan_w = image->w;
         return run_wgrad_like(g, ws, st);
     }
     FpropLike f;
@@ -2376,6 +2396,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
         g.dw = static_cast<float*>(out);
         g.colsum = db; g.colsum_of_patch = 0;
         g.math = d->math;
+        if (conv) g.plan_batch = conv->batch, g.plan_h = conv->h, g.plan_w = conv->w;
         return run_wgrad_like(g, ws, st);
     }
     FpropLike f;

@@ -59,3 +59,17 @@ def test_channel_major(n, c_in, h, w, c_out, dtype):
     assert_f32(dw.view(c_out, c_in).cpu(), torch.einsum("nop,nip->oi", dyd, xd).cpu(), "dw")
     assert_f32(db.cpu(), dyd.sum((0, 2)).cpu(), "db")
     ops.device_status()
+
+
+@pytest.mark.parametrize("n,c_in,h,w,c_out,layout", [(2, 126, 104, 3, 248, "nhwc"), (1, 6, 10, 33, 16, "nchw"), (3, 64, 26, 14, 96, "nchw"), (40, 48, 5, 5, 160, "nhwc")])
+def test_weight_gradients_keep_the_sums_of_their_images(n, c_in, h, w, c_out, layout):
+    """Pixels of all images in one row make fewer K blocks, which must not become longer sums: the tensor core truncates as it accumulates,
+    up to 2^-23 of the running sum per instruction of 16 products.  A block is four of them; here a slice has one or two blocks, whose
+    sums then grow to the result as the root of their number: at most 8 * 2^-23 / sqrt(slices), 3.2e-7 for the shortest."""
+    g = ConvGeometry(n, c_in, h, w, c_out, 1, 1)
+    x, _, _, dy = tensors(g, layout, torch.float16, n + h)
+    dw = ops.conv_backward_weight(g, x, dy, layout=layout, want_bias_grad=False)[0].double().view(c_out, c_in)
+    flat = (lambda t: t.double().flatten(0, 2)) if layout == "nhwc" else (lambda t: t.double().flatten(2).transpose(1, 2).flatten(0, 1))
+    want = flat(dy).t() @ flat(x)
+    assert float((dw - want).norm() / want.norm()) <= 3.2e-7
+    ops.device_status()

@@ -1268,6 +1268,35 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                         can_split ? std::min(z_cap, 8) : 1, patch_fits, P.out_f16 ? 2 : 4, P.out_mode != OUT_NCHW ? 0 : f.gather && f.s_w > 1 ? 1 : 5,
                         limited(ds->sms), &P.wb_log2, &P.hb_log2, &P.nb_log2);
     }
+    // Tile width: 256 columns run the tensor pipe best, but when that leaves SMs idle (few row tiles, narrow N) a narrower tile wins.
+    // Cost per column relative to a 256-wide tile, measured on B200: 128 -> 1.28, 64 -> 2.24; the makespan is rounds x width x cost.
+    struct Width {
+        int n_tiles = 0, bn = 0;
+        double cost = -1;
+    };
+    const auto tile_width = [&](long long m_tiles, int forced, bool by_tma) {
+        const int cand[4] = {256, 128, 64, forced};
+        const double cost[3] = {1.0, 1.28, 2.24};
+        Width best;
+        for (int i = 0; i < 4; ++i) {
+            if (forced ? i != 3 : i == 3) continue;
+            const int nt = ceil_div(N, cand[i]);
+            // (TMA stores take whole pieces of columns, and only a row's last one may be cut off: 354 x 512 -> 192 in two tiles of 96 columns
+            // by the plain epilogue 9.3 us, in three of 64 by TMA stores 6.5)
+            const int unit = b_mn_major ? 64 : forced == 16 ? 16 : nt > 1 && by_tma ? (P.out_f16 ? 64 : 32) : 32;
+            const int bn = static_cast<int>(round_up(ceil_div(N, nt), unit));
+            // (the split keeps two accumulators per tile; 256 columns would leave one buffer: 16384 x 1024 -> 1024 125 -> 150 us)
+            if (bn > 256 || (bn > 128 && P.planes == 2)) continue;
+            const double rounds = static_cast<double>(ceil_div(static_cast<int>(std::min<long long>(m_tiles * nt, 1 << 30)), limited(ds->sms)));
+            const double t = rounds * bn * (bn > 128 ? cost[0] : bn > 64 ? cost[1] : cost[2]);
+            if (best.cost < 0 || t < best.cost * 0.97) best = {nt, bn, t};  // prefer the wider tile unless the gain is clear
+        }
+        return best;
+    };
+    Width streamed;  // of a patch walk with streamed weights over more than 64 columns
+    const int out_es = P.out_f16 ? 2 : 4;
+    const bool rows_of_vectors = (static_cast<size_t>(N) * out_es) % 16 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0;
+    const int forced_width = P.planes == 2 ? std::min(tune().bn, 128) : tune().bn;
     {
         const int wq = P.phases[0].wq, hq = P.phases[0].hq;
         const double eff_patch = static_cast<double>(wq) * hq / (1.0 * round_up(wq, 8) * round_up(hq, 16));
@@ -1280,17 +1309,16 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             P.patch_bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024));
         }
         // The patch walk with streamed weights, where they do not stay: for tiles that do not pair up (pairs of 128 and 256 columns are as
-        // fast or faster by boxes: 3x3 128 -> 128 at 64 x 64, batch 64, 72 us, 73 so), which wait for their operands.  A patch is read once for all
-        // taps, but its tiles are 8 x 16 pixels of one image; so by rounds of tiles and the measured ratio of a slice's time, which falls with the
-        // taps that share a patch.  By boxes / so, us: fp16 3x3 256 -> 64 at 32 x 32, batch 64, 39.2 / 32.7; 256 -> 192 at 64 x 64 222 / 179; 64 -> 144
-        // at 31 x 31, batch 87, 28.5 / 23.1; 5x5 192 -> 24 at 99 x 99, batch 4, 61.0 / 40.7; fp32
-        // 3x3 128 -> 32 at 64 x 64, batch 16, 88.8 / 75.4; input gradient of 3 -> 234 at 145 x 145, batch 14, 966 / 766.  One tap a phase gains nothing
-        // (2x2 s2 transposed 960 -> 40 149 / 182); the four of a 4x4 s2 transposed layer a tenth in fp16 (512 -> 64 114 / 102), which is left: their sums
-        // then keep the order of boxes, and an image net's activations do not flip by rounding.  Of 90 random passes 24 take it, with 0.85 of the time in the mean.
+        // fast or faster by boxes), which wait for their operands.  A patch is read once for all taps, but its tiles are 8 x 16 pixels of one
+        // image; so by rounds of tiles and the measured ratio of a slice's time, which falls with the taps that share a patch.
+        // By boxes / so, us: fp16 3x3 256 -> 64 at 32 x 32, batch 64, 39.2 / 32.7; 256 -> 192 at 64 x 64 222 / 179; 5x5 192 -> 24 at 99 x 99,
+        // batch 4, 61.0 / 40.7; fp32 3x3 128 -> 32 at 64 x 64, batch 16, 88.8 / 75.4; 128 -> 128 at 64 x 64, batch 64, 72 / 73.
+        // One tap a phase gains nothing (2x2 s2 transposed 960 -> 40 149 / 182); the four of a 4x4 s2 transposed layer a tenth in fp16 (512 ->
+        // 64 114 / 102), which is left: their sums then keep the order of boxes, and an image net's activations do not flip by rounding.
         if (!P.patch && can_patch && patch_mode && taps_max >= 2 && !b_mn_major && !window && !f.w_batched && !f.shuf_sh && !f.add && !can_split &&
             (P.planes == 2 ? N <= 64 : P.kind == KIND_F16 && taps_max >= 6 && (N <= 64 || (N > 128 && N <= 224)))) {
             const int bytes = static_cast<int>(round_up(pw_ * ph_ * row_bytes, 1024)), sms = limited(ds->sms);
-            const double slice = (P.planes == 2 ? (N <= 32 ? 0.83 : 0.92) : N <= 32 ? 0.75 : N <= 64 ? 0.86 : 0.82) * (taps_max >= 12 ? 0.85 : 1.0);
+            const double slice = (P.planes == 2 ? (N <= 32 ? 0.83 : 0.92) : N <= 32 ? 0.75 : 0.86) * (taps_max >= 12 ? 0.85 : 1.0);
             long long patches = 0, boxes = 0;
             for (int p = 0; p < n_phases; ++p) {
                 const Phase& ph = P.phases[p];
@@ -1298,8 +1326,37 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                 boxes += 1ll * ceil_div(ph.wq, 1 << P.wb_log2) * ceil_div(ph.hq, 1 << P.hb_log2) * ceil_div(f.batch, 1 << P.nb_log2);
             }
             const auto rounds = [&](long long n) { return static_cast<double>((n + sms - 1) / sms); };
-            // (a small gain does not outlast the first patch of a single round: fp32 3x3 40 -> 40 at 52 x 52, batch 3, 17.1 us by boxes, 17.6 so)
-            if (rounds(patches) * slice <= rounds(boxes) * 0.95 && (slice < 0.9 || rounds(boxes) >= 2) && 2ll * P.planes * bytes <= 130 * 1024) {
+            bool pays;
+            if (N <= 64) {
+                // (a small gain does not outlast the first patch of a single round: fp32 3x3 40 -> 40 at 52 x 52, batch 3, 17.1 us by boxes, 17.6 so)
+                pays = rounds(patches) * slice <= rounds(boxes) * 0.95 && (slice < 0.9 || rounds(boxes) >= 2);
+            } else {
+                // More than 128 columns are one tile, two, or several of 64, of either walk; by estimated time, a slice's and a column's drain measured on
+                // 420 layers of 129 ... 224 channels (3x3 to 7x7; by boxes with their width / so: 5x5 29 -> 168 at 44 x 9, batch 3, 12.8 / 16.9 in one
+                // tile, stays; 40 -> 160 at 24 x 12, batch 8, 21.7 / 13.3 in three).  0.88 of the time by boxes alone in the mean.
+                const bool by_tma = rows_of_vectors && P.out_mode == OUT_NHWC;
+                const auto us = [&](long long m_tiles, const Width& w, double slice_us) {
+                    return rounds(m_tiles * w.n_tiles) * (c_blocks * taps_max * slice_us + 0.012 * w.bn);
+                };
+                const Width box = tile_width(boxes, forced_width, by_tma);
+                // (boxes of up to 40 channels, short rows, take longer: 3x3 24 -> 216 at 15 x 85, batch 40, 30.5 / 21.7)
+                double best = (f.a_c <= 40 ? 1.1 : 0.92) * us(boxes, box, box.bn <= 64 ? 0.27 : box.bn <= 128 ? 0.34 : 0.5);
+                for (int i = 0; i < 3 && !forced_width; ++i) {
+                    const int unit = i > 0 && by_tma && P.out_f16 ? 64 : 32, bn = i == 2 ? 64 : static_cast<int>(round_up(ceil_div(N, 1 + i), unit));
+                    const Width w = {ceil_div(N, bn), bn, 0.0};
+                    const double so = us(patches, w, bn <= 64 ? 0.17 : std::max(0.25, 0.002 * bn));
+                    if (so < best) {
+                        best = so;
+                        streamed = w;
+                    }
+                }
+                pays = streamed.bn > 0;
+            }
+            if (2ll * P.planes * bytes > 130 * 1024) {
+                pays = false;
+                streamed = Width();
+            }
+            if (pays) {
                 P.patch = 1;
                 P.patch_w = pw_;
                 P.patch_h = ph_;
@@ -1324,41 +1381,18 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     // TMA where there are many (from a round of tiles of eight columns on: transposed 5x5 s3 5 -> 8 at 128 x 24, batch 58, short 229 us, TMA
     // 162; linear 155624 x 16 -> 8 20.5 and 18.5; below it the short one saves 0.3 us: 1x1 s2 15 -> 4 at 24 x 64, batch 75, 10.4 and 11.9).
     // (Never phase-packed columns: they belong to several output pixels, and the packed image may be larger than the output.)
-    const int out_es = P.out_f16 ? 2 : 4;
     const bool short_rows = N <= 8 && (P.out_f16 || (P.patch && !P.b_taps) || out_pixels * N < 8ull * kTileM * kSms);
-    const bool rows_by_tma = P.out_mode == OUT_NHWC && !P.shuf_sh && tune().tmastore && !short_rows && (static_cast<size_t>(N) * out_es) % 16 == 0 &&
-                             (reinterpret_cast<uintptr_t>(f.out) & 15) == 0;
+    const bool rows_by_tma = P.out_mode == OUT_NHWC && !P.shuf_sh && tune().tmastore && !short_rows && rows_of_vectors;
     int z_plan = 1;  // K slices per tile
-    // Tile width: 256 columns run the tensor pipe best, but when that leaves SMs idle (few row tiles,
-    // narrow N) a narrower tile wins.  Cost per column relative to a 256-wide tile, measured on B200:
-    // 128 -> 1.28, 64 -> 2.24; the makespan is rounds x width x cost.
     {
         long long m_tiles_all = 0;
         for (int p = 0; p < n_phases; ++p)
             m_tiles_all += 1ll * ceil_div(P.phases[p].wq, 1 << P.wb_log2) * ceil_div(P.phases[p].hq, 1 << P.hb_log2) *
                            ceil_div(f.batch, 1 << P.nb_log2);
-        const int forced = P.patch && !P.b_taps ? (N <= 16 ? 16 : static_cast<int>(round_up(N, 32)))
-                                   : P.planes == 2 ? std::min(tune().bn, 128) : tune().bn;
-        const int cand[4] = {256, 128, 64, forced};
-        const double cost[3] = {1.0, 1.28, 2.24};
-        double best = -1;
-        for (int i = 0; i < 4; ++i) {
-            if (forced ? i != 3 : i == 3) continue;
-            int nt = ceil_div(N, cand[i]);
-            // (TMA stores take whole pieces of columns, and only a row's last one may be cut off: 354 x 512 -> 192 in two tiles of 96 columns
-            // by the plain epilogue 9.3 us, in three of 64 by TMA stores 6.5)
-            const int unit = b_mn_major ? 64 : forced == 16 ? 16 : nt > 1 && rows_by_tma ? std::max(32, 128 / out_es) : 32;
-            int bn = static_cast<int>(round_up(ceil_div(N, nt), unit));
-            // (the split keeps two accumulators per tile; 256 columns would leave one buffer: 16384 x 1024 -> 1024 125 -> 150 us)
-            if (bn > 256 || (bn > 128 && P.planes == 2)) continue;
-            double rounds = static_cast<double>(ceil_div(static_cast<int>(std::min<long long>(m_tiles_all * nt, 1 << 30)), limited(ds->sms)));
-            double t = rounds * bn * (bn > 128 ? cost[0] : bn > 64 ? cost[1] : cost[2]);
-            if (best < 0 || t < best * 0.97) {  // prefer the wider tile unless the gain is clear
-                best = t;
-                P.n_tiles = nt;
-                P.bn = bn;
-            }
-        }
+        const int forced = P.patch && !P.b_taps ? (N <= 16 ? 16 : static_cast<int>(round_up(N, 32))) : forced_width;
+        const Width width = streamed.bn ? streamed : tile_width(m_tiles_all, forced, rows_by_tma);
+        P.n_tiles = width.n_tiles;
+        P.bn = width.bn;
         // Tiles that leave half the SMs idle under a long K loop: tile width and number of K slices together, against
         // the plan above without a split.
         if (can_split && !P.patch) {
@@ -1373,7 +1407,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
             double best_us = cost_us(P.n_tiles, P.bn, 1);
             for (int i = 0; i < 4; ++i) {
                 if (forced ? i != 3 : i == 3) continue;
-                const int nt = ceil_div(N, cand[i]);
+                const int nt = ceil_div(N, i == 3 ? forced : 256 >> i);
                 const int bn = static_cast<int>(round_up(ceil_div(N, nt), b_mn_major ? 64 : 32));
                 if (m_tiles_all * nt * 2 > limited(ds->sms) || (bn > 128 && P.planes == 2)) continue;
                 const int z_max = std::min(z_cap, std::min(static_cast<int>(limited(ds->sms) / (m_tiles_all * nt)), k_min / (P.planes == 2 ? 2 : 4)));

@@ -1274,22 +1274,33 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         int n_tiles = 0, bn = 0;
         double cost = -1;
     };
+    const int k_loop = std::max(1, c_blocks * taps_max);
     const auto tile_width = [&](long long m_tiles, int forced, bool by_tma) {
         const int cand[4] = {256, 128, 64, forced};
         const double cost[3] = {1.0, 1.28, 2.24};
         Width best;
-        for (int i = 0; i < 4; ++i) {
-            if (forced ? i != 3 : i == 3) continue;
-            const int nt = ceil_div(N, cand[i]);
-            // (TMA stores take whole pieces of columns, and only a row's last one may be cut off: 354 x 512 -> 192 in two tiles of 96 columns
-            // by the plain epilogue 9.3 us, in three of 64 by TMA stores 6.5)
-            const int unit = b_mn_major ? 64 : forced == 16 ? 16 : nt > 1 && by_tma ? (P.out_f16 ? 64 : 32) : 32;
+        const auto consider = [&](int nt, int unit, double margin, double extra) {
             const int bn = static_cast<int>(round_up(ceil_div(N, nt), unit));
             // (the split keeps two accumulators per tile; 256 columns would leave one buffer: 16384 x 1024 -> 1024 125 -> 150 us)
-            if (bn > 256 || (bn > 128 && P.planes == 2)) continue;
+            if (bn > 256 || (bn > 128 && P.planes == 2)) return;
             const double rounds = static_cast<double>(ceil_div(static_cast<int>(std::min<long long>(m_tiles * nt, 1 << 30)), limited(ds->sms)));
-            const double t = rounds * bn * (bn > 128 ? cost[0] : bn > 64 ? cost[1] : cost[2]);
-            if (best.cost < 0 || t < best.cost * 0.97) best = {nt, bn, t};  // prefer the wider tile unless the gain is clear
+            const double t = rounds * bn * (bn > 128 ? cost[0] : bn > 64 ? cost[1] : cost[2]) + extra;
+            if (best.cost < 0 || t < best.cost * margin) best = {nt, bn, t};
+        };
+        // (TMA stores take whole pieces of columns, and only a row's last one may be cut off)
+        const bool pieces = by_tma && P.out_f16 && !b_mn_major && forced != 16;
+        for (int i = forced ? 3 : 0; i < (forced ? 4 : 3); ++i) {
+            const int nt = ceil_div(N, cand[i]);
+            consider(nt, b_mn_major || (pieces && nt > 1) ? 64 : forced == 16 ? 16 : 32, 0.97, 0.0);  // prefer the wider tile unless the gain is clear
+        }
+        // Tiles that are no whole pieces have the plain epilogue, about 2 us, which a long K loop outlasts (in the makespan's units, by a slice of 96
+        // columns of 0.33 us): 354 x 512 -> 192, eight slices, two tiles of 96 columns 9.3 us, three of 64 6.5; but 5x5 300 -> 152 at 8 x 9,
+        // batch 114, 125 slices, two of 96 43.7, one of 160 59.7, and 3x3 175 -> 144, 27 slices, 20.6 and 22.8.  Fewer tiles read the boxes of A less
+        // often, which counts where their rows are short: 5x5 88 -> 144 at 90 x 5, batch 9, 24.4 in two tiles of 96, 30.7 in three of 64.
+        const bool short_boxes = mi.kb == 64 && K % 64 != 0 && K % 64 <= 40;
+        for (int i = 0; pieces && !forced && i < 3; ++i) {
+            const int nt = ceil_div(N, cand[i]);
+            if (nt > 1) consider(nt, 32, short_boxes ? 1.0 : 0.945, 2.0 / 0.33 * 96 * cost[1] / k_loop);
         }
         return best;
     };
@@ -1336,7 +1347,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                 // tile, stays; 40 -> 160 at 24 x 12, batch 8, 21.7 / 13.3 in three).  0.88 of the time by boxes alone in the mean.
                 const bool by_tma = rows_of_vectors && P.out_mode == OUT_NHWC;
                 const auto us = [&](long long m_tiles, const Width& w, double slice_us) {
-                    return rounds(m_tiles * w.n_tiles) * (c_blocks * taps_max * slice_us + 0.012 * w.bn);
+                    return rounds(m_tiles * w.n_tiles) * (k_loop * slice_us + 0.012 * w.bn);
                 };
                 const Width box = tile_width(boxes, forced_width, by_tma);
                 // (boxes of up to 40 channels, short rows, take longer: 3x3 24 -> 216 at 15 x 85, batch 40, 30.5 / 21.7)
@@ -1404,7 +1415,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                 const double rounds = static_cast<double>((tiles * z + limited(ds->sms) - 1) / limited(ds->sms));
                 return rounds * (ceil_div(k_min, z) * slice_us(bn) * products + 2.5) + (z > 1 ? split_cost_us(z) : 0.0);
             };
-            double best_us = cost_us(P.n_tiles, P.bn, 1);
+            // (the estimate that the split was fitted against is that of tiles without regard to TMA stores: 7x7 56 -> 152 at 9 x 11, batch 2, whole
+            // 17.9 us, in slices 22.7)
+            const Width any = tile_width(m_tiles_all, forced, false);
+            double best_us = std::min(cost_us(P.n_tiles, P.bn, 1), cost_us(any.n_tiles, any.bn, 1));
             for (int i = 0; i < 4; ++i) {
                 if (forced ? i != 3 : i == 3) continue;
                 const int nt = ceil_div(N, i == 3 ? forced : 256 >> i);
@@ -2041,7 +2055,9 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
                          (deep ? kReduceGroups : 1) * group_bytes, st, planes, g.dw, split, plane_elems, g.patch_c, g.plain_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
         } else {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
-            const bool deep = split >= 16 && dw_elems <= 65536;
+            // (one tap: the planes are read in dW's order, so that a thread an element is as fast from the size on where a grid of four no longer starts
+            // beside its predecessor: 307 x 177 20.5 us so, 18.1 with a thread each, 238 x 200 28.1 and 24.9; 83 x 30 x 25 21.8 and 28.1)
+            const bool deep = split >= 16 && dw_elems <= (T > 1 ? 65536 : 64 * 4 * kSms);
             const int elems = deep ? 64 : 256;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + elems - 1) / elems, 148 * 16));
             helper_launch(4 * kSms, deep ? wgrad_reduce_kernel<4> : wgrad_reduce_kernel<1>, blocks, dim3(elems, deep ? 4 : 1), 0, st, planes, g.dw, split, plane_elems,

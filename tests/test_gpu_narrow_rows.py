@@ -84,3 +84,24 @@ def test_four_and_eight_fp32_columns(c_out, n, c_in, h, w, k, s, transposed, by_
     assert clean()
     ops.device_status()
     assert (launches[2] - launches[1]) - (launches[1] - launches[0]) == (0 if by_tma else 1)
+
+
+@pytest.mark.parametrize("n,c_in,h,w,c_out,k,whole_pieces", [(114, 300, 8, 9, 152, 5, False), (9, 88, 90, 5, 144, 5, False), (5, 64, 9, 14, 192, 3, True)])
+def test_long_k_loops_are_worth_tiles_that_are_no_whole_pieces(n, c_in, h, w, c_out, k, whole_pieces):
+    """Two tiles of 96 columns leave by the plain epilogue, with a widened copy of the bias (a launch), three of 64 by TMA."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    g = ConvGeometry(n, c_in, h, w, c_out, k, k, (1, 1), (k // 2, k // 2))
+    x = torch.randn(g.act_shape("in", "nhwc"), device="cuda", generator=gen).half()
+    wt = (torch.randn(g.weight_shape(), device="cuda", generator=gen) * 0.05).half()
+    b = torch.randn(c_out, device="cuda", generator=gen).half()
+    y, clean = guarded(*g.act_shape("out", "nhwc"))
+    launches = [ops.launch_count()]
+    for bias in (None, b):
+        ops.conv_forward(g, x, wt, bias, layout="nhwc", math="f16", out=y)
+        launches.append(ops.launch_count())
+    want = torch.nn.functional.conv2d(x.permute(0, 3, 1, 2).double(), wt.double(), b.double(), padding=k // 2).permute(0, 2, 3, 1)
+    # (the bias of the plain epilogue is added to the rounded sum)
+    assert ((y.double() - want).abs() <= (want.abs() + b.double().abs()) * 2.0 ** -10 + 2.0 ** -13 * want.abs().amax()).all()
+    assert clean()
+    ops.device_status()
+    assert (launches[2] - launches[1]) - (launches[1] - launches[0]) == (0 if whole_pieces else 1)

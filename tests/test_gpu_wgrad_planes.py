@@ -10,10 +10,11 @@ pytestmark = pytest.mark.gpu
 
 
 # rows of float4s (1x1), taps side by side (several taps, whole groups of four channels), the general form (broken ones, a transposed layer), few
-# and many planes, dW that does not start on 16 bytes
+# and many planes, one tap on both sides of 37888 elements, dW that does not start on 16 bytes
 @pytest.mark.parametrize("n,c_in,hw,c_out,k,s,transposed", [
     (51, 40, 13, 16, 1, 1, False), (6, 32, 83, 17, 1, 1, False), (3, 24, 9, 33, 1, 1, False), (66, 24, 11, 80, 3, 1, False), (40, 136, 20, 9, 3, 1, False),
-    (6, 182, 73, 33, 3, 1, True), (20, 25, 24, 30, 5, 1, False), (12, 102, 17, 33, 3, 2, False), (2, 30, 6, 31, 3, 1, False)])
+    (6, 182, 73, 33, 3, 1, True), (20, 25, 24, 30, 5, 1, False), (12, 102, 17, 33, 3, 2, False), (2, 30, 6, 31, 3, 1, False),
+    (10, 177, 27, 214, 1, 1, False), (10, 177, 27, 215, 1, 1, False)])
 @pytest.mark.parametrize("math,dtype", [("f16", torch.float16), ("3xtf32", torch.float32)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_sums_over_planes(n, c_in, hw, c_out, k, s, transposed, math, dtype, shift):

@@ -2290,8 +2290,16 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
         return linear_pass(&l, pass, in0, in1, bias, out, db, ws, st, &conv);
     }
     // Other tensors become images of one row, so that channel-major stores run on over the ends of the rows (small images find better
-    // boxes in two dimensions: fp32 96 -> 384 at 14 x 14, batch 60, 20.0 us, flat 22.3).
-    if (pointwise && d->batch > 0 && d->h > 0 && d->w > 0 && 1ll * d->h * d->w <= INT_MAX / 2 && (weights || 1ll * d->h * d->w >= 512)) {
+    // boxes in two dimensions: fp32 96 -> 384 at 14 x 14, batch 60, 20.0 us, flat 22.3).  Where the one row would be whole 16-byte vectors
+    // and the image's are not, the result would go to the TMA epilogue, which takes longer than the direct one for small results (24 -> 90
+    // at 22 x 174, batch 4, 10.5 us, flat 11.8; 272 -> 5 input gradient at 104 x 6, batch 3, 8.3 and 9.5; of 68 such layers below two million
+    // values 25 lost more than 5 %, three gained as much).
+    const auto flat_pays = [&] {
+        const long long es = d->out_dtype == NML_F16 ? 2 : 4, image_pixels = 1ll * d->h * d->w;
+        const bool turns_tma = d->out_layout == NML_NCHW && d->w * es % 16 != 0 && image_pixels * es % 16 == 0;
+        return image_pixels >= 512 && !(turns_tma && pixels * (pass == NML_PASS_FORWARD ? d->c_out : d->c_in) < 2000000);
+    };
+    if (pointwise && d->batch > 0 && d->h > 0 && d->w > 0 && 1ll * d->h * d->w <= INT_MAX / 2 && (weights || flat_pays())) {
         flattened = *d;
         image = d;
         flattened.w *= d->h;

@@ -40,8 +40,9 @@ def test_fp16_rows(n, c_in, h, w, c_out, shift):
     ops.device_status()
 
 
-# images below and above the size from which results are flat, rows of whole vectors and not
-@pytest.mark.parametrize("n,c_in,h,w,c_out", [(3, 40, 22, 23, 72), (2, 70, 23, 23, 33), (5, 16, 30, 31, 200), (2, 96, 54, 54, 40)])
+# images below and above the size from which results are flat, rows of whole vectors and not, results below and above the size from which one
+# row of whole vectors leaves by TMA
+@pytest.mark.parametrize("n,c_in,h,w,c_out", [(3, 40, 22, 23, 72), (2, 70, 23, 23, 33), (5, 16, 30, 31, 200), (2, 96, 54, 54, 40), (13, 16, 54, 54, 64)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 def test_channel_major(n, c_in, h, w, c_out, dtype):
     g, math = ConvGeometry(n, c_in, h, w, c_out, 1, 1), "3xtf32" if dtype == torch.float32 else "f16"

@@ -2487,7 +2487,15 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     // of outputs, such a layer has its copy (and a workspace query, which sees no pointer, counts it); elsewhere it is refused.
     const bool any_start = d->rows >= 8192 && d->out_features % 64 == 0;
     const bool starts = (reinterpret_cast<uintptr_t>(in1) & 15) == 0;
-    if (conv && !forward && (pays || conv->add)) {
+    // 1x1 convolutions have scratch for the copy anyway, and take it also where a last group of inputs that is far from whole meets many rows of tiles,
+    // by K slices (104 <- 24 at 62 x 29, batch 66, in place 19.4 us, copied 13.1; 72 <- 688, 42408 rows, 24.5 and 17.6; 8 <- 72, 44556 rows, 13.0
+    // and 8.5; but 56 <- 576, 12980 rows, 9.3 and 10.9, 456 <- 16, 16968 rows, 10.1 and 10.6), or a long K loop (208 <- 1920, 4 rows, 14.2 and 12.2).
+    const int last = d->in_features % 64;
+    const bool short_last = last != 0 && last <= (d->in_features < 64 ? 40 : 48);
+    const bool copied = conv && !forward && d->math == NML_MATH_F16 &&
+                        ((last != 0 && d->rows >= 120000) || (short_last && d->in_features < 256 && 1ll * d->rows * ceil_div(d->out_features, 64) >= 66000) ||
+                         (short_last && last <= 40 && d->in_features < 1000 && d->out_features >= 1300));
+    if (conv && !forward && (pays || copied || conv->add)) {
         f.w_direct = 0;  // (repacked: that is the same copy)
         f.add = conv->add; f.add_mask = conv->add_mask; f.add_below = conv->add_below;
     } else

@@ -74,3 +74,18 @@ def test_weight_gradients_keep_the_sums_of_their_images(n, c_in, h, w, c_out, la
     want = flat(dy).t() @ flat(x)
     assert float((dw - want).norm() / want.norm()) <= 3.2e-7
     ops.device_status()
+
+
+@pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(66, 104, 62, 29, 24, True), (60, 72, 31, 23, 200, True), (2, 208, 1, 2, 1920, True), (30, 56, 21, 20, 576, False),
+                                                    (8, 456, 46, 46, 16, False)])
+def test_input_gradients_of_broken_groups(n, c_in, h, w, c_out, copied):
+    """Weights whose last group of 64 inputs is far from whole are transposed first (a launch more) where many tiles or a long K loop read it."""
+    g = ConvGeometry(n, c_in, h, w, c_out, 1, 1)
+    _, wt, _, dy = tensors(g, "nhwc", torch.float16, c_in)
+    launches = ops.launch_count()
+    dx = ops.conv_backward_data(g, dy, wt, layout="nhwc")
+    launches = ops.launch_count() - launches
+    want = dy.double() @ wt.double().view(c_out, c_in)
+    assert ((dx.double() - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -13 * want.abs().amax()).all()
+    ops.device_status()
+    assert launches == 1 + int(copied)

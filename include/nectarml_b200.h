@@ -384,9 +384,9 @@ int nml_debug_stalled_linear_forward(const nml_linear_desc* d, const void* x, co
 int nml_debug_copy_to_host(void* host_dst, uintptr_t device_src, size_t bytes);
 
 /* Test support: which plans ran.  Contraction launches with double tiles, with the sum of nml_conv_backward_data_add in their
- * epilogue, products that read their operands in place, batched products turned round (the columns of the result along the lanes, by
- * strips of them read in place or as an image), patch walks with streamed weights; -1 for another kind. */
-enum { NML_DEBUG_DOUBLE_TILES = 0, NML_DEBUG_SUMS = 1, NML_DEBUG_IN_PLACE = 2, NML_DEBUG_TURNED = 3, NML_DEBUG_STREAMED = 4 };
+ * epilogue, products that read their operands in place, batched products turned round (as an image), patch walks with streamed weights,
+ * batched products by strips of columns read in place; -1 for another kind. */
+enum { NML_DEBUG_DOUBLE_TILES = 0, NML_DEBUG_SUMS = 1, NML_DEBUG_IN_PLACE = 2, NML_DEBUG_TURNED = 3, NML_DEBUG_STREAMED = 4, NML_DEBUG_STRIPS = 5 };
 long long nml_debug_launch_count(int kind);
 
 #ifdef __cplusplus

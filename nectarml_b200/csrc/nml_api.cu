@@ -173,7 +173,7 @@ struct DeviceState {
 static DeviceState g_dev[64];
 static std::mutex g_dev_mutex;   // guards g_dev, g_static, g_prof and g_ref_ws
 static std::atomic<long long> g_launches{0};
-static std::atomic<long long> g_launches_of[5];  // by kind, see nml_debug_launch_count
+static std::atomic<long long> g_launches_of[6];  // by kind, see nml_debug_launch_count
 // Where kernels report an abandoned wait.  The words live in the library image, so set-up needs no
 // allocation: their device addresses come from cudaGetSymbolAddress, once per device.
 static __device__ int g_status_word;
@@ -2761,7 +2761,7 @@ int nml_device_status(int* code) {
 
 long long nml_launch_count(void) { return g_launches.load() + nml_layers_launch_count(); }
 
-long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 5 ? g_launches_of[kind].load() : -1; }
+long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 6 ? g_launches_of[kind].load() : -1; }
 
 int nml_profile_begin(int max_records) {
     if (max_records <= 0 || max_records > 1 << 16) return NML_ERR_INVALID;
@@ -3122,7 +3122,7 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
             // (fp16 rows that TMA was to read and cannot stay refused)
             const int rc = es == 2 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) != 0 ? rows_for_tma(A, K, M) : NML_OK;
             const StridedProduct g = in_place(A, B, C, n);
-            if (way == STRIPS && !rc) ++g_launches_of[NML_DEBUG_TURNED];
+            if (way == STRIPS && !rc) ++g_launches_of[NML_DEBUG_STRIPS];
             return rc ? rc : way == STRIPS ? run_rows(g, nullptr) : run_strided(g, plan_strided(g, planning_sms()), bump.ds, PDL_NORMAL, nullptr);
         }
         FpropLike f;

@@ -8,7 +8,7 @@ from nectarml_b200 import _lib, _nectarml, ops
 import numpy as np
 
 pytestmark = pytest.mark.gpu
-IN_PLACE, TURNED = 2, 3  # kinds of nml_debug_launch_count
+IN_PLACE, TURNED, STRIPS = 2, 3, 5  # kinds of nml_debug_launch_count
 
 
 def product(a, b, batch, m, k, n):
@@ -28,9 +28,10 @@ def test_strips(batch, m, n, k, shift):
     a = make(batch * m * k) if k % 8 else torch.randn(batch * m * k, device="cuda", generator=gen).half()
     b = make(batch * k * n)
     lib = _lib.load()
-    before = lib.nml_debug_launch_count(TURNED), lib.nml_debug_launch_count(IN_PLACE), ops.launch_count()
+    counts = lambda: [lib.nml_debug_launch_count(kind) for kind in (STRIPS, TURNED, IN_PLACE)] + [ops.launch_count()]  # noqa: E731
+    before = counts()
     got = product(a, b, batch, m, k, n)
-    assert (lib.nml_debug_launch_count(TURNED), lib.nml_debug_launch_count(IN_PLACE), ops.launch_count()) == (before[0] + 1, before[1], before[2] + 1)
+    assert counts() == [before[0] + 1, before[1], before[2], before[3] + 1]
     ad, bd = a.double().view(batch, m, k), b.double().view(batch, k, n)
     want, terms = (ad @ bd).cpu(), (ad.abs() @ bd.abs()).cpu()
     # one rounding to fp16 (half an ulp, 2^-25 among the smallest), fp32 sums that lose at most 2^-22 of their terms' size a step of 16

@@ -206,7 +206,7 @@ def test_wide_bias_gradient_sums(fin, fout, sums):
     ops.device_status()
 
 
-DOUBLE_TILES, IN_PLACE, TURNED = 0, 2, 3  # kinds of nml_debug_launch_count
+DOUBLE_TILES, IN_PLACE, TURNED, STRIPS = 0, 2, 3, 5  # kinds of nml_debug_launch_count
 
 
 def launches_of(kind):
@@ -214,18 +214,21 @@ def launches_of(kind):
 
 
 # turned round, in fp16 and where the sizes say so in fp32: one row tile and several, columns of one pixel tile and of three, K of no whole
-# vector, entries of one column tile and of more
-@pytest.mark.parametrize("batch,m,k,n,fp32_too", [
-    (100, 129, 96, 65, False), (300, 127, 64, 63, False), (64, 333, 64, 333, False), (40, 257, 130, 257, True), (103, 3010, 2, 39, True), (64, 130, 72, 261, False)])
-def test_batched_matmul_turned_round(batch, m, k, n, fp32_too):
+# vector and of whole ones (read in place), entries of one column tile and of more, two K slices on both sides of eight groups of rows an SM; up
+# to there, and in fp16 with K of one slice, strips read in place take such products (`strips`)
+@pytest.mark.parametrize("batch,m,k,n,fp32_too,strips", [
+    (100, 129, 96, 65, False, True), (300, 127, 64, 63, False, True), (64, 333, 64, 333, False, True), (40, 257, 130, 257, True, False),
+    (103, 3010, 2, 39, True, False), (64, 130, 72, 261, False, True), (40, 257, 136, 257, False, False), (20, 333, 192, 333, False, False),
+    (74, 512, 96, 255, False, True), (74, 513, 96, 255, False, False), (148, 520, 72, 65, False, False)])
+def test_batched_matmul_turned_round(batch, m, k, n, fp32_too, strips):
     gen = torch.Generator(device="cuda").manual_seed(m + n)
     a, b = torch.randn(batch, m, k, device="cuda", generator=gen), torch.randn(batch, k, n, device="cuda", generator=gen)
     for dt, code in ((torch.float16, F16),) + (((torch.float32, F32),) if fp32_too else ()):
         ad, bd = a.to(dt), b.to(dt)
         torch.cuda.synchronize()
-        before = launches_of(TURNED)
+        before = launches_of(TURNED), launches_of(STRIPS)
         ptr = _nectarml.tensor.matmul(ad.data_ptr(), bd.data_ptr(), a.shape, b.shape, code)
-        assert launches_of(TURNED) - before == 1
+        assert (launches_of(TURNED) - before[0], launches_of(STRIPS) - before[1]) == ((0, 1) if strips and dt == torch.float16 else (1, 0))
         want = (ad.double() @ bd.double()).cpu().numpy()
         if dt == torch.float32:
             assert_f32(fetch(ptr, (batch, m, n)), want, "fp32")

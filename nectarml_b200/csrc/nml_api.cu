@@ -3097,11 +3097,16 @@ int nml_ref_matmul(uintptr_t a_ptr, uintptr_t b_ptr, const int* a_shape, int a_r
         if (g_sm_limit.load(std::memory_order_relaxed) == 0) {
             // Strips of 128 columns, read in place (gemm_rows_kernel), for K loops of one or two slices.  Stores of 64 bytes that start anywhere bound
             // large results whichever way they go, and two slices of both operands then cost more here than a conversion (28 x 726 x 96 x 844
-            // 24.6 us, turned 19.6; 128 x 511 x 128 x 513 57 and 51); very large ones are equal or up to 3 % slower (60 x 900 x 32 x 999 50.1 and 48.5).
-            const double groups = static_cast<double>(n) * ceil_div(N, kTileM) * ceil_div(M, kRowsBn) / sms;
-            if (es == 2 && K <= kRowsMaxK && N >= 32 && M >= 32 && groups <= (K <= 64 ? 32.0 : 8.0)) return STRIPS;
-            const StridedPlan plan = plan_strided(in_place(nullptr, nullptr, nullptr, n), sms);
+            // 24.6 us, turned 19.6; 128 x 511 x 128 x 513 57 and 51).  From eight groups of rows an SM on, by estimate against the conversions
+            // (110 x 855 x 20 x 324, whose strips make 1.1 waves, 39.7 and 32.6; 88 x 682 x 55 x 451 42.1 and 35.1; of 567 random products 5 are
+            // slower so by more than 5 %, without the estimate 12).
+            const StridedProduct g = in_place(nullptr, nullptr, nullptr, n);
             const double result = n * static_cast<double>(M) * N * 1e-6;
+            const double groups = static_cast<double>(n) * ceil_div(N, kTileM) * ceil_div(M, kRowsBn) / sms;
+            if (es == 2 && K <= kRowsMaxK && N >= 32 && M >= 32 && groups <= (K <= 64 ? 32.0 : 8.0) &&
+                (groups < 8.0 || 1.33 * plan_rows(g, sms).us + 0.32 * result - 0.7 <= 0.95 * std::min(rows_us, turned_us)))
+                return STRIPS;
+            const StridedPlan plan = plan_strided(g, sms);
             place_us = es == 4 ? 5.9 + 0.92 * plan.loop_us + 2.0 * (plan.waves - 1.0) + 0.32 * result
                                : 5.65 + 1.4 * plan.loop_us + 1.8 * (plan.waves - 1.0) + 0.28 * result;
         }

@@ -214,12 +214,13 @@ def launches_of(kind):
 
 
 # turned round, in fp16 and where the sizes say so in fp32: one row tile and several, columns of one pixel tile and of three, K of no whole
-# vector and of whole ones (read in place), entries of one column tile and of more, two K slices on both sides of eight groups of rows an SM; up
-# to there, and in fp16 with K of one slice, strips read in place take such products (`strips`)
+# vector and of whole ones (read in place), entries of one column tile and of more, two K slices on both sides of eight groups of rows an SM, one
+# slice above it with strips that make 2.2 waves and one; up to there, and above by estimate, strips read in place take fp16 products (`strips`)
 @pytest.mark.parametrize("batch,m,k,n,fp32_too,strips", [
     (100, 129, 96, 65, False, True), (300, 127, 64, 63, False, True), (64, 333, 64, 333, False, True), (40, 257, 130, 257, True, False),
     (103, 3010, 2, 39, True, False), (64, 130, 72, 261, False, True), (40, 257, 136, 257, False, False), (20, 333, 192, 333, False, False),
-    (74, 512, 96, 255, False, True), (74, 513, 96, 255, False, False), (148, 520, 72, 65, False, False)])
+    (74, 512, 96, 255, False, True), (74, 513, 96, 255, False, False), (148, 520, 72, 65, False, False),
+    (44, 80, 11, 1819, False, False), (74, 600, 48, 255, False, True)])
 def test_batched_matmul_turned_round(batch, m, k, n, fp32_too, strips):
     gen = torch.Generator(device="cuda").manual_seed(m + n)
     a, b = torch.randn(batch, m, k, device="cuda", generator=gen), torch.randn(batch, k, n, device="cuda", generator=gen)

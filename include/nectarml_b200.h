@@ -385,8 +385,12 @@ int nml_debug_copy_to_host(void* host_dst, uintptr_t device_src, size_t bytes);
 
 /* Test support: which plans ran.  Contraction launches with double tiles, with the sum of nml_conv_backward_data_add in their
  * epilogue, products that read their operands in place, batched products turned round (as an image), patch walks with streamed weights,
- * batched products by strips of columns read in place; -1 for another kind. */
-enum { NML_DEBUG_DOUBLE_TILES = 0, NML_DEBUG_SUMS = 1, NML_DEBUG_IN_PLACE = 2, NML_DEBUG_TURNED = 3, NML_DEBUG_STREAMED = 4, NML_DEBUG_STRIPS = 5 };
+ * batched products by strips of columns read in place, finishing passes of K splits and sums over the planes of a weight gradient with several
+ * threads to a result, passes of 1x1 convolutions as Linear layers; -1 for another kind. */
+enum {
+    NML_DEBUG_DOUBLE_TILES = 0, NML_DEBUG_SUMS = 1, NML_DEBUG_IN_PLACE = 2, NML_DEBUG_TURNED = 3, NML_DEBUG_STREAMED = 4, NML_DEBUG_STRIPS = 5,
+    NML_DEBUG_DEEP_FINISH = 6, NML_DEBUG_DEEP_SUMS = 7, NML_DEBUG_POINTWISE = 8
+};
 long long nml_debug_launch_count(int kind);
 
 #ifdef __cplusplus

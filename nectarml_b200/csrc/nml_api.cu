@@ -94,8 +94,9 @@ static EncodeTiledFn get_encode_fn() {
 //   NML_TUNE_WTRANS   0: Linear input-gradients never take a transposed copy of the weights
 //   NML_TUNE_PAIR128  0: CTA pairs only for 256-column tiles
 //   NML_TUNE_NARROW   0: few-channel layers always take eight channels per pixel
+//   NML_TUNE_DEEP     0: finishing passes of K splits always by a thread to a result
 struct Tune {
-    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow;
+    int stages, bn, ka, l2promo, pair, tmastore, epi8, patch, shuffle, fsplit, wpatch, wcoal, wtrans, pair128, narrow, deep;
 };
 static const Tune& tune() {
     static Tune t;
@@ -120,6 +121,7 @@ static const Tune& tune() {
         t.wtrans = env("NML_TUNE_WTRANS", 1);
         t.pair128 = env("NML_TUNE_PAIR128", 1);
         t.narrow = env("NML_TUNE_NARROW", 1);
+        t.deep = env("NML_TUNE_DEEP", 1);
     });
     return t;
 }
@@ -173,7 +175,7 @@ struct DeviceState {
 static DeviceState g_dev[64];
 static std::mutex g_dev_mutex;   // guards g_dev, g_static, g_prof and g_ref_ws
 static std::atomic<long long> g_launches{0};
-static std::atomic<long long> g_launches_of[6];  // by kind, see nml_debug_launch_count
+static std::atomic<long long> g_launches_of[9];  // by kind, see nml_debug_launch_count
 // Where kernels report an abandoned wait.  The words live in the library image, so set-up needs no
 // allocation: their device addresses come from cudaGetSymbolAddress, once per device.
 static __device__ int g_status_word;
@@ -1664,7 +1666,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         const int vec = (!nchw && N % 4 == 0 && (reinterpret_cast<uintptr_t>(f.out) & 15) == 0) ? 1 : 0;
         const size_t items = vec ? total / 4 : total;
         // (from 64 x 2 x 2 pixels of 512 channels, 32768 items of 9 planes, a thread an item is as fast: 18.6 us, eight 19.5)
-        const bool deep = P.fsplit >= kFinishLanes && items <= 16384;
+        const bool deep = P.fsplit >= kFinishLanes && items <= 16384 && tune().deep;
         // (values one by one: a thread each while the grid still overlaps its predecessor; 3x3 s2 72 -> 77 at 58 x 58, batch 9, 34.1 us, a grid above
         // that limit 38.3)
         const size_t quarter = (total + 1023) / 1024;
@@ -1676,6 +1678,7 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
         };
         if (f.out_dtype == NML_F16) finish(deep ? finish_rows_deep_kernel<__half> : finish_rows_kernel<__half>, static_cast<__half*>(f.out), 0);
         else finish(deep ? finish_rows_deep_kernel<float> : finish_rows_kernel<float>, static_cast<float*>(f.out), f.round_f16);
+        if (deep) ++g_launches_of[NML_DEBUG_DEEP_FINISH];
         ++g_launches;
         NML_CUDA(cudaGetLastError());
     }
@@ -2042,7 +2045,9 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         const int row_len4 = P.wpatch ? static_cast<int>(total4) : g.patch_c / 4;
         const size_t group_bytes = kReducePlain * 64 * (P.n_taps | 1) * sizeof(float);
         // Many planes of a small gradient: several threads an element, or a few blocks walk the planes one load latency at a time.
+        bool several = false;
         if (rows4 && split > 8 && (P.wpatch || total4 <= 16384)) {
+            several = true;
             helper_launch(4 * kSms, wgrad_reduce_deep4_kernel, static_cast<unsigned>((total4 + 31) / 32), dim3(32, 8), 0, st, planes, g.dw, split, plane_elems, total4,
                           row_len4, static_cast<size_t>(plane_rows));
         } else if (rows4) {
@@ -2051,6 +2056,7 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
         } else if (!P.wpatch && !P.kw_pack && g.patch_c % 4 == 0 && g.plain_c <= 65535 && group_bytes <= 48 * 1024) {
             const dim3 blocks(ceil_div(g.patch_c, 64), ceil_div(g.plain_c, kReducePlain));
             const bool deep = split >= 4 * kReduceGroups && blocks.x * blocks.y <= kSms && kReduceGroups * group_bytes <= 48 * 1024;
+            several = deep;
             helper_launch(4 * kSms, deep ? wgrad_reduce_taps_kernel<kReduceGroups> : wgrad_reduce_taps_kernel<1>, blocks, dim3(256, deep ? kReduceGroups : 1),
                          (deep ? kReduceGroups : 1) * group_bytes, st, planes, g.dw, split, plane_elems, g.patch_c, g.plain_c, P.n_taps, P.c_blocks, mi.kb, plane_rows);
         } else {
@@ -2058,12 +2064,14 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             // (one tap: the planes are read in dW's order, so that a thread an element is as fast from the size on where a grid of four no longer starts
             // beside its predecessor: 307 x 177 20.5 us so, 18.1 with a thread each, 238 x 200 28.1 and 24.9; 83 x 30 x 25 21.8 and 28.1)
             const bool deep = split >= 16 && dw_elems <= (T > 1 ? 65536 : 64 * 4 * kSms);
+            several = deep;
             const int elems = deep ? 64 : 256;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + elems - 1) / elems, 148 * 16));
             helper_launch(4 * kSms, deep ? wgrad_reduce_kernel<4> : wgrad_reduce_kernel<1>, blocks, dim3(elems, deep ? 4 : 1), 0, st, planes, g.dw, split, plane_elems,
                           dw_elems, layout, g.patch_c, P.n_taps, P.kw_count, P.c_blocks, mi.kb, plane_rows);
         }
         ++g_launches;
+        if (several) ++g_launches_of[NML_DEBUG_DEEP_SUMS];
         NML_CUDA(cudaGetLastError());
     }
     if (later.out) {
@@ -2287,6 +2295,7 @@ static int conv_pass(const nml_conv_desc* d, int pass, const void* in0, const vo
         l.rows = static_cast<int>(pixels); l.in_features = d->c_in; l.out_features = d->c_out;
         l.in_dtype = d->in_dtype; l.out_dtype = d->out_dtype; l.w_dtype = d->w_dtype; l.math = d->math; l.round_out_f16 = d->round_out_f16;
         const Pointwise conv = {add, add_mask, add_below, d->batch, d->h, d->w};
+        if (!ws.dry) ++g_launches_of[NML_DEBUG_POINTWISE];
         return linear_pass(&l, pass, in0, in1, bias, out, db, ws, st, &conv);
     }
     // Other tensors become images of one row, so that channel-major stores run on over the ends of the rows (small images find better
@@ -2761,7 +2770,7 @@ int nml_device_status(int* code) {
 
 long long nml_launch_count(void) { return g_launches.load() + nml_layers_launch_count(); }
 
-long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 6 ? g_launches_of[kind].load() : -1; }
+long long nml_debug_launch_count(int kind) { return kind >= 0 && kind < 9 ? g_launches_of[kind].load() : -1; }
 
 int nml_profile_begin(int max_records) {
     if (max_records <= 0 || max_records > 1 << 16) return NML_ERR_INVALID;

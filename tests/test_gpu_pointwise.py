@@ -3,10 +3,15 @@ import pytest
 import torch
 
 from gpu_util import assert_f32
-from nectarml_b200 import ops
+from nectarml_b200 import _lib, ops
 from nectarml_b200.ops import ConvGeometry
 
 pytestmark = pytest.mark.gpu
+
+
+def as_linear():
+    """Passes of 1x1 layers that went through the Linear layer's rules so far."""
+    return _lib.load().nml_debug_launch_count(8)
 
 
 def tensors(g, layout, dtype, seed, shift=0):
@@ -28,6 +33,7 @@ def test_fp16_rows(n, c_in, h, w, c_out, shift):
     wd, rows = wt.double().view(c_out, c_in), n * h * w
     xd, dyd = x.double().view(rows, c_in), dy.double().view(rows, c_out)
     want = xd @ wd.t() + b.double()
+    before = as_linear()
     y = ops.conv_forward(g, x, wt, b, layout="nhwc").double().view(rows, c_out)
     # one rounding to fp16, or two where a ragged row's bias is added to the rounded sum
     assert ((y - want).abs() <= 2.0 ** -10 * (want.abs() + b.double().abs() + want.abs().amax() / 64)).all()
@@ -37,6 +43,7 @@ def test_fp16_rows(n, c_in, h, w, c_out, shift):
     dw, db = ops.conv_backward_weight(g, x, dy, layout="nhwc")
     assert_f32(dw.view(c_out, c_in).cpu(), (dyd.t() @ xd).cpu(), "dw")
     assert_f32(db.cpu(), dyd.sum(0).cpu(), "db")
+    assert as_linear() == before + 3
     ops.device_status()
 
 

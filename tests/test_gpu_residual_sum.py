@@ -11,10 +11,11 @@ from nectarml_b200.ops import ConvGeometry
 pytestmark = pytest.mark.gpu
 
 
-# a tile of one and of several pieces, ragged pixels, the patch walk, the phases of a strided gather, a K loop split over CTAs, channels
-# that no TMA store takes
+# a tile of one and of several pieces, ragged pixels, the patch walk, the phases of a strided gather, a K loop split over CTAs, widths that
+# end within a piece, and eight channels, which no TMA store takes (accepted for the phases of a stride alone)
 @pytest.mark.parametrize("n,c_in,hw,c_out,k,s", [
-    (4, 256, 28, 64, 1, 1), (3, 64, 13, 128, 3, 1), (2, 128, 15, 64, 3, 2), (2, 512, 4, 512, 3, 1), (3, 24, 9, 40, 3, 1), (2, 72, 11, 16, 1, 1), (5, 320, 7, 64, 1, 2)])
+    (4, 256, 28, 64, 1, 1), (3, 64, 13, 128, 3, 1), (2, 128, 15, 64, 3, 2), (2, 512, 4, 512, 3, 1), (3, 24, 9, 40, 3, 1), (2, 72, 11, 16, 1, 1), (5, 320, 7, 64, 1, 2),
+    (3, 8, 11, 40, 3, 2), (2, 8, 64, 24, 1, 2)])
 @pytest.mark.parametrize("masked", [False, True])
 def test_input_gradient_with_an_addend(n, c_in, hw, c_out, k, s, masked):
     gen = torch.Generator(device="cuda").manual_seed(c_in + hw)
@@ -50,6 +51,13 @@ def test_sums_beside_pairs(n, c_in, hw, c_out, k, s, kernels):
     before = ops.launch_count()
     test_input_gradient_with_an_addend(n, c_in, hw, c_out, k, s, True)
     assert ops.launch_count() - before == kernels
+
+
+@pytest.mark.parametrize("c_in,hw,k,s,in_epilogue", [(24, 9, 3, 1, True), (72, 11, 1, 1, True), (72, 12, 3, 2, True), (8, 11, 3, 2, False), (8, 12, 1, 2, False)])
+def test_sums_of_narrow_results(c_in, hw, k, s, in_epilogue):
+    before = sums_in_epilogues()
+    test_input_gradient_with_an_addend(2, c_in, hw, 40, k, s, True)
+    assert sums_in_epilogues() - before == int(in_epilogue)
 
 
 # the mask's bytes may start anywhere: widths whose pieces are whole groups of eight bytes, and one whose are not

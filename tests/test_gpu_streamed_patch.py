@@ -21,10 +21,11 @@ def conv(x, w, g):
 
 
 # one channel block and a broken one, taps in whole stages and not (9 of 9, 25 and 49 of fewer; 4 a phase in fp32), one column tile of 16 ... 192 columns,
-# tiles hanging over the image, several tiles per CTA
+# tiles hanging over the image, several tiles per CTA, the phases of a strided gather: nine taps each, and 9, 12, 12 and 16
 @pytest.mark.parametrize("n,c_in,hw,c_out,k,s,transposed", [
     (9, 256, 32, 64, 3, 1, False), (9, 200, 31, 24, 5, 1, False), (87, 64, 31, 144, 3, 1, False), (4, 136, 48, 192, 3, 1, False), (40, 520, 16, 9, 3, 1, True),
-    (3, 256, 61, 40, 7, 1, False), (9, 640, 47, 16, 3, 1, False)])
+    (3, 256, 61, 40, 7, 1, False), (9, 640, 47, 16, 3, 1, False),
+    (4, 200, 47, 40, 6, 2, True), (3, 136, 61, 24, 7, 2, True)])
 def test_fp16(n, c_in, hw, c_out, k, s, transposed):
     gen = torch.Generator(device="cuda").manual_seed(c_in + c_out)
     g = ConvGeometry(n, c_in, hw, hw, c_out, k, k, (s, s), (k // 2 if s == 1 else 1,) * 2, transposed=transposed)

@@ -611,9 +611,9 @@ static void choose_box(int bits, int gw, int gh, int gn, int s_w, int s_h, int* 
         }
     }
     // A box at least 2^prefer_w_log2 pixels wide (whole 128-byte runs for pixel-major stores) is taken
-    // when it costs at most 15 % more tiles and no further round of them (or 3 % more rounds:
-    // fp32 1x1 16 -> 832 at 54 x 54, batch 40, boxes of eight pixels in 43 rounds 442 us, of 32 in 44 105 us): 3x3 96 -> 96 at 56 x 56, batch 16, fp16 31.1 -> 27.6 us
-    // with 392 tiles instead of 448; 128 -> 128 at 28 x 28, batch 16, 112 tiles instead of 98 in one round, 17.1 -> 15.9.
+    // when it costs at most 15 % more tiles and no further round of them, or 3 % more rounds: fp32 1x1 16 -> 832 at 54 x 54, batch 144, boxes
+    // of eight pixels in 156 rounds 1337 us, wide ones in 157 452 (of 327 random channel-major layers of many rounds five took 0.56 to 0.95
+    // of the time so, none more than 1.04; with 6 % three gain and three lose as much).  3x3 96 -> 96 at 56 x 56, batch 16, fp16 31.1 -> 27.6 us with 392 tiles instead of 448; 128 -> 128 at 28 x 28, batch 16, 112 tiles instead of 98 in one round, 17.1 -> 15.9.
     // 3xTF32 tiles are 128 columns wide: 256 -> 256 at 56 x 56, batch 8, 392 tiles instead of 448 154 -> 124 us.  Their narrow
     // boxes have to save a round of several, though: where all run at once nothing overlaps the drain (`split`; 128 -> 384 at
     // 28 x 28, batch 8, 49.1 us in two rounds of wide boxes, 54.2 in one of narrow ones).
@@ -716,33 +716,33 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
             P.w_coalesce = (tune().wcoal && 32 * run * 4 <= P.ring_bytes && P.num_tiles <= limited(ds->sms)) ? 1 : 0;
         }
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
+    } else if (P.patch && P.b_taps) {
+        // [B stages][patch buffers]: two channel blocks' patches, and the taps of as much of a channel block to a stage as two stages
+        // have room for.  (What a stage costs besides its MMAs, about 400 clocks, is spread over its taps: 3x3 256 -> 64 at 32 x 32, batch 64,
+        // two taps to a stage 44 us, three 38, five 35, nine 33.)
+        P.ka = 1;
+        const int slice = P.planes * P.bn * 128, patches = P.planes * P.patch_bytes;
+        P.stg_bufs = 1;
+        int avail = 232448 - fixed - P.epi_warps * kStagingBufBytes - 2 * patches;
+        if (avail < 3 * slice && P.epi_warps == 8) {
+            P.epi_warps = 4;
+            P.epi_alt = 0;
+            P.tbufs_log2 = std::min(P.tbufs_log2, 1);
+            avail += 4 * kStagingBufBytes;
+        }
+        if (avail < 2 * slice) return NML_ERR_UNSUPPORTED;  // (two patches of 130 KB at most leave more)
+        const int most = std::max(1, std::min(P.planes == 2 ? kStreamTapsSplit : kStreamTaps, avail / slice / 2));
+        P.b_taps = ceil_div(P.b_taps, ceil_div(P.b_taps, most));
+        P.stages = std::min(8, avail / (P.b_taps * slice));
+        avail -= P.stages * P.b_taps * slice;
+        P.a_stages = std::min(4, 2 + avail / patches);
+        P.a_ring_off = P.stages * P.b_taps * slice;
+        P.ring_bytes = P.a_ring_off + P.a_stages * patches;
+        P.issuers = 1;
+        smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
     } else if (P.patch) {
         // [resident B slices][patch buffers][staging][bias][barriers]
         P.ka = 1;
-        if (P.b_taps) {
-            // [B stages][patch buffers]: two channel blocks' patches, and the taps of as much of a channel block to a stage as two stages
-            // have room for.  (What a stage costs besides its MMAs, about 400 clocks, is spread over its taps: 3x3 256 -> 64 at 32 x 32, batch 64,
-            // two taps to a stage 44 us, three 38, five 35, nine 33.)
-            const int slice = P.planes * P.bn * 128, patches = P.planes * P.patch_bytes;
-            P.stg_bufs = 1;
-            int avail = 232448 - fixed - P.epi_warps * kStagingBufBytes - 2 * patches;
-            if (avail < 3 * slice && P.epi_warps == 8) {
-                P.epi_warps = 4;
-                P.epi_alt = 0;
-                P.tbufs_log2 = std::min(P.tbufs_log2, 1);
-                avail += 4 * kStagingBufBytes;
-            }
-            if (avail < 2 * slice) return NML_ERR_UNSUPPORTED;  // (two patches of 130 KB at most leave more)
-            const int most = std::max(1, std::min(P.planes == 2 ? kStreamTapsSplit : kStreamTaps, avail / slice / 2));
-            P.b_taps = ceil_div(P.b_taps, ceil_div(P.b_taps, most));
-            P.stages = std::min(8, avail / (P.b_taps * slice));
-            avail -= P.stages * P.b_taps * slice;
-            P.a_stages = std::min(4, 2 + avail / patches);
-            P.a_ring_off = P.stages * P.b_taps * slice;
-            P.ring_bytes = P.a_ring_off + P.a_stages * patches;
-            P.issuers = 1;
-            smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
-        } else {
         const int res_bytes = P.c_blocks * P.n_taps * P.bn * P.b_row_bytes;  // the taps of every phase
         P.stg_bufs = P.epi_warps == 8 ? 1 : 2;  // (alternate groups return to a buffer after two tiles; patches need the room)
         int avail = 232448 - fixed - P.epi_warps * P.stg_bufs * kStagingBufBytes;
@@ -764,7 +764,6 @@ static int launch_kernel(KParams& P, DeviceState* ds, cudaStream_t st, int* open
         P.a_ring_off = static_cast<int>(round_up(res_bytes, 1024));
         P.ring_bytes = P.a_ring_off + P.a_stages * P.patch_bytes;
         smem = static_cast<size_t>(P.ring_bytes) + P.epi_warps * P.stg_bufs * kStagingBufBytes + fixed;
-        }
     } else {
     // (a double tile's warps have one buffer each, or none where they store from registers)
     int stages2 = P.dbl ? 0 : (232448 - fixed - P.epi_warps * 2 * kStagingBufBytes) / stage_bytes;

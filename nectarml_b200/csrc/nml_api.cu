@@ -271,7 +271,7 @@ static int load_helper_kernels() {
         (const void*)pack_phase_weights_kernel<__half, float>, (const void*)pack_phase_weights_kernel<__half, __half>,
         (const void*)to_float_kernel<__half>, (const void*)colsum_finish_kernel,
         (const void*)add_masked_kernel, (const void*)repack_half_tile_kernel, (const void*)repack_half_rows_kernel, (const void*)wgrad_reduce_taps_kernel<1>, (const void*)wgrad_reduce_taps_kernel<kReduceGroups>,
-        (const void*)wgrad_reduce_rows4_kernel, (const void*)wgrad_reduce_kernel<1>, (const void*)wgrad_reduce_kernel<4>, (const void*)wgrad_reduce_deep4_kernel,
+        (const void*)wgrad_reduce_rows4_kernel, (const void*)wgrad_reduce_kernel, (const void*)wgrad_reduce_lanes_kernel, (const void*)wgrad_reduce_deep4_kernel,
     };
     for (const void* f : fns) {
         cudaFuncAttributes a;
@@ -2062,11 +2062,11 @@ static int run_wgrad_like(const WgradLike& g, Bump& ws, cudaStream_t st) {
             const int layout = P.wpatch ? 0 : P.kw_pack ? 2 : 1;
             // (one tap: the planes are read in dW's order, so that a thread an element is as fast from the size on where a grid of four no longer starts
             // beside its predecessor: 307 x 177 20.5 us so, 18.1 with a thread each, 238 x 200 28.1 and 24.9; 83 x 30 x 25 21.8 and 28.1)
-            const bool deep = split >= 16 && dw_elems <= (T > 1 ? 65536 : 64 * 4 * kSms);
+            const bool deep = split >= 16 && dw_elems <= (T > 1 ? 65536 : 256 / kReduceLanes * 4 * kSms);
             several = deep;
-            const int elems = deep ? 64 : 256;
+            const int elems = deep ? 256 / kReduceLanes : 256;
             const int blocks = static_cast<int>(std::min<size_t>((dw_elems + elems - 1) / elems, 148 * 16));
-            helper_launch(4 * kSms, deep ? wgrad_reduce_kernel<4> : wgrad_reduce_kernel<1>, blocks, dim3(elems, deep ? 4 : 1), 0, st, planes, g.dw, split, plane_elems,
+            helper_launch(4 * kSms, deep ? wgrad_reduce_lanes_kernel : wgrad_reduce_kernel, blocks, dim3(elems, deep ? kReduceLanes : 1), 0, st, planes, g.dw, split, plane_elems,
                           dw_elems, layout, g.patch_c, P.n_taps, P.kw_count, P.c_blocks, mi.kb, plane_rows);
         }
         ++g_launches;

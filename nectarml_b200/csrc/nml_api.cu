@@ -2476,7 +2476,12 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     f.a_c = forward ? d->in_features : d->out_features;
     f.w = in1; f.w_dtype = d->w_dtype; f.d0 = d->out_features; f.d1 = d->in_features; f.kh = f.kw = 1;
     f.k_is_dim0 = forward ? 0 : 1;
-    f.w_direct = conv ? 2 : 1;
+    // Short rows of weights take TMA long to read in place, which a 1x1 convolution's copy (rows of whole slices) pays for where many tiles read
+    // them: 8 -> 96, 82650 rows, 18.0 us in place, copied 11.1; 104 -> 176, 105560 rows, 22.6 and 17.4; 8 -> 77, 27522 rows, 15.3 and 13.7; but
+    // 24 -> 150, 57876 rows, 27.3 and 26.6, 64 -> 313, 86848 rows, 59.8 and 61.7.
+    const long long row_tiles = 1ll * ceil_div(d->rows, kTileM) * ceil_div(d->out_features, 256);
+    const bool short_k = d->in_features <= 128 && d->in_features % 64 != 0 && row_tiles >= (d->in_features == 8 ? 1 : 4) * static_cast<long long>(kSms);
+    f.w_direct = !conv ? 1 : forward && short_k ? 0 : 2;
     // Input gradient: W [out][in] read in place is an MN-major B operand.  Where its rows are no whole groups of 64 it takes a load per
     // group and excludes CTA pairs, and a transposed fp16 copy W^T [in][out] (one coalesced pass over the weights, counted in the
     // pass's duration) pays from 2.2e9 products on, with 128 outputs (two K slices) and more: 12000 x 520 -> 2048 55.6 -> 36.4 us, 8192 x 328
@@ -2499,9 +2504,9 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     // by K slices (104 <- 24 at 62 x 29, batch 66, in place 19.4 us, copied 13.1; 72 <- 688, 42408 rows, 24.5 and 17.6; 8 <- 72, 44556 rows, 13.0
     // and 8.5; but 56 <- 576, 12980 rows, 9.3 and 10.9, 456 <- 16, 16968 rows, 10.1 and 10.6), or a long K loop (208 <- 1920, 4 rows, 14.2 and 12.2).
     const int last = d->in_features % 64;
-    const bool short_last = last != 0 && last <= (d->in_features < 64 ? 40 : 48);
+    const bool short_last = last != 0 && last <= (d->in_features < 64 ? 40 : d->in_features < 256 ? 56 : 48);
     const bool copied = conv && !forward && d->math == NML_MATH_F16 &&
-                        ((last != 0 && d->rows >= 120000) || (short_last && d->in_features < 256 && 1ll * d->rows * ceil_div(d->out_features, 64) >= 66000) ||
+                        ((last != 0 && d->rows >= 120000) || (short_last && d->in_features < 256 && 1ll * d->rows * ceil_div(d->out_features, 64) >= 60000) ||
                          (short_last && last <= 40 && d->in_features < 1000 && d->out_features >= 1300));
     if (conv && !forward && (pays || copied || conv->add)) {
         f.w_direct = 0;  // (repacked: that is the same copy)

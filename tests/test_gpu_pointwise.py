@@ -83,7 +83,7 @@ def test_weight_gradients_keep_the_sums_of_their_images(n, c_in, h, w, c_out, la
     ops.device_status()
 
 
-@pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(66, 104, 62, 29, 24, True), (60, 72, 31, 23, 200, True), (2, 208, 1, 2, 1920, True), (30, 56, 21, 20, 576, False),
+@pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(66, 104, 62, 29, 24, True), (60, 72, 31, 23, 200, True), (31, 248, 128, 16, 24, True), (2, 208, 1, 2, 1920, True), (30, 56, 21, 20, 576, False),
                                                     (8, 456, 46, 46, 16, False)])
 def test_input_gradients_of_broken_groups(n, c_in, h, w, c_out, copied):
     """Weights whose last group of 64 inputs is far from whole are transposed first (a launch more) where many tiles or a long K loop read it."""
@@ -94,5 +94,20 @@ def test_input_gradients_of_broken_groups(n, c_in, h, w, c_out, copied):
     launches = ops.launch_count() - launches
     want = dy.double() @ wt.double().view(c_out, c_in)
     assert ((dx.double() - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -13 * want.abs().amax()).all()
+    ops.device_status()
+    assert launches == 1 + int(copied)
+
+
+@pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(64, 8, 21, 16, 200, True), (41, 104, 47, 41, 24, True), (41, 40, 47, 41, 24, True), (41, 64, 47, 41, 24, False),
+                                                    (20, 104, 47, 41, 24, False), (30, 8, 25, 24, 24, False)])
+def test_short_rows_of_weights(n, c_in, h, w, c_out, copied):
+    """Weights of few input channels are copied into rows of whole slices (a launch more) where many tiles read them."""
+    g = ConvGeometry(n, c_in, h, w, c_out, 1, 1)
+    x, wt, _, _ = tensors(g, "nhwc", torch.float16, c_in)
+    launches = ops.launch_count()
+    y = ops.conv_forward(g, x, wt, None, layout="nhwc")
+    launches = ops.launch_count() - launches
+    want = x.double() @ wt.double().view(c_out, c_in).t()
+    assert ((y.double() - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -13 * want.abs().amax()).all()
     ops.device_status()
     assert launches == 1 + int(copied)

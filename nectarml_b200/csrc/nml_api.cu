@@ -1343,12 +1343,12 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
                 // (a small gain does not outlast the first patch of a single round: fp32 3x3 40 -> 40 at 52 x 52, batch 3, 17.1 us by boxes, 17.6 so)
                 pays = rounds(patches) * slice <= rounds(boxes) * 0.95 && (slice < 0.9 || rounds(boxes) >= 2);
             } else {
-                // More than 128 columns are one tile, two, or several of 64, of either walk; by estimated time, a slice's and a column's drain measured on
+                // More than 128 columns are one tile, two, or several of 64, of either walk; by estimated time, of a slice, a column's drain and a round fitted to
                 // 420 layers of 129 ... 224 channels (3x3 to 7x7; by boxes with their width / so: 5x5 29 -> 168 at 44 x 9, batch 3, 12.8 / 16.9 in one
                 // tile, stays; 40 -> 160 at 24 x 12, batch 8, 21.7 / 13.3 in three).  0.88 of the time by boxes alone in the mean.
                 const bool by_tma = rows_of_vectors && P.out_mode == OUT_NHWC;
                 const auto us = [&](long long m_tiles, const Width& w, double slice_us) {
-                    return rounds(m_tiles * w.n_tiles) * (k_loop * slice_us + 0.012 * w.bn);
+                    return rounds(m_tiles * w.n_tiles) * (k_loop * slice_us + 0.012 * w.bn + 0.6);
                 };
                 const Width box = tile_width(boxes, forced_width, by_tma);
                 // (boxes of up to 40 channels, short rows, take longer: 3x3 24 -> 216 at 15 x 85, batch 40, 30.5 / 21.7)

@@ -2480,7 +2480,7 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     // them: 8 -> 96, 82650 rows, 18.0 us in place, copied 11.1; 104 -> 176, 105560 rows, 22.6 and 17.4; 8 -> 77, 27522 rows, 15.3 and 13.7; but
     // 24 -> 150, 57876 rows, 27.3 and 26.6, 64 -> 313, 86848 rows, 59.8 and 61.7.
     const long long row_tiles = 1ll * ceil_div(d->rows, kTileM) * ceil_div(d->out_features, 256);
-    const bool short_k = d->in_features <= 128 && d->in_features % 64 != 0 && row_tiles >= (d->in_features == 8 ? 1 : 4) * static_cast<long long>(kSms);
+    const bool short_k = d->in_features <= 128 && d->in_features % 64 != 0 && row_tiles >= (d->in_features == 8 && d->out_features >= 48 ? 1 : 4) * static_cast<long long>(kSms);
     f.w_direct = !conv ? 1 : forward && short_k ? 0 : 2;
     // Input gradient: W [out][in] read in place is an MN-major B operand.  Where its rows are no whole groups of 64 it takes a load per
     // group and excludes CTA pairs, and a transposed fp16 copy W^T [in][out] (one coalesced pass over the weights, counted in the
@@ -2502,12 +2502,14 @@ static int linear_pass(const nml_linear_desc* d, int pass, const void* in0, cons
     const bool starts = (reinterpret_cast<uintptr_t>(in1) & 15) == 0;
     // 1x1 convolutions have scratch for the copy anyway, and take it also where a last group of inputs that is far from whole meets many rows of tiles,
     // by K slices (104 <- 24 at 62 x 29, batch 66, in place 19.4 us, copied 13.1; 72 <- 688, 42408 rows, 24.5 and 17.6; 8 <- 72, 44556 rows, 13.0
-    // and 8.5; but 56 <- 576, 12980 rows, 9.3 and 10.9, 456 <- 16, 16968 rows, 10.1 and 10.6), or a long K loop (208 <- 1920, 4 rows, 14.2 and 12.2).
+    // and 8.5; but 56 <- 576, 12980 rows, 9.3 and 10.9, 456 <- 16, 16968 rows, 10.1 and 10.6), or a long K loop (208 <- 1920, 4 rows, 14.2 and 12.2),
+    // or where the output gradient is converted anyway, beside the copy (392 <- 4, 46560 rows, 22.7 and 17.1; 512 <- 2, 113344 rows, 37.0 and 29.1).
     const int last = d->in_features % 64;
     const bool short_last = last != 0 && last <= (d->in_features < 64 ? 40 : d->in_features < 256 ? 56 : 48);
     const bool copied = conv && !forward && d->math == NML_MATH_F16 &&
                         ((last != 0 && d->rows >= 120000) || (short_last && d->in_features < 256 && 1ll * d->rows * ceil_div(d->out_features, 64) >= 60000) ||
-                         (short_last && last <= 40 && d->in_features < 1000 && d->out_features >= 1300));
+                         (short_last && last <= 40 && d->in_features < 1000 && d->out_features >= 1300) ||
+                         (d->out_features < 64 && d->out_features % 8 != 0 && 1ll * ceil_div(d->rows, kTileM) * ceil_div(d->in_features, 256) >= 2 * kSms));
     if (conv && !forward && (pays || copied || conv->add)) {
         f.w_direct = 0;  // (repacked: that is the same copy)
         f.add = conv->add; f.add_mask = conv->add_mask; f.add_below = conv->add_below;

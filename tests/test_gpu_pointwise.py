@@ -83,7 +83,7 @@ def test_weight_gradients_keep_the_sums_of_their_images(n, c_in, h, w, c_out, la
     ops.device_status()
 
 
-@pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(66, 104, 62, 29, 24, True), (60, 72, 31, 23, 200, True), (31, 248, 128, 16, 24, True), (2, 208, 1, 2, 1920, True), (30, 56, 21, 20, 576, False),
+@pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(66, 104, 62, 29, 24, True), (60, 72, 31, 23, 200, True), (31, 248, 128, 16, 24, True), (2, 208, 1, 2, 1920, True), (16, 480, 64, 43, 1, True), (4, 480, 64, 43, 1, False), (30, 56, 21, 20, 576, False),
                                                     (8, 456, 46, 46, 16, False)])
 def test_input_gradients_of_broken_groups(n, c_in, h, w, c_out, copied):
     """Weights whose last group of 64 inputs is far from whole are transposed first (a launch more) where many tiles or a long K loop read it."""
@@ -95,7 +95,7 @@ def test_input_gradients_of_broken_groups(n, c_in, h, w, c_out, copied):
     want = dy.double() @ wt.double().view(c_out, c_in)
     assert ((dx.double() - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -13 * want.abs().amax()).all()
     ops.device_status()
-    assert launches == 1 + int(copied)
+    assert launches == 1 + int(copied) + int(c_out % 8 != 0)  # (output gradients of broken vectors are converted)
 
 
 @pytest.mark.parametrize("n,c_in,h,w,c_out,copied", [(64, 8, 21, 16, 200, True), (41, 104, 47, 41, 24, True), (41, 40, 47, 41, 24, True), (41, 64, 47, 41, 24, False),

@@ -1391,9 +1391,10 @@ static int run_fprop_like(const FpropLike& f, Bump& ws, cudaStream_t st, int* op
     // Row-major results by TMA stores (see below), where the geometry allows them.  Up to eight columns have a short epilogue of their own, for
     // fp16 (one vector a row at most) and for the 16-column tiles of the resident patch walk.  Four and eight fp32 columns of other walks leave by
     // TMA where there are many (from a round of tiles of eight columns on: transposed 5x5 s3 5 -> 8 at 128 x 24, batch 58, short 229 us, TMA
-    // 162; linear 155624 x 16 -> 8 20.5 and 18.5; below it the short one saves 0.3 us: 1x1 s2 15 -> 4 at 24 x 64, batch 75, 10.4 and 11.9).
+    // 162; linear 155624 x 16 -> 8 20.5 and 18.5; below it the short one saves 0.3 us: 1x1 s2 15 -> 4 at 24 x 64, batch 75, 10.4 and
+    // 11.9) or have an fp16 bias, of which the short one wants a widened copy, a launch (linear 8 x 640 -> 8 7.4 and 6.2).
     // (Never phase-packed columns: they belong to several output pixels, and the packed image may be larger than the output.)
-    const bool short_rows = N <= 8 && (P.out_f16 || (P.patch && !P.b_taps) || out_pixels * N < 8ull * kTileM * kSms);
+    const bool short_rows = N <= 8 && (P.out_f16 || (P.patch && !P.b_taps) || (out_pixels * N < 8ull * kTileM * kSms && !bias_is_f16));
     const bool rows_by_tma = P.out_mode == OUT_NHWC && !P.shuf_sh && tune().tmastore && !short_rows && rows_of_vectors;
     int z_plan = 1;  // K slices per tile
     {

@@ -59,12 +59,12 @@ def test_convolution_rows(n, c_in, hw, c_out, k, s, transposed, dtype):
     ops.device_status()
 
 
-# four and eight fp32 columns: by TMA from 148 * 128 rows of eight columns on, below by the short epilogue, which takes a widened copy of an fp16
-# bias (a launch more); a few K slices, phases, and resident weights (tiles of 16
+# four and eight fp32 columns: by TMA from 148 * 128 rows of eight columns on, below so only with an fp16 bias, of which the short epilogue
+# takes a widened copy (a launch more); a few K slices, phases, and resident weights (tiles of 16
 # columns, always the short epilogue)
 @pytest.mark.parametrize("c_out", [4, 8])
 @pytest.mark.parametrize("n,c_in,h,w,k,s,transposed,by_tma", [
-    (1, 160, 148, 256, 1, 1, False, True), (1, 160, 147, 128, 1, 1, False, False), (3, 100, 151, 171, 1, 1, False, True), (2, 256, 75, 70, 1, 2, True, True),
+    (1, 160, 148, 256, 1, 1, False, True), (1, 160, 147, 128, 1, 1, False, True), (3, 100, 151, 171, 1, 1, False, True), (2, 256, 75, 70, 1, 2, True, True),
     (2, 40, 149, 167, 3, 1, False, False)])
 def test_four_and_eight_fp32_columns(c_out, n, c_in, h, w, k, s, transposed, by_tma):
     gen = torch.Generator(device="cuda").manual_seed(c_in + c_out)
@@ -74,14 +74,14 @@ def test_four_and_eight_fp32_columns(c_out, n, c_in, h, w, k, s, transposed, by_
     b = torch.randn(c_out, device="cuda", generator=gen).half()
     y, clean = guarded(*g.act_shape("out", "nhwc"), dtype=torch.float32)
     launches = [ops.launch_count()]
-    ops.conv_forward(g, x, wt, None, layout="nhwc", math="f16", out=y)
-    launches.append(ops.launch_count())
-    ops.conv_forward(g, x, wt, b, layout="nhwc", math="f16", out=y)
-    launches.append(ops.launch_count())
     conv = torch.nn.functional.conv_transpose2d if transposed else torch.nn.functional.conv2d
-    want = conv(x.permute(0, 3, 1, 2).double(), wt.double(), b.double(), stride=s, padding=k // 2).permute(0, 2, 3, 1)
-    assert (y.double() - want).abs().max() <= 1e-5 * want.abs().max()
-    assert clean()
+    want = conv(x.permute(0, 3, 1, 2).double(), wt.double(), stride=s, padding=k // 2).permute(0, 2, 3, 1)
+    for bias in (None, b):
+        ops.conv_forward(g, x, wt, bias, layout="nhwc", math="f16", out=y)
+        launches.append(ops.launch_count())
+        ref = want if bias is None else want + bias.double()
+        assert (y.double() - ref).abs().max() <= 1e-5 * ref.abs().max()
+        assert clean()
     ops.device_status()
     assert (launches[2] - launches[1]) - (launches[1] - launches[0]) == (0 if by_tma else 1)
 
